@@ -1,0 +1,195 @@
+// Exact search for a few queries: one pass over the rows, a thread per row (row_scan.cuh), the k best kept per CTA.
+//
+// The bound is the pass over the rows: 1M x 128 fp32 is 512 MB, 78 us at the measured copy rate.  Each distance is
+// the reference's chain over ascending dimensions, so what the CTAs keep is final.  Up to eight queries share the
+// pass (about 10 instructions per 16 row bytes and query keep it below the memory's time); a tensor-core tile of
+// 128 query rows would be mostly empty there.
+#pragma once
+
+#include "block_select.cuh"
+#include "dense.cuh"
+#include "row_scan.cuh"
+
+namespace vb200 {
+
+// Distance of one row to the query (widened, in shared memory), rows fetched sixteen bytes at a time with four
+// loads in flight where their alignment allows.
+template <typename E>
+__device__ __forceinline__ float
+bf_exact_distance(const E* __restrict__ x, const float* qf, uint32_t dim, bool l2) {
+    constexpr uint32_t VEC = 16 / sizeof(E);
+    float s = 0.f;
+    auto step = [&](float v, float q) {
+        if (l2) {
+            const float t = __fsub_rn(v, q);
+            s = fmaf(t, t, s);
+        } else {
+            s = fmaf(v, q, s);
+        }
+    };
+    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0 && dim % VEC == 0) {
+        const uint4* xv = reinterpret_cast<const uint4*>(x);
+        const uint32_t nv = dim / VEC;
+        for (uint32_t v0 = 0; v0 < nv; v0 += 4) {
+            uint4 w[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                w[u] = v0 + u < nv ? __ldg(xv + v0 + u) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                if (v0 + u < nv) {
+                    E e[VEC];
+                    *reinterpret_cast<uint4*>(e) = w[u];
+#pragma unroll
+                    for (uint32_t j = 0; j < VEC; ++j) {
+                        step(widen(e[j]), qf[(v0 + u) * VEC + j]);
+                    }
+                }
+            }
+        }
+    } else {
+        for (uint32_t d = 0; d < dim; ++d) {
+            step(widen(x[d]), qf[d]);
+        }
+    }
+    return l2 ? s : __fsub_rn(1.0f, s);
+}
+
+constexpr int BF_STREAM_QUERIES = 8;
+
+struct BfStream {
+    const void* queries;        // [nq x dim] fp32, or bf16 bit patterns
+    uint32_t nq, dim;
+    const unsigned char* base;  // [n x dim] rows in the index's type
+    uint64_t n;
+    uint32_t k, cap;            // results per query; per-CTA candidate buffer (a power of two >= k + 128)
+    uint32_t* bound;            // [nq] ordered value of some query's k-th best so far, 0xFFFFFFFF = none
+    uint64_t* part;             // [nq][grid][k]
+    const float* masked;        // [n] +inf for rows that are removed or filtered out, or null
+};
+
+template <int FMT, bool L2, int QN, int UNIT>
+__global__ void __launch_bounds__(RS_ROWS)
+bf_stream_kernel(const BfStream p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr uint32_t ELEM = FMT == ROW_F32 ? 4 : 2;
+    const uint32_t qpad = (p.dim + 7) / 8 * 8;
+    float* qs = reinterpret_cast<float*>(smem + RS_STAGES * RS_STAGE);
+    TileSelect<QN> ts;
+    float* unused;
+    tile_carve<QN>(reinterpret_cast<unsigned char*>(qs + QN * qpad), p.cap, 0, unused, ts);
+    ts.k = p.k;
+    ts.cap = p.cap;
+    const uint32_t q0 = blockIdx.y * QN;
+    const int here = static_cast<int>(p.nq - q0 < QN ? p.nq - q0 : QN);
+    for (uint32_t i = threadIdx.x; i < QN * qpad; i += RS_ROWS) {
+        const uint32_t qi = i / qpad, d = i - qi * qpad;
+        float v = 0.f;
+        if (static_cast<int>(qi) < here && d < p.dim) {
+            const uint64_t at = static_cast<uint64_t>(q0 + qi) * p.dim + d;
+            v = FMT == ROW_F32 ? static_cast<const float*>(p.queries)[at]
+                               : half_decode<SCAN_FMT_BF16>(static_cast<const uint16_t*>(p.queries)[at]);
+        }
+        qs[i] = v;
+    }
+    if (threadIdx.x < QN) {
+        const int qi = threadIdx.x;
+        ts.cnt[qi] = 0;
+        ts.qa[qi] = 0.f;
+        ts.qidx[qi] = q0 + qi;
+        ts.slot[qi] = (q0 + qi) * gridDim.x + blockIdx.x;
+        ts.set_bound(qi, qi < here ? 0xFFFFFFFFu : 0u);
+    }
+    __syncthreads();
+    uint32_t rounds = 0;
+    RowAcc<FMT, L2, QN> acc;
+    row_stream<UNIT>(p.base, static_cast<uint64_t>(p.dim) * ELEM, p.dim * ELEM, p.dim, p.n, blockIdx.x, gridDim.x, smem, qs, qpad, acc,
+                     [&](uint64_t row, bool valid) {
+                         if (valid) {
+#pragma unroll
+                             for (int i = 0; i < QN; ++i) {
+                                 if (i < here) {
+                                     const float v = L2 ? acc.acc[i] : __fsub_rn(1.0f, acc.acc[i]);
+                                     if (v <= ts.thrq[i] && (p.masked == nullptr || __ldg(p.masked + row) < INFINITY)) {
+                                         ts.push(i, v, static_cast<uint32_t>(row));
+                                     }
+                                 }
+                             }
+                         }
+                         __syncthreads();
+                         ts.make_room(here);
+                         __syncthreads();
+                         // every now and then the bounds of the CTAs meet
+                         if ((rounds++ & 7u) == 7u) {
+                             if (static_cast<int>(threadIdx.x) < here) {
+                                 const int qi = threadIdx.x;
+                                 const uint32_t mine = ts.thr[qi];
+                                 const uint32_t u = mine < 0xFF800000u ? atomicMin(p.bound + q0 + qi, mine)
+                                                                       : *reinterpret_cast<volatile uint32_t*>(p.bound + q0 + qi);
+                                 if (u < mine) {
+                                     ts.set_bound(qi, u);
+                                 }
+                             }
+                             __syncthreads();
+                         }
+                     });
+    __syncthreads();
+    ts.finish(here, p.part, p.bound);
+}
+
+// One CTA per query: the k best of its `n` partial keys (payload = row), as results.
+template <int T>
+__global__ void __launch_bounds__(T)
+bf_pick_kernel(const uint64_t* __restrict__ part, uint32_t n, uint32_t k, const int64_t* __restrict__ labels,
+               int64_t* __restrict__ ids, float* __restrict__ dists) {
+    __shared__ SelectScratch sel;
+    __shared__ __align__(16) uint64_t keys[SELECT_CAP];
+    __shared__ __align__(16) uint64_t best[1024];
+    const uint64_t* mine = part + static_cast<uint64_t>(blockIdx.x) * n;
+    const uint32_t found = block_select<T>(load_source([&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i) >> 32); }),
+                                           [&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i)); }, n, k, keys, sel);
+    block_sort_to<T>(keys, found, k, best);
+    for (uint32_t i = threadIdx.x; i < k; i += T) {
+        const bool there = i < found;
+        ids[static_cast<uint64_t>(blockIdx.x) * k + i] = there ? __ldg(labels + static_cast<uint32_t>(best[i])) : -1;
+        dists[static_cast<uint64_t>(blockIdx.x) * k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
+    }
+}
+
+// One CTA per query: the kcand best of its row of `n` nominating scores, re-scored in the reference's operation
+// order (an FMA chain over the dimensions, one thread per candidate: FP32Quantizer::ComputeDistImpl,
+// src/quantization/fp32_quantizer.cpp:163-190; HalfPrecisionQuantizer,
+// src/quantization/scalar_quantization/half_precision_quantizer.cpp:54-123), the k best of those as results.
+// Infinite scores belong to rows that are filtered out.
+template <typename E, int T>
+__global__ void __launch_bounds__(T)
+bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const E* __restrict__ queries, uint32_t dim,
+               const E* __restrict__ base, uint32_t kcand, uint32_t k, int metric, const int64_t* __restrict__ labels,
+               int64_t* __restrict__ ids, float* __restrict__ dists) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SelectScratch sel;
+    __shared__ __align__(16) uint64_t keys[SELECT_CAP];
+    __shared__ __align__(16) uint64_t best[1024];
+    float* qf = reinterpret_cast<float*>(smem);
+    const uint64_t q = blockIdx.x;
+    for (uint32_t d = threadIdx.x; d < dim; d += T) {
+        qf[d] = widen(queries[q * dim + d]);
+    }
+    const ScoreSource<true> src{reinterpret_cast<const uint32_t*>(scores + q * ld)};
+    const uint32_t found = block_select<T>(src, [](uint32_t i) { return i; }, n, kcand, keys, sel);
+    block_sort_to<T>(keys, found, kcand, best);
+    const uint32_t have = min(found, kcand);
+    for (uint32_t i = threadIdx.x; i < have; i += T) {
+        const uint32_t row = static_cast<uint32_t>(best[i]);
+        keys[i] = make_key(bf_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, metric == VB200_METRIC_L2), row);
+    }
+    block_sort_to<T>(keys, have, k, best);
+    for (uint32_t i = threadIdx.x; i < k; i += T) {
+        const bool there = i < have;
+        ids[q * k + i] = there ? __ldg(labels + static_cast<uint32_t>(best[i])) : -1;
+        dists[q * k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
+    }
+}
+
+}  // namespace vb200

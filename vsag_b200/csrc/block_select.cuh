@@ -1,0 +1,320 @@
+// Exact selection of the k smallest of n values by one CTA, without sorting the n values.
+//
+// What bounds it is the passes over the values, so it makes two: the first keeps one minimum per group of a
+// few values (groups interleave, so that neighbouring values land in different groups), and the k-th smallest
+// of those minima is an upper bound of the k-th smallest value, because the minima are k distinct values.  With
+// two or more groups per wanted value the bound lets through about 1.3 k values; the second pass collects
+// those, and only they are sorted.  Values that tie or crowd in such a way that the collection does not fit are
+// narrowed down by histograms over the ordered bit patterns until it does.
+#pragma once
+
+#include "common.cuh"
+
+namespace vb200 {
+
+constexpr uint32_t ORDERED_INF = 0xFF800000u;     // float_to_ordered(+inf): larger patterns are NaNs, never selected
+constexpr uint32_t SELECT_BINS = 1024;
+constexpr uint32_t SELECT_GROUPS = 1024;          // group minima kept at most
+constexpr uint32_t SELECT_CAP = 2048;             // values collected at most
+
+struct SelectScratch {
+    uint32_t hist[SELECT_BINS];       // also the group minima's home: the two are never needed together
+    uint32_t minima[SELECT_GROUPS];
+    uint32_t warp_part[32];
+    uint32_t lo, hi, total, pick, upto, before, count;
+};
+
+// Inclusive prefix sum over the T threads of the CTA; every thread calls it, `part` is a scratch of 32 words.
+template <int T>
+__device__ __forceinline__ uint32_t
+block_inclusive_sum(uint32_t v, uint32_t* part) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= static_cast<uint32_t>(o)) {
+            v += u;
+        }
+    }
+    __syncthreads();
+    if (lane == 31) {
+        part[warp] = v;
+    }
+    __syncthreads();
+    uint32_t add = 0;
+#pragma unroll
+    for (int w = 0; w < T / 32; ++w) {
+        add += static_cast<uint32_t>(w) < warp ? part[w] : 0u;
+    }
+    return v + add;
+}
+
+// A source hands out n ordered values: at(i) is value number i; walk calls visit(i, value) for a share of the
+// numbers, thread `first` of `step`, such that the shares of first = 0 .. step-1 cover every number once.  The
+// loads of several values are issued together: a thread waits for memory once per batch.
+template <typename Load>
+struct LoadSource {   // any load(i)
+    Load load;
+    __device__ __forceinline__ uint32_t
+    at(uint32_t i) const {
+        return load(i);
+    }
+    template <typename Visit>
+    __device__ __forceinline__ void
+    walk(uint32_t first, uint32_t step, uint32_t n, Visit visit) const {
+        uint32_t i = first;
+        for (; i < n && n - i > 7 * step; i += 8 * step) {
+            uint32_t u[8];
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                u[j] = load(i + j * step);
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                visit(i + j * step, u[j]);
+            }
+        }
+        for (; i < n; i += step) {
+            visit(i, load(i));
+        }
+    }
+};
+
+template <typename Load>
+__device__ __forceinline__ LoadSource<Load>
+load_source(Load load) {
+    return LoadSource<Load>{load};
+}
+
+// Scores in memory, 16-byte aligned and readable up to a multiple of four.
+template <bool SKIP_INF = false>
+struct ScoreSource {
+    const uint32_t* scores;   // fp32 bit patterns
+    __device__ __forceinline__ static uint32_t
+    ordered(uint32_t b) {
+        const uint32_t u = (b & 0x80000000u) ? ~b : (b | 0x80000000u);   // float_to_ordered
+        return SKIP_INF && u == ORDERED_INF ? 0xFFFFFFFFu : u;
+    }
+    __device__ __forceinline__ uint32_t
+    at(uint32_t i) const {
+        return ordered(__ldg(scores + i));
+    }
+    template <typename Visit>
+    __device__ __forceinline__ void
+    walk(uint32_t first, uint32_t step, uint32_t n, Visit visit) const {
+        const uint32_t n4 = (n + 3) / 4;
+        const uint4* v = reinterpret_cast<const uint4*>(scores);
+        for (uint32_t i = first; i < n4; i += 4 * step) {
+            uint4 u[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                u[j] = i + j * step < n4 ? __ldg(v + i + j * step) : make_uint4(0x7FFFFFFFu, 0x7FFFFFFFu, 0x7FFFFFFFu, 0x7FFFFFFFu);
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t at4 = 4 * (i + j * step);
+                const uint32_t w[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+#pragma unroll
+                for (uint32_t c = 0; c < 4; ++c) {
+                    if (at4 + c < n) {
+                        visit(at4 + c, ordered(w[c]));
+                    }
+                }
+            }
+        }
+    }
+};
+
+// An ordered value t such that at least k of the n values are <= t, and at most `cap` unless more than that
+// tie at t exactly.  *upto = how many are <= t.  Values above ORDERED_INF do not take part; with fewer than k
+// taking part, t = ORDERED_INF.
+template <int T, typename Source>
+__device__ uint32_t
+block_bound(const Source& src, uint32_t n, uint32_t k, uint32_t cap, SelectScratch& s, uint32_t* upto) {
+    uint32_t mn = 0xFFFFFFFFu, mx = 0, have = 0;
+    src.walk(threadIdx.x, T, n, [&](uint32_t, uint32_t u) {
+        if (u <= ORDERED_INF) {
+            mn = min(mn, u);
+            mx = max(mx, u);
+            ++have;
+        }
+    });
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s.lo = 0xFFFFFFFFu;
+        s.hi = 0;
+        s.total = 0;
+    }
+    __syncthreads();
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    have = __reduce_add_sync(0xffffffffu, have);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&s.lo, mn);
+        atomicMax(&s.hi, mx);
+        atomicAdd(&s.total, have);
+    }
+    __syncthreads();
+    uint32_t lo = s.lo, hi = s.hi, below = 0;
+    if (s.total <= k) {
+        *upto = s.total;
+        return ORDERED_INF;
+    }
+    for (;;) {
+        const uint32_t range = hi - lo;
+        const uint32_t shift = range < SELECT_BINS ? 0u : static_cast<uint32_t>(22 - __clz(range));   // range >> shift < 1024
+        for (uint32_t b = threadIdx.x; b < SELECT_BINS; b += T) {
+            s.hist[b] = 0;
+        }
+        __syncthreads();
+        src.walk(threadIdx.x, T, n, [&](uint32_t, uint32_t u) {
+            if (u >= lo && u <= hi) {
+                atomicAdd(&s.hist[(u - lo) >> shift], 1u);
+            }
+        });
+        __syncthreads();
+        constexpr int PER = SELECT_BINS / T;
+        uint32_t c[PER], sum = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            c[j] = s.hist[threadIdx.x * PER + j];
+            sum += c[j];
+        }
+        const uint32_t incl = block_inclusive_sum<T>(sum, s.warp_part);
+        uint32_t run = below + incl - sum;
+        if (run < k && run + sum >= k) {
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
+                if (run < k && run + c[j] >= k) {
+                    s.pick = threadIdx.x * PER + j;
+                    s.upto = run + c[j];
+                    s.before = run;
+                }
+                run += c[j];
+            }
+        }
+        __syncthreads();
+        const uint32_t bin = s.pick, reached = s.upto, before = s.before;
+        __syncthreads();
+        const uint32_t bin_lo = lo + (bin << shift);
+        const uint32_t last = bin_lo + ((1u << shift) - 1u);
+        if (reached <= cap || shift == 0) {
+            *upto = reached;
+            return min(last, hi);
+        }
+        below = before;
+        hi = min(last, hi);
+        lo = bin_lo;
+    }
+}
+
+// The k smallest of the n values (ties: smallest payload first) among a few more, unsorted, as
+// (value << 32 | payload(i)) in keys[SELECT_CAP]; returns how many were collected (>= k when that many take
+// part, <= SELECT_CAP).  k <= 1024.  Every value is read two or three times.
+template <int T, typename Source, typename Payload>
+__device__ uint32_t
+block_select(const Source& src, const Payload& payload, uint32_t n, uint32_t k, uint64_t* keys, SelectScratch& s) {
+    uint32_t bound = ORDERED_INF;
+    bool counted = false;
+    if (n > 256 && n > k) {
+        // groups: T threads times a power of two, two or more per wanted value as far as they go
+        uint32_t per = 1;
+        while (per * T < 2 * k && per * 2 * T <= SELECT_GROUPS) {
+            per <<= 1;
+        }
+        const uint32_t groups = per * T;
+        if (4 * k <= 3 * groups) {
+            for (uint32_t g = 0; g < per; ++g) {
+                uint32_t mn = 0xFFFFFFFFu;
+                src.walk(g * T + threadIdx.x, groups, n, [&](uint32_t, uint32_t u) { mn = min(mn, u); });
+                s.minima[g * T + threadIdx.x] = mn;
+            }
+            __syncthreads();
+            uint32_t upto;
+            bound = block_bound<T>(load_source([&](uint32_t i) { return s.minima[i]; }), groups, k, k + k / 8 + 8, s, &upto);
+        } else {
+            uint32_t upto;
+            bound = block_bound<T>(src, n, k, SELECT_CAP, s, &upto);
+            counted = upto <= SELECT_CAP;
+        }
+    }
+    auto collect = [&](uint32_t t, bool strict) -> uint32_t {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s.count = 0;
+        }
+        __syncthreads();
+        src.walk(threadIdx.x, T, n, [&](uint32_t i, uint32_t u) {
+            if (u <= ORDERED_INF && (strict ? u < t : u <= t)) {
+                const uint32_t slot = atomicAdd(&s.count, 1u);
+                if (slot < SELECT_CAP) {
+                    keys[slot] = (static_cast<uint64_t>(u) << 32) | payload(i);
+                }
+            }
+        });
+        __syncthreads();
+        return s.count;
+    };
+    uint32_t count = collect(bound, false);
+    if (count <= SELECT_CAP || counted) {
+        return count;
+    }
+    uint32_t upto;
+    bound = block_bound<T>(src, n, k, SELECT_CAP, s, &upto);
+    if (upto <= SELECT_CAP) {
+        return collect(bound, false);
+    }
+    // more values tie at the k-th than fit: everything below it, then the ties with the smallest payloads
+    const uint32_t below = collect(bound, true);
+    uint32_t ties;
+    const uint32_t last = block_bound<T>(
+        load_source([&](uint32_t i) { return src.at(i) == bound ? min(payload(i), ORDERED_INF) : 0xFFFFFFFFu; }), n, k - below, k - below, s, &ties);
+    for (uint32_t i = threadIdx.x; i < n; i += T) {
+        if (src.at(i) == bound) {
+            const uint32_t p = payload(i);
+            if (p <= last) {
+                const uint32_t slot = atomicAdd(&s.count, 1u);
+                if (slot < SELECT_CAP) {
+                    keys[slot] = (static_cast<uint64_t>(bound) << 32) | p;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    return min(s.count, SELECT_CAP);
+}
+
+// Sorts `count` distinct keys and leaves the `keep` smallest, ascending, in out (a different buffer).  Up to 512
+// keys every thread counts how many are smaller than its own, one pass and one barrier instead of a sorting
+// network's many; more go through the network (keys must then have room for the next power of two).
+template <int T>
+__device__ __forceinline__ void
+block_sort_to(uint64_t* keys, uint32_t count, uint32_t keep, uint64_t* out) {
+    __syncthreads();
+    if (count <= 512) {
+        for (uint32_t i = threadIdx.x; i < count; i += T) {
+            const uint64_t mine = keys[i];
+            uint32_t rank = 0;
+#pragma unroll 8
+            for (uint32_t j = 0; j < count; ++j) {
+                rank += keys[j] < mine ? 1u : 0u;
+            }
+            if (rank < keep) {
+                out[rank] = mine;
+            }
+        }
+        __syncthreads();
+        return;
+    }
+    const uint32_t n2 = next_pow2(count);
+    for (uint32_t i = count + threadIdx.x; i < n2; i += T) {
+        keys[i] = KEY_INF;
+    }
+    block_bitonic_sort(keys, n2);
+    for (uint32_t i = threadIdx.x; i < keep && i < count; i += T) {
+        out[i] = keys[i];
+    }
+    __syncthreads();
+}
+
+}  // namespace vb200

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "bf_stream.cuh"
 #include "dense.cuh"
 #include "kmeans.cuh"
 #include "comm.cuh"
@@ -11,6 +12,8 @@
 namespace vb200 {
 
 constexpr uint32_t BF_SLACK = 16;                 // candidates kept beyond k before re-scoring
+constexpr double BF_MATRIX_SCORES = 4e8;          // scores of a batch that goes through a score matrix, at most
+constexpr size_t BF_PINNED_BYTES = 256 * 1024;    // host results of a search that pass through pinned memory, at most
 constexpr uint64_t BF_COL_CHUNK = uint64_t{1} << 20;
 constexpr uint64_t BF_SLAB_FLOATS = uint64_t{256} << 20;  // 1 GiB of scores
 
@@ -258,6 +261,8 @@ struct vb200_bf {
     TcWorkspace tc;
     DevBuf<int64_t> out_ids;
     DevBuf<float> out_dists;
+    DevBuf<uint32_t> stream_bound;   // per query: a bound of its k-th best distance while rows stream by
+    PinnedBuf pinned;                // small host inputs and results
     std::mutex mu;
 };
 
@@ -481,19 +486,12 @@ vb200_bf_remove(vb200_bf_t ix, const int64_t* labels, uint64_t count, uint64_t* 
     return 0;
 }
 
-// Leaves the k best keys (payload = row) per query in ix->keys.
+// What every search starts with: the queries on the device (normalised for cosine, rounded for bf16 rows) and
+// the score bias per row -- |x|^2 for L2, none for IP, +inf for rows that are removed or filtered out.
 static int
-bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
+bf_stage(vb200_bf* ix, const float* queries, uint64_t nq, const float** q_out, const float** bias_out, bool* masked_out) {
     const uint32_t dim = ix->dim;
     const uint64_t n = ix->n;
-    uint32_t kcand = k + BF_SLACK;
-    if (kcand > n) {
-        kcand = static_cast<uint32_t>(n);
-    }
-    VB_CHECK_ARG(kcand <= 1024, "k = %u is too large (limit %u)", k, 1024 - BF_SLACK);
-    const bool l2 = ix->metric == VB200_METRIC_L2;
-    const bool bf16 = ix->quant == VB200_QUANT_BF16;
-
     const float* q_dev = queries;
     if (!is_device_pointer(queries)) {
         VB_TRY(ix->q_f32.reserve(nq * dim));
@@ -506,58 +504,88 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
         VB_TRY(normalize_rows_f32(q_dev, nq, dim, ix->q_unit.ptr));
         q_dev = ix->q_unit.ptr;
     }
-    if (bf16) {
+    if (ix->quant == VB200_QUANT_BF16) {
         VB_TRY(ix->q_bf16.reserve(nq * dim));
         VB_LAUNCH(float_to_bf16_kernel, static_cast<uint32_t>((nq * dim + 255) / 256), 256, 0, q_dev,
                   nq * dim, ix->q_bf16.ptr);
     }
-    // score bias per row: |x|^2 for L2, none for IP; +inf for rows that are removed or filtered out
-    const float* bias_all = l2 ? ix->norms.ptr : nullptr;
-    {
-        const vb200_filter* f = ix->filter;
-        const bool user_deny = f != nullptr && f->deny_inner_bits != nullptr && f->n_inner_bits > 0;
-        const bool user_labels = f != nullptr && f->invalid_label_bits != nullptr && f->n_label_bits > 0;
-        if (ix->n_removed > 0 || user_deny || user_labels) {
-            DevInput<uint32_t> deny;
-            DevInput<uint64_t> lbits;
-            if (user_deny) {
-                VB_TRY(deny.bind(f->deny_inner_bits, (f->n_inner_bits + 31) / 32));
-            }
-            if (user_labels) {
-                VB_TRY(lbits.bind(f->invalid_label_bits, (f->n_label_bits + 63) / 64));
-            }
-            VB_TRY(ix->masked_bias.reserve(n));
-            VB_LAUNCH(bf_masked_bias_kernel, static_cast<uint32_t>((n + 255) / 256), 256, 0, bias_all, n,
-                      ix->n_removed > 0 ? ix->tombstones.ptr : nullptr, user_deny ? deny.ptr : nullptr,
-                      user_deny ? f->n_inner_bits : 0, ix->labels.ptr, user_labels ? lbits.ptr : nullptr,
-                      user_labels ? f->n_label_bits : 0, ix->masked_bias.ptr);
-            VB_TRY(sync_stream());   // the staged bitmaps end with this scope
-            bias_all = ix->masked_bias.ptr;
+    const float* bias_all = ix->metric == VB200_METRIC_L2 ? ix->norms.ptr : nullptr;
+    const vb200_filter* f = ix->filter;
+    const bool user_deny = f != nullptr && f->deny_inner_bits != nullptr && f->n_inner_bits > 0;
+    const bool user_labels = f != nullptr && f->invalid_label_bits != nullptr && f->n_label_bits > 0;
+    *masked_out = ix->n_removed > 0 || user_deny || user_labels;
+    if (*masked_out) {
+        DevInput<uint32_t> deny;
+        DevInput<uint64_t> lbits;
+        if (user_deny) {
+            VB_TRY(deny.bind(f->deny_inner_bits, (f->n_inner_bits + 31) / 32));
         }
+        if (user_labels) {
+            VB_TRY(lbits.bind(f->invalid_label_bits, (f->n_label_bits + 63) / 64));
+        }
+        VB_TRY(ix->masked_bias.reserve(n));
+        VB_LAUNCH(bf_masked_bias_kernel, static_cast<uint32_t>((n + 255) / 256), 256, 0, bias_all, n,
+                  ix->n_removed > 0 ? ix->tombstones.ptr : nullptr, user_deny ? deny.ptr : nullptr,
+                  user_deny ? f->n_inner_bits : 0, ix->labels.ptr, user_labels ? lbits.ptr : nullptr,
+                  user_labels ? f->n_label_bits : 0, ix->masked_bias.ptr);
+        VB_TRY(sync_stream());   // the staged bitmaps end with this scope
+        bias_all = ix->masked_bias.ptr;
     }
+    *q_out = q_dev;
+    *bias_out = bias_all;
+    return 0;
+}
+
+// The rows as tiled bf16 terms for the tensor cores, made at the first search that needs them after an add.
+static int
+bf_tile_base(vb200_bf* ix) {
+    if (ix->tiled_valid) {
+        return 0;
+    }
+    const size_t elems = tc_tiled_elems(ix->n, ix->dim);
+    VB_TRY(ix->base_hi.reserve(elems));
+    if (ix->quant == VB200_QUANT_BF16) {
+        VB_TRY(tc_pretile_bf16(ix->base_bf16.ptr, ix->n, ix->dim, ix->base_hi.ptr));
+    } else {
+        VB_TRY(ix->base_lo.reserve(elems));
+        VB_TRY(tc_pretile_f32(ix->base_f32.ptr, ix->n, ix->dim, ix->base_hi.ptr, ix->base_lo.ptr));
+    }
+    ix->tiled_valid = true;
+    return 0;
+}
+
+static int
+bf_tile_queries(vb200_bf* ix, const float* q_dev, uint64_t nq) {
+    const size_t q_elems = tc_tiled_elems(nq, ix->dim);
+    VB_TRY(ix->q_hi.reserve(q_elems));
+    if (ix->quant == VB200_QUANT_BF16) {
+        return tc_pretile_bf16(ix->q_bf16.ptr, nq, ix->dim, ix->q_hi.ptr);
+    }
+    VB_TRY(ix->q_lo.reserve(q_elems));
+    return tc_pretile_f32(q_dev, nq, ix->dim, ix->q_hi.ptr, ix->q_lo.ptr);
+}
+
+// Leaves the k best keys (payload = row) per query in ix->keys.
+static int
+bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
+    const uint32_t dim = ix->dim;
+    const uint64_t n = ix->n;
+    uint32_t kcand = k + BF_SLACK;
+    if (kcand > n) {
+        kcand = static_cast<uint32_t>(n);
+    }
+    VB_CHECK_ARG(kcand <= 1024, "k = %u is too large (limit %u)", k, 1024 - BF_SLACK);
+    const bool l2 = ix->metric == VB200_METRIC_L2;
+    const bool bf16 = ix->quant == VB200_QUANT_BF16;
+    const float *q_dev = nullptr, *bias_all = nullptr;
+    bool masked = false;
+    VB_TRY(bf_stage(ix, queries, nq, &q_dev, &bias_all, &masked));
     // Large problems nominate candidates on the tensor cores; the exact re-scoring below is the
     // same either way.
     if (tensor_cores_enabled() && kcand <= tc_max_candidates(bf16 ? 1 : 3) && static_cast<double>(nq) * n * dim >= 2e10) {
         const uint32_t chunks = (dim + TC_KC - 1) / TC_KC;
-        if (!ix->tiled_valid) {
-            const size_t elems = tc_tiled_elems(n, dim);
-            VB_TRY(ix->base_hi.reserve(elems));
-            if (bf16) {
-                VB_TRY(tc_pretile_bf16(ix->base_bf16.ptr, n, dim, ix->base_hi.ptr));
-            } else {
-                VB_TRY(ix->base_lo.reserve(elems));
-                VB_TRY(tc_pretile_f32(ix->base_f32.ptr, n, dim, ix->base_hi.ptr, ix->base_lo.ptr));
-            }
-            ix->tiled_valid = true;
-        }
-        const size_t q_elems = tc_tiled_elems(nq, dim);
-        VB_TRY(ix->q_hi.reserve(q_elems));
-        if (bf16) {
-            VB_TRY(tc_pretile_bf16(ix->q_bf16.ptr, nq, dim, ix->q_hi.ptr));
-        } else {
-            VB_TRY(ix->q_lo.reserve(q_elems));
-            VB_TRY(tc_pretile_f32(q_dev, nq, dim, ix->q_hi.ptr, ix->q_lo.ptr));
-        }
+        VB_TRY(bf_tile_base(ix));
+        VB_TRY(bf_tile_queries(ix, q_dev, nq));
         TcOperand a{ix->q_hi.ptr, bf16 ? nullptr : ix->q_lo.ptr, nq, chunks};
         VB_TRY(ix->cand.reserve(nq * kcand));
         VB_TRY(ix->row_bound.reserve(nq));
@@ -658,6 +686,125 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
     return 0;
 }
 
+// A few queries: one pass over the rows (bf_stream.cuh) straight to results in device or pinned memory.
+static int
+bf_search_stream(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k, int64_t* ids_dev, float* dists_dev) {
+    const uint32_t dim = ix->dim;
+    const bool l2 = ix->metric == VB200_METRIC_L2, bf16 = ix->quant == VB200_QUANT_BF16;
+    const float *q_dev = nullptr, *bias = nullptr;
+    bool masked = false;
+    VB_TRY(bf_stage(ix, queries, nq, &q_dev, &bias, &masked));
+    BfStream p{};
+    p.queries = bf16 ? static_cast<const void*>(ix->q_bf16.ptr) : q_dev;
+    p.nq = static_cast<uint32_t>(nq);
+    p.dim = dim;
+    p.base = bf16 ? reinterpret_cast<const unsigned char*>(ix->base_bf16.ptr) : reinterpret_cast<const unsigned char*>(ix->base_f32.ptr);
+    p.n = ix->n;
+    p.k = k;
+    p.cap = next_pow2(k + RS_ROWS);
+    p.masked = masked ? bias : nullptr;
+    uint32_t qn = 1;
+    while (qn < nq && qn < BF_STREAM_QUERIES) {
+        qn *= 2;
+    }
+    auto smem_of = [&](uint32_t q) {
+        return RS_STAGES * RS_STAGE + static_cast<size_t>(q) * ((dim + 7) / 8 * 8) * sizeof(float) +
+               static_cast<size_t>(q) * (p.cap * sizeof(uint64_t) + 6 * sizeof(uint32_t));
+    };
+    while (qn > 1 && smem_of(qn) > 110 * 1024) {
+        qn /= 2;
+    }
+    const size_t smem = smem_of(qn);
+    VB_CHECK_ARG(smem <= 220 * 1024, "dim = %u is too large for the row scan", dim);
+    const size_t row_bytes = static_cast<size_t>(dim) * (bf16 ? 2 : 4);
+    const int unit = row_bytes % 16 == 0 ? 16 : (row_bytes % 4 == 0 ? 4 : 2);
+    void (*kernel)(const BfStream) = nullptr;
+#define VB_BF_UNIT(FMT, L2, QN)                                                                            \
+    kernel = unit == 16 ? bf_stream_kernel<FMT, L2, QN, 16>                                                \
+                        : (FMT == ROW_F32 || unit == 4 ? bf_stream_kernel<FMT, L2, QN, 4>                  \
+                                                       : bf_stream_kernel<FMT, L2, QN, FMT == ROW_F32 ? 4 : 2>)
+#define VB_BF_QN(FMT, L2)                          \
+    switch (qn) {                                  \
+        case 1: VB_BF_UNIT(FMT, L2, 1); break;     \
+        case 2: VB_BF_UNIT(FMT, L2, 2); break;     \
+        case 4: VB_BF_UNIT(FMT, L2, 4); break;     \
+        default: VB_BF_UNIT(FMT, L2, 8); break;    \
+    }
+    if (bf16) {
+        if (l2) {
+            VB_BF_QN(ROW_BF16, true)
+        } else {
+            VB_BF_QN(ROW_BF16, false)
+        }
+    } else if (l2) {
+        VB_BF_QN(ROW_F32, true)
+    } else {
+        VB_BF_QN(ROW_F32, false)
+    }
+#undef VB_BF_QN
+#undef VB_BF_UNIT
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    int per_sm = 0;
+    VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, RS_ROWS, smem));
+    const uint64_t chunks = (ix->n + RS_ROWS - 1) / RS_ROWS;
+    const uint32_t tiles = static_cast<uint32_t>((nq + qn - 1) / qn);
+    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(chunks, static_cast<uint64_t>(sm_count()) * std::max(per_sm, 1)));
+    VB_CHECK_ARG(nq * grid * k < 0xFFFFFFFFull, "query batch too large");
+    VB_TRY(ix->part.reserve(nq * grid * k));
+    VB_TRY(ix->stream_bound.reserve(nq));
+    VB_CUDA(cudaMemsetAsync(ix->stream_bound.ptr, 0xFF, nq * sizeof(uint32_t), current_stream()));
+    p.part = ix->part.ptr;
+    p.bound = ix->stream_bound.ptr;
+    VB_LAUNCH(kernel, dim3(grid, tiles), RS_ROWS, smem, p);
+    VB_LAUNCH(bf_pick_kernel<1024>, static_cast<uint32_t>(nq), 1024, 0, ix->part.ptr, grid * k, k, ix->labels.ptr, ids_dev, dists_dev);
+    return 0;
+}
+
+// Batches whose score matrix is worth writing: tensor-core scores in slices of queries whose scores stay in L2,
+// then a CTA per query that selects, re-scores and writes its results.
+constexpr uint64_t BF_SLICE_SCORES = uint64_t{24} << 20;   // 96 MiB of the 126 MB L2
+
+static int
+bf_search_scores(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k, int64_t* ids_dev, float* dists_dev) {
+    const uint32_t dim = ix->dim;
+    const bool l2 = ix->metric == VB200_METRIC_L2, bf16 = ix->quant == VB200_QUANT_BF16;
+    const float *q_dev = nullptr, *bias = nullptr;
+    bool masked = false;
+    VB_TRY(bf_stage(ix, queries, nq, &q_dev, &bias, &masked));
+    VB_TRY(bf_tile_base(ix));
+    VB_TRY(bf_tile_queries(ix, q_dev, nq));
+    const uint32_t chunks = (dim + TC_KC - 1) / TC_KC;
+    const uint64_t ld = (ix->n + 127) / 128 * 128;
+    uint64_t slice = BF_SLICE_SCORES / ld / TC_BM * TC_BM;   // whole row tiles
+    slice = slice < TC_BM ? TC_BM : slice;
+    VB_TRY(ix->scores.reserve(std::min(slice, nq) * ld));
+    VB_TRY(ix->tc.error_flag.reserve(2));
+    VB_CUDA(cudaMemsetAsync(ix->tc.error_flag.ptr, 0, 2 * sizeof(int), current_stream()));
+    const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks};
+    const uint32_t kcand = static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n));
+    const size_t smem = dim * sizeof(float);
+    VB_CHECK_ARG(smem <= 180 * 1024, "dim = %u is too large for the exact re-scoring step", dim);
+    for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
+        const uint64_t m = std::min(slice, nq - q0);
+        const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
+        const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks};
+        VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, bias, ix->scores.ptr, ld, ix->tc.error_flag.ptr));
+        if (bf16) {
+            auto kernel = bf_rows_kernel<uint16_t, 512>;
+            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 8192 ? 40 * 1024 : 0)));
+            VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, ix->scores.ptr, ld, static_cast<uint32_t>(ix->n),
+                      ix->q_bf16.ptr + q0 * dim, dim, ix->base_bf16.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k,
+                      dists_dev + q0 * k);
+        } else {
+            auto kernel = bf_rows_kernel<float, 512>;
+            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 8192 ? 40 * 1024 : 0)));
+            VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, ix->scores.ptr, ld, static_cast<uint32_t>(ix->n), q_dev + q0 * dim, dim,
+                      ix->base_f32.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k, dists_dev + q0 * k);
+        }
+    }
+    return 0;
+}
+
 static int
 bf_check_search(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
     VB_CHECK_ARG(ix != nullptr, "null index");
@@ -689,17 +836,69 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
         VB_CUDA(cudaMemcpy(dists, hd.data(), total * sizeof(float), cudaMemcpyDefault));
         return 0;
     }
+    // results go straight to device buffers, or to pinned memory when they are small; else through buffers here
+    const bool host_ids = !is_device_pointer(ids), host_d = !is_device_pointer(dists);
+    const bool pin_out = (host_ids || host_d) && total * 12 <= BF_PINNED_BYTES;
+    if (pin_out) {
+        VB_TRY(ix->pinned.reserve(total * 12));
+    } else {
+        if (host_ids) {
+            VB_TRY(ix->out_ids.reserve(total));
+        }
+        if (host_d) {
+            VB_TRY(ix->out_dists.reserve(total));
+        }
+    }
+    int64_t* pin_ids = static_cast<int64_t*>(ix->pinned.ptr);
+    float* pin_dists = pin_out ? reinterpret_cast<float*>(pin_ids + total) : nullptr;
+    int64_t* ids_dev = !host_ids ? ids : (pin_out ? pin_ids : ix->out_ids.ptr);
+    float* dists_dev = !host_d ? dists : (pin_out ? pin_dists : ix->out_dists.ptr);
+    const bool k_fits = std::min<uint64_t>(k + BF_SLACK, ix->n) <= 1024;
+    bool flagged = false;
+    int rc = 0;
     ix->filter = filter;
-    const int search_status = bf_search_keys(ix, queries, nq, k);
+    // Up to eight queries share one pass over the rows; more go to the tensor cores -- through a score matrix
+    // while that is cheaper than selecting as the scores appear (measured: up to about 4e8 scores), see
+    // bf_search_keys for the rest.
+    if (nq <= BF_STREAM_QUERIES && k_fits) {
+        rc = bf_search_stream(ix, queries, nq, k, ids_dev, dists_dev);
+    } else if (tensor_cores_enabled() && k_fits && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES) {
+        rc = bf_search_scores(ix, queries, nq, k, ids_dev, dists_dev);
+        flagged = true;
+    } else {
+        rc = bf_search_keys(ix, queries, nq, k);
+        if (rc == 0) {
+            VB_LAUNCH(bf_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ix->keys.ptr, total,
+                      ix->labels.ptr, ids_dev, dists_dev, nullptr);
+        }
+    }
     ix->filter = nullptr;
-    VB_TRY(search_status);
-    VB_TRY(ix->out_ids.reserve(total));
-    VB_TRY(ix->out_dists.reserve(total));
-    VB_LAUNCH(bf_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ix->keys.ptr, total,
-              ix->labels.ptr, ix->out_ids.ptr, ix->out_dists.ptr, nullptr);
-    VB_TRY(copy_out(ids, ix->out_ids.ptr, total));
-    VB_TRY(copy_out(dists, ix->out_dists.ptr, total));
-    return sync_stream();
+    VB_TRY(rc);
+    if (!pin_out) {
+        if (host_ids) {
+            VB_CUDA(cudaMemcpyAsync(ids, ids_dev, total * sizeof(int64_t), cudaMemcpyDeviceToHost, current_stream()));
+        }
+        if (host_d) {
+            VB_CUDA(cudaMemcpyAsync(dists, dists_dev, total * sizeof(float), cudaMemcpyDeviceToHost, current_stream()));
+        }
+    }
+    int flag = 0;
+    if (flagged) {
+        VB_CUDA(cudaMemcpyAsync(&flag, ix->tc.error_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, current_stream()));
+    }
+    VB_TRY(sync_stream());
+    if ((flag & 1) != 0) {
+        VB_FAIL(VB200_INTERNAL_ERROR, "tensor-core kernel gave up on a bounded wait");
+    }
+    if (pin_out) {
+        if (host_ids) {
+            std::memcpy(ids, ids_dev, total * sizeof(int64_t));
+        }
+        if (host_d) {
+            std::memcpy(dists, dists_dev, total * sizeof(float));
+        }
+    }
+    return 0;
 }
 
 extern "C" int

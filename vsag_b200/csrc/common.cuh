@@ -78,6 +78,10 @@ extern std::atomic<uint64_t> g_kernel_launches;
 
 int sm_count();
 
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device; asks the driver only when that is
+// more than it was allowed before.
+int allow_dynamic_smem(const void* kernel, size_t bytes);
+
 // ---------------------------------------------------------------------------------------------
 // device memory
 // ---------------------------------------------------------------------------------------------

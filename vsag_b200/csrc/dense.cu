@@ -2,6 +2,9 @@
 // state (error text, stream, launch counter).
 #include "dense.cuh"
 
+#include <map>
+#include <utility>
+
 namespace vb200 {
 
 // ---------------------------------------------------------------------------------------------
@@ -49,6 +52,24 @@ sm_count() {
         cached[dev].store(n, std::memory_order_relaxed);
     }
     return n;
+}
+
+int
+allow_dynamic_smem(const void* kernel, size_t bytes) {
+    if (bytes <= 40 * 1024) {   // static shared memory counts against the 48 KiB default too
+        return 0;
+    }
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int dev = 0;
+    VB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& have = allowed[{kernel, dev}];
+    if (bytes > have) {
+        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+        have = bytes;
+    }
+    return 0;
 }
 
 bool

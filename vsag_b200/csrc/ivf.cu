@@ -6,6 +6,7 @@
 
 #include "dense.cuh"
 #include "ivf_scan.cuh"
+#include "ivf_pairs.cuh"
 #include "comm.cuh"
 #include "ivf_scan_tc.cuh"
 #include "kmeans.cuh"
@@ -98,6 +99,11 @@ struct SearchWorkspace {
     bool opt_deadline = false;
     DevBuf<int64_t> out_ids;
     DevBuf<float> out_dists;
+    // searches of small batches (ivf_pairs.cuh): the pairs' places, their rows' scores, and pinned memory that
+    // small host inputs and results pass through
+    DevBuf<uint32_t> pair_base, query_rows;
+    DevBuf<float> pair_scores;
+    PinnedBuf pinned;
 };
 
 }  // namespace vb200
@@ -133,6 +139,7 @@ struct vb200_ivf {
     DevBuf<uint32_t> list_off;
     std::vector<uint32_t> list_off_host;
     uint32_t max_list_len = 0;   // the longest list this index (shard) holds
+    std::vector<uint64_t> longest_rows;   // [nlist + 1] rows of the i longest lists together
     bool balls_valid = false;    // the covering balls describe the lists as they are stored
     bool use_residual = false;       // SQ8: lists hold the codes of x - centroid (IVF use_residual)
     DevBuf<float> res_bias;          // [n_stored] L2 residual bias of every stored code (bucket_datacell.h:642-649)
@@ -2296,6 +2303,37 @@ route_sync_and_check(SearchWorkspace& ws) {
     return route_flag_check(word);
 }
 
+// out[(q, r)] = the distance chain between every query and every row (see route_dist_kernel).
+static int
+launch_row_chains(const float* queries, uint64_t nq, uint64_t q_stride, const float* rows, uint32_t n_rows, uint32_t dim, bool l2,
+                  bool one_minus, float* out, uint64_t ld) {
+    const uint32_t chunks = (n_rows + RS_ROWS - 1) / RS_ROWS;
+    // As many queries per CTA as still leave two CTAs for every SM: a row fetched once serves them all.
+    uint32_t qn = 8;
+    while (qn > 1 && static_cast<uint64_t>(chunks) * ((nq + qn - 1) / qn) < 2ull * static_cast<uint32_t>(sm_count())) {
+        qn /= 2;
+    }
+    auto smem_of = [&](uint32_t n) { return RS_STAGES * RS_STAGE + static_cast<size_t>(n) * ((dim + 3) / 4 * 4) * sizeof(float); };
+    while (qn > 1 && smem_of(qn) > 100 * 1024) {
+        qn /= 2;
+    }
+    const size_t smem = smem_of(qn);
+    VB_CHECK_ARG(smem <= 220 * 1024, "dim = %u is too large for the routing kernel", dim);
+    const uint64_t tiles = (nq + qn - 1) / qn;
+    VB_CHECK_ARG(tiles <= 65535, "too many query tiles");
+    const bool wide = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
+    using Kernel = void (*)(const float*, uint32_t, uint64_t, const float*, uint32_t, uint32_t, int, float*, uint64_t);
+#define VB_ROW_CHAINS(QN)                                                                          \
+    (l2 ? (wide ? route_dist_kernel<true, QN, 16> : route_dist_kernel<true, QN, 4>)                \
+        : (wide ? route_dist_kernel<false, QN, 16> : route_dist_kernel<false, QN, 4>))
+    const Kernel kernel = qn == 8 ? VB_ROW_CHAINS(8) : (qn == 4 ? VB_ROW_CHAINS(4) : (qn == 2 ? VB_ROW_CHAINS(2) : VB_ROW_CHAINS(1)));
+#undef VB_ROW_CHAINS
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    VB_LAUNCH(kernel, dim3(chunks, static_cast<uint32_t>(tiles)), RS_ROWS, smem, queries, static_cast<uint32_t>(nq), q_stride, rows,
+              n_rows, dim, one_minus ? 1 : 0, out, ld);
+    return 0;
+}
+
 static int
 ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe, int32_t* probes_dev,
                  float* dists_dev) {
@@ -2404,20 +2442,22 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         VB_TRY(tc_scores(ix->tc, a, b, 3, l2 ? -2.0f : -1.0f, l2 ? ix->c_sq.ptr : nullptr, ws.scores.ptr, ld));
         VB_TRY(select_rows(ws.scores.ptr, nq, nlist, ld, ncand, 0, ws.cand.ptr, ncand));
     } else {
-        uint64_t slab = (uint64_t{256} << 20) / nlist;  // rows of a 1 GiB score slab
-        if (slab < 1) {
-            slab = 1;
-        }
-        if (slab > nq) {
-            slab = nq;
-        }
+        uint64_t slab = (uint64_t{256} << 20) / nlist;  // rows of a 1 GiB distance slab
+        slab = slab < 1 ? 1 : (slab > 65535 ? 65535 : slab);   // (a launch takes 65535 query tiles)
+        slab = slab > nq ? nq : slab;
         VB_TRY(ws.scores.reserve(slab * nlist));
         for (uint64_t b = 0; b < nq; b += slab) {
-            uint64_t n = nq - b < slab ? nq - b : slab;
-            VB_TRY(dense_scores_f32(q_dev + b * ix->dim, n, ix->centroids.ptr, nlist, ix->dim,
-                                    l2 ? -2.0f : -1.0f, l2 ? ix->c_sq.ptr : nullptr, ws.scores.ptr, nlist));
-            VB_TRY(select_rows(ws.scores.ptr, n, nlist, nlist, ncand, 0, ws.cand.ptr + b * ncand, ncand));
+            const uint64_t n = nq - b < slab ? nq - b : slab;
+            VB_TRY(launch_row_chains(q_dev + b * ix->dim, n, ix->dim, ix->centroids.ptr, nlist, ix->dim, l2, true, ws.scores.ptr, nlist));
+            PairsPrepare pp{};
+            pp.dist = ws.scores.ptr;
+            pp.nlist = nlist;
+            pp.nprobe = nprobe;
+            pp.probes = probes_dev + b * nprobe;
+            pp.probe_dists = dists_dev != nullptr ? dists_dev + b * nprobe : nullptr;
+            VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(n), PAIR_THREADS, 0, pp);
         }
+        return 0;
     }
     uint32_t n2 = next_pow2(ncand < 2 ? 2 : ncand);
     VB_LAUNCH(route_finalize_kernel, static_cast<uint32_t>(nq), 128, n2 * sizeof(uint64_t) + ix->dim * sizeof(float), q_dev,
@@ -2519,6 +2559,42 @@ struct ScanProfile {
     }
 };
 static ScanProfile g_scan_profile;
+
+// The id filter of the running search in the scan's parameters: tombstones and / or the caller's filter.
+static int
+bind_id_filter(vb200_ivf* ix, ScanParams& p) {
+    SearchWorkspace& ws = ix->ws;
+    cudaStream_t st = current_stream();
+    const vb200_filter* f = ws.filter;
+    const bool user_deny = f != nullptr && f->deny_inner_bits != nullptr && f->n_inner_bits > 0;
+    const bool user_labels = f != nullptr && f->invalid_label_bits != nullptr && f->n_label_bits > 0;
+    if (ix->n_removed > 0 || user_deny || user_labels) {
+        p.filter_pos_inner = ix->pos_inner.ptr;
+        p.labels = ix->labels.ptr;
+        if (user_deny) {
+            const uint64_t words = (ix->n_total + 31) / 32;
+            const uint64_t extra_words = (f->n_inner_bits + 31) / 32;
+            DevInput<uint32_t> extra;
+            VB_TRY(extra.bind(f->deny_inner_bits, extra_words));
+            VB_TRY(ws.deny_bits.reserve(words));
+            VB_LAUNCH(deny_merge_kernel, static_cast<uint32_t>((words + 255) / 256), 256, 0, ix->tombstones.ptr,
+                      ix->tomb_words, extra.ptr, extra_words, words, ws.deny_bits.ptr);
+            VB_TRY(sync_stream());   // `extra` may be a staging copy that ends with this scope
+            p.deny_inner_bits = ws.deny_bits.ptr;
+        } else if (ix->n_removed > 0) {
+            p.deny_inner_bits = ix->tombstones.ptr;
+        }
+        if (user_labels) {
+            const uint64_t words = (f->n_label_bits + 63) / 64;
+            VB_TRY(ws.label_bits.reserve(words));
+            VB_CUDA(cudaMemcpyAsync(ws.label_bits.ptr, f->invalid_label_bits, words * sizeof(uint64_t),
+                                    cudaMemcpyDefault, st));
+            p.invalid_label_bits = ws.label_bits.ptr;
+            p.n_label_bits = f->n_label_bits;
+        }
+    }
+    return 0;
+}
 
 // Scans the probed lists of every query and leaves, per query, the kscan best as keys
 // (payload = inner id) in ws.keys.
@@ -2697,37 +2773,7 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
         p.ball_count = ix->ball_count.ptr;
     }
     p.scanned = reinterpret_cast<unsigned long long*>(ws.scalars.ptr + 3);
-    {
-        // id filter: tombstones and / or the caller's filter of this search
-        const vb200_filter* f = ws.filter;
-        const bool user_deny = f != nullptr && f->deny_inner_bits != nullptr && f->n_inner_bits > 0;
-        const bool user_labels = f != nullptr && f->invalid_label_bits != nullptr && f->n_label_bits > 0;
-        if (ix->n_removed > 0 || user_deny || user_labels) {
-            p.filter_pos_inner = ix->pos_inner.ptr;
-            p.labels = ix->labels.ptr;
-            if (user_deny) {
-                const uint64_t words = (ix->n_total + 31) / 32;
-                const uint64_t extra_words = (f->n_inner_bits + 31) / 32;
-                DevInput<uint32_t> extra;
-                VB_TRY(extra.bind(f->deny_inner_bits, extra_words));
-                VB_TRY(ws.deny_bits.reserve(words));
-                VB_LAUNCH(deny_merge_kernel, static_cast<uint32_t>((words + 255) / 256), 256, 0, ix->tombstones.ptr,
-                          ix->tomb_words, extra.ptr, extra_words, words, ws.deny_bits.ptr);
-                VB_TRY(sync_stream());   // `extra` may be a staging copy that ends with this scope
-                p.deny_inner_bits = ws.deny_bits.ptr;
-            } else if (ix->n_removed > 0) {
-                p.deny_inner_bits = ix->tombstones.ptr;
-            }
-            if (user_labels) {
-                const uint64_t words = (f->n_label_bits + 63) / 64;
-                VB_TRY(ws.label_bits.reserve(words));
-                VB_CUDA(cudaMemcpyAsync(ws.label_bits.ptr, f->invalid_label_bits, words * sizeof(uint64_t),
-                                        cudaMemcpyDefault, st));
-                p.invalid_label_bits = ws.label_bits.ptr;
-                p.n_label_bits = f->n_label_bits;
-            }
-        }
-    }
+    VB_TRY(bind_id_filter(ix, p));
     if (sq8) {
         const uint32_t dpad32 = ix->kchunks * 16;
         if (tc_scan) {
@@ -2942,6 +2988,17 @@ check_search_ready(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k,
     return 0;
 }
 
+// Candidates of a search whose results are reranked: factor * k, one at least.
+static int
+rerank_depth(uint32_t k, float factor, uint32_t* kscan) {
+    VB_CHECK_ARG(factor > 0.0f, "factor must be positive when use_reorder is true, got %f", factor);
+    *kscan = static_cast<uint32_t>(static_cast<int64_t>(factor * static_cast<float>(k)));
+    if (*kscan < 1) {
+        *kscan = 1;
+    }
+    return 0;
+}
+
 // Full pipeline up to per-query keys with inner-id payloads (k of them, ascending) in *keys_out.
 static int
 ivf_search_keys(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, uint32_t nprobe,
@@ -2953,11 +3010,7 @@ ivf_search_keys(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, ui
     uint32_t kscan = k;
     const bool rerank = ix->use_reorder && !ws.opt_no_reorder;
     if (rerank) {
-        VB_CHECK_ARG(factor > 0.0f, "factor must be positive when use_reorder is true, got %f", factor);
-        kscan = static_cast<uint32_t>(static_cast<int64_t>(factor * static_cast<float>(k)));
-        if (kscan < 1) {
-            kscan = 1;
-        }
+        VB_TRY(rerank_depth(k, factor, &kscan));
     }
     // buckets_per_data > 1: the scan looks for that many times as many postings, duplicates of a vector are
     // folded afterwards (IVF::search scales topk before and de-duplicates after, ivf.cpp:1722-1727, :1799-1825)
@@ -3030,6 +3083,242 @@ ivf_search_keys(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, ui
     return 0;
 }
 
+// Bytes of host inputs and results that pass through pinned memory of the handle: below this the copies of
+// pageable memory cost more in driver time than the transfer itself.
+constexpr size_t PINNED_IO_BYTES = 256 * 1024;
+
+// True when the batch goes pair by pair (ivf_pairs.cuh).  The line: with six or more queries per probed list a
+// tile of queries per list saves the lists' traffic (6 x 500 rows of 128 bytes fill an L1-sized tile); below it
+// every pair on its own is faster for every codec.  Large SQ8 batches with shallow k prune most of their pairs
+// away on the grouped path, which pays from about a gigabyte of probed codes on.
+static bool
+ivf_pairs_fit(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe) {
+    const SearchWorkspace& ws = ix->ws;
+    if (ix->quant == VB200_QUANT_SQ8_UNIFORM || ix->use_residual || ix->buckets_per_data > 1 || ws.opt_deadline ||
+        ws.exchange != nullptr || ix->n_stored == 0) {
+        return false;
+    }
+    if (kscan + SQ8_SLACK > 1024 - SCAN_THREADS) {
+        return false;   // (the scan depth limit of the grouped path, which reports it)
+    }
+    if (static_cast<double>(nq) * nprobe >= 6.0 * ix->nlist) {
+        return false;
+    }
+    const double rows = static_cast<double>(nq) * nprobe * (static_cast<double>(ix->n_stored) / ix->nlist);
+    if (ix->quant == VB200_QUANT_SQ8 && rows * ix->code_size > 1e9) {
+        return false;
+    }
+    return nprobe <= ix->nlist;
+}
+
+// The search of a small batch from queries to results.  ids / dists: host or device.
+static int
+ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, uint32_t kscan, uint32_t nprobe, bool rerank,
+                 const int32_t* bucket_ids, int64_t* ids, float* dists) {
+    SearchWorkspace& ws = ix->ws;
+    cudaStream_t st = current_stream();
+    const uint32_t dim = ix->dim, nlist = ix->nlist;
+    const bool sq8 = ix->quant == VB200_QUANT_SQ8, l2 = ix->metric == VB200_METRIC_L2;
+    // host buffers: [queries | ids | dists] in pinned memory when small
+    const size_t q_bytes = nq * dim * sizeof(float), total = nq * k;
+    const bool host_q = !is_device_pointer(queries), host_ids = !is_device_pointer(ids), host_d = !is_device_pointer(dists);
+    const bool pin_q = host_q && q_bytes <= PINNED_IO_BYTES;
+    const bool pin_out = (host_ids || host_d) && total * 12 <= PINNED_IO_BYTES;
+    const size_t ids_at = pin_q ? (q_bytes + 15) / 16 * 16 : 0, dists_at = ids_at + (pin_out ? total * sizeof(int64_t) : 0);
+    const size_t rows_at = dists_at + (pin_out ? (total * sizeof(float) + 15) / 16 * 16 : 0);
+    VB_TRY(ws.pinned.reserve(rows_at + nq * sizeof(uint32_t)));
+    unsigned char* pin = static_cast<unsigned char*>(ws.pinned.ptr);
+    const float* q_dev = queries;
+    if (host_q) {
+        VB_TRY(ws.queries.reserve(nq * dim));
+        const void* from = queries;
+        if (pin_q) {
+            std::memcpy(pin, queries, q_bytes);
+            from = pin;
+        }
+        VB_CUDA(cudaMemcpyAsync(ws.queries.ptr, from, q_bytes, cudaMemcpyHostToDevice, st));
+        q_dev = ws.queries.ptr;
+    }
+    if (ix->cosine) {
+        VB_TRY(ws.q_unit.reserve(nq * dim));
+        VB_TRY(normalize_rows_f32(q_dev, nq, dim, ws.q_unit.ptr));
+        q_dev = ws.q_unit.ptr;
+    }
+    VB_TRY(reserve_scalars(ws));
+    VB_TRY(ws.probes.reserve(nq * nprobe));
+    VB_TRY(ws.pair_base.reserve(nq * nprobe));
+    VB_TRY(ws.query_rows.reserve(nq));
+    // a query's stretch of the score buffer holds its probed lists whichever they are; batches whose stretches
+    // together pass a gigabyte go in slices
+    const uint64_t stride = (ix->longest_rows[nprobe] + 31) / 32 * 32;
+    VB_CHECK_ARG(stride < 0xFFFFFFFFull, "the probed lists hold too many rows");
+    uint64_t slice = (uint64_t{256} << 20) / (stride > 0 ? stride : 1);
+    slice = slice < 1 ? 1 : (slice > nq ? nq : slice);
+    VB_TRY(ws.pair_scores.reserve(slice * stride));
+    if (sq8) {
+        VB_TRY(ws.qw8.reserve(nq * 3 * ix->dpad));
+        VB_TRY(ws.qscale.reserve(nq));
+        VB_TRY(ws.qa.reserve(nq));
+    }
+    PairsPrepare pp{};
+    pp.nlist = nlist;
+    pp.nprobe = nprobe;
+    pp.list_off = ix->list_off.ptr;
+    pp.probes = ws.probes.ptr;
+    pp.t = PairTable{ws.pair_base.ptr, ws.query_rows.ptr, stride, ws.pair_scores.ptr};
+    if (sq8) {
+        pp.queries = q_dev;
+        pp.dim = dim;
+        pp.dpad = ix->dpad;
+        pp.scale = ix->sq_scale.ptr;
+        pp.mid = ix->sq_mid.ptr;
+        pp.metric = ix->metric;
+        pp.qw8 = ws.qw8.ptr;
+        pp.qscale = ws.qscale.ptr;
+        pp.qa = ws.qa.ptr;
+    }
+    bool routed_on_tensor_cores = false;
+    if (bucket_ids != nullptr) {
+        VB_CUDA(cudaMemcpyAsync(ws.probes.ptr, bucket_ids, nq * nprobe * sizeof(int32_t), cudaMemcpyDefault, st));
+    } else if (tensor_cores_enabled() && nq >= 256 && nlist >= 1024) {
+        VB_TRY(ivf_route_device(ix, q_dev, nq, nprobe, ws.probes.ptr, nullptr));
+        routed_on_tensor_cores = true;
+    } else {
+        VB_CHECK_ARG((nprobe + ROUTE_SLACK < nlist ? nprobe + ROUTE_SLACK : nlist) <= 1024,
+                     "scan_buckets_count %u is too large (limit %u)", nprobe, 1024 - ROUTE_SLACK);
+        VB_TRY(ws.scores.reserve(nq * nlist));
+        VB_TRY(launch_row_chains(q_dev, nq, dim, ix->centroids.ptr, nlist, dim, l2, true, ws.scores.ptr, nlist));
+        pp.dist = ws.scores.ptr;
+    }
+    VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, 0, pp);
+    const float* q_scan = q_dev;
+    if (ix->quant == VB200_QUANT_RABITQ) {
+        VB_TRY(ws.qproc.reserve(nq * (dim + 1)));
+        VB_TRY(rabitq_process_query_device(q_dev, nq, dim, ix->rotation.ptr, ix->rq_centroid.ptr, ws.qproc.ptr, &ws.qrot));
+        q_scan = ws.qproc.ptr;
+    }
+
+    ScanFinalize f{};
+    ScanParams& p = f.scan.s;
+    p.codes = ix->codes.ptr;
+    p.code_stride = ix->code_stride;
+    p.dim = dim;
+    p.dpad = ix->dpad;
+    p.list_off = ix->list_off.ptr;
+    p.nlist = nlist;
+    p.queries = q_scan;
+    p.qa = ws.qa.ptr;
+    p.code_norm = ix->code_norm.ptr;
+    p.coef_b = l2 ? 1.0f : 0.0f;
+    p.coef_c = l2 ? -2.0f : -1.0f;
+    p.inv_sqrt_d = 1.0f / sqrtf(static_cast<float>(dim));
+    p.metric = ix->metric;
+    VB_TRY(bind_id_filter(ix, p));
+    f.scan.t = pp.t;
+    f.scan.probes = ws.probes.ptr;
+    f.scan.nprobe = nprobe;
+    f.scan.qw8 = ws.qw8.ptr;
+    f.scan.qscale = ws.qscale.ptr;
+    f.scan.row_bytes = ix->quant == VB200_QUANT_RABITQ ? rabitq_bits_bytes(dim) : ix->code_size;
+    f.scan.qstride = sq8 ? ix->dpad : (dim + 127) / 128 * 128;
+    // one CTA for every 128 rows of a list of ordinary length, longer lists in turns
+    const uint64_t mean_len = ix->n_stored / nlist;
+    f.scan.per_pair = static_cast<uint32_t>(std::min<uint64_t>((ix->max_list_len + RS_ROWS - 1) / RS_ROWS, mean_len / RS_ROWS + 2));
+    f.kscan = kscan;
+    f.kcand = sq8 ? kscan + SQ8_SLACK : kscan;
+    f.k = k;
+    f.lower = ix->lower.ptr;
+    f.diff = ix->diff.ptr;
+    f.pos_inner = ix->pos_inner.ptr;
+    f.labels = ix->labels.ptr;
+    f.flat = rerank ? ix->flat.ptr : nullptr;
+    f.rows_scanned = reinterpret_cast<uint32_t*>(pin + rows_at);
+    if (!pin_out) {
+        VB_TRY(ws.out_ids.reserve(total));
+        VB_TRY(ws.out_dists.reserve(total));
+    }
+    int64_t* ids_dev = !host_ids ? ids : (pin_out ? reinterpret_cast<int64_t*>(pin + ids_at) : ws.out_ids.ptr);
+    float* dists_dev = !host_d ? dists : (pin_out ? reinterpret_cast<float*>(pin + dists_at) : ws.out_dists.ptr);
+
+    const size_t scan_smem = RS_STAGES * RS_STAGE + (sq8 ? 3 * static_cast<size_t>(ix->dpad) : f.scan.qstride * sizeof(float));
+    const size_t final_smem = (2 * static_cast<size_t>(nprobe) + (sq8 ? 3 : (rerank ? 1 : 0)) * static_cast<size_t>(dim)) * sizeof(float);
+    VB_CHECK_ARG(scan_smem <= 220 * 1024 && final_smem <= 180 * 1024, "dim = %u is too large for the scan", dim);
+    void (*scan_kernel)(const PairScan) = nullptr;
+    void (*final_kernel)(const ScanFinalize) = nullptr;
+#define VB_PAIRS(FMT)                                                                                \
+    {                                                                                                \
+        scan_kernel = l2 ? pair_scan_kernel<FMT, true> : pair_scan_kernel<FMT, false>;               \
+        final_kernel = l2 ? scan_finalize_kernel<FMT, true> : scan_finalize_kernel<FMT, false>;      \
+    }
+    switch (ix->quant) {
+        case VB200_QUANT_SQ8: VB_PAIRS(ROW_SQ8) break;
+        case VB200_QUANT_FP32: VB_PAIRS(ROW_F32) break;
+        case VB200_QUANT_BF16: VB_PAIRS(ROW_BF16) break;
+        case VB200_QUANT_FP16: VB_PAIRS(ROW_FP16) break;
+        default:
+            scan_kernel = pair_scan_kernel<ROW_RABITQ, true>;
+            final_kernel = scan_finalize_kernel<ROW_RABITQ, true>;
+            break;
+    }
+#undef VB_PAIRS
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(scan_kernel), scan_smem));
+    // (beside about 34 KiB of static shared memory)
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(final_kernel), final_smem + (final_smem > 12 * 1024 ? 40 * 1024 : 0)));
+    for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
+        const uint64_t n = std::min(slice, nq - q0);
+        ScanFinalize g = f;
+        g.scan.probes += q0 * nprobe;
+        g.scan.t.base += q0 * nprobe;
+        g.scan.t.rows += q0;
+        g.scan.s.queries += q0 * (ix->quant == VB200_QUANT_RABITQ ? dim + 1 : dim);
+        g.queries = q_dev + q0 * dim;
+        if (sq8) {
+            g.scan.s.qa += q0;
+            g.scan.qscale += q0;
+            g.scan.qw8 += q0 * 3 * ix->dpad;
+        }
+        g.rows_scanned += q0;
+        g.ids = ids_dev + q0 * k;
+        g.dists = dists_dev + q0 * k;
+        const uint64_t blocks = n * nprobe * g.scan.per_pair;
+        VB_CHECK_ARG(blocks <= 0x7fffffffull, "query batch too large");
+        if (q0 == 0) {
+            VB_CUDA(cudaEventRecord(ix->ev_scan_begin, st));
+        }
+        VB_LAUNCH(scan_kernel, static_cast<uint32_t>(blocks), RS_ROWS, scan_smem, g.scan);
+        if (q0 + n == nq) {
+            VB_CUDA(cudaEventRecord(ix->ev_scan_end, st));
+            ix->scan_timed = true;
+        }
+        VB_LAUNCH(final_kernel, static_cast<uint32_t>(n), PAIR_THREADS, final_smem, g);
+    }
+    ws.pruning = false;
+    if (!pin_out) {
+        if (host_ids) {
+            VB_CUDA(cudaMemcpyAsync(ids, ids_dev, total * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        }
+        if (host_d) {
+            VB_CUDA(cudaMemcpyAsync(dists, dists_dev, total * sizeof(float), cudaMemcpyDeviceToHost, st));
+        }
+    }
+    VB_TRY(routed_on_tensor_cores ? route_sync_and_check(ws) : sync_stream());
+    if (pin_out) {
+        if (host_ids) {
+            std::memcpy(ids, pin + ids_at, total * sizeof(int64_t));
+        }
+        if (host_d) {
+            std::memcpy(dists, pin + dists_at, total * sizeof(float));
+        }
+    }
+    const uint32_t* rows_scanned = reinterpret_cast<const uint32_t*>(pin + rows_at);
+    uint64_t rows = 0;
+    for (uint64_t i = 0; i < nq; ++i) {
+        rows += rows_scanned[i];
+    }
+    ix->last_scan_bytes = ix->last_scanned_bytes = static_cast<int64_t>(rows * ix->code_size);
+    return 0;
+}
+
 }  // namespace vb200
 
 // =============================================================================================
@@ -3049,6 +3338,10 @@ ivf_refresh_scan_order(vb200_ivf* ix) {
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
         return off[a + 1] - off[a] > off[b + 1] - off[b];
     });
+    ix->longest_rows.assign(nlist + 1, 0);
+    for (uint32_t i = 0; i < nlist; ++i) {
+        ix->longest_rows[i + 1] = ix->longest_rows[i] + (off[order[i] + 1] - off[order[i]]);
+    }
     VB_TRY(ix->scan_order.reserve(nlist));
     VB_CUDA(cudaMemcpyAsync(ix->scan_order.ptr, order.data(), nlist * sizeof(uint32_t), cudaMemcpyHostToDevice,
                             current_stream()));
@@ -3918,8 +4211,6 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
         }
     }
     const uint64_t total = nq * k;
-    VB_TRY(ws.out_ids.reserve(total));
-    VB_TRY(ws.out_dists.reserve(total));
     if (ix->n_total == 0) {
         // Empty index: every slot padded, like the Dim=0 dataset of IndexImpl (index_impl.h:60-63).
         std::vector<int64_t> hi(total, -1);
@@ -3929,6 +4220,24 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
         ix->last_scan_bytes = 0;
         return 0;
     }
+    {
+        const uint32_t np = nprobe > ix->nlist ? ix->nlist : nprobe;
+        const bool rerank = ix->use_reorder && !ws.opt_no_reorder;
+        if (np == nprobe || bucket_ids == nullptr) {
+            uint32_t kscan = k;
+            if (rerank) {
+                VB_TRY(rerank_depth(k, factor, &kscan));
+            }
+            if (ivf_pairs_fit(ix, nq, kscan, np)) {
+                ws.filter = filter;
+                const int rc = ivf_search_pairs(ix, queries, nq, k, kscan, np, rerank, bucket_ids, ids, dists);
+                ws.filter = nullptr;
+                return rc;
+            }
+        }
+    }
+    VB_TRY(ws.out_ids.reserve(total));
+    VB_TRY(ws.out_dists.reserve(total));
     const uint64_t* keys = nullptr;
     ws.filter = filter;
     const int search_status = ivf_search_keys(ix, queries, nq, k, nprobe, factor, bucket_ids, &keys);

@@ -1,0 +1,454 @@
+// Searches of small batches: every (query, probed list) pair is scanned on its own.
+//
+// When a list is probed by only a few queries of the batch there is nothing to gain from collecting the queries
+// of a list into a tile, and the passes that do it (count, prefix sums, work items, places), the bounds and the
+// second phase cost more than the rows.  Such a batch takes three or four launches here instead of fifteen:
+//   route_dist_kernel     every centroid distance, as the reference's chain (no candidates, no re-scoring)
+//   pairs_prepare_kernel  a CTA per query: its nprobe nearest lists, where each list's scores go, SQ8 weights
+//   pair_scan_kernel      a CTA per (pair, 128 rows): one score per row, written where the CTA above said
+//   scan_finalize_kernel  a CTA per query: the k best of its scores, exact re-scoring, rerank, labels
+#pragma once
+
+#include "block_select.cuh"
+#include "row_scan.cuh"
+
+namespace vb200 {
+
+constexpr int PAIR_THREADS = 256;   // of the per-query kernels
+
+struct PairTable {
+    uint32_t* base;    // [nq x nprobe] a pair's first score within its query's stretch
+    uint32_t* rows;    // [nq] scores of each query
+    uint64_t stride;   // scores between the stretches of neighbouring queries
+    float* scores;
+};
+
+// out[(q, r)] for every row r of `rows` and query q: L2 = sum of fma(t, t, .), t = row - query; otherwise the
+// inner product chain, as it is (ONE_MINUS 0) or taken from one (1).  grid.x = row chunks, grid.y = query tiles.
+template <bool L2, int QN, int UNIT>
+__global__ void __launch_bounds__(RS_ROWS)
+route_dist_kernel(const float* __restrict__ queries, uint32_t nq, uint64_t q_stride, const float* __restrict__ rows, uint32_t n_rows,
+                  uint32_t dim, int one_minus, float* __restrict__ out, uint64_t ld) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* qs = reinterpret_cast<float*>(smem + RS_STAGES * RS_STAGE);
+    const uint32_t qpad = (dim + 3) / 4 * 4;
+    const uint32_t q0 = blockIdx.y * QN;
+    for (uint32_t i = threadIdx.x; i < QN * qpad; i += RS_ROWS) {
+        const uint32_t qi = i / qpad, d = i - qi * qpad;
+        qs[i] = (q0 + qi < nq && d < dim) ? __ldg(queries + (q0 + qi) * q_stride + d) : 0.f;
+    }
+    RowAcc<ROW_F32, L2, QN> acc;
+    row_stream<UNIT>(reinterpret_cast<const unsigned char*>(rows), static_cast<uint64_t>(dim) * 4, dim * 4, dim, n_rows, blockIdx.x,
+                     gridDim.x, smem, qs, qpad, acc, [&](uint64_t row, bool valid) {
+                         if (valid) {
+#pragma unroll
+                             for (int i = 0; i < QN; ++i) {
+                                 if (q0 + i < nq) {
+                                     const float v = acc.acc[i];
+                                     out[(q0 + i) * ld + row] = (!L2 && one_minus != 0) ? __fsub_rn(1.0f, v) : v;
+                                 }
+                             }
+                         }
+                     });
+}
+
+struct PairsPrepare {
+    const float* dist;        // [nq x nlist] exact centroid distances, or null: `probes` is given
+    uint32_t nlist, nprobe;
+    int32_t* probes;          // [nq x nprobe] nearest first
+    float* probe_dists;       // [nq x nprobe] or null
+    const uint32_t* list_off;
+    PairTable t;
+    // SQ8 (null qw8: none): the int8 weight terms, their scale and the query's constant (see sq8_query_prep_kernel)
+    const float* queries;
+    uint32_t dim, dpad;
+    const float *scale, *mid;
+    int metric;
+    int8_t* qw8;              // [nq][3][dpad]
+    float *qscale, *qa;
+};
+
+__device__ __forceinline__ float
+pair_block_sum(float v, float* part) {
+    for (int o = 16; o > 0; o >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    v = 0.f;
+    for (int w = 0; w < PAIR_THREADS / 32; ++w) {
+        v += part[w];
+    }
+    return v;
+}
+
+__device__ __forceinline__ float
+pair_block_max(float v, float* part) {
+    for (int o = 16; o > 0; o >>= 1) {
+        v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    v = part[0];
+    for (int w = 1; w < PAIR_THREADS / 32; ++w) {
+        v = fmaxf(v, part[w]);
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(PAIR_THREADS)
+pairs_prepare_kernel(const PairsPrepare p) {
+    __shared__ SelectScratch sel;
+    __shared__ __align__(16) uint64_t keys[SELECT_CAP];
+    __shared__ __align__(16) uint64_t best[1024];
+    __shared__ float part[PAIR_THREADS / 32];
+    const uint64_t q = blockIdx.x;
+    int32_t* probes = p.probes + q * p.nprobe;
+    if (p.dist != nullptr) {
+        const float* row = p.dist + q * p.nlist;
+        const uint32_t found = block_select<PAIR_THREADS>(load_source([&](uint32_t i) { return float_to_ordered(__ldg(row + i)); }),
+                                                          [](uint32_t i) { return i; }, p.nlist, p.nprobe, keys, sel);
+        block_sort_to<PAIR_THREADS>(keys, found, p.nprobe, best);
+        for (uint32_t i = threadIdx.x; i < p.nprobe; i += PAIR_THREADS) {
+            const bool have = i < found;
+            probes[i] = have ? static_cast<int32_t>(static_cast<uint32_t>(best[i])) : -1;
+            if (p.probe_dists != nullptr) {
+                p.probe_dists[q * p.nprobe + i] = have ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
+            }
+        }
+        __syncthreads();
+    }
+    if (p.t.rows == nullptr) {
+        return;   // only the routing is wanted
+    }
+    uint32_t run = 0;
+    for (uint32_t i0 = 0; i0 < p.nprobe; i0 += PAIR_THREADS) {
+        const uint32_t i = i0 + threadIdx.x;
+        uint32_t len = 0;
+        if (i < p.nprobe) {
+            const int32_t l = probes[i];
+            if (l >= 0 && static_cast<uint32_t>(l) < p.nlist) {
+                len = p.list_off[l + 1] - p.list_off[l];
+            }
+        }
+        const uint32_t incl = block_inclusive_sum<PAIR_THREADS>(len, sel.warp_part);
+        if (i < p.nprobe) {
+            p.t.base[q * p.nprobe + i] = run + incl - len;
+        }
+        if (threadIdx.x == PAIR_THREADS - 1) {
+            sel.total = run + incl;
+        }
+        __syncthreads();
+        run = sel.total;
+    }
+    if (threadIdx.x == 0) {
+        p.t.rows[q] = run;
+    }
+    if (p.qw8 == nullptr) {
+        return;
+    }
+    const float* src = p.queries + q * p.dim;
+    float qq = 0.f, qm = 0.f, wmax = 0.f;
+    for (uint32_t d = threadIdx.x; d < p.dim; d += PAIR_THREADS) {
+        const float v = __ldg(src + d);
+        qq = fmaf(v, v, qq);
+        qm = fmaf(v, __ldg(p.mid + d), qm);
+        wmax = fmaxf(wmax, fabsf(v * __ldg(p.scale + d)));
+    }
+    qq = pair_block_sum(qq, part);
+    qm = pair_block_sum(qm, part);
+    wmax = pair_block_max(wmax, part);
+    const float s = wmax > 0.f && wmax < INFINITY ? wmax / 127.0f : 1.0f;
+    int8_t* t = p.qw8 + q * 3 * p.dpad;
+    for (uint32_t d = threadIdx.x; d < p.dpad; d += PAIR_THREADS) {
+        const float u = d < p.dim ? __ldg(src + d) * __ldg(p.scale + d) / s : 0.f;
+        const float t1 = fminf(fmaxf(rintf(u), -127.f), 127.f);
+        const float v2 = (u - t1) * 254.0f;
+        const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
+        const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
+        t[d] = static_cast<int8_t>(static_cast<int>(t1));
+        t[p.dpad + d] = static_cast<int8_t>(static_cast<int>(t2));
+        t[2 * p.dpad + d] = static_cast<int8_t>(static_cast<int>(t3));
+    }
+    if (threadIdx.x == 0) {
+        p.qscale[q] = s;
+        p.qa[q] = p.metric == VB200_METRIC_L2 ? fmaf(-2.0f, qm, qq) : 1.0f - qm;
+    }
+}
+
+struct PairScan {
+    ScanParams s;             // rows, list_off, filter, SQ8 / RaBitQ constants (queries = processed ones for RaBitQ)
+    PairTable t;
+    const int32_t* probes;
+    uint32_t nprobe;
+    uint32_t per_pair;        // CTAs per pair: CTA c takes chunks c, c + per_pair, ... of the list
+    uint32_t row_bytes;       // of a row that the scan reads
+    const int8_t* qw8;        // SQ8: [nq][3][dpad]
+    const float* qscale;
+    uint32_t qstride;         // query values in shared memory: floats (SQ8: bytes of a term)
+};
+
+// The bit pattern of the score of a row that the id filter rejects: a NaN, which no selection takes.
+constexpr uint32_t SCORE_FILTERED = 0x7FFFFFFFu;
+
+// est, record norm and error -> the reference's distance (ivf_rabitq_scan_kernel).
+__device__ __forceinline__ float
+rabitq_distance(float ip, float bn, float err, float qn) {
+    if (static_cast<double>(fabsf(err)) < 1e-5) {   // float compared with a double literal, as in the reference
+        err = err >= 0.f ? 1.0f : -1.0f;
+    }
+    const float est = __fdiv_rn(ip, err);
+    const float p3 = __fmul_rn(__fmul_rn(__fmul_rn(-2.0f, bn), qn), est);
+    return __fadd_rn(__fadd_rn(__fmul_rn(bn, bn), __fmul_rn(qn, qn)), p3);
+}
+
+// The query of a pair as the codec's chain reads it, in shared memory (qstride values, zero padded).
+template <int FMT>
+__device__ __forceinline__ void
+stage_query(const PairScan& p, uint64_t q, float* qs, uint32_t threads) {
+    if (FMT == ROW_SQ8) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.qw8 + q * 3 * p.qstride);
+        for (uint32_t i = threadIdx.x; i < 3 * p.qstride / 16; i += threads) {
+            reinterpret_cast<uint4*>(qs)[i] = __ldg(src + i);
+        }
+        return;
+    }
+    const uint32_t dim = p.s.dim;
+    const float* src = p.s.queries + q * (FMT == ROW_RABITQ ? dim + 1 : dim);
+    for (uint32_t d = threadIdx.x; d < p.qstride; d += threads) {
+        float v = d < dim ? __ldg(src + d) : 0.f;
+        if (FMT == ROW_BF16) {
+            v = half_decode<SCAN_FMT_BF16>(half_encode<SCAN_FMT_BF16>(v));
+        } else if (FMT == ROW_FP16) {
+            v = half_decode<SCAN_FMT_FP16>(half_encode<SCAN_FMT_FP16>(v));
+        } else if (FMT == ROW_RABITQ) {
+            v = __fmul_rn(p.s.inv_sqrt_d, v);
+        }
+        qs[d] = v;
+    }
+}
+
+template <int FMT, bool L2>
+__global__ void __launch_bounds__(RS_ROWS)
+pair_scan_kernel(const PairScan p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* qs = reinterpret_cast<float*>(smem + RS_STAGES * RS_STAGE);
+    const uint32_t pair = blockIdx.x / p.per_pair, first = blockIdx.x - pair * p.per_pair;
+    const uint32_t q = pair / p.nprobe;
+    const int32_t l = __ldg(p.probes + pair);
+    if (l < 0 || static_cast<uint32_t>(l) >= p.s.nlist) {
+        return;
+    }
+    const uint32_t lbeg = __ldg(p.s.list_off + l), len = __ldg(p.s.list_off + l + 1) - lbeg;
+    if (first * RS_ROWS >= len) {
+        return;
+    }
+    stage_query<FMT>(p, q, qs, RS_ROWS);
+    uint32_t* out = reinterpret_cast<uint32_t*>(p.t.scores + q * p.t.stride + p.t.base[pair]);
+    float qa = 0.f, cq = 0.f, qn = 0.f;
+    if (FMT == ROW_SQ8) {
+        qa = __ldg(p.s.qa + q);
+        cq = p.s.coef_c * __ldg(p.qscale + q);
+    } else if (FMT == ROW_RABITQ) {
+        qn = __ldg(p.s.queries + static_cast<uint64_t>(q) * (p.s.dim + 1) + p.s.dim);
+    }
+    const uint8_t* rows = p.s.codes + static_cast<uint64_t>(lbeg) * p.s.code_stride;
+    RowAcc<FMT, L2, 1> acc;
+    row_stream<16>(rows, p.s.code_stride, p.row_bytes, p.s.dim, len, first, p.per_pair, smem, qs, p.qstride, acc,
+                   [&](uint64_t row, bool valid) {
+                       if (!valid) {
+                           return;
+                       }
+                       const uint32_t pos = lbeg + static_cast<uint32_t>(row);
+                       float v;
+                       if constexpr (FMT == ROW_SQ8) {
+                           const float low = static_cast<float>(acc.a2 * 254 + acc.a3);
+                           const float f = fmaf(low, 1.0f / 64516.0f, static_cast<float>(acc.a1));
+                           v = fmaf(cq, f, p.s.coef_b * __ldg(p.s.code_norm + pos)) + qa;
+                       } else if constexpr (FMT == ROW_RABITQ) {
+                           const float* tail = reinterpret_cast<const float*>(rows + row * p.s.code_stride + p.row_bytes);
+                           v = rabitq_distance(acc.acc[0], __ldg(tail), __ldg(tail + 1), qn);
+                       } else {
+                           v = L2 ? acc.acc[0] : __fsub_rn(1.0f, acc.acc[0]);
+                       }
+                       uint32_t bits = __float_as_uint(v);
+                       if (p.s.filter_pos_inner != nullptr && scan_row_filtered(p.s, pos)) {
+                           bits = SCORE_FILTERED;
+                       }
+                       out[row] = bits;
+                   });
+}
+
+struct ScanFinalize {
+    PairScan scan;             // the scan whose scores are read
+    uint32_t kscan, k;         // results of the scan per query; results of the search (fewer with a rerank)
+    uint32_t kcand;            // candidates taken from the scores: kscan, and more when they are re-scored
+    const float *lower, *diff; // SQ8
+    const float* queries;      // [nq x dim] plain queries (SQ8 re-scoring, rerank)
+    const uint32_t* pos_inner;
+    const int64_t* labels;
+    const float* flat;         // rerank: fp32 rows by inner id, or null
+    uint32_t* rows_scanned;    // [nq] rows of each query's lists (pinned host memory)
+    int64_t* ids;
+    float* dists;
+};
+
+// Exact SQ8 distance in the reference's operation order (sq8_rescore_kernel); q, lower and diff in shared memory.
+__device__ __forceinline__ float
+sq8_exact_distance(const uint8_t* code, uint32_t dim, bool l2, const float* q, const float* lo, const float* di) {
+    const float inv255 = 1.0f / 255.0f;
+    float s = 0.f;
+    for (uint32_t d0 = 0; d0 < dim; d0 += 64) {
+        uint4 raw[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            raw[u] = d0 + u * 16 < dim ? __ldg(reinterpret_cast<const uint4*>(code + d0 + u * 16)) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t words[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                const uint32_t d = d0 + u * 16 + j;
+                if (d < dim) {
+                    const float byte = static_cast<float>((words[j >> 2] >> ((j & 3u) * 8)) & 0xFFu);
+                    const float x = fmaf(__fmul_rn(byte, inv255), di[d], lo[d]);
+                    if (l2) {
+                        const float t = __fsub_rn(q[d], x);
+                        s = fmaf(t, t, s);
+                    } else {
+                        s = fmaf(q[d], x, s);
+                    }
+                }
+            }
+        }
+    }
+    return l2 ? s : __fsub_rn(1.0f, s);
+}
+
+// A score's place among its query's -> the row's position: the pair whose stretch holds it is the last one that
+// starts at or before the place (an empty list shares its start with the pair after it).
+struct ScorePosition {
+    const uint32_t* base;    // (shared memory) first place of every pair
+    const uint32_t* start;   // (shared memory) first position of its list
+    uint32_t nprobe;
+    __device__ __forceinline__ uint32_t
+    operator()(uint32_t i) const {
+        uint32_t lo = 0, hi = nprobe;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (base[mid] <= i) {
+                lo = mid;
+            } else {
+                hi = mid;
+            }
+        }
+        return start[lo] + (i - base[lo]);
+    }
+};
+
+// Dynamic shared memory: [2][nprobe] pair places and list starts, [rerank or SQ8: query, SQ8: lower, diff] floats.
+template <int FMT, bool L2>
+__global__ void __launch_bounds__(PAIR_THREADS)
+scan_finalize_kernel(const ScanFinalize p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SelectScratch sel;
+    __shared__ __align__(16) uint64_t keys[SELECT_CAP];
+    __shared__ __align__(16) uint64_t best[1024];
+    const PairScan& sc = p.scan;
+    uint32_t* base_s = reinterpret_cast<uint32_t*>(smem);
+    uint32_t* start_s = base_s + sc.nprobe;
+    float* qs = reinterpret_cast<float*>(start_s + sc.nprobe);
+    const uint64_t q = blockIdx.x;
+    const uint32_t nprobe = sc.nprobe, dim = sc.s.dim;
+    const uint32_t n = sc.t.rows[q];
+    const uint32_t* scores = reinterpret_cast<const uint32_t*>(sc.t.scores + q * sc.t.stride);
+    for (uint32_t i = threadIdx.x; i < nprobe; i += PAIR_THREADS) {
+        const int32_t l = __ldg(sc.probes + q * nprobe + i);
+        base_s[i] = __ldg(sc.t.base + q * nprobe + i);
+        start_s[i] = l >= 0 && static_cast<uint32_t>(l) < sc.s.nlist ? __ldg(sc.s.list_off + l) : 0u;
+    }
+    if (FMT == ROW_SQ8 || p.flat != nullptr) {
+        const float* src = p.queries + q * dim;
+        for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
+            qs[d] = __ldg(src + d);
+            if (FMT == ROW_SQ8) {
+                qs[dim + d] = __ldg(p.lower + d);
+                qs[2 * dim + d] = __ldg(p.diff + d);
+            }
+        }
+    }
+    __syncthreads();
+    const ScorePosition position{base_s, start_s, nprobe};
+    const ScoreSource<> value{scores};
+    const uint32_t found = block_select<PAIR_THREADS>(value, position, n, p.kcand, keys, sel);
+    if (threadIdx.x == 0) {
+        p.rows_scanned[q] = n;
+    }
+    uint32_t have = found;
+    if (FMT == ROW_SQ8) {
+        // the kcand best by the ranking form, then their exact distances
+        block_sort_to<PAIR_THREADS>(keys, found, p.kcand, best);
+        have = min(found, p.kcand);
+        for (uint32_t i = threadIdx.x; i < have; i += PAIR_THREADS) {
+            const uint32_t pos = static_cast<uint32_t>(best[i]);
+            keys[i] = make_key(sq8_exact_distance(sc.s.codes + static_cast<uint64_t>(pos) * sc.s.code_stride, dim, L2, qs, qs + dim,
+                                                  qs + 2 * dim),
+                               pos);
+        }
+    }
+    block_sort_to<PAIR_THREADS>(keys, have, p.kscan, best);
+    have = min(have, p.kscan);
+    const uint64_t* final_keys = best;
+    if (p.flat != nullptr) {
+        // FlattenReorder::Reorder (rerank_kernel): a warp per candidate, the fp32 row by inner id
+        const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        for (uint32_t c = warp; c < have; c += PAIR_THREADS / 32) {
+            const uint32_t inner = __ldg(p.pos_inner + static_cast<uint32_t>(best[c]));
+            const float* x = p.flat + static_cast<uint64_t>(inner) * dim;
+            float s = 0.f;
+            for (uint32_t d0 = lane; d0 < dim; d0 += 256) {
+                float v[8];
+#pragma unroll
+                for (uint32_t u = 0; u < 8; ++u) {
+                    v[u] = d0 + u * 32 < dim ? __ldg(x + d0 + u * 32) : 0.f;
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 8; ++u) {
+                    const uint32_t d = d0 + u * 32;
+                    if (d < dim) {
+                        if (L2) {
+                            const float t = qs[d] - v[u];
+                            s = fmaf(t, t, s);
+                        } else {
+                            s = fmaf(qs[d], v[u], s);
+                        }
+                    }
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+            }
+            if (lane == 0) {
+                keys[c] = make_key(L2 ? s : 1.0f - s, inner);
+            }
+        }
+        block_sort_to<PAIR_THREADS>(keys, have, p.k, best);
+    }
+    for (uint32_t i = threadIdx.x; i < p.k; i += PAIR_THREADS) {
+        const bool there = i < have;
+        const uint64_t key = there ? final_keys[i] : KEY_INF;
+        const uint32_t id = static_cast<uint32_t>(key);
+        const uint32_t inner = there ? (p.flat != nullptr ? id : __ldg(p.pos_inner + id)) : 0u;
+        p.ids[q * p.k + i] = there ? __ldg(p.labels + inner) : -1;
+        p.dists[q * p.k + i] = there ? ordered_to_float(static_cast<uint32_t>(key >> 32)) : INFINITY;
+    }
+}
+
+}  // namespace vb200

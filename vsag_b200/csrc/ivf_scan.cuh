@@ -921,7 +921,7 @@ ivf_sq8_first_kernel(const ScanParams p, const int8_t* __restrict__ qw8, const f
 // Exact SQ8 distances of the survivors, in the reference's operation order (one thread per
 // candidate walks the dimensions upward: SQ8ComputeL2Sqr / SQ8ComputeIP with Width 1), then a
 // sort by (distance, position).  cand/out payloads are code positions.
-__global__ void __launch_bounds__(128)
+static __global__ void __launch_bounds__(128)
 sq8_rescore_kernel(const float* __restrict__ queries, uint32_t dim, const uint8_t* __restrict__ codes,
                    uint32_t code_stride, const float* __restrict__ lower, const float* __restrict__ diff,
                    const uint64_t* __restrict__ cand, uint32_t ncand, uint32_t n2, uint32_t k, int metric,
