@@ -7,6 +7,7 @@
 #include "dense.cuh"
 #include "ivf_scan.cuh"
 #include "ivf_pairs.cuh"
+#include "ivf_tiles.cuh"
 #include "comm.cuh"
 #include "ivf_scan_tc.cuh"
 #include "kmeans.cuh"
@@ -104,6 +105,10 @@ struct SearchWorkspace {
     DevBuf<uint32_t> pair_base, query_rows;
     DevBuf<float> pair_scores;
     PinnedBuf pinned;
+    // the same as tensor-core tiles (ivf_tiles.cuh): pairs grouped by list
+    DevBuf<uint32_t> tile_count, tile_rank, tile_tables, tile_pairs;
+    DevBuf<TileItem> tile_items;
+    DevBuf<int32_t> qsum;
 };
 
 }  // namespace vb200
@@ -125,7 +130,7 @@ struct vb200_ivf {
     DevBuf<float> centroids, c_sq;
     DevBuf<float> lower, diff;           // SQ8, padded to dpad
     DevBuf<float> sq_scale, sq_mid;      // SQ8: diff/255 and lower + 128*diff/255, padded to dpad
-    DevBuf<float> code_norm;             // SQ8: |decoded code|^2 per position
+    DevBuf<float> code_norm;             // SQ8, fp32, bf16, fp16: |decoded row|^2 per position
     // SQ8 tensor-core scan: a second copy of the lists as signed bytes (code - 128) in 8-row groups of
     // 16-byte cores, the shared-memory layout of the MMA's A operand; group_off[l] = first group of list l
     DevBuf<int8_t> codes_t;
@@ -139,6 +144,7 @@ struct vb200_ivf {
     DevBuf<uint32_t> list_off;
     std::vector<uint32_t> list_off_host;
     uint32_t max_list_len = 0;   // the longest list this index (shard) holds
+    DevBuf<float> row_max;       // [0] largest norm of a stored row, [1] RaBitQ: largest norm / |error term|
     std::vector<uint64_t> longest_rows;   // [nlist + 1] rows of the i longest lists together
     bool balls_valid = false;    // the covering balls describe the lists as they are stored
     bool use_residual = false;       // SQ8: lists hold the codes of x - centroid (IVF use_residual)
@@ -3086,35 +3092,138 @@ ivf_search_keys(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, ui
 // Bytes of host inputs and results that pass through pinned memory of the handle: below this the copies of
 // pageable memory cost more in driver time than the transfer itself.
 constexpr size_t PINNED_IO_BYTES = 256 * 1024;
+constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which tiles pay (3.1: 141 us as pairs, 162 as tiles)
 
-// True when the batch goes pair by pair (ivf_pairs.cuh).  The line: with six or more queries per probed list a
-// tile of queries per list saves the lists' traffic (6 x 500 rows of 128 bytes fill an L1-sized tile); below it
-// every pair on its own is faster for every codec.  Large SQ8 batches with shallow k prune most of their pairs
-// away on the grouped path, which pays from about a gigabyte of probed codes on.
+// How a batch is scanned into scores (ivf_pairs.cuh, ivf_tiles.cuh): not at all, pair by pair, or as tiles.
+enum ScoreScan { SCAN_GROUPED = 0, SCAN_PAIRS = 1, SCAN_TILES = 2 };
+
+struct TilePlan {
+    uint32_t qt, pieces, stages, b_bufs, per_sm;
+    size_t smem;
+};
+
+// Shared memory of a tile launch: the B operand of an item (two when they fit) and 2 .. 6 pieces of rows, two CTAs
+// per SM when that leaves room for them.  False when not even one CTA fits.
 static bool
-ivf_pairs_fit(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe) {
-    const SearchWorkspace& ws = ix->ws;
-    if (ix->quant == VB200_QUANT_SQ8_UNIFORM || ix->use_residual || ix->buckets_per_data > 1 || ws.opt_deadline ||
-        ws.exchange != nullptr || ix->n_stored == 0) {
-        return false;
+tile_plan(const vb200_ivf* ix, double pairs_per_list, TilePlan* plan) {
+    const bool int8 = ix->quant == VB200_QUANT_SQ8 || ix->quant == VB200_QUANT_RABITQ, f32 = ix->quant == VB200_QUANT_FP32;
+    plan->pieces = (ix->dim + (int8 ? 127 : 63)) / (int8 ? 128 : 64);
+    const size_t stage = (f32 ? 2 : 1) * TILE_A_TERM;
+    const uint32_t b_terms = int8 ? 3 : (f32 ? 2 : 1);
+    for (uint32_t per_sm = 2; per_sm >= 1; --per_sm) {
+        const size_t room = per_sm == 2 ? 108 * 1024 : 218 * 1024;
+        for (uint32_t qt = pairs_per_list > 14.0 ? 32 : 16; qt >= 16; qt /= 2) {
+            const size_t b = static_cast<size_t>(plan->pieces) * b_terms * qt * TILE_PIECE;
+            for (uint32_t bufs = 2; bufs >= 1; --bufs) {
+                if (bufs * b + (per_sm == 2 ? 2 : 3) * stage <= room) {
+                    plan->qt = qt;
+                    plan->b_bufs = bufs;
+                    plan->per_sm = per_sm;
+                    plan->stages = static_cast<uint32_t>(std::min<size_t>((room - bufs * b) / stage, TILE_MAX_STAGES));
+                    plan->smem = bufs * b + plan->stages * stage + 1024;   // (room to start on a 1 KiB boundary)
+                    return true;
+                }
+            }
+        }
     }
-    if (kscan + SQ8_SLACK > 1024 - SCAN_THREADS) {
-        return false;   // (the scan depth limit of the grouped path, which reports it)
-    }
-    if (static_cast<double>(nq) * nprobe >= 6.0 * ix->nlist) {
-        return false;
-    }
-    const double rows = static_cast<double>(nq) * nprobe * (static_cast<double>(ix->n_stored) / ix->nlist);
-    if (ix->quant == VB200_QUANT_SQ8 && rows * ix->code_size > 1e9) {
-        return false;
-    }
-    return nprobe <= ix->nlist;
+    return false;
 }
 
-// The search of a small batch from queries to results.  ids / dists: host or device.
+// The line between pairs and tiles: from about four queries per probed list on a tile per list saves more of the
+// lists' traffic than grouping the pairs costs (three small launches).  SQ8 batches with k shallow against the
+// lists keep the pruning scan once they are large: their first list gives a bound that rules most pairs out.
+static ScoreScan
+ivf_score_scan(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe, TilePlan* plan) {
+    const SearchWorkspace& ws = ix->ws;
+    if (ix->quant == VB200_QUANT_SQ8_UNIFORM || ix->use_residual || ix->buckets_per_data > 1 || ws.opt_deadline ||
+        ws.exchange != nullptr || ix->n_stored == 0 || nprobe > ix->nlist) {
+        return SCAN_GROUPED;
+    }
+    if (kscan + SQ8_SLACK > 1024 - SCAN_THREADS) {
+        return SCAN_GROUPED;   // (the scan depth limit of the grouped path, which reports it)
+    }
+    const bool sq8 = ix->quant == VB200_QUANT_SQ8;
+    const double per_list = static_cast<double>(nq) * nprobe / ix->nlist;
+    const double mean_len = static_cast<double>(ix->n_stored) / ix->nlist;
+    const double rows = static_cast<double>(nq) * nprobe * mean_len;
+    if (tensor_cores_enabled() && per_list >= TILE_MIN_QUERIES && nq * ix->longest_rows[nprobe] < (uint64_t{1} << 28) &&
+        nq * nprobe < (uint64_t{1} << 31) && tile_plan(ix, per_list, plan)) {
+        const bool prunes = sq8 && ix->prune_lists && ix->codes_t.ptr != nullptr && 8.0 * (kscan + SQ8_SLACK) <= mean_len && rows > 4e6;
+        if (!prunes) {
+            return SCAN_TILES;
+        }
+    }
+    if (per_list >= 6.0 || (sq8 && rows * ix->code_size > 1e9)) {
+        return SCAN_GROUPED;
+    }
+    return SCAN_PAIRS;
+}
+
+// Groups the pairs by list and scans the lists as tiles into the score buffer.
 static int
-ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, uint32_t kscan, uint32_t nprobe, bool rerank,
-                 const int32_t* bucket_ids, int64_t* ids, float* dists) {
+launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& plan) {
+    SearchWorkspace& ws = ix->ws;
+    const uint32_t nlist = ix->nlist, nprobe = sc.nprobe;
+    const uint64_t pairs = nq * nprobe;
+    const uint64_t max_items = pairs / plan.qt + std::min<uint64_t>(pairs, nlist);
+    VB_TRY(ws.tile_tables.reserve(3 * static_cast<size_t>(nlist) + 1));
+    VB_TRY(ws.tile_pairs.reserve(pairs));
+    VB_TRY(ws.tile_items.reserve(max_items));
+    TileGroup g{};
+    g.count = ws.tile_count.ptr;
+    g.rank = ws.tile_rank.ptr;
+    g.probes = sc.probes;
+    g.pairs = static_cast<uint32_t>(pairs);
+    g.nlist = nlist;
+    g.qt = plan.qt;
+    g.order = ix->scan_order.ptr;
+    g.pair_off = ws.tile_tables.ptr;
+    g.item_off = ws.tile_tables.ptr + nlist;
+    g.list_pairs = ws.tile_tables.ptr + 2 * static_cast<size_t>(nlist);
+    g.n_items = ws.tile_tables.ptr + 3 * static_cast<size_t>(nlist);
+    g.pair_ids = ws.tile_pairs.ptr;
+    g.items = ws.tile_items.ptr;
+    VB_LAUNCH(tile_places_kernel, 1, 1024, 0, g);
+    VB_LAUNCH(tile_scatter_kernel, static_cast<uint32_t>((std::max<uint64_t>(pairs, nlist) + 255) / 256), 256, 0, g);
+    TileScan t{};
+    t.s = sc.s;
+    t.t = sc.t;
+    t.nprobe = nprobe;
+    t.items = g.items;
+    t.n_items = g.n_items;
+    t.pair_ids = g.pair_ids;
+    t.pieces = plan.pieces;
+    t.stages = plan.stages;
+    t.b_bufs = plan.b_bufs;
+    t.qw8 = sc.qw8;
+    t.qscale = sc.qscale;
+    t.qsum = ws.qsum.ptr;
+    t.qstride = ix->quant == VB200_QUANT_RABITQ ? (ix->dim + 15) / 16 * 16 : ix->dpad;
+    t.row_norm = ix->code_norm.ptr;
+    t.l2 = ix->metric == VB200_METRIC_L2 ? 1u : 0u;
+    t.spin_limit = tc_spin_limit();
+    t.error_flag = reinterpret_cast<int*>(ws.scalars.ptr + 4);
+    void (*kernel)(const TileScan) = nullptr;
+#define VB_TILE(FMT) kernel = plan.qt == 32 ? tile_scan_kernel<FMT, 32> : tile_scan_kernel<FMT, 16>
+    switch (ix->quant) {
+        case VB200_QUANT_SQ8: VB_TILE(ROW_SQ8); break;
+        case VB200_QUANT_FP32: VB_TILE(ROW_F32); break;
+        case VB200_QUANT_BF16: VB_TILE(ROW_BF16); break;
+        case VB200_QUANT_FP16: VB_TILE(ROW_FP16); break;
+        default: VB_TILE(ROW_RABITQ); break;
+    }
+#undef VB_TILE
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), plan.smem));
+    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(max_items, static_cast<uint64_t>(sm_count()) * plan.per_sm));
+    VB_LAUNCH(kernel, grid, TILE_THREADS, plan.smem, t);
+    return 0;
+}
+
+// The search of a batch through a score per (query, row of its lists), from queries to results.  `plan`: the tile
+// launch, or null to scan pair by pair.  ids / dists: host or device.
+static int
+ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, uint32_t kscan, uint32_t nprobe, bool rerank,
+                  const TilePlan* plan, const int32_t* bucket_ids, int64_t* ids, float* dists) {
     SearchWorkspace& ws = ix->ws;
     cudaStream_t st = current_stream();
     const uint32_t dim = ix->dim, nlist = ix->nlist;
@@ -3126,7 +3235,8 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
     const bool pin_out = (host_ids || host_d) && total * 12 <= PINNED_IO_BYTES;
     const size_t ids_at = pin_q ? (q_bytes + 15) / 16 * 16 : 0, dists_at = ids_at + (pin_out ? total * sizeof(int64_t) : 0);
     const size_t rows_at = dists_at + (pin_out ? (total * sizeof(float) + 15) / 16 * 16 : 0);
-    VB_TRY(ws.pinned.reserve(rows_at + nq * sizeof(uint32_t)));
+    const size_t scalars_at = (rows_at + nq * sizeof(uint32_t) + 15) / 16 * 16;
+    VB_TRY(ws.pinned.reserve(scalars_at + SCALARS * sizeof(uint64_t)));
     unsigned char* pin = static_cast<unsigned char*>(ws.pinned.ptr);
     const float* q_dev = queries;
     if (host_q) {
@@ -3153,7 +3263,7 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
     const uint64_t stride = (ix->longest_rows[nprobe] + 31) / 32 * 32;
     VB_CHECK_ARG(stride < 0xFFFFFFFFull, "the probed lists hold too many rows");
     uint64_t slice = (uint64_t{256} << 20) / (stride > 0 ? stride : 1);
-    slice = slice < 1 ? 1 : (slice > nq ? nq : slice);
+    slice = slice < 1 ? 1 : (slice > nq || plan != nullptr ? nq : slice);
     VB_TRY(ws.pair_scores.reserve(slice * stride));
     if (sq8) {
         VB_TRY(ws.qw8.reserve(nq * 3 * ix->dpad));
@@ -3177,6 +3287,15 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
         pp.qscale = ws.qscale.ptr;
         pp.qa = ws.qa.ptr;
     }
+    if (plan != nullptr) {
+        if (ws.tile_count.cap < nlist) {
+            VB_TRY(ws.tile_count.reserve(nlist));
+            VB_CUDA(cudaMemsetAsync(ws.tile_count.ptr, 0, nlist * sizeof(uint32_t), st));   // tile_places_kernel leaves it cleared
+        }
+        VB_TRY(ws.tile_rank.reserve(nq * nprobe));
+        pp.count = ws.tile_count.ptr;
+        pp.rank = ws.tile_rank.ptr;
+    }
     bool routed_on_tensor_cores = false;
     if (bucket_ids != nullptr) {
         VB_CUDA(cudaMemcpyAsync(ws.probes.ptr, bucket_ids, nq * nprobe * sizeof(int32_t), cudaMemcpyDefault, st));
@@ -3196,6 +3315,14 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
         VB_TRY(ws.qproc.reserve(nq * (dim + 1)));
         VB_TRY(rabitq_process_query_device(q_dev, nq, dim, ix->rotation.ptr, ix->rq_centroid.ptr, ws.qproc.ptr, &ws.qrot));
         q_scan = ws.qproc.ptr;
+        if (plan != nullptr) {
+            const uint32_t qstride = (dim + 15) / 16 * 16;
+            VB_TRY(ws.qw8.reserve(nq * 3 * qstride));
+            VB_TRY(ws.qscale.reserve(nq));
+            VB_TRY(ws.qsum.reserve(nq * 4));
+            VB_LAUNCH(rabitq_terms_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, 0, ws.qproc.ptr, dim, qstride,
+                      1.0f / sqrtf(static_cast<float>(dim)), ws.qw8.ptr, ws.qscale.ptr, ws.qsum.ptr);
+        }
     }
 
     ScanFinalize f{};
@@ -3225,7 +3352,10 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
     const uint64_t mean_len = ix->n_stored / nlist;
     f.scan.per_pair = static_cast<uint32_t>(std::min<uint64_t>((ix->max_list_len + RS_ROWS - 1) / RS_ROWS, mean_len / RS_ROWS + 2));
     f.kscan = kscan;
-    f.kcand = sq8 ? kscan + SQ8_SLACK : kscan;
+    // candidates beyond kscan: room between what is kept and what is dropped (see scan_finalize_kernel); the one-bit
+    // estimates lie closer together than their worst-case rounding
+    f.kcand = !sq8 && plan == nullptr ? kscan : kscan + (ix->quant == VB200_QUANT_RABITQ ? std::min<uint32_t>(64, 1024 - kscan) : SQ8_SLACK);
+    f.row_max = ix->row_max.ptr;
     f.k = k;
     f.lower = ix->lower.ptr;
     f.diff = ix->diff.ptr;
@@ -3241,27 +3371,35 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
     float* dists_dev = !host_d ? dists : (pin_out ? reinterpret_cast<float*>(pin + dists_at) : ws.out_dists.ptr);
 
     const size_t scan_smem = RS_STAGES * RS_STAGE + (sq8 ? 3 * static_cast<size_t>(ix->dpad) : f.scan.qstride * sizeof(float));
-    const size_t final_smem = (2 * static_cast<size_t>(nprobe) + (sq8 ? 3 : (rerank ? 1 : 0)) * static_cast<size_t>(dim)) * sizeof(float);
+    const size_t final_smem = (2 * static_cast<size_t>(nprobe) + 4 + (sq8 || rerank ? (dim + 3) / 4 * 4 : 0) +
+                               (sq8 ? 2 * dim : (plan != nullptr ? f.scan.qstride : 0))) * sizeof(float);
     VB_CHECK_ARG(scan_smem <= 220 * 1024 && final_smem <= 180 * 1024, "dim = %u is too large for the scan", dim);
     void (*scan_kernel)(const PairScan) = nullptr;
     void (*final_kernel)(const ScanFinalize) = nullptr;
-#define VB_PAIRS(FMT)                                                                                \
-    {                                                                                                \
-        scan_kernel = l2 ? pair_scan_kernel<FMT, true> : pair_scan_kernel<FMT, false>;               \
-        final_kernel = l2 ? scan_finalize_kernel<FMT, true> : scan_finalize_kernel<FMT, false>;      \
+#define VB_FINAL(FMT, APPROX) (l2 ? scan_finalize_kernel<FMT, true, APPROX> : scan_finalize_kernel<FMT, false, APPROX>)
+#define VB_PAIRS(FMT)                                                                       \
+    {                                                                                       \
+        scan_kernel = l2 ? pair_scan_kernel<FMT, true> : pair_scan_kernel<FMT, false>;      \
+        final_kernel = plan != nullptr ? VB_FINAL(FMT, true) : VB_FINAL(FMT, false);        \
     }
     switch (ix->quant) {
-        case VB200_QUANT_SQ8: VB_PAIRS(ROW_SQ8) break;
+        case VB200_QUANT_SQ8:
+            scan_kernel = l2 ? pair_scan_kernel<ROW_SQ8, true> : pair_scan_kernel<ROW_SQ8, false>;
+            final_kernel = VB_FINAL(ROW_SQ8, true);
+            break;
         case VB200_QUANT_FP32: VB_PAIRS(ROW_F32) break;
         case VB200_QUANT_BF16: VB_PAIRS(ROW_BF16) break;
         case VB200_QUANT_FP16: VB_PAIRS(ROW_FP16) break;
         default:
             scan_kernel = pair_scan_kernel<ROW_RABITQ, true>;
-            final_kernel = scan_finalize_kernel<ROW_RABITQ, true>;
+            final_kernel = plan != nullptr ? scan_finalize_kernel<ROW_RABITQ, true, true> : scan_finalize_kernel<ROW_RABITQ, true, false>;
             break;
     }
 #undef VB_PAIRS
-    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(scan_kernel), scan_smem));
+#undef VB_FINAL
+    if (plan == nullptr) {
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(scan_kernel), scan_smem));
+    }
     // (beside about 34 KiB of static shared memory)
     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(final_kernel), final_smem + (final_smem > 12 * 1024 ? 40 * 1024 : 0)));
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
@@ -3280,12 +3418,16 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
         g.rows_scanned += q0;
         g.ids = ids_dev + q0 * k;
         g.dists = dists_dev + q0 * k;
-        const uint64_t blocks = n * nprobe * g.scan.per_pair;
-        VB_CHECK_ARG(blocks <= 0x7fffffffull, "query batch too large");
         if (q0 == 0) {
             VB_CUDA(cudaEventRecord(ix->ev_scan_begin, st));
         }
-        VB_LAUNCH(scan_kernel, static_cast<uint32_t>(blocks), RS_ROWS, scan_smem, g.scan);
+        if (plan != nullptr) {
+            VB_TRY(launch_tiles(ix, g.scan, nq, *plan));
+        } else {
+            const uint64_t blocks = n * nprobe * g.scan.per_pair;
+            VB_CHECK_ARG(blocks <= 0x7fffffffull, "query batch too large");
+            VB_LAUNCH(scan_kernel, static_cast<uint32_t>(blocks), RS_ROWS, scan_smem, g.scan);
+        }
         if (q0 + n == nq) {
             VB_CUDA(cudaEventRecord(ix->ev_scan_end, st));
             ix->scan_timed = true;
@@ -3301,7 +3443,21 @@ ivf_search_pairs(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, u
             VB_CUDA(cudaMemcpyAsync(dists, dists_dev, total * sizeof(float), cudaMemcpyDeviceToHost, st));
         }
     }
-    VB_TRY(routed_on_tensor_cores ? route_sync_and_check(ws) : sync_stream());
+    uint64_t* scalars = reinterpret_cast<uint64_t*>(pin + scalars_at);
+    const bool flagged = routed_on_tensor_cores || plan != nullptr;
+    if (flagged) {
+        VB_CUDA(cudaMemcpyAsync(scalars, ws.scalars.ptr, SCALARS * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    }
+    VB_TRY(sync_stream());
+    if (flagged) {
+        if (routed_on_tensor_cores) {
+            VB_TRY(route_flag_check(scalars[8]));
+        }
+        if (plan != nullptr && scalars[4] != 0) {
+            VB_CUDA(cudaMemsetAsync(ws.scalars.ptr + 4, 0, sizeof(uint64_t), st));
+            VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
+        }
+    }
     if (pin_out) {
         if (host_ids) {
             std::memcpy(ids, pin + ids_at, total * sizeof(int64_t));
@@ -3746,6 +3902,23 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
             VB_LAUNCH(sq8_residual_bias_kernel, static_cast<uint32_t>((n_new_stored + 127) / 128), 128, 0, new_codes.ptr,
                       n_new_stored, dim, stride, ix->lower.ptr, ix->diff.ptr, new_off_dev.ptr, nlist, ix->centroids.ptr,
                       ix->metric, ix->res_bias.ptr, new_norm.ptr);
+        }
+    }
+    if (n_new_stored > 0 && ix->quant != VB200_QUANT_SQ8_UNIFORM) {
+        VB_TRY(ix->row_max.reserve(2));
+        VB_CUDA(cudaMemsetAsync(ix->row_max.ptr, 0, 2 * sizeof(float), current_stream()));
+        const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n_new_stored + 7) / 8, 16ull * sm_count()));
+        if (ix->quant != VB200_QUANT_SQ8 && ix->quant != VB200_QUANT_RABITQ) {
+            VB_TRY(new_norm.reserve(n_new_stored));
+        }
+        const uint8_t* codes = new_codes.ptr;
+        float *norm = new_norm.ptr, *top = ix->row_max.ptr;
+        switch (ix->quant) {
+            case VB200_QUANT_FP32: VB_LAUNCH(record_norms_kernel<ROW_F32>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
+            case VB200_QUANT_BF16: VB_LAUNCH(record_norms_kernel<ROW_BF16>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
+            case VB200_QUANT_FP16: VB_LAUNCH(record_norms_kernel<ROW_FP16>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
+            case VB200_QUANT_SQ8: VB_LAUNCH(record_norms_kernel<ROW_SQ8>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
+            default: VB_LAUNCH(record_norms_kernel<ROW_RABITQ>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
         }
     }
     if (ix->quant == VB200_QUANT_SQ8) {
@@ -4228,9 +4401,12 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
             if (rerank) {
                 VB_TRY(rerank_depth(k, factor, &kscan));
             }
-            if (ivf_pairs_fit(ix, nq, kscan, np)) {
+            TilePlan plan{};
+            const ScoreScan how = ivf_score_scan(ix, nq, kscan, np, &plan);
+            if (how != SCAN_GROUPED) {
                 ws.filter = filter;
-                const int rc = ivf_search_pairs(ix, queries, nq, k, kscan, np, rerank, bucket_ids, ids, dists);
+                const int rc = ivf_search_scores(ix, queries, nq, k, kscan, np, rerank, how == SCAN_TILES ? &plan : nullptr, bucket_ids, ids,
+                                                 dists);
                 ws.filter = nullptr;
                 return rc;
             }

@@ -59,6 +59,8 @@ struct PairsPrepare {
     float* probe_dists;       // [nq x nprobe] or null
     const uint32_t* list_off;
     PairTable t;
+    uint32_t* count;          // [nlist] += 1 per pair of a list that is not empty, or null
+    uint32_t* rank;           // [nq x nprobe] which of its list's pairs each is (0xFFFFFFFF: empty list)
     // SQ8 (null qw8: none): the int8 weight terms, their scale and the query's constant (see sq8_query_prep_kernel)
     const float* queries;
     uint32_t dim, dpad;
@@ -136,6 +138,9 @@ pairs_prepare_kernel(const PairsPrepare p) {
             if (l >= 0 && static_cast<uint32_t>(l) < p.nlist) {
                 len = p.list_off[l + 1] - p.list_off[l];
             }
+            if (p.count != nullptr) {
+                p.rank[q * p.nprobe + i] = len > 0 ? atomicAdd(p.count + l, 1u) : 0xFFFFFFFFu;
+            }
         }
         const uint32_t incl = block_inclusive_sum<PAIR_THREADS>(len, sel.warp_part);
         if (i < p.nprobe) {
@@ -179,6 +184,106 @@ pairs_prepare_kernel(const PairsPrepare p) {
     if (threadIdx.x == 0) {
         p.qscale[q] = s;
         p.qa[q] = p.metric == VB200_METRIC_L2 ? fmaf(-2.0f, qm, qq) : 1.0f - qm;
+    }
+}
+
+// RaBitQ: the values sv_d = inv_sqrt_d * q_d of the estimator as three int8 terms, their scale and the terms' sums.
+__global__ void __launch_bounds__(PAIR_THREADS)
+rabitq_terms_kernel(const float* __restrict__ queries, uint32_t dim, uint32_t qstride, float inv_sqrt_d, int8_t* __restrict__ qw8,
+                    float* __restrict__ qscale, int32_t* __restrict__ qsum) {
+    __shared__ float part[PAIR_THREADS / 32];
+    __shared__ int32_t sums[3];
+    const uint64_t q = blockIdx.x;
+    const float* src = queries + q * (dim + 1);
+    float wmax = 0.f;
+    for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
+        wmax = fmaxf(wmax, fabsf(__fmul_rn(inv_sqrt_d, __ldg(src + d))));
+    }
+    if (threadIdx.x < 3) {
+        sums[threadIdx.x] = 0;
+    }
+    wmax = pair_block_max(wmax, part);
+    const float s = wmax > 0.f && wmax < INFINITY ? wmax / 127.0f : 1.0f;
+    int8_t* t = qw8 + q * 3 * qstride;
+    int32_t n1 = 0, n2 = 0, n3 = 0;
+    for (uint32_t d = threadIdx.x; d < qstride; d += PAIR_THREADS) {
+        const float u = d < dim ? __fmul_rn(inv_sqrt_d, __ldg(src + d)) / s : 0.f;
+        const float t1 = fminf(fmaxf(rintf(u), -127.f), 127.f);
+        const float v2 = (u - t1) * 254.0f;
+        const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
+        const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
+        t[d] = static_cast<int8_t>(static_cast<int>(t1));
+        t[qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
+        t[2 * qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
+        n1 += static_cast<int>(t1);
+        n2 += static_cast<int>(t2);
+        n3 += static_cast<int>(t3);
+    }
+    n1 = __reduce_add_sync(0xffffffffu, n1);
+    n2 = __reduce_add_sync(0xffffffffu, n2);
+    n3 = __reduce_add_sync(0xffffffffu, n3);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sums[0], n1);
+        atomicAdd(&sums[1], n2);
+        atomicAdd(&sums[2], n3);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        qsum[4 * q + threadIdx.x] = sums[threadIdx.x];
+    }
+    if (threadIdx.x == 0) {
+        qscale[q] = s;
+    }
+}
+
+// Squared norms of the stored rows and the largest norm (RaBitQ: of the norms and norm / |error| in the records;
+// SQ8: of the norms already in `norm`).  A warp per row; top[] is cleared by the caller.
+template <int FMT>
+__global__ void __launch_bounds__(256)
+record_norms_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim, uint32_t stride, float* __restrict__ norm,
+                    float* __restrict__ top) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warp = (static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5, warps = static_cast<uint64_t>(gridDim.x) * 8;
+    float most = 0.f, gain = 0.f;
+    if (FMT == ROW_SQ8 || FMT == ROW_RABITQ) {
+        for (uint64_t r = warp * 32 + lane; r < n; r += warps * 32) {
+            if (FMT == ROW_SQ8) {
+                most = fmaxf(most, norm[r]);
+            } else {
+                const float* tail = reinterpret_cast<const float*>(codes + r * stride + ((dim + 7) / 8 + 3) / 4 * 4);
+                const float err = fabsf(tail[1]);
+                most = fmaxf(most, tail[0]);
+                gain = fmaxf(gain, tail[0] / (err < 1e-5f ? 1.0f : err));
+            }
+        }
+    } else {
+        for (uint64_t r = warp; r < n; r += warps) {
+            float s = 0.f;
+            for (uint32_t d = lane; d < dim; d += 32) {
+                float v;
+                if (FMT == ROW_F32) {
+                    v = reinterpret_cast<const float*>(codes + r * stride)[d];
+                } else {
+                    v = half_decode<FMT == ROW_BF16 ? SCAN_FMT_BF16 : SCAN_FMT_FP16>(reinterpret_cast<const uint16_t*>(codes + r * stride)[d]);
+                }
+                s = fmaf(v, v, s);
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+            }
+            if (lane == 0) {
+                norm[r] = s;
+            }
+            most = fmaxf(most, s);
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        gain = fmaxf(gain, __shfl_xor_sync(0xffffffffu, gain, o));
+    }
+    if (lane == 0) {   // non-negative floats order like their bit patterns
+        atomicMax(reinterpret_cast<int*>(top), __float_as_int(FMT == ROW_RABITQ ? most : sqrtf(most) * 1.000001f));
+        atomicMax(reinterpret_cast<int*>(top + 1), __float_as_int(gain * 1.000001f));
     }
 }
 
@@ -290,6 +395,7 @@ struct ScanFinalize {
     uint32_t kscan, k;         // results of the scan per query; results of the search (fewer with a rerank)
     uint32_t kcand;            // candidates taken from the scores: kscan, and more when they are re-scored
     const float *lower, *diff; // SQ8
+    const float* row_max;      // [0] largest row norm of the index; RaBitQ: [1] largest norm / |error|
     const float* queries;      // [nq x dim] plain queries (SQ8 re-scoring, rerank)
     const uint32_t* pos_inner;
     const int64_t* labels;
@@ -353,58 +459,161 @@ struct ScorePosition {
     }
 };
 
-// Dynamic shared memory: [2][nprobe] pair places and list starts, [rerank or SQ8: query, SQ8: lower, diff] floats.
+// Exact distance of one code record in the reference's operation order; qc: the query as the codec's chain reads it
+// (stage_query), zero padded.  Four 16-byte loads in flight.
 template <int FMT, bool L2>
+__device__ __forceinline__ float
+record_exact_distance(const uint8_t* rec, uint32_t dim, uint32_t row_bytes, const float* qc, float qn) {
+    RowAcc<FMT, L2, 1> acc;
+    acc.clear();
+    constexpr uint32_t UD = RowAcc<FMT, L2, 1>::UNIT_DIMS;
+    const uint4* v = reinterpret_cast<const uint4*>(rec);
+    const uint32_t units = (dim + UD - 1) / UD;
+    for (uint32_t u0 = 0; u0 < units; u0 += 4) {
+        uint4 w[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            w[j] = u0 + j < units ? __ldg(v + u0 + j) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t d0 = (u0 + j) * UD;
+            if (d0 + UD <= dim) {
+                acc.unit(w[j], qc, 0, d0);
+            } else if (d0 < dim) {
+                acc.tail(w[j], qc, 0, d0, dim - d0);
+            }
+        }
+    }
+    if constexpr (FMT == ROW_RABITQ) {
+        const float* tail = reinterpret_cast<const float*>(rec + row_bytes);
+        return rabitq_distance(acc.acc[0], __ldg(tail), __ldg(tail + 1), qn);
+    } else {
+        return L2 ? acc.acc[0] : __fsub_rn(1.0f, acc.acc[0]);
+    }
+}
+
+// Dynamic shared memory: [2][nprobe] pair places and list starts; [rerank or SQ8] the plain query; [SQ8] lower and
+// diff, or [other codecs re-scored after tiles] the query as the codec reads it (qstride floats).
+// APPROX: the scores only rank (SQ8's integer form, tensor-core tiles).  The kcand best by score are re-scored
+// exactly; a row that was not among them has an exact distance of at least (the last kept score - margin), margin
+// bounding the difference between score and exact distance, so when the kscan-th exact distance is below that the
+// result is the exact one.  Otherwise (scores crowded within the rounding of the arithmetic) every row of the query
+// is scored exactly here.
+template <int FMT, bool L2, bool APPROX>
 __global__ void __launch_bounds__(PAIR_THREADS)
 scan_finalize_kernel(const ScanFinalize p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
+    __shared__ float part[PAIR_THREADS / 32];
     const PairScan& sc = p.scan;
-    uint32_t* base_s = reinterpret_cast<uint32_t*>(smem);
-    uint32_t* start_s = base_s + sc.nprobe;
-    float* qs = reinterpret_cast<float*>(start_s + sc.nprobe);
     const uint64_t q = blockIdx.x;
     const uint32_t nprobe = sc.nprobe, dim = sc.s.dim;
+    uint32_t* base_s = reinterpret_cast<uint32_t*>(smem);
+    uint32_t* start_s = base_s + sc.nprobe;
+    const bool plain = FMT == ROW_SQ8 || p.flat != nullptr;
+    float* qs = reinterpret_cast<float*>(smem + (2 * nprobe * sizeof(uint32_t) + 15) / 16 * 16);
+    float* qc = qs + (plain ? (dim + 3) / 4 * 4 : 0u);     // SQ8: lower, then diff
     const uint32_t n = sc.t.rows[q];
-    const uint32_t* scores = reinterpret_cast<const uint32_t*>(sc.t.scores + q * sc.t.stride);
+    uint32_t* scores = reinterpret_cast<uint32_t*>(sc.t.scores + q * sc.t.stride);
     for (uint32_t i = threadIdx.x; i < nprobe; i += PAIR_THREADS) {
         const int32_t l = __ldg(sc.probes + q * nprobe + i);
         base_s[i] = __ldg(sc.t.base + q * nprobe + i);
         start_s[i] = l >= 0 && static_cast<uint32_t>(l) < sc.s.nlist ? __ldg(sc.s.list_off + l) : 0u;
     }
-    if (FMT == ROW_SQ8 || p.flat != nullptr) {
+    if (plain) {
         const float* src = p.queries + q * dim;
         for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
             qs[d] = __ldg(src + d);
             if (FMT == ROW_SQ8) {
-                qs[dim + d] = __ldg(p.lower + d);
-                qs[2 * dim + d] = __ldg(p.diff + d);
+                qc[d] = __ldg(p.lower + d);
+                qc[dim + d] = __ldg(p.diff + d);
             }
         }
     }
+    if (APPROX && FMT != ROW_SQ8) {
+        stage_query<FMT>(sc, q, qc, PAIR_THREADS);
+    }
     __syncthreads();
     const ScorePosition position{base_s, start_s, nprobe};
-    const ScoreSource<> value{scores};
-    const uint32_t found = block_select<PAIR_THREADS>(value, position, n, p.kcand, keys, sel);
+    auto exact = [&](uint32_t pos) -> float {
+        const uint8_t* rec = sc.s.codes + static_cast<uint64_t>(pos) * sc.s.code_stride;
+        if constexpr (FMT == ROW_SQ8) {
+            return sq8_exact_distance(rec, dim, L2, qs, qc, qc + dim);
+        } else {
+            const float qn = FMT == ROW_RABITQ ? __ldg(sc.s.queries + q * (dim + 1) + dim) : 0.f;
+            return record_exact_distance<FMT, L2>(rec, dim, sc.row_bytes, qc, qn);
+        }
+    };
+    uint32_t found = block_select<PAIR_THREADS>(ScoreSource<>{scores}, position, n, p.kcand, keys, sel);
     if (threadIdx.x == 0) {
         p.rows_scanned[q] = n;
     }
-    uint32_t have = found;
-    if (FMT == ROW_SQ8) {
-        // the kcand best by the ranking form, then their exact distances
+    if (APPROX) {
         block_sort_to<PAIR_THREADS>(keys, found, p.kcand, best);
-        have = min(found, p.kcand);
-        for (uint32_t i = threadIdx.x; i < have; i += PAIR_THREADS) {
+        const uint32_t kept = min(found, p.kcand);
+        const float last = kept > 0 ? ordered_to_float(static_cast<uint32_t>(best[kept - 1] >> 32)) : 0.f;
+        for (uint32_t i = threadIdx.x; i < kept; i += PAIR_THREADS) {
             const uint32_t pos = static_cast<uint32_t>(best[i]);
-            keys[i] = make_key(sq8_exact_distance(sc.s.codes + static_cast<uint64_t>(pos) * sc.s.code_stride, dim, L2, qs, qs + dim,
-                                                  qs + 2 * dim),
-                               pos);
+            keys[i] = make_key(exact(pos), pos);
         }
+        bool sure = found < p.kcand;   // nothing was dropped
+        block_sort_to<PAIR_THREADS>(keys, kept, p.kscan, best);
+        found = kept;
+        if (!sure && kept >= p.kscan) {
+            const float kth = ordered_to_float(static_cast<uint32_t>(best[p.kscan - 1] >> 32));
+            float margin, offset = 0.f;
+            const float rows_max = __ldg(p.row_max);
+            if constexpr (FMT == ROW_RABITQ) {
+                const float qn = __ldg(sc.s.queries + q * (dim + 1) + dim);
+                // the dropped parts of the int8 terms and the additions' rounding, through 2 |x| |q| / error
+                const float ip = dim * (__ldg(sc.qscale + q) * (0.5f / 64516.0f) + 1.2e-7f);
+                margin = 2.0f * qn * __ldg(p.row_max + 1) * ip + 1e-6f * (rows_max + qn) * (rows_max + qn);
+            } else {
+                float qq = 0.f, mm = 0.f;
+                for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
+                    const float v = FMT == ROW_SQ8 ? qs[d] : qc[d];
+                    qq = fmaf(v, v, qq);
+                    if (FMT == ROW_SQ8) {
+                        const float mid = fmaf(qc[dim + d], 128.0f / 255.0f, qc[d]);
+                        mm = fmaf(mid, mid, mm);
+                    }
+                }
+                qq = pair_block_sum(qq, part);
+                const float qn = sqrtf(qq);
+                float size = qn + rows_max;
+                margin = 0.f;
+                if constexpr (FMT == ROW_SQ8) {
+                    size += sqrtf(pair_block_sum(mm, part));
+                    margin = 2.0f * dim * 128.0f * __ldg(sc.qscale + q) * (0.5f / 64516.0f);
+                } else {
+                    offset = L2 ? qq : 1.0f;
+                    if (FMT == ROW_F32) {
+                        margin = 2.0f * qn * rows_max * (3.0f / 262144.0f);   // three dropped products of 2^-18
+                    }
+                }
+                margin += (dim + 16) * 1.2e-7f * size * size;   // fp32 sums of either side
+            }
+            sure = kth < last + offset - margin;
+        }
+        if (!sure && n > 0) {
+            for (uint32_t i = threadIdx.x; i < n; i += PAIR_THREADS) {
+                if (ScoreSource<>::ordered(scores[i]) <= ORDERED_INF) {
+                    scores[i] = __float_as_uint(exact(position(i)));
+                }
+            }
+            __syncthreads();
+            const volatile uint32_t* rescored = scores;
+            found = block_select<PAIR_THREADS>(load_source([&](uint32_t i) { return ScoreSource<>::ordered(rescored[i]); }), position, n,
+                                               p.kscan, keys, sel);
+            block_sort_to<PAIR_THREADS>(keys, found, p.kscan, best);
+        }
+    } else {
+        block_sort_to<PAIR_THREADS>(keys, found, p.kscan, best);
     }
-    block_sort_to<PAIR_THREADS>(keys, have, p.kscan, best);
-    have = min(have, p.kscan);
+    uint32_t have = min(found, p.kscan);
     const uint64_t* final_keys = best;
     if (p.flat != nullptr) {
         // FlattenReorder::Reorder (rerank_kernel): a warp per candidate, the fp32 row by inner id
