@@ -7,54 +7,9 @@
 #pragma once
 
 #include "block_select.cuh"
-#include "dense.cuh"
 #include "row_scan.cuh"
 
 namespace vb200 {
-
-// Distance of one row to the query (widened, in shared memory), rows fetched sixteen bytes at a time with four
-// loads in flight where their alignment allows.
-template <typename E>
-__device__ __forceinline__ float
-bf_exact_distance(const E* __restrict__ x, const float* qf, uint32_t dim, bool l2) {
-    constexpr uint32_t VEC = 16 / sizeof(E);
-    float s = 0.f;
-    auto step = [&](float v, float q) {
-        if (l2) {
-            const float t = __fsub_rn(v, q);
-            s = fmaf(t, t, s);
-        } else {
-            s = fmaf(v, q, s);
-        }
-    };
-    if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0 && dim % VEC == 0) {
-        const uint4* xv = reinterpret_cast<const uint4*>(x);
-        const uint32_t nv = dim / VEC;
-        for (uint32_t v0 = 0; v0 < nv; v0 += 4) {
-            uint4 w[4];
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
-                w[u] = v0 + u < nv ? __ldg(xv + v0 + u) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
-                if (v0 + u < nv) {
-                    E e[VEC];
-                    *reinterpret_cast<uint4*>(e) = w[u];
-#pragma unroll
-                    for (uint32_t j = 0; j < VEC; ++j) {
-                        step(widen(e[j]), qf[(v0 + u) * VEC + j]);
-                    }
-                }
-            }
-        }
-    } else {
-        for (uint32_t d = 0; d < dim; ++d) {
-            step(widen(x[d]), qf[d]);
-        }
-    }
-    return l2 ? s : __fsub_rn(1.0f, s);
-}
 
 constexpr int BF_STREAM_QUERIES = 8;
 
@@ -182,7 +137,7 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
     const uint32_t have = min(found, kcand);
     for (uint32_t i = threadIdx.x; i < have; i += T) {
         const uint32_t row = static_cast<uint32_t>(best[i]);
-        keys[i] = make_key(bf_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, metric == VB200_METRIC_L2), row);
+        keys[i] = make_key(row_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, metric == VB200_METRIC_L2), row);
     }
     block_sort_to<T>(keys, have, k, best);
     for (uint32_t i = threadIdx.x; i < k; i += T) {

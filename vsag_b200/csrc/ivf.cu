@@ -774,84 +774,6 @@ sq8_query_prep_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t d
 // search kernels
 // ---------------------------------------------------------------------------------------------
 
-// Re-scores the routing candidates of one query exactly and orders them: distance ascending,
-// lower list id first on ties.  L2: FMA chain of (q-c)^2 over d ascending; IP: 1 - chain of q*c
-// (the loop of IVF::route_buckets_only, src/algorithm/ivf/ivf.cpp:1589-1660).
-__global__ void __launch_bounds__(128)
-route_finalize_kernel(const float* __restrict__ queries, uint32_t dim,
-                      const float* __restrict__ centroids, const uint64_t* __restrict__ cand,
-                      uint32_t ncand, uint32_t n2, uint32_t nprobe, int metric,
-                      int32_t* __restrict__ probes, float* __restrict__ probe_dists) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint64_t* keys = reinterpret_cast<uint64_t*>(smem_raw);
-    float* qs = reinterpret_cast<float*>(keys + n2);   // the query, staged once for all candidates
-    const float* q = queries + static_cast<uint64_t>(blockIdx.x) * dim;
-    const uint64_t* cq = cand + static_cast<uint64_t>(blockIdx.x) * ncand;
-    for (uint32_t d = threadIdx.x; d < dim; d += blockDim.x) {
-        qs[d] = q[d];
-    }
-    __syncthreads();
-    const bool vec4 = (dim & 3u) == 0;   // centroid rows are then 16-byte aligned
-    for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) {
-        uint64_t key = KEY_INF;
-        if (i < ncand && cq[i] != KEY_INF) {
-            uint32_t list = static_cast<uint32_t>(cq[i]);
-            const float* c = centroids + static_cast<uint64_t>(list) * dim;
-            float s = 0.f;
-            // one chain per candidate, dimensions in ascending order, as the reference computes it
-            if (vec4) {
-                const float4* c4 = reinterpret_cast<const float4*>(c);
-                const float4* q4 = reinterpret_cast<const float4*>(qs);
-                if (metric == VB200_METRIC_L2) {
-#pragma unroll 4
-                    for (uint32_t d4 = 0; d4 < (dim >> 2); ++d4) {
-                        const float4 cv = __ldg(c4 + d4), qv = q4[d4];
-                        float t = __fsub_rn(qv.x, cv.x);
-                        s = fmaf(t, t, s);
-                        t = __fsub_rn(qv.y, cv.y);
-                        s = fmaf(t, t, s);
-                        t = __fsub_rn(qv.z, cv.z);
-                        s = fmaf(t, t, s);
-                        t = __fsub_rn(qv.w, cv.w);
-                        s = fmaf(t, t, s);
-                    }
-                } else {
-#pragma unroll 4
-                    for (uint32_t d4 = 0; d4 < (dim >> 2); ++d4) {
-                        const float4 cv = __ldg(c4 + d4), qv = q4[d4];
-                        s = fmaf(qv.x, cv.x, s);
-                        s = fmaf(qv.y, cv.y, s);
-                        s = fmaf(qv.z, cv.z, s);
-                        s = fmaf(qv.w, cv.w, s);
-                    }
-                    s = __fsub_rn(1.0f, s);
-                }
-            } else if (metric == VB200_METRIC_L2) {
-                for (uint32_t d = 0; d < dim; ++d) {
-                    float t = __fsub_rn(qs[d], __ldg(c + d));
-                    s = fmaf(t, t, s);
-                }
-            } else {
-                for (uint32_t d = 0; d < dim; ++d) {
-                    s = fmaf(qs[d], __ldg(c + d), s);
-                }
-                s = __fsub_rn(1.0f, s);
-            }
-            key = make_key(s, list);
-        }
-        keys[i] = key;
-    }
-    block_bitonic_sort(keys, n2);
-    for (uint32_t i = threadIdx.x; i < nprobe; i += blockDim.x) {
-        uint64_t key = keys[i];
-        uint64_t o = static_cast<uint64_t>(blockIdx.x) * nprobe + i;
-        probes[o] = key == KEY_INF ? -1 : static_cast<int32_t>(static_cast<uint32_t>(key));
-        if (probe_dists != nullptr) {
-            probe_dists[o] = key == KEY_INF ? INFINITY : ordered_to_float(static_cast<uint32_t>(key >> 32));
-        }
-    }
-}
-
 __device__ __forceinline__ bool
 probe_is_live(int32_t l, uint32_t nlist, uint32_t rank, uint32_t world, const uint32_t* list_off) {
     if (l < 0 || static_cast<uint32_t>(l) >= nlist || static_cast<uint32_t>(l) % world != rank) {
@@ -2340,9 +2262,22 @@ launch_row_chains(const float* queries, uint64_t nq, uint64_t q_stride, const fl
     return 0;
 }
 
+constexpr uint64_t ROUTE_MATRIX_SCORES = uint64_t{24} << 20;   // 96 MiB of the 126 MB L2
+
+// Tiles of the tensor-core kernel are 128 x 128: with fewer queries or lists they are mostly padding.
+static bool
+routes_on_tensor_cores(const vb200_ivf* ix, uint64_t nq) {
+    return tensor_cores_enabled() && nq >= 256 && ix->nlist >= 1024;
+}
+
+// Exact routing.  prepare (optional): what pairs_prepare_kernel is to do beyond routing; *prepared tells whether it
+// was done here (the threshold path leaves it to the caller).
 static int
-ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe, int32_t* probes_dev,
-                 float* dists_dev) {
+ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe, int32_t* probes_dev, float* dists_dev,
+                 const PairsPrepare* prepare = nullptr, bool* prepared = nullptr) {
+    if (prepared != nullptr) {
+        *prepared = true;
+    }
     SearchWorkspace& ws = ix->ws;
     VB_TRY(reserve_scalars(ws));
     int* route_flag = reinterpret_cast<int*>(ws.scalars.ptr + 8);
@@ -2354,10 +2289,24 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
     VB_TRY(ws.cand.reserve(nq * ncand));
     const bool l2 = ix->metric == VB200_METRIC_L2;
     const uint64_t ld = (static_cast<uint64_t>(nlist) + 3) / 4 * 4;
-    if (tensor_cores_enabled() && nq >= 256 && nlist >= 1024 && nq * ld <= (uint64_t{1} << 30)) {
-        // Scores from the tcgen05 kernel (split-bf16, good to ~1e-5 relative) nominate the
-        // candidates; the exact re-scoring below orders them and drops the slack, as on the
-        // SIMT path.
+    PairsPrepare pp{};
+    if (prepare != nullptr) {
+        pp = *prepare;
+    }
+    pp.nlist = nlist;
+    pp.nprobe = nprobe;
+    pp.ncand = ncand;
+    pp.ld = ld;
+    pp.queries = q_dev;
+    pp.dim = ix->dim;
+    pp.centroids = ix->centroids.ptr;
+    pp.metric = ix->metric;
+    pp.probes = probes_dev;
+    pp.probe_dists = dists_dev;
+    const size_t route_smem = ix->dim * sizeof(float);
+    VB_CHECK_ARG(route_smem <= 180 * 1024, "dim = %u is too large for the routing kernel", ix->dim);
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_kernel), route_smem + (route_smem > 8192 ? 40 * 1024 : 0)));
+    if (routes_on_tensor_cores(ix, nq)) {
         const uint32_t chunks = (ix->dim + TC_KC - 1) / TC_KC;
         if (!ix->c_tiled) {
             const size_t elems = tc_tiled_elems(nlist, ix->dim);
@@ -2374,7 +2323,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         VB_TRY(tc_pretile_f32(q_dev, nq, ix->dim, ws.q_hi.ptr, ws.q_lo.ptr));
         TcOperand a{ws.q_hi.ptr, ws.q_lo.ptr, nq, chunks};
         TcOperand b{ix->c_hi.ptr, ix->c_lo.ptr, nlist, chunks};
-        // Large list counts: no score matrix.  The scores against a sample of the centroids (the first
+        // Score matrices larger than ROUTE_MATRIX_SCORES over large list counts: no matrix.  The scores against a sample of the centroids (the first
         // `sample` of them; centroid numbering carries no geometry) give each query a threshold; one pass
         // of the tensor-core kernel over all centroids then keeps, unsorted, only what scores below it --
         // about rank * nlist / sample per query -- and one small kernel per query orders those and
@@ -2384,7 +2333,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         // and a lower rank they are only very likely, and a query that ends up with fewer than ncand is
         // answered exactly by route_pick_kernel like one whose lists overflowed.
         uint32_t sample = 0, rank = 0;
-        for (uint32_t s = 1024; s <= 4096 && sample == 0; s *= 2) {
+        for (uint32_t s = 1024; nq * ld > ROUTE_MATRIX_SCORES && s <= 4096 && sample == 0; s *= 2) {
             uint64_t r = (4ull * ncand * s + nlist - 1) / nlist;   // (3x and 5x measured slower: exact fallbacks, longer sorts)
             r = r < 16 ? 16 : r;
             r = r > ncand ? ncand : r;
@@ -2440,13 +2389,27 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
                 VB_LAUNCH(route_pick_kernel, static_cast<uint32_t>((nq + per_block - 1) / per_block), 256, smem, q_dev, nq, per_block,
                           ix->dim, ix->centroids.ptr, ws.route_keys.ptr, ws.route_cnt.ptr, lists, cap, ncand, nprobe, ix->metric,
                           probes_dev, dists_dev, handled, nlist);
+                if (prepared != nullptr) {
+                    *prepared = false;
+                }
                 return 0;
             }
-            VB_TRY(sync_stream());   // (more lists than the pick kernels take: the score-matrix path below)
         }
-        VB_TRY(ws.scores.reserve(nq * ld));
-        VB_TRY(tc_scores(ix->tc, a, b, 3, l2 ? -2.0f : -1.0f, l2 ? ix->c_sq.ptr : nullptr, ws.scores.ptr, ld));
-        VB_TRY(select_rows(ws.scores.ptr, nq, nlist, ld, ncand, 0, ws.cand.ptr, ncand));
+        // Otherwise the score matrix, in slices of whole row tiles that stay in L2, and a CTA per query that selects,
+        // re-scores exactly and goes on with whatever the caller wants prepared.
+        uint64_t slice = ROUTE_MATRIX_SCORES / ld / TC_BM * TC_BM;
+        slice = slice < TC_BM ? TC_BM : slice;
+        VB_TRY(ws.scores.reserve(std::min(slice, nq) * ld));
+        for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
+            const uint64_t m = std::min(slice, nq - q0);
+            const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
+            VB_TRY(tc_scores(ix->tc, TcOperand{ws.q_hi.ptr + off, ws.q_lo.ptr + off, m, chunks}, b, 3, l2 ? -2.0f : -1.0f,
+                             l2 ? ix->c_sq.ptr : nullptr, ws.scores.ptr, ld, route_flag));
+            PairsPrepare part = pp.from(q0);
+            part.scores = ws.scores.ptr;
+            VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(m), PAIR_THREADS, route_smem, part);
+        }
+        return 0;
     } else {
         uint64_t slab = (uint64_t{256} << 20) / nlist;  // rows of a 1 GiB distance slab
         slab = slab < 1 ? 1 : (slab > 65535 ? 65535 : slab);   // (a launch takes 65535 query tiles)
@@ -2455,20 +2418,13 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         for (uint64_t b = 0; b < nq; b += slab) {
             const uint64_t n = nq - b < slab ? nq - b : slab;
             VB_TRY(launch_row_chains(q_dev + b * ix->dim, n, ix->dim, ix->centroids.ptr, nlist, ix->dim, l2, true, ws.scores.ptr, nlist));
-            PairsPrepare pp{};
-            pp.dist = ws.scores.ptr;
-            pp.nlist = nlist;
-            pp.nprobe = nprobe;
-            pp.probes = probes_dev + b * nprobe;
-            pp.probe_dists = dists_dev != nullptr ? dists_dev + b * nprobe : nullptr;
-            VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(n), PAIR_THREADS, 0, pp);
+            PairsPrepare part = pp.from(b);
+            part.dist = ws.scores.ptr;
+            part.ld = nlist;
+            VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(n), PAIR_THREADS, 0, part);
         }
         return 0;
     }
-    uint32_t n2 = next_pow2(ncand < 2 ? 2 : ncand);
-    VB_LAUNCH(route_finalize_kernel, static_cast<uint32_t>(nq), 128, n2 * sizeof(uint64_t) + ix->dim * sizeof(float), q_dev,
-              ix->dim, ix->centroids.ptr, ws.cand.ptr, ncand, n2, nprobe, ix->metric, probes_dev,
-              dists_dev);
     return 0;
 }
 
@@ -3296,33 +3252,33 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         pp.count = ws.tile_count.ptr;
         pp.rank = ws.tile_rank.ptr;
     }
-    bool routed_on_tensor_cores = false;
+    bool routed_on_tensor_cores = false, prepared = false;
     if (bucket_ids != nullptr) {
         VB_CUDA(cudaMemcpyAsync(ws.probes.ptr, bucket_ids, nq * nprobe * sizeof(int32_t), cudaMemcpyDefault, st));
-    } else if (tensor_cores_enabled() && nq >= 256 && nlist >= 1024) {
-        VB_TRY(ivf_route_device(ix, q_dev, nq, nprobe, ws.probes.ptr, nullptr));
-        routed_on_tensor_cores = true;
     } else {
-        VB_CHECK_ARG((nprobe + ROUTE_SLACK < nlist ? nprobe + ROUTE_SLACK : nlist) <= 1024,
-                     "scan_buckets_count %u is too large (limit %u)", nprobe, 1024 - ROUTE_SLACK);
-        VB_TRY(ws.scores.reserve(nq * nlist));
-        VB_TRY(launch_row_chains(q_dev, nq, dim, ix->centroids.ptr, nlist, dim, l2, true, ws.scores.ptr, nlist));
-        pp.dist = ws.scores.ptr;
+        VB_TRY(ivf_route_device(ix, q_dev, nq, nprobe, ws.probes.ptr, nullptr, &pp, &prepared));
+        routed_on_tensor_cores = routes_on_tensor_cores(ix, nq);
     }
-    VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, 0, pp);
+    if (!prepared) {
+        VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, 0, pp);
+    }
     const float* q_scan = q_dev;
     if (ix->quant == VB200_QUANT_RABITQ) {
         VB_TRY(ws.qproc.reserve(nq * (dim + 1)));
-        VB_TRY(rabitq_process_query_device(q_dev, nq, dim, ix->rotation.ptr, ix->rq_centroid.ptr, ws.qproc.ptr, &ws.qrot));
         q_scan = ws.qproc.ptr;
+        VB_TRY(ws.qrot.reserve(nq * dim));
+        VB_TRY(launch_row_chains(q_dev, nq, dim, ix->rotation.ptr, dim, dim, false, false, ws.qrot.ptr, dim));
+        const uint32_t qstride = (dim + 15) / 16 * 16;
         if (plan != nullptr) {
-            const uint32_t qstride = (dim + 15) / 16 * 16;
             VB_TRY(ws.qw8.reserve(nq * 3 * qstride));
             VB_TRY(ws.qscale.reserve(nq));
             VB_TRY(ws.qsum.reserve(nq * 4));
-            VB_LAUNCH(rabitq_terms_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, 0, ws.qproc.ptr, dim, qstride,
-                      1.0f / sqrtf(static_cast<float>(dim)), ws.qw8.ptr, ws.qscale.ptr, ws.qsum.ptr);
         }
+        const size_t smem = dim * sizeof(float);
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(rabitq_query_kernel), smem));
+        VB_LAUNCH(rabitq_query_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, smem, ws.qrot.ptr, dim, ix->rq_centroid.ptr, qstride,
+                  1.0f / sqrtf(static_cast<float>(dim)), ws.qproc.ptr, plan != nullptr ? ws.qw8.ptr : static_cast<int8_t*>(nullptr),
+                  ws.qscale.ptr, ws.qsum.ptr);
     }
 
     ScanFinalize f{};

@@ -53,8 +53,11 @@ route_dist_kernel(const float* __restrict__ queries, uint32_t nq, uint64_t q_str
 }
 
 struct PairsPrepare {
-    const float* dist;        // [nq x nlist] exact centroid distances, or null: `probes` is given
-    uint32_t nlist, nprobe;
+    const float* dist;        // [nq x ld] exact centroid distances, or
+    const float* scores;      // [nq x ld] scores that nominate ncand centroids for exact distances; both null: `probes` is given
+    uint64_t ld;
+    uint32_t nlist, nprobe, ncand;
+    const float* centroids;   // [nlist x dim] (with scores)
     int32_t* probes;          // [nq x nprobe] nearest first
     float* probe_dists;       // [nq x nprobe] or null
     const uint32_t* list_off;
@@ -68,6 +71,27 @@ struct PairsPrepare {
     int metric;
     int8_t* qw8;              // [nq][3][dpad]
     float *qscale, *qa;
+    // The same for the queries from q0 on (dist and scores are the caller's to set).
+    PairsPrepare
+    from(uint64_t q0) const {
+        PairsPrepare p = *this;
+        p.probes += q0 * nprobe;
+        p.probe_dists += p.probe_dists != nullptr ? q0 * nprobe : 0;
+        p.queries += q0 * dim;
+        if (p.t.rows != nullptr) {
+            p.t.base += q0 * nprobe;
+            p.t.rows += q0;
+        }
+        if (p.count != nullptr) {
+            p.rank += q0 * nprobe;
+        }
+        if (p.qw8 != nullptr) {
+            p.qw8 += q0 * 3 * dpad;
+            p.qscale += q0;
+            p.qa += q0;
+        }
+        return p;
+    }
 };
 
 __device__ __forceinline__ float
@@ -112,10 +136,29 @@ pairs_prepare_kernel(const PairsPrepare p) {
     __shared__ float part[PAIR_THREADS / 32];
     const uint64_t q = blockIdx.x;
     int32_t* probes = p.probes + q * p.nprobe;
-    if (p.dist != nullptr) {
-        const float* row = p.dist + q * p.nlist;
-        const uint32_t found = block_select<PAIR_THREADS>(load_source([&](uint32_t i) { return float_to_ordered(__ldg(row + i)); }),
-                                                          [](uint32_t i) { return i; }, p.nlist, p.nprobe, keys, sel);
+    if (p.dist != nullptr || p.scores != nullptr) {
+        uint32_t found;
+        if (p.scores != nullptr) {
+            // IVF::route_buckets_only's loop (src/algorithm/ivf/ivf.cpp:1589-1660) over the nominated centroids:
+            // distance ascending, lower list id first on ties
+            extern __shared__ __align__(16) unsigned char smem[];
+            float* qs = reinterpret_cast<float*>(smem);
+            for (uint32_t d = threadIdx.x; d < p.dim; d += PAIR_THREADS) {
+                qs[d] = __ldg(p.queries + q * p.dim + d);
+            }
+            const ScoreSource<> src{reinterpret_cast<const uint32_t*>(p.scores + q * p.ld)};
+            found = block_select<PAIR_THREADS>(src, [](uint32_t i) { return i; }, p.nlist, p.ncand, keys, sel);
+            block_sort_to<PAIR_THREADS>(keys, found, p.ncand, best);
+            found = min(found, p.ncand);
+            for (uint32_t i = threadIdx.x; i < found; i += PAIR_THREADS) {
+                const uint32_t l = static_cast<uint32_t>(best[i]);
+                keys[i] = make_key(row_exact_distance(p.centroids + static_cast<uint64_t>(l) * p.dim, qs, p.dim, p.metric == VB200_METRIC_L2), l);
+            }
+        } else {
+            const float* row = p.dist + q * p.ld;
+            found = block_select<PAIR_THREADS>(load_source([&](uint32_t i) { return float_to_ordered(__ldg(row + i)); }),
+                                               [](uint32_t i) { return i; }, p.nlist, p.nprobe, keys, sel);
+        }
         block_sort_to<PAIR_THREADS>(keys, found, p.nprobe, best);
         for (uint32_t i = threadIdx.x; i < p.nprobe; i += PAIR_THREADS) {
             const bool have = i < found;
@@ -187,34 +230,62 @@ pairs_prepare_kernel(const PairsPrepare p) {
     }
 }
 
-// RaBitQ: the values sv_d = inv_sqrt_d * q_d of the estimator as three int8 terms, their scale and the terms' sums.
+// RaBitQ queries: rotated rows t[nq x dim] -> the processed query (RaBitQuantizer::ProcessQueryImpl,
+// rabitq_quantizer.cpp:2130-2217: centred, divided by the norm of the ascending chain, the norm behind) and, with
+// qw8, the values sv_d = inv_sqrt_d * q_d of the estimator as three int8 terms, their scale and the terms' sums.  The
+// chain is one thread's, over values the whole CTA put into shared memory.
 __global__ void __launch_bounds__(PAIR_THREADS)
-rabitq_terms_kernel(const float* __restrict__ queries, uint32_t dim, uint32_t qstride, float inv_sqrt_d, int8_t* __restrict__ qw8,
-                    float* __restrict__ qscale, int32_t* __restrict__ qsum) {
+rabitq_query_kernel(const float* __restrict__ t, uint32_t dim, const float* __restrict__ centroid, uint32_t qstride, float inv_sqrt_d,
+                    float* __restrict__ out, int8_t* __restrict__ qw8, float* __restrict__ qscale, int32_t* __restrict__ qsum) {
+    extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float part[PAIR_THREADS / 32];
+    __shared__ float s_norm;
     __shared__ int32_t sums[3];
+    float* df = reinterpret_cast<float*>(smem);
     const uint64_t q = blockIdx.x;
-    const float* src = queries + q * (dim + 1);
-    float wmax = 0.f;
+    const float* src = t + q * dim;
     for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
-        wmax = fmaxf(wmax, fabsf(__fmul_rn(inv_sqrt_d, __ldg(src + d))));
+        df[d] = __fsub_rn(__ldg(src + d), __ldg(centroid + d));
     }
     if (threadIdx.x < 3) {
         sums[threadIdx.x] = 0;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float s = 0.f;
+#pragma unroll 16
+        for (uint32_t d = 0; d < dim; ++d) {
+            s = fmaf(df[d], df[d], s);
+        }
+        s_norm = s < 1e-5f ? 1.0f : __fsqrt_rn(s);
+        out[q * (dim + 1) + dim] = s_norm;
+    }
+    __syncthreads();
+    const float norm = s_norm;
+    float wmax = 0.f;
+    for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
+        const float v = __fdiv_rn(df[d], norm);
+        out[q * (dim + 1) + d] = v;
+        const float w = __fmul_rn(inv_sqrt_d, v);
+        df[d] = w;   // (this thread's own element)
+        wmax = fmaxf(wmax, fabsf(w));
+    }
+    if (qw8 == nullptr) {
+        return;
+    }
     wmax = pair_block_max(wmax, part);
     const float s = wmax > 0.f && wmax < INFINITY ? wmax / 127.0f : 1.0f;
-    int8_t* t = qw8 + q * 3 * qstride;
+    int8_t* terms = qw8 + q * 3 * qstride;
     int32_t n1 = 0, n2 = 0, n3 = 0;
     for (uint32_t d = threadIdx.x; d < qstride; d += PAIR_THREADS) {
-        const float u = d < dim ? __fmul_rn(inv_sqrt_d, __ldg(src + d)) / s : 0.f;
+        const float u = d < dim ? df[d] / s : 0.f;
         const float t1 = fminf(fmaxf(rintf(u), -127.f), 127.f);
         const float v2 = (u - t1) * 254.0f;
         const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
         const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
-        t[d] = static_cast<int8_t>(static_cast<int>(t1));
-        t[qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
-        t[2 * qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
+        terms[d] = static_cast<int8_t>(static_cast<int>(t1));
+        terms[qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
+        terms[2 * qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
         n1 += static_cast<int>(t1);
         n2 += static_cast<int>(t2);
         n3 += static_cast<int>(t3);
