@@ -85,6 +85,13 @@ int allow_dynamic_smem(const void* kernel, size_t bytes);
 // ---------------------------------------------------------------------------------------------
 // device memory
 // ---------------------------------------------------------------------------------------------
+// Device memory comes from a pool of the library (dense.cu): freeing a buffer costs no device-wide synchronisation and
+// the next one of its size no trip to the driver.  Both are ordered with the calling thread's current stream: a call
+// uses one stream and has completed when it returns, so a buffer is never still in use on another.
+cudaError_t pool_malloc(void** p, size_t bytes);
+void pool_free(void* p);
+void pool_trim();
+
 template <typename T>
 struct DevBuf {
     T* ptr = nullptr;
@@ -111,7 +118,7 @@ struct DevBuf {
     }
     void release() {
         if (ptr != nullptr) {
-            cudaFree(ptr);
+            pool_free(ptr);
         }
         ptr = nullptr;
         cap = 0;
@@ -126,10 +133,10 @@ struct DevBuf {
             return 0;
         }
         void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+        cudaError_t e = pool_malloc(&p, n * sizeof(T));
         if (e != cudaSuccess) {
             cudaGetLastError();
-            VB_FAIL(VB200_NO_ENOUGH_MEMORY, "cudaMalloc of %zu bytes failed: %s", n * sizeof(T),
+            VB_FAIL(VB200_NO_ENOUGH_MEMORY, "allocation of %zu bytes of device memory failed: %s", n * sizeof(T),
                     cudaGetErrorString(e));
         }
         ptr = static_cast<T*>(p);
@@ -209,6 +216,12 @@ copy_out(T* dst, const T* src_dev, size_t n) {
     VB_CUDA(cudaMemcpyAsync(dst, src_dev, n * sizeof(T), kind, current_stream()));
     return 0;
 }
+
+// copy_out to pageable host memory: large copies go through pinned memory in pieces, several threads filling the
+// caller's pages while the next piece crosses the bus (dense.cu).  Completes before it returns.
+int copy_to_host(void* dst, const void* src_dev, size_t bytes);
+// The same for `rows` rows of `width` bytes that lie `pitch` bytes apart on the device.
+int copy_rows_to_host(void* dst, const void* src_dev, size_t width, size_t pitch, uint64_t rows);
 
 inline int
 sync_stream() {

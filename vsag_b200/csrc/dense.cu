@@ -3,6 +3,9 @@
 #include "dense.cuh"
 
 #include <map>
+#include <set>
+#include <system_error>
+#include <thread>
 #include <utility>
 
 namespace vb200 {
@@ -70,6 +73,166 @@ allow_dynamic_smem(const void* kernel, size_t bytes) {
         have = bytes;
     }
     return 0;
+}
+
+// ---------------------------------------------------------------------------------------------
+// device memory pool
+// ---------------------------------------------------------------------------------------------
+constexpr uint64_t POOL_KEEP_BYTES = uint64_t{2} << 30;   // freed memory a device's pool holds on to, at most
+
+// The current device's pool, made at its first use; nullptr when the device has none (plain allocations then).
+static cudaMemPool_t
+device_pool() {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    static bool tried[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    if (!tried[dev]) {
+        tried[dev] = true;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        uint64_t keep = POOL_KEEP_BYTES;
+        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
+            pools[dev] = pool;
+        } else {
+            cudaGetLastError();
+        }
+    }
+    return pools[dev];
+}
+
+// Buffers the pool could not serve (rare): they go back the plain way.
+static std::mutex g_plain_mu;
+static std::set<void*> g_plain;
+
+cudaError_t
+pool_malloc(void** p, size_t bytes) {
+    cudaMemPool_t pool = device_pool();
+    if (pool != nullptr) {
+        const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, current_stream());
+        if (e == cudaSuccess) {
+            return e;
+        }
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);   // what is left may still do as one plain allocation
+    }
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_plain_mu);
+        g_plain.insert(*p);
+    }
+    return e;
+}
+
+void
+pool_free(void* p) {
+    {
+        std::lock_guard<std::mutex> lock(g_plain_mu);
+        if (!g_plain.empty() && g_plain.erase(p) > 0) {
+            cudaFree(p);
+            return;
+        }
+    }
+    if (cudaFreeAsync(p, current_stream()) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(p);
+    }
+}
+
+void
+pool_trim() {
+    cudaMemPool_t pool = device_pool();
+    if (pool != nullptr) {
+        cudaMemPoolTrimTo(pool, 0);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// large copies to pageable memory
+// ---------------------------------------------------------------------------------------------
+constexpr size_t HOST_PIECE = size_t{4} << 20;
+constexpr unsigned HOST_COPY_THREADS = 4;
+
+int
+copy_rows_to_host(void* dst, const void* src_dev, size_t width, size_t pitch, uint64_t rows) {
+    const size_t bytes = width * rows;
+    cudaPointerAttributes attr{};
+    const bool pageable = cudaPointerGetAttributes(&attr, dst) != cudaSuccess || attr.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    cudaStream_t st = current_stream();
+    static std::mutex mu;
+    std::unique_lock<std::mutex> lock(mu, std::defer_lock);
+    static PinnedBuf* pieces = nullptr;   // two pieces, kept for the life of the process (8 MiB)
+    if (!pageable || bytes < HOST_PIECE || width > HOST_PIECE || !lock.try_lock()) {
+        VB_CUDA(cudaMemcpy2DAsync(dst, width, src_dev, pitch, width, rows, cudaMemcpyDefault, st));
+        return sync_stream();
+    }
+    if (pieces == nullptr) {
+        pieces = new (std::nothrow) PinnedBuf;
+    }
+    if (pieces == nullptr || pieces->reserve(2 * HOST_PIECE) != 0) {
+        VB_CUDA(cudaMemcpy2DAsync(dst, width, src_dev, pitch, width, rows, cudaMemcpyDefault, st));
+        return sync_stream();
+    }
+    unsigned char* pin = static_cast<unsigned char*>(pieces->ptr);
+    const uint64_t per = HOST_PIECE / width;
+    auto request = [&](uint64_t r0, int half) -> int {
+        const uint64_t m = rows - r0 < per ? rows - r0 : per;
+        const unsigned char* from = static_cast<const unsigned char*>(src_dev) + r0 * pitch;
+        if (width == pitch) {
+            VB_CUDA(cudaMemcpyAsync(pin + half * HOST_PIECE, from, m * width, cudaMemcpyDeviceToHost, st));
+        } else {
+            VB_CUDA(cudaMemcpy2DAsync(pin + half * HOST_PIECE, width, from, pitch, width, m, cudaMemcpyDeviceToHost, st));
+        }
+        return 0;
+    };
+    VB_TRY(request(0, 0));
+    int half = 0;
+    for (uint64_t r0 = 0; r0 < rows; r0 += per, half ^= 1) {
+        VB_TRY(sync_stream());
+        if (r0 + per < rows) {
+            VB_TRY(request(r0 + per, half ^ 1));
+        }
+        // the caller's pages are often touched here for the first time: several threads share the faults
+        const size_t m = (rows - r0 < per ? rows - r0 : per) * width;
+        unsigned char* to = static_cast<unsigned char*>(dst) + r0 * width;
+        const unsigned char* from = pin + half * HOST_PIECE;
+        std::thread helpers[HOST_COPY_THREADS - 1];
+        const size_t part = (m + HOST_COPY_THREADS - 1) / HOST_COPY_THREADS;
+        unsigned started = 0;
+        size_t at = part < m ? part : m;
+        try {
+            for (; started < HOST_COPY_THREADS - 1 && at < m; ++started) {
+                const size_t len = m - at < part ? m - at : part;
+                helpers[started] = std::thread([=] { std::memcpy(to + at, from + at, len); });
+                at += len;
+            }
+        } catch (const std::system_error&) {   // no more threads: the rest is copied here
+        }
+        std::memcpy(to, from, part < m ? part : m);
+        if (at < m) {
+            std::memcpy(to + at, from + at, m - at);
+        }
+        for (unsigned i = 0; i < started; ++i) {
+            helpers[i].join();
+        }
+    }
+    return 0;
+}
+
+int
+copy_to_host(void* dst, const void* src_dev, size_t bytes) {
+    const size_t width = bytes % 16 == 0 && bytes > 0 ? 16 : 1;
+    return copy_rows_to_host(dst, src_dev, width, width, bytes / width);
 }
 
 bool

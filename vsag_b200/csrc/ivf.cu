@@ -106,7 +106,8 @@ struct SearchWorkspace {
     DevBuf<float> pair_scores;
     PinnedBuf pinned;
     // the same as tensor-core tiles (ivf_tiles.cuh): pairs grouped by list
-    DevBuf<uint32_t> tile_count, tile_rank, tile_tables, tile_pairs;
+    DevBuf<uint32_t> tile_count, tile_rank, tile_tables, tile_pairs, pair_minima;
+    DevBuf<uint32_t> rerank_ids, rerank_done;
     DevBuf<TileItem> tile_items;
     DevBuf<int32_t> qsum;
 };
@@ -3054,31 +3055,30 @@ constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which
 enum ScoreScan { SCAN_GROUPED = 0, SCAN_PAIRS = 1, SCAN_TILES = 2 };
 
 struct TilePlan {
-    uint32_t qt, pieces, stages, b_bufs, per_sm;
+    uint32_t qt, pieces, stages, b_bufs;
     size_t smem;
 };
 
-// Shared memory of a tile launch: the B operand of an item (two when they fit) and 2 .. 6 pieces of rows, two CTAs
-// per SM when that leaves room for them.  False when not even one CTA fits.
+// Shared memory of a tile launch (one CTA per SM): the B operand of an item, two when they fit, and 3 .. 6 pieces of
+// rows.  The more queries an item holds the less often a list is read again: as many as the average list has, since
+// empty columns cost little.  False when nothing fits.
 static bool
 tile_plan(const vb200_ivf* ix, double pairs_per_list, TilePlan* plan) {
     const bool int8 = ix->quant == VB200_QUANT_SQ8 || ix->quant == VB200_QUANT_RABITQ, f32 = ix->quant == VB200_QUANT_FP32;
     plan->pieces = (ix->dim + (int8 ? 127 : 63)) / (int8 ? 128 : 64);
     const size_t stage = (f32 ? 2 : 1) * TILE_A_TERM;
     const uint32_t b_terms = int8 ? 3 : (f32 ? 2 : 1);
-    for (uint32_t per_sm = 2; per_sm >= 1; --per_sm) {
-        const size_t room = per_sm == 2 ? 108 * 1024 : 218 * 1024;
-        for (uint32_t qt = pairs_per_list > 14.0 ? 32 : 16; qt >= 16; qt /= 2) {
-            const size_t b = static_cast<size_t>(plan->pieces) * b_terms * qt * TILE_PIECE;
-            for (uint32_t bufs = 2; bufs >= 1; --bufs) {
-                if (bufs * b + (per_sm == 2 ? 2 : 3) * stage <= room) {
-                    plan->qt = qt;
-                    plan->b_bufs = bufs;
-                    plan->per_sm = per_sm;
-                    plan->stages = static_cast<uint32_t>(std::min<size_t>((room - bufs * b) / stage, TILE_MAX_STAGES));
-                    plan->smem = bufs * b + plan->stages * stage + 1024;   // (room to start on a 1 KiB boundary)
-                    return true;
-                }
+    const size_t room = 208 * 1024;   // of 227 KiB: static shared memory and the step to a 1 KiB boundary
+    uint32_t qt = pairs_per_list > 28.0 ? 64 : (pairs_per_list > 14.0 ? 32 : 16);
+    for (; qt >= 16; qt /= 2) {
+        const size_t b = static_cast<size_t>(plan->pieces) * b_terms * qt * TILE_PIECE;
+        for (uint32_t bufs = 2; bufs >= 1; --bufs) {
+            if (bufs * b + 3 * stage <= room) {
+                plan->qt = qt;
+                plan->b_bufs = bufs;
+                plan->stages = static_cast<uint32_t>(std::min<size_t>((room - bufs * b) / stage, TILE_MAX_STAGES));
+                plan->smem = bufs * b + plan->stages * stage + 1024;
+                return true;
             }
         }
     }
@@ -3121,7 +3121,9 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     SearchWorkspace& ws = ix->ws;
     const uint32_t nlist = ix->nlist, nprobe = sc.nprobe;
     const uint64_t pairs = nq * nprobe;
-    const uint64_t max_items = pairs / plan.qt + std::min<uint64_t>(pairs, nlist);
+    // sum over lists of ceil(pairs / qt) * ceil(rows / segment), from above
+    const uint64_t max_items = nq * sc.t.stride / (static_cast<uint64_t>(plan.qt) * TILE_SEGMENT) + pairs / plan.qt +
+                               ix->n_stored / TILE_SEGMENT + std::min<uint64_t>(pairs, nlist) + 1;
     VB_TRY(ws.tile_tables.reserve(3 * static_cast<size_t>(nlist) + 1));
     VB_TRY(ws.tile_pairs.reserve(pairs));
     VB_TRY(ws.tile_items.reserve(max_items));
@@ -3133,6 +3135,7 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     g.nlist = nlist;
     g.qt = plan.qt;
     g.order = ix->scan_order.ptr;
+    g.list_off = ix->list_off.ptr;
     g.pair_off = ws.tile_tables.ptr;
     g.item_off = ws.tile_tables.ptr + nlist;
     g.list_pairs = ws.tile_tables.ptr + 2 * static_cast<size_t>(nlist);
@@ -3160,7 +3163,8 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     t.spin_limit = tc_spin_limit();
     t.error_flag = reinterpret_cast<int*>(ws.scalars.ptr + 4);
     void (*kernel)(const TileScan) = nullptr;
-#define VB_TILE(FMT) kernel = plan.qt == 32 ? tile_scan_kernel<FMT, 32> : tile_scan_kernel<FMT, 16>
+#define VB_TILE(FMT) \
+    kernel = plan.qt == 64 ? tile_scan_kernel<FMT, 64> : (plan.qt == 32 ? tile_scan_kernel<FMT, 32> : tile_scan_kernel<FMT, 16>)
     switch (ix->quant) {
         case VB200_QUANT_SQ8: VB_TILE(ROW_SQ8); break;
         case VB200_QUANT_FP32: VB_TILE(ROW_F32); break;
@@ -3170,7 +3174,7 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     }
 #undef VB_TILE
     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), plan.smem));
-    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(max_items, static_cast<uint64_t>(sm_count()) * plan.per_sm));
+    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(max_items, static_cast<uint64_t>(sm_count())));
     VB_LAUNCH(kernel, grid, TILE_THREADS, plan.smem, t);
     return 0;
 }
@@ -3216,7 +3220,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     VB_TRY(ws.query_rows.reserve(nq));
     // a query's stretch of the score buffer holds its probed lists whichever they are; batches whose stretches
     // together pass a gigabyte go in slices
-    const uint64_t stride = (ix->longest_rows[nprobe] + 31) / 32 * 32;
+    const uint64_t stride = (ix->longest_rows[nprobe] + (plan != nullptr ? 31ull * nprobe : 0) + 31) / 32 * 32;
     VB_CHECK_ARG(stride < 0xFFFFFFFFull, "the probed lists hold too many rows");
     uint64_t slice = (uint64_t{256} << 20) / (stride > 0 ? stride : 1);
     slice = slice < 1 ? 1 : (slice > nq || plan != nullptr ? nq : slice);
@@ -3231,7 +3235,10 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     pp.nprobe = nprobe;
     pp.list_off = ix->list_off.ptr;
     pp.probes = ws.probes.ptr;
-    pp.t = PairTable{ws.pair_base.ptr, ws.query_rows.ptr, stride, ws.pair_scores.ptr};
+    if (plan != nullptr) {
+        VB_TRY(ws.pair_minima.reserve(nq * stride / 32));
+    }
+    pp.t = PairTable{ws.pair_base.ptr, ws.query_rows.ptr, stride, ws.pair_scores.ptr, plan != nullptr ? ws.pair_minima.ptr : nullptr};
     if (sq8) {
         pp.queries = q_dev;
         pp.dim = dim;
@@ -3317,7 +3324,15 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     f.diff = ix->diff.ptr;
     f.pos_inner = ix->pos_inner.ptr;
     f.labels = ix->labels.ptr;
-    f.flat = rerank ? ix->flat.ptr : nullptr;
+    if (rerank) {
+        VB_TRY(ws.rerank_ids.reserve(nq * kscan));
+        VB_TRY(ws.keys.reserve(nq * kscan));
+        if (ws.rerank_done.cap < nq) {
+            VB_TRY(ws.rerank_done.reserve(nq));
+            VB_CUDA(cudaMemsetAsync(ws.rerank_done.ptr, 0, ws.rerank_done.cap * sizeof(uint32_t), st));   // rerank_rows_kernel leaves it cleared
+        }
+        f.rerank_ids = ws.rerank_ids.ptr;
+    }
     f.rows_scanned = reinterpret_cast<uint32_t*>(pin + rows_at);
     if (!pin_out) {
         VB_TRY(ws.out_ids.reserve(total));
@@ -3327,7 +3342,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     float* dists_dev = !host_d ? dists : (pin_out ? reinterpret_cast<float*>(pin + dists_at) : ws.out_dists.ptr);
 
     const size_t scan_smem = RS_STAGES * RS_STAGE + (sq8 ? 3 * static_cast<size_t>(ix->dpad) : f.scan.qstride * sizeof(float));
-    const size_t final_smem = (2 * static_cast<size_t>(nprobe) + 4 + (sq8 || rerank ? (dim + 3) / 4 * 4 : 0) +
+    const size_t final_smem = (2 * static_cast<size_t>(nprobe) + 4 + (sq8 ? (dim + 3) / 4 * 4 : 0) +
                                (sq8 ? 2 * dim : (plan != nullptr ? f.scan.qstride : 0))) * sizeof(float);
     VB_CHECK_ARG(scan_smem <= 220 * 1024 && final_smem <= 180 * 1024, "dim = %u is too large for the scan", dim);
     void (*scan_kernel)(const PairScan) = nullptr;
@@ -3372,6 +3387,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
             g.scan.qw8 += q0 * 3 * ix->dpad;
         }
         g.rows_scanned += q0;
+        g.rerank_ids += rerank ? q0 * kscan : 0;
         g.ids = ids_dev + q0 * k;
         g.dists = dists_dev + q0 * k;
         if (q0 == 0) {
@@ -3389,6 +3405,25 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
             ix->scan_timed = true;
         }
         VB_LAUNCH(final_kernel, static_cast<uint32_t>(n), PAIR_THREADS, final_smem, g);
+    }
+    if (rerank) {
+        Rerank r{};
+        r.queries = q_dev;
+        r.flat = ix->flat.ptr;
+        r.dim = dim;
+        r.ncand = kscan;
+        r.k = k;
+        r.ids = ws.rerank_ids.ptr;
+        r.keys = ws.keys.ptr;
+        r.done = ws.rerank_done.ptr;
+        r.labels = ix->labels.ptr;
+        r.out_ids = ids_dev;
+        r.out_dists = dists_dev;
+        auto kernel = l2 ? rerank_rows_kernel<true> : rerank_rows_kernel<false>;
+        const size_t smem = dim * sizeof(float);
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 24 * 1024 ? 20 * 1024 : 0)));
+        VB_CHECK_ARG(nq * RERANK_PARTS <= 0x7fffffffull, "query batch too large");
+        VB_LAUNCH(kernel, static_cast<uint32_t>(nq * RERANK_PARTS), PAIR_THREADS, smem, r);
     }
     ws.pruning = false;
     if (!pin_out) {
@@ -4224,6 +4259,14 @@ vb200_ivf_get_rows(vb200_ivf_t ix, float* rows) {
     return sync_stream();
 }
 
+__global__ void
+widen_ids_kernel(const uint32_t* __restrict__ in, uint64_t n, int64_t* __restrict__ out) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) {
+        out[i] = in[i];
+    }
+}
+
 extern "C" int
 vb200_ivf_get_lists(vb200_ivf_t ix, int64_t* list_sizes, uint8_t* codes, int64_t* inner_ids) {
     VB_CHECK_ARG(ix != nullptr, "null index");
@@ -4238,16 +4281,13 @@ vb200_ivf_get_lists(vb200_ivf_t ix, int64_t* list_sizes, uint8_t* codes, int64_t
     }
     if (codes != nullptr) {
         VB_CHECK_ARG(!is_device_pointer(codes), "get_lists writes host memory");
-        VB_CUDA(cudaMemcpy2D(codes, ix->code_size, ix->codes.ptr, ix->code_stride, ix->code_size,
-                             ix->n_stored, cudaMemcpyDeviceToHost));
+        VB_TRY(copy_rows_to_host(codes, ix->codes.ptr, ix->code_size, ix->code_stride, ix->n_stored));
     }
     if (inner_ids != nullptr) {
-        std::vector<uint32_t> tmp(ix->n_stored);
-        VB_CUDA(cudaMemcpy(tmp.data(), ix->pos_inner.ptr, ix->n_stored * sizeof(uint32_t),
-                           cudaMemcpyDeviceToHost));
-        for (uint64_t i = 0; i < ix->n_stored; ++i) {
-            inner_ids[i] = tmp[i];
-        }
+        DevBuf<int64_t> wide;
+        VB_TRY(wide.reserve(ix->n_stored));
+        VB_LAUNCH(widen_ids_kernel, static_cast<uint32_t>((ix->n_stored + 255) / 256), 256, 0, ix->pos_inner.ptr, ix->n_stored, wide.ptr);
+        VB_TRY(copy_to_host(inner_ids, wide.ptr, ix->n_stored * sizeof(int64_t)));
     }
     return 0;
 }

@@ -21,6 +21,9 @@ struct PairTable {
     uint32_t* rows;    // [nq] scores of each query
     uint64_t stride;   // scores between the stretches of neighbouring queries
     float* scores;
+    // Tiles: every pair starts on a multiple of 32 scores (rows past a list's end count as filtered) and the smallest
+    // of each 32 stands, as an ordered value, in minima[query * stride / 32 + place / 32].  null: pairs back to back.
+    uint32_t* minima;
 };
 
 // out[(q, r)] for every row r of `rows` and query q: L2 = sum of fma(t, t, .), t = row - query; otherwise the
@@ -172,6 +175,7 @@ pairs_prepare_kernel(const PairsPrepare p) {
     if (p.t.rows == nullptr) {
         return;   // only the routing is wanted
     }
+    const uint32_t round = p.t.minima != nullptr ? 31u : 0u;
     uint32_t run = 0;
     for (uint32_t i0 = 0; i0 < p.nprobe; i0 += PAIR_THREADS) {
         const uint32_t i = i0 + threadIdx.x;
@@ -184,6 +188,7 @@ pairs_prepare_kernel(const PairsPrepare p) {
             if (p.count != nullptr) {
                 p.rank[q * p.nprobe + i] = len > 0 ? atomicAdd(p.count + l, 1u) : 0xFFFFFFFFu;
             }
+            len = (len + round) & ~round;
         }
         const uint32_t incl = block_inclusive_sum<PAIR_THREADS>(len, sel.warp_part);
         if (i < p.nprobe) {
@@ -470,7 +475,7 @@ struct ScanFinalize {
     const float* queries;      // [nq x dim] plain queries (SQ8 re-scoring, rerank)
     const uint32_t* pos_inner;
     const int64_t* labels;
-    const float* flat;         // rerank: fp32 rows by inner id, or null
+    uint32_t* rerank_ids;      // [nq x kscan] rerank: the candidates go here instead of to the results, or null
     uint32_t* rows_scanned;    // [nq] rows of each query's lists (pinned host memory)
     int64_t* ids;
     float* dists;
@@ -530,6 +535,18 @@ struct ScorePosition {
     }
 };
 
+constexpr uint32_t FINAL_GROUPS = 1024;   // groups of 32 scores looked into at most
+
+// Place number i of the scores in the listed groups -> the row's position.
+struct GroupPosition {
+    const uint32_t* ids;
+    ScorePosition position;
+    __device__ __forceinline__ uint32_t
+    operator()(uint32_t i) const {
+        return position(ids[i >> 5] * 32 + (i & 31u));
+    }
+};
+
 // Exact distance of one code record in the reference's operation order; qc: the query as the codec's chain reads it
 // (stage_query), zero padded.  Four 16-byte loads in flight.
 template <int FMT, bool L2>
@@ -564,7 +581,7 @@ record_exact_distance(const uint8_t* rec, uint32_t dim, uint32_t row_bytes, cons
     }
 }
 
-// Dynamic shared memory: [2][nprobe] pair places and list starts; [rerank or SQ8] the plain query; [SQ8] lower and
+// Dynamic shared memory: [2][nprobe] pair places and list starts; [SQ8] the plain query, lower and
 // diff, or [other codecs re-scored after tiles] the query as the codec reads it (qstride floats).
 // APPROX: the scores only rank (SQ8's integer form, tensor-core tiles).  The kcand best by score are re-scored
 // exactly; a row that was not among them has an exact distance of at least (the last kept score - margin), margin
@@ -578,13 +595,14 @@ scan_finalize_kernel(const ScanFinalize p) {
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
+    __shared__ uint32_t group_ids[APPROX ? FINAL_GROUPS : 1];
     __shared__ float part[PAIR_THREADS / 32];
     const PairScan& sc = p.scan;
     const uint64_t q = blockIdx.x;
     const uint32_t nprobe = sc.nprobe, dim = sc.s.dim;
     uint32_t* base_s = reinterpret_cast<uint32_t*>(smem);
     uint32_t* start_s = base_s + sc.nprobe;
-    const bool plain = FMT == ROW_SQ8 || p.flat != nullptr;
+    const bool plain = FMT == ROW_SQ8;
     float* qs = reinterpret_cast<float*>(smem + (2 * nprobe * sizeof(uint32_t) + 15) / 16 * 16);
     float* qc = qs + (plain ? (dim + 3) / 4 * 4 : 0u);     // SQ8: lower, then diff
     const uint32_t n = sc.t.rows[q];
@@ -618,9 +636,57 @@ scan_finalize_kernel(const ScanFinalize p) {
             return record_exact_distance<FMT, L2>(rec, dim, sc.row_bytes, qc, qn);
         }
     };
-    uint32_t found = block_select<PAIR_THREADS>(ScoreSource<>{scores}, position, n, p.kcand, keys, sel);
-    if (threadIdx.x == 0) {
-        p.rows_scanned[q] = n;
+    uint32_t found = 0;
+    bool selected = false;
+    if (APPROX && sc.t.minima != nullptr) {
+        // First the groups of 32 scores that can hold one of the kcand best: those whose smallest is not above the
+        // kcand-th smallest minimum.  Then the scores of those groups alone.
+        const uint32_t* minima = sc.t.minima + q * (sc.t.stride / 32);
+        const uint32_t groups = n / 32;
+        uint32_t upto;
+        const uint32_t bound = block_bound<PAIR_THREADS>(load_source([&](uint32_t i) { return __ldg(minima + i); }), groups, p.kcand,
+                                                         p.kcand + p.kcand / 8 + 8, sel, &upto);
+        if (upto <= FINAL_GROUPS) {
+            if (threadIdx.x == 0) {
+                sel.count = 0;
+            }
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < groups; i += PAIR_THREADS) {
+                if (__ldg(minima + i) <= bound) {
+                    group_ids[atomicAdd(&sel.count, 1u)] = i;
+                }
+            }
+            __syncthreads();
+            const uint32_t m = sel.count;
+            __syncthreads();
+            const auto at = [&](uint32_t i) -> uint32_t { return group_ids[i >> 5] * 32 + (i & 31u); };
+            const GroupPosition where{group_ids, position};
+            found = block_select<PAIR_THREADS>(load_source([&](uint32_t i) { return ScoreSource<>::ordered(__ldg(scores + at(i))); }), where,
+                                               m * 32, p.kcand, keys, sel);
+            selected = true;
+        }
+    }
+    if (!selected) {
+        found = block_select<PAIR_THREADS>(ScoreSource<>{scores}, position, n, p.kcand, keys, sel);
+    }
+    if (p.rows_scanned != nullptr) {
+        uint32_t rows = 0;
+        for (uint32_t i = threadIdx.x; i < nprobe; i += PAIR_THREADS) {
+            const int32_t l = __ldg(sc.probes + q * nprobe + i);
+            rows += l >= 0 && static_cast<uint32_t>(l) < sc.s.nlist ? __ldg(sc.s.list_off + l + 1) - __ldg(sc.s.list_off + l) : 0u;
+        }
+        if (threadIdx.x == 0) {
+            sel.total = 0;
+        }
+        __syncthreads();
+        rows = __reduce_add_sync(0xffffffffu, rows);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&sel.total, rows);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            p.rows_scanned[q] = sel.total;
+        }
     }
     if (APPROX) {
         block_sort_to<PAIR_THREADS>(keys, found, p.kcand, best);
@@ -685,24 +751,71 @@ scan_finalize_kernel(const ScanFinalize p) {
         block_sort_to<PAIR_THREADS>(keys, found, p.kscan, best);
     }
     uint32_t have = min(found, p.kscan);
-    const uint64_t* final_keys = best;
-    if (p.flat != nullptr) {
-        // FlattenReorder::Reorder (rerank_kernel): a warp per candidate, the fp32 row by inner id
-        const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        for (uint32_t c = warp; c < have; c += PAIR_THREADS / 32) {
-            const uint32_t inner = __ldg(p.pos_inner + static_cast<uint32_t>(best[c]));
-            const float* x = p.flat + static_cast<uint64_t>(inner) * dim;
+    if (p.rerank_ids != nullptr) {
+        // the candidates of the rerank, by inner id; 0xFFFFFFFF = none
+        for (uint32_t i = threadIdx.x; i < p.kscan; i += PAIR_THREADS) {
+            p.rerank_ids[q * p.kscan + i] = i < have ? __ldg(p.pos_inner + static_cast<uint32_t>(best[i])) : 0xFFFFFFFFu;
+        }
+        return;
+    }
+    for (uint32_t i = threadIdx.x; i < p.k; i += PAIR_THREADS) {
+        const bool there = i < have;
+        const uint64_t key = there ? best[i] : KEY_INF;
+        const uint32_t inner = there ? __ldg(p.pos_inner + static_cast<uint32_t>(key)) : 0u;
+        p.ids[q * p.k + i] = there ? __ldg(p.labels + inner) : -1;
+        p.dists[q * p.k + i] = there ? ordered_to_float(static_cast<uint32_t>(key >> 32)) : INFINITY;
+    }
+}
+
+// FlattenReorder::Reorder (src/impl/reorder/flatten_reorder.cpp:76-118): the fp32 distance of every candidate, a warp
+// per candidate (lanes stride the dimensions, partial sums meet in a tree), then the k best as results.  The bound is
+// reading the candidates' rows from memory, so a query's candidates are spread over RERANK_PARTS CTAs with a whole
+// row (1024 dimensions) requested at once per warp; the CTA that finishes a query last orders its distances.
+constexpr uint32_t RERANK_PARTS = 4;
+
+struct Rerank {
+    const float* queries;
+    const float* flat;         // [n x dim] rows by inner id
+    uint32_t dim, ncand, k;
+    const uint32_t* ids;       // [nq x ncand] inner ids, 0xFFFFFFFF = none
+    uint64_t* keys;            // [nq x ncand]
+    uint32_t* done;            // [nq] zero before and after
+    const int64_t* labels;
+    int64_t* out_ids;
+    float* out_dists;
+};
+
+template <bool L2>
+__global__ void __launch_bounds__(PAIR_THREADS)
+rerank_rows_kernel(const Rerank p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(16) uint64_t keys[1024];
+    __shared__ __align__(16) uint64_t best[1024];
+    __shared__ uint32_t last;
+    float* qs = reinterpret_cast<float*>(smem);
+    const uint64_t q = blockIdx.x / RERANK_PARTS;
+    const uint32_t part = blockIdx.x % RERANK_PARTS;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (uint32_t d = threadIdx.x; d < p.dim; d += PAIR_THREADS) {
+        qs[d] = __ldg(p.queries + q * p.dim + d);
+    }
+    __syncthreads();
+    for (uint32_t c = part * (PAIR_THREADS / 32) + warp; c < p.ncand; c += RERANK_PARTS * (PAIR_THREADS / 32)) {
+        const uint32_t inner = __ldg(p.ids + q * p.ncand + c);
+        uint64_t key = KEY_INF;
+        if (inner != 0xFFFFFFFFu) {
+            const float* x = p.flat + static_cast<uint64_t>(inner) * p.dim;
             float s = 0.f;
-            for (uint32_t d0 = lane; d0 < dim; d0 += 256) {
-                float v[8];
+            for (uint32_t d0 = lane; d0 < p.dim; d0 += 1024) {
+                float v[32];
 #pragma unroll
-                for (uint32_t u = 0; u < 8; ++u) {
-                    v[u] = d0 + u * 32 < dim ? __ldg(x + d0 + u * 32) : 0.f;
+                for (uint32_t u = 0; u < 32; ++u) {
+                    v[u] = d0 + u * 32 < p.dim ? __ldg(x + d0 + u * 32) : 0.f;
                 }
 #pragma unroll
-                for (uint32_t u = 0; u < 8; ++u) {
+                for (uint32_t u = 0; u < 32; ++u) {
                     const uint32_t d = d0 + u * 32;
-                    if (d < dim) {
+                    if (d < p.dim) {
                         if (L2) {
                             const float t = qs[d] - v[u];
                             s = fmaf(t, t, s);
@@ -715,19 +828,43 @@ scan_finalize_kernel(const ScanFinalize p) {
             for (int o = 16; o > 0; o >>= 1) {
                 s += __shfl_xor_sync(0xffffffffu, s, o);
             }
-            if (lane == 0) {
-                keys[c] = make_key(L2 ? s : 1.0f - s, inner);
-            }
+            key = make_key(L2 ? s : 1.0f - s, inner);
         }
-        block_sort_to<PAIR_THREADS>(keys, have, p.k, best);
+        if (lane == 0) {
+            p.keys[q * p.ncand + c] = key;
+        }
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(p.done + q, 1u) == RERANK_PARTS - 1 ? 1u : 0u;
+    }
+    __syncthreads();
+    if (last == 0) {
+        return;
+    }
+    if (threadIdx.x == 0) {
+        p.done[q] = 0;
+    }
+    __threadfence();
+    __shared__ uint32_t have;
+    if (threadIdx.x == 0) {
+        have = 0;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < p.ncand; i += PAIR_THREADS) {
+        const uint64_t key = *reinterpret_cast<const volatile uint64_t*>(p.keys + q * p.ncand + i);
+        if (key != KEY_INF) {
+            keys[atomicAdd(&have, 1u)] = key;
+        }
+    }
+    __syncthreads();
+    const uint32_t n = have;
+    block_sort_to<PAIR_THREADS>(keys, n, p.k, best);
     for (uint32_t i = threadIdx.x; i < p.k; i += PAIR_THREADS) {
-        const bool there = i < have;
-        const uint64_t key = there ? final_keys[i] : KEY_INF;
-        const uint32_t id = static_cast<uint32_t>(key);
-        const uint32_t inner = there ? (p.flat != nullptr ? id : __ldg(p.pos_inner + id)) : 0u;
-        p.ids[q * p.k + i] = there ? __ldg(p.labels + inner) : -1;
-        p.dists[q * p.k + i] = there ? ordered_to_float(static_cast<uint32_t>(key >> 32)) : INFINITY;
+        const bool there = i < n;
+        p.out_ids[q * p.k + i] = there ? __ldg(p.labels + static_cast<uint32_t>(best[i])) : -1;
+        p.out_dists[q * p.k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
     }
 }
 

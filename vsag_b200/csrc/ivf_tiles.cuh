@@ -1,6 +1,6 @@
 // List scan of a batch as tensor-core tiles that write scores.
 //
-// A work item is one inverted list against up to 32 (or 16) of the queries that probe it: the rows are read once
+// A work item is one inverted list against up to 64 (32, 16) of the queries that probe it: the rows are read once
 // for all of them, 128 at a time, and a tile [128 rows x queries] of inner products comes out of tcgen05.mma.  The
 // epilogue turns each into a ranking score and stores it where the query's scores go (ivf_pairs.cuh); a CTA per
 // query then selects, re-scores its candidates in the reference's operation order and checks that the margin
@@ -20,8 +20,8 @@
 //   sq8         code - 128 as signed bytes against three int8 terms of the query's weights, exact int32 sums
 //   rabitq      the sign bits as bytes 0 / 1 against three int8 terms of the query; sum over set bits = (sum of all
 //               terms + signed sum) / 2
-// Each thread requests its part of the next piece before it converts the current one, so about 32 KB per CTA are
-// always in flight from memory.
+// Each loader thread holds its part of the next two or three pieces in registers while it converts the current one,
+// across tiles and items, so 64 KB or more per SM are always in flight.
 #pragma once
 
 #include "ivf_pairs.cuh"
@@ -31,12 +31,12 @@ namespace vb200 {
 
 constexpr int TILE_LOAD_WARPS = 8;
 constexpr int TILE_LOADERS = 32 * TILE_LOAD_WARPS;
-constexpr int TILE_EPI_WARPS = 4;
-constexpr int TILE_THREADS = 32 * (TILE_EPI_WARPS + 1 + TILE_LOAD_WARPS);   // warps 0-3 epilogue, 4 MMA, 5-12 loaders
+constexpr int TILE_EPI_WARPS = 8;
+constexpr int TILE_THREADS = 32 * (TILE_EPI_WARPS + 1 + TILE_LOAD_WARPS);   // warps 0-7 epilogue, 8 MMA, then the loaders
 constexpr uint32_t TILE_PIECE = 128;                        // operand bytes per row and piece
 constexpr uint32_t TILE_A_TERM = 128 * TILE_PIECE;          // 16 KiB
 constexpr uint32_t TILE_MAX_STAGES = 6;
-constexpr uint32_t TILE_ACC_COLS = 128;                     // tensor-memory columns per accumulator, two of them
+constexpr uint32_t TILE_ACC_COLS = 256;                     // tensor-memory columns per accumulator, two of them
 
 // How a codec becomes MMA operands.
 template <int FMT>
@@ -47,8 +47,12 @@ struct TileFmt {
     static constexpr uint32_t PIECE_DIMS = INT8 ? 128 : 64;
 };
 
+// Lists of very different lengths are the rule (a list that many queries probe is often a long one): an item is at
+// most TILE_SEGMENT rows of a list, so that no CTA is left with one long list at the end.
+constexpr uint32_t TILE_SEGMENT = 1024;
+
 struct TileItem {
-    uint32_t list, pair0, nqt, pad;
+    uint32_t list, pair0, nqt, row0;   // rows row0 .. row0 + TILE_SEGMENT of the list
 };
 
 struct TileScan {
@@ -79,6 +83,7 @@ struct TileGroup {
     const int32_t* probes;    // [pairs]
     uint32_t pairs, nlist, qt;
     const uint32_t* order;    // [nlist] lists, longest first: items that finish last are short
+    const uint32_t* list_off;
     uint32_t* pair_off;       // [nlist]
     uint32_t* item_off;       // [nlist]
     uint32_t* list_pairs;     // [nlist] the counts, kept
@@ -96,7 +101,7 @@ tile_places_kernel(const TileGroup g) {
     }
     constexpr uint32_t PER = 4;
     for (uint32_t l0 = 0; l0 < g.nlist; l0 += 1024 * PER) {
-        uint32_t list[PER], cnt[PER], sum = 0, tiles = 0;
+        uint32_t list[PER], cnt[PER], its[PER], sum = 0, tiles = 0;
 #pragma unroll
         for (uint32_t j = 0; j < PER; ++j) {
             const uint32_t i = l0 + threadIdx.x * PER + j;
@@ -105,8 +110,11 @@ tile_places_kernel(const TileGroup g) {
 #pragma unroll
         for (uint32_t j = 0; j < PER; ++j) {
             cnt[j] = list[j] != 0xFFFFFFFFu ? g.count[list[j]] : 0u;
+            its[j] = cnt[j] > 0 ? (cnt[j] + g.qt - 1) / g.qt *
+                                      ((__ldg(g.list_off + list[j] + 1) - __ldg(g.list_off + list[j]) + TILE_SEGMENT - 1) / TILE_SEGMENT)
+                                : 0u;
             sum += cnt[j];
-            tiles += (cnt[j] + g.qt - 1) / g.qt;
+            tiles += its[j];
         }
         const uint32_t sum_incl = block_inclusive_sum<1024>(sum, part);
         const uint32_t tile_incl = block_inclusive_sum<1024>(tiles, part);
@@ -124,7 +132,7 @@ tile_places_kernel(const TileGroup g) {
                 g.list_pairs[list[j]] = cnt[j];
                 g.count[list[j]] = 0;
                 at += cnt[j];
-                tat += (cnt[j] + g.qt - 1) / g.qt;
+                tat += its[j];
             }
         }
         __syncthreads();
@@ -148,8 +156,11 @@ tile_scatter_kernel(const TileGroup g) {
         const uint32_t n = g.list_pairs[e];
         TileItem* dst = g.items + g.item_off[e];
         const uint32_t p0 = g.pair_off[e];
-        for (uint32_t i = 0; i * g.qt < n; ++i) {
-            dst[i] = TileItem{e, p0 + i * g.qt, min(g.qt, n - i * g.qt), 0u};
+        const uint32_t len = n > 0 ? __ldg(g.list_off + e + 1) - __ldg(g.list_off + e) : 0u;
+        for (uint32_t row0 = 0; row0 < len; row0 += TILE_SEGMENT) {
+            for (uint32_t i = 0; i * g.qt < n; ++i) {
+                *dst++ = TileItem{e, p0 + i * g.qt, min(g.qt, n - i * g.qt), row0};
+            }
         }
     }
 }
@@ -162,9 +173,9 @@ struct TileShared {
     uint32_t tmem_base, failed;
     // where the running item's scores go and its queries' constants: a copy per epilogue warp, which therefore never
     // wait for one another
-    uint64_t out[TILE_EPI_WARPS][32];
-    float c0[TILE_EPI_WARPS][32], c1[TILE_EPI_WARPS][32];
-    int32_t t1[TILE_EPI_WARPS][32], t2[TILE_EPI_WARPS][32], t3[TILE_EPI_WARPS][32];
+    uint64_t out[TILE_EPI_WARPS][64];
+    float c0[TILE_EPI_WARPS][64], c1[TILE_EPI_WARPS][64];
+    int32_t t1[TILE_EPI_WARPS][64], t2[TILE_EPI_WARPS][64], t3[TILE_EPI_WARPS][64];
 };
 
 // Instruction descriptor of kind::f16 with fp16 operands (bf16: umma_idesc_bf16).
@@ -216,6 +227,7 @@ spread_bits16(uint32_t b) {
 template <int FMT>
 struct TileUnit {
     uint4 raw[FMT == ROW_F32 ? 2 : 1];
+    uint2 bits;   // RaBitQ
     __device__ __forceinline__ void
     load(const uint8_t* row, bool valid, uint32_t piece, uint32_t kc, uint32_t dim) {
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -225,7 +237,7 @@ struct TileUnit {
             raw[0] = valid && d0 < dim ? __ldg(src) : zero;
             raw[FMT == ROW_F32 ? 1 : 0] = valid && d0 + 4 < dim ? __ldg(src + 1) : zero;
         } else if (FMT == ROW_RABITQ) {
-            // (the loader of this codec takes 64 dimensions of a row per unit: see tile_scan_kernel)
+            // (64 sign bits per thread: see tile_scan_kernel)
         } else {
             const uint32_t per = FMT == ROW_SQ8 ? 16 : 8;
             const uint32_t d0 = piece * (8 * per) + kc * per;
@@ -297,9 +309,9 @@ tile_publish(uint64_t* bar, uint32_t lane) {
     }
 }
 
-// QT queries per item at most (16 or 32).
+// QT queries per item at most (16, 32 or 64).
 template <int FMT, int QT>
-__global__ void __launch_bounds__(TILE_THREADS, 2)
+__global__ void __launch_bounds__(TILE_THREADS, 1)
 tile_scan_kernel(const TileScan p) {
     using F = TileFmt<FMT>;
     constexpr uint32_t N = F::B_TERMS * QT;                  // rows of B, columns of the accumulator
@@ -342,49 +354,109 @@ tile_scan_kernel(const TileScan p) {
         // ---------------- loaders: code records -> operands ----------------
         const uint32_t lt = threadIdx.x - 32 * (TILE_EPI_WARPS + 1);
         const uint32_t lwarp = lt >> 5;
+        constexpr uint32_t SETS = FMT == ROW_F32 ? 2 : 4;    // pieces requested ahead, in registers
+        constexpr uint32_t UNITS = 1024 / TILE_LOADERS;      // 16-byte operand units per thread and piece
+        // Where the loads are; items are dealt round-robin, and a cursor reads the next item's description while it
+        // works through the current one.
+        struct Cursor {
+            uint32_t item, lbeg, len, pair0, nqt, next_lbeg, next_len, next_pair0, next_nqt, r0, piece;
+        };
+        auto describe = [&](uint32_t item, uint32_t& lbeg, uint32_t& len, uint32_t& pair0, uint32_t& nqt) {
+            lbeg = len = pair0 = nqt = 0;
+            if (item < n_items) {
+                const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
+                lbeg = __ldg(p.s.list_off + d.x) + d.w;
+                len = min(__ldg(p.s.list_off + d.x + 1) - lbeg, TILE_SEGMENT);
+                pair0 = d.y;
+                nqt = d.z;
+            }
+        };
+        auto start = [&](Cursor& c) {
+            c.item = blockIdx.x;
+            c.r0 = c.piece = 0;
+            describe(c.item, c.lbeg, c.len, c.pair0, c.nqt);
+            describe(c.item + gridDim.x, c.next_lbeg, c.next_len, c.next_pair0, c.next_nqt);
+        };
+        auto advance = [&](Cursor& c) {
+            if (++c.piece < pieces) {
+                return;
+            }
+            c.piece = 0;
+            c.r0 += 128;
+            if (c.r0 < c.len) {
+                return;
+            }
+            c.r0 = 0;
+            c.item += gridDim.x;
+            c.lbeg = c.next_lbeg;
+            c.len = c.next_len;
+            c.pair0 = c.next_pair0;
+            c.nqt = c.next_nqt;
+            describe(c.item + gridDim.x, c.next_lbeg, c.next_len, c.next_pair0, c.next_nqt);
+        };
+        // eight lanes on the line of a row, four rows per warp and step
+        const uint32_t kc = lane & 7u, rr = lwarp * (128 / TILE_LOAD_WARPS) + (lane >> 3);
+        TileUnit<FMT> u[SETS][UNITS];
+        auto request = [&](const Cursor& c, TileUnit<FMT> (&set)[UNITS]) {
+            if (c.item >= n_items) {
+                return;
+            }
+            const uint8_t* rows = p.s.codes + static_cast<uint64_t>(c.lbeg) * p.s.code_stride;
+            if (FMT == ROW_RABITQ) {
+                // a thread takes 64 dimensions of one row: eight bytes of sign bits, four k-cores
+                const uint32_t r = c.r0 + (lt >> 1), part = lt & 1u;
+                set[0].bits = r < c.len && c.piece * 128 + part * 64 < dim
+                                  ? __ldg(reinterpret_cast<const uint2*>(rows + static_cast<uint64_t>(r) * p.s.code_stride + c.piece * 16 + part * 8))
+                                  : make_uint2(0u, 0u);
+                return;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < UNITS; ++j) {
+                const uint32_t r = c.r0 + rr + j * 4;
+                set[j].load(rows + static_cast<uint64_t>(r < c.len ? r : 0u) * p.s.code_stride, r < c.len, c.piece, kc, dim);
+            }
+        };
         uint32_t stage = 0, phase = 0, filled = 0, n_mine = 0;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_mine) {
-            const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
-            const uint32_t lbeg = __ldg(p.s.list_off + d.x), len = __ldg(p.s.list_off + d.x + 1) - lbeg;
+        auto load_queries = [&](const Cursor& c) -> bool {
             const uint32_t buf = p.b_bufs == 2 ? n_mine & 1u : 0u;
             if (n_mine >= p.b_bufs) {
                 // (use number n_mine / b_bufs of this buffer: the use before it must have been multiplied)
-                ok = tile_wait(&sh.b_free[buf], ((n_mine / p.b_bufs) - 1u) & 1u, failed, p.spin_limit, lane);
-                if (!ok) {
-                    break;
+                if (!tile_wait(&sh.b_free[buf], ((n_mine / p.b_bufs) - 1u) & 1u, failed, p.spin_limit, lane)) {
+                    return false;
                 }
             }
             unsigned char* bd = b_smem + buf * b_bytes;
+            const uint32_t per_row = pieces * 8;             // units of a row of B
             if (F::INT8) {
-                const uint32_t per_row = pieces * 8;         // 16-byte units of a term
-                for (uint32_t u = lt; u < N * per_row; u += TILE_LOADERS) {
-                    const uint32_t r = u / per_row, c = u - r * per_row;
+#pragma unroll 4
+                for (uint32_t i = lt; i < N * per_row; i += TILE_LOADERS) {
+                    const uint32_t r = i / per_row, k = i - r * per_row;
                     const uint32_t term = r / QT, qi = r - term * QT;
                     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (qi < d.z && c * 16 < p.qstride) {
-                        const uint32_t q = __ldg(p.pair_ids + d.y + qi) / p.nprobe;
-                        v = __ldg(reinterpret_cast<const uint4*>(p.qw8 + (static_cast<uint64_t>(q) * 3 + term) * p.qstride + c * 16));
+                    if (qi < c.nqt && k * 16 < p.qstride) {
+                        const uint32_t q = __ldg(p.pair_ids + c.pair0 + qi) / p.nprobe;
+                        v = __ldg(reinterpret_cast<const uint4*>(p.qw8 + (static_cast<uint64_t>(q) * 3 + term) * p.qstride + k * 16));
                     }
-                    *reinterpret_cast<uint4*>(bd + (c >> 3) * B_PIECE + swizzled(r, c & 7u)) = v;
+                    *reinterpret_cast<uint4*>(bd + (k >> 3) * B_PIECE + swizzled(r, k & 7u)) = v;
                 }
             } else {
-                const uint32_t per_row = pieces * 8;         // units of eight dimensions
-                for (uint32_t u = lt; u < QT * per_row; u += TILE_LOADERS) {
-                    const uint32_t qi = u / per_row, c = u - qi * per_row;
+#pragma unroll 2
+                for (uint32_t i = lt; i < QT * per_row; i += TILE_LOADERS) {
+                    const uint32_t qi = i / per_row, k = i - qi * per_row;
                     float x[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        x[i] = 0.f;
+                    for (int e = 0; e < 8; ++e) {
+                        x[e] = 0.f;
                     }
-                    if (qi < d.z) {
-                        const uint32_t q = __ldg(p.pair_ids + d.y + qi) / p.nprobe;
-                        const float* src = p.s.queries + static_cast<uint64_t>(q) * dim + c * 8;
+                    if (qi < c.nqt) {
+                        const uint32_t q = __ldg(p.pair_ids + c.pair0 + qi) / p.nprobe;
+                        const float* src = p.s.queries + static_cast<uint64_t>(q) * dim + k * 8;
 #pragma unroll
-                        for (uint32_t i = 0; i < 8; ++i) {
-                            x[i] = c * 8 + i < dim ? __ldg(src + i) : 0.f;
+                        for (uint32_t e = 0; e < 8; ++e) {
+                            x[e] = k * 8 + e < dim ? __ldg(src + e) : 0.f;
                         }
                     }
-                    unsigned char* dst = bd + (c >> 3) * B_PIECE + swizzled(qi, c & 7u);
+                    unsigned char* dst = bd + (k >> 3) * B_PIECE + swizzled(qi, k & 7u);
                     if (FMT == ROW_F32) {
                         uint4 hi, lo;
                         split_bf16x8(x, hi, lo);
@@ -394,63 +466,68 @@ tile_scan_kernel(const TileScan p) {
                         constexpr int HF = FMT == ROW_BF16 ? SCAN_FMT_BF16 : SCAN_FMT_FP16;
                         uint32_t w[4];
 #pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) {
-                            const uint32_t a = qi < d.z && c * 8 + 2 * i < dim ? half_encode<HF>(x[2 * i]) : 0u;
-                            const uint32_t b = qi < d.z && c * 8 + 2 * i + 1 < dim ? half_encode<HF>(x[2 * i + 1]) : 0u;
-                            w[i] = a | (b << 16);
+                        for (uint32_t e = 0; e < 4; ++e) {
+                            const uint32_t lo = qi < c.nqt && k * 8 + 2 * e < dim ? half_encode<HF>(x[2 * e]) : 0u;
+                            const uint32_t hi = qi < c.nqt && k * 8 + 2 * e + 1 < dim ? half_encode<HF>(x[2 * e + 1]) : 0u;
+                            w[e] = lo | (hi << 16);
                         }
                         *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
             }
             tile_publish(&sh.b_full[buf], lane);
-            const uint8_t* rows = p.s.codes + static_cast<uint64_t>(lbeg) * p.s.code_stride;
-            for (uint32_t r0 = 0; r0 < len && ok; r0 += 128) {
-                for (uint32_t piece = 0; piece < pieces; ++piece) {
-                    unsigned char* dst = smem + stage * STAGE;
-                    if (FMT == ROW_RABITQ) {
-                        // a thread takes 64 dimensions of one row: eight bytes of sign bits, four k-cores
-                        const uint32_t r = lt >> 1, half = lt & 1u;
-                        uint2 bits = make_uint2(0u, 0u);
-                        if (r0 + r < len && piece * 128 + half * 64 < dim) {
-                            bits = __ldg(reinterpret_cast<const uint2*>(rows + static_cast<uint64_t>(r0 + r) * p.s.code_stride + piece * 16 + half * 8));
-                        }
-                        if (filled >= stages) {
-                            ok = tile_wait(&sh.freed[stage], phase ^ 1u, failed, p.spin_limit, lane);
-                        }
-                        if (!ok) {
-                            break;
-                        }
-                        *reinterpret_cast<uint4*>(dst + swizzled(r, half * 4)) = spread_bits16(bits.x & 0xFFFFu);
-                        *reinterpret_cast<uint4*>(dst + swizzled(r, half * 4 + 1)) = spread_bits16(bits.x >> 16);
-                        *reinterpret_cast<uint4*>(dst + swizzled(r, half * 4 + 2)) = spread_bits16(bits.y & 0xFFFFu);
-                        *reinterpret_cast<uint4*>(dst + swizzled(r, half * 4 + 3)) = spread_bits16(bits.y >> 16);
-                    } else {
-                        // four units per thread: eight lanes on the line of a row, four rows per warp and step
-                        TileUnit<FMT> u[4];
-                        const uint32_t kc = lane & 7u, rr = lwarp * 16 + (lane >> 3);
+            ++n_mine;
+            return true;
+        };
+        Cursor now, ahead;
+        start(now);
+        start(ahead);
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; ++j) {
-                            const uint32_t r = r0 + rr + j * 4;
-                            u[j].load(rows + static_cast<uint64_t>(r < len ? r : 0u) * p.s.code_stride, r < len, piece, kc, dim);
-                        }
-                        if (filled >= stages) {
-                            ok = tile_wait(&sh.freed[stage], phase ^ 1u, failed, p.spin_limit, lane);
-                        }
-                        if (!ok) {
-                            break;
-                        }
+        for (uint32_t s = 0; s < SETS; ++s) {
+            request(ahead, u[s]);
+            if (ahead.item < n_items) {
+                advance(ahead);
+            }
+        }
+        while (now.item < n_items && ok) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; ++j) {
-                            u[j].store(dst + swizzled(rr + j * 4, kc), piece, kc, dim);
-                        }
+            for (uint32_t s = 0; s < SETS; ++s) {
+                if (now.item >= n_items || !ok) {
+                    break;
+                }
+                if (now.r0 == 0 && now.piece == 0) {
+                    ok = load_queries(now);
+                }
+                if (ok && filled >= stages) {
+                    ok = tile_wait(&sh.freed[stage], phase ^ 1u, failed, p.spin_limit, lane);
+                }
+                if (!ok) {
+                    break;
+                }
+                unsigned char* dst = smem + stage * STAGE;
+                if (FMT == ROW_RABITQ) {
+                    const uint32_t r = lt >> 1, part = lt & 1u;
+                    const uint2 bits = u[s][0].bits;
+                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4)) = spread_bits16(bits.x & 0xFFFFu);
+                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4 + 1)) = spread_bits16(bits.x >> 16);
+                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4 + 2)) = spread_bits16(bits.y & 0xFFFFu);
+                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4 + 3)) = spread_bits16(bits.y >> 16);
+                } else {
+#pragma unroll
+                    for (uint32_t j = 0; j < UNITS; ++j) {
+                        u[s][j].store(dst + swizzled(rr + j * 4, kc), now.piece, kc, dim);
                     }
-                    tile_publish(&sh.full[stage], lane);
-                    ++filled;
-                    if (++stage == stages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                }
+                tile_publish(&sh.full[stage], lane);
+                request(ahead, u[s]);
+                if (ahead.item < n_items) {
+                    advance(ahead);
+                }
+                advance(now);
+                ++filled;
+                if (++stage == stages) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
         }
@@ -463,8 +540,8 @@ tile_scan_kernel(const TileScan p) {
             const uint64_t a0 = umma_desc_sw128(smem_u32(smem)), b0 = umma_desc_sw128(smem_u32(b_smem));
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, tiles = 0, n_mine = 0;
             for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_mine) {
-                const uint32_t l = __ldg(&p.items[item].list);
-                const uint32_t len = __ldg(p.s.list_off + l + 1) - __ldg(p.s.list_off + l);
+                const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
+                const uint32_t len = min(__ldg(p.s.list_off + d.x + 1) - __ldg(p.s.list_off + d.x) - d.w, TILE_SEGMENT);
                 const uint32_t buf = p.b_bufs == 2 ? n_mine & 1u : 0u;
                 ok = tcs_wait(&sh.b_full[buf], (n_mine / p.b_bufs) & 1u, failed, p.spin_limit);
                 for (uint32_t r0 = 0; r0 < len && ok; r0 += 128) {
@@ -517,27 +594,28 @@ tile_scan_kernel(const TileScan p) {
         }
         __syncwarp();
     } else {
-        // ---------------- epilogue: one thread per row of the tile ----------------
-        const uint32_t row = warp * 32 + lane;
+        // ---------------- epilogue: one thread per row of the tile, two warps per 32 rows share the queries ----------------
+        const uint32_t quarter = warp & 3u, half = warp >> 2;
+        const uint32_t row = quarter * 32 + lane;
         uint32_t tile = 0;
         const bool filtered = p.s.filter_pos_inner != nullptr;
         for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
             const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
-            const uint32_t lbeg = __ldg(p.s.list_off + d.x), len = __ldg(p.s.list_off + d.x + 1) - lbeg;
-            const uint32_t par = warp;
+            const uint32_t lbeg = __ldg(p.s.list_off + d.x) + d.w, len = min(__ldg(p.s.list_off + d.x + 1) - lbeg, TILE_SEGMENT);
             __syncwarp();
-            if (lane < d.z) {
-                const uint32_t pair = __ldg(p.pair_ids + d.y + lane), q = pair / p.nprobe, j = lane;
-                sh.out[par][j] = q * p.t.stride + __ldg(p.t.base + pair);
+            for (uint32_t j = lane; j < QT; j += 32) {
+                const bool used = j < d.z;
+                const uint32_t pair = used ? __ldg(p.pair_ids + d.y + j) : 0u, q = pair / p.nprobe;
+                sh.out[warp][j] = used ? q * p.t.stride + __ldg(p.t.base + pair) + d.w : 0u;
                 if (FMT == ROW_SQ8) {
-                    sh.c0[par][j] = __ldg(p.s.qa + q);
-                    sh.c1[par][j] = p.s.coef_c * __ldg(p.qscale + q);
+                    sh.c0[warp][j] = used ? __ldg(p.s.qa + q) : 0.f;
+                    sh.c1[warp][j] = used ? p.s.coef_c * __ldg(p.qscale + q) : 0.f;
                 } else if (FMT == ROW_RABITQ) {
-                    sh.c0[par][j] = __ldg(p.s.queries + static_cast<uint64_t>(q) * (dim + 1) + dim);
-                    sh.c1[par][j] = __ldg(p.qscale + q);
-                    sh.t1[par][j] = __ldg(p.qsum + 4 * q);
-                    sh.t2[par][j] = __ldg(p.qsum + 4 * q + 1);
-                    sh.t3[par][j] = __ldg(p.qsum + 4 * q + 2);
+                    sh.c0[warp][j] = used ? __ldg(p.s.queries + static_cast<uint64_t>(q) * (dim + 1) + dim) : 0.f;
+                    sh.c1[warp][j] = used ? __ldg(p.qscale + q) : 0.f;
+                    sh.t1[warp][j] = used ? __ldg(p.qsum + 4 * q) : 0;
+                    sh.t2[warp][j] = used ? __ldg(p.qsum + 4 * q + 1) : 0;
+                    sh.t3[warp][j] = used ? __ldg(p.qsum + 4 * q + 2) : 0;
                 }
             }
             __syncwarp();
@@ -553,59 +631,72 @@ tile_scan_kernel(const TileScan p) {
                     const float* tail = reinterpret_cast<const float*>(p.s.codes + static_cast<uint64_t>(pos) * p.s.code_stride + p.s.dpad / 8);
                     x0 = __ldg(tail);
                     x1 = __ldg(tail + 1);
+                    if (fabsf(x1) < 1e-5f) {
+                        x1 = x1 >= 0.f ? 1.0f : -1.0f;
+                    }
+                    x1 = -2.0f * x0 / x1;
+                    x0 *= x0;
                 } else if (p.l2 != 0) {
                     x0 = __ldg(p.row_norm + pos);
                 }
-                const bool drop = filtered && valid && scan_row_filtered(p.s, pos);
+                const bool drop = !valid || (filtered && scan_row_filtered(p.s, pos));
                 ok = tile_wait(&sh.acc_full[acc], (tile >> 1) & 1u, failed, p.spin_limit, lane);
                 if (!ok) {
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t taddr = tmem_base + ((warp * 32u) << 16) + acc * TILE_ACC_COLS;
-#pragma unroll
-                for (uint32_t g = 0; g < QT; g += 8) {
-                    if (g >= d.z) {
-                        break;
-                    }
-                    uint32_t v1[8], v2[8], v3[8];
-                    tmem_load_8(taddr + g, v1);
-                    if (F::B_TERMS >= 2) {
-                        tmem_load_8(taddr + QT + g, v2);
-                    }
-                    if (F::B_TERMS >= 3) {
-                        tmem_load_8(taddr + 2 * QT + g, v3);
-                    }
-                    tmem_load_wait();
-                    if (valid) {
+                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * TILE_ACC_COLS;
+                if (r0 + quarter * 32 < len) {   // (the warp's rows are one group of 32 scores)
+                    // the last read of an accumulator is followed by its hand-over; columns past the item's queries hold
+                    // products with zero and are not stored
+                    for (uint32_t g = half * 8; g < d.z; g += 16) {
+                        uint32_t v1[8], v2[8], v3[8];
+                        tmem_load_8(taddr + g, v1);
+                        if (F::B_TERMS >= 2) {
+                            tmem_load_8(taddr + QT + g, v2);
+                        }
+                        if (F::B_TERMS >= 3) {
+                            tmem_load_8(taddr + 2 * QT + g, v3);
+                        }
+                        tmem_load_wait();
+                        float v[8];
 #pragma unroll
                         for (uint32_t i = 0; i < 8; ++i) {
                             const uint32_t j = g + i;
-                            if (j >= d.z) {
-                                break;
-                            }
-                            float v;
                             if (FMT == ROW_SQ8) {
                                 const float low = static_cast<float>(static_cast<int32_t>(v2[i]) * 254 + static_cast<int32_t>(v3[i]));
                                 const float f = fmaf(low, 1.0f / 64516.0f, static_cast<float>(static_cast<int32_t>(v1[i])));
-                                v = fmaf(sh.c1[par][j], f, x0) + sh.c0[par][j];
+                                v[i] = fmaf(sh.c1[warp][j], f, x0) + sh.c0[warp][j];
                             } else if (FMT == ROW_RABITQ) {
-                                const int32_t u1 = 2 * static_cast<int32_t>(v1[i]) - sh.t1[par][j];
-                                const int32_t u2 = 2 * static_cast<int32_t>(v2[i]) - sh.t2[par][j];
-                                const int32_t u3 = 2 * static_cast<int32_t>(v3[i]) - sh.t3[par][j];
+                                // |x|^2 + |q|^2 - 2 |x| |q| (ip / error); the set bits' sum S gives ip = 2 S - (sum of all)
+                                const int32_t u1 = 2 * static_cast<int32_t>(v1[i]) - sh.t1[warp][j];
+                                const int32_t u2 = 2 * static_cast<int32_t>(v2[i]) - sh.t2[warp][j];
+                                const int32_t u3 = 2 * static_cast<int32_t>(v3[i]) - sh.t3[warp][j];
                                 const float f = fmaf(static_cast<float>(u2 * 254 + u3), 1.0f / 64516.0f, static_cast<float>(u1));
-                                v = rabitq_distance(f * sh.c1[par][j], x0, x1, sh.c0[par][j]);
+                                const float qn = sh.c0[warp][j];
+                                v[i] = fmaf(x1 * qn, f * sh.c1[warp][j], fmaf(qn, qn, x0));
                             } else {
                                 float ip = __uint_as_float(v1[i]);
                                 if (FMT == ROW_F32) {
                                     ip += __uint_as_float(v2[i]);
                                 }
-                                v = p.l2 != 0 ? fmaf(-2.0f, ip, x0) : -ip;
+                                v[i] = p.l2 != 0 ? fmaf(-2.0f, ip, x0) : -ip;
                             }
-                            reinterpret_cast<uint32_t*>(p.t.scores)[sh.out[par][j] + r] = drop ? SCORE_FILTERED : __float_as_uint(v);
+                        }
+                        uint32_t least = 0;   // of column g + lane
+#pragma unroll
+                        for (uint32_t i = 0; i < 8; ++i) {
+                            const uint32_t bits = drop ? SCORE_FILTERED : __float_as_uint(v[i]);
+                            if (g + i < d.z) {
+                                reinterpret_cast<uint32_t*>(p.t.scores)[sh.out[warp][g + i] + r] = bits;
+                            }
+                            const uint32_t low = __reduce_min_sync(0xffffffffu, ScoreSource<>::ordered(bits));
+                            least = lane == i ? low : least;
+                        }
+                        if (lane < 8 && g + lane < d.z) {
+                            p.t.minima[(sh.out[warp][g + lane] + r0 + quarter * 32) >> 5] = least;
                         }
                     }
-                    __syncwarp();
                 }
                 tc_fence_before_sync();
                 __syncwarp();

@@ -2,13 +2,16 @@
 // dense kernel with a fused argmin epilogue, and the centroid update.
 #include "kmeans.cuh"
 
+#include <algorithm>
 #include <random>
+#include <vector>
 
 #include <cstdlib>
 
 #include <cub/device/device_radix_sort.cuh>
 
 #include "dense.cuh"
+#include "kpp.cuh"
 
 namespace vb200 {
 
@@ -511,6 +514,8 @@ vb200_release_workspaces(void) {
     std::lock_guard<std::mutex> lock(g_kmeans_ws_mu);
     delete g_kmeans_ws;
     g_kmeans_ws = nullptr;
+    (void)sync_stream();   // what was freed is free now
+    pool_trim();
     return 0;
 }
 
@@ -773,6 +778,71 @@ kpp_copy_row_kernel(const float* __restrict__ x, uint64_t row, uint32_t dim, uin
     }
 }
 
+// All rounds as one cooperative launch (kpp.cuh).  *done = false when the device cannot hold the grid (an SM limit on
+// the context): the caller then seeds round by round.
+static int
+kpp_run_rounds(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, uint64_t first, const std::vector<double>& u, float* min_d,
+               uint32_t* state, float* centroids_dev, int64_t* picked_dev, bool* done) {
+    *done = false;
+    const uint32_t sms = static_cast<uint32_t>(sm_count());
+    const size_t qpad = (dim + 3) / 4 * 4;
+    // rows per CTA when every SM takes a share (at least 16 rows: fewer are not worth a CTA in the barriers)
+    const uint64_t resident_per = std::max<uint64_t>((n + sms - 1) / sms, 16);
+    const size_t resident_bytes = (qpad + resident_per * ((dim | 1u) + 1)) * sizeof(float);
+    const bool resident = resident_bytes <= 216 * 1024;
+    const bool wide = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0;
+    const size_t smem = resident ? resident_bytes : RS_STAGES * RS_STAGE + qpad * sizeof(float);
+    if (smem > 216 * 1024) {
+        return 0;
+    }
+    const void* kernel = resident ? reinterpret_cast<const void*>(kpp_rounds_kernel<true, 4, 512>)
+                                  : (wide ? reinterpret_cast<const void*>(kpp_rounds_kernel<false, 16, RS_ROWS>)
+                                          : reinterpret_cast<const void*>(kpp_rounds_kernel<false, 4, RS_ROWS>));
+    const int threads = resident ? 512 : RS_ROWS;
+    VB_TRY(allow_dynamic_smem(kernel, smem));
+    int per_sm = 0;
+    VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    if (per_sm < 1) {
+        return 0;
+    }
+    KppRounds p{};
+    p.x = x_dev;
+    p.n = n;
+    p.dim = dim;
+    p.k = k;
+    if (resident) {
+        p.per = resident_per;
+    } else {
+        const uint64_t most = std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, (n + RS_ROWS - 1) / RS_ROWS);
+        p.per = (n + most - 1) / most;
+    }
+    const uint64_t grid = (n + p.per - 1) / p.per;
+    p.first = first;
+    DevBuf<double> draws, part;
+    DevBuf<unsigned long long> pick;
+    VB_TRY(draws.reserve(k));
+    VB_TRY(part.reserve(grid));
+    VB_TRY(pick.reserve(1));
+    VB_CUDA(cudaMemcpyAsync(draws.ptr, u.data(), k * sizeof(double), cudaMemcpyHostToDevice, current_stream()));
+    p.u = draws.ptr;
+    p.min_d = min_d;
+    p.part = part.ptr;
+    p.pick = pick.ptr;
+    p.centroids = centroids_dev;
+    p.picked = picked_dev;
+    p.state = state;
+    void* args[] = {&p};
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(static_cast<uint32_t>(grid)), dim3(threads), args, smem, current_stream());
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    VB_CUDA(e);
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    *done = true;
+    return sync_stream();   // the draws are the caller's
+}
+
 // centroids_dev[k x dim] and (optionally) picked_dev[k] on the device.  The generator and its
 // distributions are the C++ library's, exactly the objects the reference draws from; only the
 // seed is the caller's (the reference takes it from std::random_device).
@@ -790,17 +860,25 @@ kmeans_pp_init_device(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, 
     VB_LAUNCH(kpp_fill_kernel, static_cast<uint32_t>((n + 255) / 256), 256, 0, min_d.ptr, n, state.ptr);
     std::mt19937 gen(seed);
     std::uniform_int_distribution<uint64_t> any_row(0, n - 1);
-    VB_LAUNCH(kpp_copy_row_kernel, 1, 128, 0, x_dev, any_row(gen), dim, 0u, centroids_dev, picked_dev);
-    const size_t smem = (static_cast<size_t>((dim + 31) / 32) * 32 + 8 * 32 * 33) * sizeof(float);
-    VB_CHECK_ARG(smem <= 200 * 1024, "dim too large for the seeding kernel");
-    VB_CUDA(cudaFuncSetAttribute(kpp_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)));
+    const uint64_t first = any_row(gen);
     std::uniform_real_distribution<double> unit(0.0, 1.0);
+    std::vector<double> u(k, 0.0);
     for (uint32_t c = 1; c < k; ++c) {
-        VB_LAUNCH(kpp_update_kernel, n_part, 256, smem, x_dev, n, dim,
-                  centroids_dev + static_cast<size_t>(c - 1) * dim, min_d.ptr, part.ptr);
-        VB_LAUNCH(kpp_pick_kernel, 1, 1024, 0, x_dev, n, dim, min_d.ptr, part.ptr, n_part, unit(gen), c,
-                  centroids_dev, picked_dev, state.ptr);
+        u[c] = unit(gen);
+    }
+    bool done = false;
+    VB_TRY(kpp_run_rounds(x_dev, n, dim, k, first, u, min_d.ptr, state.ptr, centroids_dev, picked_dev, &done));
+    if (!done) {
+        VB_LAUNCH(kpp_copy_row_kernel, 1, 128, 0, x_dev, first, dim, 0u, centroids_dev, picked_dev);
+        const size_t smem = (static_cast<size_t>((dim + 31) / 32) * 32 + 8 * 32 * 33) * sizeof(float);
+        VB_CHECK_ARG(smem <= 200 * 1024, "dim too large for the seeding kernel");
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kpp_update_kernel), smem));
+        for (uint32_t c = 1; c < k; ++c) {
+            VB_LAUNCH(kpp_update_kernel, n_part, 256, smem, x_dev, n, dim,
+                      centroids_dev + static_cast<size_t>(c - 1) * dim, min_d.ptr, part.ptr);
+            VB_LAUNCH(kpp_pick_kernel, 1, 1024, 0, x_dev, n, dim, min_d.ptr, part.ptr, n_part, u[c], c,
+                      centroids_dev, picked_dev, state.ptr);
+        }
     }
     uint32_t first_flat = 0xFFFFFFFFu;
     VB_CUDA(cudaMemcpyAsync(&first_flat, state.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, current_stream()));

@@ -271,7 +271,7 @@ row_stream(const unsigned char* base, uint64_t row_stride, uint32_t row_bytes, u
     cp_async_wait_group<0>();
 }
 
-// Distance of one row to the query (widened, in shared memory), rows fetched sixteen bytes at a time with four
+// Distance of one row to the query (widened, in shared memory), rows fetched sixteen bytes at a time with eight
 // loads in flight where their alignment allows.
 template <typename E>
 __device__ __forceinline__ float
@@ -289,14 +289,14 @@ row_exact_distance(const E* __restrict__ x, const float* qf, uint32_t dim, bool 
     if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0 && dim % VEC == 0) {
         const uint4* xv = reinterpret_cast<const uint4*>(x);
         const uint32_t nv = dim / VEC;
-        for (uint32_t v0 = 0; v0 < nv; v0 += 4) {
-            uint4 w[4];
+        for (uint32_t v0 = 0; v0 < nv; v0 += 8) {
+            uint4 w[8];
 #pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
+            for (uint32_t u = 0; u < 8; ++u) {
                 w[u] = v0 + u < nv ? __ldg(xv + v0 + u) : make_uint4(0, 0, 0, 0);
             }
 #pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
+            for (uint32_t u = 0; u < 8; ++u) {
                 if (v0 + u < nv) {
                     E e[VEC];
                     *reinterpret_cast<uint4*>(e) = w[u];
