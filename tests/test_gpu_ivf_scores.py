@@ -25,6 +25,7 @@ def build(engine, oracle, quant, metric, n, dim, nlist, reorder=False):
 @pytest.mark.parametrize("quant", ["QUANT_FP32", "QUANT_BF16", "QUANT_FP16", "QUANT_SQ8", "QUANT_RABITQ"])
 @pytest.mark.parametrize("dim,n,nlist,nprobe,nq,k", [
     (1, 700, 5, 3, 40, 3),           # one dimension
+    (40, 2100, 6, 3, 300, 5),        # part of a piece, more queries than an item holds
     (65, 3001, 7, 4, 90, 10),        # one past a piece, several items per list
     (128, 4096, 16, 5, 33, 33),      # whole pieces
     (200, 2500, 40, 6, 30, 7),       # items of a few queries

@@ -106,7 +106,9 @@ struct SearchWorkspace {
     DevBuf<float> pair_scores;
     PinnedBuf pinned;
     // the same as tensor-core tiles (ivf_tiles.cuh): pairs grouped by list
-    DevBuf<uint32_t> tile_count, tile_rank, tile_tables, tile_pairs, pair_minima;
+    DevBuf<uint32_t> tile_count, tile_rank, tile_tables, pair_minima, pos_mask;
+    DevBuf<TilePair> tile_pairs;
+    DevBuf<uint16_t> tile_terms;
     DevBuf<uint32_t> rerank_ids, rerank_done;
     DevBuf<TileItem> tile_items;
     DevBuf<int32_t> qsum;
@@ -145,6 +147,8 @@ struct vb200_ivf {
     DevBuf<uint32_t> list_off;
     std::vector<uint32_t> list_off_host;
     uint32_t max_list_len = 0;   // the longest list this index (shard) holds
+    CUtensorMap row_map{};       // the stored rows for the tile scan's copies (fp32, bf16, fp16, RaBitQ)
+    bool has_row_map = false;
     DevBuf<float> row_max;       // [0] largest norm of a stored row, [1] RaBitQ: largest norm / |error term|
     std::vector<uint64_t> longest_rows;   // [nlist + 1] rows of the i longest lists together
     bool balls_valid = false;    // the covering balls describe the lists as they are stored
@@ -3055,31 +3059,38 @@ constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which
 enum ScoreScan { SCAN_GROUPED = 0, SCAN_PAIRS = 1, SCAN_TILES = 2 };
 
 struct TilePlan {
-    uint32_t qt, pieces, stages, b_bufs;
+    uint32_t qt, pieces, stages, b_bufs, raw_pitch;
     size_t smem;
 };
 
-// Shared memory of a tile launch (one CTA per SM): the B operand of an item, two when they fit, and 3 .. 6 pieces of
-// rows.  The more queries an item holds the less often a list is read again: as many as the average list has, since
-// empty columns cost little.  False when nothing fits.
+// Bytes between the rows of sign bits in shared memory: 16 times an odd number, so that four rows a step apart fall
+// on different banks.
+static uint32_t
+tile_raw_pitch(uint32_t dim) {
+    return 16 * ((dim + 127) / 128 | 1u);
+}
+
+// Shared memory of a tile launch (one CTA per SM): the B operand of an item, two when they fit beside four pieces of
+// rows, and as many pieces as are left.  The more queries an item holds the less often a list is read again, and
+// queries that an item lacks cost nothing; so as many as fit.  False when nothing fits.
 static bool
-tile_plan(const vb200_ivf* ix, double pairs_per_list, TilePlan* plan) {
-    const bool int8 = ix->quant == VB200_QUANT_SQ8 || ix->quant == VB200_QUANT_RABITQ, f32 = ix->quant == VB200_QUANT_FP32;
+tile_plan(const vb200_ivf* ix, TilePlan* plan) {
+    const bool rabitq = ix->quant == VB200_QUANT_RABITQ, int8 = ix->quant == VB200_QUANT_SQ8 || rabitq, f32 = ix->quant == VB200_QUANT_FP32;
     plan->pieces = (ix->dim + (int8 ? 127 : 63)) / (int8 ? 128 : 64);
-    const size_t stage = (f32 ? 2 : 1) * TILE_A_TERM;
+    plan->raw_pitch = rabitq ? tile_raw_pitch(ix->dim) : 0;
+    const size_t stage = (f32 ? 2 : 1) * TILE_A_TERM, raw = 2 * 128 * static_cast<size_t>(plan->raw_pitch);
     const uint32_t b_terms = int8 ? 3 : (f32 ? 2 : 1);
-    const size_t room = 208 * 1024;   // of 227 KiB: static shared memory and the step to a 1 KiB boundary
-    uint32_t qt = pairs_per_list > 28.0 ? 64 : (pairs_per_list > 14.0 ? 32 : 16);
-    for (; qt >= 16; qt /= 2) {
-        const size_t b = static_cast<size_t>(plan->pieces) * b_terms * qt * TILE_PIECE;
-        for (uint32_t bufs = 2; bufs >= 1; --bufs) {
-            if (bufs * b + 3 * stage <= room) {
-                plan->qt = qt;
-                plan->b_bufs = bufs;
-                plan->stages = static_cast<uint32_t>(std::min<size_t>((room - bufs * b) / stage, TILE_MAX_STAGES));
-                plan->smem = bufs * b + plan->stages * stage + 1024;
-                return true;
-            }
+    const size_t room = 220 * 1024;   // of 227 KiB: static shared memory and the step to a 1 KiB boundary
+    constexpr uint32_t CHOICES[5][2] = {{64, 2}, {32, 2}, {32, 1}, {16, 2}, {16, 1}};
+    for (const auto& choice : CHOICES) {
+        const uint32_t qt = choice[0], bufs = choice[1];
+        const size_t fixed = raw + static_cast<size_t>(bufs) * plan->pieces * b_terms * qt * TILE_PIECE;
+        if (fixed + (f32 ? 3 : 4) * stage <= room) {
+            plan->qt = qt;
+            plan->b_bufs = bufs;
+            plan->stages = static_cast<uint32_t>(std::min<size_t>((room - fixed) / stage, TILE_MAX_STAGES));
+            plan->smem = fixed + plan->stages * stage + 1024;
+            return true;
         }
     }
     return false;
@@ -3102,8 +3113,8 @@ ivf_score_scan(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe
     const double per_list = static_cast<double>(nq) * nprobe / ix->nlist;
     const double mean_len = static_cast<double>(ix->n_stored) / ix->nlist;
     const double rows = static_cast<double>(nq) * nprobe * mean_len;
-    if (tensor_cores_enabled() && per_list >= TILE_MIN_QUERIES && nq * ix->longest_rows[nprobe] < (uint64_t{1} << 28) &&
-        nq * nprobe < (uint64_t{1} << 31) && tile_plan(ix, per_list, plan)) {
+    if (tensor_cores_enabled() && per_list >= TILE_MIN_QUERIES && nq * nprobe < (uint64_t{1} << 31) &&
+        (sq8 ? ix->codes_t.ptr != nullptr : ix->has_row_map) && tile_plan(ix, plan)) {
         const bool prunes = sq8 && ix->prune_lists && ix->codes_t.ptr != nullptr && 8.0 * (kscan + SQ8_SLACK) <= mean_len && rows > 4e6;
         if (!prunes) {
             return SCAN_TILES;
@@ -3115,6 +3126,16 @@ ivf_score_scan(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe
     return SCAN_PAIRS;
 }
 
+// mask bit = the id filter of `p` rejects the row at that position.
+__global__ void __launch_bounds__(256)
+position_mask_kernel(const ScanParams p, uint64_t n, uint32_t* __restrict__ mask) {
+    const uint64_t pos = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
+    const uint32_t word = __ballot_sync(0xffffffffu, pos < n && scan_row_filtered(p, static_cast<uint32_t>(pos)));
+    if ((threadIdx.x & 31) == 0 && pos < n) {
+        mask[pos >> 5] = word;
+    }
+}
+
 // Groups the pairs by list and scans the lists as tiles into the score buffer.
 static int
 launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& plan) {
@@ -3124,7 +3145,7 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     // sum over lists of ceil(pairs / qt) * ceil(rows / segment), from above
     const uint64_t max_items = nq * sc.t.stride / (static_cast<uint64_t>(plan.qt) * TILE_SEGMENT) + pairs / plan.qt +
                                ix->n_stored / TILE_SEGMENT + std::min<uint64_t>(pairs, nlist) + 1;
-    VB_TRY(ws.tile_tables.reserve(3 * static_cast<size_t>(nlist) + 1));
+    VB_TRY(ws.tile_tables.reserve(3 * static_cast<size_t>(nlist) + 2));
     VB_TRY(ws.tile_pairs.reserve(pairs));
     VB_TRY(ws.tile_items.reserve(max_items));
     TileGroup g{};
@@ -3139,31 +3160,45 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     g.pair_off = ws.tile_tables.ptr;
     g.item_off = ws.tile_tables.ptr + nlist;
     g.list_pairs = ws.tile_tables.ptr + 2 * static_cast<size_t>(nlist);
-    g.n_items = ws.tile_tables.ptr + 3 * static_cast<size_t>(nlist);
-    g.pair_ids = ws.tile_pairs.ptr;
+    g.queue = ws.tile_tables.ptr + 3 * static_cast<size_t>(nlist);
+    g.tile_pairs = ws.tile_pairs.ptr;
     g.items = ws.tile_items.ptr;
+    g.nprobe = nprobe;
+    g.t = sc.t;
+    g.group_off = ix->quant == VB200_QUANT_SQ8 ? ix->group_off.ptr : nullptr;
     VB_LAUNCH(tile_places_kernel, 1, 1024, 0, g);
     VB_LAUNCH(tile_scatter_kernel, static_cast<uint32_t>((std::max<uint64_t>(pairs, nlist) + 255) / 256), 256, 0, g);
     TileScan t{};
     t.s = sc.s;
     t.t = sc.t;
-    t.nprobe = nprobe;
+    t.map = ix->row_map;
     t.items = g.items;
-    t.n_items = g.n_items;
-    t.pair_ids = g.pair_ids;
+    t.queue = g.queue;
+    t.pairs = g.tile_pairs;
     t.pieces = plan.pieces;
     t.stages = plan.stages;
     t.b_bufs = plan.b_bufs;
-    t.qw8 = sc.qw8;
+    t.raw_pitch = plan.raw_pitch;
+    t.kchunks = ix->kchunks;
+    t.codes_t = ix->codes_t.ptr;
+    t.terms = ix->quant == VB200_QUANT_SQ8 || ix->quant == VB200_QUANT_RABITQ ? reinterpret_cast<const unsigned char*>(sc.qw8)
+                                                                              : reinterpret_cast<const unsigned char*>(ws.tile_terms.ptr);
     t.qscale = sc.qscale;
     t.qsum = ws.qsum.ptr;
-    t.qstride = ix->quant == VB200_QUANT_RABITQ ? (ix->dim + 15) / 16 * 16 : ix->dpad;
+    if (sc.s.filter_pos_inner != nullptr) {
+        // the id filter as a bitmap over positions: looked up row by row it is three dependent reads per tile
+        VB_TRY(ws.pos_mask.reserve((ix->n_stored + 31) / 32));
+        VB_LAUNCH(position_mask_kernel, static_cast<uint32_t>((ix->n_stored + 255) / 256), 256, 0, sc.s, ix->n_stored, ws.pos_mask.ptr);
+        t.pos_mask = ws.pos_mask.ptr;
+    }
     t.row_norm = ix->code_norm.ptr;
     t.l2 = ix->metric == VB200_METRIC_L2 ? 1u : 0u;
     t.spin_limit = tc_spin_limit();
     t.error_flag = reinterpret_cast<int*>(ws.scalars.ptr + 4);
     void (*kernel)(const TileScan) = nullptr;
-#define VB_TILE(FMT) \
+    int threads = 0;
+#define VB_TILE(FMT)                    \
+    threads = TileFmt<FMT>::THREADS;    \
     kernel = plan.qt == 64 ? tile_scan_kernel<FMT, 64> : (plan.qt == 32 ? tile_scan_kernel<FMT, 32> : tile_scan_kernel<FMT, 16>)
     switch (ix->quant) {
         case VB200_QUANT_SQ8: VB_TILE(ROW_SQ8); break;
@@ -3175,7 +3210,7 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
 #undef VB_TILE
     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), plan.smem));
     const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(max_items, static_cast<uint64_t>(sm_count())));
-    VB_LAUNCH(kernel, grid, TILE_THREADS, plan.smem, t);
+    VB_LAUNCH(kernel, grid, threads, plan.smem, t);
     return 0;
 }
 
@@ -3188,6 +3223,23 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     cudaStream_t st = current_stream();
     const uint32_t dim = ix->dim, nlist = ix->nlist;
     const bool sq8 = ix->quant == VB200_QUANT_SQ8, l2 = ix->metric == VB200_METRIC_L2;
+    // a query's stretch of the score buffer holds its probed lists whichever they are; batches whose stretches
+    // together pass a gigabyte go in slices (a tile launch needs all its queries' stretches: whole searches then)
+    const uint64_t stride = (ix->longest_rows[nprobe] + (plan != nullptr ? 31ull * nprobe : 0) + 31) / 32 * 32;
+    VB_CHECK_ARG(stride < 0xFFFFFFFFull, "the probed lists hold too many rows");
+    uint64_t slice = (uint64_t{256} << 20) / (stride > 0 ? stride : 1);
+    slice = slice < 1 ? 1 : (slice > nq ? nq : slice);
+    if (plan != nullptr && slice < nq) {
+        int64_t bytes = 0;
+        const uint64_t parts = (nq + slice - 1) / slice, each = (nq + parts - 1) / parts;
+        for (uint64_t q0 = 0; q0 < nq; q0 += each) {
+            VB_TRY(ivf_search_scores(ix, queries + q0 * dim, std::min(each, nq - q0), k, kscan, nprobe, rerank, plan,
+                                     bucket_ids != nullptr ? bucket_ids + q0 * nprobe : nullptr, ids + q0 * k, dists + q0 * k));
+            bytes += ix->last_scan_bytes;
+        }
+        ix->last_scan_bytes = ix->last_scanned_bytes = bytes;
+        return 0;
+    }
     // host buffers: [queries | ids | dists] in pinned memory when small
     const size_t q_bytes = nq * dim * sizeof(float), total = nq * k;
     const bool host_q = !is_device_pointer(queries), host_ids = !is_device_pointer(ids), host_d = !is_device_pointer(dists);
@@ -3218,15 +3270,10 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     VB_TRY(ws.probes.reserve(nq * nprobe));
     VB_TRY(ws.pair_base.reserve(nq * nprobe));
     VB_TRY(ws.query_rows.reserve(nq));
-    // a query's stretch of the score buffer holds its probed lists whichever they are; batches whose stretches
-    // together pass a gigabyte go in slices
-    const uint64_t stride = (ix->longest_rows[nprobe] + (plan != nullptr ? 31ull * nprobe : 0) + 31) / 32 * 32;
-    VB_CHECK_ARG(stride < 0xFFFFFFFFull, "the probed lists hold too many rows");
-    uint64_t slice = (uint64_t{256} << 20) / (stride > 0 ? stride : 1);
-    slice = slice < 1 ? 1 : (slice > nq || plan != nullptr ? nq : slice);
     VB_TRY(ws.pair_scores.reserve(slice * stride));
+    const uint32_t qstride8 = plan != nullptr ? plan->pieces * 128 : ix->dpad;   // bytes of an int8 term
     if (sq8) {
-        VB_TRY(ws.qw8.reserve(nq * 3 * ix->dpad));
+        VB_TRY(ws.qw8.reserve(nq * 3 * qstride8));
         VB_TRY(ws.qscale.reserve(nq));
         VB_TRY(ws.qa.reserve(nq));
     }
@@ -3239,10 +3286,17 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         VB_TRY(ws.pair_minima.reserve(nq * stride / 32));
     }
     pp.t = PairTable{ws.pair_base.ptr, ws.query_rows.ptr, stride, ws.pair_scores.ptr, plan != nullptr ? ws.pair_minima.ptr : nullptr};
+    pp.queries = q_dev;
+    pp.dim = dim;
+    if (plan != nullptr && !sq8 && ix->quant != VB200_QUANT_RABITQ) {
+        const bool f32 = ix->quant == VB200_QUANT_FP32;
+        pp.term_dims = plan->pieces * 64;
+        pp.term_fmt = f32 ? ROW_F32 : (ix->quant == VB200_QUANT_BF16 ? ROW_BF16 : ROW_FP16);
+        VB_TRY(ws.tile_terms.reserve(nq * pp.term_dims * (f32 ? 2 : 1)));
+        pp.terms = ws.tile_terms.ptr;
+    }
     if (sq8) {
-        pp.queries = q_dev;
-        pp.dim = dim;
-        pp.dpad = ix->dpad;
+        pp.qstride = qstride8;
         pp.scale = ix->sq_scale.ptr;
         pp.mid = ix->sq_mid.ptr;
         pp.metric = ix->metric;
@@ -3275,7 +3329,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         q_scan = ws.qproc.ptr;
         VB_TRY(ws.qrot.reserve(nq * dim));
         VB_TRY(launch_row_chains(q_dev, nq, dim, ix->rotation.ptr, dim, dim, false, false, ws.qrot.ptr, dim));
-        const uint32_t qstride = (dim + 15) / 16 * 16;
+        const uint32_t qstride = plan != nullptr ? qstride8 : 0;
         if (plan != nullptr) {
             VB_TRY(ws.qw8.reserve(nq * 3 * qstride));
             VB_TRY(ws.qscale.reserve(nq));
@@ -3384,7 +3438,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         if (sq8) {
             g.scan.s.qa += q0;
             g.scan.qscale += q0;
-            g.scan.qw8 += q0 * 3 * ix->dpad;
+            g.scan.qw8 += q0 * 3 * qstride8;
         }
         g.rows_scanned += q0;
         g.rerank_ids += rerank ? q0 * kscan : 0;
@@ -3876,6 +3930,55 @@ ivf_append_row_data(vb200_ivf* ix, const int64_t* ids, const float* rows_dev, ui
     return 0;
 }
 
+// The tensor map through which the tile scan copies stored rows, 128 at a time; false where there is none (SQ8 has a
+// tiled copy instead).
+static bool
+make_row_map(const vb200_ivf* ix, const uint8_t* codes, uint64_t n, CUtensorMap* map) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<Encode>(fn);
+    }();
+    if (encode == nullptr || n == 0 || n >= 0x7FFFFF00ull) {
+        return false;
+    }
+    CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_UINT16;
+    CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B;
+    cuuint64_t extent = ix->dim;
+    cuuint32_t box = 64;
+    switch (ix->quant) {
+        case VB200_QUANT_BF16:
+        case VB200_QUANT_FP16: break;
+        case VB200_QUANT_FP32:
+            type = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+            swizzle = CU_TENSOR_MAP_SWIZZLE_NONE;
+            box = 32;
+            break;
+        case VB200_QUANT_RABITQ:
+            type = CU_TENSOR_MAP_DATA_TYPE_UINT8;
+            swizzle = CU_TENSOR_MAP_SWIZZLE_NONE;
+            extent = ix->code_stride;
+            box = tile_raw_pitch(ix->dim);   // (what it reads past a record is zero)
+            if (box > 240) {
+                return false;
+            }
+            break;
+        default: return false;
+    }
+    const cuuint64_t extents[2] = {extent, n}, strides[1] = {ix->code_stride};
+    const cuuint32_t boxes[2] = {box, 128}, steps[2] = {1, 1};
+    return encode(map, type, 2, const_cast<uint8_t*>(codes), extents, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // What every change of the lists recomputes (SQ8: the norm of every decoded code and the covering
 // balls of every list), then the new arrays replace the old ones.
 static int
@@ -3899,8 +4002,8 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
         VB_TRY(ix->row_max.reserve(2));
         VB_CUDA(cudaMemsetAsync(ix->row_max.ptr, 0, 2 * sizeof(float), current_stream()));
         const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n_new_stored + 7) / 8, 16ull * sm_count()));
-        if (ix->quant != VB200_QUANT_SQ8 && ix->quant != VB200_QUANT_RABITQ) {
-            VB_TRY(new_norm.reserve(n_new_stored));
+        if (ix->quant != VB200_QUANT_SQ8) {
+            VB_TRY(new_norm.reserve(n_new_stored * (ix->quant == VB200_QUANT_RABITQ ? 2 : 1)));
         }
         const uint8_t* codes = new_codes.ptr;
         float *norm = new_norm.ptr, *top = ix->row_max.ptr;
@@ -3932,7 +4035,7 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
     }
     DevBuf<int8_t> new_tiled;
     DevBuf<uint32_t> new_group_off;
-    if (ix->quant == VB200_QUANT_SQ8 && n_new_stored > 0 && dim <= 512) {
+    if (ix->quant == VB200_QUANT_SQ8 && n_new_stored > 0 && dim <= 2048) {
         // the tiled signed copy the tensor-core scan reads (a 128-row tile past a list's end runs into the
         // next list or into 16 groups of padding; those rows are masked by the list length)
         const uint32_t kchunks = (dim + 31) / 32 * 2;
@@ -3957,6 +4060,7 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
         ix->kchunks = kchunks;
     }
     VB_TRY(sync_stream());
+    ix->has_row_map = make_row_map(ix, new_codes.ptr, n_new_stored, &ix->row_map);
     ix->codes_t = std::move(new_tiled);
     ix->group_off = std::move(new_group_off);
     ix->code_norm = std::move(new_norm);

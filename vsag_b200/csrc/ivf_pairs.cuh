@@ -9,6 +9,8 @@
 //   scan_finalize_kernel  a CTA per query: the k best of its scores, exact re-scoring, rerank, labels
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include "block_select.cuh"
 #include "row_scan.cuh"
 
@@ -72,8 +74,13 @@ struct PairsPrepare {
     uint32_t dim, dpad;
     const float *scale, *mid;
     int metric;
-    int8_t* qw8;              // [nq][3][dpad]
+    int8_t* qw8;              // [nq][3][qstride]
+    uint32_t qstride;
     float *qscale, *qa;
+    // fp32 / bf16 / fp16 tiles (null: none): the query as operand rows of the tile scan, [nq][2 or 1][term_dims] 16-bit
+    uint16_t* terms;
+    uint32_t term_dims;       // a multiple of 64, zero past dim
+    int term_fmt;             // ROW_F32: bf16 hi and lo terms, ROW_BF16 / ROW_FP16: the codes
     // The same for the queries from q0 on (dist and scores are the caller's to set).
     PairsPrepare
     from(uint64_t q0) const {
@@ -89,9 +96,12 @@ struct PairsPrepare {
             p.rank += q0 * nprobe;
         }
         if (p.qw8 != nullptr) {
-            p.qw8 += q0 * 3 * dpad;
+            p.qw8 += q0 * 3 * qstride;
             p.qscale += q0;
             p.qa += q0;
+        }
+        if (p.terms != nullptr) {
+            p.terms += q0 * term_dims * (term_fmt == ROW_F32 ? 2 : 1);
         }
         return p;
     }
@@ -203,10 +213,28 @@ pairs_prepare_kernel(const PairsPrepare p) {
     if (threadIdx.x == 0) {
         p.t.rows[q] = run;
     }
+    const float* src = p.queries + q * p.dim;
+    if (p.terms != nullptr) {
+        uint16_t* t = p.terms + q * p.term_dims * (p.term_fmt == ROW_F32 ? 2 : 1);
+        for (uint32_t e = threadIdx.x; e < p.term_dims; e += PAIR_THREADS) {
+            if (p.term_fmt == ROW_F32) {
+                // place e of a piece of 64: unit e / 8 holds dimensions 4 u .. + 3 and 32 + 4 u .. + 3 (tile_scan_kernel)
+                const uint32_t u = (e & 63u) >> 3, i = e & 7u;
+                const uint32_t d = (e & ~63u) + (i < 4 ? 4 * u + i : 28 + 4 * u + i);
+                const float v = d < p.dim ? __ldg(src + d) : 0.f;
+                const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+                t[e] = __bfloat16_as_ushort(hi);
+                t[p.term_dims + e] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(hi)));
+            } else if (e >= p.dim) {
+                t[e] = 0;
+            } else {
+                t[e] = p.term_fmt == ROW_BF16 ? half_encode<SCAN_FMT_BF16>(__ldg(src + e)) : half_encode<SCAN_FMT_FP16>(__ldg(src + e));
+            }
+        }
+    }
     if (p.qw8 == nullptr) {
         return;
     }
-    const float* src = p.queries + q * p.dim;
     float qq = 0.f, qm = 0.f, wmax = 0.f;
     for (uint32_t d = threadIdx.x; d < p.dim; d += PAIR_THREADS) {
         const float v = __ldg(src + d);
@@ -218,16 +246,16 @@ pairs_prepare_kernel(const PairsPrepare p) {
     qm = pair_block_sum(qm, part);
     wmax = pair_block_max(wmax, part);
     const float s = wmax > 0.f && wmax < INFINITY ? wmax / 127.0f : 1.0f;
-    int8_t* t = p.qw8 + q * 3 * p.dpad;
-    for (uint32_t d = threadIdx.x; d < p.dpad; d += PAIR_THREADS) {
+    int8_t* t = p.qw8 + q * 3 * p.qstride;
+    for (uint32_t d = threadIdx.x; d < p.qstride; d += PAIR_THREADS) {
         const float u = d < p.dim ? __ldg(src + d) * __ldg(p.scale + d) / s : 0.f;
         const float t1 = fminf(fmaxf(rintf(u), -127.f), 127.f);
         const float v2 = (u - t1) * 254.0f;
         const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
         const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
         t[d] = static_cast<int8_t>(static_cast<int>(t1));
-        t[p.dpad + d] = static_cast<int8_t>(static_cast<int>(t2));
-        t[2 * p.dpad + d] = static_cast<int8_t>(static_cast<int>(t3));
+        t[p.qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
+        t[2 * p.qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
     }
     if (threadIdx.x == 0) {
         p.qscale[q] = s;
@@ -288,9 +316,11 @@ rabitq_query_kernel(const float* __restrict__ t, uint32_t dim, const float* __re
         const float v2 = (u - t1) * 254.0f;
         const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
         const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
-        terms[d] = static_cast<int8_t>(static_cast<int>(t1));
-        terms[qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
-        terms[2 * qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
+        // bit 8 b + s of 32 sign bits becomes byte 4 s + b of the tile scan's operand
+        const uint32_t at = (d & ~31u) + (d & 7u) * 4 + ((d & 31u) >> 3);
+        terms[at] = static_cast<int8_t>(static_cast<int>(t1));
+        terms[qstride + at] = static_cast<int8_t>(static_cast<int>(t2));
+        terms[2 * qstride + at] = static_cast<int8_t>(static_cast<int>(t3));
         n1 += static_cast<int>(t1);
         n2 += static_cast<int>(t2);
         n3 += static_cast<int>(t3);
@@ -312,7 +342,7 @@ rabitq_query_kernel(const float* __restrict__ t, uint32_t dim, const float* __re
     }
 }
 
-// Squared norms of the stored rows and the largest norm (RaBitQ: of the norms and norm / |error| in the records;
+// Squared norms of the stored rows and the largest norm (RaBitQ: |x|^2 and -2 |x| / error, largest norm / |error|;
 // SQ8: of the norms already in `norm`).  A warp per row; top[] is cleared by the caller.
 template <int FMT>
 __global__ void __launch_bounds__(256)
@@ -327,9 +357,10 @@ record_norms_kernel(const uint8_t* __restrict__ codes, uint64_t n, uint32_t dim,
                 most = fmaxf(most, norm[r]);
             } else {
                 const float* tail = reinterpret_cast<const float*>(codes + r * stride + ((dim + 7) / 8 + 3) / 4 * 4);
-                const float err = fabsf(tail[1]);
+                const float err = fabsf(tail[1]) < 1e-5f ? (tail[1] >= 0.f ? 1.0f : -1.0f) : tail[1];
                 most = fmaxf(most, tail[0]);
-                gain = fmaxf(gain, tail[0] / (err < 1e-5f ? 1.0f : err));
+                gain = fmaxf(gain, tail[0] / fabsf(err));
+                reinterpret_cast<float2*>(norm)[r] = make_float2(tail[0] * tail[0], -2.0f * tail[0] / err);
             }
         }
     } else {

@@ -8,67 +8,80 @@
 // exactly).  Nothing is selected here, so no bounds, no buffers and no second phase are needed, and the kernel's
 // time is that of reading the lists once (a few percent of them are probed by more queries than one item holds).
 //
-// The rows keep their stored form; the loader warps turn a piece of 128 bytes of operand per row into the layout
-// the MMA descriptors describe on its way to shared memory.  That is the 128-byte swizzle -- a row's piece is one
-// 128-byte line, its 16-byte units permuted by the row number -- because eight lanes can then read one line of a
-// row and write one line of the operand: with unswizzled cores either the loads touch a line per lane or the stores
-// hit the same banks, and the kernel spent 82 % of its cycles on those wavefronts (500 us instead of 280 for
-// 1000 queries against 32 lists each of 500k x 128 fp32).  The codecs:
-//   fp32        two bf16 terms x = hi + lo; hi*hi + lo*hi and hi*lo are accumulated (the dropped terms are below
-//               2^-16 |x||q|)
-//   bf16, fp16  the codes as they are; every product is exact in fp32
-//   sq8         code - 128 as signed bytes against three int8 terms of the query's weights, exact int32 sums
-//   rabitq      the sign bits as bytes 0 / 1 against three int8 terms of the query; sum over set bits = (sum of all
-//               terms + signed sum) / 2
-// Each loader thread holds its part of the next two or three pieces in registers while it converts the current one,
-// across tiles and items, so 64 KB or more per SM are always in flight.
+// Every role of the CTA runs on warps of its own and is a few steps ahead of the one it feeds: one takes items from
+// the queue and copies rows, four gather the next item's queries, eight convert where the codec needs it, one thread
+// issues the MMAs, eight warps drain them.  (With the loads, the conversions and the gathering of an item on the same
+// warps, and the item's constants read by the epilogue, the kernel waited for one latency after another: 390 to
+// 560 us instead of TILE_F32_US for 1000 queries against 32 lists each of 500k x 128 fp32.)  How rows become operands:
+//   fp32        two bf16 terms x = hi + lo, made in place in shared memory; hi*hi + lo*hi and hi*lo are accumulated
+//               (the dropped terms are below 2^-16 |x||q|)
+//   bf16, fp16  the codes as they are (TMA with the 128-byte swizzle); every product is exact in fp32
+//   sq8         the tiled copy of the codes as signed bytes code - 128, against three int8 terms of the query's
+//               weights: exact int32 sums
+//   rabitq      the sign bits as bytes 0 / 1, spread in shared memory, against three int8 terms of the query; sum over
+//               set bits = (sum of all terms + signed sum) / 2
 #pragma once
+
+#include <cuda.h>   // CUtensorMap
 
 #include "ivf_pairs.cuh"
 #include "ivf_scan_tc.cuh"
 
 namespace vb200 {
 
-constexpr int TILE_LOAD_WARPS = 8;
-constexpr int TILE_LOADERS = 32 * TILE_LOAD_WARPS;
-constexpr int TILE_EPI_WARPS = 8;
-constexpr int TILE_THREADS = 32 * (TILE_EPI_WARPS + 1 + TILE_LOAD_WARPS);   // warps 0-7 epilogue, 8 MMA, then the loaders
+constexpr int TILE_EPI_WARPS = 8;                           // warps 0-7; 8 issues the MMAs, 9 copies rows,
+constexpr int TILE_QUERY_WARPS = 4;                         // 10-13 gather queries,
+constexpr int TILE_CONV_WARPS = 8;                          // 14-21 convert
 constexpr uint32_t TILE_PIECE = 128;                        // operand bytes per row and piece
 constexpr uint32_t TILE_A_TERM = 128 * TILE_PIECE;          // 16 KiB
-constexpr uint32_t TILE_MAX_STAGES = 6;
+constexpr uint32_t TILE_MAX_STAGES = 8;
+constexpr uint32_t TILE_DESCS = 4;                          // items described ahead
 constexpr uint32_t TILE_ACC_COLS = 256;                     // tensor-memory columns per accumulator, two of them
 
 // How a codec becomes MMA operands.
 template <int FMT>
 struct TileFmt {
     static constexpr bool INT8 = FMT == ROW_SQ8 || FMT == ROW_RABITQ;
+    static constexpr bool CONVERT = FMT == ROW_F32 || FMT == ROW_RABITQ;
     static constexpr uint32_t A_TERMS = FMT == ROW_F32 ? 2 : 1;
     static constexpr uint32_t B_TERMS = INT8 ? 3 : (FMT == ROW_F32 ? 2 : 1);
     static constexpr uint32_t PIECE_DIMS = INT8 ? 128 : 64;
+    static constexpr uint32_t STAGE = A_TERMS * TILE_A_TERM;
+    static constexpr int THREADS = 32 * (TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS + (CONVERT ? TILE_CONV_WARPS : 0));
 };
 
 // Lists of very different lengths are the rule (a list that many queries probe is often a long one): an item is at
 // most TILE_SEGMENT rows of a list, so that no CTA is left with one long list at the end.
 constexpr uint32_t TILE_SEGMENT = 1024;
 
-struct TileItem {
-    uint32_t list, pair0, nqt, row0;   // rows row0 .. row0 + TILE_SEGMENT of the list
+struct alignas(16) TileItem {
+    uint32_t lbeg, len, pair0, nqt;   // rows lbeg .. lbeg + len against pairs pair0 .. pair0 + nqt
+    uint32_t row0, goff, pad0, pad1;  // their number within the list, and their first 8-row group (SQ8)
+};
+
+struct alignas(16) TilePair {
+    uint32_t q, pad;
+    uint64_t out;                     // where the scores of the (query, list) pair begin
 };
 
 struct TileScan {
-    ScanParams s;               // rows, list_off, filter, constants; queries (RaBitQ: processed)
+    CUtensorMap map;            // the stored rows (not SQ8)
+    ScanParams s;               // constants; queries (RaBitQ: processed)
     PairTable t;
-    uint32_t nprobe;
     const TileItem* items;
-    const uint32_t* n_items;    // [1]
-    const uint32_t* pair_ids;   // pairs (query * nprobe + rank) grouped by list
+    uint32_t* queue;            // [0] number of items, [1] the next one to take
+    const TilePair* pairs;      // grouped by list
     uint32_t pieces;            // of a row: dimensions over PIECE_DIMS, rounded up
     uint32_t stages, b_bufs;
-    uint32_t qstride;           // int8 terms: bytes per term
-    const int8_t* qw8;          // [nq][3][qstride]
-    const float* qscale;        // [nq]
+    uint32_t raw_pitch;         // RaBitQ: bytes between rows of sign bits in shared memory
+    uint32_t kchunks;           // SQ8: 16-byte cores per row of the tiled copy
+    const int8_t* codes_t;      // SQ8: the tiled copy
+    const unsigned char* terms; // [nq][B_TERMS][pieces * 128 bytes] the queries' operand rows
+    const float* qscale;        // [nq] of the int8 terms
     const int32_t* qsum;        // RaBitQ: [nq][4] sums of the three terms
-    const float* row_norm;      // L2 over fp32 / bf16 / fp16 rows: |x|^2 by position (the score leaves |q|^2 out)
+    const float* row_norm;      // |x|^2 by position (L2 over fp32 / bf16 / fp16 rows; the score leaves |q|^2 out);
+                                // RaBitQ: pairs |x|^2, -2 |x| / error
+    const uint32_t* pos_mask;   // bit by position: the id filter rejects the row; or null
     uint32_t l2;
     uint32_t spin_limit;
     int* error_flag;
@@ -87,9 +100,12 @@ struct TileGroup {
     uint32_t* pair_off;       // [nlist]
     uint32_t* item_off;       // [nlist]
     uint32_t* list_pairs;     // [nlist] the counts, kept
-    uint32_t* n_items;
-    uint32_t* pair_ids;
+    uint32_t* queue;          // [0] number of items, [1] cleared
+    TilePair* tile_pairs;
     TileItem* items;
+    uint32_t nprobe;
+    PairTable t;
+    const uint32_t* group_off; // SQ8 or null
 };
 
 __global__ void __launch_bounds__(1024)
@@ -138,7 +154,8 @@ tile_places_kernel(const TileGroup g) {
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        *g.n_items = carry[1];
+        g.queue[0] = carry[1];
+        g.queue[1] = 0;
     }
 }
 
@@ -149,17 +166,20 @@ tile_scatter_kernel(const TileGroup g) {
         const int32_t l = __ldg(g.probes + e);
         const uint32_t r = __ldg(g.rank + e);
         if (r != 0xFFFFFFFFu) {
-            g.pair_ids[__ldg(g.pair_off + l) + r] = e;
+            const uint32_t q = e / g.nprobe;
+            g.tile_pairs[__ldg(g.pair_off + l) + r] = TilePair{q, 0u, q * g.t.stride + __ldg(g.t.base + e)};
         }
     }
     if (e < g.nlist) {
         const uint32_t n = g.list_pairs[e];
         TileItem* dst = g.items + g.item_off[e];
         const uint32_t p0 = g.pair_off[e];
-        const uint32_t len = n > 0 ? __ldg(g.list_off + e + 1) - __ldg(g.list_off + e) : 0u;
+        const uint32_t lbeg = __ldg(g.list_off + e);
+        const uint32_t len = n > 0 ? __ldg(g.list_off + e + 1) - lbeg : 0u;
+        const uint32_t goff = g.group_off != nullptr ? __ldg(g.group_off + e) : 0u;
         for (uint32_t row0 = 0; row0 < len; row0 += TILE_SEGMENT) {
             for (uint32_t i = 0; i * g.qt < n; ++i) {
-                *dst++ = TileItem{e, p0 + i * g.qt, min(g.qt, n - i * g.qt), row0};
+                *dst++ = TileItem{lbeg + row0, min(len - row0, TILE_SEGMENT), p0 + i * g.qt, min(g.qt, n - i * g.qt), row0, goff + row0 / 8, 0u, 0u};
             }
         }
     }
@@ -167,22 +187,19 @@ tile_scatter_kernel(const TileGroup g) {
 
 // ---- the kernel -----------------------------------------------------------------------------
 struct TileShared {
-    uint64_t full[TILE_MAX_STAGES], freed[TILE_MAX_STAGES];
-    uint64_t b_full[2], b_free[2];
+    uint64_t full[TILE_MAX_STAGES], freed[TILE_MAX_STAGES];   // operand stages
+    uint64_t raw_full[TILE_MAX_STAGES], raw_free[2];          // rows as they are stored, before conversion
+    uint64_t desc_full[TILE_DESCS], desc_free[TILE_DESCS];
+    uint64_t item_full[2], item_free[2];                      // B operand and constants of an item
+    uint64_t b_free[2];
     uint64_t acc_full[2], acc_free[2];
     uint32_t tmem_base, failed;
-    // where the running item's scores go and its queries' constants: a copy per epilogue warp, which therefore never
-    // wait for one another
-    uint64_t out[TILE_EPI_WARPS][64];
-    float c0[TILE_EPI_WARPS][64], c1[TILE_EPI_WARPS][64];
-    int32_t t1[TILE_EPI_WARPS][64], t2[TILE_EPI_WARPS][64], t3[TILE_EPI_WARPS][64];
+    TileItem desc[TILE_DESCS];
+    // two items deep: where the scores of the item's queries go and their constants
+    alignas(16) uint64_t out[2][64];
+    float c0[2][64], c1[2][64];
+    int32_t t1[2][64], t2[2][64], t3[2][64];
 };
-
-// Instruction descriptor of kind::f16 with fp16 operands (bf16: umma_idesc_bf16).
-__host__ __device__ constexpr uint32_t
-umma_idesc_f16(uint32_t m, uint32_t n) {
-    return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
 
 // Two bf16 terms of eight values: x = hi + lo.
 __device__ __forceinline__ void
@@ -216,66 +233,14 @@ swizzled(uint32_t r, uint32_t kc) {
     return r * 128 + ((kc ^ (r & 7u)) << 4);
 }
 
-// 16 sign bits -> 16 bytes of 0 / 1.
-__device__ __forceinline__ uint4
-spread_bits16(uint32_t b) {
-    auto four = [](uint32_t n) { return (n * 0x00204081u) & 0x01010101u; };
-    return make_uint4(four(b & 15u), four((b >> 4) & 15u), four((b >> 8) & 15u), four((b >> 12) & 15u));
+// One box of a tiled tensor map -> shared memory, completion counted in bytes on `bar`.
+__device__ __forceinline__ void
+tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
 }
-
-// One 16-byte operand unit per A term of row `row` (a code record), k-core `kc` of piece `piece`.
-template <int FMT>
-struct TileUnit {
-    uint4 raw[FMT == ROW_F32 ? 2 : 1];
-    uint2 bits;   // RaBitQ
-    __device__ __forceinline__ void
-    load(const uint8_t* row, bool valid, uint32_t piece, uint32_t kc, uint32_t dim) {
-        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        if (FMT == ROW_F32) {
-            const uint32_t d0 = piece * 64 + kc * 8;
-            const uint4* src = reinterpret_cast<const uint4*>(row + static_cast<size_t>(d0) * 4);
-            raw[0] = valid && d0 < dim ? __ldg(src) : zero;
-            raw[FMT == ROW_F32 ? 1 : 0] = valid && d0 + 4 < dim ? __ldg(src + 1) : zero;
-        } else if (FMT == ROW_RABITQ) {
-            // (64 sign bits per thread: see tile_scan_kernel)
-        } else {
-            const uint32_t per = FMT == ROW_SQ8 ? 16 : 8;
-            const uint32_t d0 = piece * (8 * per) + kc * per;
-            raw[0] = valid && d0 < dim ? __ldg(reinterpret_cast<const uint4*>(row + static_cast<size_t>(d0) * (FMT == ROW_SQ8 ? 1 : 2))) : zero;
-        }
-    }
-    __device__ __forceinline__ void
-    store(unsigned char* dst, uint32_t piece, uint32_t kc, uint32_t dim) const {
-        if (FMT == ROW_F32) {
-            float x[8];
-            const uint4 a = raw[0], b = raw[FMT == ROW_F32 ? 1 : 0];
-            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-            const uint32_t d0 = piece * 64 + kc * 8;
-#pragma unroll
-            for (uint32_t i = 0; i < 8; ++i) {
-                x[i] = d0 + i < dim ? __uint_as_float(w[i]) : 0.f;
-            }
-            uint4 hi, lo;
-            split_bf16x8(x, hi, lo);
-            *reinterpret_cast<uint4*>(dst) = hi;
-            *reinterpret_cast<uint4*>(dst + TILE_A_TERM) = lo;
-        } else if (FMT == ROW_SQ8) {
-            *reinterpret_cast<uint4*>(dst) = make_uint4(raw[0].x ^ 0x80808080u, raw[0].y ^ 0x80808080u, raw[0].z ^ 0x80808080u,
-                                                        raw[0].w ^ 0x80808080u);
-        } else {
-            uint32_t w[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
-            const uint32_t d0 = piece * 64 + kc * 8;
-            if (d0 + 8 > dim) {   // bytes past the last dimension are not defined
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) {
-                    const uint32_t keep = (d0 + 2 * i < dim ? 0x0000FFFFu : 0u) | (d0 + 2 * i + 1 < dim ? 0xFFFF0000u : 0u);
-                    w[i] &= keep;
-                }
-            }
-            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-    }
-};
 
 // 8 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void
@@ -284,6 +249,14 @@ tmem_load_8(uint32_t taddr, uint32_t (&r)[8]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr)
                  : "memory");
+}
+
+// Smallest of the warp's fp32 bit patterns; NaNs do not take part (all NaN: NaN).
+__device__ __forceinline__ float
+warp_min_f32(uint32_t bits) {
+    float out;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(out) : "f"(__uint_as_float(bits)));
+    return out;
 }
 
 // A warp's wait: one lane polls (32 lanes polling one barrier are 32 operations on it, and eight warps of them kept
@@ -309,14 +282,23 @@ tile_publish(uint64_t* bar, uint32_t lane) {
     }
 }
 
+// kind::f16 (fp16 or bf16 operands) and kind::i8 instruction descriptors, M 128.
+template <int FMT>
+__device__ __forceinline__ uint32_t
+tile_idesc(uint32_t n) {
+    if (TileFmt<FMT>::INT8) {
+        return umma_idesc_s8(128, n);
+    }
+    return FMT == ROW_FP16 ? umma_idesc_f16(128, n) : umma_idesc_bf16(128, n);
+}
+
 // QT queries per item at most (16, 32 or 64).
 template <int FMT, int QT>
-__global__ void __launch_bounds__(TILE_THREADS, 1)
-tile_scan_kernel(const TileScan p) {
+__global__ void __launch_bounds__(TileFmt<FMT>::THREADS, 1)
+tile_scan_kernel(const __grid_constant__ TileScan p) {
     using F = TileFmt<FMT>;
-    constexpr uint32_t N = F::B_TERMS * QT;                  // rows of B, columns of the accumulator
-    constexpr uint32_t STAGE = F::A_TERMS * TILE_A_TERM;
-    constexpr uint32_t B_PIECE = N * TILE_PIECE;
+    constexpr uint32_t STAGE = F::STAGE;
+    constexpr uint32_t B_PIECE = F::B_TERMS * QT * TILE_PIECE;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ TileShared sh;
     // the swizzle permutes by address bits: blocks start on 1 KiB
@@ -325,14 +307,22 @@ tile_scan_kernel(const TileScan p) {
     const uint32_t stages = p.stages, pieces = p.pieces, dim = p.s.dim;
     unsigned char* const b_smem = smem + stages * STAGE;
     const uint32_t b_bytes = pieces * B_PIECE;
+    unsigned char* const raw_smem = b_smem + p.b_bufs * b_bytes;
     const volatile uint32_t* failed = &sh.failed;
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < stages; ++s) {
-            mbar_init(&sh.full[s], TILE_LOAD_WARPS);
+            mbar_init(&sh.full[s], F::CONVERT ? TILE_CONV_WARPS : 1);
             mbar_init(&sh.freed[s], 1);
+            mbar_init(&sh.raw_full[s], 1);
+        }
+        for (uint32_t i = 0; i < TILE_DESCS; ++i) {
+            mbar_init(&sh.desc_full[i], 1);
+            mbar_init(&sh.desc_free[i], TILE_EPI_WARPS + 1 + TILE_QUERY_WARPS + (F::CONVERT ? TILE_CONV_WARPS : 0));
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&sh.b_full[i], TILE_LOAD_WARPS);
+            mbar_init(&sh.raw_free[i], TILE_CONV_WARPS);
+            mbar_init(&sh.item_full[i], TILE_QUERY_WARPS);
+            mbar_init(&sh.item_free[i], TILE_EPI_WARPS);
             mbar_init(&sh.b_free[i], 1);
             mbar_init(&sh.acc_full[i], 1);
             mbar_init(&sh.acc_free[i], TILE_EPI_WARPS);
@@ -347,203 +337,142 @@ tile_scan_kernel(const TileScan p) {
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = sh.tmem_base;
-    const uint32_t n_items = *p.n_items;
     bool ok = true;
-
-    if (warp > TILE_EPI_WARPS) {
-        // ---------------- loaders: code records -> operands ----------------
-        const uint32_t lt = threadIdx.x - 32 * (TILE_EPI_WARPS + 1);
-        const uint32_t lwarp = lt >> 5;
-        constexpr uint32_t SETS = FMT == ROW_F32 ? 2 : 4;    // pieces requested ahead, in registers
-        constexpr uint32_t UNITS = 1024 / TILE_LOADERS;      // 16-byte operand units per thread and piece
-        // Where the loads are; items are dealt round-robin, and a cursor reads the next item's description while it
-        // works through the current one.
-        struct Cursor {
-            uint32_t item, lbeg, len, pair0, nqt, next_lbeg, next_len, next_pair0, next_nqt, r0, piece;
-        };
-        auto describe = [&](uint32_t item, uint32_t& lbeg, uint32_t& len, uint32_t& pair0, uint32_t& nqt) {
-            lbeg = len = pair0 = nqt = 0;
-            if (item < n_items) {
-                const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
-                lbeg = __ldg(p.s.list_off + d.x) + d.w;
-                len = min(__ldg(p.s.list_off + d.x + 1) - lbeg, TILE_SEGMENT);
-                pair0 = d.y;
-                nqt = d.z;
-            }
-        };
-        auto start = [&](Cursor& c) {
-            c.item = blockIdx.x;
-            c.r0 = c.piece = 0;
-            describe(c.item, c.lbeg, c.len, c.pair0, c.nqt);
-            describe(c.item + gridDim.x, c.next_lbeg, c.next_len, c.next_pair0, c.next_nqt);
-        };
-        auto advance = [&](Cursor& c) {
-            if (++c.piece < pieces) {
-                return;
-            }
-            c.piece = 0;
-            c.r0 += 128;
-            if (c.r0 < c.len) {
-                return;
-            }
-            c.r0 = 0;
-            c.item += gridDim.x;
-            c.lbeg = c.next_lbeg;
-            c.len = c.next_len;
-            c.pair0 = c.next_pair0;
-            c.nqt = c.next_nqt;
-            describe(c.item + gridDim.x, c.next_lbeg, c.next_len, c.next_pair0, c.next_nqt);
-        };
-        // eight lanes on the line of a row, four rows per warp and step
-        const uint32_t kc = lane & 7u, rr = lwarp * (128 / TILE_LOAD_WARPS) + (lane >> 3);
-        TileUnit<FMT> u[SETS][UNITS];
-        auto request = [&](const Cursor& c, TileUnit<FMT> (&set)[UNITS]) {
-            if (c.item >= n_items) {
-                return;
-            }
-            const uint8_t* rows = p.s.codes + static_cast<uint64_t>(c.lbeg) * p.s.code_stride;
-            if (FMT == ROW_RABITQ) {
-                // a thread takes 64 dimensions of one row: eight bytes of sign bits, four k-cores
-                const uint32_t r = c.r0 + (lt >> 1), part = lt & 1u;
-                set[0].bits = r < c.len && c.piece * 128 + part * 64 < dim
-                                  ? __ldg(reinterpret_cast<const uint2*>(rows + static_cast<uint64_t>(r) * p.s.code_stride + c.piece * 16 + part * 8))
-                                  : make_uint2(0u, 0u);
-                return;
-            }
-#pragma unroll
-            for (uint32_t j = 0; j < UNITS; ++j) {
-                const uint32_t r = c.r0 + rr + j * 4;
-                set[j].load(rows + static_cast<uint64_t>(r < c.len ? r : 0u) * p.s.code_stride, r < c.len, c.piece, kc, dim);
-            }
-        };
-        uint32_t stage = 0, phase = 0, filled = 0, n_mine = 0;
-        auto load_queries = [&](const Cursor& c) -> bool {
-            const uint32_t buf = p.b_bufs == 2 ? n_mine & 1u : 0u;
-            if (n_mine >= p.b_bufs) {
-                // (use number n_mine / b_bufs of this buffer: the use before it must have been multiplied)
-                if (!tile_wait(&sh.b_free[buf], ((n_mine / p.b_bufs) - 1u) & 1u, failed, p.spin_limit, lane)) {
-                    return false;
-                }
-            }
-            unsigned char* bd = b_smem + buf * b_bytes;
-            const uint32_t per_row = pieces * 8;             // units of a row of B
-            if (F::INT8) {
-#pragma unroll 4
-                for (uint32_t i = lt; i < N * per_row; i += TILE_LOADERS) {
-                    const uint32_t r = i / per_row, k = i - r * per_row;
-                    const uint32_t term = r / QT, qi = r - term * QT;
-                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (qi < c.nqt && k * 16 < p.qstride) {
-                        const uint32_t q = __ldg(p.pair_ids + c.pair0 + qi) / p.nprobe;
-                        v = __ldg(reinterpret_cast<const uint4*>(p.qw8 + (static_cast<uint64_t>(q) * 3 + term) * p.qstride + k * 16));
-                    }
-                    *reinterpret_cast<uint4*>(bd + (k >> 3) * B_PIECE + swizzled(r, k & 7u)) = v;
-                }
-            } else {
-#pragma unroll 2
-                for (uint32_t i = lt; i < QT * per_row; i += TILE_LOADERS) {
-                    const uint32_t qi = i / per_row, k = i - qi * per_row;
-                    float x[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        x[e] = 0.f;
-                    }
-                    if (qi < c.nqt) {
-                        const uint32_t q = __ldg(p.pair_ids + c.pair0 + qi) / p.nprobe;
-                        const float* src = p.s.queries + static_cast<uint64_t>(q) * dim + k * 8;
-#pragma unroll
-                        for (uint32_t e = 0; e < 8; ++e) {
-                            x[e] = k * 8 + e < dim ? __ldg(src + e) : 0.f;
-                        }
-                    }
-                    unsigned char* dst = bd + (k >> 3) * B_PIECE + swizzled(qi, k & 7u);
-                    if (FMT == ROW_F32) {
-                        uint4 hi, lo;
-                        split_bf16x8(x, hi, lo);
-                        *reinterpret_cast<uint4*>(dst) = hi;
-                        *reinterpret_cast<uint4*>(dst + QT * 128) = lo;
-                    } else {
-                        constexpr int HF = FMT == ROW_BF16 ? SCAN_FMT_BF16 : SCAN_FMT_FP16;
-                        uint32_t w[4];
-#pragma unroll
-                        for (uint32_t e = 0; e < 4; ++e) {
-                            const uint32_t lo = qi < c.nqt && k * 8 + 2 * e < dim ? half_encode<HF>(x[2 * e]) : 0u;
-                            const uint32_t hi = qi < c.nqt && k * 8 + 2 * e + 1 < dim ? half_encode<HF>(x[2 * e + 1]) : 0u;
-                            w[e] = lo | (hi << 16);
-                        }
-                        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                }
-            }
-            tile_publish(&sh.b_full[buf], lane);
-            ++n_mine;
-            return true;
-        };
-        Cursor now, ahead;
-        start(now);
-        start(ahead);
-#pragma unroll
-        for (uint32_t s = 0; s < SETS; ++s) {
-            request(ahead, u[s]);
-            if (ahead.item < n_items) {
-                advance(ahead);
-            }
+    // The item number n of this CTA; false at the end of the queue or when another role has failed.
+    auto next_item = [&](uint32_t n, TileItem& it) -> bool {
+        const uint32_t slot = n % TILE_DESCS;
+        ok = tile_wait(&sh.desc_full[slot], (n / TILE_DESCS) & 1u, failed, p.spin_limit, lane);
+        if (!ok) {
+            return false;
         }
-        while (now.item < n_items && ok) {
-#pragma unroll
-            for (uint32_t s = 0; s < SETS; ++s) {
-                if (now.item >= n_items || !ok) {
-                    break;
-                }
-                if (now.r0 == 0 && now.piece == 0) {
-                    ok = load_queries(now);
-                }
-                if (ok && filled >= stages) {
-                    ok = tile_wait(&sh.freed[stage], phase ^ 1u, failed, p.spin_limit, lane);
-                }
+        it = sh.desc[slot];
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive(&sh.desc_free[slot]);
+        }
+        return it.len != 0;
+    };
+
+    if (warp == TILE_EPI_WARPS + 1) {
+        // ---------------- the work queue and the copies of rows ----------------
+        const uint32_t n_items = p.queue[0];
+        uint32_t stage = 0, phase = 0, filled = 0, raw = 0;
+        auto fetch = [&](uint32_t i) -> TileItem {
+            TileItem it{};
+            if (i < n_items) {
+                const uint4* src = reinterpret_cast<const uint4*>(p.items + i);
+                const uint4 a = __ldg(src), b = __ldg(src + 1);
+                it = TileItem{a.x, a.y, a.z, a.w, b.x, b.y, 0u, 0u};
+            }
+            return it;
+        };
+        auto ticket = [&]() -> uint32_t {   // (the same number for all lanes)
+            uint32_t t = 0;
+            if (lane == 0) {
+                t = atomicAdd(p.queue + 1, 1u);
+            }
+            return t;
+        };
+        // the next item's description and the ticket after it are under way while an item's rows are copied
+        TileItem next = fetch(__shfl_sync(0xffffffffu, ticket(), 0));
+        uint32_t after = ticket();
+        for (uint32_t n = 0;; ++n) {
+            const uint32_t slot = n % TILE_DESCS;
+            if (n >= TILE_DESCS) {
+                ok = tile_wait(&sh.desc_free[slot], (n / TILE_DESCS - 1u) & 1u, failed, p.spin_limit, lane);
                 if (!ok) {
                     break;
                 }
-                unsigned char* dst = smem + stage * STAGE;
+            }
+            const TileItem it = next;
+            if (lane == 0) {
+                sh.desc[slot] = it;
+                mbar_arrive(&sh.desc_full[slot]);
+            }
+            if (it.len == 0) {
+                break;
+            }
+            next = fetch(__shfl_sync(0xffffffffu, after, 0));
+            after = ticket();
+            for (uint32_t r0 = 0; r0 < it.len && ok; r0 += 128) {
                 if (FMT == ROW_RABITQ) {
-                    const uint32_t r = lt >> 1, part = lt & 1u;
-                    const uint2 bits = u[s][0].bits;
-                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4)) = spread_bits16(bits.x & 0xFFFFu);
-                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4 + 1)) = spread_bits16(bits.x >> 16);
-                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4 + 2)) = spread_bits16(bits.y & 0xFFFFu);
-                    *reinterpret_cast<uint4*>(dst + swizzled(r, part * 4 + 3)) = spread_bits16(bits.y >> 16);
-                } else {
-#pragma unroll
-                    for (uint32_t j = 0; j < UNITS; ++j) {
-                        u[s][j].store(dst + swizzled(rr + j * 4, kc), now.piece, kc, dim);
+                    // the sign bits of 128 rows at once
+                    const uint32_t buf = raw & 1u;
+                    if (raw >= 2) {
+                        ok = tile_wait(&sh.raw_free[buf], (raw / 2 - 1u) & 1u, failed, p.spin_limit, lane);
+                    }
+                    if (ok && lane == 0) {
+                        mbar_expect_tx(&sh.raw_full[buf], 128 * p.raw_pitch);
+                        tma_load_2d(raw_smem + buf * 128 * p.raw_pitch, &p.map, 0, it.lbeg + r0, &sh.raw_full[buf]);
+                    }
+                    ++raw;
+                    continue;
+                }
+                for (uint32_t piece = 0; piece < pieces; ++piece) {
+                    if (filled >= stages) {
+                        ok = tile_wait(&sh.freed[stage], phase ^ 1u, failed, p.spin_limit, lane);
+                        if (!ok) {
+                            break;
+                        }
+                    }
+                    unsigned char* dst = smem + stage * STAGE;
+                    if (FMT == ROW_SQ8) {
+                        // the tiled signed copy: of every 8-row group its cores of this piece, 16 groups
+                        const uint32_t cores = min(8u, p.kchunks - piece * 8);
+                        if (lane == 0) {
+                            mbar_expect_tx(&sh.full[stage], 16 * cores * 128);
+                        }
+                        __syncwarp();
+                        if (lane < 16) {
+                            const int8_t* src = p.codes_t + (static_cast<uint64_t>(it.goff + r0 / 8 + lane) * p.kchunks + piece * 8) * 128;
+                            bulk_copy_g2s(dst + lane * 1024, src, cores * 128, &sh.full[stage]);
+                        }
+                    } else if (lane == 0) {
+                        uint64_t* bar = F::CONVERT ? &sh.raw_full[stage] : &sh.full[stage];
+                        mbar_expect_tx(bar, STAGE);
+                        if (FMT == ROW_F32) {
+                            tma_load_2d(dst, &p.map, piece * 64, it.lbeg + r0, bar);
+                            tma_load_2d(dst + TILE_A_TERM, &p.map, piece * 64 + 32, it.lbeg + r0, bar);
+                        } else {
+                            tma_load_2d(dst, &p.map, piece * 64, it.lbeg + r0, bar);
+                        }
+                    }
+                    ++filled;
+                    if (++stage == stages) {
+                        stage = 0;
+                        phase ^= 1u;
                     }
                 }
-                tile_publish(&sh.full[stage], lane);
-                request(ahead, u[s]);
-                if (ahead.item < n_items) {
-                    advance(ahead);
-                }
-                advance(now);
-                ++filled;
-                if (++stage == stages) {
-                    stage = 0;
-                    phase ^= 1u;
-                }
+            }
+            if (!ok) {
+                break;
             }
         }
     } else if (warp == TILE_EPI_WARPS) {
         // ---------------- MMA issue (one thread) ----------------
         if (lane == 0) {
-            constexpr uint32_t idesc = F::INT8 ? umma_idesc_s8(128, N)
-                                               : (FMT == ROW_FP16 ? umma_idesc_f16(128, N) : umma_idesc_bf16(128, N));
-            constexpr uint32_t idesc_lo = umma_idesc_bf16(128, QT);   // fp32: lo terms of the rows against hi terms of the queries
-            const uint64_t a0 = umma_desc_sw128(smem_u32(smem)), b0 = umma_desc_sw128(smem_u32(b_smem));
-            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, tiles = 0, n_mine = 0;
-            for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_mine) {
-                const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
-                const uint32_t len = min(__ldg(p.s.list_off + d.x + 1) - __ldg(p.s.list_off + d.x) - d.w, TILE_SEGMENT);
-                const uint32_t buf = p.b_bufs == 2 ? n_mine & 1u : 0u;
-                ok = tcs_wait(&sh.b_full[buf], (n_mine / p.b_bufs) & 1u, failed, p.spin_limit);
+            const uint64_t a0 = FMT == ROW_SQ8 ? umma_desc(smem_u32(smem), 128, 1024) : umma_desc_sw128(smem_u32(smem));
+            const uint64_t b0 = umma_desc_sw128(smem_u32(b_smem));
+            constexpr uint32_t A_STEP = FMT == ROW_SQ8 ? 16 : 2;   // descriptor units per k-step of 32 bytes
+            // k-steps of the last piece: the rest of the row (fp32: a step holds eight of the first 32 dimensions)
+            const uint32_t rest = dim - (pieces - 1) * F::PIECE_DIMS;
+            const uint32_t last_steps = FMT == ROW_F32 ? min(4u, (rest + 7) / 8) : (rest + F::PIECE_DIMS / 4 - 1) / (F::PIECE_DIMS / 4);
+            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0, tiles = 0;
+            for (uint32_t n = 0; ok; ++n) {
+                const uint32_t slot = n % TILE_DESCS;
+                ok = tcs_wait(&sh.desc_full[slot], (n / TILE_DESCS) & 1u, failed, p.spin_limit);
+                if (!ok) {
+                    break;
+                }
+                const uint32_t len = sh.desc[slot].len, nqt = sh.desc[slot].nqt;
+                mbar_arrive(&sh.desc_free[slot]);
+                if (len == 0) {
+                    break;
+                }
+                const uint32_t qn = (nqt + 15) & ~15u;
+                const uint32_t idesc = tile_idesc<FMT>(F::B_TERMS * qn), idesc_lo = tile_idesc<FMT>(qn);
+                const uint32_t buf = p.b_bufs == 2 ? n & 1u : 0u;
+                ok = tcs_wait(&sh.item_full[n & 1u], (n >> 1) & 1u, failed, p.spin_limit);
                 for (uint32_t r0 = 0; r0 < len && ok; r0 += 128) {
                     if (tiles >= 2) {
                         ok = tcs_wait(&sh.acc_free[acc], acc_phase ^ 1u, failed, p.spin_limit);
@@ -560,16 +489,16 @@ tile_scan_kernel(const TileScan p) {
                         tc_fence_after_sync();
                         const uint64_t a = a0 + (stage * STAGE >> 4);
                         const uint64_t b = b0 + ((buf * b_bytes + piece * B_PIECE) >> 4);
-#pragma unroll
-                        for (uint32_t ks = 0; ks < 4; ++ks) {
+                        const uint32_t steps = piece + 1 == pieces ? last_steps : 4u;
+                        for (uint32_t ks = 0; ks < steps; ++ks) {
                             const uint32_t accumulate = (piece | ks) != 0 ? 1u : 0u;
                             if (F::INT8) {
-                                umma_s8(d_tmem, a + ks * 2, b + ks * 2, idesc, accumulate);
+                                umma_s8(d_tmem, a + ks * A_STEP, b + ks * 2, idesc, accumulate);
                             } else {
-                                umma_bf16(d_tmem, a + ks * 2, b + ks * 2, idesc, accumulate);
+                                umma_bf16(d_tmem, a + ks * A_STEP, b + ks * 2, idesc, accumulate);
                             }
-                            if (FMT == ROW_F32) {
-                                umma_bf16(d_tmem, a + (TILE_A_TERM >> 4) + ks * 2, b + ks * 2, idesc_lo, 1u);
+                            if (FMT == ROW_F32) {   // lo terms of the rows against hi terms of the queries
+                                umma_bf16(d_tmem, a + (TILE_A_TERM >> 4) + ks * A_STEP, b + ks * 2, idesc_lo, 1u);
                             }
                         }
                         umma_commit(&sh.freed[stage]);
@@ -593,108 +522,238 @@ tile_scan_kernel(const TileScan p) {
             }
         }
         __syncwarp();
-    } else {
+    } else if (warp > TILE_EPI_WARPS + 1 && warp < TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS) {
+        // ---------------- an item ahead: the queries' terms (B) and constants ----------------
+        // Query j belongs to warp j % 4 of the role, lane j / 4 of it: no warp waits for another.
+        const uint32_t qwarp = warp - (TILE_EPI_WARPS + 2);
+        const uint32_t j = lane * TILE_QUERY_WARPS + qwarp;
+        TileItem it;
+        for (uint32_t n = 0; next_item(n, it); ++n) {
+            const uint32_t slot = n & 1u, buf = p.b_bufs == 2 ? slot : 0u;
+            // (while the waits run, the pairs are on their way)
+            uint32_t q = 0;
+            uint64_t out = 0;
+            if (j < it.nqt) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.pairs + it.pair0 + j));
+                q = v.x;
+                out = (static_cast<uint64_t>(v.z) | (static_cast<uint64_t>(v.w) << 32)) + it.row0;
+            }
+            if (n >= 2) {
+                ok = tile_wait(&sh.item_free[slot], ((n >> 1) - 1u) & 1u, failed, p.spin_limit, lane);
+            }
+            if (ok && n >= p.b_bufs) {
+                ok = tile_wait(&sh.b_free[buf], (n / p.b_bufs - 1u) & 1u, failed, p.spin_limit, lane);
+            }
+            if (!ok) {
+                break;
+            }
+            unsigned char* bd = b_smem + buf * b_bytes;
+            const uint32_t per_row = pieces * 8;             // 16-byte units of a term
+            const uint32_t qn = (it.nqt + 15) & ~15u;
+            // (the rows of queries past the item's are left as they are: their columns are not read)
+            for (uint32_t i = 0; i * TILE_QUERY_WARPS + qwarp < it.nqt; ++i) {
+                const uint64_t qq = __shfl_sync(0xffffffffu, q, i);
+                const uint32_t qi = i * TILE_QUERY_WARPS + qwarp;
+                const unsigned char* src = p.terms + qq * F::B_TERMS * per_row * 16;
+                for (uint32_t u = lane; u < F::B_TERMS * per_row; u += 32) {
+                    const uint32_t term = u / per_row, k = u - term * per_row;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                     smem_u32(bd + (k >> 3) * B_PIECE + swizzled(term * qn + qi, k & 7u))),
+                                 "l"(src + u * 16)
+                                 : "memory");
+                }
+            }
+            if (j < it.nqt) {
+                sh.out[slot][j] = out;
+                if (FMT == ROW_SQ8) {
+                    sh.c0[slot][j] = __ldg(p.s.qa + q);
+                    sh.c1[slot][j] = p.s.coef_c * __ldg(p.qscale + q);
+                } else if (FMT == ROW_RABITQ) {
+                    sh.c0[slot][j] = __ldg(p.s.queries + static_cast<uint64_t>(q) * (dim + 1) + dim);
+                    sh.c1[slot][j] = __ldg(p.qscale + q);
+                    const int4 t = __ldg(reinterpret_cast<const int4*>(p.qsum) + q);
+                    sh.t1[slot][j] = t.x;
+                    sh.t2[slot][j] = t.y;
+                    sh.t3[slot][j] = t.z;
+                }
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            tile_publish(&sh.item_full[slot], lane);
+        }
+    } else if (F::CONVERT && warp >= TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS) {
+        // ---------------- stored rows -> operands, in shared memory ----------------
+        const uint32_t cwarp = warp - (TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS);
+        constexpr uint32_t ROWS = 128 / TILE_CONV_WARPS;     // of every tile, for a warp
+        const uint32_t kc = lane & 7u, rr = cwarp * ROWS + (lane >> 3);   // eight lanes per row, four rows at a time
+        uint32_t stage = 0, phase = 0, filled = 0, raw = 0;
+        TileItem it;
+        for (uint32_t n = 0; ok && next_item(n, it); ++n) {
+            for (uint32_t r0 = 0; r0 < it.len && ok; r0 += 128) {
+                const unsigned char* bits = raw_smem + (raw & 1u) * 128 * p.raw_pitch;
+                if (FMT == ROW_RABITQ) {
+                    ok = tile_wait(&sh.raw_full[raw & 1u], (raw >> 1) & 1u, failed, p.spin_limit, lane);
+                }
+                for (uint32_t piece = 0; piece < pieces && ok; ++piece) {
+                    unsigned char* dst = smem + stage * STAGE;
+                    if (FMT == ROW_RABITQ) {
+                        if (filled >= stages) {
+                            ok = tile_wait(&sh.freed[stage], phase ^ 1u, failed, p.spin_limit, lane);
+                        }
+                        if (!ok) {
+                            break;
+                        }
+                        // bits s, s + 8, s + 16, s + 24 of a word become the four bytes of one: two instructions per
+                        // four dimensions (the queries' terms are in the same order, see rabitq_query_kernel)
+                        uint32_t w[ROWS / 4];
+#pragma unroll
+                        for (uint32_t j = 0; j < ROWS / 4; ++j) {
+                            w[j] = *reinterpret_cast<const uint32_t*>(bits + (rr + j * 4) * p.raw_pitch + piece * 16 + (kc >> 1) * 4) >> ((kc & 1u) * 4);
+                        }
+#pragma unroll
+                        for (uint32_t j = 0; j < ROWS / 4; ++j) {
+                            constexpr uint32_t ONES = 0x01010101u;
+                            *reinterpret_cast<uint4*>(dst + swizzled(rr + j * 4, kc)) =
+                                make_uint4(w[j] & ONES, (w[j] >> 1) & ONES, (w[j] >> 2) & ONES, (w[j] >> 3) & ONES);
+                        }
+                    } else {
+                        // fp32, in place: dimensions 0-31 of the piece lie in the first block and 32-63 in the second,
+                        // 128 bytes of either per row; the hi terms take the row's line of the first, the lo terms of
+                        // the second.  Unit kc holds dimensions 4 kc .. + 3 and 32 + 4 kc .. + 3 (the queries' terms too).
+                        ok = tile_wait(&sh.raw_full[stage], phase, failed, p.spin_limit, lane);
+                        if (!ok) {
+                            break;
+                        }
+                        uint4 a[ROWS / 4], b[ROWS / 4];
+#pragma unroll
+                        for (uint32_t j = 0; j < ROWS / 4; ++j) {
+                            const unsigned char* src = dst + (rr + j * 4) * 128 + kc * 16;
+                            a[j] = *reinterpret_cast<const uint4*>(src);
+                            b[j] = *reinterpret_cast<const uint4*>(src + TILE_A_TERM);
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (uint32_t j = 0; j < ROWS / 4; ++j) {
+                            const float x[8] = {__uint_as_float(a[j].x), __uint_as_float(a[j].y), __uint_as_float(a[j].z), __uint_as_float(a[j].w),
+                                                __uint_as_float(b[j].x), __uint_as_float(b[j].y), __uint_as_float(b[j].z), __uint_as_float(b[j].w)};
+                            uint4 hi, lo;
+                            split_bf16x8(x, hi, lo);
+                            *reinterpret_cast<uint4*>(dst + swizzled(rr + j * 4, kc)) = hi;
+                            *reinterpret_cast<uint4*>(dst + TILE_A_TERM + swizzled(rr + j * 4, kc)) = lo;
+                        }
+                    }
+                    tile_publish(&sh.full[stage], lane);
+                    ++filled;
+                    if (++stage == stages) {
+                        stage = 0;
+                        phase ^= 1u;
+                    }
+                }
+                if (FMT == ROW_RABITQ) {
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sh.raw_free[raw & 1u]);
+                    }
+                    ++raw;
+                }
+            }
+        }
+    } else if (warp < TILE_EPI_WARPS) {
         // ---------------- epilogue: one thread per row of the tile, two warps per 32 rows share the queries ----------------
         const uint32_t quarter = warp & 3u, half = warp >> 2;
         const uint32_t row = quarter * 32 + lane;
         uint32_t tile = 0;
-        const bool filtered = p.s.filter_pos_inner != nullptr;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const uint4 d = __ldg(reinterpret_cast<const uint4*>(p.items + item));
-            const uint32_t lbeg = __ldg(p.s.list_off + d.x) + d.w, len = min(__ldg(p.s.list_off + d.x + 1) - lbeg, TILE_SEGMENT);
-            __syncwarp();
-            for (uint32_t j = lane; j < QT; j += 32) {
-                const bool used = j < d.z;
-                const uint32_t pair = used ? __ldg(p.pair_ids + d.y + j) : 0u, q = pair / p.nprobe;
-                sh.out[warp][j] = used ? q * p.t.stride + __ldg(p.t.base + pair) + d.w : 0u;
-                if (FMT == ROW_SQ8) {
-                    sh.c0[warp][j] = used ? __ldg(p.s.qa + q) : 0.f;
-                    sh.c1[warp][j] = used ? p.s.coef_c * __ldg(p.qscale + q) : 0.f;
-                } else if (FMT == ROW_RABITQ) {
-                    sh.c0[warp][j] = used ? __ldg(p.s.queries + static_cast<uint64_t>(q) * (dim + 1) + dim) : 0.f;
-                    sh.c1[warp][j] = used ? __ldg(p.qscale + q) : 0.f;
-                    sh.t1[warp][j] = used ? __ldg(p.qsum + 4 * q) : 0;
-                    sh.t2[warp][j] = used ? __ldg(p.qsum + 4 * q + 1) : 0;
-                    sh.t3[warp][j] = used ? __ldg(p.qsum + 4 * q + 2) : 0;
-                }
-            }
-            __syncwarp();
-            for (uint32_t r0 = 0; r0 < len; r0 += 128, ++tile) {
-                const uint32_t r = r0 + row, acc = tile & 1u;
-                const bool valid = r < len;
-                const uint32_t pos = lbeg + (valid ? r : 0u);
-                // what the row contributes to its scores
-                float x0 = 0.f, x1 = 1.f;
-                if (FMT == ROW_SQ8) {
-                    x0 = p.s.coef_b * __ldg(p.s.code_norm + pos);
-                } else if (FMT == ROW_RABITQ) {
-                    const float* tail = reinterpret_cast<const float*>(p.s.codes + static_cast<uint64_t>(pos) * p.s.code_stride + p.s.dpad / 8);
-                    x0 = __ldg(tail);
-                    x1 = __ldg(tail + 1);
-                    if (fabsf(x1) < 1e-5f) {
-                        x1 = x1 >= 0.f ? 1.0f : -1.0f;
+        TileItem it;
+        for (uint32_t n = 0; ok && next_item(n, it); ++n) {
+            const uint32_t slot = n & 1u;
+            const uint32_t qn = (it.nqt + 15) & ~15u;
+            // what a row contributes to its scores, one tile ahead: whether it takes part, its norm terms
+            struct RowPart {
+                float x0, x1;
+                bool drop;
+            };
+            auto row_part = [&](uint32_t r) -> RowPart {
+                RowPart part{0.f, 0.f, true};
+                if (r < it.len) {
+                    const uint32_t pos = it.lbeg + r;
+                    if (FMT == ROW_SQ8) {
+                        part.x0 = p.s.coef_b * __ldg(p.row_norm + pos);
+                    } else if (FMT == ROW_RABITQ) {
+                        const float2 v = __ldg(reinterpret_cast<const float2*>(p.row_norm) + pos);
+                        part.x0 = v.x;
+                        part.x1 = v.y;
+                    } else if (p.l2 != 0) {
+                        part.x0 = __ldg(p.row_norm + pos);
                     }
-                    x1 = -2.0f * x0 / x1;
-                    x0 *= x0;
-                } else if (p.l2 != 0) {
-                    x0 = __ldg(p.row_norm + pos);
+                    part.drop = p.pos_mask != nullptr && ((__ldg(p.pos_mask + (pos >> 5)) >> (pos & 31u)) & 1u) != 0;
                 }
-                const bool drop = !valid || (filtered && scan_row_filtered(p.s, pos));
+                return part;
+            };
+            RowPart ahead = row_part(row);
+            ok = tile_wait(&sh.item_full[slot], (n >> 1) & 1u, failed, p.spin_limit, lane);
+            for (uint32_t r0 = 0; r0 < it.len && ok; r0 += 128, ++tile) {
+                const uint32_t r = r0 + row, acc = tile & 1u;
+                const RowPart part = ahead;
+                if (r0 + 128 < it.len) {
+                    ahead = row_part(r + 128);
+                }
+                const float x0 = part.x0, x1 = part.x1;
                 ok = tile_wait(&sh.acc_full[acc], (tile >> 1) & 1u, failed, p.spin_limit, lane);
                 if (!ok) {
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * TILE_ACC_COLS;
-                if (r0 + quarter * 32 < len) {   // (the warp's rows are one group of 32 scores)
-                    // the last read of an accumulator is followed by its hand-over; columns past the item's queries hold
-                    // products with zero and are not stored
-                    for (uint32_t g = half * 8; g < d.z; g += 16) {
+                if (r0 + quarter * 32 < it.len) {   // (the warp's rows are one group of 32 scores)
+                    uint32_t* const scores = reinterpret_cast<uint32_t*>(p.t.scores) + r;
+                    for (uint32_t g = half * 8; g < it.nqt; g += 16) {
                         uint32_t v1[8], v2[8], v3[8];
                         tmem_load_8(taddr + g, v1);
                         if (F::B_TERMS >= 2) {
-                            tmem_load_8(taddr + QT + g, v2);
+                            tmem_load_8(taddr + qn + g, v2);
                         }
                         if (F::B_TERMS >= 3) {
-                            tmem_load_8(taddr + 2 * QT + g, v3);
+                            tmem_load_8(taddr + 2 * qn + g, v3);
+                        }
+                        // destinations in wide reads, before the stores: a read between two of them would wait
+                        ulonglong2 to[4];
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i) {
+                            to[i] = *reinterpret_cast<const ulonglong2*>(&sh.out[slot][g + 2 * i]);
                         }
                         tmem_load_wait();
-                        float v[8];
+                        float least = 0.f;   // of column g + lane
 #pragma unroll
                         for (uint32_t i = 0; i < 8; ++i) {
                             const uint32_t j = g + i;
+                            float v;
                             if (FMT == ROW_SQ8) {
                                 const float low = static_cast<float>(static_cast<int32_t>(v2[i]) * 254 + static_cast<int32_t>(v3[i]));
                                 const float f = fmaf(low, 1.0f / 64516.0f, static_cast<float>(static_cast<int32_t>(v1[i])));
-                                v[i] = fmaf(sh.c1[warp][j], f, x0) + sh.c0[warp][j];
+                                v = fmaf(sh.c1[slot][j], f, x0) + sh.c0[slot][j];
                             } else if (FMT == ROW_RABITQ) {
                                 // |x|^2 + |q|^2 - 2 |x| |q| (ip / error); the set bits' sum S gives ip = 2 S - (sum of all)
-                                const int32_t u1 = 2 * static_cast<int32_t>(v1[i]) - sh.t1[warp][j];
-                                const int32_t u2 = 2 * static_cast<int32_t>(v2[i]) - sh.t2[warp][j];
-                                const int32_t u3 = 2 * static_cast<int32_t>(v3[i]) - sh.t3[warp][j];
+                                const int32_t u1 = 2 * static_cast<int32_t>(v1[i]) - sh.t1[slot][j];
+                                const int32_t u2 = 2 * static_cast<int32_t>(v2[i]) - sh.t2[slot][j];
+                                const int32_t u3 = 2 * static_cast<int32_t>(v3[i]) - sh.t3[slot][j];
                                 const float f = fmaf(static_cast<float>(u2 * 254 + u3), 1.0f / 64516.0f, static_cast<float>(u1));
-                                const float qn = sh.c0[warp][j];
-                                v[i] = fmaf(x1 * qn, f * sh.c1[warp][j], fmaf(qn, qn, x0));
+                                const float qn2 = sh.c0[slot][j];
+                                v = fmaf(x1 * qn2, f * sh.c1[slot][j], fmaf(qn2, qn2, x0));
                             } else {
                                 float ip = __uint_as_float(v1[i]);
                                 if (FMT == ROW_F32) {
                                     ip += __uint_as_float(v2[i]);
                                 }
-                                v[i] = p.l2 != 0 ? fmaf(-2.0f, ip, x0) : -ip;
+                                v = p.l2 != 0 ? fmaf(-2.0f, ip, x0) : -ip;
                             }
-                        }
-                        uint32_t least = 0;   // of column g + lane
-#pragma unroll
-                        for (uint32_t i = 0; i < 8; ++i) {
-                            const uint32_t bits = drop ? SCORE_FILTERED : __float_as_uint(v[i]);
-                            if (g + i < d.z) {
-                                reinterpret_cast<uint32_t*>(p.t.scores)[sh.out[warp][g + i] + r] = bits;
+                            const uint32_t bits = part.drop ? SCORE_FILTERED : __float_as_uint(v);
+                            if (j < it.nqt) {
+                                scores[(i & 1u) != 0 ? to[i >> 1].y : to[i >> 1].x] = bits;
                             }
-                            const uint32_t low = __reduce_min_sync(0xffffffffu, ScoreSource<>::ordered(bits));
+                            const float low = warp_min_f32(bits);
                             least = lane == i ? low : least;
                         }
-                        if (lane < 8 && g + lane < d.z) {
-                            p.t.minima[(sh.out[warp][g + lane] + r0 + quarter * 32) >> 5] = least;
+                        if (lane < 8 && g + lane < it.nqt) {
+                            p.t.minima[(sh.out[slot][g + lane] + r0 + quarter * 32) >> 5] = ScoreSource<>::ordered(__float_as_uint(least));
                         }
                     }
                 }
@@ -703,6 +762,10 @@ tile_scan_kernel(const TileScan p) {
                 if (lane == 0) {
                     mbar_arrive(&sh.acc_free[acc]);
                 }
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&sh.item_free[slot]);
             }
         }
     }
@@ -713,7 +776,7 @@ tile_scan_kernel(const TileScan p) {
     tc_fence_before_sync();
     __syncthreads();
     if (sh.failed != 0) {
-        tc_drain_pause();   // a wait gave up: let the MMAs still in flight land before the CTA lets go
+        tc_drain_pause();   // a wait gave up: let the copies and MMAs still in flight land before the CTA lets go
         __syncthreads();
     }
     if (warp == TILE_EPI_WARPS) {

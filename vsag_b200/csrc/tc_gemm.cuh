@@ -238,6 +238,12 @@ umma_idesc_bf16(uint32_t m, uint32_t n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
+// The same with fp16 A and B.
+__host__ __device__ constexpr uint32_t
+umma_idesc_f16(uint32_t m, uint32_t n) {
+    return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
+
 // ---- host API (tc_gemm.cu) ------------------------------------------------------------------
 
 // Polls a bounded wait of the tensor-core kernels may take before it gives up (default
