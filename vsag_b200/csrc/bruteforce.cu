@@ -614,7 +614,7 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
             const bool first = tile0 == 0;
             uint32_t lists = 1;
             VB_TRY(tc_candidates(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, bias_all != nullptr ? bias_all + row0 : nullptr,
-                                 kcand, static_cast<uint32_t>(row0), ix->tc_out, &lists, nullptr, nullptr,
+                                 kcand, static_cast<uint32_t>(row0), ix->tc_out, &lists, nullptr,
                                  first ? nullptr : ix->row_bound.ptr));
             VB_LAUNCH(bf_merge_kernel, static_cast<uint32_t>(nq), 256, merge_smem, ix->tc_out.ptr,
                       static_cast<uint64_t>(lists) * kcand, first ? static_cast<const uint64_t*>(nullptr) : ix->cand.ptr,

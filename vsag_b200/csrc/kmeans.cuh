@@ -18,8 +18,14 @@ struct KMeansWorkspace {
     // tensor-core path: tiled bf16 terms of the points (kept while the same rows are assigned
     // again, i.e. across Lloyd iterations) and of the centroids, candidates, kernel scratch
     DevBuf<uint16_t> x_hi, x_lo, c_hi, c_lo;
-    DevBuf<float> x_sq;       // |x_i|^2 of the tiled rows
-    DevBuf<float> margin;     // 1e-3 * max_j |c_j|
+    // nominations work on rows and centroids minus `shift`, scaled by `scale`, as fp16 terms (kmeans_assign_tc)
+    DevBuf<float> shift, c_shifted, cs_sq;
+    float scale = 0.f;
+    bool half_off = false;        // too many rows were undecided that way: split bf16 terms from now on
+    DevBuf<float> x_norm, xs_norm;   // |x_i| and |x_i - shift|, rounded up
+    DevBuf<float> extremes;       // [0] largest |element| of the shifted rows and centroids, [1] max |c - shift|, [2] max |c|
+    DevBuf<float> row_margin;     // twice the largest error of a row's scores
+    DevBuf<float> x_sq;           // |x_i|^2, for the mean error
     DevBuf<float> row_bound;  // score of each row against its previous centroid (warm start)
     // rows whose tensor-core candidate lists may have lost a column (flagged by the kernel) are decided by
     // the fixed-order kernel over all centroids
@@ -35,6 +41,7 @@ struct KMeansWorkspace {
     forget_points() {
         tiled_rows = nullptr;
         tiled_n = 0;
+        half_off = false;
     }
 };
 

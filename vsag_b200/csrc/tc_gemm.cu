@@ -5,6 +5,7 @@
 #include <cstdlib>
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 namespace vb200 {
 
@@ -37,10 +38,11 @@ widen_in(uint16_t v) {  // bf16 bit pattern
 // so a [128 x 64] chunk is 16 KiB contiguous: 8x8-element cores of 128 B, the 8 cores of an 8-row
 // group back to back (1 KiB per group).  Out-of-range rows / dimensions are zero.
 // ---------------------------------------------------------------------------------------------
-template <typename T, bool SPLIT>
+template <typename T, bool SPLIT, bool HALF = false>
 __global__ void
 tc_pretile_kernel(const T* __restrict__ src, uint64_t rows, uint32_t dim, uint32_t chunks,
-                  uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, uint64_t total_units) {
+                  uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, uint64_t total_units,
+                  const float* __restrict__ shift, float scale) {
     uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // one 8-element core row
     if (u >= total_units) {
         return;
@@ -59,6 +61,10 @@ tc_pretile_kernel(const T* __restrict__ src, uint64_t rows, uint32_t dim, uint32
         float x = 0.f;
         if (r < rows && e0 + i < dim) {
             x = widen_in(src[r * dim + e0 + i]);
+        }
+        if (HALF) {
+            h[i] = r < rows && e0 + i < dim ? __half_as_ushort(__float2half_rn(fminf(fmaxf((x - __ldg(shift + e0 + i)) * scale, -65504.0f), 65504.0f))) : uint16_t{0};
+            continue;
         }
         __nv_bfloat16 bh = __float2bfloat16_rn(x);
         h[i] = __bfloat16_as_ushort(bh);
@@ -96,10 +102,10 @@ pretile_launch(const T* src, uint64_t rows, uint32_t dim, uint16_t* hi, uint16_t
     VB_CHECK_ARG(blocks <= 0x7fffffffu, "pretile: matrix too large");
     if (lo != nullptr) {
         auto kernel = tc_pretile_kernel<T, true>;
-        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units);
+        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units, static_cast<const float*>(nullptr), 1.0f);
     } else {
         auto kernel = tc_pretile_kernel<T, false>;
-        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units);
+        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units, static_cast<const float*>(nullptr), 1.0f);
     }
     return 0;
 }
@@ -107,6 +113,19 @@ pretile_launch(const T* src, uint64_t rows, uint32_t dim, uint16_t* hi, uint16_t
 int
 tc_pretile_f32(const float* src_dev, uint64_t rows, uint32_t dim, uint16_t* hi_dev, uint16_t* lo_dev) {
     return pretile_launch<float>(src_dev, rows, dim, hi_dev, lo_dev);
+}
+
+int
+tc_pretile_f16(const float* src_dev, uint64_t rows, uint32_t dim, const float* shift_dev, float scale, uint16_t* dst_dev) {
+    if (rows == 0) {
+        return 0;
+    }
+    const uint64_t units = tc_tiled_elems(rows, dim) / 8, blocks = (units + 255) / 256;
+    VB_CHECK_ARG(blocks <= 0x7fffffffu, "pretile: matrix too large");
+    auto kernel = tc_pretile_kernel<float, false, true>;
+    VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src_dev, rows, dim, (dim + TC_KC - 1) / TC_KC, dst_dev,
+              static_cast<uint16_t*>(nullptr), units, shift_dev, scale);
+    return 0;
 }
 
 int
@@ -256,7 +275,8 @@ tc_candidates_kernel(const TcParams p) {
         // Written for latency: 32-bit counters that wrap by compare instead of divide, descriptors
         // prepared once per stage.
         if (lane == 0) {
-            const uint32_t idesc_one = umma_idesc_bf16(TC_BM, TC_BN), idesc_two = umma_idesc_bf16(TC_BM, 2 * TC_BN);
+            const uint32_t idesc_one = p.half ? umma_idesc_f16(TC_BM, TC_BN) : umma_idesc_bf16(TC_BM, TC_BN);
+            const uint32_t idesc_two = p.half ? umma_idesc_f16(TC_BM, 2 * TC_BN) : umma_idesc_bf16(TC_BM, 2 * TC_BN);
             // Descriptor of stage 0 / operand 0; the others differ only in the start-address field,
             // which counts 16-byte units, so they are this value plus small constants kept in registers.
             const uint64_t desc0 = umma_desc(smem_u32(smem), 128, 1024);
@@ -467,9 +487,7 @@ tc_candidates_kernel(const TcParams p) {
             }
             // SMALL_M: the four best scores of the row, ascending, with their columns
             float bs0 = INFINITY, bs1 = INFINITY, bs2 = INFINITY, bs3 = INFINITY;
-            const float margin = (SMALL_M && p.a_sq != nullptr && p.margin_scale != nullptr && valid_row)
-                                     ? __ldg(p.margin_scale) * sqrtf(__ldg(p.a_sq + grow))
-                                     : -1.f;
+            const float margin = (SMALL_M && p.row_margin != nullptr && valid_row) ? __ldg(p.row_margin + grow) : -1.f;
             float bound = (margin >= 0.f && p.row_bound != nullptr) ? __ldg(p.row_bound + grow) + margin : INFINITY;
             uint32_t bc0 = 0xFFFFFFFFu, bc1 = 0xFFFFFFFFu, bc2 = 0xFFFFFFFFu, bc3 = 0xFFFFFFFFu;
             for (uint64_t t = t0; t < t1 && ok; t += step, ++gtile) {
@@ -812,8 +830,10 @@ tc_max_candidates(uint32_t n_terms) {
 int
 tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha,
               const float* bias_dev, uint32_t m, uint32_t col_base, DevBuf<uint64_t>& out,
-              uint32_t* n_split_out, const float* a_sq_dev, const float* margin_scale_dev,
-              const float* row_bound_dev, uint32_t* row_flags_dev, uint32_t* n_flagged_out) {
+              uint32_t* n_split_out, const float* row_margin_dev, const float* row_bound_dev, uint32_t* row_flags_dev,
+              uint32_t* n_flagged_out) {
+    const bool half = n_terms == TC_HALF;
+    n_terms = half ? 1 : n_terms;
     VB_CHECK_ARG(a.rows > 0 && b.rows > 0, "tc_candidates: empty operand");
     VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_candidates: operand depths differ");
     VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_candidates: 1 or 3 terms");
@@ -865,6 +885,7 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     p.a = a;
     p.b = b;
     p.n_terms = n_terms;
+    p.half = half ? 1u : 0u;
     p.alpha = alpha;
     p.bias = bias_dev;
     p.interleaved = interleaved ? 1u : 0u;
@@ -885,8 +906,7 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
             }
         }
     }
-    p.a_sq = a_sq_dev;
-    p.margin_scale = margin_scale_dev;
+    p.row_margin = row_margin_dev;
     p.row_bound = row_bound_dev;
     p.m = m;
     // Per-row candidate buffers: a few times m so compactions are rare, within what the per-warp

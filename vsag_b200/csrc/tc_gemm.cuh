@@ -9,6 +9,10 @@
 // the product is taken as hi*hi + hi*lo + lo*hi (three MMAs per k-step; the dropped lo*lo term is
 // ~2^-18 relative).  bf16 inputs use one term.
 //
+// Where the caller can bound what one rounding of either operand does to a score (k-means: the margin on its
+// nominations), fp32 inputs go through as one fp16 term scaled by a power of two: 2^-11 relative per operand, a third
+// of the MMAs.
+//
 // Operands are pre-tiled in global memory so that a [128 rows x 64 k] chunk is one contiguous
 // 16 KiB block already in the shared-memory layout the MMA descriptors describe (K-major, no
 // swizzle: 8x8 core matrices of 128 B, cores adjacent along K 128 B apart, 8-row groups 1 KiB
@@ -39,11 +43,11 @@ struct TcOperand {
 
 struct TcParams {
     TcOperand a, b;
-    uint32_t n_terms;         // 1 (bf16 inputs) or 3 (split fp32 inputs)
+    uint32_t n_terms;         // 1 (bf16 inputs, scaled fp16) or 3 (split fp32 inputs)
+    uint32_t half;            // 1: the terms are fp16
     float alpha;
     const float* bias;        // [b.rows] or nullptr
-    const float* a_sq;        // [a.rows] |A_i|^2, or nullptr            } used by the m <= 4 mode to skip
-    const float* margin_scale;// device scalar: 1e-3 * max_j |B_j|, or nullptr } columns that cannot win
+    const float* row_margin;  // [a.rows] or nullptr; m <= 4 mode: columns this much behind a row's best cannot win
     const float* row_bound;   // [a.rows] a score some column is known to reach (warm start), or nullptr
     uint32_t m;               // candidates kept per row
     uint32_t cap;             // per-row buffer, power of two >= m + 32
@@ -244,6 +248,8 @@ umma_idesc_f16(uint32_t m, uint32_t n) {
     return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
+constexpr uint32_t TC_HALF = 2;   // n_terms of tc_candidates for one scaled fp16 term per operand
+
 // ---- host API (tc_gemm.cu) ------------------------------------------------------------------
 
 // Polls a bounded wait of the tensor-core kernels may take before it gives up (default
@@ -258,6 +264,9 @@ int tc_pretile_f32(const float* src_dev, uint64_t rows, uint32_t dim, uint16_t* 
 // bf16 rows (bit patterns) -> tiled layout.
 int tc_pretile_bf16(const uint16_t* src_dev, uint64_t rows, uint32_t dim, uint16_t* hi_dev);
 
+// (fp32 rows - shift) * scale (a power of two) -> one fp16 term in the tiled layout; shift[dim] on the device.
+int tc_pretile_f16(const float* src_dev, uint64_t rows, uint32_t dim, const float* shift_dev, float scale, uint16_t* dst_dev);
+
 struct TcWorkspace {
     DevBuf<uint64_t> scratch;
     DevBuf<int> error_flag;
@@ -266,19 +275,18 @@ struct TcWorkspace {
 // For every row of A the m best columns of B by alpha * <a, b> + bias, as keys in
 // out_dev[a_rows][n_split * TC_COL_GROUPS][m]; the number of lists per row (n_split * TC_COL_GROUPS) is
 // chosen here and returned in n_split_out.
-// a_sq_dev / margin_scale_dev (both optional, m <= 4 only): squared row norms of A and a device scalar
-// c such that |approximate score - exact score| << c * |A_i|; columns scoring worse than the row's
-// best by more than that margin are not nominated at all.  row_bound_dev (optional): with the margin
-// (m <= 4), per row the exact score of some column: nothing worse than it plus the margin is visited;
-// with m > 4, per row a score that columns must stay below to be of use (e.g. the m-th best score found
-// in another column range): columns at or above it are not nominated.
+// n_terms: 1, 3, or TC_HALF for one scaled fp16 term per operand (alpha then undoes the scales).
+// row_margin_dev (optional, m <= 4 only): per row twice the largest error of a score; columns scoring worse than the
+// row's best by more than that are not nominated at all.  row_bound_dev (optional): with the margin (m <= 4), per
+// row the exact score of some column: nothing worse than it plus the margin is visited; with m > 4, per row a score
+// that columns must stay below to be of use (e.g. the m-th best score found in another column range): columns at or
+// above it are not nominated.
 // row_flags_dev / n_flagged_out (optional, with the margin): rows whose candidate lists may have lost a
 // column within the margin (see TcParams::row_flags) are marked and counted; the array must be zeroed by
 // the caller.
 int tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha,
                   const float* bias_dev, uint32_t m, uint32_t col_base, DevBuf<uint64_t>& out,
-                  uint32_t* n_split_out, const float* a_sq_dev = nullptr,
-                  const float* margin_scale_dev = nullptr, const float* row_bound_dev = nullptr,
+                  uint32_t* n_split_out, const float* row_margin_dev = nullptr, const float* row_bound_dev = nullptr,
                   uint32_t* row_flags_dev = nullptr, uint32_t* n_flagged_out = nullptr);
 
 // Every column of B whose score alpha * <a, b> + bias lies below the row's threshold row_thr_dev[row],
