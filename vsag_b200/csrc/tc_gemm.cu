@@ -218,7 +218,7 @@ tc_candidates_kernel(const TcParams p) {
         mbar_init(&sh.a_free, 1);
         for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(&sh.acc_full[a], 1);
-            mbar_init(&sh.acc_free[a], TC_EPI_THREADS);
+            mbar_init(&sh.acc_free[a], TC_EPI_WARPS);
         }
         sh.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -492,8 +492,7 @@ tc_candidates_kernel(const TcParams p) {
             uint32_t bc0 = 0xFFFFFFFFu, bc1 = 0xFFFFFFFFu, bc2 = 0xFFFFFFFFu, bc3 = 0xFFFFFFFFu;
             for (uint64_t t = t0; t < t1 && ok; t += step, ++gtile) {
                 const uint32_t acc = static_cast<uint32_t>(gtile & 1);
-                ok = mbar_wait_relaxed(&sh.acc_full[acc], static_cast<uint32_t>((gtile >> 1) & 1), p.spin_limit);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(&sh.acc_full[acc], static_cast<uint32_t>((gtile >> 1) & 1), p.spin_limit);
                 if (!ok) {
                     break;
                 }
@@ -518,7 +517,10 @@ tc_candidates_kernel(const TcParams p) {
                 if (half + 1 == step) {
                     // the accumulator is in registers now: hand it back before doing the selection
                     tc_fence_before_sync();
-                    mbar_arrive(&sh.acc_free[acc]);
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sh.acc_free[acc]);
+                    }
                 }
 
                 {
@@ -605,43 +607,33 @@ tc_candidates_kernel(const TcParams p) {
                     const float mn = fminf(fminf(m4[0], m4[1]), fminf(m4[2], m4[3]));
                     if (SMALL_M) {
                         if (mn < bound) {
-                            // rare path: visit only the elements that beat the bound
-                            float tmp[32];
-                            uint32_t hits = 0;
+                            // few elements pass: found through the levels of the tree (an index that is not a constant
+                            // would put the scores into local memory, for the whole warp whenever one row has a candidate)
+                            auto insert = [&](float v, uint32_t col) {
+                                // into the ascending quadruple (bs0 <= bs1 <= bs2 <= bs3)
+                                const bool l0 = v < bs0, l1 = v < bs1, l2 = v < bs2, l3 = v < bs3;
+                                bs3 = l2 ? bs2 : (l3 ? v : bs3);
+                                bc3 = l2 ? bc2 : (l3 ? col : bc3);
+                                bs2 = l1 ? bs1 : (l2 ? v : bs2);
+                                bc2 = l1 ? bc1 : (l2 ? col : bc2);
+                                bs1 = l0 ? bs0 : (l1 ? v : bs1);
+                                bc1 = l0 ? bc0 : (l1 ? col : bc1);
+                                bs0 = l0 ? v : bs0;
+                                bc0 = l0 ? col : bc0;
+                            };
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) {
-                                tmp[i] = sc[i];
-                                hits |= (sc[i] < bound ? 1u : 0u) << i;
-                            }
-                            while (hits != 0) {
-                                const uint32_t i = __ffs(hits) - 1;
-                                hits &= hits - 1;
-                                const float s = tmp[i];
-                                if (s < bs3) {
-                                    // insert into the ascending quadruple (bs0 <= bs1 <= bs2 <= bs3)
-                                    const uint32_t col = c0 + i;
-                                    if (s < bs2) {
-                                        bs3 = bs2;
-                                        bc3 = bc2;
-                                        if (s < bs1) {
-                                            bs2 = bs1;
-                                            bc2 = bc1;
-                                            if (s < bs0) {
-                                                bs1 = bs0;
-                                                bc1 = bc0;
-                                                bs0 = s;
-                                                bc0 = col;
-                                            } else {
-                                                bs1 = s;
-                                                bc1 = col;
+                            for (int g = 0; g < 4; ++g) {
+                                if (m4[g] < bound) {
+#pragma unroll
+                                    for (int i = g; i < 16; i += 4) {
+                                        if (m16[i] < bound) {
+                                            if (sc[i] < bound) {
+                                                insert(sc[i], c0 + i);
                                             }
-                                        } else {
-                                            bs2 = s;
-                                            bc2 = col;
+                                            if (sc[i + 16] < bound) {
+                                                insert(sc[i + 16], c0 + i + 16);
+                                            }
                                         }
-                                    } else {
-                                        bs3 = s;
-                                        bc3 = col;
                                     }
                                 }
                             }
@@ -654,10 +646,11 @@ tc_candidates_kernel(const TcParams p) {
                                && (p.diag & 4u) == 0
 #endif
                     ) {
-                        // few elements pass: test them in pairs through the first level of the tree
+                        // few elements pass: test them in pairs through the first levels of the tree
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            if (m16[i] < thr) {
+                        for (int g = 0; g < 16; ++g) {
+                            const int i = (g & 3) * 4 + (g >> 2);   // (the four of a second-level minimum together)
+                            if (m4[i & 3] < thr && m16[i] < thr) {
                                 if (THRESH) {
                                     if (sc[i] < thr) {
                                         if (cnt < p.cap) {

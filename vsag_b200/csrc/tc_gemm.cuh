@@ -125,25 +125,26 @@ mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = TC_SPIN_LIMIT) {
     return false;
 }
 
-// The same wait for the many epilogue threads: between polls they sleep, so that their polling
-// does not take issue slots from the three single threads that feed the tensor core.
+// The same wait for the many epilogue warps: one lane polls, and each poll may suspend it in hardware for up to a
+// microsecond, so that the polling takes no issue slots from the three single threads that feed the tensor core and
+// ends as soon as the phase does.
 __device__ __forceinline__ bool
-mbar_wait_relaxed(uint64_t* bar, uint32_t parity, uint32_t limit = TC_SPIN_LIMIT) {
-    for (uint32_t spin = 0; spin < limit; ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (done) {
-            return true;
+mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit) {
+    uint32_t done = 0;
+    if ((threadIdx.x & 31) == 0) {
+        for (uint32_t spin = 0; spin < limit && done == 0; ++spin) {
+            asm volatile(
+                "{\n.reg .pred p;\n"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+                "selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
+                : "memory");
         }
-        __nanosleep(128);
     }
-    return false;
+    done = __shfl_sync(0xffffffffu, done, 0);
+    __syncwarp();
+    return done != 0;
 }
 
 // One contiguous global -> shared bulk copy, completion counted in bytes on `bar`.
