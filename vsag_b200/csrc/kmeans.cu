@@ -53,12 +53,12 @@ tensor_cores_enabled() {
     return v == 1;
 }
 
-// Picks, among each row's candidate centroids, the one the reference's arithmetic prefers:
-// score = fma(-2, <c, x>, |c|^2) with the inner product as one ascending FMA chain, lowest index
-// on ties (src/impl/cluster/kmeans_cluster.cpp:262-284).  `lanes` (a power of two <= 32) threads
-// share a row.  Candidates whose nominating score lies further than the row's margin behind the best one
-// cannot be the pick; when a single one is left -- nearly always -- it needs no exact score, unless the
-// caller wants the score itself (best_out).
+// The pick among each row's candidate centroids: the one the reference's arithmetic prefers, score = fma(-2, <c, x>,
+// |c|^2) with the inner product as one ascending FMA chain, lowest index on ties
+// (src/impl/cluster/kmeans_cluster.cpp:262-284).  Candidates whose nominating score lies further than the row's margin
+// behind the best one cannot be it; when a single one is left -- nearly always -- it needs no exact score, unless the
+// caller wants the score itself (best_out).  The rows with more go to a list, whose rows take four lanes each: scored
+// on the spot, two such rows of a warp kept the other thirty lanes waiting for their chains (390 us a pass over 1M rows).
 __device__ __forceinline__ float
 kmeans_exact_score(const float* __restrict__ c, const float* __restrict__ x, uint32_t dim, float c_sq, bool vec) {
     float ip = 0.f;
@@ -91,73 +91,105 @@ kmeans_exact_score(const float* __restrict__ c, const float* __restrict__ x, uin
     return fmaf(-2.0f, ip, c_sq);
 }
 
-__global__ void __launch_bounds__(128)
-kmeans_pick_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, const float* __restrict__ centroids,
-                   const float* __restrict__ c_sq, const uint64_t* __restrict__ cand, uint32_t per_row,
-                   const float* __restrict__ row_margin, uint32_t lanes, int32_t* __restrict__ labels,
-                   float* __restrict__ best_out) {
-    const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t i = t / lanes;
-    const uint32_t sub = static_cast<uint32_t>(t % lanes);
-    const bool live = i < n;
+constexpr uint32_t PICK_LANES = 4;
+
+__global__ void __launch_bounds__(256)
+kmeans_single_kernel(uint64_t n, const uint64_t* __restrict__ cand, uint32_t per_row, const float* __restrict__ row_margin,
+                     int32_t* __restrict__ labels, uint32_t* __restrict__ close) {
+    const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x) / PICK_LANES;
+    const uint32_t sub = threadIdx.x % PICK_LANES;
     const uint64_t* ci = cand + i * per_row;
-    uint64_t least = KEY_INF;
-    if (live) {
-        for (uint32_t j = sub; j < per_row; j += lanes) {
-            const uint64_t key = ci[j];
+    uint64_t least = KEY_INF, next = KEY_INF;   // the two smallest keys of this lane, then of the row
+    if (i < n) {
+        for (uint32_t j = sub; j < per_row; j += PICK_LANES) {
+            const uint64_t key = __ldg(ci + j);
+            next = key < least ? least : (key < next ? key : next);
             least = key < least ? key : least;
         }
     }
-    for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
-        const uint64_t other = __shfl_xor_sync(0xffffffffu, least, off);
-        least = other < least ? other : least;
+#pragma unroll
+    for (uint32_t off = PICK_LANES >> 1; off > 0; off >>= 1) {
+        const uint64_t a = __shfl_xor_sync(0xffffffffu, least, off), b = __shfl_xor_sync(0xffffffffu, next, off);
+        next = a < least ? (least < b ? least : b) : (a < next ? a : next);
+        least = a < least ? a : least;
     }
-    float limit = INFINITY;
-    if (live && least != KEY_INF) {
-        limit = ordered_to_float(static_cast<uint32_t>(least >> 32)) + __ldg(row_margin + i);
+    if (i >= n || sub != 0) {
+        return;
     }
-    uint32_t within = 0;
-    if (live) {
-        for (uint32_t j = sub; j < per_row; j += lanes) {
-            const uint64_t key = ci[j];
-            within += key != KEY_INF && ordered_to_float(static_cast<uint32_t>(key >> 32)) <= limit ? 1u : 0u;
-        }
+    if (least == KEY_INF) {
+        labels[i] = 0;
+        return;
     }
-    for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
-        within += __shfl_xor_sync(0xffffffffu, within, off);
+    labels[i] = static_cast<int32_t>(static_cast<uint32_t>(least));
+    if (next != KEY_INF &&
+        ordered_to_float(static_cast<uint32_t>(next >> 32)) <= ordered_to_float(static_cast<uint32_t>(least >> 32)) + __ldg(row_margin + i)) {
+        close[1 + atomicAdd(close, 1u)] = static_cast<uint32_t>(i);
     }
-    float best = INFINITY;
-    uint32_t best_col = 0x7fffffffu;
-    if (live && within == 1 && best_out == nullptr) {
-        best_col = static_cast<uint32_t>(least);
-    } else if (live) {
-        const float* xi = x + i * dim;
-        const bool vec = (dim & 3u) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(centroids)) & 15u) == 0;
-        for (uint32_t j = sub; j < per_row; j += lanes) {
-            const uint64_t key = ci[j];
-            if (key == KEY_INF || ordered_to_float(static_cast<uint32_t>(key >> 32)) > limit) {
-                continue;
+}
+
+// Exact scores of the candidates of the rows in close[1 .. close[0]] (null: of all n rows), four lanes per row.
+__global__ void __launch_bounds__(256)
+kmeans_pick_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, const float* __restrict__ centroids,
+                   const float* __restrict__ c_sq, const uint64_t* __restrict__ cand, uint32_t per_row,
+                   const float* __restrict__ row_margin, const uint32_t* __restrict__ close, int32_t* __restrict__ labels,
+                   float* __restrict__ best_out) {
+    const uint64_t count = close != nullptr ? close[0] : n;
+    const uint32_t sub = threadIdx.x % PICK_LANES;
+    const bool vec = (dim & 3u) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(centroids)) & 15u) == 0;
+    const uint64_t step = static_cast<uint64_t>(gridDim.x) * 256 / PICK_LANES;
+    for (uint64_t e0 = static_cast<uint64_t>(blockIdx.x) * 256 / PICK_LANES; e0 < count; e0 += step) {
+        const uint64_t e = e0 + threadIdx.x / PICK_LANES;
+        const bool live = e < count;
+        const uint64_t i = !live ? 0 : (close != nullptr ? close[1 + e] : e);
+        const uint64_t* ci = cand + i * per_row;
+        uint64_t least = KEY_INF;
+        if (live) {
+            for (uint32_t j = sub; j < per_row; j += PICK_LANES) {
+                const uint64_t key = __ldg(ci + j);
+                least = key < least ? key : least;
             }
-            const uint32_t col = static_cast<uint32_t>(key);
-            const float score = kmeans_exact_score(centroids + static_cast<uint64_t>(col) * dim, xi, dim, __ldg(c_sq + col), vec);
-            if (score < best || (score == best && col < best_col)) {
-                best = score;
-                best_col = col;
+        }
+#pragma unroll
+        for (uint32_t off = PICK_LANES >> 1; off > 0; off >>= 1) {
+            const uint64_t other = __shfl_xor_sync(0xffffffffu, least, off);
+            least = other < least ? other : least;
+        }
+        float best = INFINITY;
+        uint32_t best_col = 0x7fffffffu;
+        if (live && least != KEY_INF) {
+            const float limit = ordered_to_float(static_cast<uint32_t>(least >> 32)) + __ldg(row_margin + i);
+            // the row's candidates within the limit, dealt to its lanes in turn
+            uint32_t turn = 0;
+            for (uint32_t j = 0; j < per_row; ++j) {
+                const uint64_t key = __ldg(ci + j);
+                if (key == KEY_INF || ordered_to_float(static_cast<uint32_t>(key >> 32)) > limit) {
+                    continue;
+                }
+                if (turn++ % PICK_LANES != sub) {
+                    continue;
+                }
+                const uint32_t col = static_cast<uint32_t>(key);
+                const float score = kmeans_exact_score(centroids + static_cast<uint64_t>(col) * dim, x + i * dim, dim, __ldg(c_sq + col), vec);
+                if (score < best || (score == best && col < best_col)) {
+                    best = score;
+                    best_col = col;
+                }
             }
         }
-    }
-    for (uint32_t off = lanes >> 1; off > 0; off >>= 1) {
-        float ob = __shfl_xor_sync(0xffffffffu, best, off);
-        uint32_t oc = __shfl_xor_sync(0xffffffffu, best_col, off);
-        if (ob < best || (ob == best && oc < best_col)) {
-            best = ob;
-            best_col = oc;
+#pragma unroll
+        for (uint32_t off = PICK_LANES >> 1; off > 0; off >>= 1) {
+            float ob = __shfl_xor_sync(0xffffffffu, best, off);
+            uint32_t oc = __shfl_xor_sync(0xffffffffu, best_col, off);
+            if (ob < best || (ob == best && oc < best_col)) {
+                best = ob;
+                best_col = oc;
+            }
         }
-    }
-    if (live && sub == 0) {
-        labels[i] = best_col == 0x7fffffffu ? 0 : static_cast<int32_t>(best_col);
-        if (best_out != nullptr) {
-            best_out[i] = best;
+        if (live && sub == 0) {
+            labels[i] = best_col == 0x7fffffffu ? 0 : static_cast<int32_t>(best_col);
+            if (best_out != nullptr) {
+                best_out[i] = best;
+            }
         }
     }
 }
@@ -280,65 +312,46 @@ kmeans_row_prep_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, co
     }
 }
 
-// labels of the rows in `rows` over all centroids, exactly; a CTA per row (for a few rows: as a matrix product over
-// 128-row tiles they took one CTA 560 us).
-__global__ void __launch_bounds__(512)
+// The best centroid of the rows in `rows` over all centroids, exactly, as keys: grid.x = a few rows, grid.y = shares of
+// the centroids, which stream through shared memory (as a matrix product over 128-row tiles a few rows took one CTA
+// 560 us, as a CTA per row with the centroids read by a thread each 75 us).
+template <int UNIT>
+__global__ void __launch_bounds__(RS_ROWS)
 kmeans_few_rows_kernel(const float* __restrict__ x, uint32_t dim, const float* __restrict__ centroids, const float* __restrict__ c_sq,
-                       uint32_t k, const uint32_t* __restrict__ rows, int32_t* __restrict__ labels, float* __restrict__ best_out) {
+                       uint32_t k, const uint32_t* __restrict__ rows, unsigned long long* __restrict__ keys) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ unsigned long long least;
-    float* xs = reinterpret_cast<float*>(smem);
+    float* xs = reinterpret_cast<float*>(smem + RS_STAGES * RS_STAGE);
     const uint64_t i = rows[blockIdx.x];
-    for (uint32_t d = threadIdx.x; d < dim; d += 512) {
-        xs[d] = x[i * dim + d];
+    const uint32_t qpad = (dim + 3) / 4 * 4;
+    for (uint32_t d = threadIdx.x; d < qpad; d += RS_ROWS) {
+        xs[d] = d < dim ? x[i * dim + d] : 0.f;
     }
-    if (threadIdx.x == 0) {
-        least = KEY_INF;
-    }
-    __syncthreads();
-    const bool vec = (dim & 3u) == 0 && (reinterpret_cast<uintptr_t>(centroids) & 15u) == 0;
     uint64_t mine = KEY_INF;
-    for (uint32_t j = threadIdx.x; j < k; j += 512) {
-        const float* c = centroids + static_cast<uint64_t>(j) * dim;
-        float ip = 0.f;
-        if (vec) {
-            for (uint32_t d = 0; d < dim; d += 32) {
-                float4 v[8];
-#pragma unroll
-                for (uint32_t u = 0; u < 8; ++u) {
-                    v[u] = d + 4 * u < dim ? __ldg(reinterpret_cast<const float4*>(c + d) + u) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (uint32_t u = 0; u < 8; ++u) {
-                    if (d + 4 * u < dim) {
-                        const float4 w = *reinterpret_cast<const float4*>(xs + d + 4 * u);
-                        ip = fmaf(v[u].x, w.x, ip);
-                        ip = fmaf(v[u].y, w.y, ip);
-                        ip = fmaf(v[u].z, w.z, ip);
-                        ip = fmaf(v[u].w, w.w, ip);
-                    }
-                }
-            }
-        } else {
-            for (uint32_t d = 0; d < dim; ++d) {
-                ip = fmaf(__ldg(c + d), xs[d], ip);
-            }
-        }
-        const uint64_t key = make_key(fmaf(-2.0f, ip, __ldg(c_sq + j)), j);
-        mine = key < mine ? key : mine;
-    }
+    RowAcc<ROW_F32, false, 1> acc;
+    row_stream<UNIT>(reinterpret_cast<const unsigned char*>(centroids), static_cast<uint64_t>(dim) * 4, dim * 4, dim, k, blockIdx.y,
+                     gridDim.y, smem, xs, qpad, acc, [&](uint64_t j, bool valid) {
+                         if (valid) {
+                             const uint64_t key = make_key(fmaf(-2.0f, acc.acc[0], __ldg(c_sq + j)), static_cast<uint32_t>(j));
+                             mine = key < mine ? key : mine;
+                         }
+                     });
     for (int off = 16; off > 0; off >>= 1) {
         const uint64_t other = __shfl_xor_sync(0xffffffffu, mine, off);
         mine = other < mine ? other : mine;
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&least, static_cast<unsigned long long>(mine));
+        atomicMin(keys + blockIdx.x, static_cast<unsigned long long>(mine));
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        labels[i] = static_cast<int32_t>(static_cast<uint32_t>(least));
+}
+
+__global__ void
+kmeans_keys_to_labels_kernel(const unsigned long long* __restrict__ keys, uint32_t count, const uint32_t* __restrict__ rows,
+                             int32_t* __restrict__ labels, float* __restrict__ best_out) {
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < count) {
+        labels[rows[e]] = static_cast<int32_t>(static_cast<uint32_t>(keys[e]));
         if (best_out != nullptr) {
-            best_out[i] = ordered_to_float(static_cast<uint32_t>(least >> 32));
+            best_out[rows[e]] = ordered_to_float(static_cast<uint32_t>(keys[e] >> 32));
         }
     }
 }
@@ -376,7 +389,7 @@ kmeans_scatter_labels_kernel(const uint32_t* __restrict__ rows, uint64_t count, 
 
 constexpr uint32_t KMEANS_TC_CANDIDATES = 4;
 constexpr uint64_t KMEANS_TC_SLICE = uint64_t{1} << 22;  // rows tiled at once
-constexpr uint32_t KMEANS_FEW_ROWS = 4096;               // undecided rows that a CTA each decides
+constexpr uint32_t KMEANS_FEW_ROWS = 4096;               // undecided rows that CTAs of their own decide
 
 // Assignment through the tensor cores: candidates nominated by approximate scores, winner by the exact rule above.
 //
@@ -464,11 +477,18 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
         VB_TRY(tc_candidates(ws.tc, a, b, half ? TC_HALF : 3, half ? -2.0f / (ws.scale * ws.scale) : -2.0f, ws.cs_sq.ptr, m, 0, ws.cand,
                              &n_split, ws.row_margin.ptr, row_bound, ws.row_flags.ptr, &n_flagged));
         const uint32_t per_row = n_split * m;
-        const uint32_t lanes = per_row >= 32 ? 32u : next_pow2(per_row);
-        const uint64_t threads = rows * lanes;
-        VB_LAUNCH(kmeans_pick_kernel, static_cast<uint32_t>((threads + 127) / 128), 128, 0, x_dev + r0 * dim, rows,
-                  dim, centroids_dev, ws.c_sq.ptr, ws.cand.ptr, per_row, ws.row_margin.ptr, lanes, labels_dev + r0,
-                  best_dev != nullptr ? best_dev + r0 : nullptr);
+        float* best = best_dev != nullptr ? best_dev + r0 : nullptr;
+        const uint32_t* close = nullptr;
+        if (best == nullptr) {
+            VB_TRY(ws.close_rows.reserve(rows + 1));
+            VB_CUDA(cudaMemsetAsync(ws.close_rows.ptr, 0, sizeof(uint32_t), st));
+            VB_LAUNCH(kmeans_single_kernel, static_cast<uint32_t>((rows * PICK_LANES + 255) / 256), 256, 0, rows, ws.cand.ptr, per_row,
+                      ws.row_margin.ptr, labels_dev + r0, ws.close_rows.ptr);
+            close = ws.close_rows.ptr;
+        }
+        const uint32_t pick_blocks = static_cast<uint32_t>(std::min<uint64_t>((rows * PICK_LANES + 255) / 256, 8ull * sm_count()));
+        VB_LAUNCH(kmeans_pick_kernel, pick_blocks, 256, 0, x_dev + r0 * dim, rows, dim, centroids_dev, ws.c_sq.ptr, ws.cand.ptr, per_row,
+                  ws.row_margin.ptr, close, labels_dev + r0, best);
         if (n_flagged > 0) {
             // A candidate list of these rows ended full of columns within the error margin of its best (many
             // near-equal centroids, or data far from the origin): the exact winner may not have been
@@ -478,10 +498,19 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
             VB_CUDA(cudaMemsetAsync(ws.flagged_count.ptr, 0, sizeof(uint32_t), st));
             VB_LAUNCH(kmeans_collect_flagged_kernel, static_cast<uint32_t>((rows + 255) / 256), 256, 0, ws.row_flags.ptr,
                       rows, ws.flagged_rows.ptr, ws.flagged_count.ptr);
-            const size_t smem = dim * sizeof(float);
-            if (n_flagged <= KMEANS_FEW_ROWS && smem <= 40 * 1024) {
-                VB_LAUNCH(kmeans_few_rows_kernel, n_flagged, 512, smem, x_dev + r0 * dim, dim, centroids_dev, ws.c_sq.ptr, k,
-                          ws.flagged_rows.ptr, labels_dev + r0, best_dev != nullptr ? best_dev + r0 : nullptr);
+            const size_t smem = RS_STAGES * RS_STAGE + (dim + 3) / 4 * 4 * sizeof(float);
+            if (n_flagged <= KMEANS_FEW_ROWS && smem <= 200 * 1024) {
+                VB_TRY(ws.flagged_keys.reserve(n_flagged));
+                VB_CUDA(cudaMemsetAsync(ws.flagged_keys.ptr, 0xFF, n_flagged * sizeof(unsigned long long), st));
+                auto kernel = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(centroids_dev) & 15) == 0 ? kmeans_few_rows_kernel<16>
+                                                                                                     : kmeans_few_rows_kernel<4>;
+                VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+                const uint32_t chunks128 = (k + RS_ROWS - 1) / RS_ROWS;
+                const uint32_t shares = std::min(chunks128, std::max(1u, 4u * static_cast<uint32_t>(sm_count()) / n_flagged));
+                VB_LAUNCH(kernel, dim3(n_flagged, shares), RS_ROWS, smem, x_dev + r0 * dim, dim, centroids_dev, ws.c_sq.ptr, k,
+                          ws.flagged_rows.ptr, ws.flagged_keys.ptr);
+                VB_LAUNCH(kmeans_keys_to_labels_kernel, (n_flagged + 255) / 256, 256, 0, ws.flagged_keys.ptr, n_flagged, ws.flagged_rows.ptr,
+                          labels_dev + r0, best);
             } else {
                 VB_TRY(ws.flagged_x.reserve(static_cast<size_t>(n_flagged) * dim));
                 VB_TRY(ws.flagged_labels.reserve(n_flagged));

@@ -26,11 +26,13 @@ struct KMeansWorkspace {
     DevBuf<float> extremes;       // [0] largest |element| of the shifted rows and centroids, [1] max |c - shift|, [2] max |c|
     DevBuf<float> row_margin;     // twice the largest error of a row's scores
     DevBuf<float> x_sq;           // |x_i|^2, for the mean error
+    DevBuf<uint32_t> close_rows;  // [0] how many, then the rows with several candidates within the margin
+    DevBuf<unsigned long long> flagged_keys;
     DevBuf<float> row_bound;  // score of each row against its previous centroid (warm start)
     // rows whose tensor-core candidate lists may have lost a column (flagged by the kernel) are decided by
     // the fixed-order kernel over all centroids
     DevBuf<uint32_t> row_flags, flagged_rows, flagged_count;
-    DevBuf<float> flagged_x, flagged_best;
+    DevBuf<float> flagged_x, flagged_best;   // (many of them)
     DevBuf<int32_t> flagged_labels;
     const float* tiled_rows = nullptr;
     uint64_t tiled_n = 0;
