@@ -303,7 +303,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
     __shared__ TileShared sh;
     // the swizzle permutes by address bits: blocks start on 1 KiB
     unsigned char* const smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t stages = p.stages, pieces = p.pieces, dim = p.s.dim;
     unsigned char* const b_smem = smem + stages * STAGE;
     const uint32_t b_bytes = pieces * B_PIECE;
@@ -450,7 +450,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
         }
     } else if (warp == TILE_EPI_WARPS) {
         // ---------------- MMA issue (one thread) ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             const uint64_t a0 = FMT == ROW_SQ8 ? umma_desc(smem_u32(smem), 128, 1024) : umma_desc_sw128(smem_u32(smem));
             const uint64_t b0 = umma_desc_sw128(smem_u32(b_smem));
             constexpr uint32_t A_STEP = FMT == ROW_SQ8 ? 16 : 2;   // descriptor units per k-step of 32 bytes

@@ -193,21 +193,24 @@ tc_candidates_kernel(const TcParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ TcShared sh;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n_ops = p.n_terms == 3 ? 4u : 2u;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t n_terms_op = p.n_terms == 3 ? 2u : 1u;                       // bf16 terms per operand
     // resident-A mode: [A tile: chunks x terms][ring of B stages]; otherwise a ring of [A terms][B terms]
-    const uint32_t a_region_bytes = p.a_resident ? p.a.chunks * n_terms_op * TC_CHUNK_BYTES : 0u;
+    // pair mode: an item has two A tiles ([chunk][tile][term]), each with accumulators of its own
+    const uint32_t a_tiles = p.pair ? 2u : 1u;
+    const uint32_t a_region_bytes = p.a_resident ? p.a.chunks * a_tiles * n_terms_op * TC_CHUNK_BYTES : 0u;
     // wide mode: a stage holds two consecutive B tiles, term by term ([hi t][hi t+1][lo t][lo t+1]), so
     // that one 128 x 256 x 16 MMA reads both; the accumulators are 256 columns each.
     const uint32_t step = p.wide ? 2u : 1u;
-    const uint32_t acc_cols = step * TC_BN;
-    const uint32_t stage_bytes = ((p.a_resident ? 0u : n_terms_op) + n_terms_op * step) * TC_CHUNK_BYTES;
-    (void)n_ops;
+    const uint32_t tile_cols = step * TC_BN;             // tensor-memory columns of one A tile
+    const uint32_t acc_cols = a_tiles * tile_cols;
+    const uint32_t n_acc = acc_cols > 256 ? 1u : 2u;     // accumulators: two while they fit the 512 columns
+    const uint32_t stage_bytes = ((p.a_resident ? 0u : n_terms_op * a_tiles) + n_terms_op * step) * TC_CHUNK_BYTES;
     const uint32_t chunks = p.a.chunks;
     const uint64_t m_tiles = (p.a.rows + TC_BM - 1) / TC_BM;
     const uint64_t n_tiles = (p.b.rows + TC_BN - 1) / TC_BN;
-    const uint64_t n_items = m_tiles * p.n_split;
+    const uint64_t m_units = (m_tiles + a_tiles - 1) / a_tiles;   // items per share of B
+    const uint64_t n_items = m_units * p.n_split;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < p.stages; ++s) {
@@ -224,7 +227,7 @@ tc_candidates_kernel(const TcParams p) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == TC_EPI_WARPS) {
-        tmem_alloc(&sh.tmem_base, 2 * acc_cols);  // two fp32 accumulators of 128 (256 when wide) columns
+        tmem_alloc(&sh.tmem_base, n_acc * acc_cols);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -239,7 +242,10 @@ tc_candidates_kernel(const TcParams p) {
     // queue walks the row tiles of one share before the next share, so the CTAs running at any moment
     // sweep B front to back together and a B tile fetched from DRAM by one of them is an L2 hit for the
     // others -- what a base far larger than L2 needs when there are many row tiles.
-    const uint32_t m_tiles32 = static_cast<uint32_t>(m_tiles);
+    const uint32_t m_tiles32 = static_cast<uint32_t>(m_units);
+    // the row tile of A that tile `a` of an item copies (an odd number of tiles: the last one twice, its rows are not valid)
+    const uint32_t last_tile = static_cast<uint32_t>(m_tiles) - 1;
+    auto a_tile = [&](uint32_t unit, uint32_t a) -> uint32_t { return min(unit * a_tiles + a, last_tile); };
     auto open_item = [&](uint32_t item, uint32_t& mtile, uint32_t& split, uint32_t& tiles) {
         if (p.interleaved) {
             split = item / m_tiles32;
@@ -274,7 +280,7 @@ tc_candidates_kernel(const TcParams p) {
         // ---------------- MMA issue (one thread) ----------------
         // Written for latency: 32-bit counters that wrap by compare instead of divide, descriptors
         // prepared once per stage.
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_one = p.half ? umma_idesc_f16(TC_BM, TC_BN) : umma_idesc_bf16(TC_BM, TC_BN);
             const uint32_t idesc_two = p.half ? umma_idesc_f16(TC_BM, 2 * TC_BN) : umma_idesc_bf16(TC_BM, 2 * TC_BN);
             // Descriptor of stage 0 / operand 0; the others differ only in the start-address field,
@@ -299,7 +305,7 @@ tc_candidates_kernel(const TcParams p) {
                 }
                 for (uint32_t t = 0; t < tiles && ok; t += step) {
                     const uint32_t idesc = (tiles - t >= 2 && step == 2) ? idesc_two : idesc_one;
-                    if (tiles_started >= 2) {
+                    if (tiles_started >= n_acc) {
                         // the epilogue must have drained this accumulator's previous tile
                         ok = mbar_wait(&sh.acc_free[acc], acc_phase ^ 1u, p.spin_limit);
                         if (!ok) {
@@ -314,27 +320,27 @@ tc_candidates_kernel(const TcParams p) {
                             break;
                         }
                         tc_fence_after_sync();
-#pragma unroll
-                        for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
 #ifdef VB200_TC_DIAG
-                            if ((p.diag & 2u) != 0) {
-                                continue;
-                            }
+                        if ((p.diag & 2u) == 0)
 #endif
+                        for (uint32_t t2 = 0; t2 < a_tiles; ++t2) {
+                            const uint32_t d = d_tmem + t2 * tile_cols;
+                            const uint64_t a_at = a_res ? desc0 + (c * a_tiles + t2) * n_terms_op * op_units : stage_desc + t2 * n_terms_op * op_units;
+                            const uint64_t b_at = a_res ? stage_desc : stage_desc + a_tiles * n_terms_op * op_units;
                             // a k-step of 16 elements = two 8-element cores: 256 B = 16 descriptor units
-                            const uint64_t koff = kk * 16;
-                            const uint32_t accumulate = (c == 0 && kk == 0) ? 0u : 1u;
                             if (p.n_terms == 3) {
-                                const uint64_t a_hi = (a_res ? desc0 + c * 2 * op_units : stage_desc) + koff;
-                                const uint64_t b_hi = (a_res ? stage_desc : stage_desc + 2 * op_units) + koff;
-                                const uint64_t a_lo = a_hi + op_units, b_lo = b_hi + step * op_units;
-                                umma_bf16(d_tmem, a_hi, b_hi, idesc, accumulate);
-                                umma_bf16(d_tmem, a_hi, b_lo, idesc, 1u);
-                                umma_bf16(d_tmem, a_lo, b_hi, idesc, 1u);
+                                const uint64_t b_lo = b_at + step * op_units;
+#pragma unroll
+                                for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
+                                    umma_bf16(d, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
+                                    umma_bf16(d, a_at + kk * 16, b_lo + kk * 16, idesc, 1u);
+                                    umma_bf16(d, a_at + op_units + kk * 16, b_at + kk * 16, idesc, 1u);
+                                }
                             } else {
-                                const uint64_t a = (a_res ? desc0 + c * op_units : stage_desc) + koff;
-                                const uint64_t b = (a_res ? stage_desc : stage_desc + op_units) + koff;
-                                umma_bf16(d_tmem, a, b, idesc, accumulate);
+#pragma unroll
+                                for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
+                                    umma_bf16(d, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
+                                }
                             }
                         }
                         umma_commit(&sh.freed[m_stage]);
@@ -352,7 +358,7 @@ tc_candidates_kernel(const TcParams p) {
                         }
                     }
                     ++tiles_started;
-                    if (++acc == 2) {
+                    if (++acc == n_acc) {
                         acc = 0;
                         acc_phase ^= 1u;
                     }
@@ -368,7 +374,7 @@ tc_candidates_kernel(const TcParams p) {
         // ---------------- operand copies: one thread for A, one for B ----------------
         // The copy engine of an SM moves a 16 KiB bulk copy at well under the rate the MMAs eat
         // operands when a single thread issues them one after the other; two issuers overlap.
-        if (lane == 0) {
+        if (elect_one()) {
             const bool is_a = warp == TC_EPI_WARPS + 1;
             const TcOperand& op = is_a ? p.a : p.b;
             const uint32_t terms = n_terms_op;
@@ -392,24 +398,26 @@ tc_candidates_kernel(const TcParams p) {
                     }
                     mbar_expect_tx(&sh.a_full, a_region_bytes);
                     for (uint32_t c = 0; c < chunks; ++c) {
-                        const size_t off = (static_cast<size_t>(mtile) * chunks + c) * TC_CHUNK_ELEMS;
-                        unsigned char* dst = smem + c * terms * TC_CHUNK_BYTES;
-                        bulk_copy_g2s(dst, op.hi + off, TC_CHUNK_BYTES, &sh.a_full);
-                        if (terms == 2) {
-                            bulk_copy_g2s(dst + TC_CHUNK_BYTES, op.lo + off, TC_CHUNK_BYTES, &sh.a_full);
+                        for (uint32_t t2 = 0; t2 < a_tiles; ++t2) {
+                            const size_t off = (static_cast<size_t>(a_tile(mtile, t2)) * chunks + c) * TC_CHUNK_ELEMS;
+                            unsigned char* dst = smem + (c * a_tiles + t2) * terms * TC_CHUNK_BYTES;
+                            bulk_copy_g2s(dst, op.hi + off, TC_CHUNK_BYTES, &sh.a_full);
+                            if (terms == 2) {
+                                bulk_copy_g2s(dst + TC_CHUNK_BYTES, op.lo + off, TC_CHUNK_BYTES, &sh.a_full);
+                            }
                         }
                     }
                     ++n_loaded;
                 }
             } else {
                 // ring of stages; in resident-A mode the B thread fills whole stages
-                const uint32_t op_off = (is_a || a_res) ? 0u : terms * TC_CHUNK_BYTES;   // A terms first, then B terms
+                const uint32_t op_off = (is_a || a_res) ? 0u : a_tiles * terms * TC_CHUNK_BYTES;   // A first, then B
                 uint32_t stage = 0, phase = 0, count = 0;
                 for (uint32_t item = blockIdx.x; item < n_items32 && ok; item += gridDim.x) {
                     uint32_t mtile, split, tiles;
                     open_item(item, mtile, split, tiles);
                     for (uint32_t t = 0; t < tiles && ok; t += step) {
-                        const uint32_t here = is_a ? 1u : (tiles - t >= step ? step : 1u);   // B tiles of this step
+                        const uint32_t here = is_a ? a_tiles : (tiles - t >= step ? step : 1u);   // tiles of this step
                         for (uint32_t c = 0; c < chunks; ++c) {
                             if (count >= p.stages) {
                                 // the stage's previous use must have been consumed by the tensor core
@@ -421,13 +429,13 @@ tc_candidates_kernel(const TcParams p) {
                             unsigned char* dst = smem + a_region_bytes + stage * stage_bytes + op_off;
                             mbar_expect_tx(&sh.full[stage], terms * here * TC_CHUNK_BYTES);
                             for (uint32_t slot = 0; slot < here; ++slot) {
-                                const size_t row_tile = is_a ? mtile : tile_at(split, mtile, tiles, t + slot);
+                                const size_t row_tile = is_a ? a_tile(mtile, slot) : tile_at(split, mtile, tiles, t + slot);
                                 const size_t off = (row_tile * chunks + c) * TC_CHUNK_ELEMS;
-                                const uint32_t slots = is_a ? 1u : step;   // slots per term in the stage
-                                bulk_copy_g2s(dst + slot * TC_CHUNK_BYTES, op.hi + off, TC_CHUNK_BYTES, &sh.full[stage]);
+                                // A: tile by tile with its terms together; B: term by term (one MMA spans its tiles)
+                                const uint32_t hi_at = is_a ? slot * terms : slot, lo_at = is_a ? slot * terms + 1 : step + slot;
+                                bulk_copy_g2s(dst + hi_at * TC_CHUNK_BYTES, op.hi + off, TC_CHUNK_BYTES, &sh.full[stage]);
                                 if (terms == 2) {
-                                    bulk_copy_g2s(dst + (slots + slot) * TC_CHUNK_BYTES, op.lo + off, TC_CHUNK_BYTES,
-                                                  &sh.full[stage]);
+                                    bulk_copy_g2s(dst + lo_at * TC_CHUNK_BYTES, op.lo + off, TC_CHUNK_BYTES, &sh.full[stage]);
                                 }
                             }
                             ++count;
@@ -446,10 +454,14 @@ tc_candidates_kernel(const TcParams p) {
         __syncwarp();
     } else {
         // ---------------- epilogue: drain the accumulator, keep the m best per row ----------------
-        const uint32_t quarter = warp & 3u;          // TMEM lanes 32 * quarter .. + 31
-        const uint32_t cgroup = warp >> 2;           // columns 32 * cgroup .. + 31 of every tile
-        const uint32_t row = quarter * 32 + lane;
-        uint64_t* buf = p.scratch + ((static_cast<uint64_t>(blockIdx.x) * TC_BM + row) * TC_COL_GROUPS + cgroup) * p.cap;
+        // A warp drains 32 rows (a quarter of an A tile's TMEM lanes) of a share of the step's columns: four warps share
+        // a row, or two when the other two have the second A tile.
+        const uint32_t quarter = warp & 3u;
+        const uint32_t groups = TC_COL_GROUPS / a_tiles;
+        const uint32_t a_sub = (warp >> 2) / groups, cgroup = (warp >> 2) % groups;
+        const uint32_t warp_cols = tile_cols / groups, halves = warp_cols / 32;
+        const uint32_t row = a_sub * TC_BM + quarter * 32 + lane, item_rows = a_tiles * TC_BM;
+        uint64_t* buf = p.scratch + ((static_cast<uint64_t>(blockIdx.x) * item_rows + row) * groups + cgroup) * p.cap;
         uint64_t* sort_area = reinterpret_cast<uint64_t*>(smem + a_region_bytes + static_cast<size_t>(p.stages) * stage_bytes) +
                               static_cast<size_t>(warp) * p.cap;
         uint64_t gtile = 0;
@@ -459,7 +471,7 @@ tc_candidates_kernel(const TcParams p) {
             open_item(static_cast<uint32_t>(item), m_tile32, split32, tiles32);
             const uint64_t m_tile = m_tile32, split = split32;
             const uint64_t t0 = 0, t1 = tiles32;   // the item's B tiles by their number within its share
-            const uint64_t grow = m_tile * TC_BM + row;
+            const uint64_t grow = m_tile * item_rows + row;
             const bool valid_row = grow < p.a.rows;
             uint32_t cnt = 0;
             float thr = INFINITY;
@@ -469,16 +481,15 @@ tc_candidates_kernel(const TcParams p) {
             }
             if (THRESH) {
                 thr = valid_row ? __ldg(p.row_bound + grow) : -INFINITY;
-                list = p.out + ((grow * p.n_split + split) * TC_COL_GROUPS + cgroup) * p.cap;
+                list = p.out + ((grow * p.n_split + split) * groups + cgroup) * p.cap;
             }
             // bias of the warp's 32 columns: fetched one tile ahead into a register (lane = column),
             // handed to the other lanes through the warp's own shared-memory slot
             const bool has_bias = p.bias != nullptr;
             // first global column of this warp's block `half` in the tile step that starts at B tile t
             auto block_col = [&](uint64_t t, uint32_t half) -> uint64_t {
-                return p.wide ? static_cast<uint64_t>(tile_at(split32, m_tile32, tiles32, static_cast<uint32_t>(t) + (cgroup >> 1))) * TC_BN +
-                                    (cgroup & 1u) * 64 + half * 32
-                              : static_cast<uint64_t>(tile_at(split32, m_tile32, tiles32, static_cast<uint32_t>(t))) * TC_BN + cgroup * 32;
+                const uint32_t col = cgroup * warp_cols + half * 32;   // within the step's columns
+                return static_cast<uint64_t>(tile_at(split32, m_tile32, tiles32, static_cast<uint32_t>(t) + col / TC_BN)) * TC_BN + col % TC_BN;
             };
             float next_bias = 0.f;
             if (has_bias) {
@@ -491,30 +502,30 @@ tc_candidates_kernel(const TcParams p) {
             float bound = (margin >= 0.f && p.row_bound != nullptr) ? __ldg(p.row_bound + grow) + margin : INFINITY;
             uint32_t bc0 = 0xFFFFFFFFu, bc1 = 0xFFFFFFFFu, bc2 = 0xFFFFFFFFu, bc3 = 0xFFFFFFFFu;
             for (uint64_t t = t0; t < t1 && ok; t += step, ++gtile) {
-                const uint32_t acc = static_cast<uint32_t>(gtile & 1);
-                ok = mbar_wait_warp(&sh.acc_full[acc], static_cast<uint32_t>((gtile >> 1) & 1), p.spin_limit);
+                const uint32_t acc = n_acc == 2 ? static_cast<uint32_t>(gtile & 1) : 0u;
+                ok = mbar_wait_warp(&sh.acc_full[acc], static_cast<uint32_t>((n_acc == 2 ? gtile >> 1 : gtile) & 1), p.spin_limit);
                 if (!ok) {
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t here = (t1 - t >= step) ? step : 1u;              // B tiles in this step
-                const bool tile_present = p.wide ? (cgroup >> 1) < here : true;  // this warp's B tile exists
-                for (uint32_t half = 0; half < step; ++half) {
-                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * acc_cols +
-                                       (p.wide ? cgroup * 64 + half * 32 : cgroup * 32);
+                for (uint32_t half = 0; half < halves; ++half) {
+                const uint32_t step_col = cgroup * warp_cols + half * 32;
+                const bool tile_present = step_col / TC_BN < here;              // the block's B tile exists
+                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * acc_cols + a_sub * tile_cols + step_col;
                 const uint64_t n0 = block_col(t, half);
                 const bool whole_tile = valid_row && tile_present && n0 + 32 <= p.b.rows;
                 if (has_bias) {
                     __syncwarp();
                     sh.bias[warp][lane] = next_bias;
-                    const bool more = half + 1 < step || t + step < t1;
-                    const uint64_t nn = (half + 1 < step ? n0 + 32 : block_col(t + step, 0)) + lane;
+                    const bool more = half + 1 < halves || t + step < t1;
+                    const uint64_t nn = (half + 1 < halves ? block_col(t, half + 1) : block_col(t + step, 0)) + lane;
                     next_bias = (more && nn < p.b.rows) ? __ldg(p.bias + nn) : 0.f;
                     __syncwarp();
                 }
                 uint32_t r[32];
                 tmem_load_32(taddr, r);
-                if (half + 1 == step) {
+                if (half + 1 == halves) {
                     // the accumulator is in registers now: hand it back before doing the selection
                     tc_fence_before_sync();
                     __syncwarp();
@@ -686,7 +697,7 @@ tc_candidates_kernel(const TcParams p) {
             }
             if (THRESH) {
                 if (valid_row) {
-                    p.out_count[(grow * p.n_split + split) * TC_COL_GROUPS + cgroup] = cnt;
+                    p.out_count[(grow * p.n_split + split) * groups + cgroup] = cnt;
                     if (cnt > p.cap) {
                         atomicOr(p.error_flag, 2);
                     }
@@ -701,7 +712,7 @@ tc_candidates_kernel(const TcParams p) {
                     }
                 }
                 if (valid_row) {
-                    uint64_t* dst = p.out + ((grow * p.n_split + split) * TC_COL_GROUPS + cgroup) * p.m;
+                    uint64_t* dst = p.out + ((grow * p.n_split + split) * groups + cgroup) * p.m;
                     const float fs[4] = {bs0, bs1, bs2, bs3};
                     const uint32_t fc[4] = {bc0, bc1, bc2, bc3};
 #pragma unroll
@@ -720,10 +731,10 @@ tc_candidates_kernel(const TcParams p) {
 #endif
                 for (uint32_t owner = 0; owner < 32; ++owner) {
                     tc_compact_row(buf, cnt, thr, owner, lane, p.m, sort_area);
-                    const uint64_t orow = m_tile * TC_BM + quarter * 32 + owner;
+                    const uint64_t orow = m_tile * item_rows + a_sub * TC_BM + quarter * 32 + owner;
                     if (orow < p.a.rows) {
                         uint32_t c = __shfl_sync(0xffffffffu, cnt, owner);
-                        uint64_t* dst = p.out + ((orow * p.n_split + split) * TC_COL_GROUPS + cgroup) * p.m;
+                        uint64_t* dst = p.out + ((orow * p.n_split + split) * groups + cgroup) * p.m;
                         for (uint32_t i = lane; i < p.m; i += 32) {
                             dst[i] = i < c ? sort_area[i] : KEY_INF;
                         }
@@ -748,13 +759,13 @@ tc_candidates_kernel(const TcParams p) {
         __syncthreads();
     }
     if (warp == TC_EPI_WARPS) {
-        tmem_dealloc(tmem_base, 2 * acc_cols);
+        tmem_dealloc(tmem_base, n_acc * acc_cols);
     }
 }
 
 // Shared memory a launch may use for operand stages and sort areas (the rest of the 227 KiB holds
 // the barriers, the bias slots and alignment slack).
-constexpr size_t TC_SMEM_BUDGET = 232448 - 4096;
+constexpr size_t TC_SMEM_BUDGET = 232448 - 3072;
 constexpr uint32_t TC_MIN_STAGES = 2;
 
 static size_t
@@ -773,32 +784,46 @@ tc_cap_max(uint32_t n_terms) {
     return cap_max;
 }
 
-// Shared-memory plan of a launch: whether the A tile of an item stays resident (it does when it
-// is at most 64 KiB, i.e. up to 128 dimensions of split fp32 or 256 of bf16: every B tile of the
-// item then costs only its own bytes), and as many ring stages as fit beside it and the sort
-// areas.  VB200_TC_STAGES / VB200_TC_A_RESIDENT=0 override the choices (for experiments).
+// Shared-memory plan of a launch.  What bounds the kernel is the rate at which an SM takes operand tiles out of L2
+// (28 to 36 bytes a cycle measured, with and without the MMAs), so the plan asks for the fewest operand bytes per
+// 128 x 128 block of products:
+//   * the A tiles of an item stay resident when they take at most 64 KiB (128 KiB as a pair): every B tile of the item
+//     then costs only its own bytes;
+//   * pair: two row tiles of A share every B tile, half the B bytes.  It needs enough row tiles that items of 256 rows
+//     still fill the SMs (16 here: with fewer, the launch is short and its items are what is scarce), and room for
+//     three stages.  With resident A the two accumulators of a step are 2 x 128 columns and double-buffered; streamed A
+//     of one term takes both, two B tiles as well (256 x 256 in all 512 columns: 64 KiB per four blocks instead of 96);
+//   * wide: otherwise two B tiles per MMA, with one-term inputs or resident A.
+// VB200_TC_STAGES / VB200_TC_A_RESIDENT=0 / VB200_TC_WIDE=0 / VB200_TC_PAIR=0 override the choices (for experiments).
 static void
 tc_plan(TcParams& p, size_t sort_bytes, size_t* smem_bytes) {
     const uint32_t terms = p.n_terms == 3 ? 2u : 1u;
     const size_t chunk = TC_CHUNK_BYTES;
-    const size_t a_region = static_cast<size_t>(p.a.chunks) * terms * chunk;
-    const char* env_res = std::getenv("VB200_TC_A_RESIDENT");
-    const char* env_wide = std::getenv("VB200_TC_WIDE");
-    bool resident = a_region <= 65536 && !(env_res != nullptr && env_res[0] == '0');
-    auto stage_bytes = [&](bool res, bool wide) { return ((res ? 0 : terms) + terms * (wide ? 2 : 1)) * chunk; };
-    auto fits = [&](bool res, bool wide, uint32_t stages) {
-        return sort_bytes + (res ? a_region : 0) + stages * stage_bytes(res, wide) <= TC_SMEM_BUDGET;
+    const uint64_t m_tiles = (p.a.rows + TC_BM - 1) / TC_BM;
+    const size_t a_tile_bytes = static_cast<size_t>(p.a.chunks) * terms * chunk;
+    auto off = [](const char* name) {
+        const char* env = std::getenv(name);
+        return env != nullptr && env[0] == '0';
     };
-    if (resident && !fits(true, false, TC_MIN_STAGES)) {
-        resident = false;
-    }
-    // Two B tiles per MMA whenever a stage stays affordable: bf16 inputs, or a resident A tile.
-    bool wide = (terms == 1 || resident) && !(env_wide != nullptr && env_wide[0] == '0');
-    if (wide && !fits(resident, true, TC_MIN_STAGES)) {
+    auto stage_bytes = [&](bool res, bool pair, bool wide) {
+        return ((res ? 0 : terms * (pair ? 2 : 1)) + terms * (wide ? 2 : 1)) * chunk;
+    };
+    auto fits = [&](bool res, bool pair, bool wide, uint32_t stages) {
+        return sort_bytes + (res ? a_tile_bytes * (pair ? 2 : 1) : 0) + stages * stage_bytes(res, pair, wide) <= TC_SMEM_BUDGET;
+    };
+    bool resident = a_tile_bytes <= 65536 && !off("VB200_TC_A_RESIDENT");
+    bool pair = m_tiles >= 16 && !off("VB200_TC_PAIR"), wide = false;
+    if (pair && resident && fits(true, true, false, 3)) {
         wide = false;
+    } else if (pair && !resident && terms == 1 && fits(false, true, true, 3)) {
+        wide = true;
+    } else {
+        pair = false;
+        resident = resident && fits(true, false, false, TC_MIN_STAGES);
+        wide = (terms == 1 || resident) && !off("VB200_TC_WIDE") && fits(resident, false, true, TC_MIN_STAGES);
     }
-    const size_t fixed = sort_bytes + (resident ? a_region : 0);
-    uint32_t stages = static_cast<uint32_t>((TC_SMEM_BUDGET - fixed) / stage_bytes(resident, wide));
+    const size_t fixed = sort_bytes + (resident ? a_tile_bytes * (pair ? 2 : 1) : 0);
+    uint32_t stages = static_cast<uint32_t>((TC_SMEM_BUDGET - fixed) / stage_bytes(resident, pair, wide));
     if (stages > TC_MAX_STAGES) {
         stages = TC_MAX_STAGES;
     }
@@ -812,7 +837,20 @@ tc_plan(TcParams& p, size_t sort_bytes, size_t* smem_bytes) {
     p.stages = stages;
     p.a_resident = resident ? 1u : 0u;
     p.wide = wide ? 1u : 0u;
-    *smem_bytes = fixed + stages * stage_bytes(resident, wide) + 1024;
+    p.pair = pair ? 1u : 0u;
+    *smem_bytes = fixed + stages * stage_bytes(resident, pair, wide);
+}
+
+// Items of a launch per share of B (row tiles, or pairs of them), and the lists that every row has per share.
+static uint64_t
+tc_row_items(const TcParams& p) {
+    const uint64_t rows = p.pair ? 2 * TC_BM : TC_BM;
+    return (p.a.rows + rows - 1) / rows;
+}
+
+static uint32_t
+tc_groups(const TcParams& p) {
+    return p.pair ? TC_COL_GROUPS / 2 : TC_COL_GROUPS;
 }
 
 uint32_t
@@ -831,7 +869,26 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_candidates: operand depths differ");
     VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_candidates: 1 or 3 terms");
     VB_CHECK_ARG(m >= 1 && m <= 480, "tc_candidates: m out of range");
-    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
+    TcParams p{};
+    p.a = a;
+    p.b = b;
+    p.n_terms = n_terms;
+    // Per-row candidate buffers: a few times m so compactions are rare, within what the per-warp
+    // shared-memory sort areas can hold next to the operand stages.
+    {
+        const uint32_t cap_max = tc_cap_max(n_terms);
+        uint32_t cap = next_pow2(4 * m < 64 ? 64 : 4 * m);
+        if (cap > cap_max) {
+            cap = cap_max;
+        }
+        VB_CHECK_ARG(m <= 4 || m + 32 <= cap, "tc_candidates: m = %u too large for the shared-memory sort area", m);
+        p.cap = cap;
+    }
+    const bool small_m = m <= 4;
+    const size_t sort_bytes = small_m ? 0 : TC_EPI_WARPS * static_cast<size_t>(p.cap) * sizeof(uint64_t);
+    size_t smem = 0;
+    tc_plan(p, sort_bytes, &smem);
+    const uint64_t m_tiles = tc_row_items(p);
     const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     uint64_t n_split = (2ull * sms + m_tiles - 1) / m_tiles;
@@ -874,10 +931,6 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     const uint64_t items = m_tiles * n_split;
     const uint32_t grid = static_cast<uint32_t>(items < sms ? items : sms);
 
-    TcParams p{};
-    p.a = a;
-    p.b = b;
-    p.n_terms = n_terms;
     p.half = half ? 1u : 0u;
     p.alpha = alpha;
     p.bias = bias_dev;
@@ -902,23 +955,12 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     p.row_margin = row_margin_dev;
     p.row_bound = row_bound_dev;
     p.m = m;
-    // Per-row candidate buffers: a few times m so compactions are rare, within what the per-warp
-    // shared-memory sort areas can hold next to the operand stages.
-    {
-        const uint32_t cap_max = tc_cap_max(n_terms);
-        uint32_t cap = next_pow2(4 * m < 64 ? 64 : 4 * m);
-        if (cap > cap_max) {
-            cap = cap_max;
-        }
-        VB_CHECK_ARG(m <= 4 || m + 32 <= cap, "tc_candidates: m = %u too large for the shared-memory sort area", m);
-        p.cap = cap;
-    }
     p.n_split = static_cast<uint32_t>(n_split);
     p.tiles_per_split = static_cast<uint32_t>(tiles_per_split);
     p.col_base = col_base;
     VB_TRY(ws.scratch.reserve(static_cast<size_t>(grid) * TC_BM * TC_COL_GROUPS * p.cap));
     VB_TRY(ws.error_flag.reserve(2));
-    VB_TRY(out.reserve(static_cast<size_t>(a.rows) * n_split * TC_COL_GROUPS * m));
+    VB_TRY(out.reserve(static_cast<size_t>(a.rows) * n_split * tc_groups(p) * m));
     VB_CUDA(cudaMemsetAsync(ws.error_flag.ptr, 0, 2 * sizeof(int), current_stream()));
     p.scratch = ws.scratch.ptr;
     p.out = out.ptr;
@@ -926,10 +968,6 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     p.spin_limit = tc_spin_limit();
     p.row_flags = row_flags_dev;
 
-    const bool small_m = m <= 4;
-    const size_t sort_bytes = small_m ? 0 : TC_EPI_WARPS * static_cast<size_t>(p.cap) * sizeof(uint64_t);
-    size_t smem = 0;
-    tc_plan(p, sort_bytes, &smem);
     auto kernel = small_m ? tc_candidates_kernel<0> : tc_candidates_kernel<1>;
     VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     VB_LAUNCH(kernel, grid, TC_THREADS, smem, p);
@@ -939,7 +977,7 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     if ((flags[0] & 1) != 0) {
         VB_FAIL(VB200_INTERNAL_ERROR, "tensor-core kernel gave up on a bounded wait");
     }
-    *n_split_out = static_cast<uint32_t>(n_split) * TC_COL_GROUPS;
+    *n_split_out = static_cast<uint32_t>(n_split) * tc_groups(p);
     if (n_flagged_out != nullptr) {
         *n_flagged_out = static_cast<uint32_t>(flags[1]);
     }
@@ -955,7 +993,13 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
     VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_below_threshold: operand depths differ");
     VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_below_threshold: 1 or 3 terms");
     VB_CHECK_ARG(row_thr_dev != nullptr, "tc_below_threshold: thresholds missing");
-    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
+    TcParams p{};
+    p.a = a;
+    p.b = b;
+    p.n_terms = n_terms;
+    size_t smem = 0;
+    tc_plan(p, 0, &smem);
+    const uint64_t m_tiles = tc_row_items(p);
     const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     // More column ranges per row tile than the sorted modes take: a list costs nothing but its
@@ -975,7 +1019,7 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
     }
     const uint64_t tiles_per_split = (n_tiles + n_split - 1) / n_split;
     n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
-    const uint32_t lists = static_cast<uint32_t>(n_split) * TC_COL_GROUPS;
+    const uint32_t lists = static_cast<uint32_t>(n_split) * tc_groups(p);
     // list capacity: a list's expected share plus eight standard deviations of a Poisson count and a few more
     // (3.5 x the share at least), within the caller's limit per row.  An overflowing list costs its row a slow
     // exact answer, and with many short lists per row a multiple of the mean alone is passed every few thousand lists.
@@ -995,10 +1039,6 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
                  lists, max_per_row);
     const uint64_t items = m_tiles * n_split;
     const uint32_t grid = static_cast<uint32_t>(items < sms ? items : sms);
-    TcParams p{};
-    p.a = a;
-    p.b = b;
-    p.n_terms = n_terms;
     p.alpha = alpha;
     p.bias = bias_dev;
     p.row_bound = row_thr_dev;
@@ -1016,8 +1056,6 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
     p.out_count = out_count.ptr;
     p.error_flag = deferred_flag_dev != nullptr ? deferred_flag_dev : ws.error_flag.ptr;
     p.spin_limit = tc_spin_limit();
-    size_t smem = 0;
-    tc_plan(p, 0, &smem);
     auto kernel = tc_candidates_kernel<3>;
     VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     VB_LAUNCH(kernel, grid, TC_THREADS, smem, p);
@@ -1047,7 +1085,13 @@ tc_scores(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_te
     VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_scores: 1 or 3 terms");
     VB_CHECK_ARG(ld >= b.rows && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(scores_dev) & 15) == 0,
                  "tc_scores: the score matrix must be 16-byte aligned with a row stride that is a multiple of 4");
-    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
+    TcParams p{};
+    p.a = a;
+    p.b = b;
+    p.n_terms = n_terms;
+    size_t smem = 0;
+    tc_plan(p, 0, &smem);
+    const uint64_t m_tiles = tc_row_items(p);
     const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     uint64_t n_split = (2ull * sms + m_tiles - 1) / m_tiles;
@@ -1061,10 +1105,6 @@ tc_scores(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_te
     n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
     const uint64_t items = m_tiles * n_split;
     const uint32_t grid = static_cast<uint32_t>(items < sms ? items : sms);
-    TcParams p{};
-    p.a = a;
-    p.b = b;
-    p.n_terms = n_terms;
     p.alpha = alpha;
     p.bias = bias_dev;
     p.m = 0;
@@ -1079,8 +1119,6 @@ tc_scores(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_te
     }
     p.error_flag = deferred_flag_dev != nullptr ? deferred_flag_dev : ws.error_flag.ptr;
     p.spin_limit = tc_spin_limit();
-    size_t smem = 0;
-    tc_plan(p, 0, &smem);
     auto kernel = tc_candidates_kernel<2>;
     VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     VB_LAUNCH(kernel, grid, TC_THREADS, smem, p);

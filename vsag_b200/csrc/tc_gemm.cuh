@@ -28,7 +28,7 @@ constexpr uint32_t TC_BN = 128;           // rows of B (output columns) per tile
 constexpr uint32_t TC_KC = 64;            // k elements per chunk
 constexpr uint32_t TC_CHUNK_ELEMS = 128 * TC_KC;
 constexpr uint32_t TC_CHUNK_BYTES = TC_CHUNK_ELEMS * 2;   // 16 KiB
-constexpr uint32_t TC_COL_GROUPS = 4;      // epilogue warps per TMEM lane quarter; each takes 32 of a tile's columns
+constexpr uint32_t TC_COL_GROUPS = 4;      // epilogue warps per TMEM lane quarter
 constexpr uint32_t TC_EPI_WARPS = 4 * TC_COL_GROUPS;
 constexpr uint32_t TC_EPI_THREADS = 32 * TC_EPI_WARPS;
 constexpr uint32_t TC_THREADS = TC_EPI_THREADS + 96;   // + one warp each to issue the MMAs, the A copies and the B copies
@@ -53,7 +53,8 @@ struct TcParams {
     uint32_t cap;             // per-row buffer, power of two >= m + 32
     uint32_t stages;          // operand stages in shared memory (2 .. 6)
     uint32_t a_resident;      // 1: the A tile of a work item stays in shared memory for all its B tiles
-    uint32_t wide;            // 1: two B tiles per MMA (128 x 256 x 16), 512 TMEM columns
+    uint32_t wide;            // 1: two B tiles per MMA (128 x 256 x 16)
+    uint32_t pair;            // 1: a work item is two row tiles of A: every B tile fetched serves 256 rows
     uint32_t n_split;         // shares of B's tiles per row tile
     uint32_t tiles_per_split; // B tiles per share when the shares are contiguous
 #ifdef VB200_TC_DIAG
@@ -61,10 +62,10 @@ struct TcParams {
 #endif
     uint32_t window;          // 0, or a power of two: tiles per window of the staggered walk over a share
     uint32_t interleaved;     // 1: share s holds tiles s, s + n_split, ...; the queue walks row tiles within a share
-    uint64_t* scratch;        // [grid][128][TC_COL_GROUPS][cap] candidate buffers
-    uint64_t* out;            // [a.rows][n_split][TC_COL_GROUPS][m] keys (ordered score << 32 | column), KEY_INF padded
-                              // (threshold mode: [a.rows][n_split][TC_COL_GROUPS][cap], unsorted, with out_count)
-    uint32_t* out_count;      // threshold mode: [a.rows][n_split][TC_COL_GROUPS] entries offered to each list
+    uint64_t* scratch;        // [grid][rows of an item][lists][cap] candidate buffers
+    uint64_t* out;            // [a.rows][n_split][groups][m] keys (ordered score << 32 | column), KEY_INF padded; groups = the
+                              // epilogue warps that share a row, tc_groups() (threshold mode: [...][cap], unsorted, with out_count)
+    uint32_t* out_count;      // threshold mode: [a.rows][n_split][groups] entries offered to each list
     uint32_t col_base;        // added to column indices in the keys
     float* store;             // score-matrix mode: [a.rows][store_ld] fp32 scores instead of candidates
     uint64_t store_ld;        // row stride of `store` in floats (multiple of 4, store 16-byte aligned)
@@ -190,6 +191,19 @@ umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uin
         : "memory");
 }
 
+// One thread of a converged warp.  By elect.sync and not by a lane number: the compiler then knows that a single thread
+// is inside and feeds the MMA and bulk-copy instructions, whose operands are warp-uniform, without a loop over lanes.
+__device__ __forceinline__ bool
+elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(one));
+    return one != 0;
+}
+
 // Arrives on `bar` once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void
 umma_commit(uint64_t* bar) {
@@ -274,7 +288,7 @@ struct TcWorkspace {
 };
 
 // For every row of A the m best columns of B by alpha * <a, b> + bias, as keys in
-// out_dev[a_rows][n_split * TC_COL_GROUPS][m]; the number of lists per row (n_split * TC_COL_GROUPS) is
+// out_dev[a_rows][lists][m]; the number of lists per row is
 // chosen here and returned in n_split_out.
 // n_terms: 1, 3, or TC_HALF for one scaled fp16 term per operand (alpha then undoes the scales).
 // row_margin_dev (optional, m <= 4 only): per row twice the largest error of a score; columns scoring worse than the
