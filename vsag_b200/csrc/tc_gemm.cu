@@ -196,28 +196,23 @@ tc_candidates_kernel(const TcParams p) {
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t n_terms_op = p.n_terms == 3 ? 2u : 1u;                       // bf16 terms per operand
     // resident-A mode: [A tile: chunks x terms][ring of B stages]; otherwise a ring of [A terms][B terms]
-    // pair mode: an item has two A tiles ([chunk][tile][term]), each with accumulators of its own
-    const uint32_t a_tiles = p.pair ? 2u : 1u;
-    const uint32_t a_region_bytes = p.a_resident ? p.a.chunks * a_tiles * n_terms_op * TC_CHUNK_BYTES : 0u;
+    const uint32_t a_region_bytes = p.a_resident ? p.a.chunks * n_terms_op * TC_CHUNK_BYTES : 0u;
     // wide mode: a stage holds two consecutive B tiles, term by term ([hi t][hi t+1][lo t][lo t+1]), so
     // that one 128 x 256 x 16 MMA reads both; the accumulators are 256 columns each.
     const uint32_t step = p.wide ? 2u : 1u;
-    const uint32_t tile_cols = step * TC_BN;             // tensor-memory columns of one A tile
-    const uint32_t acc_cols = a_tiles * tile_cols;
-    const uint32_t n_acc = acc_cols > 256 ? 1u : 2u;     // accumulators: two while they fit the 512 columns
-    const uint32_t stage_bytes = ((p.a_resident ? 0u : n_terms_op * a_tiles) + n_terms_op * step) * TC_CHUNK_BYTES;
+    const uint32_t acc_cols = step * TC_BN;
+    const uint32_t stage_bytes = ((p.a_resident ? 0u : n_terms_op) + n_terms_op * step) * TC_CHUNK_BYTES;
     const uint32_t chunks = p.a.chunks;
     const uint64_t m_tiles = (p.a.rows + TC_BM - 1) / TC_BM;
     const uint64_t n_tiles = (p.b.rows + TC_BN - 1) / TC_BN;
-    const uint64_t m_units = (m_tiles + a_tiles - 1) / a_tiles;   // items per share of B
-    const uint64_t n_items = m_units * p.n_split;
+    const uint64_t n_items = m_tiles * p.n_split;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < p.stages; ++s) {
-            mbar_init(&sh.full[s], p.a_resident ? 1 : 2);   // one arrival (with its byte count) per copy thread filling it
+            mbar_init(&sh.full[s], TC_COPY_WARPS);   // one arrival (with its byte count) per copy thread
             mbar_init(&sh.freed[s], 1);
         }
-        mbar_init(&sh.a_full, 1);
+        mbar_init(&sh.a_full, TC_COPY_WARPS);
         mbar_init(&sh.a_free, 1);
         for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(&sh.acc_full[a], 1);
@@ -227,7 +222,7 @@ tc_candidates_kernel(const TcParams p) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == TC_EPI_WARPS) {
-        tmem_alloc(&sh.tmem_base, n_acc * acc_cols);
+        tmem_alloc(&sh.tmem_base, 2 * acc_cols);  // two fp32 accumulators of 128 (256 when wide) columns
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -242,10 +237,7 @@ tc_candidates_kernel(const TcParams p) {
     // queue walks the row tiles of one share before the next share, so the CTAs running at any moment
     // sweep B front to back together and a B tile fetched from DRAM by one of them is an L2 hit for the
     // others -- what a base far larger than L2 needs when there are many row tiles.
-    const uint32_t m_tiles32 = static_cast<uint32_t>(m_units);
-    // the row tile of A that tile `a` of an item copies (an odd number of tiles: the last one twice, its rows are not valid)
-    const uint32_t last_tile = static_cast<uint32_t>(m_tiles) - 1;
-    auto a_tile = [&](uint32_t unit, uint32_t a) -> uint32_t { return min(unit * a_tiles + a, last_tile); };
+    const uint32_t m_tiles32 = static_cast<uint32_t>(m_tiles);
     auto open_item = [&](uint32_t item, uint32_t& mtile, uint32_t& split, uint32_t& tiles) {
         if (p.interleaved) {
             split = item / m_tiles32;
@@ -262,18 +254,9 @@ tc_candidates_kernel(const TcParams p) {
             tiles = t1 > t0 ? t1 - t0 : 0;
         }
     };
-    // B tile number u of share `split`.  With p.window > 0 (a power of two) the share is walked in windows
-    // of that many tiles and every row tile starts each window at its own offset, wrapping round: the CTAs
-    // that sweep a share together then ask L2 for different tiles at any moment instead of all for the same
-    // lines, while a window still passes through L2 once.
-    auto tile_at = [&](uint32_t split, uint32_t mtile, uint32_t tiles, uint32_t u) -> uint32_t {
-        if (p.window != 0) {
-            const uint32_t w0 = u & ~(p.window - 1u);
-            const uint32_t len = tiles - w0 < p.window ? tiles - w0 : p.window;
-            uint32_t r = (u - w0) + ((mtile * 29u) & (p.window - 1u));
-            r = len == p.window ? (r & (p.window - 1u)) : r % len;
-            u = w0 + r;
-        }
+    // B tile number u of share `split`.  (Row tiles that start a share at different tiles, so as not to ask L2 for the
+    // same lines together, were slower: 91 against 86 ms over 6M x 768 rows.)
+    auto tile_at = [&](uint32_t split, uint32_t u) -> uint32_t {
         return p.interleaved ? split + u * p.n_split : split * p.tiles_per_split + u;
     };
     if (warp == TC_EPI_WARPS) {
@@ -305,7 +288,7 @@ tc_candidates_kernel(const TcParams p) {
                 }
                 for (uint32_t t = 0; t < tiles && ok; t += step) {
                     const uint32_t idesc = (tiles - t >= 2 && step == 2) ? idesc_two : idesc_one;
-                    if (tiles_started >= n_acc) {
+                    if (tiles_started >= 2) {
                         // the epilogue must have drained this accumulator's previous tile
                         ok = mbar_wait(&sh.acc_free[acc], acc_phase ^ 1u, p.spin_limit);
                         if (!ok) {
@@ -323,23 +306,22 @@ tc_candidates_kernel(const TcParams p) {
 #ifdef VB200_TC_DIAG
                         if ((p.diag & 2u) == 0)
 #endif
-                        for (uint32_t t2 = 0; t2 < a_tiles; ++t2) {
-                            const uint32_t d = d_tmem + t2 * tile_cols;
-                            const uint64_t a_at = a_res ? desc0 + (c * a_tiles + t2) * n_terms_op * op_units : stage_desc + t2 * n_terms_op * op_units;
-                            const uint64_t b_at = a_res ? stage_desc : stage_desc + a_tiles * n_terms_op * op_units;
+                        {
+                            const uint64_t a_at = a_res ? desc0 + c * n_terms_op * op_units : stage_desc;
+                            const uint64_t b_at = a_res ? stage_desc : stage_desc + n_terms_op * op_units;
                             // a k-step of 16 elements = two 8-element cores: 256 B = 16 descriptor units
                             if (p.n_terms == 3) {
                                 const uint64_t b_lo = b_at + step * op_units;
 #pragma unroll
                                 for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
-                                    umma_bf16(d, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
-                                    umma_bf16(d, a_at + kk * 16, b_lo + kk * 16, idesc, 1u);
-                                    umma_bf16(d, a_at + op_units + kk * 16, b_at + kk * 16, idesc, 1u);
+                                    umma_bf16(d_tmem, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
+                                    umma_bf16(d_tmem, a_at + kk * 16, b_lo + kk * 16, idesc, 1u);
+                                    umma_bf16(d_tmem, a_at + op_units + kk * 16, b_at + kk * 16, idesc, 1u);
                                 }
                             } else {
 #pragma unroll
                                 for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
-                                    umma_bf16(d, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
+                                    umma_bf16(d_tmem, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
                                 }
                             }
                         }
@@ -358,7 +340,7 @@ tc_candidates_kernel(const TcParams p) {
                         }
                     }
                     ++tiles_started;
-                    if (++acc == n_acc) {
+                    if (++acc == 2) {
                         acc = 0;
                         acc_phase ^= 1u;
                     }
@@ -371,24 +353,29 @@ tc_candidates_kernel(const TcParams p) {
         }
         __syncwarp();
     } else if (warp > TC_EPI_WARPS) {
-        // ---------------- operand copies: one thread for A, one for B ----------------
-        // The copy engine of an SM moves a 16 KiB bulk copy at well under the rate the MMAs eat
-        // operands when a single thread issues them one after the other; two issuers overlap.
+        // ---------------- operand copies ----------------
+        // What one thread has in flight moves at 34 bytes a cycle, so every 16 KiB chunk is copied in equal parts by
+        // several.
         if (elect_one()) {
-            const bool is_a = warp == TC_EPI_WARPS + 1;
-            const TcOperand& op = is_a ? p.a : p.b;
+            constexpr uint32_t PART = TC_CHUNK_BYTES / TC_COPY_WARPS;
+            const uint32_t at = (warp - (TC_EPI_WARPS + 1)) * PART;
             const uint32_t terms = n_terms_op;
             const bool a_res = p.a_resident != 0;
             bool ok = true;
-            if (is_a && a_res) {
-                // the whole A tile of an item at once, into the resident region
-                uint32_t a_phase = 0, n_loaded = 0;
-                for (uint32_t item = blockIdx.x; item < n_items32 && ok; item += gridDim.x) {
-                    uint32_t mtile, split, tiles;
-                    open_item(item, mtile, split, tiles);
-                    if (tiles == 0) {
-                        continue;
-                    }
+            // this thread's part of both terms of a chunk
+            auto copy = [&](const TcOperand& op, size_t tile, uint32_t c, unsigned char* hi, unsigned char* lo, uint64_t* bar) {
+                const size_t off = (tile * chunks + c) * TC_CHUNK_BYTES + at;
+                bulk_copy_g2s(hi + at, reinterpret_cast<const unsigned char*>(op.hi) + off, PART, bar);
+                if (terms == 2) {
+                    bulk_copy_g2s(lo + at, reinterpret_cast<const unsigned char*>(op.lo) + off, PART, bar);
+                }
+            };
+            uint32_t stage = 0, phase = 0, count = 0, a_phase = 0, n_loaded = 0;
+            for (uint32_t item = blockIdx.x; item < n_items32 && ok; item += gridDim.x) {
+                uint32_t mtile, split, tiles;
+                open_item(item, mtile, split, tiles);
+                if (a_res && tiles > 0) {
+                    // the whole A tile of the item at once, into the resident region
                     if (n_loaded > 0) {
                         ok = mbar_wait(&sh.a_free, a_phase, p.spin_limit);   // previous item's MMAs are done with it
                         a_phase ^= 1u;
@@ -396,53 +383,40 @@ tc_candidates_kernel(const TcParams p) {
                             break;
                         }
                     }
-                    mbar_expect_tx(&sh.a_full, a_region_bytes);
+                    mbar_expect_tx(&sh.a_full, a_region_bytes / TC_COPY_WARPS);
                     for (uint32_t c = 0; c < chunks; ++c) {
-                        for (uint32_t t2 = 0; t2 < a_tiles; ++t2) {
-                            const size_t off = (static_cast<size_t>(a_tile(mtile, t2)) * chunks + c) * TC_CHUNK_ELEMS;
-                            unsigned char* dst = smem + (c * a_tiles + t2) * terms * TC_CHUNK_BYTES;
-                            bulk_copy_g2s(dst, op.hi + off, TC_CHUNK_BYTES, &sh.a_full);
-                            if (terms == 2) {
-                                bulk_copy_g2s(dst + TC_CHUNK_BYTES, op.lo + off, TC_CHUNK_BYTES, &sh.a_full);
-                            }
-                        }
+                        unsigned char* dst = smem + c * terms * TC_CHUNK_BYTES;
+                        copy(p.a, mtile, c, dst, dst + TC_CHUNK_BYTES, &sh.a_full);
                     }
                     ++n_loaded;
                 }
-            } else {
-                // ring of stages; in resident-A mode the B thread fills whole stages
-                const uint32_t op_off = (is_a || a_res) ? 0u : a_tiles * terms * TC_CHUNK_BYTES;   // A first, then B
-                uint32_t stage = 0, phase = 0, count = 0;
-                for (uint32_t item = blockIdx.x; item < n_items32 && ok; item += gridDim.x) {
-                    uint32_t mtile, split, tiles;
-                    open_item(item, mtile, split, tiles);
-                    for (uint32_t t = 0; t < tiles && ok; t += step) {
-                        const uint32_t here = is_a ? a_tiles : (tiles - t >= step ? step : 1u);   // tiles of this step
-                        for (uint32_t c = 0; c < chunks; ++c) {
-                            if (count >= p.stages) {
-                                // the stage's previous use must have been consumed by the tensor core
-                                ok = mbar_wait(&sh.freed[stage], phase ^ 1u, p.spin_limit);
-                                if (!ok) {
-                                    break;
-                                }
+                for (uint32_t t = 0; t < tiles && ok; t += step) {
+                    const uint32_t here = tiles - t >= step ? step : 1u;   // B tiles of this step
+                    const uint32_t a_here = a_res ? 0u : 1u;
+                    const uint32_t b0 = tile_at(split, t), b1 = tile_at(split, t + 1);
+                    for (uint32_t c = 0; c < chunks; ++c) {
+                        if (count >= p.stages) {
+                            // the stage's previous use must have been consumed by the tensor core
+                            ok = mbar_wait(&sh.freed[stage], phase ^ 1u, p.spin_limit);
+                            if (!ok) {
+                                break;
                             }
-                            unsigned char* dst = smem + a_region_bytes + stage * stage_bytes + op_off;
-                            mbar_expect_tx(&sh.full[stage], terms * here * TC_CHUNK_BYTES);
-                            for (uint32_t slot = 0; slot < here; ++slot) {
-                                const size_t row_tile = is_a ? a_tile(mtile, slot) : tile_at(split, mtile, tiles, t + slot);
-                                const size_t off = (row_tile * chunks + c) * TC_CHUNK_ELEMS;
-                                // A: tile by tile with its terms together; B: term by term (one MMA spans its tiles)
-                                const uint32_t hi_at = is_a ? slot * terms : slot, lo_at = is_a ? slot * terms + 1 : step + slot;
-                                bulk_copy_g2s(dst + hi_at * TC_CHUNK_BYTES, op.hi + off, TC_CHUNK_BYTES, &sh.full[stage]);
-                                if (terms == 2) {
-                                    bulk_copy_g2s(dst + lo_at * TC_CHUNK_BYTES, op.lo + off, TC_CHUNK_BYTES, &sh.full[stage]);
-                                }
-                            }
-                            ++count;
-                            if (++stage == p.stages) {
-                                stage = 0;
-                                phase ^= 1u;
-                            }
+                        }
+                        unsigned char* dst = smem + a_region_bytes + stage * stage_bytes;
+                        mbar_expect_tx(&sh.full[stage], terms * (a_here + here) * PART);
+                        if (!a_res) {   // A terms first, then B terms
+                            copy(p.a, mtile, c, dst, dst + TC_CHUNK_BYTES, &sh.full[stage]);
+                            dst += terms * TC_CHUNK_BYTES;
+                        }
+                        copy(p.b, b0, c, dst, dst + step * TC_CHUNK_BYTES, &sh.full[stage]);
+                        if (here == 2) {
+                            dst += TC_CHUNK_BYTES;
+                            copy(p.b, b1, c, dst, dst + step * TC_CHUNK_BYTES, &sh.full[stage]);
+                        }
+                        ++count;
+                        if (++stage == p.stages) {
+                            stage = 0;
+                            phase ^= 1u;
                         }
                     }
                 }
@@ -454,14 +428,11 @@ tc_candidates_kernel(const TcParams p) {
         __syncwarp();
     } else {
         // ---------------- epilogue: drain the accumulator, keep the m best per row ----------------
-        // A warp drains 32 rows (a quarter of an A tile's TMEM lanes) of a share of the step's columns: four warps share
-        // a row, or two when the other two have the second A tile.
-        const uint32_t quarter = warp & 3u;
-        const uint32_t groups = TC_COL_GROUPS / a_tiles;
-        const uint32_t a_sub = (warp >> 2) / groups, cgroup = (warp >> 2) % groups;
-        const uint32_t warp_cols = tile_cols / groups, halves = warp_cols / 32;
-        const uint32_t row = a_sub * TC_BM + quarter * 32 + lane, item_rows = a_tiles * TC_BM;
-        uint64_t* buf = p.scratch + ((static_cast<uint64_t>(blockIdx.x) * item_rows + row) * groups + cgroup) * p.cap;
+        const uint32_t quarter = warp & 3u;          // TMEM lanes 32 * quarter .. + 31
+        const uint32_t cgroup = warp >> 2;           // of every step's columns a quarter: 32, or two blocks of 32
+        const uint32_t warp_cols = acc_cols / TC_COL_GROUPS;
+        const uint32_t row = quarter * 32 + lane;
+        uint64_t* buf = p.scratch + ((static_cast<uint64_t>(blockIdx.x) * TC_BM + row) * TC_COL_GROUPS + cgroup) * p.cap;
         uint64_t* sort_area = reinterpret_cast<uint64_t*>(smem + a_region_bytes + static_cast<size_t>(p.stages) * stage_bytes) +
                               static_cast<size_t>(warp) * p.cap;
         uint64_t gtile = 0;
@@ -471,7 +442,7 @@ tc_candidates_kernel(const TcParams p) {
             open_item(static_cast<uint32_t>(item), m_tile32, split32, tiles32);
             const uint64_t m_tile = m_tile32, split = split32;
             const uint64_t t0 = 0, t1 = tiles32;   // the item's B tiles by their number within its share
-            const uint64_t grow = m_tile * item_rows + row;
+            const uint64_t grow = m_tile * TC_BM + row;
             const bool valid_row = grow < p.a.rows;
             uint32_t cnt = 0;
             float thr = INFINITY;
@@ -481,20 +452,24 @@ tc_candidates_kernel(const TcParams p) {
             }
             if (THRESH) {
                 thr = valid_row ? __ldg(p.row_bound + grow) : -INFINITY;
-                list = p.out + ((grow * p.n_split + split) * groups + cgroup) * p.cap;
+                list = p.out + ((grow * p.n_split + split) * TC_COL_GROUPS + cgroup) * p.cap;
             }
-            // bias of the warp's 32 columns: fetched one tile ahead into a register (lane = column),
-            // handed to the other lanes through the warp's own shared-memory slot
+            // bias of the warp's columns: fetched a whole step ahead into registers (lane = column of a block of 32), handed
+            // to the other lanes through the warp's own shared-memory slot.  (A block ahead is less than L2 takes.)
             const bool has_bias = p.bias != nullptr;
             // first global column of this warp's block `half` in the tile step that starts at B tile t
             auto block_col = [&](uint64_t t, uint32_t half) -> uint64_t {
                 const uint32_t col = cgroup * warp_cols + half * 32;   // within the step's columns
-                return static_cast<uint64_t>(tile_at(split32, m_tile32, tiles32, static_cast<uint32_t>(t) + col / TC_BN)) * TC_BN + col % TC_BN;
+                return static_cast<uint64_t>(tile_at(split32, static_cast<uint32_t>(t) + col / TC_BN)) * TC_BN + col % TC_BN;
             };
-            float next_bias = 0.f;
+            float bias0 = 0.f, bias1 = 0.f, next0 = 0.f, next1 = 0.f;
+            auto bias_of = [&](uint64_t t, uint32_t half) -> float {
+                const uint64_t nn = t < t1 ? block_col(t, half) + lane : p.b.rows;
+                return nn < p.b.rows ? __ldg(p.bias + nn) : 0.f;
+            };
             if (has_bias) {
-                const uint64_t nn = block_col(t0, 0) + lane;
-                next_bias = (t0 < t1 && nn < p.b.rows) ? __ldg(p.bias + nn) : 0.f;
+                next0 = bias_of(t0, 0);
+                next1 = step == 2 ? bias_of(t0, 1) : 0.f;
             }
             // SMALL_M: the four best scores of the row, ascending, with their columns
             float bs0 = INFINITY, bs1 = INFINITY, bs2 = INFINITY, bs3 = INFINITY;
@@ -502,30 +477,33 @@ tc_candidates_kernel(const TcParams p) {
             float bound = (margin >= 0.f && p.row_bound != nullptr) ? __ldg(p.row_bound + grow) + margin : INFINITY;
             uint32_t bc0 = 0xFFFFFFFFu, bc1 = 0xFFFFFFFFu, bc2 = 0xFFFFFFFFu, bc3 = 0xFFFFFFFFu;
             for (uint64_t t = t0; t < t1 && ok; t += step, ++gtile) {
-                const uint32_t acc = n_acc == 2 ? static_cast<uint32_t>(gtile & 1) : 0u;
-                ok = mbar_wait_warp(&sh.acc_full[acc], static_cast<uint32_t>((n_acc == 2 ? gtile >> 1 : gtile) & 1), p.spin_limit);
+                const uint32_t acc = static_cast<uint32_t>(gtile & 1);
+                if (has_bias) {
+                    bias0 = next0;
+                    bias1 = next1;
+                    next0 = bias_of(t + step, 0);
+                    next1 = step == 2 ? bias_of(t + step, 1) : 0.f;
+                }
+                ok = mbar_wait_warp(&sh.acc_full[acc], static_cast<uint32_t>((gtile >> 1) & 1), p.spin_limit);
                 if (!ok) {
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t here = (t1 - t >= step) ? step : 1u;              // B tiles in this step
-                for (uint32_t half = 0; half < halves; ++half) {
+                for (uint32_t half = 0; half < step; ++half) {
                 const uint32_t step_col = cgroup * warp_cols + half * 32;
                 const bool tile_present = step_col / TC_BN < here;              // the block's B tile exists
-                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * acc_cols + a_sub * tile_cols + step_col;
+                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * acc_cols + step_col;
                 const uint64_t n0 = block_col(t, half);
                 const bool whole_tile = valid_row && tile_present && n0 + 32 <= p.b.rows;
                 if (has_bias) {
                     __syncwarp();
-                    sh.bias[warp][lane] = next_bias;
-                    const bool more = half + 1 < halves || t + step < t1;
-                    const uint64_t nn = (half + 1 < halves ? block_col(t, half + 1) : block_col(t + step, 0)) + lane;
-                    next_bias = (more && nn < p.b.rows) ? __ldg(p.bias + nn) : 0.f;
+                    sh.bias[warp][lane] = half == 0 ? bias0 : bias1;
                     __syncwarp();
                 }
                 uint32_t r[32];
                 tmem_load_32(taddr, r);
-                if (half + 1 == halves) {
+                if (half + 1 == step) {
                     // the accumulator is in registers now: hand it back before doing the selection
                     tc_fence_before_sync();
                     __syncwarp();
@@ -697,7 +675,7 @@ tc_candidates_kernel(const TcParams p) {
             }
             if (THRESH) {
                 if (valid_row) {
-                    p.out_count[(grow * p.n_split + split) * groups + cgroup] = cnt;
+                    p.out_count[(grow * p.n_split + split) * TC_COL_GROUPS + cgroup] = cnt;
                     if (cnt > p.cap) {
                         atomicOr(p.error_flag, 2);
                     }
@@ -712,7 +690,7 @@ tc_candidates_kernel(const TcParams p) {
                     }
                 }
                 if (valid_row) {
-                    uint64_t* dst = p.out + ((grow * p.n_split + split) * groups + cgroup) * p.m;
+                    uint64_t* dst = p.out + ((grow * p.n_split + split) * TC_COL_GROUPS + cgroup) * p.m;
                     const float fs[4] = {bs0, bs1, bs2, bs3};
                     const uint32_t fc[4] = {bc0, bc1, bc2, bc3};
 #pragma unroll
@@ -731,10 +709,10 @@ tc_candidates_kernel(const TcParams p) {
 #endif
                 for (uint32_t owner = 0; owner < 32; ++owner) {
                     tc_compact_row(buf, cnt, thr, owner, lane, p.m, sort_area);
-                    const uint64_t orow = m_tile * item_rows + a_sub * TC_BM + quarter * 32 + owner;
+                    const uint64_t orow = m_tile * TC_BM + quarter * 32 + owner;
                     if (orow < p.a.rows) {
                         uint32_t c = __shfl_sync(0xffffffffu, cnt, owner);
-                        uint64_t* dst = p.out + ((orow * p.n_split + split) * groups + cgroup) * p.m;
+                        uint64_t* dst = p.out + ((orow * p.n_split + split) * TC_COL_GROUPS + cgroup) * p.m;
                         for (uint32_t i = lane; i < p.m; i += 32) {
                             dst[i] = i < c ? sort_area[i] : KEY_INF;
                         }
@@ -759,7 +737,7 @@ tc_candidates_kernel(const TcParams p) {
         __syncthreads();
     }
     if (warp == TC_EPI_WARPS) {
-        tmem_dealloc(tmem_base, n_acc * acc_cols);
+        tmem_dealloc(tmem_base, 2 * acc_cols);
     }
 }
 
@@ -784,46 +762,35 @@ tc_cap_max(uint32_t n_terms) {
     return cap_max;
 }
 
-// Shared-memory plan of a launch.  What bounds the kernel is the rate at which an SM takes operand tiles out of L2
-// (28 to 36 bytes a cycle measured, with and without the MMAs), so the plan asks for the fewest operand bytes per
-// 128 x 128 block of products:
-//   * the A tiles of an item stay resident when they take at most 64 KiB (128 KiB as a pair): every B tile of the item
-//     then costs only its own bytes;
-//   * pair: two row tiles of A share every B tile, half the B bytes.  It needs enough row tiles that items of 256 rows
-//     still fill the SMs (16 here: with fewer, the launch is short and its items are what is scarce), and room for
-//     three stages.  With resident A the two accumulators of a step are 2 x 128 columns and double-buffered; streamed A
-//     of one term takes both, two B tiles as well (256 x 256 in all 512 columns: 64 KiB per four blocks instead of 96);
-//   * wide: otherwise two B tiles per MMA, with one-term inputs or resident A.
-// VB200_TC_STAGES / VB200_TC_A_RESIDENT=0 / VB200_TC_WIDE=0 / VB200_TC_PAIR=0 override the choices (for experiments).
+// Shared-memory plan of a launch: whether the A tile of an item stays resident (it does when it
+// is at most 64 KiB, i.e. up to 128 dimensions of split fp32 or 256 of bf16: every B tile of the
+// item then costs only its own bytes), and as many ring stages as fit beside it and the sort
+// areas.  VB200_TC_STAGES / VB200_TC_A_RESIDENT=0 / VB200_TC_WIDE=0 override the choices (for experiments).
+// (Two A tiles that share every B tile, with accumulators of 256 x 256 in all of tensor memory or 2 x 128 x 128, halve
+// the bytes but leave nothing to overlap the epilogue with: 85 against 77 ms over 6M x 768 bf16 rows and 10000 queries,
+// 1.50 against 1.48 ms over 1M x 128 rows and 4096 centroids.)
 static void
 tc_plan(TcParams& p, size_t sort_bytes, size_t* smem_bytes) {
     const uint32_t terms = p.n_terms == 3 ? 2u : 1u;
     const size_t chunk = TC_CHUNK_BYTES;
-    const uint64_t m_tiles = (p.a.rows + TC_BM - 1) / TC_BM;
-    const size_t a_tile_bytes = static_cast<size_t>(p.a.chunks) * terms * chunk;
-    auto off = [](const char* name) {
-        const char* env = std::getenv(name);
-        return env != nullptr && env[0] == '0';
+    const size_t a_region = static_cast<size_t>(p.a.chunks) * terms * chunk;
+    const char* env_res = std::getenv("VB200_TC_A_RESIDENT");
+    const char* env_wide = std::getenv("VB200_TC_WIDE");
+    bool resident = a_region <= 65536 && !(env_res != nullptr && env_res[0] == '0');
+    auto stage_bytes = [&](bool res, bool wide) { return ((res ? 0 : terms) + terms * (wide ? 2 : 1)) * chunk; };
+    auto fits = [&](bool res, bool wide, uint32_t stages) {
+        return sort_bytes + (res ? a_region : 0) + stages * stage_bytes(res, wide) <= TC_SMEM_BUDGET;
     };
-    auto stage_bytes = [&](bool res, bool pair, bool wide) {
-        return ((res ? 0 : terms * (pair ? 2 : 1)) + terms * (wide ? 2 : 1)) * chunk;
-    };
-    auto fits = [&](bool res, bool pair, bool wide, uint32_t stages) {
-        return sort_bytes + (res ? a_tile_bytes * (pair ? 2 : 1) : 0) + stages * stage_bytes(res, pair, wide) <= TC_SMEM_BUDGET;
-    };
-    bool resident = a_tile_bytes <= 65536 && !off("VB200_TC_A_RESIDENT");
-    bool pair = m_tiles >= 16 && !off("VB200_TC_PAIR"), wide = false;
-    if (pair && resident && fits(true, true, false, 3)) {
-        wide = false;
-    } else if (pair && !resident && terms == 1 && fits(false, true, true, 3)) {
-        wide = true;
-    } else {
-        pair = false;
-        resident = resident && fits(true, false, false, TC_MIN_STAGES);
-        wide = (terms == 1 || resident) && !off("VB200_TC_WIDE") && fits(resident, false, true, TC_MIN_STAGES);
+    if (resident && !fits(true, false, TC_MIN_STAGES)) {
+        resident = false;
     }
-    const size_t fixed = sort_bytes + (resident ? a_tile_bytes * (pair ? 2 : 1) : 0);
-    uint32_t stages = static_cast<uint32_t>((TC_SMEM_BUDGET - fixed) / stage_bytes(resident, pair, wide));
+    // Two B tiles per MMA whenever a stage stays affordable: bf16 inputs, or a resident A tile.
+    bool wide = (terms == 1 || resident) && !(env_wide != nullptr && env_wide[0] == '0');
+    if (wide && !fits(resident, true, TC_MIN_STAGES)) {
+        wide = false;
+    }
+    const size_t fixed = sort_bytes + (resident ? a_region : 0);
+    uint32_t stages = static_cast<uint32_t>((TC_SMEM_BUDGET - fixed) / stage_bytes(resident, wide));
     if (stages > TC_MAX_STAGES) {
         stages = TC_MAX_STAGES;
     }
@@ -837,20 +804,7 @@ tc_plan(TcParams& p, size_t sort_bytes, size_t* smem_bytes) {
     p.stages = stages;
     p.a_resident = resident ? 1u : 0u;
     p.wide = wide ? 1u : 0u;
-    p.pair = pair ? 1u : 0u;
-    *smem_bytes = fixed + stages * stage_bytes(resident, pair, wide);
-}
-
-// Items of a launch per share of B (row tiles, or pairs of them), and the lists that every row has per share.
-static uint64_t
-tc_row_items(const TcParams& p) {
-    const uint64_t rows = p.pair ? 2 * TC_BM : TC_BM;
-    return (p.a.rows + rows - 1) / rows;
-}
-
-static uint32_t
-tc_groups(const TcParams& p) {
-    return p.pair ? TC_COL_GROUPS / 2 : TC_COL_GROUPS;
+    *smem_bytes = fixed + stages * stage_bytes(resident, wide);
 }
 
 uint32_t
@@ -878,6 +832,9 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     {
         const uint32_t cap_max = tc_cap_max(n_terms);
         uint32_t cap = next_pow2(4 * m < 64 ? 64 : 4 * m);
+        if (cap > 256) {
+            cap = next_pow2(2 * m);   // (a fourth stage of 48 KiB beside the sort areas is worth more than rarer compactions)
+        }
         if (cap > cap_max) {
             cap = cap_max;
         }
@@ -888,7 +845,7 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     const size_t sort_bytes = small_m ? 0 : TC_EPI_WARPS * static_cast<size_t>(p.cap) * sizeof(uint64_t);
     size_t smem = 0;
     tc_plan(p, sort_bytes, &smem);
-    const uint64_t m_tiles = tc_row_items(p);
+    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
     const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     uint64_t n_split = (2ull * sms + m_tiles - 1) / m_tiles;
@@ -941,17 +898,6 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
         p.diag = env != nullptr ? static_cast<uint32_t>(std::atoi(env)) : 0u;
     }
 #endif
-    p.window = 0;
-    if (interleaved) {
-        p.window = 64;
-        const char* env = std::getenv("VB200_TC_WINDOW");   // tuning aid: 0 or a power of two
-        if (env != nullptr && env[0] != 0) {
-            const uint32_t w = static_cast<uint32_t>(std::atoi(env));
-            if ((w & (w - 1u)) == 0) {
-                p.window = w;
-            }
-        }
-    }
     p.row_margin = row_margin_dev;
     p.row_bound = row_bound_dev;
     p.m = m;
@@ -960,7 +906,7 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     p.col_base = col_base;
     VB_TRY(ws.scratch.reserve(static_cast<size_t>(grid) * TC_BM * TC_COL_GROUPS * p.cap));
     VB_TRY(ws.error_flag.reserve(2));
-    VB_TRY(out.reserve(static_cast<size_t>(a.rows) * n_split * tc_groups(p) * m));
+    VB_TRY(out.reserve(static_cast<size_t>(a.rows) * n_split * TC_COL_GROUPS * m));
     VB_CUDA(cudaMemsetAsync(ws.error_flag.ptr, 0, 2 * sizeof(int), current_stream()));
     p.scratch = ws.scratch.ptr;
     p.out = out.ptr;
@@ -977,7 +923,7 @@ tc_candidates(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t 
     if ((flags[0] & 1) != 0) {
         VB_FAIL(VB200_INTERNAL_ERROR, "tensor-core kernel gave up on a bounded wait");
     }
-    *n_split_out = static_cast<uint32_t>(n_split) * tc_groups(p);
+    *n_split_out = static_cast<uint32_t>(n_split) * TC_COL_GROUPS;
     if (n_flagged_out != nullptr) {
         *n_flagged_out = static_cast<uint32_t>(flags[1]);
     }
@@ -999,7 +945,7 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
     p.n_terms = n_terms;
     size_t smem = 0;
     tc_plan(p, 0, &smem);
-    const uint64_t m_tiles = tc_row_items(p);
+    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
     const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     // More column ranges per row tile than the sorted modes take: a list costs nothing but its
@@ -1019,7 +965,7 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
     }
     const uint64_t tiles_per_split = (n_tiles + n_split - 1) / n_split;
     n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
-    const uint32_t lists = static_cast<uint32_t>(n_split) * tc_groups(p);
+    const uint32_t lists = static_cast<uint32_t>(n_split) * TC_COL_GROUPS;
     // list capacity: a list's expected share plus eight standard deviations of a Poisson count and a few more
     // (3.5 x the share at least), within the caller's limit per row.  An overflowing list costs its row a slow
     // exact answer, and with many short lists per row a multiple of the mean alone is passed every few thousand lists.
@@ -1091,7 +1037,7 @@ tc_scores(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_te
     p.n_terms = n_terms;
     size_t smem = 0;
     tc_plan(p, 0, &smem);
-    const uint64_t m_tiles = tc_row_items(p);
+    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
     const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     uint64_t n_split = (2ull * sms + m_tiles - 1) / m_tiles;

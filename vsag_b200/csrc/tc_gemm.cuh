@@ -31,7 +31,8 @@ constexpr uint32_t TC_CHUNK_BYTES = TC_CHUNK_ELEMS * 2;   // 16 KiB
 constexpr uint32_t TC_COL_GROUPS = 4;      // epilogue warps per TMEM lane quarter
 constexpr uint32_t TC_EPI_WARPS = 4 * TC_COL_GROUPS;
 constexpr uint32_t TC_EPI_THREADS = 32 * TC_EPI_WARPS;
-constexpr uint32_t TC_THREADS = TC_EPI_THREADS + 96;   // + one warp each to issue the MMAs, the A copies and the B copies
+constexpr uint32_t TC_COPY_WARPS = 2;     // warps whose elected threads issue the operand copies, an equal part of every chunk each
+constexpr uint32_t TC_THREADS = (TC_EPI_WARPS + 1 + TC_COPY_WARPS) * 32;
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 24;
 
 struct TcOperand {
@@ -54,18 +55,16 @@ struct TcParams {
     uint32_t stages;          // operand stages in shared memory (2 .. 6)
     uint32_t a_resident;      // 1: the A tile of a work item stays in shared memory for all its B tiles
     uint32_t wide;            // 1: two B tiles per MMA (128 x 256 x 16)
-    uint32_t pair;            // 1: a work item is two row tiles of A: every B tile fetched serves 256 rows
     uint32_t n_split;         // shares of B's tiles per row tile
     uint32_t tiles_per_split; // B tiles per share when the shares are contiguous
 #ifdef VB200_TC_DIAG
     uint32_t diag;            // timing experiments only: bit 0 skips the selection, bit 1 the MMAs
 #endif
-    uint32_t window;          // 0, or a power of two: tiles per window of the staggered walk over a share
     uint32_t interleaved;     // 1: share s holds tiles s, s + n_split, ...; the queue walks row tiles within a share
-    uint64_t* scratch;        // [grid][rows of an item][lists][cap] candidate buffers
-    uint64_t* out;            // [a.rows][n_split][groups][m] keys (ordered score << 32 | column), KEY_INF padded; groups = the
-                              // epilogue warps that share a row, tc_groups() (threshold mode: [...][cap], unsorted, with out_count)
-    uint32_t* out_count;      // threshold mode: [a.rows][n_split][groups] entries offered to each list
+    uint64_t* scratch;        // [grid][128][TC_COL_GROUPS][cap] candidate buffers
+    uint64_t* out;            // [a.rows][n_split][TC_COL_GROUPS][m] keys (ordered score << 32 | column), KEY_INF padded
+                              // (threshold mode: [a.rows][n_split][TC_COL_GROUPS][cap], unsorted, with out_count)
+    uint32_t* out_count;      // threshold mode: [a.rows][n_split][TC_COL_GROUPS] entries offered to each list
     uint32_t col_base;        // added to column indices in the keys
     float* store;             // score-matrix mode: [a.rows][store_ld] fp32 scores instead of candidates
     uint64_t store_ld;        // row stride of `store` in floats (multiple of 4, store 16-byte aligned)
