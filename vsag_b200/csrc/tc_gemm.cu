@@ -536,10 +536,8 @@ tc_candidates_kernel(const TcParams p) {
 #pragma unroll
                             for (int i = 0; i < 32; i += 4) {
                                 const float4 b4 = *reinterpret_cast<const float4*>(&sh.bias[warp][i]);
-                                sc[i] = fmaf(p.alpha, __uint_as_float(r[i]), b4.x);
-                                sc[i + 1] = fmaf(p.alpha, __uint_as_float(r[i + 1]), b4.y);
-                                sc[i + 2] = fmaf(p.alpha, __uint_as_float(r[i + 2]), b4.z);
-                                sc[i + 3] = fmaf(p.alpha, __uint_as_float(r[i + 3]), b4.w);
+                                fma_pair(sc[i], sc[i + 1], __uint_as_float(r[i]), __uint_as_float(r[i + 1]), p.alpha, b4.x, b4.y);
+                                fma_pair(sc[i + 2], sc[i + 3], __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]), p.alpha, b4.z, b4.w);
                             }
                         } else {
 #pragma unroll
@@ -583,17 +581,19 @@ tc_candidates_kernel(const TcParams p) {
                         }
                         continue;
                     }
-                    // minimum as a tree: a serial chain of 32 dependent fminf would stall the warp
-                    float m16[16], m4[4];
+                    // minimum as a tree of threes: 16 instructions, and a serial chain of 32 would stall the warp
+                    float m11[11], m4[4];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        m16[i] = fminf(sc[i], sc[i + 16]);
+                    for (int i = 0; i < 10; ++i) {
+                        m11[i] = min3(sc[i], sc[i + 11], sc[i + 22 < 32 ? i + 22 : i]);
                     }
+                    m11[10] = fminf(sc[10], sc[21]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        m4[i] = fminf(fminf(m16[i], m16[i + 4]), fminf(m16[i + 8], m16[i + 12]));
+                    for (int i = 0; i < 3; ++i) {
+                        m4[i] = min3(m11[i], m11[i + 4], m11[i + 8]);
                     }
-                    const float mn = fminf(fminf(m4[0], m4[1]), fminf(m4[2], m4[3]));
+                    m4[3] = fminf(m11[3], m11[7]);
+                    const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
                     if (SMALL_M) {
                         if (mn < bound) {
                             // few elements pass: found through the levels of the tree (an index that is not a constant
@@ -614,13 +614,13 @@ tc_candidates_kernel(const TcParams p) {
                             for (int g = 0; g < 4; ++g) {
                                 if (m4[g] < bound) {
 #pragma unroll
-                                    for (int i = g; i < 16; i += 4) {
-                                        if (m16[i] < bound) {
-                                            if (sc[i] < bound) {
-                                                insert(sc[i], c0 + i);
-                                            }
-                                            if (sc[i + 16] < bound) {
-                                                insert(sc[i + 16], c0 + i + 16);
+                                    for (int i = g; i < 11; i += 4) {
+                                        if (m11[i] < bound) {
+#pragma unroll
+                                            for (int e = i; e < 32; e += 11) {
+                                                if (sc[e] < bound) {
+                                                    insert(sc[e], c0 + e);
+                                                }
                                             }
                                         }
                                     }
@@ -635,30 +635,25 @@ tc_candidates_kernel(const TcParams p) {
                                && (p.diag & 4u) == 0
 #endif
                     ) {
-                        // few elements pass: test them in pairs through the first levels of the tree
+                        // few elements pass: test them through the levels of the tree
 #pragma unroll
-                        for (int g = 0; g < 16; ++g) {
-                            const int i = (g & 3) * 4 + (g >> 2);   // (the four of a second-level minimum together)
-                            if (m4[i & 3] < thr && m16[i] < thr) {
-                                if (THRESH) {
-                                    if (sc[i] < thr) {
-                                        if (cnt < p.cap) {
-                                            list[cnt] = make_key(sc[i], c0 + i + p.col_base);
+                        for (int g = 0; g < 4; ++g) {
+                            if (m4[g] < thr) {
+#pragma unroll
+                                for (int i = g; i < 11; i += 4) {
+                                    if (m11[i] < thr) {
+#pragma unroll
+                                        for (int e = i; e < 32; e += 11) {
+                                            if (sc[e] < thr) {
+                                                const uint64_t key = make_key(sc[e], c0 + e + p.col_base);
+                                                if (!THRESH) {
+                                                    buf[cnt] = key;
+                                                } else if (cnt < p.cap) {
+                                                    list[cnt] = key;
+                                                }
+                                                ++cnt;
+                                            }
                                         }
-                                        ++cnt;
-                                    }
-                                    if (sc[i + 16] < thr) {
-                                        if (cnt < p.cap) {
-                                            list[cnt] = make_key(sc[i + 16], c0 + i + 16 + p.col_base);
-                                        }
-                                        ++cnt;
-                                    }
-                                } else {
-                                    if (sc[i] < thr) {
-                                        buf[cnt++] = make_key(sc[i], c0 + i + p.col_base);
-                                    }
-                                    if (sc[i + 16] < thr) {
-                                        buf[cnt++] = make_key(sc[i + 16], c0 + i + 16 + p.col_base);
                                     }
                                 }
                             }

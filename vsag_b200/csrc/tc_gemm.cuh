@@ -190,6 +190,26 @@ umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uin
         : "memory");
 }
 
+// Two fused multiply-adds in one instruction, (a0, a1) * s + (b0, b1); each is rounded as fmaf rounds.
+__device__ __forceinline__ void
+fma_pair(float& d0, float& d1, float a0, float a1, float s, float b0, float b1) {
+    asm("{\n.reg .b64 a, s, b, d;\n"
+        "mov.b64 a, {%2, %3};\n"
+        "mov.b64 s, {%4, %4};\n"
+        "mov.b64 b, {%5, %6};\n"
+        "fma.rn.f32x2 d, a, s, b;\n"
+        "mov.b64 {%0, %1}, d;\n}"
+        : "=f"(d0), "=f"(d1)
+        : "f"(a0), "f"(a1), "f"(s), "f"(b0), "f"(b1));
+}
+
+__device__ __forceinline__ float
+min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 // One thread of a converged warp.  By elect.sync and not by a lane number: the compiler then knows that a single thread
 // is inside and feeds the MMA and bulk-copy instructions, whose operands are warp-uniform, without a loop over lanes.
 __device__ __forceinline__ bool
