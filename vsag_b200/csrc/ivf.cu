@@ -1313,8 +1313,21 @@ pair_group_kernel(const int32_t* __restrict__ probes, uint64_t total, uint32_t n
         counters[i] = 0;
     }
     grid.sync();
-    for (uint64_t e = tid; e < total; e += nthreads) {
-        pair_count_one(e, probes, nprobe, first_live, nlist, rank, world, list_off, t, phase_sel, drop);
+    // the first phase has one pair of every query: walk those alone, not all pairs
+    const bool firsts = phase_sel == 0;
+    const uint64_t walk = firsts ? total / nprobe : total;
+    auto pair_at = [&](uint64_t i) -> uint64_t {
+        if (!firsts) {
+            return i;
+        }
+        const uint32_t pr = first_live[i];
+        return pr < nprobe ? i * nprobe + pr : total;
+    };
+    for (uint64_t i = tid; i < walk; i += nthreads) {
+        const uint64_t e = pair_at(i);
+        if (e < total) {
+            pair_count_one(e, probes, nprobe, first_live, nlist, rank, world, list_off, t, phase_sel, drop);
+        }
     }
     grid.sync();
     if (gridDim.x == 1) {
@@ -1327,8 +1340,11 @@ pair_group_kernel(const int32_t* __restrict__ probes, uint64_t total, uint32_t n
     for (uint64_t i = tid; i < 2ull * nlist; i += nthreads) {
         pair_items_one(static_cast<uint32_t>(i % nlist), static_cast<uint32_t>(i / nlist), t, list_off, group_off, order, qt);
     }
-    for (uint64_t e = tid; e < total; e += nthreads) {
-        pair_scatter_one(e, probes, nprobe, first_live, nlist, rank, world, list_off, t, phase_sel, drop);
+    for (uint64_t i = tid; i < walk; i += nthreads) {
+        const uint64_t e = pair_at(i);
+        if (e < total) {
+            pair_scatter_one(e, probes, nprobe, first_live, nlist, rank, world, list_off, t, phase_sel, drop);
+        }
     }
 }
 
