@@ -60,7 +60,7 @@ struct SearchWorkspace {
     DevBuf<int32_t> probes;     // [nq x nprobe]
     DevBuf<float> probe_dists;
     // pair grouping, one set per scan phase (nearest list first, then the rest)
-    DevBuf<uint32_t> pair_ctr;     // pair counts and scatter cursors of both phases: 4 x [nlist]
+    DevBuf<uint32_t> pair_ctr;     // pair counts and scatter cursors of both phases: 4 x [nlist]; the segments' sums after them
     DevBuf<uint32_t> pair_off[2];  // [nlist + 1]
     DevBuf<uint32_t> item_off[2];  // [nlist + 1]
     DevBuf<ScanItemDesc> item_map[2];  // [pairs of the phase] at most: the work items of the phase
@@ -1296,8 +1296,105 @@ pair_scatter_kernel(const int32_t* __restrict__ probes, uint64_t total, uint32_t
     }
 }
 
+// The prefix sums and the work items of both phases by the whole grid, a segment of the list positions per CTA: sums of
+// the segments | the sums before a CTA's own, then its positions.  (One CTA per phase asks L2 for four words of every
+// list through a single SM: 35 of the 53 us that the grouping of 10000 queries over 16384 lists took.)
+__device__ __forceinline__ unsigned long long
+pair_block_sum(unsigned long long v, unsigned long long (&s_warp)[33]) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int off = 16; off > 0; off >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, off);
+    }
+    __syncthreads();
+    if (lane == 0) {
+        s_warp[warp] = v;
+    }
+    __syncthreads();
+    unsigned long long sum = 0;
+    for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
+        sum += s_warp[w];
+    }
+    return sum;
+}
+
+__device__ __forceinline__ void
+pair_scan_grid(cooperative_groups::grid_group& grid, const PairTables& tables, const uint32_t* __restrict__ list_off,
+               const uint32_t* __restrict__ group_off, const uint32_t* __restrict__ order, uint32_t* __restrict__ parts,
+               uint32_t nlist, uint32_t qt, uint32_t code_size, uint64_t* __restrict__ scalars) {
+    __shared__ unsigned long long s_warp[33];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t seg = (nlist + gridDim.x - 1) / gridDim.x;
+    const uint32_t beg = min(blockIdx.x * seg, nlist), end = min(beg + seg, nlist);
+    // pairs in the low word, items in the high word: neither reaches 2^32
+    auto count_of = [&](uint32_t ph, uint32_t pos) -> unsigned long long {
+        const uint32_t c = __ldcg((ph == 0 ? tables.cnt[0] : tables.cnt[1]) + __ldg(order + pos));
+        return c | static_cast<unsigned long long>((c + qt - 1) / qt) << 32;
+    };
+    unsigned long long bytes = 0;
+    for (uint32_t ph = 0; ph < 2; ++ph) {
+        unsigned long long mine = 0;
+        for (uint32_t pos = beg + threadIdx.x; pos < end; pos += blockDim.x) {
+            const uint32_t l = __ldg(order + pos);
+            const unsigned long long v = count_of(ph, pos);
+            mine += v;
+            bytes += (v & 0xFFFFFFFFull) * (__ldg(list_off + l + 1) - __ldg(list_off + l)) * code_size;
+        }
+        mine = pair_block_sum(mine, s_warp);
+        if (threadIdx.x == 0) {
+            parts[2 * (ph * gridDim.x + blockIdx.x)] = static_cast<uint32_t>(mine);
+            parts[2 * (ph * gridDim.x + blockIdx.x) + 1] = static_cast<uint32_t>(mine >> 32);
+        }
+    }
+    bytes = pair_block_sum(bytes, s_warp);
+    if (threadIdx.x == 0 && bytes != 0) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(scalars), bytes);   // logical scan volume, both phases
+    }
+    grid.sync();
+    for (uint32_t ph = 0; ph < 2; ++ph) {
+        unsigned long long before = 0;
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += blockDim.x) {
+            before += __ldcg(parts + 2 * (ph * gridDim.x + b)) |
+                      static_cast<unsigned long long>(__ldcg(parts + 2 * (ph * gridDim.x + b) + 1)) << 32;
+        }
+        before = pair_block_sum(before, s_warp);
+        uint32_t* pair_off = ph == 0 ? tables.off[0] : tables.off[1];
+        uint32_t* item_off = ph == 0 ? tables.item_off[0] : tables.item_off[1];
+        for (uint32_t p0 = beg; p0 < end; p0 += blockDim.x) {
+            const uint32_t pos = p0 + threadIdx.x;
+            const unsigned long long v = pos < end ? count_of(ph, pos) : 0ull;
+            unsigned long long incl = v;
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, off);
+                if (lane >= static_cast<uint32_t>(off)) {
+                    incl += up;
+                }
+            }
+            __syncthreads();   // the reads of s_warp before this are done
+            if (lane == 31) {
+                s_warp[warp] = incl;
+            }
+            __syncthreads();
+            unsigned long long at = before + incl - v;
+            for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
+                const unsigned long long sum = s_warp[w];
+                at += w < warp ? sum : 0ull;
+                before += sum;
+            }
+            if (pos < end) {
+                pair_off[__ldg(order + pos)] = static_cast<uint32_t>(at);
+                item_off[pos] = static_cast<uint32_t>(at >> 32);
+                pair_items_one(pos, ph, tables, list_off, group_off, order, qt);   // (reads what this thread has just written)
+            }
+        }
+        if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+            pair_off[nlist] = static_cast<uint32_t>(before);
+            item_off[nlist] = static_cast<uint32_t>(before >> 32);
+        }
+    }
+}
+
 // Groups the (query, probed list) pairs by list and writes the scan's work queue, in one cooperative launch:
-// clear the counters | count the pairs of every list | prefix sums (one CTA per phase) | work items and the
+// clear the counters | count the pairs of every list | prefix sums and work items (two stages) | the
 // pairs' places, with a grid-wide barrier between the stages.  As four launches the stages cost more in launch
 // and drain latency than in work.
 __global__ void __launch_bounds__(1024, 1)
@@ -1330,16 +1427,8 @@ pair_group_kernel(const int32_t* __restrict__ probes, uint64_t total, uint32_t n
         }
     }
     grid.sync();
-    if (gridDim.x == 1) {
-        pair_scan_block(0, t, list_off, order, nlist, qt, code_size, scalars);
-        pair_scan_block(1, t, list_off, order, nlist, qt, code_size, scalars);
-    } else if (blockIdx.x < 2) {
-        pair_scan_block(blockIdx.x, t, list_off, order, nlist, qt, code_size, scalars);
-    }
+    pair_scan_grid(grid, t, list_off, group_off, order, counters + 4ull * nlist, nlist, qt, code_size, scalars);
     grid.sync();
-    for (uint64_t i = tid; i < 2ull * nlist; i += nthreads) {
-        pair_items_one(static_cast<uint32_t>(i % nlist), static_cast<uint32_t>(i / nlist), t, list_off, group_off, order, qt);
-    }
     for (uint64_t i = tid; i < walk; i += nthreads) {
         const uint64_t e = pair_at(i);
         if (e < total) {
@@ -2635,7 +2724,7 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
     VB_LAUNCH(first_live_kernel, static_cast<uint32_t>((nq + 255) / 256), 256, 0, probes_dev, nq, nprobe, nlist,
               ix->shard_rank, ix->shard_world, ix->list_off.ptr,
               (ws.exchange != nullptr && ix->shard_world > 1) ? 1 : 0, ws.first_live.ptr);
-    VB_TRY(ws.pair_ctr.reserve(4 * static_cast<size_t>(nlist)));
+    VB_TRY(ws.pair_ctr.reserve(4 * static_cast<size_t>(nlist) + 4 * static_cast<size_t>(sm_count())));
     PairTables tables{};
     for (uint32_t ph = 0; ph < 2; ++ph) {
         tables.cnt[ph] = ws.pair_ctr.ptr + static_cast<size_t>(ph) * nlist;
