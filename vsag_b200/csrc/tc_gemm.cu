@@ -565,7 +565,16 @@ tc_candidates_kernel(const TcParams p) {
                         // 32 consecutive floats of this thread's row: eight 16-byte stores
                         if (valid_row && tile_present) {
                             float* dst = p.store + grow * p.store_ld + c0;
-                            if (whole_tile) {
+                            if (whole_tile && p.store_wide) {
+                                // whole 32-byte sectors: a lane's rows are a stride apart, so nothing joins two halves
+#pragma unroll
+                                for (int i = 0; i < 32; i += 8) {
+                                    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + i), "f"(sc[i]),
+                                                 "f"(sc[i + 1]), "f"(sc[i + 2]), "f"(sc[i + 3]), "f"(sc[i + 4]), "f"(sc[i + 5]),
+                                                 "f"(sc[i + 6]), "f"(sc[i + 7])
+                                                 : "memory");
+                                }
+                            } else if (whole_tile) {
 #pragma unroll
                                 for (int i = 0; i < 32; i += 4) {
                                     *reinterpret_cast<float4*>(dst + i) = make_float4(sc[i], sc[i + 1], sc[i + 2], sc[i + 3]);
@@ -1054,6 +1063,7 @@ tc_scores(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint32_t n_te
     p.tiles_per_split = static_cast<uint32_t>(tiles_per_split);
     p.store = scores_dev;
     p.store_ld = ld;
+    p.store_wide = (ld % 8 == 0 && (reinterpret_cast<uintptr_t>(scores_dev) & 31) == 0) ? 1u : 0u;
     if (deferred_flag_dev == nullptr) {
         VB_TRY(ws.error_flag.reserve(2));
         VB_CUDA(cudaMemsetAsync(ws.error_flag.ptr, 0, 2 * sizeof(int), current_stream()));

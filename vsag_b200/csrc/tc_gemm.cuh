@@ -68,6 +68,7 @@ struct TcParams {
     uint32_t col_base;        // added to column indices in the keys
     float* store;             // score-matrix mode: [a.rows][store_ld] fp32 scores instead of candidates
     uint64_t store_ld;        // row stride of `store` in floats (multiple of 4, store 16-byte aligned)
+    uint32_t store_wide;      // 1: rows of `store` start on 32-byte boundaries
     int* error_flag;          // [0] set non-zero if a bounded wait gave up; [1] counts the rows flagged below
     uint32_t spin_limit;      // polls a wait may take before it gives up
     uint32_t* row_flags;      // m <= 4 mode with a margin, optional: [a.rows], set to 1 for a row one of whose
