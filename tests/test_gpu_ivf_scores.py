@@ -80,3 +80,20 @@ def test_exact_search_of_few_queries(engine, oracle, n, nq, k, quant, dim):
             want = oracle.bf_search_bf16(oracle.float_to_bf16(base), q, k, metric=metric)
         assert np.array_equal(got[1], want[1])
         assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 20_004])
+def test_selection_reads_the_passing_groups(engine, oracle, n):
+    """Rows of scores around sixteen values per group, the best ones in one group of a thread and tied across many."""
+    dim, nq, k = 24, 17, 20
+    rng = np.random.default_rng(n)
+    base = rng.integers(-3, 4, (n, dim)).astype(np.float32)
+    q = rng.integers(-3, 4, (nq, dim)).astype(np.float32)
+    base[5::2048] = q[0]            # many of query 0's best belong to one thread
+    base[n // 2:n // 2 + 40] = q[1]  # more exact ties than results
+    ix = engine.BfHandle(dim, 0, engine.QUANT_FP32)
+    ix.add(base, np.arange(n, dtype=np.int64))
+    got = ix.search(q, k)
+    want = oracle.bf_search_fp32(base, q, k, 0)
+    assert np.array_equal(got[1], want[1])
+    assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)

@@ -16,7 +16,7 @@
 // Operands are pre-tiled in global memory so that a [128 rows x 64 k] chunk is one contiguous
 // 16 KiB block already in the shared-memory layout the MMA descriptors describe (K-major, no
 // swizzle: 8x8 core matrices of 128 B, cores adjacent along K 128 B apart, 8-row groups 1 KiB
-// apart).  A chunk therefore moves with a single bulk copy that completes on an mbarrier.
+// apart).  A chunk, or half of one, therefore moves with a single bulk copy that completes on an mbarrier.
 #pragma once
 
 #include "common.cuh"
@@ -30,7 +30,6 @@ constexpr uint32_t TC_CHUNK_ELEMS = 128 * TC_KC;
 constexpr uint32_t TC_CHUNK_BYTES = TC_CHUNK_ELEMS * 2;   // 16 KiB
 constexpr uint32_t TC_COL_GROUPS = 4;      // epilogue warps per TMEM lane quarter
 constexpr uint32_t TC_EPI_WARPS = 4 * TC_COL_GROUPS;
-constexpr uint32_t TC_EPI_THREADS = 32 * TC_EPI_WARPS;
 constexpr uint32_t TC_COPY_WARPS = 2;     // warps whose elected threads issue the operand copies, an equal part of every chunk each
 constexpr uint32_t TC_THREADS = (TC_EPI_WARPS + 1 + TC_COPY_WARPS) * 32;
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 24;
