@@ -1,0 +1,63 @@
+"""Searches that nominate rows by approximate scores must return the exact answer whatever the data: where the scores
+cannot tell the nearest rows apart, or overflow, the exact distances decide."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import assert_topk_equal, mixture
+
+pytestmark = pytest.mark.gpu
+
+
+def exactly(got, want):
+    assert np.array_equal(got[1], want[1])
+    assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)
+
+
+@pytest.mark.parametrize("quant", ["fp32", "bf16"])
+@pytest.mark.parametrize("metric", [0, 1])
+@pytest.mark.parametrize("offset,n,dim,nq,k", [
+    (50.0, 20_000, 128, 17, 10),     # scores of 3e5 with differences of 1
+    (100.0, 30_011, 33, 9, 1),       # rows of 4 (fp32) and 2 (bf16) bytes alignment
+    (30.0, 4_000, 24, 300, 40),      # many queries, nearly all of them undecided
+    (0.0, 4_000, 24, 300, 40),       # nearly none
+])
+def test_exact_batches_far_from_the_origin(engine, oracle, quant, metric, offset, n, dim, nq, k):
+    """The matrix of split-bf16 scores keeps k + 16 rows per query; far from the origin the true neighbours are not
+    among them, and the batch has to notice."""
+    base = (offset + 0.1 * mixture(3, n, dim, 30, 1.0)).astype(np.float32)
+    q = (offset + 0.1 * mixture(4, nq, dim, 30, 1.0)).astype(np.float32)
+    ix = engine.BfHandle(dim, metric, engine.QUANT_FP32 if quant == "fp32" else engine.QUANT_BF16)
+    ix.add(base[: n // 3], np.arange(n // 3, dtype=np.int64))
+    ix.add(base[n // 3:], np.arange(n // 3, n, dtype=np.int64))
+    got = ix.search(q, k)
+    if quant == "fp32":
+        want = oracle.bf_search_fp32(base, q, k, metric)
+    else:
+        want = oracle.bf_search_bf16(oracle.float_to_bf16(base), q, k, metric=metric)
+    exactly(got, want)
+    # the same with half of the rows filtered out, and a batch whose queries come one at a time
+    gone = np.zeros((n + 31) // 32, np.uint32)
+    gone[:] = 0x55555555
+    left = np.flatnonzero(np.arange(n) % 2 == 1)
+    got = ix.search_filtered(q, k, deny_inner_bits=gone)
+    if quant == "fp32":
+        want = oracle.bf_search_fp32(base[left], q, k, metric)
+    else:
+        want = oracle.bf_search_bf16(oracle.float_to_bf16(base[left]), q, k, metric=metric)
+    exactly(got, (np.where(want[0] >= 0, left[want[0]], -1), want[1]))
+    one = ix.search(q[5:6].copy(), k)
+    assert np.array_equal(one[1][0], ix.search(q, k)[1][5])
+
+
+def test_exact_batches_with_overflowing_norms(engine, oracle):
+    """Rows whose squared norm is infinite have finite distances to queries beside them."""
+    n, dim, k = 1500, 16, 5
+    base = mixture(5, n, dim, 10, 0.3)
+    base[::7] += np.float32(3e19)
+    q = np.ascontiguousarray(base[:40])
+    ix = engine.BfHandle(dim, 0, engine.QUANT_FP32)
+    ix.add(base, np.arange(n, dtype=np.int64))
+    got = ix.search(q, k)
+    exactly(got, oracle.bf_search_fp32(base, q, k, 0))

@@ -14,7 +14,8 @@ namespace vb200 {
 constexpr int BF_STREAM_QUERIES = 8;
 
 struct BfStream {
-    const void* queries;        // [nq x dim] fp32, or bf16 bit patterns
+    const void* queries;        // [.. x dim] fp32, or bf16 bit patterns
+    const uint32_t* pick;       // [nq] the queries' rows in `queries`, or null: 0 .. nq - 1
     uint32_t nq, dim;
     const unsigned char* base;  // [n x dim] rows in the index's type
     uint64_t n;
@@ -42,7 +43,7 @@ bf_stream_kernel(const BfStream p) {
         const uint32_t qi = i / qpad, d = i - qi * qpad;
         float v = 0.f;
         if (static_cast<int>(qi) < here && d < p.dim) {
-            const uint64_t at = static_cast<uint64_t>(q0 + qi) * p.dim + d;
+            const uint64_t at = static_cast<uint64_t>(p.pick != nullptr ? __ldg(p.pick + q0 + qi) : q0 + qi) * p.dim + d;
             v = FMT == ROW_F32 ? static_cast<const float*>(p.queries)[at]
                                : half_decode<SCAN_FMT_BF16>(static_cast<const uint16_t*>(p.queries)[at]);
         }
@@ -93,11 +94,12 @@ bf_stream_kernel(const BfStream p) {
     ts.finish(here, p.part, p.bound);
 }
 
-// One CTA per query: the k best of its `n` partial keys (payload = row), as results.
+// One CTA per query: the k best of its `n` partial keys (payload = row), as results of query pick[blockIdx.x] (null: its own
+// number).
 template <int T>
 __global__ void __launch_bounds__(T)
-bf_pick_kernel(const uint64_t* __restrict__ part, uint32_t n, uint32_t k, const int64_t* __restrict__ labels,
-               int64_t* __restrict__ ids, float* __restrict__ dists) {
+bf_pick_kernel(const uint64_t* __restrict__ part, uint32_t n, uint32_t k, const uint32_t* __restrict__ pick,
+               const int64_t* __restrict__ labels, int64_t* __restrict__ ids, float* __restrict__ dists) {
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
@@ -105,36 +107,92 @@ bf_pick_kernel(const uint64_t* __restrict__ part, uint32_t n, uint32_t k, const 
     const uint32_t found = block_select<T>(load_source([&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i) >> 32); }),
                                            [&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i)); }, n, k, keys, sel);
     block_sort_to<T>(keys, found, k, best);
+    const uint64_t q = pick != nullptr ? __ldg(pick + blockIdx.x) : blockIdx.x;
     for (uint32_t i = threadIdx.x; i < k; i += T) {
         const bool there = i < found;
-        ids[static_cast<uint64_t>(blockIdx.x) * k + i] = there ? __ldg(labels + static_cast<uint32_t>(best[i])) : -1;
-        dists[static_cast<uint64_t>(blockIdx.x) * k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
+        ids[q * k + i] = there ? __ldg(labels + static_cast<uint32_t>(best[i])) : -1;
+        dists[q * k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
     }
+}
+
+// *top = the largest norm of the rows whose squared norms are given, rounded up (one launch per add; never lowered).
+__global__ void __launch_bounds__(256)
+bf_row_max_kernel(const float* __restrict__ sq, uint64_t n, float* __restrict__ top) {
+    float most = 0.f;
+    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x; i < n; i += static_cast<uint64_t>(gridDim.x) * 256) {
+        most = fmaxf(most, __ldg(sq + i));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+    }
+    if ((threadIdx.x & 31) == 0) {   // non-negative floats order like their bit patterns
+        atomicMax(reinterpret_cast<int*>(top), __float_as_int(sqrtf(most) * 1.001f));
+    }
+}
+
+// How far a nominating score may be from the distance it stands for, so that a query knows whether a row that was not
+// nominated can belong to its results.  With X = the largest |x| and Q = |q|:
+//   IP  the score -<x, q> and the exact 1 - <x, q> differ by (chain + matrix) X Q and the rounding of the subtraction
+//   L2  |x|^2 - 2 <x, q> + |q|^2 and the exact chain differ by chain (X^2 + Q^2 + d) + 2 matrix X Q, d the distance
+// chain = the rounding of a sum of dim products in fp32, (dim + 16) 2^-24; matrix = that of the tensor cores' sums.  Those
+// take 16 products and the running sum per step, each cut to 24 bits or more: below (17/16) dim 2^-24 per term pair; with
+// split terms three pairs and the dropped products, 3 * 2^-18.
+struct BfMargin {
+    const float* row_max;   // X
+    float chain, matrix;
+    uint32_t* unsure;       // [0] = number of queries whose nominations may not be enough, then their numbers
+    uint32_t q_base;        // number of the launch's first query
+};
+
+template <int T>
+__device__ __forceinline__ float
+bf_block_sum(float v, float* part) {
+    for (int o = 16; o > 0; o >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    v = 0.f;
+    for (int w = 0; w < T / 32; ++w) {
+        v += part[w];
+    }
+    return v;
 }
 
 // One CTA per query: the kcand best of its row of `n` nominating scores, re-scored in the reference's operation
 // order (an FMA chain over the dimensions, one thread per candidate: FP32Quantizer::ComputeDistImpl,
 // src/quantization/fp32_quantizer.cpp:163-190; HalfPrecisionQuantizer,
 // src/quantization/scalar_quantization/half_precision_quantizer.cpp:54-123), the k best of those as results.
-// Infinite scores belong to rows that are filtered out.
+// Infinite scores belong to rows that are filtered out.  A query is sure of its results when the k-th of them is nearer
+// than the last nominated score allows any other row to be; the others are listed for an exact pass (bf_stream_kernel).
+// Without the test a data offset of 50 (128 dimensions, spread 0.1) left a fifth of the true neighbours among the nominated.
 template <typename E, int T>
 __global__ void __launch_bounds__(T)
 bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const E* __restrict__ queries, uint32_t dim,
                const E* __restrict__ base, uint32_t kcand, uint32_t k, int metric, const int64_t* __restrict__ labels,
-               int64_t* __restrict__ ids, float* __restrict__ dists) {
+               int64_t* __restrict__ ids, float* __restrict__ dists, const BfMargin m) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
+    __shared__ float part[T / 32];
     float* qf = reinterpret_cast<float*>(smem);
     const uint64_t q = blockIdx.x;
+    float qq = 0.f;
     for (uint32_t d = threadIdx.x; d < dim; d += T) {
-        qf[d] = widen(queries[q * dim + d]);
+        const float v = widen(queries[q * dim + d]);
+        qf[d] = v;
+        qq = fmaf(v, v, qq);
     }
+    qq = bf_block_sum<T>(qq, part);
     const ScoreSource<true> src{reinterpret_cast<const uint32_t*>(scores + q * ld)};
     const uint32_t found = block_select<T>(src, [](uint32_t i) { return i; }, n, kcand, keys, sel);
     block_sort_to<T>(keys, found, kcand, best);
     const uint32_t have = min(found, kcand);
+    const float last = have > 0 ? ordered_to_float(static_cast<uint32_t>(best[have - 1] >> 32)) : 0.f;
     for (uint32_t i = threadIdx.x; i < have; i += T) {
         const uint32_t row = static_cast<uint32_t>(best[i]);
         keys[i] = make_key(row_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, metric == VB200_METRIC_L2), row);
@@ -144,6 +202,18 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
         const bool there = i < have;
         ids[q * k + i] = there ? __ldg(labels + static_cast<uint32_t>(best[i])) : -1;
         dists[q * k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
+    }
+    if (threadIdx.x == 0) {
+        const bool l2 = metric == VB200_METRIC_L2;
+        const bool dropped = n > kcand && found >= kcand;   // (then kcand > k)
+        const float kth = dropped ? ordered_to_float(static_cast<uint32_t>(best[k - 1] >> 32)) : 0.f;
+        const float top = __ldg(m.row_max), size = top * sqrtf(qq);
+        float margin = l2 ? fmaf(m.chain, top * top + qq + kth, 2.0f * m.matrix * size) : fmaf(m.chain + m.matrix, size, 3e-7f);
+        margin += 1e-30f;   // (products below the smallest normal number round absolutely)
+        // not finite: scores may have overflowed, and rows with them are not even among the counted
+        if (!(margin < INFINITY) || (dropped && !(kth < last + (l2 ? qq : 1.0f) - margin))) {
+            m.unsure[1 + atomicAdd(m.unsure, 1u)] = m.q_base + static_cast<uint32_t>(q);
+        }
     }
 }
 

@@ -262,6 +262,8 @@ struct vb200_bf {
     DevBuf<int64_t> out_ids;
     DevBuf<float> out_dists;
     DevBuf<uint32_t> stream_bound;   // per query: a bound of its k-th best distance while rows stream by
+    DevBuf<float> row_max;           // the largest norm of a row
+    DevBuf<uint32_t> unsure;         // queries whose nominations may not have been enough: their number, then which
     PinnedBuf pinned;                // small host inputs and results
     std::mutex mu;
 };
@@ -326,6 +328,12 @@ bf_append_labels_and_norms(vb200_bf* ix, const int64_t* ids, uint64_t count) {
     } else {
         VB_TRY(row_sqnorm_bf16(ix->base_bf16.ptr + ix->n * ix->dim, count, ix->dim, ix->norms.ptr + ix->n));
     }
+    if (ix->row_max.ptr == nullptr) {
+        VB_TRY(ix->row_max.reserve(1));
+        VB_CUDA(cudaMemsetAsync(ix->row_max.ptr, 0, sizeof(float), current_stream()));
+    }
+    VB_LAUNCH(bf_row_max_kernel, static_cast<uint32_t>(std::min<uint64_t>((count + 1023) / 1024, 4ull * sm_count())), 256, 0,
+              ix->norms.ptr + ix->n, count, ix->row_max.ptr);
     {
         // tombstone words for the new rows
         const uint64_t words = (ix->n + count + 31) / 32;
@@ -686,35 +694,42 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
     return 0;
 }
 
-// A few queries: one pass over the rows (bf_stream.cuh) straight to results in device or pinned memory.
+// The queries on the device and the rows' masks, as bf_stage leaves them.
+struct BfStaged {
+    const float *queries = nullptr, *bias = nullptr;
+    bool masked = false;
+};
+
+static size_t
+bf_stream_smem(uint32_t dim, uint32_t cap, uint32_t qn) {
+    return RS_STAGES * RS_STAGE + static_cast<size_t>(qn) * ((dim + 7) / 8 * 8) * sizeof(float) +
+           static_cast<size_t>(qn) * (cap * sizeof(uint64_t) + 6 * sizeof(uint32_t));
+}
+
+// Exact distances of a few queries: one pass over the rows (bf_stream.cuh) straight to results in device or pinned memory.
+// pick (optional, device): the queries' numbers among the staged ones, whose results go to the same numbers.
 static int
-bf_search_stream(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k, int64_t* ids_dev, float* dists_dev) {
+bf_stream_queries(vb200_bf* ix, const BfStaged& staged, uint64_t nq, const uint32_t* pick, uint32_t k, int64_t* ids_dev, float* dists_dev) {
     const uint32_t dim = ix->dim;
     const bool l2 = ix->metric == VB200_METRIC_L2, bf16 = ix->quant == VB200_QUANT_BF16;
-    const float *q_dev = nullptr, *bias = nullptr;
-    bool masked = false;
-    VB_TRY(bf_stage(ix, queries, nq, &q_dev, &bias, &masked));
     BfStream p{};
-    p.queries = bf16 ? static_cast<const void*>(ix->q_bf16.ptr) : q_dev;
+    p.queries = bf16 ? static_cast<const void*>(ix->q_bf16.ptr) : staged.queries;
+    p.pick = pick;
     p.nq = static_cast<uint32_t>(nq);
     p.dim = dim;
     p.base = bf16 ? reinterpret_cast<const unsigned char*>(ix->base_bf16.ptr) : reinterpret_cast<const unsigned char*>(ix->base_f32.ptr);
     p.n = ix->n;
     p.k = k;
     p.cap = next_pow2(k + RS_ROWS);
-    p.masked = masked ? bias : nullptr;
+    p.masked = staged.masked ? staged.bias : nullptr;
     uint32_t qn = 1;
     while (qn < nq && qn < BF_STREAM_QUERIES) {
         qn *= 2;
     }
-    auto smem_of = [&](uint32_t q) {
-        return RS_STAGES * RS_STAGE + static_cast<size_t>(q) * ((dim + 7) / 8 * 8) * sizeof(float) +
-               static_cast<size_t>(q) * (p.cap * sizeof(uint64_t) + 6 * sizeof(uint32_t));
-    };
-    while (qn > 1 && smem_of(qn) > 110 * 1024) {
+    while (qn > 1 && bf_stream_smem(dim, p.cap, qn) > 110 * 1024) {
         qn /= 2;
     }
-    const size_t smem = smem_of(qn);
+    const size_t smem = bf_stream_smem(dim, p.cap, qn);
     VB_CHECK_ARG(smem <= 220 * 1024, "dim = %u is too large for the row scan", dim);
     const size_t row_bytes = static_cast<size_t>(dim) * (bf16 ? 2 : 4);
     const int unit = row_bytes % 16 == 0 ? 16 : (row_bytes % 4 == 0 ? 4 : 2);
@@ -748,31 +763,33 @@ bf_search_stream(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k, in
     VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, RS_ROWS, smem));
     const uint64_t chunks = (ix->n + RS_ROWS - 1) / RS_ROWS;
     const uint32_t tiles = static_cast<uint32_t>((nq + qn - 1) / qn);
-    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(chunks, static_cast<uint64_t>(sm_count()) * std::max(per_sm, 1)));
-    VB_CHECK_ARG(nq * grid * k < 0xFFFFFFFFull, "query batch too large");
+    // one wave of CTAs: with several tiles of queries each takes a larger share of the rows
+    const uint64_t slots = static_cast<uint64_t>(sm_count()) * std::max(per_sm, 1);
+    const uint32_t grid = static_cast<uint32_t>(std::min(chunks, std::max<uint64_t>(slots / tiles, 1)));
+    VB_CHECK_ARG(nq * grid * k < 0xFFFFFFFFull && tiles <= 65535, "query batch too large");
     VB_TRY(ix->part.reserve(nq * grid * k));
     VB_TRY(ix->stream_bound.reserve(nq));
     VB_CUDA(cudaMemsetAsync(ix->stream_bound.ptr, 0xFF, nq * sizeof(uint32_t), current_stream()));
     p.part = ix->part.ptr;
     p.bound = ix->stream_bound.ptr;
     VB_LAUNCH(kernel, dim3(grid, tiles), RS_ROWS, smem, p);
-    VB_LAUNCH(bf_pick_kernel<1024>, static_cast<uint32_t>(nq), 1024, 0, ix->part.ptr, grid * k, k, ix->labels.ptr, ids_dev, dists_dev);
+    VB_LAUNCH(bf_pick_kernel<1024>, static_cast<uint32_t>(nq), 1024, 0, ix->part.ptr, grid * k, k, pick, ix->labels.ptr, ids_dev, dists_dev);
     return 0;
 }
 
 // Batches whose score matrix is worth writing: tensor-core scores in slices of queries,
-// then a CTA per query that selects, re-scores and writes its results.
+// then a CTA per query that selects, re-scores and writes its results.  Leaves in ix->unsure the queries for which that
+// may not have been enough.
 // Slices of 512 MiB: with slices that stay in L2 (96 MiB) the launches are too short to fill the SMs, and the scores they
 // save from a trip to HBM cost less than that (1000 queries over 100k x 128 rows: 8 slices 632 us, 4 517, 2 481, 1 431).
 constexpr uint64_t BF_SLICE_SCORES = uint64_t{128} << 20;
+constexpr uint64_t BF_UNSURE_SLICE = 4096;   // of those queries that are streamed at once (their partial results: k keys each per CTA)
 
 static int
-bf_search_scores(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k, int64_t* ids_dev, float* dists_dev) {
+bf_search_scores(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k, int64_t* ids_dev, float* dists_dev) {
     const uint32_t dim = ix->dim;
     const bool l2 = ix->metric == VB200_METRIC_L2, bf16 = ix->quant == VB200_QUANT_BF16;
-    const float *q_dev = nullptr, *bias = nullptr;
-    bool masked = false;
-    VB_TRY(bf_stage(ix, queries, nq, &q_dev, &bias, &masked));
+    const float* q_dev = staged.queries;
     VB_TRY(bf_tile_base(ix));
     VB_TRY(bf_tile_queries(ix, q_dev, nq));
     const uint32_t chunks = (dim + TC_KC - 1) / TC_KC;
@@ -780,28 +797,36 @@ bf_search_scores(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k, in
     uint64_t slice = BF_SLICE_SCORES / ld / TC_BM * TC_BM;   // whole row tiles
     slice = slice < TC_BM ? TC_BM : slice;
     VB_TRY(ix->scores.reserve(std::min(slice, nq) * ld));
+    VB_TRY(ix->unsure.reserve(nq + 1));
+    VB_CUDA(cudaMemsetAsync(ix->unsure.ptr, 0, sizeof(uint32_t), current_stream()));
     VB_TRY(ix->tc.error_flag.reserve(2));
     VB_CUDA(cudaMemsetAsync(ix->tc.error_flag.ptr, 0, 2 * sizeof(int), current_stream()));
     const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks};
     const uint32_t kcand = static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n));
     const size_t smem = dim * sizeof(float);
     VB_CHECK_ARG(smem <= 180 * 1024, "dim = %u is too large for the exact re-scoring step", dim);
+    BfMargin margin{};
+    margin.row_max = ix->row_max.ptr;
+    margin.chain = static_cast<float>(dim + 16) * 6.0e-8f;
+    margin.matrix = bf16 ? 2.0f * margin.chain : 4.0f * margin.chain + 3.0f / 262144.0f;
+    margin.unsure = ix->unsure.ptr;
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
         const uint64_t m = std::min(slice, nq - q0);
         const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
         const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks};
-        VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, bias, ix->scores.ptr, ld, ix->tc.error_flag.ptr));
+        margin.q_base = static_cast<uint32_t>(q0);
+        VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, staged.bias, ix->scores.ptr, ld, ix->tc.error_flag.ptr));
         if (bf16) {
             auto kernel = bf_rows_kernel<uint16_t, 512>;
             VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 8192 ? 40 * 1024 : 0)));
             VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, ix->scores.ptr, ld, static_cast<uint32_t>(ix->n),
                       ix->q_bf16.ptr + q0 * dim, dim, ix->base_bf16.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k,
-                      dists_dev + q0 * k);
+                      dists_dev + q0 * k, margin);
         } else {
             auto kernel = bf_rows_kernel<float, 512>;
             VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 8192 ? 40 * 1024 : 0)));
             VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, ix->scores.ptr, ld, static_cast<uint32_t>(ix->n), q_dev + q0 * dim, dim,
-                      ix->base_f32.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k, dists_dev + q0 * k);
+                      ix->base_f32.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k, dists_dev + q0 * k, margin);
         }
     }
     return 0;
@@ -856,41 +881,64 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
     int64_t* ids_dev = !host_ids ? ids : (pin_out ? pin_ids : ix->out_ids.ptr);
     float* dists_dev = !host_d ? dists : (pin_out ? pin_dists : ix->out_dists.ptr);
     const bool k_fits = std::min<uint64_t>(k + BF_SLACK, ix->n) <= 1024;
-    bool flagged = false;
+    const bool streams = k_fits && bf_stream_smem(ix->dim, next_pow2(k + RS_ROWS), 1) <= 220 * 1024;
+    const bool scores = tensor_cores_enabled() && streams && nq > BF_STREAM_QUERIES && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES;
+    BfStaged staged;
+    bool keyed = false;
     int rc = 0;
     ix->filter = filter;
     // Up to eight queries share one pass over the rows; more go to the tensor cores -- through a score matrix
     // while that is cheaper than selecting as the scores appear (measured: up to about 4e8 scores), see
     // bf_search_keys for the rest.
     if (nq <= BF_STREAM_QUERIES && k_fits) {
-        rc = bf_search_stream(ix, queries, nq, k, ids_dev, dists_dev);
-    } else if (tensor_cores_enabled() && k_fits && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES) {
-        rc = bf_search_scores(ix, queries, nq, k, ids_dev, dists_dev);
-        flagged = true;
+        rc = bf_stage(ix, queries, nq, &staged.queries, &staged.bias, &staged.masked);
+        if (rc == 0) {
+            rc = bf_stream_queries(ix, staged, nq, nullptr, k, ids_dev, dists_dev);
+        }
+    } else if (scores) {
+        rc = bf_stage(ix, queries, nq, &staged.queries, &staged.bias, &staged.masked);
+        if (rc == 0) {
+            rc = bf_search_scores(ix, staged, nq, k, ids_dev, dists_dev);
+        }
     } else {
         rc = bf_search_keys(ix, queries, nq, k);
-        if (rc == 0) {
-            VB_LAUNCH(bf_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ix->keys.ptr, total,
-                      ix->labels.ptr, ids_dev, dists_dev, nullptr);
-        }
+        keyed = true;
     }
     ix->filter = nullptr;
     VB_TRY(rc);
-    if (!pin_out) {
-        if (host_ids) {
-            VB_CUDA(cudaMemcpyAsync(ids, ids_dev, total * sizeof(int64_t), cudaMemcpyDeviceToHost, current_stream()));
-        }
-        if (host_d) {
-            VB_CUDA(cudaMemcpyAsync(dists, dists_dev, total * sizeof(float), cudaMemcpyDeviceToHost, current_stream()));
-        }
+    if (keyed) {
+        VB_LAUNCH(bf_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ix->keys.ptr, total, ix->labels.ptr, ids_dev,
+                  dists_dev, nullptr);
     }
+    auto results_to_host = [&]() -> int {
+        if (!pin_out) {
+            if (host_ids) {
+                VB_CUDA(cudaMemcpyAsync(ids, ids_dev, total * sizeof(int64_t), cudaMemcpyDeviceToHost, current_stream()));
+            }
+            if (host_d) {
+                VB_CUDA(cudaMemcpyAsync(dists, dists_dev, total * sizeof(float), cudaMemcpyDeviceToHost, current_stream()));
+            }
+        }
+        return 0;
+    };
+    VB_TRY(results_to_host());
     int flag = 0;
-    if (flagged) {
+    uint32_t unsure = 0;
+    if (scores) {
         VB_CUDA(cudaMemcpyAsync(&flag, ix->tc.error_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, current_stream()));
+        VB_CUDA(cudaMemcpyAsync(&unsure, ix->unsure.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, current_stream()));
     }
     VB_TRY(sync_stream());
     if ((flag & 1) != 0) {
         VB_FAIL(VB200_INTERNAL_ERROR, "tensor-core kernel gave up on a bounded wait");
+    }
+    if (unsure > 0) {
+        for (uint64_t u0 = 0; u0 < unsure; u0 += BF_UNSURE_SLICE) {
+            VB_TRY(bf_stream_queries(ix, staged, std::min<uint64_t>(BF_UNSURE_SLICE, unsure - u0), ix->unsure.ptr + 1 + u0, k, ids_dev,
+                                     dists_dev));
+        }
+        VB_TRY(results_to_host());
+        VB_TRY(sync_stream());
     }
     if (pin_out) {
         if (host_ids) {
