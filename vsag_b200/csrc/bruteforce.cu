@@ -818,13 +818,13 @@ bf_search_scores(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k, 
         VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, staged.bias, ix->scores.ptr, ld, ix->tc.error_flag.ptr));
         if (bf16) {
             auto kernel = bf_rows_kernel<uint16_t, 512>;
-            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 8192 ? 40 * 1024 : 0)));
+            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
             VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, ix->scores.ptr, ld, static_cast<uint32_t>(ix->n),
                       ix->q_bf16.ptr + q0 * dim, dim, ix->base_bf16.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k,
                       dists_dev + q0 * k, margin);
         } else {
             auto kernel = bf_rows_kernel<float, 512>;
-            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 8192 ? 40 * 1024 : 0)));
+            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
             VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, ix->scores.ptr, ld, static_cast<uint32_t>(ix->n), q_dev + q0 * dim, dim,
                       ix->base_f32.ptr, kcand, k, ix->metric, ix->labels.ptr, ids_dev + q0 * k, dists_dev + q0 * k, margin);
         }

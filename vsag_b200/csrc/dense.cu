@@ -59,15 +59,18 @@ sm_count() {
 
 int
 allow_dynamic_smem(const void* kernel, size_t bytes) {
-    if (bytes <= 40 * 1024) {   // static shared memory counts against the 48 KiB default too
-        return 0;
-    }
     static std::mutex mu;
     static std::map<std::pair<const void*, int>, size_t> allowed;
     int dev = 0;
     VB_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
     size_t& have = allowed[{kernel, dev}];
+    if (have == 0) {
+        // what the kernel may take unasked: 48 KiB less its static shared memory
+        cudaFuncAttributes attr{};
+        VB_CUDA(cudaFuncGetAttributes(&attr, kernel));
+        have = static_cast<size_t>(attr.maxDynamicSharedSizeBytes);
+    }
     if (bytes > have) {
         VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         have = bytes;

@@ -2415,7 +2415,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
     pp.probe_dists = dists_dev;
     const size_t route_smem = ix->dim * sizeof(float);
     VB_CHECK_ARG(route_smem <= 180 * 1024, "dim = %u is too large for the routing kernel", ix->dim);
-    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_kernel), route_smem + (route_smem > 8192 ? 40 * 1024 : 0)));
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_kernel), route_smem));
     if (routes_on_tensor_cores(ix, nq)) {
         const uint32_t chunks = (ix->dim + TC_KC - 1) / TC_KC;
         if (!ix->c_tiled) {
@@ -3530,8 +3530,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     if (plan == nullptr) {
         VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(scan_kernel), scan_smem));
     }
-    // (beside about 34 KiB of static shared memory)
-    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(final_kernel), final_smem + (final_smem > 12 * 1024 ? 40 * 1024 : 0)));
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(final_kernel), final_smem));
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
         const uint64_t n = std::min(slice, nq - q0);
         ScanFinalize g = f;
@@ -3580,7 +3579,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         r.out_dists = dists_dev;
         auto kernel = l2 ? rerank_rows_kernel<true> : rerank_rows_kernel<false>;
         const size_t smem = dim * sizeof(float);
-        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem + (smem > 24 * 1024 ? 20 * 1024 : 0)));
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
         VB_CHECK_ARG(nq * RERANK_PARTS <= 0x7fffffffull, "query batch too large");
         VB_LAUNCH(kernel, static_cast<uint32_t>(nq * RERANK_PARTS), PAIR_THREADS, smem, r);
     }
