@@ -144,24 +144,6 @@ struct BfMargin {
     uint32_t q_base;        // number of the launch's first query
 };
 
-template <int T>
-__device__ __forceinline__ float
-bf_block_sum(float v, float* part) {
-    for (int o = 16; o > 0; o >>= 1) {
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
-        part[threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    v = 0.f;
-    for (int w = 0; w < T / 32; ++w) {
-        v += part[w];
-    }
-    return v;
-}
-
 // One CTA per query: the kcand best of its row of `n` nominating scores, re-scored in the reference's operation
 // order (an FMA chain over the dimensions, one thread per candidate: FP32Quantizer::ComputeDistImpl,
 // src/quantization/fp32_quantizer.cpp:163-190; HalfPrecisionQuantizer,
@@ -178,21 +160,29 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
-    __shared__ float part[T / 32];
+    __shared__ float s_qq, s_top;
     float* qf = reinterpret_cast<float*>(smem);
     const uint64_t q = blockIdx.x;
-    float qq = 0.f;
     for (uint32_t d = threadIdx.x; d < dim; d += T) {
-        const float v = widen(queries[q * dim + d]);
-        qf[d] = v;
-        qq = fmaf(v, v, qq);
+        qf[d] = widen(queries[q * dim + d]);
     }
-    qq = bf_block_sum<T>(qq, part);
     const ScoreSource<true> src{reinterpret_cast<const uint32_t*>(scores + q * ld)};
     const uint32_t found = block_select<T>(src, [](uint32_t i) { return i; }, n, kcand, keys, sel);
     block_sort_to<T>(keys, found, kcand, best);
     const uint32_t have = min(found, kcand);
     const float last = have > 0 ? ordered_to_float(static_cast<uint32_t>(best[have - 1] >> 32)) : 0.f;
+    if (threadIdx.x / 32 == T / 32 - 1) {   // (while the first warps wait for the candidates' rows)
+        const float top = __ldg(m.row_max);
+        float qq = 0.f;
+        for (uint32_t d = threadIdx.x % 32; d < dim; d += 32) {
+            qq = fmaf(qf[d], qf[d], qq);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        }
+        s_qq = qq;
+        s_top = top;
+    }
     for (uint32_t i = threadIdx.x; i < have; i += T) {
         const uint32_t row = static_cast<uint32_t>(best[i]);
         keys[i] = make_key(row_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, metric == VB200_METRIC_L2), row);
@@ -207,7 +197,7 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
         const bool l2 = metric == VB200_METRIC_L2;
         const bool dropped = n > kcand && found >= kcand;   // (then kcand > k)
         const float kth = dropped ? ordered_to_float(static_cast<uint32_t>(best[k - 1] >> 32)) : 0.f;
-        const float top = __ldg(m.row_max), size = top * sqrtf(qq);
+        const float top = s_top, qq = s_qq, size = top * sqrtf(qq);
         float margin = l2 ? fmaf(m.chain, top * top + qq + kth, 2.0f * m.matrix * size) : fmaf(m.chain + m.matrix, size, 3e-7f);
         margin += 1e-30f;   // (products below the smallest normal number round absolutely)
         // not finite: scores may have overflowed, and rows with them are not even among the counted

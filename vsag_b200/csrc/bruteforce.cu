@@ -263,7 +263,8 @@ struct vb200_bf {
     DevBuf<float> out_dists;
     DevBuf<uint32_t> stream_bound;   // per query: a bound of its k-th best distance while rows stream by
     DevBuf<float> row_max;           // the largest norm of a row
-    DevBuf<uint32_t> unsure;         // queries whose nominations may not have been enough: their number, then which
+    // a batch's score matrix: [0] the kernel's error flag, [1] how many queries' nominations may not have been enough, then which
+    DevBuf<uint32_t> unsure;
     PinnedBuf pinned;                // small host inputs and results
     std::mutex mu;
 };
@@ -797,10 +798,9 @@ bf_search_scores(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k, 
     uint64_t slice = BF_SLICE_SCORES / ld / TC_BM * TC_BM;   // whole row tiles
     slice = slice < TC_BM ? TC_BM : slice;
     VB_TRY(ix->scores.reserve(std::min(slice, nq) * ld));
-    VB_TRY(ix->unsure.reserve(nq + 1));
-    VB_CUDA(cudaMemsetAsync(ix->unsure.ptr, 0, sizeof(uint32_t), current_stream()));
-    VB_TRY(ix->tc.error_flag.reserve(2));
-    VB_CUDA(cudaMemsetAsync(ix->tc.error_flag.ptr, 0, 2 * sizeof(int), current_stream()));
+    VB_TRY(ix->unsure.reserve(nq + 2));
+    VB_CUDA(cudaMemsetAsync(ix->unsure.ptr, 0, 2 * sizeof(uint32_t), current_stream()));
+    int* const error_flag = reinterpret_cast<int*>(ix->unsure.ptr);
     const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks};
     const uint32_t kcand = static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n));
     const size_t smem = dim * sizeof(float);
@@ -809,13 +809,13 @@ bf_search_scores(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k, 
     margin.row_max = ix->row_max.ptr;
     margin.chain = static_cast<float>(dim + 16) * 6.0e-8f;
     margin.matrix = bf16 ? 2.0f * margin.chain : 4.0f * margin.chain + 3.0f / 262144.0f;
-    margin.unsure = ix->unsure.ptr;
+    margin.unsure = ix->unsure.ptr + 1;
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
         const uint64_t m = std::min(slice, nq - q0);
         const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
         const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks};
         margin.q_base = static_cast<uint32_t>(q0);
-        VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, staged.bias, ix->scores.ptr, ld, ix->tc.error_flag.ptr));
+        VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, staged.bias, ix->scores.ptr, ld, error_flag));
         if (bf16) {
             auto kernel = bf_rows_kernel<uint16_t, 512>;
             VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
@@ -922,19 +922,17 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
         return 0;
     };
     VB_TRY(results_to_host());
-    int flag = 0;
-    uint32_t unsure = 0;
+    uint32_t report[2] = {0, 0};   // of the score matrix: error flag, unsure queries
     if (scores) {
-        VB_CUDA(cudaMemcpyAsync(&flag, ix->tc.error_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, current_stream()));
-        VB_CUDA(cudaMemcpyAsync(&unsure, ix->unsure.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, current_stream()));
+        VB_CUDA(cudaMemcpyAsync(report, ix->unsure.ptr, sizeof(report), cudaMemcpyDeviceToHost, current_stream()));
     }
     VB_TRY(sync_stream());
-    if ((flag & 1) != 0) {
+    if ((report[0] & 1) != 0) {
         VB_FAIL(VB200_INTERNAL_ERROR, "tensor-core kernel gave up on a bounded wait");
     }
-    if (unsure > 0) {
-        for (uint64_t u0 = 0; u0 < unsure; u0 += BF_UNSURE_SLICE) {
-            VB_TRY(bf_stream_queries(ix, staged, std::min<uint64_t>(BF_UNSURE_SLICE, unsure - u0), ix->unsure.ptr + 1 + u0, k, ids_dev,
+    if (report[1] > 0) {
+        for (uint64_t u0 = 0; u0 < report[1]; u0 += BF_UNSURE_SLICE) {
+            VB_TRY(bf_stream_queries(ix, staged, std::min<uint64_t>(BF_UNSURE_SLICE, report[1] - u0), ix->unsure.ptr + 2 + u0, k, ids_dev,
                                      dists_dev));
         }
         VB_TRY(results_to_host());
