@@ -3320,10 +3320,11 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
 }
 
 // The search of a batch through a score per (query, row of its lists), from queries to results.  `plan`: the tile
-// launch, or null to scan pair by pair.  ids / dists: host or device.
+// launch, or null to scan pair by pair.  ids / dists: host or device.  *repeats: bucket_ids name a list twice for some
+// query; the search is then the grouped path's, which scans it twice, and the results here are to be thrown away.
 static int
 ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, uint32_t kscan, uint32_t nprobe, bool rerank,
-                  const TilePlan* plan, const int32_t* bucket_ids, int64_t* ids, float* dists) {
+                  const TilePlan* plan, const int32_t* bucket_ids, int64_t* ids, float* dists, bool* repeats) {
     SearchWorkspace& ws = ix->ws;
     cudaStream_t st = current_stream();
     const uint32_t dim = ix->dim, nlist = ix->nlist;
@@ -3337,9 +3338,9 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     if (plan != nullptr && slice < nq) {
         int64_t bytes = 0;
         const uint64_t parts = (nq + slice - 1) / slice, each = (nq + parts - 1) / parts;
-        for (uint64_t q0 = 0; q0 < nq; q0 += each) {
+        for (uint64_t q0 = 0; q0 < nq && !*repeats; q0 += each) {
             VB_TRY(ivf_search_scores(ix, queries + q0 * dim, std::min(each, nq - q0), k, kscan, nprobe, rerank, plan,
-                                     bucket_ids != nullptr ? bucket_ids + q0 * nprobe : nullptr, ids + q0 * k, dists + q0 * k));
+                                     bucket_ids != nullptr ? bucket_ids + q0 * nprobe : nullptr, ids + q0 * k, dists + q0 * k, repeats));
             bytes += ix->last_scan_bytes;
         }
         ix->last_scan_bytes = ix->last_scanned_bytes = bytes;
@@ -3353,8 +3354,11 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     const size_t ids_at = pin_q ? (q_bytes + 15) / 16 * 16 : 0, dists_at = ids_at + (pin_out ? total * sizeof(int64_t) : 0);
     const size_t rows_at = dists_at + (pin_out ? (total * sizeof(float) + 15) / 16 * 16 : 0);
     const size_t scalars_at = (rows_at + nq * sizeof(uint32_t) + 15) / 16 * 16;
-    VB_TRY(ws.pinned.reserve(scalars_at + SCALARS * sizeof(uint64_t)));
+    const size_t repeats_at = scalars_at + SCALARS * sizeof(uint64_t);
+    VB_TRY(ws.pinned.reserve(repeats_at + sizeof(uint32_t)));
     unsigned char* pin = static_cast<unsigned char*>(ws.pinned.ptr);
+    volatile uint32_t* repeated = reinterpret_cast<uint32_t*>(pin + repeats_at);
+    *repeated = 0;
     const float* q_dev = queries;
     if (host_q) {
         VB_TRY(ws.queries.reserve(nq * dim));
@@ -3421,6 +3425,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     bool routed_on_tensor_cores = false, prepared = false;
     if (bucket_ids != nullptr) {
         VB_CUDA(cudaMemcpyAsync(ws.probes.ptr, bucket_ids, nq * nprobe * sizeof(int32_t), cudaMemcpyDefault, st));
+        pp.repeats = reinterpret_cast<uint32_t*>(pin + repeats_at);
     } else {
         VB_TRY(ivf_route_device(ix, q_dev, nq, nprobe, ws.probes.ptr, nullptr, &pp, &prepared));
         routed_on_tensor_cores = routes_on_tensor_cores(ix, nq);
@@ -3606,6 +3611,10 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
             VB_CUDA(cudaMemsetAsync(ws.scalars.ptr + 4, 0, sizeof(uint64_t), st));
             VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
         }
+    }
+    if (*repeated != 0) {
+        *repeats = true;
+        return 0;
     }
     if (pin_out) {
         if (host_ids) {
@@ -4609,10 +4618,13 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
             const ScoreScan how = ivf_score_scan(ix, nq, kscan, np, &plan);
             if (how != SCAN_GROUPED) {
                 ws.filter = filter;
+                bool repeats = false;
                 const int rc = ivf_search_scores(ix, queries, nq, k, kscan, np, rerank, how == SCAN_TILES ? &plan : nullptr, bucket_ids, ids,
-                                                 dists);
+                                                 dists, &repeats);
                 ws.filter = nullptr;
-                return rc;
+                if (rc != 0 || !repeats) {
+                    return rc;
+                }
             }
         }
     }

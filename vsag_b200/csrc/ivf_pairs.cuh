@@ -67,6 +67,8 @@ struct PairsPrepare {
     float* probe_dists;       // [nq x nprobe] or null
     const uint32_t* list_off;
     PairTable t;
+    uint32_t* repeats;        // probes that a caller gave may name a list twice, which a query's stretch of scores has no room
+                              // for: the later one is taken out and *repeats becomes 1; null: the probes are distinct
     uint32_t* count;          // [nlist] += 1 per pair of a list that is not empty, or null
     uint32_t* rank;           // [nq x nprobe] which of its list's pairs each is (0xFFFFFFFF: empty list)
     // SQ8 (null qw8: none): the int8 weight terms, their scale and the query's constant (see sq8_query_prep_kernel)
@@ -191,7 +193,18 @@ pairs_prepare_kernel(const PairsPrepare p) {
         const uint32_t i = i0 + threadIdx.x;
         uint32_t len = 0;
         if (i < p.nprobe) {
-            const int32_t l = probes[i];
+            int32_t l = probes[i];
+            if (p.repeats != nullptr && l >= 0) {
+                // (the first of its kind is never changed, so it does not matter which of the others is gone already)
+                bool again = false;
+                for (uint32_t j = 0; j < i && !again; ++j) {
+                    again = *const_cast<const volatile int32_t*>(probes + j) == l;
+                }
+                if (again) {
+                    l = probes[i] = -1;
+                    *p.repeats = 1;
+                }
+            }
             if (l >= 0 && static_cast<uint32_t>(l) < p.nlist) {
                 len = p.list_off[l + 1] - p.list_off[l];
             }
