@@ -42,3 +42,29 @@ def test_finalising_kernel_at_the_edge_of_its_shared_memory(dim, nlist, nprobe, 
     code = SEARCH.format(root=root, dim=dim, nlist=nlist, nprobe=nprobe, nq=nq)
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stdout + done.stderr
+
+
+ADD = """
+import sys
+import numpy as np
+sys.path[:0] = [{root!r}, {root!r} + "/tests"]
+from conftest import mixture
+from vsag_b200 import engine
+
+dim = {dim}
+x = mixture(1, 400, dim, 4, 0.2)
+ix = engine.IvfHandle(dim, {metric}, 4, engine.QUANT_SQ8)
+ix.train(x, iters=1)
+ix.add(x, np.arange(len(x), dtype=np.int64))
+ids, dists = ix.search(x[:9], 1, 4)
+assert np.mean(ids[:, 0] == np.arange(9)) > 0.5 or {metric} == 1, ids
+"""
+
+
+@pytest.mark.parametrize("metric", [0, 2])
+@pytest.mark.parametrize("dim", [752, 767, 768, 769])
+def test_adding_rows_whose_balls_fill_the_default(dim, metric):
+    """Covering balls take 64 bytes of shared memory per dimension: 48 KiB at 768."""
+    root = str(Path(__file__).resolve().parents[1])
+    done = subprocess.run([sys.executable, "-c", ADD.format(root=root, dim=dim, metric=metric)], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stdout + done.stderr

@@ -115,9 +115,7 @@ bf_rescore(const T* queries, uint64_t nq, uint32_t dim, const T* base, const uin
     const size_t smem = n2 * sizeof(uint64_t) + dim * sizeof(float);
     VB_CHECK_ARG(smem <= 200 * 1024, "dim = %u is too large for the exact re-scoring step", dim);
     auto kernel = bf_rescore_kernel<T>;
-    if (smem > 48 * 1024) {
-        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    }
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
     VB_LAUNCH(kernel, static_cast<uint32_t>(nq), 128, smem, queries, dim, base, cand, ncand, n2, k, metric, out);
     return 0;
 }

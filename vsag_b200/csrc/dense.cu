@@ -437,10 +437,7 @@ normalize_rows_f32(const float* in, uint64_t rows, uint32_t dim, float* out) {
     }
     const size_t smem = 4 * static_cast<size_t>(dim) * sizeof(float);
     VB_CHECK_ARG(smem <= 200 * 1024, "dim too large to normalise on the device");
-    if (smem > 48 * 1024) {
-        VB_CUDA(cudaFuncSetAttribute(normalize_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
-    }
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(normalize_rows_kernel), smem));
     VB_LAUNCH(normalize_rows_kernel, static_cast<uint32_t>((rows + 3) / 4), 128, smem, in, rows, dim, out);
     return 0;
 }

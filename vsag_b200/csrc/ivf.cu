@@ -1602,10 +1602,7 @@ launch_merge(const uint64_t* part, uint64_t nq, uint64_t per_query, uint32_t k, 
              const uint8_t* slot_written = nullptr, uint32_t slot_keys = 1) {
     uint32_t cap = next_pow2(k + 256);
     size_t smem = cap * sizeof(uint64_t) + 16;
-    if (smem > 48 * 1024) {
-        VB_CUDA(cudaFuncSetAttribute(merge_keys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
-    }
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(merge_keys_kernel), smem));
     VB_LAUNCH(merge_keys_kernel, static_cast<uint32_t>(nq), 256, smem, part, per_query, k, cap, out, slot_written, slot_keys);
     return 0;
 }
@@ -2476,20 +2473,14 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
             if (lists <= 64 && n_keep <= ROUTE_PICK_SMALL) {
                 const uint32_t slots = next_pow2(lists * cap > ROUTE_PICK_SMALL ? lists * cap : ROUTE_PICK_SMALL);
                 const size_t smem = (static_cast<size_t>(slots) + ROUTE_PICK_SMALL) * sizeof(uint64_t) + ix->dim * sizeof(float);
-                if (smem > 48 * 1024) {
-                    VB_CUDA(cudaFuncSetAttribute(route_pick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(smem)));
-                }
+                VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(route_pick_kernel), smem));
                 // queries with few candidates (nearly all) are answered by a warp each; the block-per-query kernel
                 // takes what is left
                 const uint8_t* handled = nullptr;
                 const size_t warp_smem = 8 * (ROUTE_WARP_KEYS * sizeof(uint64_t) + ix->dim * sizeof(float));
                 if (ncand <= 128 && nprobe <= 128 && warp_smem <= 200 * 1024) {
                     VB_TRY(ws.route_handled.reserve(nq));
-                    if (warp_smem > 48 * 1024) {
-                        VB_CUDA(cudaFuncSetAttribute(route_pick_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(warp_smem)));
-                    }
+                    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(route_pick_warp_kernel), warp_smem));
                     VB_LAUNCH(route_pick_warp_kernel, static_cast<uint32_t>((nq + 7) / 8), 256, warp_smem, q_dev, nq, ix->dim,
                               ix->centroids.ptr, ws.route_keys.ptr, ws.route_cnt.ptr, lists, cap, ncand, nprobe, ix->metric,
                               probes_dev, dists_dev, ws.route_handled.ptr);
@@ -2569,10 +2560,7 @@ bounds_from_float_kernel(const float* __restrict__ bounds, uint64_t nq, uint32_t
 template <typename Kernel>
 static int
 launch_scan(Kernel kernel, const ScanParams& p, size_t smem) {
-    if (smem > 40 * 1024) {   // the kernels' static shared memory counts against the 48 KiB default too
-        VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
-    }
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
     int per_sm = 0;
     VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SCAN_THREADS, smem));
     if (per_sm < 1) {
@@ -2938,9 +2926,7 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
             const bool int8 = first_dpad32 != 0;
             const size_t smem = sq8_first_smem_bytes(p.k, ix->dpad, first_dpad32);
             auto kernel = int8 ? ivf_sq8_first_kernel<true, 3> : ivf_sq8_first_kernel<false, 2>;   // rows per lane: measured best
-            if (smem > 40 * 1024) {
-                VB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-            }
+            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
             int per_sm = 0;
             VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SQ8_FIRST_WARPS * 32, smem));
             if (per_sm < 1) {
@@ -3030,10 +3016,7 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
         VB_TRY(launch_merge(ws.part.ptr, nq, static_cast<uint64_t>(nprobe) * kscan, kscan, ws.merged.ptr, ws.slot_written.ptr, kscan));
         uint32_t n2 = next_pow2(kscan < 2 ? 2 : kscan);
         const size_t rescore_smem = n2 * sizeof(uint64_t) + 3 * ix->dim * sizeof(float);
-        if (rescore_smem > 48 * 1024) {
-            VB_CUDA(cudaFuncSetAttribute(sq8_rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(rescore_smem)));
-        }
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(sq8_rescore_kernel), rescore_smem));
         VB_LAUNCH(sq8_rescore_kernel, static_cast<uint32_t>(nq), 128, rescore_smem, q_dev, ix->dim,
                   ix->codes.ptr, ix->code_stride, ix->lower.ptr, ix->diff.ptr, ws.merged.ptr, kscan, n2,
                   kfinal, ix->metric, ws.keys.ptr, ix->use_residual ? ix->res_bias.ptr : static_cast<const float*>(nullptr),
@@ -4135,10 +4118,7 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
         VB_TRY(ix->list_radius.reserve(nlist));
         const size_t balls_smem = 2 * static_cast<size_t>(SQ8_BALLS) * dim * sizeof(float);
         VB_CHECK_ARG(balls_smem <= 200 * 1024, "dim too large for the list-ball kernel");
-        if (balls_smem > 48 * 1024) {
-            VB_CUDA(cudaFuncSetAttribute(sq8_list_balls_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(balls_smem)));
-        }
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(sq8_list_balls_kernel), balls_smem));
         // only the lists that grew get new balls (an add of a few rows must not cost a pass over the index)
         const uint32_t* old_off = ix->balls_valid ? ix->list_off.ptr : nullptr;
         VB_LAUNCH(sq8_list_balls_kernel, nlist, 128, balls_smem, new_codes.ptr, stride, dim, new_off_dev.ptr, old_off,
