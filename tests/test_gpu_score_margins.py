@@ -61,3 +61,37 @@ def test_exact_batches_with_overflowing_norms(engine, oracle):
     ix.add(base, np.arange(n, dtype=np.int64))
     got = ix.search(q, k)
     exactly(got, oracle.bf_search_fp32(base, q, k, 0))
+
+
+@pytest.mark.parametrize("dim,outlier,level,low,high", [
+    (518, 60.0, -0.3, 0.0, 0.1),     # the widest rows whose integer sums always fit 32 bits
+    (519, 60.0, -0.3, 0.0, 0.1),
+    (768, 60.0, -0.2, 0.0, 0.1),
+    (960, 60.0, -0.2, 0.1, 0.4),
+    (2048, 120.0, -0.2, 0.1, 0.4),
+    (2048, 60.0, 0.3, 0.3, 0.9),
+    (2049, 60.0, 0.3, 0.3, 0.9),     # no tiled copy
+])
+def test_sq8_long_rows_of_extreme_codes(engine, oracle, dim, outlier, level, low, high):
+    """Non-negative sparse rows (most codes are 0) against queries with one component far larger than the others: the
+    second integer sum of the ranking form reaches 32 bits from 519 dimensions on, at different rows for different data."""
+    n, nlist, nq, k = 1500, 4, 40, 10
+    rng = np.random.default_rng(dim)
+    filled = rng.random((n, dim)) < rng.uniform(low, high, (n, 1))
+    x = np.where(filled, 0.5 + 0.5 * rng.random((n, dim)), 0.0).astype(np.float32)
+    q = (level + 0.02 * rng.standard_normal((nq, dim))).astype(np.float32)
+    q[np.arange(nq), rng.integers(0, dim, nq)] = outlier
+    lower = x.min(axis=0)
+    diff = x.max(axis=0) - lower
+    for metric in (0, 1):
+        ix = engine.IvfHandle(dim, metric, nlist, engine.QUANT_SQ8)
+        ix.set_centroids(x[:nlist])
+        ix.set_sq8_model(lower, diff)
+        ix.add(x, np.arange(n, dtype=np.int64))
+        sizes, codes, inner = ix.get_lists()
+        off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+        probes = np.tile(np.arange(nlist, dtype=np.int32), (nq, 1))
+        want = oracle.ivf_sq8_search(codes, off, inner, lower, diff, q, probes, k, metric)
+        exactly(ix.search(q, k, nlist), want)
+        one = [ix.search(q[i:i + 1].copy(), k, nlist) for i in range(nq)]
+        exactly((np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])), want)

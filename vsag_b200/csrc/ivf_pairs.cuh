@@ -493,8 +493,7 @@ pair_scan_kernel(const PairScan p) {
                        const uint32_t pos = lbeg + static_cast<uint32_t>(row);
                        float v;
                        if constexpr (FMT == ROW_SQ8) {
-                           const float low = static_cast<float>(acc.a2 * 254 + acc.a3);
-                           const float f = fmaf(low, 1.0f / 64516.0f, static_cast<float>(acc.a1));
+                           const float f = sq8_term_sum(acc.a1, acc.a2, acc.a3, p.s.dim <= SQ8_NARROW_DIMS);
                            v = fmaf(cq, f, p.s.coef_b * __ldg(p.s.code_norm + pos)) + qa;
                        } else if constexpr (FMT == ROW_RABITQ) {
                            const float* tail = reinterpret_cast<const float*>(rows + row * p.s.code_stride + p.row_bytes);

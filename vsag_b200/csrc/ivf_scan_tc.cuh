@@ -583,7 +583,8 @@ ivf_sq8_scan_tc_kernel(const TcScanParams tp) {
                 uint32_t a1[16], a2[16], a3[16];
                 // sum_d w_d (code_d - 128) / s = A1 + (254 A2 + A3) / 254^2; |A1| < 2^22 (certain up to 256 dimensions:
                 // 127 * 128 * 256 < 2^22) converts exactly through the float whose integer image is 1.5 * 2^23 + A1,
-                // longer rows take the conversion instruction
+                // longer rows take the conversion instruction.  254 A2 + A3 fits 32 bits up to 518 dimensions; two stages and the
+                // query terms of longer rows than 448 do not fit shared memory, so none come here (nor to the int8 first phase).
                 auto partial_of = [&](int j, float cqj) -> float {
                     const int32_t low = static_cast<int32_t>(a2[j]) * 254 + static_cast<int32_t>(a3[j]);
                     const float hi = wide_sums ? static_cast<float>(static_cast<int32_t>(a1[j]))

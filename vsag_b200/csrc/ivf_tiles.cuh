@@ -727,11 +727,12 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                             const uint32_t j = g + i;
                             float v;
                             if (FMT == ROW_SQ8) {
-                                const float low = static_cast<float>(static_cast<int32_t>(v2[i]) * 254 + static_cast<int32_t>(v3[i]));
-                                const float f = fmaf(low, 1.0f / 64516.0f, static_cast<float>(static_cast<int32_t>(v1[i])));
+                                const float f = sq8_term_sum(static_cast<int32_t>(v1[i]), static_cast<int32_t>(v2[i]), static_cast<int32_t>(v3[i]),
+                                                             dim <= SQ8_NARROW_DIMS);
                                 v = fmaf(sh.c1[slot][j], f, x0) + sh.c0[slot][j];
                             } else if (FMT == ROW_RABITQ) {
-                                // |x|^2 + |q|^2 - 2 |x| |q| (ip / error); the set bits' sum S gives ip = 2 S - (sum of all)
+                                // |x|^2 + |q|^2 - 2 |x| |q| (ip / error); the set bits' sum S gives ip = 2 S - (sum of all).  (Signed
+                                // sums of terms up to 127: 254 u2 + u3 fits 32 bits to 66,000 dimensions, the row map ends at 1920.)
                                 const int32_t u1 = 2 * static_cast<int32_t>(v1[i]) - sh.t1[slot][j];
                                 const int32_t u2 = 2 * static_cast<int32_t>(v2[i]) - sh.t2[slot][j];
                                 const int32_t u3 = 2 * static_cast<int32_t>(v3[i]) - sh.t3[slot][j];

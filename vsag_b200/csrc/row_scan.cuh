@@ -95,7 +95,18 @@ struct RowAcc {   // fp32 / bf16 / fp16 rows: the chain over ascending dimension
     }
 };
 
-// SQ8: three integer sums over the int8 weight terms of one query, [3][qstride] bytes behind `q`; terms past the
+// SQ8: the sum over the three int8 terms of a query's weights, a1 + a2 / 254 + a3 / 254^2, from the exact integer sums.
+// 254 a2 + a3 reaches 127 * 128 * 255 per dimension, so it fits 32 bits up to 518 dimensions; longer rows add the two as
+// floats, whose rounding (2^-24 of a2 / 254) is far below what the terms themselves leave out.
+constexpr uint32_t SQ8_NARROW_DIMS = 518;
+
+__device__ __forceinline__ float
+sq8_term_sum(int32_t a1, int32_t a2, int32_t a3, bool narrow) {
+    const float low = narrow ? static_cast<float>(a2 * 254 + a3) : fmaf(static_cast<float>(a2), 254.0f, static_cast<float>(a3));
+    return fmaf(low, 1.0f / 64516.0f, static_cast<float>(a1));
+}
+
+// Three integer sums over the int8 weight terms of one query, [3][qstride] bytes behind `q`; terms past the
 // last dimension are zero.
 template <bool L2, int QN>
 struct RowAcc<ROW_SQ8, L2, QN> {
