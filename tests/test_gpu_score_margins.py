@@ -95,3 +95,30 @@ def test_sq8_long_rows_of_extreme_codes(engine, oracle, dim, outlier, level, low
         exactly(ix.search(q, k, nlist), want)
         one = [ix.search(q[i:i + 1].copy(), k, nlist) for i in range(nq)]
         exactly((np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])), want)
+
+
+@pytest.mark.parametrize("quant", ["QUANT_FP32", "QUANT_BF16"])
+def test_list_batches_with_overflowing_norms(engine, oracle, quant):
+    """Rows of lists whose squared norm is infinite, as tiles (a batch) and pair by pair, among them rows that are no
+    numbers and rows that the filter rejects."""
+    n, dim, nlist, nq, k = 2000, 40, 5, 60, 6
+    base = mixture(6, n, dim, nlist, 0.3)
+    base[::9] *= np.float32(3e19)
+    base[7::100] = np.nan
+    if quant == "QUANT_BF16":      # values the codec holds exactly, so that a row is its own query
+        base = (oracle.float_to_bf16(base).astype(np.uint32) << 16).view(np.float32).reshape(n, dim)
+    mine = np.flatnonzero(np.isfinite(base).all(axis=1))[:3 * nq:3]
+    q = np.ascontiguousarray(base[mine])
+    ix = engine.IvfHandle(dim, 0, nlist, getattr(engine, quant))
+    ix.set_centroids(mixture(7, nlist, dim, nlist, 0.3))
+    ix.add(base, np.arange(n, dtype=np.int64), labels=np.arange(n, dtype=np.int32) % nlist)
+    gone = np.zeros((n + 31) // 32, np.uint32)
+    gone[n // 64:] = 0x11111111
+    lists = np.tile(np.arange(nlist, dtype=np.int32), (nq, 1))
+    for bits in (None, gone):
+        many = ix.search_filtered(q, k, nlist, bucket_ids=lists, deny_inner_bits=bits)
+        one = [ix.search_filtered(q[i:i + 1].copy(), k, nlist, bucket_ids=lists[:1], deny_inner_bits=bits) for i in range(nq)]
+        assert np.array_equal(many[1], np.concatenate([o[1] for o in one]))
+        assert np.array_equal(many[0], np.concatenate([o[0] for o in one]))
+        kept = np.ones(n, bool) if bits is None else (np.unpackbits(bits.view(np.uint8), bitorder="little")[:n] == 0)
+        assert np.array_equal(many[0][kept[mine], 0], mine[kept[mine]]) and np.all(many[1][kept[mine], 0] == 0)

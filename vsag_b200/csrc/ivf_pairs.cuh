@@ -419,8 +419,9 @@ struct PairScan {
     uint32_t qstride;         // query values in shared memory: floats (SQ8: bytes of a term)
 };
 
-// The bit pattern of the score of a row that the id filter rejects: a NaN, which no selection takes.
-constexpr uint32_t SCORE_FILTERED = 0x7FFFFFFFu;
+// The bit pattern of the score of a row that the id filter rejects: a NaN, which no selection takes, and not the one that
+// arithmetic results in (0x7FFFFFFF: a score that overflowed, whose exact distance may be finite).
+constexpr uint32_t SCORE_FILTERED = 0x7FFFFFFEu;
 
 // est, record norm and error -> the reference's distance (ivf_rabitq_scan_kernel).
 __device__ __forceinline__ float
@@ -739,48 +740,49 @@ scan_finalize_kernel(const ScanFinalize p) {
             const uint32_t pos = static_cast<uint32_t>(best[i]);
             keys[i] = make_key(exact(pos), pos);
         }
-        bool sure = found < p.kcand;   // nothing was dropped
+        const bool dropped = found >= p.kcand;   // (else every row with a score is kept)
         block_sort_to<PAIR_THREADS>(keys, kept, p.kscan, best);
         found = kept;
-        if (!sure && kept >= p.kscan) {
-            const float kth = ordered_to_float(static_cast<uint32_t>(best[p.kscan - 1] >> 32));
-            float margin, offset = 0.f;
-            const float rows_max = __ldg(p.row_max);
-            if constexpr (FMT == ROW_RABITQ) {
-                const float qn = __ldg(sc.s.queries + q * (dim + 1) + dim);
-                // the dropped parts of the int8 terms and the additions' rounding, through 2 |x| |q| / error
-                const float ip = dim * (__ldg(sc.qscale + q) * (0.5f / 64516.0f) + 1.2e-7f);
-                margin = 2.0f * qn * __ldg(p.row_max + 1) * ip + 1e-6f * (rows_max + qn) * (rows_max + qn);
-            } else {
-                float qq = 0.f, mm = 0.f;
-                for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
-                    const float v = FMT == ROW_SQ8 ? qs[d] : qc[d];
-                    qq = fmaf(v, v, qq);
-                    if (FMT == ROW_SQ8) {
-                        const float mid = fmaf(qc[dim + d], 128.0f / 255.0f, qc[d]);
-                        mm = fmaf(mid, mid, mm);
-                    }
+        float margin, offset = 0.f;
+        const float rows_max = __ldg(p.row_max);
+        if constexpr (FMT == ROW_RABITQ) {
+            const float qn = __ldg(sc.s.queries + q * (dim + 1) + dim);
+            // the dropped parts of the int8 terms and the additions' rounding, through 2 |x| |q| / error
+            const float ip = dim * (__ldg(sc.qscale + q) * (0.5f / 64516.0f) + 1.2e-7f);
+            margin = 2.0f * qn * __ldg(p.row_max + 1) * ip + 1e-6f * (rows_max + qn) * (rows_max + qn);
+        } else {
+            float qq = 0.f, mm = 0.f;
+            for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
+                const float v = FMT == ROW_SQ8 ? qs[d] : qc[d];
+                qq = fmaf(v, v, qq);
+                if (FMT == ROW_SQ8) {
+                    const float mid = fmaf(qc[dim + d], 128.0f / 255.0f, qc[d]);
+                    mm = fmaf(mid, mid, mm);
                 }
-                qq = pair_block_sum(qq, part);
-                const float qn = sqrtf(qq);
-                float size = qn + rows_max;
-                margin = 0.f;
-                if constexpr (FMT == ROW_SQ8) {
-                    size += sqrtf(pair_block_sum(mm, part));
-                    margin = 2.0f * dim * 128.0f * __ldg(sc.qscale + q) * (0.5f / 64516.0f);
-                } else {
-                    offset = L2 ? qq : 1.0f;
-                    if (FMT == ROW_F32) {
-                        margin = 2.0f * qn * rows_max * (3.0f / 262144.0f);   // three dropped products of 2^-18
-                    }
-                }
-                margin += (dim + 16) * 1.2e-7f * size * size;   // fp32 sums of either side
             }
-            sure = kth < last + offset - margin;
+            qq = pair_block_sum(qq, part);
+            const float qn = sqrtf(qq);
+            float size = qn + rows_max;
+            margin = 0.f;
+            if constexpr (FMT == ROW_SQ8) {
+                size += sqrtf(pair_block_sum(mm, part));
+                margin = 2.0f * dim * 128.0f * __ldg(sc.qscale + q) * (0.5f / 64516.0f);
+            } else {
+                offset = L2 ? qq : 1.0f;
+                if (FMT == ROW_F32) {
+                    margin = 2.0f * qn * rows_max * (3.0f / 262144.0f);   // three dropped products of 2^-18
+                }
+            }
+            margin += (dim + 16) * 1.2e-7f * size * size;   // fp32 sums of either side
         }
+        margin += 1e-30f;   // (products below the smallest normal number round absolutely)
+        // A margin that is not finite: scores may have overflowed, and a row whose score is not a number is not among the
+        // found although its distance may be small.
+        const bool sure = margin < INFINITY &&
+                          (!dropped || ordered_to_float(static_cast<uint32_t>(best[p.kscan - 1] >> 32)) < last + offset - margin);
         if (!sure && n > 0) {
             for (uint32_t i = threadIdx.x; i < n; i += PAIR_THREADS) {
-                if (ScoreSource<>::ordered(scores[i]) <= ORDERED_INF) {
+                if (scores[i] != SCORE_FILTERED) {
                     scores[i] = __float_as_uint(exact(position(i)));
                 }
             }

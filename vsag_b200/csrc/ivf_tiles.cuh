@@ -744,7 +744,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                                 if (FMT == ROW_F32) {
                                     ip += __uint_as_float(v2[i]);
                                 }
-                                v = p.l2 != 0 ? fmaf(-2.0f, ip, x0) : -ip;
+                                v = fmaf(p.l2 != 0 ? -2.0f : -1.0f, ip, x0);   // (a negated NaN would rank first)
                             }
                             const uint32_t bits = part.drop ? SCORE_FILTERED : __float_as_uint(v);
                             if (j < it.nqt) {
