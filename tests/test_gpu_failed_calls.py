@@ -1,0 +1,44 @@
+"""A call that ends with an error leaves the handle usable: the next search returns what a fresh handle returns."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import mixture
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("quant,reorder", [("QUANT_FP32", False), ("QUANT_SQ8", False), ("QUANT_RABITQ", True)])
+@pytest.mark.parametrize("nq", [2, 90])
+def test_search_after_a_filter_that_cannot_be_staged(engine, oracle, quant, reorder, nq):
+    """The filter names more ids than device memory has bits for, so its copy cannot be made and the search ends after the
+    pairs of every list have been counted."""
+    from vsag_b200 import _capi
+
+    dim, n, nlist, nprobe, k = 48, 4000, 9, 5, 12
+    clip = quant == "QUANT_RABITQ"
+    x = mixture(1, n, dim, nlist, 0.3, lo=0.0 if clip else -1.0, clip=clip)
+    q = mixture(2, nq, dim, nlist, 0.3, lo=0.0 if clip else -1.0, clip=clip)
+    ix = engine.IvfHandle(dim, 0, nlist, getattr(engine, quant), use_reorder=reorder)
+    if clip:
+        ix.set_rabitq_rotation(oracle.random_rotation(dim, seed=3))
+    ix.train(x, iters=3)
+    ix.add(x, np.arange(n, dtype=np.int64))
+    want = ix.search(q, k, nprobe)
+    lib = _capi.load()
+    ids, dists = np.empty((nq, k), np.int64), np.empty((nq, k), np.float32)
+    bits = np.zeros(16, np.uint32)
+    for field in ("n_inner_bits", "n_label_bits"):
+        f = _capi.Filter()
+        f.deny_inner_bits = f.invalid_label_bits = bits.ctypes.data
+        setattr(f, field, 1 << 60)
+        for _ in range(2):
+            status = lib.vb200_ivf_search_filtered(ix._h, q.ctypes.data_as(C.c_void_p), nq, k, nprobe, 2.0, None,
+                                                   C.cast(C.byref(f), C.c_void_p), ids.ctypes.data_as(C.c_void_p),
+                                                   dists.ctypes.data_as(C.c_void_p))
+            assert status != 0
+        got = ix.search(q, k, nprobe)
+        assert np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])

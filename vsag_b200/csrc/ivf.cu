@@ -110,6 +110,9 @@ struct SearchWorkspace {
     DevBuf<TilePair> tile_pairs;
     DevBuf<uint16_t> tile_terms;
     DevBuf<uint32_t> rerank_ids, rerank_done;
+    // tile_count and rerank_done are zero between searches, left so by the kernels that use them up; a search that ended
+    // early may have left anything
+    bool counts_clear = false;
     DevBuf<TileItem> tile_items;
     DevBuf<int32_t> qsum;
 };
@@ -3396,11 +3399,22 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         pp.qscale = ws.qscale.ptr;
         pp.qa = ws.qa.ptr;
     }
-    if (plan != nullptr) {
-        if (ws.tile_count.cap < nlist) {
-            VB_TRY(ws.tile_count.reserve(nlist));
-            VB_CUDA(cudaMemsetAsync(ws.tile_count.ptr, 0, nlist * sizeof(uint32_t), st));   // tile_places_kernel leaves it cleared
+    // (reserved at their full size, so that what is cleared is what a later search may use)
+    if ((plan != nullptr && ws.tile_count.cap < nlist) || (rerank && ws.rerank_done.cap < nq)) {
+        ws.counts_clear = false;
+    }
+    VB_TRY(ws.tile_count.reserve(plan != nullptr ? nlist : 0));
+    VB_TRY(ws.rerank_done.reserve(rerank ? nq : 0));
+    if (!ws.counts_clear) {
+        if (ws.tile_count.cap > 0) {
+            VB_CUDA(cudaMemsetAsync(ws.tile_count.ptr, 0, ws.tile_count.bytes(), st));
         }
+        if (ws.rerank_done.cap > 0) {
+            VB_CUDA(cudaMemsetAsync(ws.rerank_done.ptr, 0, ws.rerank_done.bytes(), st));
+        }
+    }
+    ws.counts_clear = false;   // until this search has come to its end
+    if (plan != nullptr) {
         VB_TRY(ws.tile_rank.reserve(nq * nprobe));
         pp.count = ws.tile_count.ptr;
         pp.rank = ws.tile_rank.ptr;
@@ -3474,10 +3488,6 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     if (rerank) {
         VB_TRY(ws.rerank_ids.reserve(nq * kscan));
         VB_TRY(ws.keys.reserve(nq * kscan));
-        if (ws.rerank_done.cap < nq) {
-            VB_TRY(ws.rerank_done.reserve(nq));
-            VB_CUDA(cudaMemsetAsync(ws.rerank_done.ptr, 0, ws.rerank_done.cap * sizeof(uint32_t), st));   // rerank_rows_kernel leaves it cleared
-        }
         f.rerank_ids = ws.rerank_ids.ptr;
     }
     f.rows_scanned = reinterpret_cast<uint32_t*>(pin + rows_at);
@@ -3595,6 +3605,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
             VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
         }
     }
+    ws.counts_clear = true;
     if (*repeated != 0) {
         *repeats = true;
         return 0;
@@ -4602,6 +4613,9 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
                 const int rc = ivf_search_scores(ix, queries, nq, k, kscan, np, rerank, how == SCAN_TILES ? &plan : nullptr, bucket_ids, ids,
                                                  dists, &repeats);
                 ws.filter = nullptr;
+                if (rc != 0) {
+                    (void)cudaStreamSynchronize(current_stream());   // what was launched may use the workspace
+                }
                 if (rc != 0 || !repeats) {
                     return rc;
                 }
