@@ -56,3 +56,25 @@ def test_candidate_kernel_wait_runs_out_then_recovers(engine, oracle):
         assert lib.vb200_debug_set_wait_limit(-1) == 0
     assert np.array_equal(engine.kmeans_assign(x, c), want)
     assert np.array_equal(want, oracle.kmeans_assign(x, c)[0])
+
+
+def test_a_grouped_scan_that_gave_up_does_not_fail_the_next_tiled_one(engine):
+    """The two scans share a flag.  With k shallow against the lists a large batch is grouped, with k deep it goes as tiles."""
+    from vsag_b200 import _capi
+
+    dim, nlist, n = 32, 32, 24_000
+    x, q = mixture(405, n, dim, nlist, 0.15), mixture(406, 1200, dim, nlist, 0.15)
+    ix = engine.IvfHandle(dim, engine.METRIC_L2, nlist, engine.QUANT_SQ8)
+    ix.train(x, iters=2)
+    ix.add(x, np.arange(n, dtype=np.int64))
+    shallow, deep = ix.search(q, 5, 8), ix.search(q, 200, 8)
+    lib = _capi.load()
+    assert lib.vb200_debug_set_wait_limit(0) == 0
+    try:
+        with pytest.raises(_capi.VsagB200Error, match="bounded wait"):
+            ix.search(q, 5, 8)
+    finally:
+        assert lib.vb200_debug_set_wait_limit(-1) == 0
+    for k, want in ((200, deep), (5, shallow)):
+        again = ix.search(q, k, 8)
+        assert np.array_equal(again[0], want[0]) and np.array_equal(again[1], want[1])

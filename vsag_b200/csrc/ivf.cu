@@ -2332,6 +2332,17 @@ route_flag_check(uint64_t flag_word) {
     return 0;
 }
 
+// After a synchronisation: fails if a scan of the call reported a wait that gave up.  The flag stays set on the device: the
+// grouped scan clears it before it starts, a score path when it finds counts_clear unset.
+static int
+scan_flag_check(SearchWorkspace& ws, uint64_t flag_word) {
+    if (flag_word != 0) {
+        ws.counts_clear = false;
+        VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
+    }
+    return 0;
+}
+
 // For callers that only route: waits for the stream and reads the flag.
 static int
 route_sync_and_check(SearchWorkspace& ws) {
@@ -3412,6 +3423,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         if (ws.rerank_done.cap > 0) {
             VB_CUDA(cudaMemsetAsync(ws.rerank_done.ptr, 0, ws.rerank_done.bytes(), st));
         }
+        VB_CUDA(cudaMemsetAsync(ws.scalars.ptr + 4, 0, sizeof(uint64_t), st));   // (a scan that gave up left its flag)
     }
     ws.counts_clear = false;   // until this search has come to its end
     if (plan != nullptr) {
@@ -3600,9 +3612,8 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         if (routed_on_tensor_cores) {
             VB_TRY(route_flag_check(scalars[8]));
         }
-        if (plan != nullptr && scalars[4] != 0) {
-            VB_CUDA(cudaMemsetAsync(ws.scalars.ptr + 4, 0, sizeof(uint64_t), st));
-            VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
+        if (plan != nullptr) {
+            VB_TRY(scan_flag_check(ws, scalars[4]));
         }
     }
     ws.counts_clear = true;
@@ -4639,9 +4650,7 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
     VB_TRY(route_flag_check(scalars[8]));
     ix->last_scan_bytes = static_cast<int64_t>(scalars[0]);
     ix->last_scanned_bytes = static_cast<int64_t>(ws.pruning ? scalars[3] : scalars[0]);
-    if (scalars[4] != 0) {
-        VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
-    }
+    VB_TRY(scan_flag_check(ws, scalars[4]));
     if (timed_out != nullptr) {
         *timed_out = scalars[5] != 0 ? 1 : 0;
     }
@@ -4696,10 +4705,7 @@ vb200_ivf_search_partial(vb200_ivf_t ix, const float* queries, uint64_t nq, uint
     VB_TRY(route_flag_check(scalars[8]));
     ix->last_scan_bytes = static_cast<int64_t>(scalars[0]);
     ix->last_scanned_bytes = static_cast<int64_t>(ix->ws.pruning ? scalars[3] : scalars[0]);
-    if (scalars[4] != 0) {
-        VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
-    }
-    return 0;
+    return scan_flag_check(ix->ws, scalars[4]);
 }
 
 extern "C" int64_t
@@ -4950,9 +4956,7 @@ vb200_ivf_search_sharded(vb200_ivf_t ix, vb200_comm_t comm, const float* queries
     if (ix->n_total != 0 && ix->n_stored != 0) {
         ix->last_scan_bytes = static_cast<int64_t>(scalars[0]);
         ix->last_scanned_bytes = static_cast<int64_t>(ws.pruning ? scalars[3] : scalars[0]);
-        if (scalars[4] != 0) {
-            VB_FAIL(VB200_INTERNAL_ERROR, "the tensor-core scan gave up on a bounded wait");
-        }
+        VB_TRY(scan_flag_check(ws, scalars[4]));
     }
     return 0;
 }
