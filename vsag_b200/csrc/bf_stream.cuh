@@ -94,22 +94,22 @@ bf_stream_kernel(const BfStream p) {
     ts.finish(here, p.part, p.bound);
 }
 
-// One CTA per query: the k best of its `n` partial keys (payload = row), as results of query pick[blockIdx.x] (null: its own
-// number).
+// One CTA per query: the `keep` best of its `n` partial keys (payload = row), as the first of the k results of query
+// pick[blockIdx.x] (null: its own number).
 template <int T>
 __global__ void __launch_bounds__(T)
-bf_pick_kernel(const uint64_t* __restrict__ part, uint32_t n, uint32_t k, const uint32_t* __restrict__ pick,
+bf_pick_kernel(const uint64_t* __restrict__ part, uint32_t n, uint32_t keep, uint32_t k, const uint32_t* __restrict__ pick,
                const int64_t* __restrict__ labels, int64_t* __restrict__ ids, float* __restrict__ dists) {
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
     const uint64_t* mine = part + static_cast<uint64_t>(blockIdx.x) * n;
     const uint32_t found = block_select<T>(load_source([&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i) >> 32); }),
-                                           [&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i)); }, n, k, keys, sel);
-    block_sort_to<T>(keys, found, k, best);
+                                           [&](uint32_t i) { return static_cast<uint32_t>(__ldg(mine + i)); }, n, keep, keys, sel);
+    block_sort_to<T>(keys, found, keep, best);
     const uint64_t q = pick != nullptr ? __ldg(pick + blockIdx.x) : blockIdx.x;
     for (uint32_t i = threadIdx.x; i < k; i += T) {
-        const bool there = i < found;
+        const bool there = i < min(found, keep);
         ids[q * k + i] = there ? __ldg(labels + static_cast<uint32_t>(best[i])) : -1;
         dists[q * k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
     }

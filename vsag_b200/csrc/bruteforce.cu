@@ -699,6 +699,12 @@ struct BfStaged {
     bool masked = false;
 };
 
+// Shared memory of a CTA that streams rows for qn queries, `keep` results each (no more than there are rows).
+static uint32_t
+bf_stream_cap(uint32_t keep) {
+    return next_pow2(keep + RS_ROWS);
+}
+
 static size_t
 bf_stream_smem(uint32_t dim, uint32_t cap, uint32_t qn) {
     return RS_STAGES * RS_STAGE + static_cast<size_t>(qn) * ((dim + 7) / 8 * 8) * sizeof(float) +
@@ -718,8 +724,9 @@ bf_stream_queries(vb200_bf* ix, const BfStaged& staged, uint64_t nq, const uint3
     p.dim = dim;
     p.base = bf16 ? reinterpret_cast<const unsigned char*>(ix->base_bf16.ptr) : reinterpret_cast<const unsigned char*>(ix->base_f32.ptr);
     p.n = ix->n;
-    p.k = k;
-    p.cap = next_pow2(k + RS_ROWS);
+    const uint32_t keep = static_cast<uint32_t>(std::min<uint64_t>(k, ix->n));
+    p.k = keep;
+    p.cap = bf_stream_cap(keep);
     p.masked = staged.masked ? staged.bias : nullptr;
     uint32_t qn = 1;
     while (qn < nq && qn < BF_STREAM_QUERIES) {
@@ -765,14 +772,15 @@ bf_stream_queries(vb200_bf* ix, const BfStaged& staged, uint64_t nq, const uint3
     // one wave of CTAs: with several tiles of queries each takes a larger share of the rows
     const uint64_t slots = static_cast<uint64_t>(sm_count()) * std::max(per_sm, 1);
     const uint32_t grid = static_cast<uint32_t>(std::min(chunks, std::max<uint64_t>(slots / tiles, 1)));
-    VB_CHECK_ARG(nq * grid * k < 0xFFFFFFFFull && tiles <= 65535, "query batch too large");
-    VB_TRY(ix->part.reserve(nq * grid * k));
+    VB_CHECK_ARG(nq * grid * keep < 0xFFFFFFFFull && tiles <= 65535, "query batch too large");
+    VB_TRY(ix->part.reserve(nq * grid * keep));
     VB_TRY(ix->stream_bound.reserve(nq));
     VB_CUDA(cudaMemsetAsync(ix->stream_bound.ptr, 0xFF, nq * sizeof(uint32_t), current_stream()));
     p.part = ix->part.ptr;
     p.bound = ix->stream_bound.ptr;
     VB_LAUNCH(kernel, dim3(grid, tiles), RS_ROWS, smem, p);
-    VB_LAUNCH(bf_pick_kernel<1024>, static_cast<uint32_t>(nq), 1024, 0, ix->part.ptr, grid * k, k, pick, ix->labels.ptr, ids_dev, dists_dev);
+    VB_LAUNCH(bf_pick_kernel<1024>, static_cast<uint32_t>(nq), 1024, 0, ix->part.ptr, grid * keep, keep, k, pick, ix->labels.ptr, ids_dev,
+              dists_dev);
     return 0;
 }
 
@@ -879,7 +887,8 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
     int64_t* ids_dev = !host_ids ? ids : (pin_out ? pin_ids : ix->out_ids.ptr);
     float* dists_dev = !host_d ? dists : (pin_out ? pin_dists : ix->out_dists.ptr);
     const bool k_fits = std::min<uint64_t>(k + BF_SLACK, ix->n) <= 1024;
-    const bool streams = k_fits && bf_stream_smem(ix->dim, next_pow2(k + RS_ROWS), 1) <= 220 * 1024;
+    // (rows too long for a stream's shared memory, above 40,000 dimensions, are left to the slab of scores)
+    const bool streams = k_fits && bf_stream_smem(ix->dim, bf_stream_cap(static_cast<uint32_t>(std::min<uint64_t>(k, ix->n))), 1) <= 220 * 1024;
     const bool scores = tensor_cores_enabled() && streams && nq > BF_STREAM_QUERIES && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES;
     BfStaged staged;
     bool keyed = false;
@@ -888,7 +897,7 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
     // Up to eight queries share one pass over the rows; more go to the tensor cores -- through a score matrix
     // while that is cheaper than selecting as the scores appear (measured: up to about 4e8 scores), see
     // bf_search_keys for the rest.
-    if (nq <= BF_STREAM_QUERIES && k_fits) {
+    if (nq <= BF_STREAM_QUERIES && streams) {
         rc = bf_stage(ix, queries, nq, &staged.queries, &staged.bias, &staged.masked);
         if (rc == 0) {
             rc = bf_stream_queries(ix, staged, nq, nullptr, k, ids_dev, dists_dev);
