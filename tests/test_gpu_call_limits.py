@@ -28,3 +28,21 @@ def test_exact_search_at_its_limits(engine, oracle, n, dim, k, nq):
         ix = engine.BfHandle(dim, metric)
         ix.add(base, np.arange(n, dtype=np.int64))
         exactly(ix.search(q, k), oracle.bf_search_fp32(base, q, k, metric))
+
+
+def test_more_one_bit_queries_than_a_launch_has_tiles(engine, oracle):
+    """The queries' rotation is launched over tiles of up to eight queries, 65,535 at once."""
+    n, dim, nlist, nq, k = 300, 32, 4, 8 * 65_535 + 9, 2
+    x = mixture(1, n, dim, nlist, 0.2, lo=0.0, clip=True)
+    ix = engine.IvfHandle(dim, 0, nlist, engine.QUANT_RABITQ, use_reorder=True)
+    ix.set_rabitq_rotation(oracle.random_rotation(dim, seed=3))
+    ix.train(x, iters=2)
+    ix.add(x, np.arange(n, dtype=np.int64))
+    few = mixture(2, 1000, dim, nlist, 0.2, lo=0.0, clip=True)
+    want = ix.search(few, k, 2)
+    q = np.ascontiguousarray(np.tile(few, (nq // 1000 + 1, 1))[:nq])
+    ids, dists = ix.search(q, k, 2)
+    for at in (0, 65_000, 523_000):
+        assert np.array_equal(dists[at:at + 1000], want[1]) and np.array_equal(ids[at:at + 1000], want[0])
+    tail = nq % 1000
+    assert np.array_equal(dists[nq - tail:], want[1][:tail]) and np.array_equal(ids[nq - tail:], want[0][:tail])

@@ -2368,8 +2368,6 @@ launch_row_chains(const float* queries, uint64_t nq, uint64_t q_stride, const fl
     }
     const size_t smem = smem_of(qn);
     VB_CHECK_ARG(smem <= 220 * 1024, "dim = %u is too large for the routing kernel", dim);
-    const uint64_t tiles = (nq + qn - 1) / qn;
-    VB_CHECK_ARG(tiles <= 65535, "too many query tiles");
     const bool wide = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
     using Kernel = void (*)(const float*, uint32_t, uint64_t, const float*, uint32_t, uint32_t, int, float*, uint64_t);
 #define VB_ROW_CHAINS(QN)                                                                          \
@@ -2378,8 +2376,12 @@ launch_row_chains(const float* queries, uint64_t nq, uint64_t q_stride, const fl
     const Kernel kernel = qn == 8 ? VB_ROW_CHAINS(8) : (qn == 4 ? VB_ROW_CHAINS(4) : (qn == 2 ? VB_ROW_CHAINS(2) : VB_ROW_CHAINS(1)));
 #undef VB_ROW_CHAINS
     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
-    VB_LAUNCH(kernel, dim3(chunks, static_cast<uint32_t>(tiles)), RS_ROWS, smem, queries, static_cast<uint32_t>(nq), q_stride, rows,
-              n_rows, dim, one_minus ? 1 : 0, out, ld);
+    const uint64_t slice = 65535ull * qn;   // (query tiles are the grid's second dimension)
+    for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
+        const uint64_t m = std::min(slice, nq - q0);
+        VB_LAUNCH(kernel, dim3(chunks, static_cast<uint32_t>((m + qn - 1) / qn)), RS_ROWS, smem, queries + q0 * q_stride,
+                  static_cast<uint32_t>(m), q_stride, rows, n_rows, dim, one_minus ? 1 : 0, out + q0 * ld, ld);
+    }
     return 0;
 }
 
