@@ -122,3 +122,33 @@ def test_list_batches_with_overflowing_norms(engine, oracle, quant):
         assert np.array_equal(many[0], np.concatenate([o[0] for o in one]))
         kept = np.ones(n, bool) if bits is None else (np.unpackbits(bits.view(np.uint8), bitorder="little")[:n] == 0)
         assert np.array_equal(many[0][kept[mine], 0], mine[kept[mine]]) and np.all(many[1][kept[mine], 0] == 0)
+
+
+@pytest.mark.parametrize("quant", ["QUANT_SQ8", "QUANT_BF16", "QUANT_FP16", "QUANT_RABITQ"])
+@pytest.mark.parametrize("offset,dim,k", [(1000.0, 64, 20), (3.0, 300, 100), (0.0, 960, 100)])
+def test_crowded_scores_of_every_codec(engine, oracle, quant, offset, dim, k):
+    """Rows closer to one another than the scores' rounding, from all of them to a few: batches, which go as tiles, return
+    what the exact arithmetic of the codec gives."""
+    n, nlist, nq = 1800, 4, 40
+    clip = quant == "QUANT_RABITQ"
+    spread = 0.02 if offset > 100 else 0.2
+    if clip:
+        x, q = (mixture(s, m, dim, nlist, 0.002 if offset else 0.05, lo=0.0, clip=True) for s, m in ((5, n), (6, nq)))
+    else:
+        x, q = ((offset + mixture(s, m, dim, nlist, spread)).astype(np.float32) for s, m in ((5, n), (6, nq)))
+    for metric in (0,) if clip else (0, 1):
+        ix = engine.IvfHandle(dim, metric, nlist, getattr(engine, quant))
+        if clip:
+            ix.set_rabitq_rotation(oracle.random_rotation(dim, seed=3))
+        ix.train(x, iters=3)
+        ix.add(x, np.arange(n, dtype=np.int64))
+        got = ix.search(q, k, nlist)
+        if quant == "QUANT_SQ8":
+            sizes, codes, inner = ix.get_lists()
+            off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+            lower, diff = ix.get_sq8_model()
+            probes = np.tile(np.arange(nlist, dtype=np.int32), (nq, 1))
+            exactly(got, oracle.ivf_sq8_search(codes, off, inner, lower, diff, q, probes, k, metric))
+        else:     # one query goes pair by pair, which is the codec's own arithmetic
+            one = [ix.search(q[i:i + 1].copy(), k, nlist) for i in range(nq)]
+            exactly(got, (np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])))

@@ -135,8 +135,8 @@ bf_row_max_kernel(const float* __restrict__ sq, uint64_t n, float* __restrict__ 
 //   IP  the score -<x, q> and the exact 1 - <x, q> differ by (chain + matrix) X Q and the rounding of the subtraction
 //   L2  |x|^2 - 2 <x, q> + |q|^2 and the exact chain differ by chain (X^2 + Q^2 + d) + 2 matrix X Q, d the distance
 // chain = the rounding of a sum of dim products in fp32, (dim + 16) 2^-24; matrix = that of the tensor cores' sums.  Those
-// take 16 products and the running sum per step, each cut to 24 bits or more: below (17/16) dim 2^-24 per term pair; with
-// split terms three pairs and the dropped products, 3 * 2^-18.
+// take 16 products and the running sum per step, each cut one bit below fp32's last or lower: at most (17/16) dim 2^-24 per
+// term pair; with split terms three pairs and the dropped products, 3 * 2^-18.
 struct BfMargin {
     const float* row_max;   // X
     float chain, matrix;

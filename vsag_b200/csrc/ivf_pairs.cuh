@@ -751,29 +751,40 @@ scan_finalize_kernel(const ScanFinalize p) {
             const float ip = dim * (__ldg(sc.qscale + q) * (0.5f / 64516.0f) + 1.2e-7f);
             margin = 2.0f * qn * __ldg(p.row_max + 1) * ip + 1e-6f * (rows_max + qn) * (rows_max + qn);
         } else {
-            float qq = 0.f, mm = 0.f;
+            float qq = 0.f, ss = 0.f;
             for (uint32_t d = threadIdx.x; d < dim; d += PAIR_THREADS) {
                 const float v = FMT == ROW_SQ8 ? qs[d] : qc[d];
                 qq = fmaf(v, v, qq);
                 if (FMT == ROW_SQ8) {
-                    const float mid = fmaf(qc[dim + d], 128.0f / 255.0f, qc[d]);
-                    mm = fmaf(mid, mid, mm);
+                    const float span = fabsf(qc[d]) + fabsf(qc[dim + d]);
+                    ss = fmaf(span, span, ss);
                 }
             }
             qq = pair_block_sum(qq, part);
             const float qn = sqrtf(qq);
-            float size = qn + rows_max;
-            margin = 0.f;
+            const float kth = dropped && L2 ? ordered_to_float(static_cast<uint32_t>(best[p.kscan - 1] >> 32)) : 0.f;
+            // Q, X and S are the norms of the query, of the longest row and of |lower| + |diff|, d the k-th distance.
+            constexpr float EPS = 6.0e-8f;
+            const float chain = EPS * static_cast<float>(dim + 16);   // rounding of a chain of dim products
             if constexpr (FMT == ROW_SQ8) {
-                size += sqrtf(pair_block_sum(mm, part));
+                // The integer sums are exact, so what remains is what the terms leave out; the chains behind |x|^2 and the exact
+                // distance (X^2 and d, or X Q); the query's constant, summed by 256 threads; and the rounding of the dequantized
+                // values and of the last few operations.  (One (dim + 16) 2^-23 of (Q + X + S)^2 for all of them was five
+                // times as large: of 100 results among 390 rows a list, 960 dimensions, some queries of every batch were
+                // never sure and scored all their rows, 5.9 ms instead of 0.3.)
+                const float span = sqrtf(pair_block_sum(ss, part)), few = EPS * static_cast<float>(dim / PAIR_THREADS + 32);
                 margin = 2.0f * dim * 128.0f * __ldg(sc.qscale + q) * (0.5f / 64516.0f);
+                margin += L2 ? chain * (rows_max * rows_max + kth) + few * (qq + 2.0f * qn * span)
+                             : chain * rows_max * qn + few * (1.0f + qn * span);
             } else {
+                // The sums of the tensor cores (16 products and the running sum per step, cut one bit below fp32's last or
+                // lower; fp32 rows: two steps into one accumulator, and three dropped products of 2^-18); the exact chain
+                // (d, or X Q); the sums behind X^2 and Q^2, over 32 lanes or more.
+                const float matrix = FMT == ROW_F32 ? 2.2f * chain + 3.0f / 262144.0f : 1.1f * chain;
+                const float few = EPS * static_cast<float>(dim / 32 + 32), size = qn * rows_max;
                 offset = L2 ? qq : 1.0f;
-                if (FMT == ROW_F32) {
-                    margin = 2.0f * qn * rows_max * (3.0f / 262144.0f);   // three dropped products of 2^-18
-                }
+                margin = L2 ? chain * kth + 2.0f * matrix * size + few * (qq + rows_max * rows_max) : (chain + matrix) * size + 3e-7f;
             }
-            margin += (dim + 16) * 1.2e-7f * size * size;   // fp32 sums of either side
         }
         margin += 1e-30f;   // (products below the smallest normal number round absolutely)
         // A margin that is not finite: scores may have overflowed, and a row whose score is not a number is not among the
