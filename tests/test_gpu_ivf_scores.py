@@ -97,3 +97,24 @@ def test_selection_reads_the_passing_groups(engine, oracle, n):
     want = oracle.bf_search_fp32(base, q, k, 0)
     assert np.array_equal(got[1], want[1])
     assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)
+
+
+@pytest.mark.parametrize("n,nprobe,nq,k", [
+    (20_000, 8, 1600, 3),        # around 4e6 rows: pairs or tiles below, the pruning scan above
+    (200_000, 64, 800, 10),      # around 1.5e8 rows, k shallow
+    (60_000, 64, 2700, 110),     # the same, k deep against lists of 940 rows
+])
+def test_results_do_not_depend_on_the_scan(engine, n, nprobe, nq, k):
+    """A batch above the lines between the scans, the same queries in batches below them, lists pruned and not."""
+    dim, nlist = 32, 64
+    x, q = mixture(3, n, dim, nlist, 0.2), mixture(4, nq, dim, nlist, 0.2)
+    ix = engine.IvfHandle(dim, 0, nlist, engine.QUANT_SQ8)
+    ix.train(x[:20_000], iters=2)
+    ix.add(x, np.arange(n, dtype=np.int64))
+    want = [ix.search(q[i:i + 100].copy(), k, nprobe) for i in range(0, nq, 100)]
+    want = tuple(np.concatenate(part) for part in zip(*want))
+    for prune in (True, False):
+        ix.set_list_pruning(prune)
+        got = ix.search(q, k, nprobe)
+        assert np.array_equal(got[1], want[1])
+        assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)

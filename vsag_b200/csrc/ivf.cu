@@ -3200,9 +3200,40 @@ tile_plan(const vb200_ivf* ix, TilePlan* plan) {
     return false;
 }
 
+// Where SQ8 batches leave the score paths for the grouped scan, which keeps no scores and rules lists out by the bounds
+// of each query's nearest one.  (nq, k and n as below; microseconds, the score path against the grouped one.)
+//   lists pruned, k shallow (8 (k + 16) <= rows a list): from 3.5e6 rows as pairs, 4e6 as tiles
+//     3.9e6 of 96 dims 480 / 351, 5.9e6 of 128 909 / 525; 2.0e6 376 / 414, 2.3e6 262 / 468
+//   otherwise, as tiles: the time of a tile is its own and 0.07 per query in it, whatever comes of the scores; so from 1.5e8 rows,
+//   and from 3.5e7 where the lists do not stay in L2 and tiles are mostly empty (fewer than 40 queries a list)
+//     lists not pruned: 3.9e8 of 96 (39 a list) 5852 / 2848, 1.2e8 (12) 1772 / 1294, 3.9e7 of 300 (20) 2614 / 2030;
+//                       9.4e7 of 300 (47) 1969 / 1966, 7.8e7 of 128 1062 / 1134, 3.1e7 of 300 717 / 914
+//     pruned, k deep:   3.9e8 of 96 6022 / 1773, 1.6e8 of 128 1768 / 1357, 4.9e7 of 96 (5) 1909 / 1204, 3.1e8 of 640 7935 / 5186;
+//                       9.4e7 of 300 (47) 2044 / 2620, 4.7e7 of 128 715 / 1155, 9.4e7 of 640 2440 / 3352
+//   and from four times that where lists are not pruned and k is deep: the grouped scan selects more there (4.9e7 of 96 1912 / 2350,
+//   5e8 of 64 2045 / 2831; 3.9e8 of 96 6020 / 4134)
+// Without pruning the grouped scan of rows longer than 448 dimensions (no tensor cores) is never the faster one (2.5e7 of 960
+// 792 / 2728).
+constexpr double GROUPED_PAIR_ROWS = 3.5e6, GROUPED_TILE_ROWS = 4e6, GROUPED_ROWS = 1.5e8, GROUPED_ROWS_FAR = 3.5e7;
+constexpr double GROUPED_FAR_BYTES = 256e6, GROUPED_FAR_PER_LIST = 40.0;
+constexpr uint32_t GROUPED_TC_DIMS = 448;
+
+static bool
+sq8_batch_is_grouped(const vb200_ivf* ix, double per_list, double mean_len, double rows, uint32_t kscan) {
+    const bool shallow = 8.0 * (kscan + SQ8_SLACK) <= mean_len;
+    if (ix->prune_lists && shallow) {
+        return rows > GROUPED_TILE_ROWS;
+    }
+    if (!ix->prune_lists && ix->dim > GROUPED_TC_DIMS) {
+        return false;
+    }
+    const bool far = static_cast<double>(ix->n_stored) * ix->code_size > GROUPED_FAR_BYTES && per_list < GROUPED_FAR_PER_LIST &&
+                     ix->dim <= GROUPED_TC_DIMS;
+    return rows > (far ? GROUPED_ROWS_FAR : GROUPED_ROWS) * (ix->prune_lists || shallow ? 1.0 : 4.0);
+}
+
 // The line between pairs and tiles: from about four queries per probed list on a tile per list saves more of the
-// lists' traffic than grouping the pairs costs (three small launches).  SQ8 batches with k shallow against the
-// lists keep the pruning scan once they are large: their first list gives a bound that rules most pairs out.
+// lists' traffic than grouping the pairs costs (three small launches).
 static ScoreScan
 ivf_score_scan(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe, TilePlan* plan) {
     const SearchWorkspace& ws = ix->ws;
@@ -3219,13 +3250,16 @@ ivf_score_scan(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe
     const double rows = static_cast<double>(nq) * nprobe * mean_len;
     if (tensor_cores_enabled() && per_list >= TILE_MIN_QUERIES && nq * nprobe < (uint64_t{1} << 31) &&
         (sq8 ? ix->codes_t.ptr != nullptr : ix->has_row_map) && tile_plan(ix, plan)) {
-        const bool prunes = sq8 && ix->prune_lists && ix->codes_t.ptr != nullptr && 8.0 * (kscan + SQ8_SLACK) <= mean_len && rows > 4e6;
-        if (!prunes) {
-            return SCAN_TILES;
-        }
+        return sq8 && sq8_batch_is_grouped(ix, per_list, mean_len, rows, kscan) ? SCAN_GROUPED : SCAN_TILES;
     }
-    if (per_list >= 6.0 || (sq8 && rows * ix->code_size > 1e9)) {
+    if (per_list >= 6.0) {
         return SCAN_GROUPED;
+    }
+    if (sq8) {
+        // (pairs read a list once per query: 3.1e6 rows of 300 bytes 923 / 789, 920 / 749 not pruned; 1.2e6 of 300 772 / 760)
+        const bool few_bytes = rows * ix->code_size <= (ix->dim <= GROUPED_TC_DIMS ? 8e8 : 1e9);
+        const bool pruned = ix->prune_lists && 8.0 * (kscan + SQ8_SLACK) <= mean_len && ix->dim <= GROUPED_TC_DIMS;
+        return few_bytes && !(pruned && rows > GROUPED_PAIR_ROWS) ? SCAN_PAIRS : SCAN_GROUPED;
     }
     return SCAN_PAIRS;
 }
