@@ -118,3 +118,25 @@ def test_results_do_not_depend_on_the_scan(engine, n, nprobe, nq, k):
         got = ix.search(q, k, nprobe)
         assert np.array_equal(got[1], want[1])
         assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)
+
+
+def test_batches_beyond_the_score_buffer(engine):
+    """Scores for 2^28 (query, row) places at once: larger batches go in slices, whose results, scan time and scanned bytes
+    belong together."""
+    n, dim, nlist, k = 200_000, 32, 64, 7
+    x, q = mixture(3, n, dim, nlist, 0.2), mixture(4, 1500, dim, nlist, 0.2)
+    ix = engine.IvfHandle(dim, 0, nlist, engine.QUANT_FP32)
+    ix.train(x[:20_000], iters=2)
+    ix.add(x, np.arange(n, dtype=np.int64))
+    one, one_ms = ix.search(q[:1200].copy(), k, nlist), ix.last_scan_ms()      # below: one slice
+    one_bytes = ix.last_scanned_bytes()
+    got = ix.search(q, k, nlist)
+    assert np.array_equal(got[1][:1200], one[1]) and np.array_equal(got[0][:1200], one[0])
+    rest = ix.search(q[1200:].copy(), k, nlist)
+    assert np.array_equal(got[1][1200:], rest[1]) and np.array_equal(got[0][1200:], rest[0])
+    both = []
+    for _ in range(3):
+        ix.search(q, k, nlist)
+        both.append(ix.last_scan_ms())
+    assert ix.last_scanned_bytes() * 1200 == one_bytes * 1500
+    assert min(both) > 0.9 * min(one_ms, *(ix.search(q[:1200].copy(), k, nlist) and ix.last_scan_ms() for _ in range(3)))

@@ -184,6 +184,7 @@ struct vb200_ivf {
     int64_t last_scan_bytes = 0;
     cudaEvent_t ev_scan_begin = nullptr, ev_scan_end = nullptr;  // bracket the list-scan kernel
     bool scan_timed = false;
+    float scan_ms_before = 0.f;  // scan time of the last search's slices before the one the events belong to
 
     ~vb200_ivf() {
         if (ev_scan_begin != nullptr) {
@@ -2861,6 +2862,7 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
                   tc_scan ? ws.qw8.ptr : nullptr, tc_scan ? ws.qscale.ptr : nullptr);
     }
     VB_CUDA(cudaEventRecord(ix->ev_scan_begin, st));
+    ix->scan_ms_before = 0.f;
     g_scan_profile.mark(st);   // prep
     auto launch_phases = [&](uint32_t first, uint32_t count, uint32_t queue_slot, bool on_tensor_cores,
                              bool warp_items = false) -> int {
@@ -3370,13 +3372,20 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     slice = slice < 1 ? 1 : (slice > nq ? nq : slice);
     if (plan != nullptr && slice < nq) {
         int64_t bytes = 0;
+        float scan_ms = 0.f;
         const uint64_t parts = (nq + slice - 1) / slice, each = (nq + parts - 1) / parts;
         for (uint64_t q0 = 0; q0 < nq && !*repeats; q0 += each) {
+            if (q0 > 0) {   // (the slice before has completed)
+                float ms = 0.f;
+                VB_CUDA(cudaEventElapsedTime(&ms, ix->ev_scan_begin, ix->ev_scan_end));
+                scan_ms += ms;
+            }
             VB_TRY(ivf_search_scores(ix, queries + q0 * dim, std::min(each, nq - q0), k, kscan, nprobe, rerank, plan,
                                      bucket_ids != nullptr ? bucket_ids + q0 * nprobe : nullptr, ids + q0 * k, dists + q0 * k, repeats));
             bytes += ix->last_scan_bytes;
         }
         ix->last_scan_bytes = ix->last_scanned_bytes = bytes;
+        ix->scan_ms_before = scan_ms;
         return 0;
     }
     // host buffers: [queries | ids | dists] in pinned memory when small
@@ -3603,6 +3612,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         g.dists = dists_dev + q0 * k;
         if (q0 == 0) {
             VB_CUDA(cudaEventRecord(ix->ev_scan_begin, st));
+            ix->scan_ms_before = 0.f;
         }
         if (plan != nullptr) {
             VB_TRY(launch_tiles(ix, g.scan, nq, *plan));
@@ -4778,6 +4788,7 @@ vb200_ivf_last_scan_ms(vb200_ivf_t ix, float* ms) {
     }
     VB_CUDA(cudaEventSynchronize(ix->ev_scan_end));
     VB_CUDA(cudaEventElapsedTime(ms, ix->ev_scan_begin, ix->ev_scan_end));
+    *ms += ix->scan_ms_before;
     return 0;
 }
 
