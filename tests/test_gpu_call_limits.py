@@ -46,3 +46,19 @@ def test_more_one_bit_queries_than_a_launch_has_tiles(engine, oracle):
         assert np.array_equal(dists[at:at + 1000], want[1]) and np.array_equal(ids[at:at + 1000], want[0])
     tail = nq % 1000
     assert np.array_equal(dists[nq - tail:], want[1][:tail]) and np.array_equal(ids[nq - tail:], want[0][:tail])
+
+
+@pytest.mark.parametrize("quant", ["QUANT_FP32", "QUANT_SQ8"])
+def test_more_lists_than_the_finalising_kernel_has_room_for(engine, quant):
+    """A caller may name as many lists as there are; two words each of shared memory are too much from 23,000 on."""
+    n, dim, nlist, k = 30_000, 4, 24_000, 5
+    x, q = mixture(1, n, dim, 50, 0.3), mixture(2, 3, dim, 50, 0.3)
+    ix = engine.IvfHandle(dim, 0, nlist, getattr(engine, quant))
+    ix.set_centroids(x[:nlist])
+    if quant == "QUANT_SQ8":
+        ix.set_sq8_model(x.min(axis=0), x.max(axis=0) - x.min(axis=0))
+    ix.add(x, np.arange(n, dtype=np.int64))
+    lists = np.tile(np.arange(nlist, dtype=np.int32), (3, 1))
+    ids, dists = ix.search(q, k, nlist, bucket_ids=lists)
+    some = ix.search(q, k, 900)         # the nearest of them hold the results
+    assert np.array_equal(dists, some[1]) and np.array_equal(ids, some[0])

@@ -3161,6 +3161,19 @@ ivf_search_keys(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, ui
 constexpr size_t PINNED_IO_BYTES = 256 * 1024;
 constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which tiles pay (3.1: 141 us as pairs, 162 as tiles)
 
+// Shared memory of pair_scan_kernel and of scan_finalize_kernel; qstride: floats of a query as the codec's chain reads it (the
+// latter: 0 without tiles).
+static size_t
+score_scan_smem(const vb200_ivf* ix, uint32_t qstride) {
+    return RS_STAGES * RS_STAGE + (ix->quant == VB200_QUANT_SQ8 ? 3 * static_cast<size_t>(ix->dpad) : qstride * sizeof(float));
+}
+
+static size_t
+score_final_smem(const vb200_ivf* ix, uint32_t nprobe, uint32_t qstride) {
+    const size_t query = ix->quant == VB200_QUANT_SQ8 ? (ix->dim + 3) / 4 * 4 + 2 * static_cast<size_t>(ix->dim) : qstride;
+    return (2 * static_cast<size_t>(nprobe) + 4 + query) * sizeof(float);
+}
+
 // How a batch is scanned into scores (ivf_pairs.cuh, ivf_tiles.cuh): not at all, pair by pair, or as tiles.
 enum ScoreScan { SCAN_GROUPED = 0, SCAN_PAIRS = 1, SCAN_TILES = 2 };
 
@@ -3245,6 +3258,10 @@ ivf_score_scan(const vb200_ivf* ix, uint64_t nq, uint32_t kscan, uint32_t nprobe
     }
     if (kscan + SQ8_SLACK > 1024 - SCAN_THREADS) {
         return SCAN_GROUPED;   // (the scan depth limit of the grouped path, which reports it)
+    }
+    const uint32_t qstride = (ix->dim + 127) / 128 * 128;
+    if (score_scan_smem(ix, qstride) > 220 * 1024 || score_final_smem(ix, nprobe, qstride) > 180 * 1024) {
+        return SCAN_GROUPED;   // (more than 20,000 lists named by the caller, very long rows)
     }
     const bool sq8 = ix->quant == VB200_QUANT_SQ8;
     const double per_list = static_cast<double>(nq) * nprobe / ix->nlist;
@@ -3562,10 +3579,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     int64_t* ids_dev = !host_ids ? ids : (pin_out ? reinterpret_cast<int64_t*>(pin + ids_at) : ws.out_ids.ptr);
     float* dists_dev = !host_d ? dists : (pin_out ? reinterpret_cast<float*>(pin + dists_at) : ws.out_dists.ptr);
 
-    const size_t scan_smem = RS_STAGES * RS_STAGE + (sq8 ? 3 * static_cast<size_t>(ix->dpad) : f.scan.qstride * sizeof(float));
-    const size_t final_smem = (2 * static_cast<size_t>(nprobe) + 4 + (sq8 ? (dim + 3) / 4 * 4 : 0) +
-                               (sq8 ? 2 * dim : (plan != nullptr ? f.scan.qstride : 0))) * sizeof(float);
-    VB_CHECK_ARG(scan_smem <= 220 * 1024 && final_smem <= 180 * 1024, "dim = %u is too large for the scan", dim);
+    const size_t scan_smem = score_scan_smem(ix, f.scan.qstride), final_smem = score_final_smem(ix, nprobe, plan != nullptr ? f.scan.qstride : 0);
     void (*scan_kernel)(const PairScan) = nullptr;
     void (*final_kernel)(const ScanFinalize) = nullptr;
 #define VB_FINAL(FMT, APPROX) (l2 ? scan_finalize_kernel<FMT, true, APPROX> : scan_finalize_kernel<FMT, false, APPROX>)
