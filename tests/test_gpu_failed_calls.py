@@ -1,4 +1,5 @@
-"""A call that ends with an error leaves the handle usable: the next search returns what a fresh handle returns."""
+"""A call that ends with an error leaves the handle usable: the next search returns what a fresh handle returns.  Handles
+outlive the streams they were used on, and searches make do with the memory there is."""
 from __future__ import annotations
 
 import ctypes as C
@@ -42,3 +43,35 @@ def test_search_after_a_filter_that_cannot_be_staged(engine, oracle, quant, reor
             assert status != 0
         got = ix.search(q, k, nprobe)
         assert np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])
+
+
+def test_a_handle_outlives_its_stream(engine):
+    """Streams are the caller's: one may be destroyed before the index that was searched on it, while it is still the
+    thread's current one."""
+    from vsag_b200 import _capi
+
+    _capi.load()
+    rt = C.CDLL("libcudart.so.12")          # the runtime that the library is linked with
+    x = mixture(1, 3000, 24, 6, 0.3)
+    ids = np.arange(len(x), dtype=np.int64)
+    for round_ in range(3):
+        stream = C.c_void_p()
+        assert rt.cudaStreamCreate(C.byref(stream)) == 0
+        engine.set_stream(stream.value)
+        try:
+            ix = engine.IvfHandle(24, 0, 6, engine.QUANT_SQ8)
+            ix.train(x, iters=2)
+            ix.add(x, ids)
+            bf = engine.BfHandle(24, 0)
+            bf.add(x, ids)
+            got, want = ix.search(x[:20].copy(), 3, 6), bf.search(x[:20].copy(), 3)
+            assert np.mean(got[0][:, 0] == want[0][:, 0]) > 0.8
+            assert rt.cudaStreamDestroy(stream) == 0
+            ix.close()
+            bf.close()
+            assert _capi.load().vb200_release_workspaces() == 0
+        finally:
+            engine.set_stream(None)
+    again = engine.BfHandle(24, 0)
+    again.add(x, ids)
+    assert np.array_equal(again.search(x[:20].copy(), 3)[0], want[0])

@@ -312,6 +312,10 @@ vb200_bf_create(uint32_t dim, int metric, int quant, vb200_bf_t* out) {
 
 extern "C" int
 vb200_bf_destroy(vb200_bf_t ix) {
+    if (ix == nullptr) {
+        return 0;
+    }
+    ReleaseScope scope;
     delete ix;
     return 0;
 }

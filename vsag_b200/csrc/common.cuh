@@ -88,6 +88,19 @@ int allow_dynamic_smem(const void* kernel, size_t bytes);
 // Device memory comes from a pool of the library (dense.cu): freeing a buffer costs no device-wide synchronisation and
 // the next one of its size no trip to the driver.  Both are ordered with the calling thread's current stream: a call
 // uses one stream and has completed when it returns, so a buffer is never still in use on another.
+// Memory that outlives a call -- a handle, the kept workspaces -- is freed inside a ReleaseScope: the thread's stream may be
+// gone by then, or not be the one that the memory was used on.  The scope waits for the device and stands for the default
+// stream.
+struct ReleaseScope {
+    ReleaseScope();
+    ~ReleaseScope();
+    ReleaseScope(const ReleaseScope&) = delete;
+    ReleaseScope& operator=(const ReleaseScope&) = delete;
+
+private:
+    cudaStream_t before_;
+};
+
 cudaError_t pool_malloc(void** p, size_t bytes);
 void pool_free(void* p);
 void pool_trim();

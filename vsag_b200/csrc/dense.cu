@@ -158,6 +158,17 @@ pool_free(void* p) {
     }
 }
 
+ReleaseScope::ReleaseScope() : before_(tl_stream) {
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+    }
+    tl_stream = nullptr;
+}
+
+ReleaseScope::~ReleaseScope() {
+    tl_stream = before_;
+}
+
 void
 pool_trim() {
     cudaMemPool_t pool = device_pool();

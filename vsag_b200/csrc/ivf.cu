@@ -3813,6 +3813,10 @@ vb200_ivf_create(uint32_t dim, int metric, uint32_t nlist, int quant, int use_re
 
 extern "C" int
 vb200_ivf_destroy(vb200_ivf_t ix) {
+    if (ix == nullptr) {
+        return 0;
+    }
+    ReleaseScope scope;
     delete ix;
     return 0;
 }

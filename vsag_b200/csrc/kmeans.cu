@@ -781,6 +781,7 @@ private:
 extern "C" int
 vb200_release_workspaces(void) {
     std::lock_guard<std::mutex> lock(g_kmeans_ws_mu);
+    ReleaseScope scope;
     delete g_kmeans_ws;
     g_kmeans_ws = nullptr;
     (void)sync_stream();   // what was freed is free now
