@@ -4175,7 +4175,7 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
                  DevBuf<uint32_t>& new_off_dev, const std::vector<uint32_t>& new_off, uint64_t n_new_stored,
                  uint64_t n_total_new) {
     const uint32_t nlist = ix->nlist, dim = ix->dim, stride = ix->code_stride;
-    DevBuf<float> new_norm;
+    DevBuf<float> new_norm, new_max;
     if (ix->quant == VB200_QUANT_SQ8 && n_new_stored > 0) {
         VB_TRY(new_norm.reserve(n_new_stored));
         VB_LAUNCH(sq8_code_norm_kernel, static_cast<uint32_t>((n_new_stored + 127) / 128), 128, 0,
@@ -4188,14 +4188,14 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
         }
     }
     if (n_new_stored > 0 && ix->quant != VB200_QUANT_SQ8_UNIFORM) {
-        VB_TRY(ix->row_max.reserve(2));
-        VB_CUDA(cudaMemsetAsync(ix->row_max.ptr, 0, 2 * sizeof(float), current_stream()));
+        VB_TRY(new_max.reserve(2));
+        VB_CUDA(cudaMemsetAsync(new_max.ptr, 0, 2 * sizeof(float), current_stream()));
         const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>((n_new_stored + 7) / 8, 16ull * sm_count()));
         if (ix->quant != VB200_QUANT_SQ8) {
             VB_TRY(new_norm.reserve(n_new_stored * (ix->quant == VB200_QUANT_RABITQ ? 2 : 1)));
         }
         const uint8_t* codes = new_codes.ptr;
-        float *norm = new_norm.ptr, *top = ix->row_max.ptr;
+        float *norm = new_norm.ptr, *top = new_max.ptr;
         switch (ix->quant) {
             case VB200_QUANT_FP32: VB_LAUNCH(record_norms_kernel<ROW_F32>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
             case VB200_QUANT_BF16: VB_LAUNCH(record_norms_kernel<ROW_BF16>, blocks, 256, 0, codes, n_new_stored, dim, stride, norm, top); break;
@@ -4250,6 +4250,7 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
     ix->codes_t = std::move(new_tiled);
     ix->group_off = std::move(new_group_off);
     ix->code_norm = std::move(new_norm);
+    ix->row_max = std::move(new_max);
     ix->codes = std::move(new_codes);
     ix->pos_inner = std::move(new_inner);
     ix->list_off = std::move(new_off_dev);
