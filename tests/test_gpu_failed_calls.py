@@ -75,3 +75,65 @@ def test_a_handle_outlives_its_stream(engine):
     again = engine.BfHandle(24, 0)
     again.add(x, ids)
     assert np.array_equal(again.search(x[:20].copy(), 3)[0], want[0])
+
+
+class LittleMemory:
+    """All but `left` bytes of device memory taken while in scope, the library's own reserve given back first."""
+
+    def __init__(self, left):
+        self.left = left
+
+    def __enter__(self):
+        import torch
+
+        from vsag_b200 import _capi
+
+        _capi.load().vb200_release_workspaces()
+        torch.cuda.empty_cache()
+        self.taken = []
+        for _ in range(3):     # (the last step may be rounded up)
+            free = torch.cuda.mem_get_info()[0] - self.left
+            if free > (8 << 20):
+                self.taken.append(torch.empty(free >> 21 << 21, dtype=torch.uint8, device="cuda"))
+        assert torch.cuda.mem_get_info()[0] <= self.left + (16 << 20)
+
+    def __exit__(self, *exc):
+        import torch
+
+        self.taken = None
+        torch.cuda.empty_cache()
+
+
+def test_a_batch_whose_scores_do_not_fit(engine):
+    """200,000 rows for each of 1000 queries are 800 MB of scores; the grouped scan needs a few MB."""
+    n, dim, nlist, nq, k = 200_000, 32, 64, 1000, 5
+    x, q = mixture(3, n, dim, nlist, 0.2), mixture(4, nq, dim, nlist, 0.2)
+    ix = engine.IvfHandle(dim, 0, nlist, engine.QUANT_FP32)
+    ix.train(x[:20_000], iters=2)
+    ix.add(x, np.arange(n, dtype=np.int64))
+    want = ix.search_ex(q, k, nlist, timeout_ms=1e9)
+    with LittleMemory(400 << 20):
+        got = ix.search(q, k, nlist)
+    assert np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])
+    again = ix.search(q, k, nlist)
+    assert np.array_equal(again[1], want[1]) and np.array_equal(again[0], want[0])
+
+
+def test_exact_search_without_room_for_a_second_copy(engine):
+    """A batch of ten over rows of 400 MB, whose tiled copy is as large again."""
+    import torch
+
+    n, dim, nq, k = 1_600_000, 64, 10, 4
+    g = torch.Generator(device="cuda").manual_seed(1)
+    base = torch.rand((n, dim), generator=g, device="cuda")
+    q = base[1000:1000 + nq].cpu().numpy() + np.float32(0.01)
+    ix = engine.BfHandle(dim, 0)
+    ix.add(base, torch.arange(n, dtype=torch.int64, device="cuda"))
+    del base
+    want = [ix.search(q[i:i + 1].copy(), k) for i in range(nq)]
+    with LittleMemory(300 << 20):
+        got = ix.search(q, k)
+    for _ in range(2):
+        assert np.array_equal(got[1], np.concatenate([w[1] for w in want]))
+        assert np.array_equal(got[0], np.concatenate([w[0] for w in want]))
+        got = ix.search(q, k)

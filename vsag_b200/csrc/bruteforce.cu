@@ -893,7 +893,8 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
     const bool k_fits = std::min<uint64_t>(k + BF_SLACK, ix->n) <= 1024;
     // (rows too long for a stream's shared memory, above 40,000 dimensions, are left to the slab of scores)
     const bool streams = k_fits && bf_stream_smem(ix->dim, bf_stream_cap(static_cast<uint32_t>(std::min<uint64_t>(k, ix->n))), 1) <= 220 * 1024;
-    const bool scores = tensor_cores_enabled() && streams && nq > BF_STREAM_QUERIES && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES;
+    const bool few = nq <= BF_STREAM_QUERIES && streams;
+    bool scores = tensor_cores_enabled() && streams && !few && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES;
     BfStaged staged;
     bool keyed = false;
     int rc = 0;
@@ -901,7 +902,7 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
     // Up to eight queries share one pass over the rows; more go to the tensor cores -- through a score matrix
     // while that is cheaper than selecting as the scores appear (measured: up to about 4e8 scores), see
     // bf_search_keys for the rest.
-    if (nq <= BF_STREAM_QUERIES && streams) {
+    if (few) {
         rc = bf_stage(ix, queries, nq, &staged.queries, &staged.bias, &staged.masked);
         if (rc == 0) {
             rc = bf_stream_queries(ix, staged, nq, nullptr, k, ids_dev, dists_dev);
@@ -911,7 +912,18 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
         if (rc == 0) {
             rc = bf_search_scores(ix, staged, nq, k, ids_dev, dists_dev);
         }
-    } else {
+        if (rc == VB200_NO_ENOUGH_MEMORY) {
+            // the tiled copy of the rows did not fit beside them: the slab of scores needs none
+            (void)cudaStreamSynchronize(current_stream());
+            scores = false;
+            if (!ix->tiled_valid) {
+                ix->base_hi.release();
+                ix->base_lo.release();
+            }
+            ix->scores.release();
+        }
+    }
+    if (!few && !scores) {
         rc = bf_search_keys(ix, queries, nq, k);
         keyed = true;
     }

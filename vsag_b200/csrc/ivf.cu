@@ -4575,10 +4575,15 @@ vb200_ivf_get_lists(vb200_ivf_t ix, int64_t* list_sizes, uint8_t* codes, int64_t
         VB_TRY(copy_rows_to_host(codes, ix->codes.ptr, ix->code_size, ix->code_stride, ix->n_stored));
     }
     if (inner_ids != nullptr) {
+        // (a piece at a time: an index may have left no room for 8 bytes a row)
+        constexpr uint64_t PIECE = uint64_t{1} << 22;
         DevBuf<int64_t> wide;
-        VB_TRY(wide.reserve(ix->n_stored));
-        VB_LAUNCH(widen_ids_kernel, static_cast<uint32_t>((ix->n_stored + 255) / 256), 256, 0, ix->pos_inner.ptr, ix->n_stored, wide.ptr);
-        VB_TRY(copy_to_host(inner_ids, wide.ptr, ix->n_stored * sizeof(int64_t)));
+        VB_TRY(wide.reserve(std::min(PIECE, ix->n_stored)));
+        for (uint64_t at = 0; at < ix->n_stored; at += PIECE) {
+            const uint64_t m = std::min(PIECE, ix->n_stored - at);
+            VB_LAUNCH(widen_ids_kernel, static_cast<uint32_t>((m + 255) / 256), 256, 0, ix->pos_inner.ptr + at, m, wide.ptr);
+            VB_TRY(copy_to_host(inner_ids + at, wide.ptr, m * sizeof(int64_t)));
+        }
     }
     return 0;
 }
@@ -4699,7 +4704,11 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
                 if (rc != 0) {
                     (void)cudaStreamSynchronize(current_stream());   // what was launched may use the workspace
                 }
-                if (rc != 0 || !repeats) {
+                if (rc == VB200_NO_ENOUGH_MEMORY) {
+                    // up to a gigabyte of scores did not fit: the grouped scan keeps the k best of each pair instead
+                    ws.pair_scores.release();
+                    ws.pair_minima.release();
+                } else if (rc != 0 || !repeats) {
                     return rc;
                 }
             }
