@@ -690,7 +690,7 @@ def run_kmeans(args, ctx: Ctx, steps: int, warmup: int) -> dict:
     line = {
         "metric": "k-means Lloyd iterations, 1M x 128 rows against 4,096 centroids", "value": world * n / (ms / 1e3),
         "unit": "rows assigned/s", "n_gpus": world, "steps": steps, "warmup": warmup, "ms_per_step": ms,
-        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "bf16x3 (split fp32), fp32 accumulate",
+        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "fp16 nomination, fp32 exact decision",
         "data": "synthetic",
         "config": {"workload": "k-means training: one step = one Lloyd iteration (assignment + centroid update)",
                    "rows": n, "dim": dim, "centroids": k, "init": "first rows",
@@ -703,7 +703,7 @@ def run_kmeans(args, ctx: Ctx, steps: int, warmup: int) -> dict:
                      "peak": peak, "unit": "TFLOP/s", "frac": flops / (ms / 1e3) / 1e12 / peak, "peak_source": peak_kind,
                      "traffic": None,
                      "note": "achieved = 2*rows*centroids*dim per iteration over the whole iteration's time; the kernel "
-                             "issues three bf16 MMAs per product (hi*hi, hi*lo, lo*hi)"},
+                             "issues one fp16 MMA per product to nominate centroids, close ones are decided by exact fp32 chains"},
     }
     if rank == 0 and not env_int("VB200_BENCH_SKIP_EXTRAS", 0):
         # parity, iteration by iteration: the labels of a row sample against the oracle's assignment to
@@ -925,12 +925,12 @@ def run_rabitq(args, ctx: Ctx, steps: int, warmup: int) -> dict:
         "e2e": {"value": nq / (e2e_ms / 1e3), "unit": "queries/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": nq * dim * 4, "d2h_bytes_per_step": nq * k * 12},
         "gpu_launches": int(launches), "clocks": clocks,
-        "roofline": {"bound": "hbm", "kernel": "ivf_rabitq_scan_kernel", "achieved": lg / (k_ms / 1e3) / 1e9, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "tile_scan_kernel<RaBitQ>", "achieved": lg / (k_ms / 1e3) / 1e9, "peak": peak,
                      "unit": "GB/s", "frac": lg / (k_ms / 1e3) / 1e9 / peak, "peak_source": ctx.peaks["hbm_kind"],
                      "kernel_ms": k_ms, "traffic": None, "algorithmic_bytes": lg,
                      "step_bytes": lg + rerank_bytes, "step_frac": (lg + rerank_bytes) / (ms / 1e3) / 1e9 / peak,
-                     "note": "achieved = probed list lengths x 128 B per query tile / scan kernel time (a list probed by "
-                             "several tiles is an L2 hit after the first); step_* adds the rerank's 400 fp32 rows per query "
+                     "note": "achieved = probed list lengths x 128 B per query / scan time: logical bytes, which a tile reads once "
+                             "for up to 64 queries, so the fraction passes 1; step_* adds the rerank's 400 fp32 rows per query "
                              "over the whole step"},
     }
     if not env_int("VB200_BENCH_SKIP_EXTRAS", 0):

@@ -77,7 +77,8 @@ typedef struct vb200_comm* vb200_comm_t;
 VB200_API int vb200_last_error(char* buf, size_t buf_len);
 
 /* vb200_kmeans_train keeps its device workspace between calls (allocating it costs more than the iterations it
- * serves); this frees it.  Indexes own their workspaces and free them with the handle. */
+ * serves), and freed device memory stays in a pool of the library, up to 2 GiB per device; this gives both back to
+ * the driver (the pool of the current device).  Indexes own their workspaces and free them with the handle. */
 VB200_API int vb200_release_workspaces(void);
 
 /* CUDA stream (a cudaStream_t) the calling thread's subsequent calls launch on; NULL = the
@@ -291,7 +292,7 @@ VB200_API int vb200_ivf_get_rows(vb200_ivf_t index, float* rows);
  * src/impl/reorder/flatten_reorder.cpp:76-118).  ids[nq x k] user labels (-1 pad),
  * dists[nq x k] ascending (+inf pad).
  * bucket_ids (optional, [nq x nprobe], -1 = skip) bypasses routing like
- * SearchRequest::bucket_ids_ (include/vsag/search_request.h:227). */
+ * SearchRequest::bucket_ids_ (include/vsag/search_request.h:227); a list named twice for a query is scanned twice. */
 VB200_API int vb200_ivf_search(vb200_ivf_t index, const float* queries, uint64_t nq, uint32_t k,
                      uint32_t nprobe, float factor, const int32_t* bucket_ids, int64_t* ids,
                      float* dists);
@@ -372,8 +373,8 @@ VB200_API int64_t vb200_ivf_last_scanned_bytes(vb200_ivf_t index);
 /* Turns that list pruning off (0) or on (non-zero, the default); for cross-checks. */
 VB200_API int vb200_ivf_set_list_pruning(vb200_ivf_t index, int enable);
 
-/* Device time of the last search's list-scan kernel in milliseconds, from CUDA events recorded
- * around its launch on the stream it ran on. */
+/* Device time of the last search's list scan in milliseconds, from CUDA events recorded around it on the stream it
+ * ran on (the sum over the slices of a batch that was cut). */
 VB200_API int vb200_ivf_last_scan_ms(vb200_ivf_t index, float* ms);
 
 /* Merges `parts` partial results laid out [parts][nq][k] (as gathered from the ranks) into

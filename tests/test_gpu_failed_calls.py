@@ -120,10 +120,10 @@ def test_a_batch_whose_scores_do_not_fit(engine):
 
 
 def test_exact_search_without_room_for_a_second_copy(engine):
-    """A batch of ten over rows of 400 MB, whose tiled copy is as large again."""
+    """A batch of ten over rows of 563 MB (beyond the pool's largest block), whose tiled copy is as large again."""
     import torch
 
-    n, dim, nq, k = 1_600_000, 64, 10, 4
+    n, dim, nq, k = 2_200_000, 64, 10, 4
     g = torch.Generator(device="cuda").manual_seed(1)
     base = torch.rand((n, dim), generator=g, device="cuda")
     q = base[1000:1000 + nq].cpu().numpy() + np.float32(0.01)

@@ -18,8 +18,8 @@ constexpr uint32_t SELECT_GROUPS = 1024;          // group minima kept at most
 constexpr uint32_t SELECT_CAP = 2048;             // values collected at most
 
 struct SelectScratch {
-    uint32_t hist[SELECT_BINS];       // also the group minima's home: the two are never needed together
-    uint32_t minima[SELECT_GROUPS];
+    uint32_t hist[SELECT_BINS];
+    uint32_t minima[SELECT_GROUPS];   // per group; the second pass reads them again
     uint32_t warp_part[32];
     uint32_t lo, hi, total, pick, upto, before, count;
 };
