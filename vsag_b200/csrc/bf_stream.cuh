@@ -142,6 +142,12 @@ struct BfMargin {
     float chain, matrix;
     uint32_t* unsure;       // [0] = number of queries whose nominations may not be enough, then their numbers
     uint32_t q_base;        // number of the launch's first query
+    __device__ __forceinline__ float
+    of(bool l2, float top, float qq, float kth) const {
+        const float size = top * sqrtf(qq);
+        const float margin = l2 ? fmaf(chain, top * top + qq + kth, 2.0f * matrix * size) : fmaf(chain + matrix, size, 3e-7f);
+        return margin + 1e-30f;   // (products below the smallest normal number round absolutely)
+    }
 };
 
 // One CTA per query: the kcand best of its row of `n` nominating scores, re-scored in the reference's operation
@@ -167,10 +173,10 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
         qf[d] = widen(queries[q * dim + d]);
     }
     const ScoreSource<true> src{reinterpret_cast<const uint32_t*>(scores + q * ld)};
-    const uint32_t found = block_select<T>(src, [](uint32_t i) { return i; }, n, kcand, keys, sel);
-    block_sort_to<T>(keys, found, kcand, best);
-    const uint32_t have = min(found, kcand);
-    const float last = have > 0 ? ordered_to_float(static_cast<uint32_t>(best[have - 1] >> 32)) : 0.f;
+    uint32_t left;   // no score that was not collected is below it
+    const uint32_t have = block_select<T>(src, [](uint32_t i) { return i; }, n, kcand, keys, sel, &left);
+    const bool dropped = left < ORDERED_INF;
+    const float last = dropped ? ordered_to_float(left) : 0.f;
     if (threadIdx.x / 32 == T / 32 - 1) {   // (while the first warps wait for the candidates' rows)
         const float top = __ldg(m.row_max);
         float qq = 0.f;
@@ -184,7 +190,7 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
         s_top = top;
     }
     for (uint32_t i = threadIdx.x; i < have; i += T) {
-        const uint32_t row = static_cast<uint32_t>(best[i]);
+        const uint32_t row = static_cast<uint32_t>(keys[i]);
         keys[i] = make_key(row_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, metric == VB200_METRIC_L2), row);
     }
     block_sort_to<T>(keys, have, k, best);
@@ -195,11 +201,8 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
     }
     if (threadIdx.x == 0) {
         const bool l2 = metric == VB200_METRIC_L2;
-        const bool dropped = n > kcand && found >= kcand;   // (then kcand > k)
         const float kth = dropped ? ordered_to_float(static_cast<uint32_t>(best[k - 1] >> 32)) : 0.f;
-        const float top = s_top, qq = s_qq, size = top * sqrtf(qq);
-        float margin = l2 ? fmaf(m.chain, top * top + qq + kth, 2.0f * m.matrix * size) : fmaf(m.chain + m.matrix, size, 3e-7f);
-        margin += 1e-30f;   // (products below the smallest normal number round absolutely)
+        const float qq = s_qq, margin = m.of(l2, s_top, qq, kth);
         // not finite: scores may have overflowed, and rows with them are not even among the counted
         if (!(margin < INFINITY) || (dropped && !(kth < last + (l2 ? qq : 1.0f) - margin))) {
             m.unsure[1 + atomicAdd(m.unsure, 1u)] = m.q_base + static_cast<uint32_t>(q);

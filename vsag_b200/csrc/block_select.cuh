@@ -16,6 +16,7 @@ constexpr uint32_t ORDERED_INF = 0xFF800000u;     // float_to_ordered(+inf): lar
 constexpr uint32_t SELECT_BINS = 1024;
 constexpr uint32_t SELECT_GROUPS = 1024;          // group minima kept at most
 constexpr uint32_t SELECT_CAP = 2048;             // values collected at most
+constexpr uint32_t SELECT_RANKED = 256;           // keys sorted by counting, at most
 
 struct SelectScratch {
     uint32_t hist[SELECT_BINS];
@@ -211,10 +212,12 @@ block_bound(const Source& src, uint32_t n, uint32_t k, uint32_t cap, SelectScrat
 // The k smallest of the n values (ties: smallest payload first) among a few more, unsorted, as
 // (value << 32 | payload(i)) in keys[SELECT_CAP]; returns how many were collected (>= k when that many take
 // part, <= SELECT_CAP).  k <= 1024.  Every value is read once, and
-// the groups of the smallest ones again.
+// the groups of the smallest ones again.  *least_left (optional): no value that was not collected is below it; ORDERED_INF: every
+// value that takes part was collected.
 template <int T, typename Source, typename Payload>
 __device__ uint32_t
-block_select(const Source& src, const Payload& payload, uint32_t n, uint32_t k, uint64_t* keys, SelectScratch& s) {
+block_select(const Source& src, const Payload& payload, uint32_t n, uint32_t k, uint64_t* keys, SelectScratch& s,
+             uint32_t* least_left = nullptr) {
     uint32_t bound = ORDERED_INF;
     bool counted = false;
     uint32_t grouped = 0;   // how many groups have their minimum in s.minima
@@ -271,11 +274,17 @@ block_select(const Source& src, const Payload& payload, uint32_t n, uint32_t k, 
         return s.count;
     };
     uint32_t count = collect(bound, false);
+    if (least_left != nullptr) {
+        *least_left = bound;
+    }
     if (count <= SELECT_CAP || counted) {
         return count;
     }
     uint32_t upto;
     bound = block_bound<T>(src, n, k, SELECT_CAP, s, &upto);
+    if (least_left != nullptr) {
+        *least_left = bound;
+    }
     if (upto <= SELECT_CAP) {
         return collect(bound, false);
     }
@@ -299,14 +308,15 @@ block_select(const Source& src, const Payload& payload, uint32_t n, uint32_t k, 
     return min(s.count, SELECT_CAP);
 }
 
-// Sorts `count` distinct keys and leaves the `keep` smallest, ascending, in out (a different buffer).  Up to 512
+// Sorts `count` distinct keys and leaves the `keep` smallest, ascending, in out (a different buffer).  Up to 256
 // keys every thread counts how many are smaller than its own, one pass and one barrier instead of a sorting
-// network's many; more go through the network (keys must then have room for the next power of two).
+// network's many; more go through the network, whose instructions grow more slowly (464 keys: 27,000 a warp's share against
+// 4,300; keys must then have room for the next power of two).
 template <int T>
 __device__ __forceinline__ void
 block_sort_to(uint64_t* keys, uint32_t count, uint32_t keep, uint64_t* out) {
     __syncthreads();
-    if (count <= 512) {
+    if (count <= SELECT_RANKED) {
         for (uint32_t i = threadIdx.x; i < count; i += T) {
             const uint64_t mine = keys[i];
             uint32_t rank = 0;

@@ -162,11 +162,10 @@ pairs_prepare_kernel(const PairsPrepare p) {
                 qs[d] = __ldg(p.queries + q * p.dim + d);
             }
             const ScoreSource<> src{reinterpret_cast<const uint32_t*>(p.scores + q * p.ld)};
+            // (what was collected, a few more than ncand, is scored as it is: ordering it first cost more)
             found = block_select<PAIR_THREADS>(src, [](uint32_t i) { return i; }, p.nlist, p.ncand, keys, sel);
-            block_sort_to<PAIR_THREADS>(keys, found, p.ncand, best);
-            found = min(found, p.ncand);
             for (uint32_t i = threadIdx.x; i < found; i += PAIR_THREADS) {
-                const uint32_t l = static_cast<uint32_t>(best[i]);
+                const uint32_t l = static_cast<uint32_t>(keys[i]);
                 keys[i] = make_key(row_exact_distance(p.centroids + static_cast<uint64_t>(l) * p.dim, qs, p.dim, p.metric == VB200_METRIC_L2), l);
             }
         } else {
@@ -680,7 +679,7 @@ scan_finalize_kernel(const ScanFinalize p) {
             return record_exact_distance<FMT, L2>(rec, dim, sc.row_bytes, qc, qn);
         }
     };
-    uint32_t found = 0;
+    uint32_t found = 0, left = ORDERED_INF;   // left: no score that was not collected is below it
     bool selected = false;
     if (APPROX && sc.t.minima != nullptr) {
         // First the groups of 32 scores that can hold one of the kcand best: those whose smallest is not above the
@@ -706,12 +705,14 @@ scan_finalize_kernel(const ScanFinalize p) {
             const auto at = [&](uint32_t i) -> uint32_t { return group_ids[i >> 5] * 32 + (i & 31u); };
             const GroupPosition where{group_ids, position};
             found = block_select<PAIR_THREADS>(load_source([&](uint32_t i) { return ScoreSource<>::ordered(__ldg(scores + at(i))); }), where,
-                                               m * 32, p.kcand, keys, sel);
+                                               m * 32, p.kcand, keys, sel, &left);
+            // (the other groups' scores are above `bound`)
+            left = groups > m ? min(left, bound) : left;
             selected = true;
         }
     }
     if (!selected) {
-        found = block_select<PAIR_THREADS>(ScoreSource<>{scores}, position, n, p.kcand, keys, sel);
+        found = block_select<PAIR_THREADS>(ScoreSource<>{scores}, position, n, p.kcand, keys, sel, &left);
     }
     if (p.rows_scanned != nullptr) {
         uint32_t rows = 0;
@@ -733,16 +734,16 @@ scan_finalize_kernel(const ScanFinalize p) {
         }
     }
     if (APPROX) {
-        block_sort_to<PAIR_THREADS>(keys, found, p.kcand, best);
-        const uint32_t kept = min(found, p.kcand);
-        const float last = kept > 0 ? ordered_to_float(static_cast<uint32_t>(best[kept - 1] >> 32)) : 0.f;
-        for (uint32_t i = threadIdx.x; i < kept; i += PAIR_THREADS) {
-            const uint32_t pos = static_cast<uint32_t>(best[i]);
+        // Everything that was collected is re-scored, kcand rows and a third more at most: ordering them by score first, to drop
+        // those, cost more than their distances.
+        const bool dropped = left < ORDERED_INF;   // (else every row with a score was collected)
+        const float last = dropped ? ordered_to_float(left) : 0.f;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < found; i += PAIR_THREADS) {
+            const uint32_t pos = static_cast<uint32_t>(keys[i]);
             keys[i] = make_key(exact(pos), pos);
         }
-        const bool dropped = found >= p.kcand;   // (else every row with a score is kept)
-        block_sort_to<PAIR_THREADS>(keys, kept, p.kscan, best);
-        found = kept;
+        block_sort_to<PAIR_THREADS>(keys, found, p.kscan, best);
         float margin, offset = 0.f;
         const float rows_max = __ldg(p.row_max);
         if constexpr (FMT == ROW_RABITQ) {
