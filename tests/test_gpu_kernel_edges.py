@@ -1,0 +1,70 @@
+"""Kernels at the edges of their tiles, pieces and buffers, and searches on both sides of the lines between their paths."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import assert_topk_equal, mixture
+
+pytestmark = pytest.mark.gpu
+
+
+def exactly(got, want):
+    assert np.array_equal(got[1], want[1])
+    assert_topk_equal(got[0], got[1], want[0], want[1], rtol=0, atol=0)
+
+
+# ---- exact batches that keep what passes a threshold from a sample of the rows --------------------------------
+# 4 (k + 16) minima of 32 rows in every eighth tile of 128: from 17,281 rows with k 1, 26,497 with k 10, 60,033 with k 42
+@pytest.mark.parametrize("quant,metric,n,dim,nq,k", [
+    ("fp32", 0, 17_280, 33, 9, 1),        # the most rows without a sample, rows of 4-byte alignment
+    ("fp32", 0, 17_281, 33, 9, 1),        # the fewest with one; the last tile of the rows holds one
+    ("fp32", 1, 26_497, 96, 129, 10),     # two row tiles of queries, six of eight k-steps
+    ("bf16", 0, 26_600, 50, 128, 10),
+    ("bf16", 1, 60_100, 200, 300, 42),
+    ("fp32", 0, 70_000, 16, 1000, 10),    # a sixteenth of the rows as a sample
+])
+@pytest.mark.parametrize("order", ["mixed", "sorted"])
+def test_exact_batches_by_threshold(engine, oracle, quant, metric, n, dim, nq, k, order):
+    base, q = mixture(21, n, dim, 40, 0.25), mixture(22, nq, dim, 40, 0.25)
+    if order == "sorted":      # rows of a cluster stored together: all that is nearest to a query lies in a few tiles
+        base = np.ascontiguousarray(base[np.lexsort(base.T[:3])])
+    ix = engine.BfHandle(dim, metric, engine.QUANT_FP32 if quant == "fp32" else engine.QUANT_BF16)
+    ix.add(base, np.arange(n, dtype=np.int64))
+    got = ix.search(q, k)
+    some = slice(0, 64)
+    if quant == "fp32":
+        want = oracle.bf_search_fp32(base, q[some], k, metric)
+    else:
+        want = oracle.bf_search_bf16(oracle.float_to_bf16(base), q[some], k, metric=metric)
+    exactly((got[0][some], got[1][some]), want)
+    gone = np.full((n + 31) // 32, 0x55555555, np.uint32)      # filtered rows take the path without a sample
+    left = np.flatnonzero(np.arange(n) % 2 == 1)
+    few = ix.search_filtered(q, k, deny_inner_bits=gone)
+    if quant == "fp32":
+        want = oracle.bf_search_fp32(base[left], q[some], k, metric)
+    else:
+        want = oracle.bf_search_bf16(oracle.float_to_bf16(base[left]), q[some], k, metric=metric)
+    exactly((few[0][some], few[1][some]), (np.where(want[0] >= 0, left[want[0]], -1), want[1]))
+
+
+@pytest.mark.parametrize("kind", ["equal", "far", "nan"])
+def test_exact_batches_the_threshold_does_not_serve(engine, oracle, kind):
+    """Every row within the scores' rounding of every other, many equal ones, rows that are no numbers: the results are those
+    of the exact pass."""
+    n, dim, nq, k = 30_000, 24, 20, 10
+    base, q = mixture(23, n, dim, 30, 0.2), mixture(24, nq, dim, 30, 0.2)
+    if kind == "equal":
+        base[5_000:25_000] = base[7]
+        q[:10] = base[7]
+    elif kind == "far":
+        base, q = (base * np.float32(0.01) + np.float32(80)), (q * np.float32(0.01) + np.float32(80))
+    else:
+        base[3::11] = np.nan
+    ix = engine.BfHandle(dim, 0, engine.QUANT_FP32)
+    ix.add(base, np.arange(n, dtype=np.int64))
+    got = ix.search(q, k)
+    one = [ix.search(q[i:i + 1].copy(), k) for i in range(nq)]      # a pass over the rows in the exact arithmetic
+    assert np.array_equal(got[1], np.concatenate([o[1] for o in one]))
+    if kind != "equal":
+        assert np.array_equal(got[0], np.concatenate([o[0] for o in one]))

@@ -210,4 +210,168 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
     }
 }
 
+// thr[q] = the next float above the kcand-th smallest of the query's n minima (+inf with fewer numbers among them).  A CTA per query.
+constexpr int BF_THRESHOLD_THREADS = 128;
+
+__global__ void __launch_bounds__(BF_THRESHOLD_THREADS)
+bf_threshold_kernel(const float* __restrict__ minima, uint32_t n, uint32_t kcand, float* __restrict__ thr) {
+    __shared__ SelectScratch sel;
+    const float* mine = minima + static_cast<uint64_t>(blockIdx.x) * n;
+    uint32_t upto;
+    const uint32_t bound = block_bound<BF_THRESHOLD_THREADS>(load_source([&](uint32_t i) { return float_to_ordered(__ldg(mine + i)); }), n, kcand,
+                                                             kcand + kcand / 8 + 8, sel, &upto);
+    if (threadIdx.x == 0) {
+        thr[blockIdx.x] = bound >= ORDERED_INF ? INFINITY : ordered_to_float(bound + 1);
+    }
+}
+
+// The rows that score below a query's threshold, as tc_collect left them, to the query's results.
+struct BfCollected {
+    const uint64_t* keys;     // [queries][lists][cap] nominating score and row
+    const uint32_t* count;    // [queries][lists] entries offered
+    const float* thr;         // [queries]
+    uint32_t lists, cap;
+    uint32_t room;            // entries of one query that shared memory holds
+    const void* queries;      // [queries x dim] in the index's type
+    const void* base;
+    uint32_t dim, kcand, k;
+    int metric;
+    const int64_t* labels;
+    int64_t* ids;
+    float* dists;
+    BfMargin m;
+};
+
+// One CTA per query: gathers its lists, re-scores the kcand best in the reference's operation order (see bf_rows_kernel) and
+// keeps k.  A query is sure of its results when the k-th of them is nearer than the last nominated score -- or the threshold, if
+// no row below it was left out -- allows any other row to be.  When it is not, all collected rows are re-scored, after which
+// only those above the threshold are left out; what is not sure then, or did not fit, is listed for the exact pass.
+// Dynamic shared memory: [room] keys, [lists + 1] places, the query.
+template <typename E, int T>
+__global__ void __launch_bounds__(T)
+bf_collected_kernel(const BfCollected p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SelectScratch sel;
+    __shared__ __align__(16) uint64_t keys[SELECT_CAP];
+    __shared__ __align__(16) uint64_t best[1024];
+    __shared__ float s_qq, s_top;
+    __shared__ uint32_t s_over;
+    uint64_t* all = reinterpret_cast<uint64_t*>(smem);
+    uint32_t* place = reinterpret_cast<uint32_t*>(all + p.room);
+    float* qf = reinterpret_cast<float*>(place + p.lists + 1);
+    const uint64_t q = blockIdx.x;
+    const uint32_t dim = p.dim;
+    const bool l2 = p.metric == VB200_METRIC_L2;
+    const E* base = static_cast<const E*>(p.base);
+    for (uint32_t d = threadIdx.x; d < dim; d += T) {
+        qf[d] = widen(static_cast<const E*>(p.queries)[q * dim + d]);
+    }
+    if (threadIdx.x == 0) {
+        s_over = 0;
+    }
+    __syncthreads();
+    // where each list's entries begin
+    const uint32_t* count = p.count + q * p.lists;
+    uint32_t total = 0;
+    for (uint32_t l0 = 0; l0 < p.lists; l0 += T) {
+        const uint32_t l = l0 + threadIdx.x;
+        uint32_t c = l < p.lists ? __ldg(count + l) : 0u;
+        if (c > p.cap) {
+            s_over = 1;
+            c = p.cap;
+        }
+        const uint32_t incl = block_inclusive_sum<T>(c, sel.warp_part);
+        if (l < p.lists) {
+            place[l] = total + incl - c;
+        }
+        if (threadIdx.x == T - 1) {
+            sel.total = total + incl;
+        }
+        __syncthreads();
+        total = sel.total;
+    }
+    if (threadIdx.x == 0) {
+        place[p.lists] = total;
+    }
+    __syncthreads();
+    if (s_over != 0 || total > p.room) {
+        if (threadIdx.x == 0) {
+            p.m.unsure[1 + atomicAdd(p.m.unsure, 1u)] = p.m.q_base + static_cast<uint32_t>(q);
+        }
+        return;
+    }
+    const uint64_t* mine = p.keys + q * p.lists * p.cap;
+    for (uint32_t i = threadIdx.x; i < total; i += T) {
+        uint32_t lo = 0, hi = p.lists;   // the list that holds entry i is the last one that begins at or before it
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (place[mid] <= i) {
+                lo = mid;
+            } else {
+                hi = mid;
+            }
+        }
+        all[i] = __ldg(mine + static_cast<uint64_t>(lo) * p.cap + (i - place[lo]));
+    }
+    __syncthreads();
+    // a few more than the `keep` smallest of `all`, unsorted, in keys; how many.  No other is below *left (ORDERED_INF: no other)
+    auto smallest = [&](uint32_t keep, uint32_t* left) -> uint32_t {
+        return block_select<T>(load_source([&](uint32_t i) { return static_cast<uint32_t>(all[i] >> 32); }),
+                               [&](uint32_t i) { return static_cast<uint32_t>(all[i]); }, total, keep, keys, sel, left);
+    };
+    uint32_t left;
+    uint32_t have = smallest(p.kcand, &left);
+    const float thr = __ldg(p.thr + q);
+    float last = left < ORDERED_INF ? ordered_to_float(left) : thr;
+    bool dropped = last < INFINITY;
+    if (threadIdx.x / 32 == T / 32 - 1) {   // (while the first warps wait for the candidates' rows)
+        const float top = __ldg(p.m.row_max);
+        float qq = 0.f;
+        for (uint32_t d = threadIdx.x % 32; d < dim; d += 32) {
+            qq = fmaf(qf[d], qf[d], qq);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        }
+        s_qq = qq;
+        s_top = top;
+    }
+    for (uint32_t i = threadIdx.x; i < have; i += T) {
+        const uint32_t row = static_cast<uint32_t>(keys[i]);
+        keys[i] = make_key(row_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, l2), row);
+    }
+    block_sort_to<T>(keys, have, p.k, best);
+    const float top = s_top, qq = s_qq;
+    auto sure = [&]() -> bool {
+        if (dropped && have < p.k) {
+            return false;
+        }
+        const float kth = dropped ? ordered_to_float(static_cast<uint32_t>(best[p.k - 1] >> 32)) : 0.f;
+        const float margin = p.m.of(l2, top, qq, kth);
+        return margin < INFINITY && (!dropped || kth < last + (l2 ? qq : 1.0f) - margin);
+    };
+    bool done = sure();
+    if (!done && have < total) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < total; i += T) {
+            const uint32_t row = static_cast<uint32_t>(all[i]);
+            all[i] = make_key(row_exact_distance(base + static_cast<uint64_t>(row) * dim, qf, dim, l2), row);
+        }
+        __syncthreads();
+        have = smallest(p.k, &left);
+        block_sort_to<T>(keys, have, p.k, best);
+        last = thr;
+        dropped = thr < INFINITY;
+        done = sure();
+    }
+    for (uint32_t i = threadIdx.x; i < p.k; i += T) {
+        const bool there = i < have;
+        p.ids[q * p.k + i] = there ? __ldg(p.labels + static_cast<uint32_t>(best[i])) : -1;
+        p.dists[q * p.k + i] = there ? ordered_to_float(static_cast<uint32_t>(best[i] >> 32)) : INFINITY;
+    }
+    if (!done && threadIdx.x == 0) {
+        p.m.unsure[1 + atomicAdd(p.m.unsure, 1u)] = p.m.q_base + static_cast<uint32_t>(q);
+    }
+}
+
 }  // namespace vb200

@@ -1,6 +1,7 @@
 // Exact BruteForce kNN over fp32 or bf16 rows: dense score slabs select a few candidates more
 // than k per query, which are then re-scored in the reference's arithmetic and ordered.
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "bf_stream.cuh"
@@ -254,6 +255,7 @@ struct vb200_bf {
     DevBuf<uint16_t> base_hi, base_lo, q_hi, q_lo;
     bool tiled_valid = false;
     DevBuf<uint64_t> tc_out;
+    DevBuf<uint32_t> list_count;   // entries of every list of tc_out
     DevBuf<uint64_t> sh_local, sh_all;   // sharded search: this rank's packed [keys | labels] and the gathered ones
     DevBuf<float> row_bound;   // per query: the kcand-th candidate score after the column ranges searched so far
     TcWorkspace tc;
@@ -497,10 +499,16 @@ vb200_bf_remove(vb200_bf_t ix, const int64_t* labels, uint64_t count, uint64_t* 
     return 0;
 }
 
+// The queries on the device and the rows' masks, as bf_stage leaves them.
+struct BfStaged {
+    const float *queries = nullptr, *bias = nullptr;
+    bool masked = false;
+};
+
 // What every search starts with: the queries on the device (normalised for cosine, rounded for bf16 rows) and
 // the score bias per row -- |x|^2 for L2, none for IP, +inf for rows that are removed or filtered out.
 static int
-bf_stage(vb200_bf* ix, const float* queries, uint64_t nq, const float** q_out, const float** bias_out, bool* masked_out) {
+bf_stage(vb200_bf* ix, const float* queries, uint64_t nq, BfStaged* out) {
     const uint32_t dim = ix->dim;
     const uint64_t n = ix->n;
     const float* q_dev = queries;
@@ -524,8 +532,8 @@ bf_stage(vb200_bf* ix, const float* queries, uint64_t nq, const float** q_out, c
     const vb200_filter* f = ix->filter;
     const bool user_deny = f != nullptr && f->deny_inner_bits != nullptr && f->n_inner_bits > 0;
     const bool user_labels = f != nullptr && f->invalid_label_bits != nullptr && f->n_label_bits > 0;
-    *masked_out = ix->n_removed > 0 || user_deny || user_labels;
-    if (*masked_out) {
+    out->masked = ix->n_removed > 0 || user_deny || user_labels;
+    if (out->masked) {
         DevInput<uint32_t> deny;
         DevInput<uint64_t> lbits;
         if (user_deny) {
@@ -542,8 +550,8 @@ bf_stage(vb200_bf* ix, const float* queries, uint64_t nq, const float** q_out, c
         VB_TRY(sync_stream());   // the staged bitmaps end with this scope
         bias_all = ix->masked_bias.ptr;
     }
-    *q_out = q_dev;
-    *bias_out = bias_all;
+    out->queries = q_dev;
+    out->bias = bias_all;
     return 0;
 }
 
@@ -578,7 +586,7 @@ bf_tile_queries(vb200_bf* ix, const float* q_dev, uint64_t nq) {
 
 // Leaves the k best keys (payload = row) per query in ix->keys.
 static int
-bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
+bf_search_keys(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k) {
     const uint32_t dim = ix->dim;
     const uint64_t n = ix->n;
     uint32_t kcand = k + BF_SLACK;
@@ -588,16 +596,14 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
     VB_CHECK_ARG(kcand <= 1024, "k = %u is too large (limit %u)", k, 1024 - BF_SLACK);
     const bool l2 = ix->metric == VB200_METRIC_L2;
     const bool bf16 = ix->quant == VB200_QUANT_BF16;
-    const float *q_dev = nullptr, *bias_all = nullptr;
-    bool masked = false;
-    VB_TRY(bf_stage(ix, queries, nq, &q_dev, &bias_all, &masked));
+    const float *q_dev = staged.queries, *bias_all = staged.bias;
     // Large problems nominate candidates on the tensor cores; the exact re-scoring below is the
     // same either way.
     if (tensor_cores_enabled() && kcand <= tc_max_candidates(bf16 ? 1 : 3) && static_cast<double>(nq) * n * dim >= 2e10) {
         const uint32_t chunks = (dim + TC_KC - 1) / TC_KC;
         VB_TRY(bf_tile_base(ix));
         VB_TRY(bf_tile_queries(ix, q_dev, nq));
-        TcOperand a{ix->q_hi.ptr, bf16 ? nullptr : ix->q_lo.ptr, nq, chunks};
+        TcOperand a{ix->q_hi.ptr, bf16 ? nullptr : ix->q_lo.ptr, nq, chunks, dim};
         VB_TRY(ix->cand.reserve(nq * kcand));
         VB_TRY(ix->row_bound.reserve(nq));
         // The base goes through the tensor cores in a few column ranges of growing size (a first one of about
@@ -621,7 +627,7 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
             const uint64_t row0 = tile0 * TC_BN;
             const uint64_t rows = (tile1 * TC_BN < n ? tile1 * TC_BN : n) - row0;
             const size_t off = static_cast<size_t>(tile0) * chunks * TC_CHUNK_ELEMS;
-            TcOperand b{ix->base_hi.ptr + off, bf16 ? nullptr : ix->base_lo.ptr + off, rows, chunks};
+            TcOperand b{ix->base_hi.ptr + off, bf16 ? nullptr : ix->base_lo.ptr + off, rows, chunks, dim};
             const bool first = tile0 == 0;
             uint32_t lists = 1;
             VB_TRY(tc_candidates(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, bias_all != nullptr ? bias_all + row0 : nullptr,
@@ -696,12 +702,6 @@ bf_search_keys(vb200_bf* ix, const float* queries, uint64_t nq, uint32_t k) {
     }
     return 0;
 }
-
-// The queries on the device and the rows' masks, as bf_stage leaves them.
-struct BfStaged {
-    const float *queries = nullptr, *bias = nullptr;
-    bool masked = false;
-};
 
 // Shared memory of a CTA that streams rows for qn queries, `keep` results each (no more than there are rows).
 static uint32_t
@@ -796,6 +796,126 @@ bf_stream_queries(vb200_bf* ix, const BfStaged& staged, uint64_t nq, const uint3
 constexpr uint64_t BF_SLICE_SCORES = uint64_t{128} << 20;
 constexpr uint64_t BF_UNSURE_SLICE = 4096;   // of those queries that are streamed at once (their partial results: k keys each per CTA)
 
+static BfMargin
+bf_margin(const vb200_bf* ix) {
+    BfMargin margin{};
+    margin.row_max = ix->row_max.ptr;
+    margin.chain = static_cast<float>(ix->dim + 16) * 6.0e-8f;
+    margin.matrix = ix->quant == VB200_QUANT_BF16 ? 2.0f * margin.chain : 4.0f * margin.chain + 3.0f / 262144.0f;
+    margin.unsure = ix->unsure.ptr + 1;
+    return margin;
+}
+
+// Batches over many rows: no score is written that a threshold rules out.
+//   sample   the smallest score of every 32 rows in one tile of 128 in `stride`; of those minima the kcand-th smallest is a score
+//            that kcand rows reach, so the rows with the kcand best scores are among those that do not pass it
+//   collect  one pass over all rows appends what does not pass the query's threshold to its lists, about kcand * stride entries
+//   rows     a CTA per query selects, re-scores and writes its results (bf_collected_kernel)
+// 1000 queries over 100k x 128 fp32 rows, k 10: 13, 5, 75 and 47 us, where 121 wrote the scores and 174 selected from them.
+struct BfSample {
+    uint32_t stride = 0;       // 0: the rows are too few for a sample
+    uint64_t tiles = 0;        // in the sample
+    double most = 0.0;         // rows that a query may collect
+};
+constexpr uint32_t BF_COLLECT_KEYS = 12288;          // of a query, at most (96 KiB of shared memory)
+// Above this many products of one term the sample's share of them is more than the merges of bf_search_keys cost (10,000 queries, k 100,
+// 6M x 768 bf16 rows under the power limit: 89.2 ms against 87.2).
+constexpr double BF_COLLECT_PRODUCTS = 1.6e12;
+constexpr uint32_t BF_COLLECT_DIMS = 16384;          // the query lies beside them
+constexpr uint64_t BF_COLLECT_SLOTS = uint64_t{256} << 20;   // list entries of the queries that go together, at most (2 GiB)
+
+// The sample takes a thirty-second of the rows, or the smallest larger power of two's share whose minima are four times kcand, so
+// that the threshold is near the kcand-th best of the sample; at most an eighth, beyond which the scores are as well written.
+// (A sixty-fourth lets twice as many rows pass: 6M x 768 rows, 10,000 queries, k 100: 1.8 ms for the sample and 72.9 for
+// the pass, against 3.0 and 71.8.)
+static BfSample
+bf_sample(uint64_t n, uint32_t dim, uint32_t kcand) {
+    BfSample s;
+    if (dim > BF_COLLECT_DIMS) {
+        return s;
+    }
+    const uint64_t tiles = (n + TC_BN - 1) / TC_BN;
+    for (uint32_t stride = 32; stride >= 8; stride /= 2) {
+        const uint64_t taken = (tiles + stride - 1) / stride, minima = taken * (TC_BN / 32);
+        // a row's chance to be below: of a minimum it is kcand / minima
+        const double p = 1.0 - std::pow(1.0 - std::min(0.99, static_cast<double>(kcand) / static_cast<double>(minima)), 1.0 / 32.0);
+        // what a query may collect: the threshold is the kcand-th of a sample, its rank in all rows known to 1 / sqrt(kcand);
+        // six times that is room for all of a batch's queries (with 1.25 times the expected 31 of 10,000 did not fit)
+        const double most = p * static_cast<double>(n) * (1.0 + 6.0 / std::sqrt(static_cast<double>(kcand))) + 256.0;
+        if (minima >= 4ull * kcand && most <= BF_COLLECT_KEYS) {
+            s.stride = stride;
+            s.tiles = taken;
+            s.most = most;
+            return s;
+        }
+    }
+    return s;
+}
+
+static int
+bf_search_collected(vb200_bf* ix, const BfStaged& staged, const BfSample& sample, uint64_t nq, uint32_t k, int64_t* ids_dev,
+                    float* dists_dev) {
+    const uint32_t dim = ix->dim;
+    const bool l2 = ix->metric == VB200_METRIC_L2, bf16 = ix->quant == VB200_QUANT_BF16;
+    const float* q_dev = staged.queries;
+    const float alpha = l2 ? -2.0f : -1.0f;
+    VB_TRY(bf_tile_base(ix));
+    VB_TRY(bf_tile_queries(ix, q_dev, nq));
+    const uint32_t chunks = (dim + TC_KC - 1) / TC_KC, terms = bf16 ? 1 : 3;
+    const uint32_t kcand = static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n));
+    const uint64_t ld = sample.tiles * (TC_BN / 32);
+    // whole row tiles whose lists fit
+    TcCollect plan = tc_collect_plan(nq, ix->n, sample.most);
+    uint64_t slice = BF_COLLECT_SLOTS / (static_cast<uint64_t>(plan.lists) * plan.cap) / TC_BM * TC_BM;
+    slice = slice < TC_BM ? TC_BM : (slice > nq ? nq : slice);
+    if (slice < nq) {
+        const uint64_t parts = (nq + slice - 1) / slice;
+        slice = ((nq + parts - 1) / parts + TC_BM - 1) / TC_BM * TC_BM;
+        plan = tc_collect_plan(slice, ix->n, sample.most);
+    }
+    VB_TRY(ix->scores.reserve(slice * ld));
+    VB_TRY(ix->row_bound.reserve(slice));
+    VB_TRY(ix->tc_out.reserve(slice * plan.lists * plan.cap));
+    VB_TRY(ix->list_count.reserve(slice * plan.lists));
+    VB_TRY(ix->unsure.reserve(nq + 2));
+    VB_CUDA(cudaMemsetAsync(ix->unsure.ptr, 0, 2 * sizeof(uint32_t), current_stream()));
+    int* const error_flag = reinterpret_cast<int*>(ix->unsure.ptr);
+    const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks, dim};
+    BfCollected c{};
+    c.keys = ix->tc_out.ptr;
+    c.count = ix->list_count.ptr;
+    c.thr = ix->row_bound.ptr;
+    c.lists = plan.lists;
+    c.cap = plan.cap;
+    c.room = std::max<uint32_t>(512, std::min<uint32_t>(BF_COLLECT_KEYS, static_cast<uint32_t>(1.25 * sample.most) + 256));
+    c.dim = dim;
+    c.kcand = kcand;
+    c.k = k;
+    c.metric = ix->metric;
+    c.labels = ix->labels.ptr;
+    c.m = bf_margin(ix);
+    const size_t smem = static_cast<size_t>(c.room) * sizeof(uint64_t) + (plan.lists + 1) * sizeof(uint32_t) + dim * sizeof(float);
+    VB_CHECK_ARG(smem <= 180 * 1024, "dim = %u is too large for the exact re-scoring step", dim);
+    for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
+        const uint64_t m = std::min(slice, nq - q0);
+        const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
+        const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks, dim};
+        VB_TRY(tc_minima(a, b, terms, alpha, staged.bias, sample.stride, ix->scores.ptr, ld, error_flag));
+        VB_LAUNCH(bf_threshold_kernel, static_cast<uint32_t>(m), BF_THRESHOLD_THREADS, 0, ix->scores.ptr, static_cast<uint32_t>(ld), kcand,
+                  ix->row_bound.ptr);
+        VB_TRY(tc_collect(plan, a, b, terms, alpha, staged.bias, ix->row_bound.ptr, ix->tc_out.ptr, ix->list_count.ptr, error_flag));
+        c.queries = bf16 ? static_cast<const void*>(ix->q_bf16.ptr + q0 * dim) : q_dev + q0 * dim;
+        c.base = bf16 ? static_cast<const void*>(ix->base_bf16.ptr) : ix->base_f32.ptr;
+        c.ids = ids_dev + q0 * k;
+        c.dists = dists_dev + q0 * k;
+        c.m.q_base = static_cast<uint32_t>(q0);
+        auto kernel = bf16 ? bf_collected_kernel<uint16_t, 512> : bf_collected_kernel<float, 512>;
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+        VB_LAUNCH(kernel, static_cast<uint32_t>(m), 512, smem, c);
+    }
+    return 0;
+}
+
 static int
 bf_search_scores(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k, int64_t* ids_dev, float* dists_dev) {
     const uint32_t dim = ix->dim;
@@ -811,19 +931,15 @@ bf_search_scores(vb200_bf* ix, const BfStaged& staged, uint64_t nq, uint32_t k, 
     VB_TRY(ix->unsure.reserve(nq + 2));
     VB_CUDA(cudaMemsetAsync(ix->unsure.ptr, 0, 2 * sizeof(uint32_t), current_stream()));
     int* const error_flag = reinterpret_cast<int*>(ix->unsure.ptr);
-    const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks};
+    const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks, dim};
     const uint32_t kcand = static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n));
     const size_t smem = dim * sizeof(float);
     VB_CHECK_ARG(smem <= 180 * 1024, "dim = %u is too large for the exact re-scoring step", dim);
-    BfMargin margin{};
-    margin.row_max = ix->row_max.ptr;
-    margin.chain = static_cast<float>(dim + 16) * 6.0e-8f;
-    margin.matrix = bf16 ? 2.0f * margin.chain : 4.0f * margin.chain + 3.0f / 262144.0f;
-    margin.unsure = ix->unsure.ptr + 1;
+    BfMargin margin = bf_margin(ix);
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
         const uint64_t m = std::min(slice, nq - q0);
         const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
-        const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks};
+        const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks, dim};
         margin.q_base = static_cast<uint32_t>(q0);
         VB_TRY(tc_scores(ix->tc, a, b, bf16 ? 1 : 3, l2 ? -2.0f : -1.0f, staged.bias, ix->scores.ptr, ld, error_flag));
         if (bf16) {
@@ -894,37 +1010,42 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
     // (rows too long for a stream's shared memory, above 40,000 dimensions, are left to the slab of scores)
     const bool streams = k_fits && bf_stream_smem(ix->dim, bf_stream_cap(static_cast<uint32_t>(std::min<uint64_t>(k, ix->n))), 1) <= 220 * 1024;
     const bool few = nq <= BF_STREAM_QUERIES && streams;
-    bool scores = tensor_cores_enabled() && streams && !few && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES;
+    const bool batch = tensor_cores_enabled() && streams && !few;
+    bool scores = batch && static_cast<double>(nq) * ix->n <= BF_MATRIX_SCORES, collected = false;
     BfStaged staged;
     bool keyed = false;
-    int rc = 0;
     ix->filter = filter;
-    // Up to eight queries share one pass over the rows; more go to the tensor cores -- through a score matrix
+    int rc = bf_stage(ix, queries, nq, &staged);
+    // Up to eight queries share one pass over the rows; more go to the tensor cores, which keep what passes a threshold from a
+    // sample of the rows; where the sample would be a large part of them, or rows are filtered out, through a score matrix
     // while that is cheaper than selecting as the scores appear (measured: up to about 4e8 scores), see
     // bf_search_keys for the rest.
-    if (few) {
-        rc = bf_stage(ix, queries, nq, &staged.queries, &staged.bias, &staged.masked);
-        if (rc == 0) {
-            rc = bf_stream_queries(ix, staged, nq, nullptr, k, ids_dev, dists_dev);
-        }
-    } else if (scores) {
-        rc = bf_stage(ix, queries, nq, &staged.queries, &staged.bias, &staged.masked);
-        if (rc == 0) {
+    if (rc == 0 && few) {
+        rc = bf_stream_queries(ix, staged, nq, nullptr, k, ids_dev, dists_dev);
+    } else if (rc == 0 && batch) {
+        const BfSample sample = staged.masked ? BfSample{} : bf_sample(ix->n, ix->dim, static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n)));
+        const double products = static_cast<double>(nq) * ix->n * ix->dim * (ix->quant == VB200_QUANT_BF16 ? 1 : 3);
+        collected = sample.stride != 0 && products <= BF_COLLECT_PRODUCTS;
+        if (collected) {
+            rc = bf_search_collected(ix, staged, sample, nq, k, ids_dev, dists_dev);
+        } else if (scores) {
             rc = bf_search_scores(ix, staged, nq, k, ids_dev, dists_dev);
         }
         if (rc == VB200_NO_ENOUGH_MEMORY) {
             // the tiled copy of the rows did not fit beside them: the slab of scores needs none
             (void)cudaStreamSynchronize(current_stream());
-            scores = false;
+            collected = scores = false;
             if (!ix->tiled_valid) {
                 ix->base_hi.release();
                 ix->base_lo.release();
             }
             ix->scores.release();
+            ix->tc_out.release();
+            rc = 0;
         }
     }
-    if (!few && !scores) {
-        rc = bf_search_keys(ix, queries, nq, k);
+    if (rc == 0 && !few && !scores && !collected) {
+        rc = bf_search_keys(ix, staged, nq, k);
         keyed = true;
     }
     ix->filter = nullptr;
@@ -945,8 +1066,8 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
         return 0;
     };
     VB_TRY(results_to_host());
-    uint32_t report[2] = {0, 0};   // of the score matrix: error flag, unsure queries
-    if (scores) {
+    uint32_t report[2] = {0, 0};   // of the batch's kernels: error flag, unsure queries
+    if (scores || collected) {
         VB_CUDA(cudaMemcpyAsync(report, ix->unsure.ptr, sizeof(report), cudaMemcpyDeviceToHost, current_stream()));
     }
     VB_TRY(sync_stream());
@@ -989,7 +1110,9 @@ vb200_bf_search_partial(vb200_bf_t ix, const float* queries, uint64_t nq, uint32
         VB_CUDA(cudaMemsetAsync(labels_dev, 0xFF, total * sizeof(int64_t), current_stream()));
         return sync_stream();
     }
-    VB_TRY(bf_search_keys(ix, queries, nq, k));
+    BfStaged staged;
+    VB_TRY(bf_stage(ix, queries, nq, &staged));
+    VB_TRY(bf_search_keys(ix, staged, nq, k));
     VB_LAUNCH(bf_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ix->keys.ptr, total,
               ix->labels.ptr, labels_dev, nullptr, keys_dev);
     return sync_stream();
@@ -1016,7 +1139,9 @@ vb200_bf_search_sharded(vb200_bf_t ix, vb200_comm_t comm, const float* queries, 
     if (ix->n == 0) {
         VB_CUDA(cudaMemsetAsync(ix->sh_local.ptr, 0xFF, 2 * total * sizeof(uint64_t), st));
     } else {
-        VB_TRY(bf_search_keys(ix, queries, nq, k));
+        BfStaged staged;
+        VB_TRY(bf_stage(ix, queries, nq, &staged));
+        VB_TRY(bf_search_keys(ix, staged, nq, k));
         VB_LAUNCH(bf_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, ix->keys.ptr, total,
                   ix->labels.ptr, reinterpret_cast<int64_t*>(ix->sh_local.ptr + total), nullptr, ix->sh_local.ptr);
     }

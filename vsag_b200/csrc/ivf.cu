@@ -2445,8 +2445,8 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         VB_TRY(ws.q_hi.reserve(q_elems));
         VB_TRY(ws.q_lo.reserve(q_elems));
         VB_TRY(tc_pretile_f32(q_dev, nq, ix->dim, ws.q_hi.ptr, ws.q_lo.ptr));
-        TcOperand a{ws.q_hi.ptr, ws.q_lo.ptr, nq, chunks};
-        TcOperand b{ix->c_hi.ptr, ix->c_lo.ptr, nlist, chunks};
+        TcOperand a{ws.q_hi.ptr, ws.q_lo.ptr, nq, chunks, ix->dim};
+        TcOperand b{ix->c_hi.ptr, ix->c_lo.ptr, nlist, chunks, ix->dim};
         // Score matrices larger than ROUTE_MATRIX_SCORES over large list counts: no matrix.  The scores against a sample of the centroids (the first
         // `sample` of them; centroid numbering carries no geometry) give each query a threshold; one pass
         // of the tensor-core kernel over all centroids then keeps, unsorted, only what scores below it --
@@ -2470,7 +2470,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         if (sample != 0 && ncand <= 256) {
             const float alpha = l2 ? -2.0f : -1.0f;
             const float* bias = l2 ? ix->c_sq.ptr : nullptr;
-            TcOperand bs{ix->c_hi.ptr, ix->c_lo.ptr, sample, chunks};
+            TcOperand bs{ix->c_hi.ptr, ix->c_lo.ptr, sample, chunks, ix->dim};
             VB_TRY(ws.scores.reserve(nq * sample));
             // No wait for either tensor-core pass: what they report (a bounded wait that gave up) is OR-ed into
             // ws.scalars[8], which every caller reads when it synchronises at the end of its call; a query whose
@@ -2521,7 +2521,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
         for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
             const uint64_t m = std::min(slice, nq - q0);
             const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
-            VB_TRY(tc_scores(ix->tc, TcOperand{ws.q_hi.ptr + off, ws.q_lo.ptr + off, m, chunks}, b, 3, l2 ? -2.0f : -1.0f,
+            VB_TRY(tc_scores(ix->tc, TcOperand{ws.q_hi.ptr + off, ws.q_lo.ptr + off, m, chunks, ix->dim}, b, 3, l2 ? -2.0f : -1.0f,
                              l2 ? ix->c_sq.ptr : nullptr, ws.scores.ptr, ld, route_flag));
             PairsPrepare part = pp.from(q0);
             part.scores = ws.scores.ptr;

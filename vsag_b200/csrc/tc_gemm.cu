@@ -183,13 +183,14 @@ tc_compact_row(uint64_t* my_buf, uint32_t& my_cnt, float& my_thr, uint32_t owner
 // selection, the scores themselves are stored; MODE 3: every column scoring below the row's fixed
 // threshold (row_bound) is appended, unsorted, to the row's output list of `cap` entries -- no
 // sorting at all, the caller sizes the lists from the threshold's expected pass rate and an
-// overflowing list sets bit 1 of the error flag.
+// overflowing list sets bit 1 of the error flag.  MODE 4: one minimum per row and 32 columns is stored.
 template <int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_candidates_kernel(const TcParams p) {
     constexpr bool SMALL_M = MODE == 0;
     constexpr bool STORE = MODE == 2;
     constexpr bool THRESH = MODE == 3;
+    constexpr bool MINIMA = MODE == 4;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ TcShared sh;
 
@@ -204,7 +205,7 @@ tc_candidates_kernel(const TcParams p) {
     const uint32_t stage_bytes = ((p.a_resident ? 0u : n_terms_op) + n_terms_op * step) * TC_CHUNK_BYTES;
     const uint32_t chunks = p.a.chunks;
     const uint64_t m_tiles = (p.a.rows + TC_BM - 1) / TC_BM;
-    const uint64_t n_tiles = (p.b.rows + TC_BN - 1) / TC_BN;
+    const uint64_t n_tiles = ((p.b.rows + TC_BN - 1) / TC_BN + p.tile_stride - 1) / p.tile_stride;   // that take part
     const uint64_t n_items = m_tiles * p.n_split;
 
     if (threadIdx.x == 0) {
@@ -256,9 +257,10 @@ tc_candidates_kernel(const TcParams p) {
     };
     // B tile number u of share `split`.  (Row tiles that start a share at different tiles, so as not to ask L2 for the
     // same lines together, were slower: 91 against 86 ms over 6M x 768 rows.)
-    auto tile_at = [&](uint32_t split, uint32_t u) -> uint32_t {
+    auto number_at = [&](uint32_t split, uint32_t u) -> uint32_t {
         return p.interleaved ? split + u * p.n_split : split * p.tiles_per_split + u;
     };
+    auto tile_at = [&](uint32_t split, uint32_t u) -> uint32_t { return number_at(split, u) * p.tile_stride; };
     if (warp == TC_EPI_WARPS) {
         // ---------------- MMA issue (one thread) ----------------
         // Written for latency: 32-bit counters that wrap by compare instead of divide, descriptors
@@ -309,18 +311,41 @@ tc_candidates_kernel(const TcParams p) {
                         {
                             const uint64_t a_at = a_res ? desc0 + c * n_terms_op * op_units : stage_desc;
                             const uint64_t b_at = a_res ? stage_desc : stage_desc + n_terms_op * op_units;
+                            const uint32_t steps = c + 1 == chunks ? p.last_steps : TC_KC / 16;
                             // a k-step of 16 elements = two 8-element cores: 256 B = 16 descriptor units
+                            // (the two forms of a whole chunk stand on their own: a test per step, or a loop that is not unrolled, takes the
+                            // operands out of the uniform registers, and this thread's pace is the kernel's: k-means 20.7 -> 23.5 ms)
                             if (p.n_terms == 3) {
                                 const uint64_t b_lo = b_at + step * op_units;
+                                if (steps == TC_KC / 16) {
+#pragma unroll
+                                    for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
+                                        umma_bf16(d_tmem, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
+                                        umma_bf16(d_tmem, a_at + kk * 16, b_lo + kk * 16, idesc, 1u);
+                                        umma_bf16(d_tmem, a_at + op_units + kk * 16, b_at + kk * 16, idesc, 1u);
+                                    }
+                                } else {
+#pragma unroll
+                                    for (uint32_t kk = 0; kk < TC_KC / 16 - 1; ++kk) {
+                                        if (kk >= steps) {
+                                            break;
+                                        }
+                                        umma_bf16(d_tmem, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
+                                        umma_bf16(d_tmem, a_at + kk * 16, b_lo + kk * 16, idesc, 1u);
+                                        umma_bf16(d_tmem, a_at + op_units + kk * 16, b_at + kk * 16, idesc, 1u);
+                                    }
+                                }
+                            } else if (steps == TC_KC / 16) {
 #pragma unroll
                                 for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
                                     umma_bf16(d_tmem, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
-                                    umma_bf16(d_tmem, a_at + kk * 16, b_lo + kk * 16, idesc, 1u);
-                                    umma_bf16(d_tmem, a_at + op_units + kk * 16, b_at + kk * 16, idesc, 1u);
                                 }
                             } else {
 #pragma unroll
-                                for (uint32_t kk = 0; kk < TC_KC / 16; ++kk) {
+                                for (uint32_t kk = 0; kk < TC_KC / 16 - 1; ++kk) {
+                                    if (kk >= steps) {
+                                        break;
+                                    }
                                     umma_bf16(d_tmem, a_at + kk * 16, b_at + kk * 16, idesc, (c == 0 && kk == 0) ? 0u : 1u);
                                 }
                             }
@@ -603,6 +628,13 @@ tc_candidates_kernel(const TcParams p) {
                     }
                     m4[3] = fminf(m11[3], m11[7]);
                     const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
+                    if (MINIMA) {
+                        if (valid_row && tile_present) {
+                            p.store[grow * p.store_ld + number_at(split32, static_cast<uint32_t>(t) + step_col / TC_BN) * (TC_BN / 32) +
+                                    step_col % TC_BN / 32] = mn;
+                        }
+                        continue;
+                    }
                     if (SMALL_M) {
                         if (mn < bound) {
                             // few elements pass: found through the levels of the tree (an index that is not a constant
@@ -674,7 +706,7 @@ tc_candidates_kernel(const TcParams p) {
             if (!ok) {
                 break;
             }
-            if (STORE) {
+            if (STORE || MINIMA) {
                 continue;
             }
             if (THRESH) {
@@ -808,6 +840,8 @@ tc_plan(TcParams& p, size_t sort_bytes, size_t* smem_bytes) {
     p.stages = stages;
     p.a_resident = resident ? 1u : 0u;
     p.wide = wide ? 1u : 0u;
+    p.last_steps = p.a.dim != 0 ? (p.a.dim - (p.a.chunks - 1) * TC_KC + 15) / 16 : TC_KC / 16;
+    p.tile_stride = 1;
     *smem_bytes = fixed + stages * stage_bytes(resident, wide);
 }
 
@@ -1024,6 +1058,101 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
     *lists_out = lists;
     *cap_out = cap;
     *overflow_out = (flag & 2) != 0;
+    return 0;
+}
+
+int
+tc_minima(const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev, uint32_t tile_stride,
+          float* minima_dev, uint64_t ld, int* deferred_flag_dev) {
+    VB_CHECK_ARG(a.rows > 0 && b.rows > 0 && tile_stride > 0, "tc_minima: empty operand");
+    VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_minima: operand depths differ");
+    VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_minima: 1 or 3 terms");
+    TcParams p{};
+    p.a = a;
+    p.b = b;
+    p.n_terms = n_terms;
+    size_t smem = 0;
+    tc_plan(p, 0, &smem);
+    p.tile_stride = tile_stride;
+    const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
+    const uint64_t n_tiles = ((b.rows + TC_BN - 1) / TC_BN + tile_stride - 1) / tile_stride;
+    VB_CHECK_ARG(ld >= n_tiles * (TC_BN / 32), "tc_minima: rows of minima too short");
+    const uint32_t sms = static_cast<uint32_t>(sm_count());
+    uint64_t n_split = (2ull * sms + m_tiles - 1) / m_tiles;
+    n_split = n_split > n_tiles ? n_tiles : n_split;
+    const uint64_t tiles_per_split = (n_tiles + n_split - 1) / n_split;
+    n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
+    const uint64_t items = m_tiles * n_split;
+    p.alpha = alpha;
+    p.bias = bias_dev;
+    p.n_split = static_cast<uint32_t>(n_split);
+    p.tiles_per_split = static_cast<uint32_t>(tiles_per_split);
+    p.store = minima_dev;
+    p.store_ld = ld;
+    p.error_flag = deferred_flag_dev;
+    p.spin_limit = tc_spin_limit();
+    auto kernel = tc_candidates_kernel<4>;
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    VB_LAUNCH(kernel, static_cast<uint32_t>(items < sms ? items : sms), TC_THREADS, smem, p);
+    return 0;
+}
+
+// Shares: as many as leave the fewest CTAs idle in the last round of the persistent grid, of eight tiles or more; 3 to 32 of
+// them for many row tiles, up to two rounds' worth for a few.
+TcCollect
+tc_collect_plan(uint64_t a_rows, uint64_t b_rows, double expected_per_row) {
+    const uint64_t m_tiles = (a_rows + TC_BM - 1) / TC_BM, n_tiles = (b_rows + TC_BN - 1) / TC_BN;
+    const uint64_t sms = static_cast<uint64_t>(sm_count());
+    uint64_t best = 1;
+    double best_cost = 0.0;
+    for (uint64_t ns = 1; ns <= 2 * sms && (ns == 1 || (ns * 8 <= n_tiles && m_tiles * ns <= 8 * sms)); ++ns) {
+        // rounds of the grid, each as long as its longest share; a start-up of about two tiles per item
+        const uint64_t rounds = (m_tiles * ns + sms - 1) / sms;
+        const double cost = static_cast<double>(rounds) * (static_cast<double>((n_tiles + ns - 1) / ns) + 2.0);
+        if (ns == 1 || cost < best_cost) {
+            best_cost = cost;
+            best = ns;
+        }
+    }
+    TcCollect c{};
+    c.n_split = static_cast<uint32_t>(best);
+    c.tiles_per_split = static_cast<uint32_t>((n_tiles + best - 1) / best);
+    c.lists = c.n_split * TC_COL_GROUPS;
+    // a list's expected share plus eight standard deviations of a Poisson count and a few more
+    const double share = expected_per_row / c.lists;
+    c.cap = next_pow2(static_cast<uint32_t>(share + 8.0 * std::sqrt(share) + 8.0));
+    c.cap = c.cap < 32 ? 32 : c.cap;
+    return c;
+}
+
+int
+tc_collect(const TcCollect& plan, const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev,
+           const float* row_thr_dev, uint64_t* out_dev, uint32_t* out_count_dev, int* deferred_flag_dev) {
+    VB_CHECK_ARG(a.rows > 0 && b.rows > 0, "tc_collect: empty operand");
+    VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_collect: operand depths differ");
+    VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_collect: 1 or 3 terms");
+    TcParams p{};
+    p.a = a;
+    p.b = b;
+    p.n_terms = n_terms;
+    size_t smem = 0;
+    tc_plan(p, 0, &smem);
+    const uint64_t items = (a.rows + TC_BM - 1) / TC_BM * plan.n_split;
+    const uint64_t sms = static_cast<uint64_t>(sm_count());
+    p.alpha = alpha;
+    p.bias = bias_dev;
+    p.row_bound = row_thr_dev;
+    p.cap = plan.cap;
+    p.n_split = plan.n_split;
+    p.tiles_per_split = plan.tiles_per_split;
+    p.interleaved = 1;
+    p.out = out_dev;
+    p.out_count = out_count_dev;
+    p.error_flag = deferred_flag_dev;
+    p.spin_limit = tc_spin_limit();
+    auto kernel = tc_candidates_kernel<3>;
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    VB_LAUNCH(kernel, static_cast<uint32_t>(items < sms ? items : sms), TC_THREADS, smem, p);
     return 0;
 }
 
