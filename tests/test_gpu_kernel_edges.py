@@ -68,3 +68,16 @@ def test_exact_batches_the_threshold_does_not_serve(engine, oracle, kind):
     assert np.array_equal(got[1], np.concatenate([o[1] for o in one]))
     if kind != "equal":
         assert np.array_equal(got[0], np.concatenate([o[0] for o in one]))
+
+
+@pytest.mark.parametrize("dim", [5, 32, 96, 224, 225, 300])
+def test_means_of_clusters_of_all_lengths(engine, oracle, dim):
+    sizes = [0, 1, 7, 8, 9, 31, 32, 33, 63, 64, 95, 96, 97, 128, 160, 1023, 1024, 1025, 1056, 2100, 0]
+    labels = np.repeat(np.arange(len(sizes), dtype=np.int32), sizes)
+    rng = np.random.default_rng(dim)
+    rng.shuffle(labels)
+    x = rng.standard_normal((labels.size, dim)).astype(np.float32)
+    got = engine.kmeans_update(x, labels, len(sizes), 3)
+    want = oracle.kmeans_update(x, labels, len(sizes), 3)
+    got, want = (v[0] if isinstance(v, tuple) else v for v in (got, want))
+    assert np.array_equal(got, want)

@@ -571,137 +571,122 @@ kmeans_assign_device(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32
 // fp32 addition per row -- the order the CPU oracle uses -- so training is reproducible bit for bit:
 // rows are sorted by (label, row) with a stable radix sort, and one CTA per cluster walks its rows.
 
-// keys[i] = label of row i (k for rows without a valid label), rows[i] = i, counts[label]++.
+// keys[i] = label of row i (k for rows without a valid label), rows[i] = i.
 __global__ void
 kmeans_sort_keys_kernel(const int32_t* __restrict__ labels, uint64_t n, uint32_t k, uint32_t* __restrict__ keys,
-                        uint32_t* __restrict__ rows, int32_t* __restrict__ counts) {
+                        uint32_t* __restrict__ rows) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) {
         return;
     }
     const int32_t l = labels[i];
-    const bool ok = l >= 0 && static_cast<uint32_t>(l) < k;
-    keys[i] = ok ? static_cast<uint32_t>(l) : k;
+    keys[i] = l >= 0 && static_cast<uint32_t>(l) < k ? static_cast<uint32_t>(l) : k;
     rows[i] = static_cast<uint32_t>(i);
-    if (ok) {
-        atomicAdd(counts + l, 1);
-    }
 }
 
-// off[j] = number of rows in clusters before j (one CTA; k is small next to the rows).
-__global__ void __launch_bounds__(1024)
-kmeans_cluster_offsets_kernel(const int32_t* __restrict__ counts, uint32_t k, uint32_t* __restrict__ off) {
-    __shared__ uint32_t part[1024];
-    const uint32_t per = (k + 1023) / 1024;
-    const uint32_t j0 = threadIdx.x * per, j1 = j0 + per < k ? j0 + per : k;
-    uint32_t sum = 0;
-    for (uint32_t j = j0; j < j1; ++j) {
-        sum += static_cast<uint32_t>(counts[j]);
-    }
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (uint32_t o = 1; o < 1024; o <<= 1) {
-        const uint32_t v = threadIdx.x >= o ? part[threadIdx.x - o] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - sum;
-    for (uint32_t j = j0; j < j1; ++j) {
-        off[j] = run;
-        run += static_cast<uint32_t>(counts[j]);
-    }
-    if (threadIdx.x == 1023) {
-        off[k] = part[1023];
-    }
-}
-
-// sums[j][d] = ((x[r0][d] + x[r1][d]) + x[r2][d]) + ... over the rows r0 < r1 < ... of cluster j.  One CTA
-// per cluster, one thread per dimension (strided when dim exceeds the CTA); the loads of 32 rows are
-// issued together and a batch ahead of the additions, which stay in row order (the time is the longest cluster's chain: 396 us
-// for 1M x 128 rows in 4096 clusters with eight loads together, 335 with 32, 240 with the next 32 on their way).
-__global__ void __launch_bounds__(128)
-kmeans_sum_in_order_kernel(const float* __restrict__ x, uint32_t dim, const uint32_t* __restrict__ sorted_rows,
-                           const uint32_t* __restrict__ off, float* __restrict__ sums) {
-    const uint32_t j = blockIdx.x;
-    const uint32_t beg = off[j], end = off[j + 1];
-    for (uint32_t d = threadIdx.x; d < dim; d += blockDim.x) {
-        float s = 0.f;
-        uint32_t r = beg;
-        if (r + 32 <= end) {
-            float v[32];
-            auto load = [&](float (&w)[32], uint32_t at) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    w[i] = __ldg(x + static_cast<uint64_t>(__ldg(sorted_rows + at + i)) * dim + d);
-                }
-            };
-            auto add = [&](const float (&w)[32]) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    s = __fadd_rn(s, w[i]);
-                }
-            };
-            load(v, r);
-            for (; r + 96 <= end; r += 64) {   // a batch is on its way while the one before it is added
-                float w[32];
-                load(w, r + 32);
-                add(v);
-                load(v, r + 64);
-                add(w);
-            }
-            add(v);
-            r += 32;
-            if (r + 32 <= end) {
-                load(v, r);
-                add(v);
-                r += 32;
-            }
-        }
-        for (; r + 4 <= end; r += 4) {
-            float v[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                v[i] = __ldg(x + static_cast<uint64_t>(__ldg(sorted_rows + r + i)) * dim + d);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                s = __fadd_rn(s, v[i]);
-            }
-        }
-        for (; r < end; ++r) {
-            s = __fadd_rn(s, __ldg(x + static_cast<uint64_t>(__ldg(sorted_rows + r)) * dim + d));
-        }
-        sums[static_cast<uint64_t>(j) * dim + d] = s;
-    }
-}
-
+// off[j] = number of sorted keys below j, j = 0 .. k.  (Counted while the keys are written, an atomic per row, they took 46 us
+// for 1M rows, and the prefix sums another launch.)
 __global__ void
-kmeans_finalize_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, uint32_t k,
-                       uint32_t iter, const float* __restrict__ sums,
-                       const int32_t* __restrict__ counts, float* __restrict__ centroids) {
-    uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= static_cast<uint64_t>(k) * dim) {
+kmeans_cluster_offsets_kernel(const uint32_t* __restrict__ keys, uint64_t n, uint32_t k, uint32_t* __restrict__ off) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i > n) {
         return;
     }
-    uint32_t j = static_cast<uint32_t>(e / dim);
-    uint32_t d = static_cast<uint32_t>(e % dim);
-    int32_t c = counts[j];
-    if (c > 0) {
-        float inv = __fdiv_rn(1.0f, static_cast<float>(c));
-        centroids[e] = __fmul_rn(sums[e], inv);
-    } else {
-        uint64_t row = (static_cast<uint64_t>(j) * 2654435761ull + iter) % n;
-        centroids[e] = x[row * dim + d];
+    const uint32_t here = i < n ? keys[i] : k;
+    for (uint32_t j = i > 0 ? keys[i - 1] + 1 : 0u; j <= here; ++j) {
+        off[j] = static_cast<uint32_t>(i);
+    }
+}
+
+// centroids[j][d] = (((x[r0][d] + x[r1][d]) + x[r2][d]) + ...) / count over the rows r0 < r1 < ... of cluster j; a cluster without
+// rows takes a row of its own.  One CTA per cluster, one thread per dimension (strided when dim exceeds the CTA).  The time is
+// the longest cluster's chain: its row numbers lie in shared memory, the loads of 32 rows are issued together and a batch
+// ahead of the additions, which stay in row order (1M x 128 rows in 4096 clusters: 396 us with eight loads together, 335 with 32,
+// 240 with the next 32 on their way, 132 with the row numbers at hand and the means formed here).
+constexpr uint32_t SUM_ROWS = 1024;   // row numbers in shared memory
+
+__global__ void __launch_bounds__(256, 2)
+kmeans_mean_in_order_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, uint32_t iter, const uint32_t* __restrict__ sorted_rows,
+                            const uint32_t* __restrict__ off, int32_t* __restrict__ counts, float* __restrict__ centroids) {
+    __shared__ uint32_t row[SUM_ROWS];
+    const uint32_t j = blockIdx.x;
+    const uint32_t beg = off[j], end = off[j + 1];
+    if (threadIdx.x == 0) {
+        counts[j] = static_cast<int32_t>(end - beg);
+    }
+    for (uint32_t d0 = 0; d0 < dim; d0 += blockDim.x) {
+        const uint32_t d = d0 + threadIdx.x;
+        const bool live = d < dim;
+        const float* column = x + (live ? d : 0);
+        float s = 0.f;
+        for (uint32_t r0 = beg; r0 < end; r0 += SUM_ROWS) {
+            const uint32_t m = min(end - r0, SUM_ROWS);
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+                row[i] = __ldg(sorted_rows + r0 + i);
+            }
+            __syncthreads();
+            uint32_t r = 0;
+            if (live && m >= 32) {
+                float v[32];
+                auto load = [&](float (&w)[32], uint32_t at) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        w[i] = __ldg(column + static_cast<uint64_t>(row[at + i]) * dim);
+                    }
+                };
+                auto add = [&](const float (&w)[32]) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        s = __fadd_rn(s, w[i]);
+                    }
+                };
+                load(v, 0);
+                for (; r + 96 <= m; r += 64) {   // a batch is on its way while the one before it is added
+                    float w[32];
+                    load(w, r + 32);
+                    add(v);
+                    load(v, r + 64);
+                    add(w);
+                }
+                add(v);
+                r += 32;
+                if (r + 32 <= m) {
+                    load(v, r);
+                    add(v);
+                    r += 32;
+                }
+            }
+            for (; live && r + 8 <= m; r += 8) {
+                float v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    v[i] = __ldg(column + static_cast<uint64_t>(row[r + i]) * dim);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    s = __fadd_rn(s, v[i]);
+                }
+            }
+            for (; live && r < m; ++r) {
+                s = __fadd_rn(s, __ldg(column + static_cast<uint64_t>(row[r]) * dim));
+            }
+        }
+        if (live) {
+            if (end > beg) {
+                s = __fmul_rn(s, __fdiv_rn(1.0f, static_cast<float>(static_cast<int32_t>(end - beg))));
+            } else {
+                s = column[(static_cast<uint64_t>(j) * 2654435761ull + iter) % n * dim];
+            }
+            centroids[static_cast<uint64_t>(j) * dim + d] = s;
+        }
     }
 }
 
 int
 kmeans_update_device(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t dim,
                      const int32_t* labels_dev, uint32_t k, uint32_t iter, float* centroids_dev) {
-    const size_t kd = static_cast<size_t>(k) * dim;
     VB_CHECK_ARG(n < 0xFFFFFFFFull, "kmeans update: batch too large");
-    VB_TRY(ws.sums.reserve(kd));
     VB_TRY(ws.counts.reserve(k));
     VB_TRY(ws.sort_keys_in.reserve(n));
     VB_TRY(ws.sort_keys_out.reserve(n));
@@ -709,9 +694,8 @@ kmeans_update_device(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32
     VB_TRY(ws.sort_rows_out.reserve(n));
     VB_TRY(ws.cluster_off.reserve(static_cast<size_t>(k) + 1));
     cudaStream_t st = current_stream();
-    VB_CUDA(cudaMemsetAsync(ws.counts.ptr, 0, k * sizeof(int32_t), st));
     VB_LAUNCH(kmeans_sort_keys_kernel, static_cast<uint32_t>((n + 255) / 256), 256, 0, labels_dev, n, k,
-              ws.sort_keys_in.ptr, ws.sort_rows_in.ptr, ws.counts.ptr);
+              ws.sort_keys_in.ptr, ws.sort_rows_in.ptr);
     {
         // stable sort by label: rows of a cluster stay in ascending order
         int end_bit = 1;
@@ -729,11 +713,10 @@ kmeans_update_device(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32
                                                 end_bit, st));
         g_kernel_launches.fetch_add(1);
     }
-    VB_LAUNCH(kmeans_cluster_offsets_kernel, 1, 1024, 0, ws.counts.ptr, k, ws.cluster_off.ptr);
-    VB_LAUNCH(kmeans_sum_in_order_kernel, k, 128, 0, x_dev, dim, ws.sort_rows_out.ptr, ws.cluster_off.ptr,
-              ws.sums.ptr);
-    VB_LAUNCH(kmeans_finalize_kernel, static_cast<uint32_t>((kd + 255) / 256), 256, 0, x_dev, n, dim,
-              k, iter, ws.sums.ptr, ws.counts.ptr, centroids_dev);
+    VB_LAUNCH(kmeans_cluster_offsets_kernel, static_cast<uint32_t>(n / 256 + 1), 256, 0, ws.sort_keys_out.ptr, n, k, ws.cluster_off.ptr);
+    // (threads for the dimensions there are: the more CTAs of few dimensions an SM holds, the more rows are on their way)
+    VB_LAUNCH(kmeans_mean_in_order_kernel, k, dim <= 224 ? (dim + 31) / 32 * 32 : 256, 0, x_dev, n, dim, iter, ws.sort_rows_out.ptr,
+              ws.cluster_off.ptr, ws.counts.ptr, centroids_dev);
     return 0;
 }
 

@@ -9,7 +9,6 @@ namespace vb200 {
 struct KMeansWorkspace {
     DevBuf<float> c_sq;     // |c_j|^2
     DevBuf<float> best;     // best score per point
-    DevBuf<float> sums;     // k x dim accumulators
     DevBuf<int32_t> counts; // k
     // centroid update in a fixed order: rows sorted by (label, row), the first row of each cluster
     DevBuf<uint32_t> sort_keys_in, sort_keys_out, sort_rows_in, sort_rows_out, cluster_off;
