@@ -70,6 +70,16 @@ def test_exact_batches_the_threshold_does_not_serve(engine, oracle, kind):
         assert np.array_equal(got[0], np.concatenate([o[0] for o in one]))
 
 
+# ---- k-means ----------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n,dim", [(16, 3), (2369, 31), (5000, 32), (5001, 33), (4000, 64), (4000, 65), (4000, 80), (4001, 81), (3000, 96),
+                                   (3000, 129), (148 * 512, 8), (148 * 512 + 1, 8)])   # a row per thread, and one row more
+def test_seeding_by_rows_in_registers(engine, oracle, n, dim):
+    x = mixture(41, n, dim, 16, 0.2)
+    want_c, want_rows = oracle.kmeans_pp_init(x, 12, 47)
+    got_c, got_rows = engine.kmeans_init(x, 12, 47, want_rows=True)
+    assert np.array_equal(got_rows, want_rows) and np.array_equal(got_c, want_c)
+
+
 @pytest.mark.parametrize("dim", [5, 32, 96, 224, 225, 300])
 def test_means_of_clusters_of_all_lengths(engine, oracle, dim):
     sizes = [0, 1, 7, 8, 9, 31, 32, 33, 63, 64, 95, 96, 97, 128, 160, 1023, 1024, 1025, 1056, 2100, 0]

@@ -1038,20 +1038,30 @@ kpp_run_rounds(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, uint64_
                uint32_t* state, float* centroids_dev, int64_t* picked_dev, bool* done) {
     *done = false;
     const uint32_t sms = static_cast<uint32_t>(sm_count());
-    const size_t qpad = (dim + 3) / 4 * 4;
-    // rows per CTA when every SM takes a share (at least 16 rows: fewer are not worth a CTA in the barriers)
     const uint64_t resident_per = std::max<uint64_t>((n + sms - 1) / sms, 16);
+    constexpr int THREADS = 512;
+    // dimensions of a row in registers, where each row of a CTA has a thread (80 is what 128 registers a thread have room for)
+    const uint32_t reg = resident_per <= THREADS ? (dim <= 32 ? 32u : (dim <= 64 ? 64u : 80u)) : 0u;
+    const size_t qpad = std::max<size_t>((dim + 3) / 4 * 4, reg);
+    // rows per CTA when every SM takes a share (at least 16 rows: fewer are not worth a CTA in the barriers)
     const size_t resident_bytes = (qpad + resident_per * ((dim | 1u) + 1)) * sizeof(float);
     const bool resident = resident_bytes <= 216 * 1024;
     const bool wide = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(x_dev) & 15) == 0;
-    const size_t smem = resident ? resident_bytes : RS_STAGES * RS_STAGE + qpad * sizeof(float);
+    const size_t smem = resident ? resident_bytes : RS_STAGES * RS_STAGE + (dim + 3) / 4 * 4 * sizeof(float);
     if (smem > 216 * 1024) {
         return 0;
     }
-    const void* kernel = resident ? reinterpret_cast<const void*>(kpp_rounds_kernel<true, 4, 512>)
-                                  : (wide ? reinterpret_cast<const void*>(kpp_rounds_kernel<false, 16, RS_ROWS>)
-                                          : reinterpret_cast<const void*>(kpp_rounds_kernel<false, 4, RS_ROWS>));
-    const int threads = resident ? 512 : RS_ROWS;
+    const void* kernel = nullptr;
+    if (resident) {
+        kernel = reg == 32 ? reinterpret_cast<const void*>(kpp_rounds_kernel<true, 32, 4, THREADS>)
+                           : (reg == 64 ? reinterpret_cast<const void*>(kpp_rounds_kernel<true, 64, 4, THREADS>)
+                                        : (reg == 80 ? reinterpret_cast<const void*>(kpp_rounds_kernel<true, 80, 4, THREADS>)
+                                                     : reinterpret_cast<const void*>(kpp_rounds_kernel<true, 0, 4, THREADS>)));
+    } else {
+        kernel = wide ? reinterpret_cast<const void*>(kpp_rounds_kernel<false, 0, 16, RS_ROWS>)
+                      : reinterpret_cast<const void*>(kpp_rounds_kernel<false, 0, 4, RS_ROWS>);
+    }
+    const int threads = resident ? THREADS : RS_ROWS;
     VB_TRY(allow_dynamic_smem(kernel, smem));
     int per_sm = 0;
     VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
@@ -1066,21 +1076,27 @@ kpp_run_rounds(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, uint64_
     if (resident) {
         p.per = resident_per;
     } else {
-        const uint64_t most = std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, (n + RS_ROWS - 1) / RS_ROWS);
+        const uint64_t most = std::min<uint64_t>(std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, 32 * kpp_run(false)), (n + RS_ROWS - 1) / RS_ROWS);
         p.per = (n + most - 1) / most;
     }
     const uint64_t grid = (n + p.per - 1) / p.per;
+    if (grid > 32 * kpp_run(resident)) {
+        return 0;
+    }
     p.first = first;
-    DevBuf<double> draws, part;
-    DevBuf<unsigned long long> pick;
+    DevBuf<double> draws;
+    DevBuf<unsigned long long> words;   // the sums' two sets, the row's, and whether a wait gave up
+    const size_t n_words = 4 * grid + dim + 1;
     VB_TRY(draws.reserve(k));
-    VB_TRY(part.reserve(grid));
-    VB_TRY(pick.reserve(1));
+    VB_TRY(words.reserve(n_words));
+    VB_CUDA(cudaMemsetAsync(words.ptr, 0, n_words * sizeof(unsigned long long), current_stream()));
     VB_CUDA(cudaMemcpyAsync(draws.ptr, u.data(), k * sizeof(double), cudaMemcpyHostToDevice, current_stream()));
     p.u = draws.ptr;
     p.min_d = min_d;
-    p.part = part.ptr;
-    p.pick = pick.ptr;
+    p.part = words.ptr;
+    p.row = words.ptr + 4 * grid;
+    p.failed = reinterpret_cast<uint32_t*>(words.ptr + 4 * grid + dim);
+    p.spin_limit = tc_spin_limit();
     p.centroids = centroids_dev;
     p.picked = picked_dev;
     p.state = state;
@@ -1092,8 +1108,14 @@ kpp_run_rounds(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, uint64_
     }
     VB_CUDA(e);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    uint32_t failed = 0;
+    VB_CUDA(cudaMemcpyAsync(&failed, p.failed, sizeof(failed), cudaMemcpyDeviceToHost, current_stream()));
+    VB_TRY(sync_stream());   // (the draws are the caller's)
+    if (failed != 0) {
+        VB_FAIL(VB200_INTERNAL_ERROR, "the seeding kernel gave up on a bounded wait");
+    }
     *done = true;
-    return sync_stream();   // the draws are the caller's
+    return 0;
 }
 
 // centroids_dev[k x dim] and (optionally) picked_dev[k] on the device.  The generator and its
