@@ -70,6 +70,22 @@ def test_exact_batches_the_threshold_does_not_serve(engine, oracle, kind):
         assert np.array_equal(got[0], np.concatenate([o[0] for o in one]))
 
 
+# ---- distance chains --------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("metric", [0, 1])
+@pytest.mark.parametrize("dim", [4, 31, 32, 33, 100])
+@pytest.mark.parametrize("nq,nlist", [(1, 16), (15, 31), (16, 32), (17, 33), (33, 257), (640, 1000), (255, 1900)])
+def test_routing_by_chains(engine, oracle, metric, dim, nq, nlist):
+    nprobe = min(7, nlist)
+    c, q = mixture(31, nlist, dim, 9, 0.4), mixture(32, nq, dim, 9, 0.4)
+    ix = engine.IvfHandle(dim, metric, nlist, engine.QUANT_FP32)
+    ix.set_centroids(c)
+    got = ix.route(q, nprobe)
+    got = got[0] if isinstance(got, tuple) else got
+    want = oracle.route(q, c, nprobe, metric)
+    want = want[0] if isinstance(want, tuple) else want
+    assert np.array_equal(np.asarray(got), np.asarray(want))
+
+
 # ---- k-means ----------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("n,dim", [(16, 3), (2369, 31), (5000, 32), (5001, 33), (4000, 64), (4000, 65), (4000, 80), (4001, 81), (3000, 96),
                                    (3000, 129), (148 * 512, 8), (148 * 512 + 1, 8)])   # a row per thread, and one row more

@@ -2353,34 +2353,28 @@ route_sync_and_check(SearchWorkspace& ws) {
     return route_flag_check(word);
 }
 
-// out[(q, r)] = the distance chain between every query and every row (see route_dist_kernel).
+constexpr uint32_t ROUTE_MAX_DIM = 42496;   // longer rows have no scan: a row and its query's piece do not fit shared memory
+
+// out[(q, r)] = the distance chain between every query and every row (see row_chains_kernel).
 static int
 launch_row_chains(const float* queries, uint64_t nq, uint64_t q_stride, const float* rows, uint32_t n_rows, uint32_t dim, bool l2,
                   bool one_minus, float* out, uint64_t ld) {
-    const uint32_t chunks = (n_rows + RS_ROWS - 1) / RS_ROWS;
-    // As many queries per CTA as still leave two CTAs for every SM: a row fetched once serves them all.
-    uint32_t qn = 8;
-    while (qn > 1 && static_cast<uint64_t>(chunks) * ((nq + qn - 1) / qn) < 2ull * static_cast<uint32_t>(sm_count())) {
-        qn /= 2;
-    }
-    auto smem_of = [&](uint32_t n) { return RS_STAGES * RS_STAGE + static_cast<size_t>(n) * ((dim + 3) / 4 * 4) * sizeof(float); };
-    while (qn > 1 && smem_of(qn) > 100 * 1024) {
-        qn /= 2;
-    }
-    const size_t smem = smem_of(qn);
-    VB_CHECK_ARG(smem <= 220 * 1024, "dim = %u is too large for the routing kernel", dim);
-    const bool wide = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
+    VB_CHECK_ARG(dim <= ROUTE_MAX_DIM, "dim = %u is too large for the routing kernel", dim);
+    // 32 x 64 outputs per CTA where that makes two CTAs for every SM, else 16 x 32 (see row_chains_kernel)
+    auto tiles = [&](uint64_t m, uint64_t n) { return ((nq + m - 1) / m) * ((n_rows + n - 1) / n); };
+    const bool large = tiles(32, 64) >= 2ull * static_cast<uint32_t>(sm_count());
+    const uint32_t qn = large ? 32 : 16, rn = large ? 64 : 32;
+    const size_t smem = CHAIN_STAGES * static_cast<size_t>(qn + rn) * CHAIN_PITCH * sizeof(float);
+    const bool wide = dim % 4 == 0 && q_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(queries)) & 15) == 0;
     using Kernel = void (*)(const float*, uint32_t, uint64_t, const float*, uint32_t, uint32_t, int, float*, uint64_t);
-#define VB_ROW_CHAINS(QN)                                                                          \
-    (l2 ? (wide ? route_dist_kernel<true, QN, 16> : route_dist_kernel<true, QN, 4>)                \
-        : (wide ? route_dist_kernel<false, QN, 16> : route_dist_kernel<false, QN, 4>))
-    const Kernel kernel = qn == 8 ? VB_ROW_CHAINS(8) : (qn == 4 ? VB_ROW_CHAINS(4) : (qn == 2 ? VB_ROW_CHAINS(2) : VB_ROW_CHAINS(1)));
+#define VB_ROW_CHAINS(L2, T) (wide ? row_chains_kernel<L2, T, T, 16> : row_chains_kernel<L2, T, T, 4>)
+    const Kernel kernel = large ? (l2 ? VB_ROW_CHAINS(true, 4) : VB_ROW_CHAINS(false, 4)) : (l2 ? VB_ROW_CHAINS(true, 2) : VB_ROW_CHAINS(false, 2));
 #undef VB_ROW_CHAINS
     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
     const uint64_t slice = 65535ull * qn;   // (query tiles are the grid's second dimension)
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
         const uint64_t m = std::min(slice, nq - q0);
-        VB_LAUNCH(kernel, dim3(chunks, static_cast<uint32_t>((m + qn - 1) / qn)), RS_ROWS, smem, queries + q0 * q_stride,
+        VB_LAUNCH(kernel, dim3((n_rows + rn - 1) / rn, static_cast<uint32_t>((m + qn - 1) / qn)), CHAIN_THREADS, smem, queries + q0 * q_stride,
                   static_cast<uint32_t>(m), q_stride, rows, n_rows, dim, one_minus ? 1 : 0, out + q0 * ld, ld);
     }
     return 0;

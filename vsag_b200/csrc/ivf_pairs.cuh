@@ -3,7 +3,7 @@
 // When a list is probed by only a few queries of the batch there is nothing to gain from collecting the queries
 // of a list into a tile, and the passes that do it (count, prefix sums, work items, places), the bounds and the
 // second phase cost more than the rows.  Such a batch takes three or four launches here instead of fifteen:
-//   route_dist_kernel     every centroid distance, as the reference's chain (no candidates, no re-scoring)
+//   row_chains_kernel     every centroid distance, as the reference's chain (no candidates, no re-scoring)
 //   pairs_prepare_kernel  a CTA per query: its nprobe nearest lists, where each list's scores go, SQ8 weights
 //   pair_scan_kernel      a CTA per (pair, 128 rows): one score per row, written where the CTA above said
 //   scan_finalize_kernel  a CTA per query: the k best of its scores, exact re-scoring, rerank, labels
@@ -29,32 +29,111 @@ struct PairTable {
 };
 
 // out[(q, r)] for every row r of `rows` and query q: L2 = sum of fma(t, t, .), t = row - query; otherwise the
-// inner product chain, as it is (ONE_MINUS 0) or taken from one (1).  grid.x = row chunks, grid.y = query tiles.
-template <bool L2, int QN, int UNIT>
-__global__ void __launch_bounds__(RS_ROWS)
-route_dist_kernel(const float* __restrict__ queries, uint32_t nq, uint64_t q_stride, const float* __restrict__ rows, uint32_t n_rows,
+// inner product chain, as it is (ONE_MINUS 0) or taken from one (1).  Every chain is one thread's, over ascending dimensions.
+//
+// A tile of 8 TM queries x 16 TN rows per CTA, TM x TN chains a thread, both operands CHAIN_K dimensions at a time through shared
+// memory, CHAIN_STAGES deep.  Bound by the FMA pipe where there are CTAs for all SMs (4 x 4 chains: eight 16-byte reads of shared
+// memory per 64 steps); 2 x 2 chains where that leaves SMs without one, whose time is the chain's latency.  1000 x 960 outputs of
+// 960 dimensions: 197 us as a thread per row with eight queries (nine reads for 32 steps, two CTAs an SM), 77 now; 100 x 1024 of
+// 640: 27.5, 17 now.
+constexpr int CHAIN_THREADS = 128;
+constexpr uint32_t CHAIN_K = 32;
+constexpr int CHAIN_STAGES = 4;
+constexpr uint32_t CHAIN_PITCH = CHAIN_K + 4;   // floats between rows in shared memory: 16-byte reads of neighbouring rows meet no bank twice
+
+template <bool L2, int TM, int TN, int UNIT>
+__global__ void __launch_bounds__(CHAIN_THREADS)
+row_chains_kernel(const float* __restrict__ queries, uint32_t nq, uint64_t q_stride, const float* __restrict__ rows, uint32_t n_rows,
                   uint32_t dim, int one_minus, float* __restrict__ out, uint64_t ld) {
+    constexpr uint32_t M = 8 * TM, N = 16 * TN, ELEMS = UNIT / 4;
     extern __shared__ __align__(16) unsigned char smem[];
-    float* qs = reinterpret_cast<float*>(smem + RS_STAGES * RS_STAGE);
-    const uint32_t qpad = (dim + 3) / 4 * 4;
-    const uint32_t q0 = blockIdx.y * QN;
-    for (uint32_t i = threadIdx.x; i < QN * qpad; i += RS_ROWS) {
-        const uint32_t qi = i / qpad, d = i - qi * qpad;
-        qs[i] = (q0 + qi < nq && d < dim) ? __ldg(queries + (q0 + qi) * q_stride + d) : 0.f;
+    float* const stages = reinterpret_cast<float*>(smem);
+    const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
+    const uint32_t n0 = blockIdx.x * N, q0 = blockIdx.y * M;
+    const uint32_t steps = (dim + CHAIN_K - 1) / CHAIN_K;
+    auto request = [&](uint32_t step) {
+        if (step < steps) {
+            float* to = stages + step % CHAIN_STAGES * (M + N) * CHAIN_PITCH;
+            constexpr uint32_t PER_ROW = CHAIN_K / ELEMS;
+            for (uint32_t u = threadIdx.x; u < (M + N) * PER_ROW; u += CHAIN_THREADS) {
+                const uint32_t r = u / PER_ROW, k = u % PER_ROW * ELEMS, d = step * CHAIN_K + k;
+                const bool query = r < M;
+                const uint32_t at = query ? q0 + r : n0 + r - M;
+                const bool there = d < dim && at < (query ? nq : n_rows);
+                // (what is not there is zero: a step of it adds nothing to a chain)
+                const float* from = query ? queries + (there ? at * q_stride + d : 0) : rows + (there ? static_cast<uint64_t>(at) * dim + d : 0);
+                const uint32_t bytes = there ? UNIT : 0;
+                if (UNIT == 16) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(to + r * CHAIN_PITCH + k)), "l"(from), "r"(bytes)
+                                 : "memory");
+                } else {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(to + r * CHAIN_PITCH + k)), "l"(from), "r"(bytes)
+                                 : "memory");
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int s = 0; s < CHAIN_STAGES - 1; ++s) {
+        request(s);
     }
-    RowAcc<ROW_F32, L2, QN> acc;
-    row_stream<UNIT>(reinterpret_cast<const unsigned char*>(rows), static_cast<uint64_t>(dim) * 4, dim * 4, dim, n_rows, blockIdx.x,
-                     gridDim.x, smem, qs, qpad, acc, [&](uint64_t row, bool valid) {
-                         if (valid) {
+    float acc[TM][TN];
 #pragma unroll
-                             for (int i = 0; i < QN; ++i) {
-                                 if (q0 + i < nq) {
-                                     const float v = acc.acc[i];
-                                     out[(q0 + i) * ld + row] = (!L2 && one_minus != 0) ? __fsub_rn(1.0f, v) : v;
-                                 }
-                             }
-                         }
-                     });
+    for (int i = 0; i < TM; ++i) {
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            acc[i][j] = 0.f;
+        }
+    }
+    auto chain = [](float& a, float x, float q) {
+        if (L2) {
+            const float t = __fsub_rn(x, q);
+            a = fmaf(t, t, a);
+        } else {
+            a = fmaf(x, q, a);
+        }
+    };
+    for (uint32_t step = 0; step < steps; ++step) {
+        cp_async_wait_group<CHAIN_STAGES - 2>();
+        __syncthreads();   // this step's operands are here for everybody, and nobody reads the step before any more
+        request(step + CHAIN_STAGES - 1);
+        const float* a_at = stages + step % CHAIN_STAGES * (M + N) * CHAIN_PITCH;
+        const float* b_at = a_at + M * CHAIN_PITCH;
+#pragma unroll
+        for (uint32_t k = 0; k < CHAIN_K; k += 4) {
+            float4 a[TM], b[TN];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                a[i] = *reinterpret_cast<const float4*>(a_at + (ty + 8 * i) * CHAIN_PITCH + k);
+            }
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                b[j] = *reinterpret_cast<const float4*>(b_at + (tx + 16 * j) * CHAIN_PITCH + k);
+            }
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    chain(acc[i][j], b[j].x, a[i].x);
+                    chain(acc[i][j], b[j].y, a[i].y);
+                    chain(acc[i][j], b[j].z, a[i].z);
+                    chain(acc[i][j], b[j].w, a[i].w);
+                }
+            }
+        }
+    }
+    cp_async_wait_group<0>();
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const uint32_t q = q0 + ty + 8 * i;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const uint32_t row = n0 + tx + 16 * j;
+            if (q < nq && row < n_rows) {
+                out[q * ld + row] = (!L2 && one_minus != 0) ? __fsub_rn(1.0f, acc[i][j]) : acc[i][j];
+            }
+        }
+    }
 }
 
 struct PairsPrepare {
