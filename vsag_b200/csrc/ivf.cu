@@ -1703,115 +1703,74 @@ route_find_bin(const uint32_t* hist, uint32_t rank, uint32_t* s_bin, uint32_t* s
     __syncthreads();
 }
 
-// thr[q] = a score that at least ncand of query q's `sample` approximate scores (scores[q][0 .. sample))
-// do not exceed -- one of those scores, at most a few ranks above the ncand-th smallest -- plus a margin
-// of 1e-3 |q| max|c| that covers the rounding of the tensor-core scores on both sides: at least ncand
-// centroids score below it exactly, so every one of the query's ncand nearest centroids scores below
-// it approximately.  One CTA per query: two rounds of a 256-bin histogram over the range of the scores
-// still in question (bins follow the values' own range, so a narrow spread does not pile them into one
-// bin), then the largest score of the bins taken.
-// ROUTE_THR_PER_THREAD: scores a thread holds, sample / ROUTE_THREADS rounded up (sample <= 4096).
-template <int ROUTE_THR_PER_THREAD>
-__global__ void __launch_bounds__(ROUTE_THREADS)
-route_threshold_kernel(const float* __restrict__ scores, uint32_t sample, uint32_t ncand, const float* __restrict__ queries,
+// thr[q] = a score that at least `rank` of query q's `sample` approximate scores (scores[q][0 .. sample)) do not exceed, and at
+// most a sixteenth more, plus a margin of 1e-3 |q| max|c| that covers the rounding of the tensor-core scores on both
+// sides: the centroids that score below it exactly score below it approximately.  A warp per query holds the scores in
+// registers and halves the range of scores in question until that few are left over, which takes about ten counts of one
+// instruction per score (as a CTA per query with two rounds of a histogram 46 us for 10,000 queries and 1024 scores each; 18).
+// PER: scores a lane holds, a multiple of four; sample <= 32 PER, sample % 4 == 0.
+template <int PER>
+__global__ void __launch_bounds__(128)
+route_threshold_kernel(const float* __restrict__ scores, uint64_t nq, uint32_t sample, uint32_t rank, const float* __restrict__ queries,
                        uint32_t dim, const float* __restrict__ c_max_norm, float* __restrict__ thr) {
-    __shared__ uint32_t hist[256];
-    __shared__ float red[ROUTE_THREADS / 32];
-    __shared__ uint32_t s_bin, s_rank;
-    const uint64_t q = blockIdx.x;
-    const uint32_t tid = threadIdx.x;
-    float v[ROUTE_THR_PER_THREAD];
-    uint8_t bin1[ROUTE_THR_PER_THREAD];
-    float mn = INFINITY, mx = -INFINITY;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t q = static_cast<uint64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
+    if (q >= nq) {
+        return;
+    }
+    float v[PER];
+    const float4* src = reinterpret_cast<const float4*>(scores + q * sample);
 #pragma unroll
-    for (int i = 0; i < ROUTE_THR_PER_THREAD; ++i) {
-        const uint32_t c = tid + i * ROUTE_THREADS;
-        const float x = c < sample ? __ldg(scores + q * sample + c) : NAN;
-        v[i] = x;
-        if (x == x) {   // NaN scores take no part
-            mn = fminf(mn, x);
-            mx = fmaxf(mx, x);
-        }
+    for (int i = 0; i < PER / 4; ++i) {
+        const uint32_t at = i * 32 + lane;
+        const float4 w = at < sample / 4 ? __ldg(src + at) : make_float4(NAN, NAN, NAN, NAN);
+        v[4 * i] = w.x;
+        v[4 * i + 1] = w.y;
+        v[4 * i + 2] = w.z;
+        v[4 * i + 3] = w.w;
     }
     float qq = 0.f;
-    for (uint32_t d = tid; d < dim; d += ROUTE_THREADS) {
+    for (uint32_t d = lane; d < dim; d += 32) {
         const float x = __ldg(queries + q * dim + d);
         qq = fmaf(x, x, qq);
     }
-    // sum of the per-thread partial norms
-    for (int off = 16; off > 0; off >>= 1) {
-        qq += __shfl_xor_sync(0xffffffffu, qq, off);
+    float mn = INFINITY, mx = -INFINITY;   // (scores that are no numbers take no part)
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        mn = fminf(mn, v[i]);
+        mx = fmaxf(mx, v[i]);
     }
-    __shared__ float s_qq[ROUTE_THREADS / 32];
-    if ((tid & 31) == 0) {
-        s_qq[tid >> 5] = qq;
+    for (int o = 16; o > 0; o >>= 1) {
+        qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
-    mn = route_block_min(mn, red);
-    mx = route_block_max(mx, red);
-    float bound = mx;   // everything, when the scores do not spread (or there are fewer than ncand of them)
+    float bound = mx;   // everything, when the scores do not spread (or there are fewer than `rank` of them)
     if (mx > mn && mx < INFINITY && mn > -INFINITY) {
-        // first pass: bins over [mn, mx]
-        hist[tid] = 0;
-        __syncthreads();
-        const float scale1 = 255.0f / (mx - mn);
-#pragma unroll
-        for (int i = 0; i < ROUTE_THR_PER_THREAD; ++i) {
-            uint32_t b = 255;
-            if (v[i] == v[i]) {
-                const float t = (v[i] - mn) * scale1;
-                b = t >= 255.0f ? 255u : static_cast<uint32_t>(t);
-                atomicAdd(&hist[b], 1u);
+        float low = mn;   // fewer than `rank` scores are at or below it, or it is the smallest
+        for (int round = 0; round < 24; ++round) {
+            const float mid = low + 0.5f * (bound - low);
+            if (!(mid > low && mid < bound)) {
+                break;
             }
-            bin1[i] = static_cast<uint8_t>(b);
-        }
-        route_find_bin(hist, ncand, &s_bin, &s_rank);
-        const uint32_t b1 = s_bin, rank2 = s_rank;
-        // second pass: the scores of bin b1 alone, over their own range
-        float mn2 = INFINITY, mx2 = -INFINITY;
+            uint32_t count = 0;
 #pragma unroll
-        for (int i = 0; i < ROUTE_THR_PER_THREAD; ++i) {
-            if (v[i] == v[i] && bin1[i] == b1) {
-                mn2 = fminf(mn2, v[i]);
-                mx2 = fmaxf(mx2, v[i]);
+            for (int i = 0; i < PER; ++i) {
+                count += v[i] <= mid ? 1u : 0u;
             }
-        }
-        mn2 = route_block_min(mn2, red);
-        mx2 = route_block_max(mx2, red);
-        float pick = -INFINITY;   // the largest score taken from bin b1
-        if (mx2 > mn2) {
-            hist[tid] = 0;
-            __syncthreads();
-            const float scale2 = 255.0f / (mx2 - mn2);
-            uint8_t bin2[ROUTE_THR_PER_THREAD];
-#pragma unroll
-            for (int i = 0; i < ROUTE_THR_PER_THREAD; ++i) {
-                bin2[i] = 255;
-                if (v[i] == v[i] && bin1[i] == b1) {
-                    const float t = (v[i] - mn2) * scale2;
-                    const uint32_t b = t >= 255.0f ? 255u : static_cast<uint32_t>(t);
-                    bin2[i] = static_cast<uint8_t>(b);
-                    atomicAdd(&hist[b], 1u);
+            count = __reduce_add_sync(0xffffffffu, count);
+            if (count < rank) {
+                low = mid;
+            } else {
+                bound = mid;
+                if (count <= rank + rank / 16) {
+                    break;
                 }
             }
-            route_find_bin(hist, rank2, &s_bin, &s_rank);
-            const uint32_t b2 = s_bin;
-#pragma unroll
-            for (int i = 0; i < ROUTE_THR_PER_THREAD; ++i) {
-                if (v[i] == v[i] && bin1[i] == b1 && bin2[i] <= b2) {
-                    pick = fmaxf(pick, v[i]);
-                }
-            }
-        } else {
-            pick = mx2;   // the bin holds one value (possibly many times)
         }
-        bound = route_block_max(pick, red);
     }
-    if (tid == 0) {
-        float total = 0.f;
-        for (int w = 0; w < ROUTE_THREADS / 32; ++w) {
-            total += s_qq[w];
-        }
-        thr[q] = bound + 1e-3f * sqrtf(total) * __ldg(c_max_norm);
+    if (lane == 0) {
+        thr[q] = bound + 1e-3f * sqrtf(qq) * __ldg(c_max_norm);
     }
 }
 
@@ -2471,9 +2430,8 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
             // candidate lists overflowed is answered exactly by route_pick_kernel itself.
             VB_TRY(tc_scores(ix->tc, a, bs, 3, alpha, bias, ws.scores.ptr, sample, route_flag));
             VB_TRY(ws.route_thr.reserve(nq));
-            auto thr_kernel = sample <= 4 * ROUTE_THREADS ? route_threshold_kernel<4>
-                                                          : (sample <= 8 * ROUTE_THREADS ? route_threshold_kernel<8> : route_threshold_kernel<16>);
-            VB_LAUNCH(thr_kernel, static_cast<uint32_t>(nq), ROUTE_THREADS, 0, ws.scores.ptr, sample, rank,
+            auto thr_kernel = sample <= 1024 ? route_threshold_kernel<32> : (sample <= 2048 ? route_threshold_kernel<64> : route_threshold_kernel<128>);
+            VB_LAUNCH(thr_kernel, static_cast<uint32_t>((nq + 3) / 4), 128, 0, ws.scores.ptr, nq, sample, rank,
                       q_dev, ix->dim, ix->c_max_norm.ptr, ws.route_thr.ptr);
             uint32_t lists = 0, cap = 0;
             bool overflow = false;
