@@ -86,6 +86,22 @@ def test_routing_by_chains(engine, oracle, metric, dim, nq, nlist):
     assert np.array_equal(np.asarray(got), np.asarray(want))
 
 
+@pytest.mark.parametrize("nq,nlist", [(20, 900), (300, 1500)])      # by distances, and by scores that are re-scored
+@pytest.mark.parametrize("metric", [0, 1])
+@pytest.mark.parametrize("dim", [18, 32])                           # rows of 8- and of 16-byte alignment
+def test_routing_with_coinciding_centroids(engine, oracle, nq, nlist, metric, dim):
+    """More lists tie with the last that is wanted than a warp collects: the lowest numbers among them are probed."""
+    nprobe = 40
+    c, q = mixture(33, nlist, dim, 9, 0.4), mixture(34, nq, dim, 9, 0.4)
+    c[100:800] = c[100]
+    q[::2] = c[100]
+    ix = engine.IvfHandle(dim, metric, nlist, engine.QUANT_FP32)
+    ix.set_centroids(c)
+    got, want = ix.route(q, nprobe), oracle.route(q, c, nprobe, metric)
+    got, want = (v[0] if isinstance(v, tuple) else v for v in (got, want))
+    assert np.array_equal(np.asarray(got), np.asarray(want))
+
+
 # ---- k-means ----------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("n,dim", [(16, 3), (2369, 31), (5000, 32), (5001, 33), (4000, 64), (4000, 65), (4000, 80), (4001, 81), (3000, 96),
                                    (3000, 129), (148 * 512, 8), (148 * 512 + 1, 8)])   # a row per thread, and one row more

@@ -342,4 +342,189 @@ block_sort_to(uint64_t* keys, uint32_t count, uint32_t keep, uint64_t* out) {
     __syncthreads();
 }
 
+// ---- the same by one warp -----------------------------------------------------------------------------------
+// For a few dozen values out of some thousands a CTA spends most of its time in its forty barriers; a warp has none, keeps the
+// group minima in registers and finds the bound by halving the range of values in question (a count over the registers and one
+// reduction per step).
+constexpr uint32_t WARP_SELECT_MAX = 128;    // wanted at most
+constexpr uint32_t WARP_SELECT_CAP = 256;    // collected at most
+
+// Bitonic sort of 32 * R keys held R per lane (element e = 32 * r + lane lives in key[r] of lane e % 32):
+// compare-exchanges inside a lane when the partner is 32 or more elements away, shuffles otherwise; ascending.
+template <int R>
+__device__ __forceinline__ void
+warp_sort_registers(uint64_t (&key)[R], uint32_t lane) {
+#pragma unroll
+    for (uint32_t size = 2; size <= 32u * R; size <<= 1) {
+#pragma unroll
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= 32) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int pr = r ^ static_cast<int>(stride >> 5);
+                    if (pr > r) {
+                        const bool up = (((static_cast<uint32_t>(r) << 5) | lane) & size) == 0;
+                        const uint64_t a = key[r], b = key[pr];
+                        if ((a > b) == up) {
+                            key[r] = b;
+                            key[pr] = a;
+                        }
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint32_t e = (static_cast<uint32_t>(r) << 5) | lane;
+                    const uint64_t mine = key[r];
+                    const uint64_t other = __shfl_xor_sync(0xffffffffu, mine, stride);
+                    const bool up = (e & size) == 0;
+                    const bool lower = (lane & stride) == 0;
+                    const bool take_min = lower == up;
+                    key[r] = take_min ? (mine < other ? mine : other) : (mine > other ? mine : other);
+                }
+            }
+        }
+    }
+}
+
+// buf[0 .. 32 R) sorted ascending through registers (one warp).
+template <int R>
+__device__ __noinline__ void
+warp_sort_buffer(uint64_t* buf, uint32_t lane) {
+    uint64_t key[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        key[r] = buf[r * 32 + lane];
+    }
+    warp_sort_registers<R>(key, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        buf[r * 32 + lane] = key[r];
+    }
+    __syncwarp();
+}
+
+// Visits the n values of load(i) in order, 32 at a time with eight loads of a lane together: visit(i, value), value 0xFFFFFFFF for i >= n.
+template <typename Load, typename Visit>
+__device__ __forceinline__ void
+warp_walk(const Load& load, uint32_t n, uint32_t lane, Visit visit) {
+    for (uint32_t i0 = 0; i0 < n; i0 += 256) {
+        uint32_t u[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t i = i0 + j * 32 + lane;
+            u[j] = i < n ? load(i) : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            if (i0 + j * 32 < n) {
+                visit(i0 + j * 32 + lane, u[j], j);
+            }
+        }
+    }
+}
+
+// The smallest value in m[] of all lanes that `k` of them are at or below, or one a few ranks above it; ORDERED_INF when no more than k
+// are numbers.
+template <int PER>
+__device__ __forceinline__ uint32_t
+warp_bound(const uint32_t (&m)[PER], uint32_t k) {
+    uint32_t low = 0xFFFFFFFFu, high = 0, have = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        if (m[j] <= ORDERED_INF) {
+            low = min(low, m[j]);
+            high = max(high, m[j]);
+            ++have;
+        }
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
+    have = __reduce_add_sync(0xffffffffu, have);
+    if (have <= k) {
+        return ORDERED_INF;
+    }
+    while (low < high) {   // `k` values are at or below `high`, fewer are below `low`
+        const uint32_t mid = low + (high - low) / 2;
+        uint32_t count = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            count += m[j] <= mid ? 1u : 0u;
+        }
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (count < k) {
+            low = mid + 1;
+        } else {
+            high = mid;
+            if (count <= k + k / 16) {
+                break;
+            }
+        }
+    }
+    return high;
+}
+
+// Values of load(0 .. n) at or below t, as (value << 32 | payload(i)) in keys[WARP_SELECT_CAP]; how many there are (more than fit: the
+// first ones are there).
+template <typename Load, typename Payload>
+__device__ __forceinline__ uint32_t
+warp_collect(const Load& load, const Payload& payload, uint32_t n, uint32_t t, uint64_t* keys, uint32_t lane) {
+    uint32_t count = 0;
+    warp_walk(load, n, lane, [&](uint32_t i, uint32_t u, uint32_t) {
+        const bool take = u <= t && u <= ORDERED_INF;
+        const uint32_t mask = __ballot_sync(0xffffffffu, take);
+        if (mask != 0) {
+            const uint32_t at = count + __popc(mask & ((1u << lane) - 1u));
+            if (take && at < WARP_SELECT_CAP) {
+                keys[at] = (static_cast<uint64_t>(u) << 32) | payload(i);
+            }
+            count += __popc(mask);
+        }
+    });
+    __syncwarp();
+    return count;
+}
+
+// A few more than the k smallest of the n values, unsorted in keys[WARP_SELECT_CAP]; how many, or more than WARP_SELECT_CAP when too many
+// crowd at the k-th.  No value that was not collected is below *left (ORDERED_INF: all were collected).  k <= WARP_SELECT_MAX.
+template <typename Load, typename Payload>
+__device__ __forceinline__ uint32_t
+warp_select(const Load& load, const Payload& payload, uint32_t n, uint32_t k, uint64_t* keys, uint32_t lane, uint32_t* left) {
+    uint32_t t;
+    if (k <= 40) {   // 128 groups: three or more per wanted value
+        uint32_t m[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
+        warp_walk(load, n, lane, [&](uint32_t, uint32_t u, uint32_t j) { m[j & 3u] = min(m[j & 3u], u); });
+        t = n <= k ? ORDERED_INF : warp_bound(m, k);
+    } else {         // 256, two or more
+        uint32_t m[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            m[j] = 0xFFFFFFFFu;
+        }
+        warp_walk(load, n, lane, [&](uint32_t, uint32_t u, uint32_t j) { m[j & 7u] = min(m[j & 7u], u); });
+        t = n <= k ? ORDERED_INF : warp_bound(m, k);
+    }
+    *left = t;
+    return warp_collect(load, payload, n, t, keys, lane);
+}
+
+// keys[0 .. count) ascending, count <= WARP_SELECT_CAP (one warp).
+__device__ __forceinline__ void
+warp_sort(uint64_t* keys, uint32_t count, uint32_t lane) {
+    const uint32_t padded = count <= 32 ? 32u : (count <= 64 ? 64u : (count <= 128 ? 128u : 256u));
+    for (uint32_t i = count + lane; i < padded; i += 32) {
+        keys[i] = KEY_INF;
+    }
+    __syncwarp();
+    if (padded == 32) {
+        warp_sort_buffer<1>(keys, lane);
+    } else if (padded == 64) {
+        warp_sort_buffer<2>(keys, lane);
+    } else if (padded == 128) {
+        warp_sort_buffer<4>(keys, lane);
+    } else {
+        warp_sort_buffer<8>(keys, lane);
+    }
+}
+
 }  // namespace vb200

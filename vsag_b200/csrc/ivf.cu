@@ -1886,68 +1886,21 @@ route_exact_score4(const float* __restrict__ qs, const float* const (&c)[4], uin
 // that holds the ncand-th and everything below it, a few more than ncand keys), sorted as 64-bit keys so
 // that equal scores keep the lower list id; only if that set does not fit the small sort buffer (a
 // pile of equal scores) are all candidates sorted.
-// Bitonic sort of 32 * R keys held R per lane (element e = 32 * r + lane lives in key[r] of lane e % 32):
-// compare-exchanges inside a lane when the partner is 32 or more elements away, shuffles otherwise; ascending.
-template <int R>
-__device__ __forceinline__ void
-warp_sort_registers(uint64_t (&key)[R], uint32_t lane) {
-#pragma unroll
-    for (uint32_t size = 2; size <= 32u * R; size <<= 1) {
-#pragma unroll
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= 32) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int pr = r ^ static_cast<int>(stride >> 5);
-                    if (pr > r) {
-                        const bool up = (((static_cast<uint32_t>(r) << 5) | lane) & size) == 0;
-                        const uint64_t a = key[r], b = key[pr];
-                        if ((a > b) == up) {
-                            key[r] = b;
-                            key[pr] = a;
-                        }
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const uint32_t e = (static_cast<uint32_t>(r) << 5) | lane;
-                    const uint64_t mine = key[r];
-                    const uint64_t other = __shfl_xor_sync(0xffffffffu, mine, stride);
-                    const bool up = (e & size) == 0;
-                    const bool lower = (lane & stride) == 0;
-                    const bool take_min = lower == up;
-                    key[r] = take_min ? (mine < other ? mine : other) : (mine > other ? mine : other);
-                }
-            }
-        }
-    }
-}
-
-// buf[0 .. 32 R) sorted ascending through registers (one warp).
-template <int R>
-__device__ __noinline__ void
-warp_sort_buffer(uint64_t* buf, uint32_t lane) {
-    uint64_t key[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        key[r] = buf[r * 32 + lane];
-    }
-    warp_sort_registers<R>(key, lane);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        buf[r * 32 + lane] = key[r];
-    }
-    __syncwarp();
-}
-
 // route_pick_kernel for the common case, one warp per query and no block-wide barrier: a query whose lists hold at
-// most 512 candidates (288 expected for nprobe 64) has them sorted through registers, the
-// ncand <= 128 best re-scored exactly, one chain per lane, and sorted again.  handled[q] = 1 tells route_pick_kernel
+// most 512 candidates (288 expected for nprobe 64) has the ncand <= 128 best re-scored exactly, one chain per lane, and sorted
+// through registers.  handled[q] = 1 tells route_pick_kernel
 // (launched afterwards over all queries) to leave the query alone.
 constexpr uint32_t ROUTE_WARP_KEYS = 512;
+constexpr uint32_t ROUTE_WARP_KEPT = 256;   // of them after the bound (more: sorted before any row is fetched)
+constexpr int ROUTE_PICK_WARPS = 4;
 
-__global__ void __launch_bounds__(256, 5)   // 40 warps per SM: the sort's registers just fit
+__host__ __device__ inline size_t
+route_warp_bytes(uint32_t dim) {
+    const size_t rows = ROUTE_WARP_KEPT * sizeof(uint64_t) + WARP_ROWS_BYTES, keys = ROUTE_WARP_KEYS * sizeof(uint64_t);
+    return (rows > keys ? rows : keys) + (static_cast<size_t>(dim) + 3) / 4 * 16;
+}
+
+__global__ void __launch_bounds__(ROUTE_PICK_WARPS * 32)
 route_pick_warp_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t dim, const float* __restrict__ centroids,
                        const uint64_t* __restrict__ lists_keys, const uint32_t* __restrict__ lists_cnt, uint32_t lists,
                        uint32_t cap, uint32_t ncand, uint32_t nprobe, int metric, int32_t* __restrict__ probes,
@@ -1958,9 +1911,11 @@ route_pick_warp_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t 
     if (q >= nq) {
         return;
     }
-    uint64_t* buf = reinterpret_cast<uint64_t*>(smem_raw) + static_cast<size_t>(warp) * ROUTE_WARP_KEYS;
-    float* qs = reinterpret_cast<float*>(reinterpret_cast<uint64_t*>(smem_raw) + static_cast<size_t>(blockDim.x >> 5) * ROUTE_WARP_KEYS) +
-                static_cast<size_t>(warp) * dim;
+    // the stages of the exact distances take the place of the candidates that were not kept
+    unsigned char* const mine = smem_raw + warp * route_warp_bytes(dim);
+    uint64_t* buf = reinterpret_cast<uint64_t*>(mine);
+    unsigned char* stages = mine + ROUTE_WARP_KEPT * sizeof(uint64_t);
+    float* qs = reinterpret_cast<float*>(mine + route_warp_bytes(dim)) - (dim + 3) / 4 * 4;
     // exclusive prefix of the (clamped) list counts, two lists per lane
     const uint32_t l0 = 2 * lane, l1 = 2 * lane + 1;
     uint32_t c0 = l0 < lists ? lists_cnt[q * lists + l0] : 0u;
@@ -2001,72 +1956,55 @@ route_pick_warp_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t 
         }
     }
     __syncwarp();
-    // Only the ncand best are wanted, so most of the keys need no sorting: a pivot from a 32-key sample -- the key
-    // at 1.6 times the rank that would cut off ncand, plus two -- is counted against all keys, and when between
-    // ncand and 256 keys lie at or below it those alone are compacted to the front and sorted.  The set of the
-    // ncand smallest is the same either way (keys are distinct: the list id is their low word).
-    uint32_t n_keys = total;
-    if (total > 128) {
-        uint64_t sample[1] = {buf[(lane * total) >> 5]};
-        warp_sort_registers<1>(sample, lane);
-        uint32_t r = (ncand * 32u * 8u / 5u) / total + 2u;
-        r = r > 31u ? 31u : r;
-        const uint64_t pivot = __shfl_sync(0xffffffffu, sample[0], r);
-        uint32_t below = 0;
-        for (uint32_t i = lane; i < ROUTE_WARP_KEYS; i += 32) {
-            below += __popc(__ballot_sync(0xffffffffu, i < total && buf[i] <= pivot));
-        }
-        if (below >= ncand && below <= 256) {
-            uint32_t cnt = 0;
-            for (uint32_t i = lane; i < ROUTE_WARP_KEYS; i += 32) {   // all lanes take the same number of trips
-                const uint64_t key = i < total ? buf[i] : KEY_INF;
-                const bool keep = key <= pivot && i < total;
-                const uint32_t mask = __ballot_sync(0xffffffffu, keep);
-                __syncwarp();
-                if (keep) {
-                    buf[cnt + __popc(mask & ((1u << lane) - 1u))] = key;   // at or before its own place
-                }
-                cnt += __popc(mask);
-                __syncwarp();
-            }
-            const uint32_t pad = cnt <= 128 ? 128u : 256u;
-            for (uint32_t i = cnt + lane; i < pad; i += 32) {
-                buf[i] = KEY_INF;
-            }
-            __syncwarp();
-            n_keys = cnt;
-        }
+    // The ncand best of them, or a few more: those at or below a score that ncand of them reach.
+    uint64_t key[ROUTE_WARP_KEYS / 32];
+    uint32_t value[ROUTE_WARP_KEYS / 32];
+#pragma unroll
+    for (uint32_t j = 0; j < ROUTE_WARP_KEYS / 32; ++j) {
+        key[j] = buf[j * 32 + lane];
+        value[j] = static_cast<uint32_t>(key[j] >> 32);
     }
-    if (n_keys <= 128) {
-        warp_sort_buffer<4>(buf, lane);
-    } else if (n_keys <= 256) {
-        warp_sort_buffer<8>(buf, lane);
-    } else {
-        warp_sort_buffer<16>(buf, lane);
+    __syncwarp();
+    const uint32_t bound = warp_bound(value, ncand);
+    uint32_t count = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < ROUTE_WARP_KEYS / 32; ++j) {
+        const bool keep = value[j] <= bound && key[j] != KEY_INF;
+        const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            buf[count + __popc(mask & ((1u << lane) - 1u))] = key[j];
+        }
+        count += __popc(mask);
     }
-    // exact distances of the ncand best by approximate score, one chain per lane, dimensions ascending
+    __syncwarp();
+    if (count > ROUTE_WARP_KEPT) {   // (that many tie at the bound)
+        if (lane == 0) {
+            handled[q] = 0;
+        }
+        return;
+    }
+    if (count > 128) {
+        warp_sort(buf, count, lane);
+        count = ncand;
+    }
+    // exact distances, one chain per lane, dimensions ascending
+    warp_centroid_distances(centroids, dim, metric == VB200_METRIC_L2, qs, count, buf, stages, lane);
     uint64_t exact[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const uint32_t e = r * 32 + lane;
-        uint64_t mine = KEY_INF;
-        if (e < ncand && e < n_keys) {
-            const uint32_t list = static_cast<uint32_t>(buf[e]);
-            const float s = route_exact_score(qs, centroids + static_cast<uint64_t>(list) * dim, dim, metric);
-            mine = make_key(s, list);
-        }
-        exact[r] = mine;
+        exact[r] = e < count ? buf[e] : KEY_INF;
     }
     warp_sort_registers<4>(exact, lane);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const uint32_t i = r * 32 + lane;
         if (i < nprobe) {
-            const uint64_t key = exact[r];
+            const uint64_t best = exact[r];
             const uint64_t o = q * nprobe + i;
-            probes[o] = key == KEY_INF ? -1 : static_cast<int32_t>(static_cast<uint32_t>(key));
+            probes[o] = best == KEY_INF ? -1 : static_cast<int32_t>(static_cast<uint32_t>(best));
             if (probe_dists != nullptr) {
-                probe_dists[o] = key == KEY_INF ? INFINITY : ordered_to_float(static_cast<uint32_t>(key >> 32));
+                probe_dists[o] = best == KEY_INF ? INFINITY : ordered_to_float(static_cast<uint32_t>(best >> 32));
             }
         }
     }
@@ -2347,6 +2285,23 @@ routes_on_tensor_cores(const vb200_ivf* ix, uint64_t nq) {
     return tensor_cores_enabled() && nq >= 256 && ix->nlist >= 1024;
 }
 
+// The step between routing scores and the scan: a warp per query, or a CTA where it selects more than a warp does, or looks
+// for lists that the caller named twice.
+static int
+launch_prepare(const PairsPrepare& p, uint64_t nq) {
+    const uint32_t wanted = p.scores != nullptr ? p.ncand : p.nprobe;
+    const size_t query = p.scores != nullptr ? p.dim * sizeof(float) : 0;
+    const size_t warp_smem = PREPARE_WARPS * prepare_warp_bytes(p.scores != nullptr, p.dim);
+    if (wanted <= WARP_SELECT_MAX && p.nprobe <= WARP_SELECT_MAX && p.repeats == nullptr && warp_smem <= 64 * 1024) {
+        VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_warps_kernel), warp_smem));
+        VB_LAUNCH(pairs_prepare_warps_kernel, static_cast<uint32_t>((nq + PREPARE_WARPS - 1) / PREPARE_WARPS), PREPARE_WARPS * 32, warp_smem, p, nq);
+        return 0;
+    }
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_kernel), query));
+    VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, query, p);
+    return 0;
+}
+
 // Exact routing.  prepare (optional): what pairs_prepare_kernel is to do beyond routing; *prepared tells whether it
 // was done here (the threshold path leaves it to the caller).
 static int
@@ -2382,7 +2337,6 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
     pp.probe_dists = dists_dev;
     const size_t route_smem = ix->dim * sizeof(float);
     VB_CHECK_ARG(route_smem <= 180 * 1024, "dim = %u is too large for the routing kernel", ix->dim);
-    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_kernel), route_smem));
     if (routes_on_tensor_cores(ix, nq)) {
         const uint32_t chunks = (ix->dim + TC_KC - 1) / TC_KC;
         if (!ix->c_tiled) {
@@ -2446,11 +2400,11 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
                 // queries with few candidates (nearly all) are answered by a warp each; the block-per-query kernel
                 // takes what is left
                 const uint8_t* handled = nullptr;
-                const size_t warp_smem = 8 * (ROUTE_WARP_KEYS * sizeof(uint64_t) + ix->dim * sizeof(float));
+                const size_t warp_smem = ROUTE_PICK_WARPS * route_warp_bytes(ix->dim);
                 if (ncand <= 128 && nprobe <= 128 && warp_smem <= 200 * 1024) {
                     VB_TRY(ws.route_handled.reserve(nq));
                     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(route_pick_warp_kernel), warp_smem));
-                    VB_LAUNCH(route_pick_warp_kernel, static_cast<uint32_t>((nq + 7) / 8), 256, warp_smem, q_dev, nq, ix->dim,
+                    VB_LAUNCH(route_pick_warp_kernel, static_cast<uint32_t>((nq + ROUTE_PICK_WARPS - 1) / ROUTE_PICK_WARPS), ROUTE_PICK_WARPS * 32, warp_smem, q_dev, nq, ix->dim,
                               ix->centroids.ptr, ws.route_keys.ptr, ws.route_cnt.ptr, lists, cap, ncand, nprobe, ix->metric,
                               probes_dev, dists_dev, ws.route_handled.ptr);
                     handled = ws.route_handled.ptr;
@@ -2477,7 +2431,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
                              l2 ? ix->c_sq.ptr : nullptr, ws.scores.ptr, ld, route_flag));
             PairsPrepare part = pp.from(q0);
             part.scores = ws.scores.ptr;
-            VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(m), PAIR_THREADS, route_smem, part);
+            VB_TRY(launch_prepare(part, m));
         }
         return 0;
     } else {
@@ -2491,7 +2445,7 @@ ivf_route_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe
             PairsPrepare part = pp.from(b);
             part.dist = ws.scores.ptr;
             part.ld = nlist;
-            VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(n), PAIR_THREADS, 0, part);
+            VB_TRY(launch_prepare(part, n));
         }
         return 0;
     }
@@ -3454,7 +3408,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         routed_on_tensor_cores = routes_on_tensor_cores(ix, nq);
     }
     if (!prepared) {
-        VB_LAUNCH(pairs_prepare_kernel, static_cast<uint32_t>(nq), PAIR_THREADS, 0, pp);
+        VB_TRY(launch_prepare(pp, nq));
     }
     const float* q_scan = q_dev;
     if (ix->quant == VB200_QUANT_RABITQ) {

@@ -161,7 +161,11 @@ struct PairsPrepare {
     // fp32 / bf16 / fp16 tiles (null: none): the query as operand rows of the tile scan, [nq][2 or 1][term_dims] 16-bit
     uint16_t* terms;
     uint32_t term_dims;       // a multiple of 64, zero past dim
-    int term_fmt;             // ROW_F32: bf16 hi and lo terms, ROW_BF16 / ROW_FP16: the codes
+    int term_fmt;             // ROW_F32, ROW_F32_SPLIT: bf16 hi and lo terms, ROW_BF16 / ROW_FP16: the codes
+    __host__ __device__ uint32_t
+    term_count() const {
+        return term_fmt == ROW_F32 || term_fmt == ROW_F32_SPLIT ? 2 : 1;
+    }
     // The same for the queries from q0 on (dist and scores are the caller's to set).
     PairsPrepare
     from(uint64_t q0) const {
@@ -182,7 +186,7 @@ struct PairsPrepare {
             p.qa += q0;
         }
         if (p.terms != nullptr) {
-            p.terms += q0 * term_dims * (term_fmt == ROW_F32 ? 2 : 1);
+            p.terms += q0 * term_dims * term_count();
         }
         return p;
     }
@@ -220,6 +224,43 @@ pair_block_max(float v, float* part) {
         v = fmaxf(v, part[w]);
     }
     return v;
+}
+
+// The query as operand rows of the tile scan, by `threads` threads.
+__device__ __forceinline__ void
+pair_query_terms(const PairsPrepare& p, uint64_t q, const float* src, uint32_t thread, uint32_t threads) {
+    uint16_t* t = p.terms + q * p.term_dims * p.term_count();
+    for (uint32_t e = thread; e < p.term_dims; e += threads) {
+        if (p.term_count() == 2) {
+            // converted rows: place e of a piece of 64, unit e / 8, holds dimensions 4 u .. + 3 and 32 + 4 u .. + 3 (tile_scan_kernel)
+            const uint32_t u = (e & 63u) >> 3, i = e & 7u;
+            const uint32_t d = p.term_fmt == ROW_F32_SPLIT ? e : (e & ~63u) + (i < 4 ? 4 * u + i : 28 + 4 * u + i);
+            const float v = d < p.dim ? __ldg(src + d) : 0.f;
+            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+            t[e] = __bfloat16_as_ushort(hi);
+            t[p.term_dims + e] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(hi)));
+        } else if (e >= p.dim) {
+            t[e] = 0;
+        } else {
+            t[e] = p.term_fmt == ROW_BF16 ? half_encode<SCAN_FMT_BF16>(__ldg(src + e)) : half_encode<SCAN_FMT_FP16>(__ldg(src + e));
+        }
+    }
+}
+
+// The int8 terms of a query's SQ8 weights, s = their scale.
+__device__ __forceinline__ void
+pair_query_weights(const PairsPrepare& p, uint64_t q, const float* src, float s, uint32_t thread, uint32_t threads) {
+    int8_t* t = p.qw8 + q * 3 * p.qstride;
+    for (uint32_t d = thread; d < p.qstride; d += threads) {
+        const float u = d < p.dim ? __ldg(src + d) * __ldg(p.scale + d) / s : 0.f;
+        const float t1 = fminf(fmaxf(rintf(u), -127.f), 127.f);
+        const float v2 = (u - t1) * 254.0f;
+        const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
+        const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
+        t[d] = static_cast<int8_t>(static_cast<int>(t1));
+        t[p.qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
+        t[2 * p.qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
+    }
 }
 
 __global__ void __launch_bounds__(PAIR_THREADS)
@@ -306,22 +347,7 @@ pairs_prepare_kernel(const PairsPrepare p) {
     }
     const float* src = p.queries + q * p.dim;
     if (p.terms != nullptr) {
-        uint16_t* t = p.terms + q * p.term_dims * (p.term_fmt == ROW_F32 ? 2 : 1);
-        for (uint32_t e = threadIdx.x; e < p.term_dims; e += PAIR_THREADS) {
-            if (p.term_fmt == ROW_F32) {
-                // place e of a piece of 64: unit e / 8 holds dimensions 4 u .. + 3 and 32 + 4 u .. + 3 (tile_scan_kernel)
-                const uint32_t u = (e & 63u) >> 3, i = e & 7u;
-                const uint32_t d = (e & ~63u) + (i < 4 ? 4 * u + i : 28 + 4 * u + i);
-                const float v = d < p.dim ? __ldg(src + d) : 0.f;
-                const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-                t[e] = __bfloat16_as_ushort(hi);
-                t[p.term_dims + e] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(hi)));
-            } else if (e >= p.dim) {
-                t[e] = 0;
-            } else {
-                t[e] = p.term_fmt == ROW_BF16 ? half_encode<SCAN_FMT_BF16>(__ldg(src + e)) : half_encode<SCAN_FMT_FP16>(__ldg(src + e));
-            }
-        }
+        pair_query_terms(p, q, src, threadIdx.x, PAIR_THREADS);
     }
     if (p.qw8 == nullptr) {
         return;
@@ -337,18 +363,167 @@ pairs_prepare_kernel(const PairsPrepare p) {
     qm = pair_block_sum(qm, part);
     wmax = pair_block_max(wmax, part);
     const float s = wmax > 0.f && wmax < INFINITY ? wmax / 127.0f : 1.0f;
-    int8_t* t = p.qw8 + q * 3 * p.qstride;
-    for (uint32_t d = threadIdx.x; d < p.qstride; d += PAIR_THREADS) {
-        const float u = d < p.dim ? __ldg(src + d) * __ldg(p.scale + d) / s : 0.f;
-        const float t1 = fminf(fmaxf(rintf(u), -127.f), 127.f);
-        const float v2 = (u - t1) * 254.0f;
-        const float t2 = fminf(fmaxf(rintf(v2), -127.f), 127.f);
-        const float t3 = fminf(fmaxf(rintf((v2 - t2) * 254.0f), -127.f), 127.f);
-        t[d] = static_cast<int8_t>(static_cast<int>(t1));
-        t[p.qstride + d] = static_cast<int8_t>(static_cast<int>(t2));
-        t[2 * p.qstride + d] = static_cast<int8_t>(static_cast<int>(t3));
-    }
+    pair_query_weights(p, q, src, s, threadIdx.x, PAIR_THREADS);
     if (threadIdx.x == 0) {
+        p.qscale[q] = s;
+        p.qa[q] = p.metric == VB200_METRIC_L2 ? fmaf(-2.0f, qm, qq) : 1.0f - qm;
+    }
+}
+
+// pairs_prepare_kernel with a warp per query, for routing that selects WARP_SELECT_MAX lists or candidates at most and lists that are
+// distinct (p.repeats null): no barriers.  1000 queries against 1024 lists, 40 candidates: 32 us with a CTA per query, 20 this way; 4096 lists,
+// 72 candidates of 960 dimensions: 122, 97.
+// Dynamic shared memory per warp: [WARP_SELECT_CAP] keys, and the stages of warp_rows and the query where candidates are re-scored.
+constexpr int PREPARE_WARPS = 2;
+
+__host__ __device__ inline size_t
+prepare_warp_bytes(bool rescore, uint32_t dim) {
+    return WARP_SELECT_CAP * sizeof(uint64_t) + (rescore ? WARP_ROWS_BYTES + (static_cast<size_t>(dim) + 3) / 4 * 16 : 0);
+}
+
+// The exact distances of the centroids named by the low words of keys[0 .. count), as keys (one warp).
+__device__ __forceinline__ void
+warp_centroid_distances(const float* centroids, uint32_t dim, bool l2, const float* qs, uint32_t count, uint64_t* keys, unsigned char* stages,
+                        uint32_t lane) {
+    if (dim % 4 != 0 || (reinterpret_cast<uintptr_t>(centroids) & 15u) != 0) {   // rows that are not 16-byte aligned
+        for (uint32_t i = lane; i < count; i += 32) {
+            const uint32_t l = static_cast<uint32_t>(keys[i]);
+            keys[i] = make_key(row_exact_distance(centroids + static_cast<uint64_t>(l) * dim, qs, dim, l2), l);
+        }
+        __syncwarp();
+        return;
+    }
+    const auto row = [&](uint32_t i) { return reinterpret_cast<const unsigned char*>(centroids + static_cast<uint64_t>(static_cast<uint32_t>(keys[i])) * dim); };
+    // (a key is replaced when its batch of rows is done and its row has been read)
+    if (l2) {
+        RowAcc<ROW_F32, true, 1> acc;
+        warp_rows(count, row, dim * 4, dim, qs, 0, stages, lane, acc,
+                  [&](uint32_t i, const auto& a) { keys[i] = make_key(a.acc[0], static_cast<uint32_t>(keys[i])); });
+    } else {
+        RowAcc<ROW_F32, false, 1> acc;
+        warp_rows(count, row, dim * 4, dim, qs, 0, stages, lane, acc,
+                  [&](uint32_t i, const auto& a) { keys[i] = make_key(__fsub_rn(1.0f, a.acc[0]), static_cast<uint32_t>(keys[i])); });
+    }
+}
+
+__global__ void __launch_bounds__(PREPARE_WARPS * 32)
+pairs_prepare_warps_kernel(const PairsPrepare p, uint64_t nq) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t q = static_cast<uint64_t>(blockIdx.x) * PREPARE_WARPS + warp;
+    if (q >= nq) {
+        return;
+    }
+    unsigned char* mine = smem + warp * prepare_warp_bytes(p.scores != nullptr, p.dim);
+    uint64_t* keys = reinterpret_cast<uint64_t*>(mine);
+    int32_t* probes = p.probes + q * p.nprobe;
+    const float* query = p.queries + q * p.dim;
+    if (p.dist != nullptr || p.scores != nullptr) {
+        const float* row = (p.scores != nullptr ? p.scores : p.dist) + q * p.ld;
+        const uint32_t wanted = p.scores != nullptr ? p.ncand : p.nprobe;
+        const auto load = [&](uint32_t i) { return float_to_ordered(__ldg(row + i)); };
+        const auto number = [](uint32_t i) { return i; };
+        uint32_t left;
+        uint32_t found = warp_select(load, number, p.nlist, wanted, keys, lane, &left);
+        if (found > WARP_SELECT_CAP) {
+            // Many at the bound.  The smallest value that `wanted` are at or below, then of those equal to it the first ones.
+            uint32_t low = 0, high = left;
+            while (low < high) {
+                const uint32_t mid = low + (high - low) / 2;
+                uint32_t count = 0;
+                warp_walk(load, p.nlist, lane, [&](uint32_t, uint32_t u, uint32_t) { count += u <= mid ? 1u : 0u; });
+                count = __reduce_add_sync(0xffffffffu, count);
+                if (count < wanted) {
+                    low = mid + 1;
+                } else {
+                    high = mid;
+                }
+            }
+            found = high > 0 ? warp_collect(load, number, p.nlist, high - 1, keys, lane) : 0u;
+            warp_walk(load, p.nlist, lane, [&](uint32_t i, uint32_t u, uint32_t) {
+                const uint32_t mask = __ballot_sync(0xffffffffu, u == high && u <= ORDERED_INF);
+                const uint32_t at = found + __popc(mask & ((1u << lane) - 1u));
+                if (u == high && u <= ORDERED_INF && at < wanted) {
+                    keys[at] = (static_cast<uint64_t>(u) << 32) | i;
+                }
+                found = min(found + __popc(mask), wanted);
+            });
+            __syncwarp();
+        }
+        if (p.scores != nullptr) {
+            // IVF::route_buckets_only's loop (src/algorithm/ivf/ivf.cpp:1589-1660) over the nominated centroids:
+            // distance ascending, lower list id first on ties
+            unsigned char* stages = reinterpret_cast<unsigned char*>(keys + WARP_SELECT_CAP);
+            float* qs = reinterpret_cast<float*>(stages + WARP_ROWS_BYTES);
+            for (uint32_t d = lane; d < p.dim; d += 32) {
+                qs[d] = __ldg(query + d);
+            }
+            __syncwarp();
+            warp_centroid_distances(p.centroids, p.dim, p.metric == VB200_METRIC_L2, qs, found, keys, stages, lane);
+        }
+        warp_sort(keys, found, lane);
+        for (uint32_t i = lane; i < p.nprobe; i += 32) {
+            const bool have = i < found;
+            probes[i] = have ? static_cast<int32_t>(static_cast<uint32_t>(keys[i])) : -1;
+            if (p.probe_dists != nullptr) {
+                p.probe_dists[q * p.nprobe + i] = have ? ordered_to_float(static_cast<uint32_t>(keys[i] >> 32)) : INFINITY;
+            }
+        }
+        __syncwarp();
+    }
+    if (p.t.rows == nullptr) {
+        return;   // only the routing is wanted
+    }
+    const uint32_t round = p.t.minima != nullptr ? 31u : 0u;
+    uint32_t run = 0;
+    for (uint32_t i0 = 0; i0 < p.nprobe; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        uint32_t len = 0;
+        if (i < p.nprobe) {
+            const int32_t l = probes[i];
+            if (l >= 0 && static_cast<uint32_t>(l) < p.nlist) {
+                len = __ldg(p.list_off + l + 1) - __ldg(p.list_off + l);
+            }
+            if (p.count != nullptr) {
+                p.rank[q * p.nprobe + i] = len > 0 ? atomicAdd(p.count + l, 1u) : 0xFFFFFFFFu;
+            }
+            len = (len + round) & ~round;
+        }
+        uint32_t incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            incl += lane >= static_cast<uint32_t>(o) ? v : 0u;
+        }
+        if (i < p.nprobe) {
+            p.t.base[q * p.nprobe + i] = run + incl - len;
+        }
+        run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) {
+        p.t.rows[q] = run;
+    }
+    if (p.terms != nullptr) {
+        pair_query_terms(p, q, query, lane, 32);
+    }
+    if (p.qw8 == nullptr) {
+        return;
+    }
+    float qq = 0.f, qm = 0.f, wmax = 0.f;
+    for (uint32_t d = lane; d < p.dim; d += 32) {
+        const float v = __ldg(query + d);
+        qq = fmaf(v, v, qq);
+        qm = fmaf(v, __ldg(p.mid + d), qm);
+        wmax = fmaxf(wmax, fabsf(v * __ldg(p.scale + d)));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        qm += __shfl_xor_sync(0xffffffffu, qm, o);
+        wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+    }
+    const float s = wmax > 0.f && wmax < INFINITY ? wmax / 127.0f : 1.0f;
+    pair_query_weights(p, q, query, s, lane, 32);
+    if (lane == 0) {
         p.qscale[q] = s;
         p.qa[q] = p.metric == VB200_METRIC_L2 ? fmaf(-2.0f, qm, qq) : 1.0f - qm;
     }
