@@ -2013,6 +2013,112 @@ route_pick_warp_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t 
     }
 }
 
+// The end of a grouped SQ8 search in one launch: the kscan best keys of the query's written slots, their exact distances
+// (sq8_exact_distance), the kfinal best with inner ids for positions.  A warp per query: after list pruning a query has two
+// or three slots of k + 16 keys, which sort through registers, and a chain of the reference's arithmetic per lane.  (As a merge and a
+// re-scoring with a CTA per query each and a pass for the ids: 103 us for 10,000 queries with k 10, most of it waiting; 61.)
+// Dynamic shared memory: [2][dim] lower and diff, per warp [FINISH_KEYS] keys and the query.
+constexpr uint32_t FINISH_KEYS = WARP_SELECT_CAP;
+constexpr uint32_t FINISH_MAX_SCAN = 128, FINISH_MAX_DIM = 4096;
+constexpr uint32_t FINISH_WARPS = 4;
+
+template <bool L2, int R>
+__global__ void __launch_bounds__(FINISH_WARPS * 32)
+sq8_finish_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t dim, const uint8_t* __restrict__ codes, uint32_t code_stride,
+                  const float* __restrict__ lower, const float* __restrict__ diff, const uint64_t* __restrict__ part,
+                  const uint8_t* __restrict__ slot_written, uint32_t slots, uint32_t kscan, uint32_t kfinal,
+                  const uint32_t* __restrict__ pos_inner, uint64_t* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t* buf = reinterpret_cast<uint64_t*>(smem) + warp * FINISH_KEYS;
+    float* lo = reinterpret_cast<float*>(reinterpret_cast<uint64_t*>(smem) + FINISH_WARPS * FINISH_KEYS);
+    float* di = lo + dim;
+    float* qs = di + (warp + 1) * dim;
+    const uint64_t q = static_cast<uint64_t>(blockIdx.x) * FINISH_WARPS + warp;
+    for (uint32_t d = threadIdx.x; d < dim; d += FINISH_WARPS * 32) {
+        lo[d] = __ldg(lower + d);
+        di[d] = __ldg(diff + d);
+    }
+    if (q < nq) {
+        for (uint32_t d = lane; d < dim; d += 32) {
+            qs[d] = __ldg(queries + q * dim + d);
+        }
+    }
+    __syncthreads();
+    if (q >= nq) {
+        return;
+    }
+    uint32_t count = 0;
+    uint64_t cut = KEY_INF;    // the kscan-th best so far: what is not below it is of no use
+    auto sort = [&]() {   // buf[0 .. count) ascending, cut to kscan
+        warp_sort(buf, count, lane);
+        if (count >= kscan) {
+            count = kscan;
+            cut = buf[kscan - 1];
+        }
+    };
+    const uint8_t* written = slot_written + q * slots;
+    for (uint32_t s0 = 0; s0 < slots; s0 += 32) {
+        uint32_t mask = __ballot_sync(0xffffffffu, s0 + lane < slots && __ldg(written + s0 + lane) != 0);
+        while (mask != 0) {
+            const uint64_t* keys = part + (q * slots + s0 + __ffs(mask) - 1) * kscan;
+            mask &= mask - 1;
+            uint64_t key[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                key[r] = r * 32 + lane < kscan ? __ldg(keys + r * 32 + lane) : KEY_INF;
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                uint32_t there = __ballot_sync(0xffffffffu, key[r] < cut);
+                if (count + __popc(there) > FINISH_KEYS) {
+                    sort();
+                    there = __ballot_sync(0xffffffffu, key[r] < cut);
+                }
+                if (key[r] < cut) {
+                    buf[count + __popc(there & ((1u << lane) - 1u))] = key[r];
+                }
+                count += __popc(there);
+                __syncwarp();
+            }
+        }
+    }
+    sort();
+    uint64_t exact[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = r * 32 + lane;
+        exact[r] = KEY_INF;
+        if (i < count) {
+            const uint32_t pos = static_cast<uint32_t>(buf[i]);
+            exact[r] = make_key(sq8_exact_distance(codes + static_cast<uint64_t>(pos) * code_stride, dim, L2, qs, lo, di), pos);
+        }
+    }
+    warp_sort_registers<R>(exact, lane);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = r * 32 + lane;
+        if (i < kfinal) {
+            const uint64_t key = exact[r];
+            out[q * kfinal + i] = key == KEY_INF ? KEY_INF : ((key & 0xFFFFFFFF00000000ull) | __ldg(pos_inner + static_cast<uint32_t>(key)));
+        }
+    }
+}
+
+static int
+launch_sq8_finish(const vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t nprobe, uint32_t kscan, uint32_t kfinal, const uint64_t* part,
+                  const uint8_t* slot_written, uint64_t* out) {
+    const bool l2 = ix->metric == VB200_METRIC_L2;
+    auto kernel = kscan <= 32 ? (l2 ? sq8_finish_kernel<true, 1> : sq8_finish_kernel<false, 1>)
+                              : (kscan <= 64 ? (l2 ? sq8_finish_kernel<true, 2> : sq8_finish_kernel<false, 2>)
+                                             : (l2 ? sq8_finish_kernel<true, 4> : sq8_finish_kernel<false, 4>));
+    const size_t smem = FINISH_WARPS * FINISH_KEYS * sizeof(uint64_t) + (FINISH_WARPS + 2) * static_cast<size_t>(ix->dim) * sizeof(float);
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    VB_LAUNCH(kernel, static_cast<uint32_t>((nq + FINISH_WARPS - 1) / FINISH_WARPS), FINISH_WARPS * 32, smem, q_dev, nq, ix->dim, ix->codes.ptr,
+              ix->code_stride, ix->lower.ptr, ix->diff.ptr, part, slot_written, nprobe, kscan, kfinal, ix->pos_inner.ptr, out);
+    return 0;
+}
+
 constexpr uint32_t ROUTE_PICK_SMALL = 512;   // keys the small sort takes
 
 // One query (q) by the whole CTA.
@@ -2936,6 +3042,12 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
     }
     VB_CUDA(cudaEventRecord(ix->ev_scan_end, st));
     ix->scan_timed = true;
+    // (a warp sorts what few slots hold; unpruned a query's slots are all written, nprobe * kscan keys, and a CTA merges them)
+    if (sq8 && kscan <= FINISH_MAX_SCAN && ws.pruning && !ix->use_residual && ix->dim <= FINISH_MAX_DIM) {
+        VB_TRY(launch_sq8_finish(ix, q_dev, nq, nprobe, kscan, kfinal, ws.part.ptr, ws.slot_written.ptr, ws.keys.ptr));
+        g_scan_profile.mark(st);   // merge
+        return 0;
+    }
     if (sq8) {
         VB_TRY(launch_merge(ws.part.ptr, nq, static_cast<uint64_t>(nprobe) * kscan, kscan, ws.merged.ptr, ws.slot_written.ptr, kscan));
         uint32_t n2 = next_pow2(kscan < 2 ? 2 : kscan);
