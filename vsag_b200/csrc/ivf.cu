@@ -2817,9 +2817,9 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
     // (the warps rank with the tensor-core scan's integer weight terms when those are prepared anyway, so both
     // phases nominate with one arithmetic; VB200_FIRST_INT8=0: the SIMT scan's fp32 weights instead)
     static const bool first_int8 = !(std::getenv("VB200_FIRST_INT8") != nullptr && std::getenv("VB200_FIRST_INT8")[0] == '0');
-    const uint32_t first_dpad32 = (tc_scan && first_int8) ? ix->kchunks * 16 : 0u;
+    const bool first_tiled = tc_scan && first_int8;
     const bool warp_first = sq8 && split_phases && pruning && !tc_first && !warp_first_off && kscan <= 192 &&
-                            sq8_first_smem_bytes(kscan, ix->dpad, first_dpad32) <= 96 * 1024;
+                            (first_tiled ? first_smem_bytes(kscan, ix->kchunks) : sq8_first_smem_bytes(kscan, ix->dpad)) <= 96 * 1024;
     const uint32_t qt_first = warp_first ? 1u : (tc_first ? TCS_QT : static_cast<uint32_t>(qt));
     const uint32_t qt_second = tc_second ? TCS_QT : static_cast<uint32_t>(qt);
     VB_TRY(group_pairs(split_phases ? 0u : 2u, nullptr, qt_first));
@@ -2953,18 +2953,31 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
             return 0;
         }
         if (sq8 && warp_items) {
-            const bool int8 = first_dpad32 != 0;
-            const size_t smem = sq8_first_smem_bytes(p.k, ix->dpad, first_dpad32);
-            auto kernel = int8 ? ivf_sq8_first_kernel<true, 3> : ivf_sq8_first_kernel<false, 2>;   // rows per lane: measured best
-            VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+            FirstScan f{};
+            f.s = p;
+            f.codes_t = ix->codes_t.ptr;
+            f.group_off = ix->group_off.ptr;
+            f.kchunks = ix->kchunks;
+            f.qw8 = ws.qw8.ptr;
+            f.qscale = ws.qscale.ptr;
+            f.spin_limit = tc_spin_limit();
+            f.error_flag = reinterpret_cast<int*>(ws.scalars.ptr + 4);
+            const size_t smem = first_tiled ? first_smem_bytes(p.k, ix->kchunks) : sq8_first_smem_bytes(p.k, ix->dpad);
+            const int threads = first_tiled ? FIRST_WARPS * 32 : SQ8_FIRST_WARPS * 32;
+            const void* kernel = first_tiled ? reinterpret_cast<const void*>(ivf_sq8_first_tiled_kernel)
+                                             : reinterpret_cast<const void*>(ivf_sq8_first_kernel<2>);   // rows per lane: measured best
+            VB_TRY(allow_dynamic_smem(kernel, smem));
             int per_sm = 0;
-            VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SQ8_FIRST_WARPS * 32, smem));
+            VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
             if (per_sm < 1) {
                 VB_FAIL(VB200_INTERNAL_ERROR, "the first-phase scan does not fit an SM with %zu bytes of shared memory", smem);
             }
-            VB_LAUNCH(kernel, static_cast<uint32_t>(sm_count()) * static_cast<uint32_t>(per_sm), SQ8_FIRST_WARPS * 32, smem, p,
-                      int8 ? ws.qw8.ptr : static_cast<const int8_t*>(nullptr),
-                      int8 ? ws.qscale.ptr : static_cast<const float*>(nullptr), first_dpad32);
+            const uint32_t grid = static_cast<uint32_t>(sm_count()) * static_cast<uint32_t>(per_sm);
+            if (first_tiled) {
+                VB_LAUNCH(ivf_sq8_first_tiled_kernel, grid, threads, smem, f);
+            } else {
+                VB_LAUNCH(ivf_sq8_first_kernel<2>, grid, threads, smem, p);
+            }
             return 0;
         }
         if (sq8) {

@@ -666,14 +666,13 @@ ivf_sq8_scan_kernel(const ScanParams p) {
     }
 }
 
-// The first phase when it runs alone: every work item is one query against its nearest list, a few hundred
+// The first phase when it runs alone over lists without a tiled copy of their codes (ivf_sq8_first_tiled_kernel otherwise): every
+// work item is one query against its nearest list, a few hundred
 // rows.  A CTA per item spends most of its time in barriers and set-up, so here a warp takes an item by itself:
 // its lanes own NR rows each per round, the query's weights sit in the warp's slice of shared memory (every
 // lane reads the same word: a broadcast), candidates that beat the bound are appended through a ballot, and
-// the warp sorts its own small buffer when it fills.  The arithmetic per row is that of sq8_tile_dots_single
-// (INT8 false), so the survivors are the ones the CTA kernel would keep -- or, with INT8, that of the tensor-core
-// scan: the weights' three signed-byte terms against the codes as signed bytes (code ^ 0x80 = code - 128), three
-// exact integer dot products per four dimensions (dp4a), combined as that kernel's epilogue combines them.
+// the warp sorts its own small buffer when it fills.  The arithmetic per row is that of sq8_tile_dots_single,
+// so the survivors are the ones the CTA kernel would keep.
 constexpr int SQ8_FIRST_WARPS = 8;
 
 __host__ __device__ inline uint32_t
@@ -685,27 +684,26 @@ sq8_first_cap(uint32_t k) {
     return c;
 }
 
-// bytes of a warp's weight slot: the fp32 weights, or the three signed-byte terms of the tensor-core scan's split
+// bytes of a warp's weights
 __host__ __device__ inline uint32_t
-sq8_first_weight_bytes(uint32_t dpad, uint32_t dpad32) {
-    const uint32_t f = dpad * 4, b = dpad32 * 3;
-    return ((f > b ? f : b) + 15u) & ~15u;
+sq8_first_weight_bytes(uint32_t dpad) {
+    return (dpad * 4 + 15u) & ~15u;
 }
 
 __host__ __device__ inline size_t
-sq8_first_smem_bytes(uint32_t k, uint32_t dpad, uint32_t dpad32) {
-    return static_cast<size_t>(SQ8_FIRST_WARPS) * (static_cast<size_t>(sq8_first_cap(k)) * 8 + sq8_first_weight_bytes(dpad, dpad32));
+sq8_first_smem_bytes(uint32_t k, uint32_t dpad) {
+    return static_cast<size_t>(SQ8_FIRST_WARPS) * (static_cast<size_t>(sq8_first_cap(k)) * 8 + sq8_first_weight_bytes(dpad));
 }
 
-template <bool INT8, int NR = 2>
+template <int NR>
 __global__ void __launch_bounds__(SQ8_FIRST_WARPS * 32)
-ivf_sq8_first_kernel(const ScanParams p, const int8_t* __restrict__ qw8, const float* __restrict__ qscale, uint32_t dpad32) {
+ivf_sq8_first_kernel(const ScanParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t cap = sq8_first_cap(p.k), k = p.k, dpad = p.dpad;
     uint64_t* kb = reinterpret_cast<uint64_t*>(smem) + static_cast<size_t>(warp) * cap;
     unsigned char* w_raw = smem + static_cast<size_t>(SQ8_FIRST_WARPS) * cap * 8 +
-                           static_cast<size_t>(warp) * sq8_first_weight_bytes(dpad, dpad32);
+                           static_cast<size_t>(warp) * sq8_first_weight_bytes(dpad);
     float* w_s = reinterpret_cast<float*>(w_raw);
     const uint32_t n_items = p.item_off[0][p.nlist];
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -734,16 +732,8 @@ ivf_sq8_first_kernel(const ScanParams p, const int8_t* __restrict__ qw8, const f
             uint32_t thr = p.thr_g[q];
             float thrq = (thr >= 0xFF800000u ? INFINITY : ordered_to_float(thr)) - qa;
             uint32_t cnt = 0;
-            float cq = 0.f;   // INT8: coef_c * the query's weight scale
             __syncwarp();
-            if (INT8) {
-                const uint4* src = reinterpret_cast<const uint4*>(qw8 + static_cast<uint64_t>(q) * 3 * dpad32);
-                uint4* dst = reinterpret_cast<uint4*>(w_raw);
-                for (uint32_t i = lane; i < (3 * dpad32) >> 4; i += 32) {
-                    dst[i] = __ldg(src + i);
-                }
-                cq = p.coef_c * __ldg(qscale + q);
-            } else {
+            {
                 const float4* src = reinterpret_cast<const float4*>(p.qw + static_cast<uint64_t>(q) * dpad);
                 float4* dst = reinterpret_cast<float4*>(w_s);
                 for (uint32_t i = lane; i < (dpad >> 2); i += 32) {
@@ -791,54 +781,7 @@ ivf_sq8_first_kernel(const ScanParams p, const int8_t* __restrict__ qw8, const f
                     norm[r] = valid[r] ? __ldg(p.code_norm + lbeg + row) : 0.f;
                     acc[r] = 0.f;
                 }
-                if (INT8) {
-                    int32_t sum[NR][3];
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) {
-                        sum[r][0] = sum[r][1] = sum[r][2] = 0;
-                    }
-#pragma unroll 1
-                    for (uint32_t c = 0; c < dpad; c += 16) {
-                        int32_t x[NR][4];
-#pragma unroll
-                        for (int r = 0; r < NR; ++r) {
-                            x[r][0] = static_cast<int32_t>(nxt[r].x ^ 0x80808080u);
-                            x[r][1] = static_cast<int32_t>(nxt[r].y ^ 0x80808080u);
-                            x[r][2] = static_cast<int32_t>(nxt[r].z ^ 0x80808080u);
-                            x[r][3] = static_cast<int32_t>(nxt[r].w ^ 0x80808080u);
-                        }
-                        if (c + 16 < dpad) {
-#pragma unroll
-                            for (int r = 0; r < NR; ++r) {
-                                nxt[r] = __ldg(reinterpret_cast<const uint4*>(cp[r] + c + 16));
-                            }
-                        } else if (r0 + ROUND < len) {
-#pragma unroll
-                            for (int r = 0; r < NR; ++r) {
-                                const uint32_t row = r0 + ROUND + r * 32u + lane;
-                                nxt[r] = __ldg(reinterpret_cast<const uint4*>(p.codes + static_cast<uint64_t>(lbeg + (row < len ? row : 0)) * p.code_stride));
-                            }
-                        }
-#pragma unroll
-                        for (int t = 0; t < 3; ++t) {
-                            const uint4 wv = *reinterpret_cast<const uint4*>(w_raw + t * dpad32 + c);
-                            const int32_t wt[4] = {static_cast<int32_t>(wv.x), static_cast<int32_t>(wv.y), static_cast<int32_t>(wv.z),
-                                                   static_cast<int32_t>(wv.w)};
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                                for (int r = 0; r < NR; ++r) {
-                                    sum[r][t] = __dp4a(x[r][j], wt[j], sum[r][t]);
-                                }
-                            }
-                        }
-                    }
-                    // sum_d w_d (code_d - 128) / s = A1 + (254 A2 + A3) / 254^2, as the tensor-core scan's epilogue
-#pragma unroll
-                    for (int r = 0; r < NR; ++r) {
-                        acc[r] = fmaf(static_cast<float>(sum[r][1] * 254 + sum[r][2]), 1.0f / 64516.0f, static_cast<float>(sum[r][0]));
-                    }
-                } else {
+                {
                     const float4* wrow = reinterpret_cast<const float4*>(w_s);
 #pragma unroll 1
                     for (uint32_t c = 0; c < dpad; c += 16, wrow += 4) {
@@ -881,7 +824,7 @@ ivf_sq8_first_kernel(const ScanParams p, const int8_t* __restrict__ qw8, const f
                     float partial = 0.f;
                     bool pass = false;
                     if (valid[h]) {
-                        partial = fmaf(INT8 ? cq : p.coef_c, acc[h], p.coef_b * norm[h]);
+                        partial = fmaf(p.coef_c, acc[h], p.coef_b * norm[h]);
                         pass = partial <= thrq;
                         if (pass && p.filter_pos_inner != nullptr && scan_row_filtered(p, pos)) {
                             pass = false;

@@ -27,6 +27,7 @@
 // taking work, frees its tensor memory and returns.
 #pragma once
 
+#include "block_select.cuh"
 #include "ivf_scan.cuh"
 #include "tc_gemm.cuh"
 
@@ -805,6 +806,256 @@ inline uint32_t
 tcs_buffer_cap(uint32_t k) {
     const uint32_t cap = next_pow2(k + 32);
     return cap < 64 ? 64 : cap;
+}
+
+// The first phase when it runs alone and the lists have their tiled copy: every work item is one query against its nearest list,
+// a few hundred rows, and a warp takes an item by itself.  The rows come 64 at a time (two per lane) and 128 of their bytes at a time
+// from the tiled copy, in which eight rows' 16 bytes lie together, by bulk copies into the warp's own two stages, so that a warp
+// waits for a stage and not for each of its lanes' loads; the arithmetic is that of the tensor-core scan, the three signed-byte
+// terms of the query's weights against signed codes in exact integer dot products (dp4a).  Bound by those and the reads of shared
+// memory beside them (eleven wavefronts per 24 dp4a).  10,000 queries, 10M rows of 96 dimensions in 16384 lists: 146 us; with a lane's
+// rows read from memory 16 bytes at a time, 96 bytes apart, 208 us, three quarters of it waiting.
+constexpr int FIRST_WARPS = 4;
+constexpr uint32_t FIRST_ROWS = 64, FIRST_STAGES = 2, FIRST_CORES = 8;   // rows and 16-byte cores of each per stage
+
+// Bytes between the 8-row groups of a stage, and shared memory of a CTA.
+__host__ __device__ inline uint32_t
+first_pitch(uint32_t kchunks) {
+    return (kchunks < FIRST_CORES ? kchunks : FIRST_CORES) * 128;
+}
+
+__host__ __device__ inline size_t
+first_smem_bytes(uint32_t k, uint32_t kchunks) {
+    return FIRST_WARPS * (static_cast<size_t>(FIRST_STAGES) * (FIRST_ROWS / 8) * first_pitch(kchunks) + sq8_first_cap(k) * 8 + 3 * kchunks * 16);
+}
+
+struct FirstScan {
+    ScanParams s;
+    const int8_t* codes_t;      // [groups][kchunks][8 rows][16] signed codes
+    const uint32_t* group_off;  // first group of every list
+    uint32_t kchunks;
+    const int8_t* qw8;          // [nq][3][kchunks * 16]
+    const float* qscale;
+    uint32_t spin_limit;
+    int* error_flag;
+};
+
+static __global__ void __launch_bounds__(FIRST_WARPS * 32)
+ivf_sq8_first_tiled_kernel(const FirstScan f) {
+    const ScanParams& p = f.s;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t full[FIRST_WARPS][FIRST_STAGES];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t cap = sq8_first_cap(p.k), k = p.k, kchunks = f.kchunks, term = kchunks * 16;
+    const uint32_t pitch = first_pitch(kchunks), stage_bytes = FIRST_ROWS / 8 * pitch;
+    unsigned char* const stages = smem + warp * FIRST_STAGES * stage_bytes;
+    unsigned char* const rest = smem + FIRST_WARPS * FIRST_STAGES * stage_bytes;
+    uint64_t* const kb = reinterpret_cast<uint64_t*>(rest) + static_cast<size_t>(warp) * cap;
+    unsigned char* const w_raw = rest + static_cast<size_t>(FIRST_WARPS) * cap * 8 + warp * 3 * term;
+    if (lane == 0) {
+        for (uint32_t i = 0; i < FIRST_STAGES; ++i) {
+            mbar_init(&full[warp][i], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    const uint32_t n_items = p.item_off[0][p.nlist];
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t per_row = (kchunks + FIRST_CORES - 1) / FIRST_CORES;   // steps per 64 rows
+    uint32_t asked = 0, taken = 0;   // stages requested and consumed so far
+    bool ok = true;
+    while (ok) {
+        uint32_t item = 0;
+        if (lane == 0) {
+            item = atomicAdd(p.item_counter, 1u);
+            if (p.deadline != nullptr && scan_deadline_passed(p)) {
+                item = 0xFFFFFFFFu;
+            }
+        }
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= n_items) {
+            break;
+        }
+        const uint4 head = __ldg(reinterpret_cast<const uint4*>(p.item_map[0] + item));
+        const uint32_t list = head.x, pbeg = head.y, nqt = head.z;
+        const uint32_t lbeg = __ldg(p.list_off + list);
+        const uint32_t len = __ldg(p.list_off + list + 1) - lbeg;
+        const int8_t* const rows = f.codes_t + static_cast<uint64_t>(__ldg(f.group_off + list)) * kchunks * 128;
+        const uint32_t steps = (len + FIRST_ROWS - 1) / FIRST_ROWS * per_row;
+        for (uint32_t pi = 0; pi < nqt && ok; ++pi) {
+            // (a stage past the list's end runs into the next list or the padding behind the last; those rows are masked)
+            uint32_t ask_round = 0, ask_piece = 0;
+            auto request = [&]() {
+                if (ask_round * FIRST_ROWS >= len) {
+                    return;
+                }
+                const uint32_t cores = min(FIRST_CORES, kchunks - ask_piece * FIRST_CORES), at = asked % FIRST_STAGES;
+                if (lane == 0) {
+                    mbar_expect_tx(&full[warp][at], FIRST_ROWS / 8 * cores * 128);
+                }
+                __syncwarp();
+                if (lane < FIRST_ROWS / 8) {
+                    bulk_copy_g2s(stages + at * stage_bytes + lane * pitch,
+                                  rows + (static_cast<uint64_t>(ask_round * (FIRST_ROWS / 8) + lane) * kchunks + ask_piece * FIRST_CORES) * 128,
+                                  cores * 128, &full[warp][at]);
+                }
+                ++asked;
+                if (++ask_piece == per_row) {
+                    ask_piece = 0;
+                    ++ask_round;
+                }
+            };
+            for (uint32_t i = 0; i < FIRST_STAGES; ++i) {
+                request();
+            }
+            const uint32_t q = __ldg(p.pair_q[0] + pbeg + pi);
+            const uint32_t slot = __ldg(p.pair_slot[0] + pbeg + pi);
+            const float qa = __ldg(p.qa + q) + (p.pair_const != nullptr ? __ldg(p.pair_const + slot) : 0.f);
+            uint32_t thr = p.thr_g[q];
+            float thrq = (thr >= 0xFF800000u ? INFINITY : ordered_to_float(thr)) - qa;
+            uint32_t cnt = 0;
+            {
+                const uint4* src = reinterpret_cast<const uint4*>(f.qw8 + static_cast<uint64_t>(q) * 3 * term);
+                for (uint32_t i = lane; i < 3 * kchunks; i += 32) {
+                    reinterpret_cast<uint4*>(w_raw)[i] = __ldg(src + i);
+                }
+            }
+            const float cq = p.coef_c * __ldg(f.qscale + q);
+            __syncwarp();
+            if (lane == 0 && p.scanned != nullptr) {
+                atomicAdd(p.scanned, static_cast<unsigned long long>(len) * p.dim);
+            }
+            auto lower = [&](uint32_t t) {
+                if (t < thr) {
+                    thr = t;
+                    thrq = (t >= 0xFF800000u ? INFINITY : ordered_to_float(t)) - qa;
+                }
+            };
+            // Keeps what is not above a value that k keys are at or below, k keys or a few more (all lanes).  (As a sort of the
+            // whole buffer, five or six times an item, most of the kernel's instructions.)
+            auto compact = [&]() {
+                uint64_t key[8];
+                uint32_t value[8];
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    key[j] = j * 32 + lane < cnt ? kb[j * 32 + lane] : KEY_INF;
+                    value[j] = static_cast<uint32_t>(key[j] >> 32);
+                }
+                __syncwarp();
+                const uint32_t t = warp_bound(value, k);
+                cnt = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    const bool keep = value[j] <= t && key[j] != KEY_INF;
+                    const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+                    if (keep) {
+                        kb[cnt + __popc(mask & lt_mask)] = key[j];
+                    }
+                    cnt += __popc(mask);
+                }
+                __syncwarp();
+                if (cnt > k + k / 16) {   // more tie there than a buffer has room for, perhaps
+                    warp_sort(kb, cnt, lane);
+                    cnt = k;
+                }
+                lower(t);
+            };
+            uint32_t r0 = 0, piece = 0;
+            int32_t sum[2][3];
+            float norm[2];
+            for (uint32_t step = 0; step < steps; ++step) {
+                if (piece == 0) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t row = r0 + h * 32u + lane;
+                        norm[h] = row < len ? __ldg(p.code_norm + lbeg + row) : 0.f;
+                        sum[h][0] = sum[h][1] = sum[h][2] = 0;
+                    }
+                }
+                const uint32_t at = taken % FIRST_STAGES;
+                ok = mbar_wait_warp(&full[warp][at], (taken / FIRST_STAGES) & 1u, f.spin_limit);
+                if (!ok) {
+                    break;
+                }
+                ++taken;
+                const unsigned char* mine = stages + at * stage_bytes + (lane >> 3) * pitch + (lane & 7u) * 16;
+                const unsigned char* weights = w_raw + piece * FIRST_CORES * 16;
+                const uint32_t cores = min(FIRST_CORES, kchunks - piece * FIRST_CORES);
+#pragma unroll 2
+                for (uint32_t c = 0; c < cores; ++c) {
+                    const int4 x0 = *reinterpret_cast<const int4*>(mine + c * 128), x1 = *reinterpret_cast<const int4*>(mine + 4 * pitch + c * 128);
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        const int4 w = *reinterpret_cast<const int4*>(weights + t * term + c * 16);
+                        sum[0][t] = __dp4a(x0.x, w.x, sum[0][t]);
+                        sum[1][t] = __dp4a(x1.x, w.x, sum[1][t]);
+                        sum[0][t] = __dp4a(x0.y, w.y, sum[0][t]);
+                        sum[1][t] = __dp4a(x1.y, w.y, sum[1][t]);
+                        sum[0][t] = __dp4a(x0.z, w.z, sum[0][t]);
+                        sum[1][t] = __dp4a(x1.z, w.z, sum[1][t]);
+                        sum[0][t] = __dp4a(x0.w, w.w, sum[0][t]);
+                        sum[1][t] = __dp4a(x1.w, w.w, sum[1][t]);
+                    }
+                }
+                __syncwarp();   // nobody reads the stage any more
+                request();
+                if (++piece < per_row) {
+                    continue;
+                }
+                piece = 0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t row = r0 + h * 32u + lane, pos = lbeg + row;
+                    // sum_d w_d (code_d - 128) / s = A1 + (254 A2 + A3) / 254^2, as the tensor-core scan's epilogue
+                    const float acc = fmaf(static_cast<float>(sum[h][1] * 254 + sum[h][2]), 1.0f / 64516.0f, static_cast<float>(sum[h][0]));
+                    const float partial = fmaf(cq, acc, p.coef_b * norm[h]);
+                    const bool pass = row < len && partial <= thrq && !(p.filter_pos_inner != nullptr && scan_row_filtered(p, pos));
+                    const uint32_t mask = __ballot_sync(0xffffffffu, pass);
+                    if (mask != 0) {
+                        if (cnt + 32 > cap) {
+                            compact();
+                        }
+                        if (pass) {
+                            kb[cnt + __popc(mask & lt_mask)] = make_key(partial + qa, pos);
+                        }
+                        cnt += __popc(mask);
+                        __syncwarp();
+                    }
+                }
+                r0 += FIRST_ROWS;
+            }
+            if (!ok) {
+                break;
+            }
+            if (cnt > k) {
+                compact();
+            }
+            if (cnt >= k) {
+                warp_sort(kb, cnt, lane);
+                cnt = min(cnt, k);
+            }
+            __syncwarp();
+            uint64_t* dst = p.part + static_cast<uint64_t>(slot) * k;
+            for (uint32_t i = lane; i < k; i += 32) {
+                dst[i] = i < cnt ? kb[i] : KEY_INF;
+            }
+            if (lane == 0) {
+                if (cnt >= k) {
+                    atomicMin(p.thr_g + q, static_cast<uint32_t>(kb[k - 1] >> 32));
+                }
+                if (p.slot_written != nullptr) {
+                    p.slot_written[slot] = 1;
+                }
+            }
+            __syncwarp();
+        }
+    }
+    if (!ok) {
+        if (lane == 0) {
+            atomicOr(f.error_flag, 1);
+        }
+        tc_drain_pause();   // the copies still in flight land before the CTA lets go
+    }
 }
 
 }  // namespace vb200
