@@ -138,3 +138,23 @@ def test_pruned_batches_equal_unpruned_ones(engine, dim, k, metric):
     got = ix.search(q, k, nprobe)
     assert np.array_equal(got[1][::8], np.concatenate([w[1] for w in want]))
     assert np.array_equal(got[0][::8], np.concatenate([w[0] for w in want]))
+
+
+# ---- tiles ------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("quant", ["QUANT_FP32", "QUANT_BF16", "QUANT_SQ8", "QUANT_RABITQ"])
+@pytest.mark.parametrize("dim,nq", [(16, 12), (33, 31), (64, 33), (65, 64), (128, 65), (200, 130), (520, 9)])
+def test_tiles_equal_queries_one_by_one(engine, oracle, quant, dim, nq):
+    """Queries per list around the eight, sixteen, thirty-two and sixty-four that warps, operands and items hold; lists of one
+    row, of a tile and a row, of several segments."""
+    sizes, k = [1, 129, 2200], 10
+    labels = np.repeat(np.arange(3, dtype=np.int32), sizes)
+    x, q = mixture(61, labels.size, dim, 3, 0.4), mixture(62, nq, dim, 3, 0.4)
+    ix = engine.IvfHandle(dim, 0, 3, getattr(engine, quant))
+    if quant == "QUANT_RABITQ":
+        ix.set_rabitq_rotation(oracle.random_rotation(dim, seed=3))
+    ix.train(x, iters=1, init=np.ascontiguousarray(x[:3]))
+    ix.add(x, np.arange(labels.size, dtype=np.int64), labels=labels)
+    lists = np.tile(np.arange(3, dtype=np.int32), (nq, 1))
+    got = ix.search_filtered(q, k, 3, bucket_ids=lists)
+    one = [ix.search_filtered(q[i:i + 1].copy(), k, 3, bucket_ids=lists[:1]) for i in range(nq)]
+    exactly(got, (np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])))

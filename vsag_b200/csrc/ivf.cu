@@ -152,6 +152,7 @@ struct vb200_ivf {
     uint32_t max_list_len = 0;   // the longest list this index (shard) holds
     CUtensorMap row_map{};       // the stored rows for the tile scan's copies (fp32, bf16, fp16, RaBitQ)
     bool has_row_map = false;
+    DevBuf<uint16_t> split;      // fp32: the rows' two bf16 terms, which row_map then covers; empty where memory was short
     DevBuf<float> row_max;       // [0] largest norm of a stored row, [1] RaBitQ: largest norm / |error term|
     std::vector<uint64_t> longest_rows;   // [nlist + 1] rows of the i longest lists together
     bool balls_valid = false;    // the covering balls describe the lists as they are stored
@@ -3390,7 +3391,13 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     kernel = plan.qt == 64 ? tile_scan_kernel<FMT, 64> : (plan.qt == 32 ? tile_scan_kernel<FMT, 32> : tile_scan_kernel<FMT, 16>)
     switch (ix->quant) {
         case VB200_QUANT_SQ8: VB_TILE(ROW_SQ8); break;
-        case VB200_QUANT_FP32: VB_TILE(ROW_F32); break;
+        case VB200_QUANT_FP32:
+            if (ix->split.ptr != nullptr) {
+                VB_TILE(ROW_F32_SPLIT);
+            } else {
+                VB_TILE(ROW_F32);
+            }
+            break;
         case VB200_QUANT_BF16: VB_TILE(ROW_BF16); break;
         case VB200_QUANT_FP16: VB_TILE(ROW_FP16); break;
         default: VB_TILE(ROW_RABITQ); break;
@@ -3490,7 +3497,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     if (plan != nullptr && !sq8 && ix->quant != VB200_QUANT_RABITQ) {
         const bool f32 = ix->quant == VB200_QUANT_FP32;
         pp.term_dims = plan->pieces * 64;
-        pp.term_fmt = f32 ? ROW_F32 : (ix->quant == VB200_QUANT_BF16 ? ROW_BF16 : ROW_FP16);
+        pp.term_fmt = f32 ? (ix->split.ptr != nullptr ? ROW_F32_SPLIT : ROW_F32) : (ix->quant == VB200_QUANT_BF16 ? ROW_BF16 : ROW_FP16);
         VB_TRY(ws.tile_terms.reserve(nq * pp.term_dims * (f32 ? 2 : 1)));
         pp.terms = ws.tile_terms.ptr;
     }
@@ -4150,10 +4157,16 @@ ivf_append_row_data(vb200_ivf* ix, const int64_t* ids, const float* rows_dev, ui
     return 0;
 }
 
+// Dimensions of a term of a row in the copy that split_rows_kernel makes.
+static uint64_t
+split_pitch(uint32_t dim) {
+    return (dim + 63) / 64 * 64;
+}
+
 // The tensor map through which the tile scan copies stored rows, 128 at a time; false where there is none (SQ8 has a
 // tiled copy instead).
 static bool
-make_row_map(const vb200_ivf* ix, const uint8_t* codes, uint64_t n, CUtensorMap* map) {
+make_row_map(const vb200_ivf* ix, const uint8_t* codes, const uint16_t* split, uint64_t n, CUtensorMap* map) {
     using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -4172,12 +4185,19 @@ make_row_map(const vb200_ivf* ix, const uint8_t* codes, uint64_t n, CUtensorMap*
     }
     CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_UINT16;
     CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B;
-    cuuint64_t extent = ix->dim;
+    cuuint64_t extent = ix->dim, pitch = ix->code_stride;
     cuuint32_t box = 64;
+    const void* rows = codes;
     switch (ix->quant) {
         case VB200_QUANT_BF16:
         case VB200_QUANT_FP16: break;
         case VB200_QUANT_FP32:
+            if (split != nullptr) {
+                extent = split_pitch(ix->dim) * 2;
+                pitch = extent * sizeof(uint16_t);
+                rows = split;
+                break;
+            }
             type = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
             swizzle = CU_TENSOR_MAP_SWIZZLE_NONE;
             box = 32;
@@ -4193,9 +4213,9 @@ make_row_map(const vb200_ivf* ix, const uint8_t* codes, uint64_t n, CUtensorMap*
             break;
         default: return false;
     }
-    const cuuint64_t extents[2] = {extent, n}, strides[1] = {ix->code_stride};
+    const cuuint64_t extents[2] = {extent, n}, strides[1] = {pitch};
     const cuuint32_t boxes[2] = {box, 128}, steps[2] = {1, 1};
-    return encode(map, type, 2, const_cast<uint8_t*>(codes), extents, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+    return encode(map, type, 2, const_cast<void*>(rows), extents, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -4276,8 +4296,17 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
         VB_TRY(sync_stream());   // goff is a local
         ix->kchunks = kchunks;
     }
+    DevBuf<uint16_t> new_split;
+    if (ix->quant == VB200_QUANT_FP32 && n_new_stored > 0) {
+        const uint64_t pitch = split_pitch(dim), blocks = (n_new_stored * (pitch / 8) + 255) / 256;
+        if (blocks <= 0x7fffffffull && new_split.reserve(n_new_stored * 2 * pitch) == 0) {   // (not there: tiles convert the rows)
+            VB_LAUNCH(split_rows_kernel, static_cast<uint32_t>(blocks), 256, 0, new_codes.ptr, n_new_stored, dim, stride,
+                      static_cast<uint32_t>(pitch), new_split.ptr);
+        }
+    }
     VB_TRY(sync_stream());
-    ix->has_row_map = make_row_map(ix, new_codes.ptr, n_new_stored, &ix->row_map);
+    ix->has_row_map = make_row_map(ix, new_codes.ptr, new_split.ptr, n_new_stored, &ix->row_map);
+    ix->split = std::move(new_split);
     ix->codes_t = std::move(new_tiled);
     ix->group_off = std::move(new_group_off);
     ix->code_norm = std::move(new_norm);
@@ -4497,7 +4526,7 @@ vb200_ivf_memory_usage(vb200_ivf_t ix) {
     if (ix == nullptr) {
         return 0;
     }
-    return static_cast<int64_t>(ix->codes.bytes() + ix->codes_t.bytes() + ix->pos_inner.bytes() + ix->labels.bytes() +
+    return static_cast<int64_t>(ix->codes.bytes() + ix->codes_t.bytes() + ix->split.bytes() + ix->pos_inner.bytes() + ix->labels.bytes() +
                                 ix->flat.bytes() + ix->centroids.bytes() + ix->rotation.bytes() +
                                 ix->list_off.bytes());
 }

@@ -13,8 +13,9 @@
 // issues the MMAs, eight warps drain them.  (With the loads, the conversions and the gathering of an item on the same
 // warps, and the item's constants read by the epilogue, the kernel waited for one latency after another: 390 to
 // 560 us instead of 279 for 1000 queries against 32 lists each of 500k x 128 fp32.)  How rows become operands:
-//   fp32        two bf16 terms x = hi + lo, made in place in shared memory; hi*hi + lo*hi and hi*lo are accumulated
-//               (the dropped terms are below 2^-16 |x||q|)
+//   fp32        two bf16 terms x = hi + lo, from a copy of the rows that holds them (made with the lists; where there is no
+//               memory for it, made in place in shared memory, which a tile waits for: 280 us of the case above, 173
+//               from the copy); hi*hi + lo*hi and hi*lo are accumulated (the dropped terms are below 2^-16 |x||q|)
 //   bf16, fp16  the codes as they are (TMA with the 128-byte swizzle); every product is exact in fp32
 //   sq8         the tiled copy of the codes as signed bytes code - 128, against three int8 terms of the query's
 //               weights: exact int32 sums
@@ -29,9 +30,8 @@
 
 namespace vb200 {
 
-constexpr int TILE_EPI_WARPS = 8;                           // warps 0-7; 8 issues the MMAs, 9 copies rows,
-constexpr int TILE_QUERY_WARPS = 4;                         // 10-13 gather queries,
-constexpr int TILE_CONV_WARPS = 8;                          // 14-21 convert
+constexpr int TILE_QUERY_WARPS = 4;
+constexpr int TILE_CONV_WARPS = 8;
 constexpr uint32_t TILE_PIECE = 128;                        // operand bytes per row and piece
 constexpr uint32_t TILE_A_TERM = 128 * TILE_PIECE;          // 16 KiB
 constexpr uint32_t TILE_MAX_STAGES = 8;
@@ -42,12 +42,17 @@ constexpr uint32_t TILE_ACC_COLS = 256;                     // tensor-memory col
 template <int FMT>
 struct TileFmt {
     static constexpr bool INT8 = FMT == ROW_SQ8 || FMT == ROW_RABITQ;
+    static constexpr bool SPLIT = FMT == ROW_F32 || FMT == ROW_F32_SPLIT;
     static constexpr bool CONVERT = FMT == ROW_F32 || FMT == ROW_RABITQ;
-    static constexpr uint32_t A_TERMS = FMT == ROW_F32 ? 2 : 1;
-    static constexpr uint32_t B_TERMS = INT8 ? 3 : (FMT == ROW_F32 ? 2 : 1);
+    static constexpr uint32_t A_TERMS = SPLIT ? 2 : 1;
+    static constexpr uint32_t B_TERMS = INT8 ? 3 : (SPLIT ? 2 : 1);
     static constexpr uint32_t PIECE_DIMS = INT8 ? 128 : 64;
     static constexpr uint32_t STAGE = A_TERMS * TILE_A_TERM;
-    static constexpr int THREADS = 32 * (TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS + (CONVERT ? TILE_CONV_WARPS : 0));
+    // Warps by role: the first EPI drain accumulators, then one issues the MMAs, one copies rows, TILE_QUERY_WARPS gather queries,
+    // TILE_CONV_WARPS convert.  Of sixteen draining warps four share the columns of 32 rows: 173 us for the split fp32 rows of the
+    // case above; integer sums take more instructions a column and are no faster for it (109 against 123 us).
+    static constexpr int EPI = CONVERT || INT8 ? 8 : 16;
+    static constexpr int THREADS = 32 * (EPI + 2 + TILE_QUERY_WARPS + (CONVERT ? TILE_CONV_WARPS : 0));
 };
 
 // Lists of very different lengths are the rule (a list that many queries probe is often a long one): an item is at
@@ -65,7 +70,7 @@ struct alignas(16) TilePair {
 };
 
 struct TileScan {
-    CUtensorMap map;            // the stored rows (not SQ8)
+    CUtensorMap map;            // the stored rows, or their bf16 terms (not SQ8)
     ScanParams s;               // constants; queries (RaBitQ: processed)
     PairTable t;
     const TileItem* items;
@@ -219,6 +224,40 @@ split_bf16x8(const float (&x)[8], uint4& hi, uint4& lo) {
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// fp32 rows (16-byte aligned) -> [rows][2][pitch] bf16 terms, zero past dim; pitch = dim rounded up to 64.  A thread per eight dimensions.
+__global__ void __launch_bounds__(256)
+split_rows_kernel(const uint8_t* __restrict__ rows, uint64_t n, uint32_t dim, uint32_t stride, uint32_t pitch, uint16_t* __restrict__ out) {
+    const uint64_t e = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
+    const uint32_t units = pitch / 8;
+    const uint64_t r = e / units;
+    if (r >= n) {
+        return;
+    }
+    const uint32_t d0 = static_cast<uint32_t>(e - r * units) * 8;
+    const float* src = reinterpret_cast<const float*>(rows + r * stride);
+    float x[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i += 4) {
+        if (d0 + i + 4 <= dim) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(src + d0 + i));
+            x[i] = v.x;
+            x[i + 1] = v.y;
+            x[i + 2] = v.z;
+            x[i + 3] = v.w;
+        } else {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                x[i + j] = d0 + i + j < dim ? __ldg(src + d0 + i + j) : 0.f;
+            }
+        }
+    }
+    uint4 hi, lo;
+    split_bf16x8(x, hi, lo);
+    uint16_t* to = out + r * 2 * pitch + d0;
+    *reinterpret_cast<uint4*>(to) = hi;
+    *reinterpret_cast<uint4*>(to + pitch) = lo;
+}
+
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: 8-row groups of 1 KiB; a k-step of 32 bytes is two
 // 16-byte units further into the line.
 __device__ __forceinline__ uint64_t
@@ -299,6 +338,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
     using F = TileFmt<FMT>;
     constexpr uint32_t STAGE = F::STAGE;
     constexpr uint32_t B_PIECE = F::B_TERMS * QT * TILE_PIECE;
+    constexpr uint32_t COL_STEP = F::EPI / 4 * 8;   // columns that the warps of 32 rows drain at a time
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ TileShared sh;
     // the swizzle permutes by address bits: blocks start on 1 KiB
@@ -317,20 +357,20 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
         }
         for (uint32_t i = 0; i < TILE_DESCS; ++i) {
             mbar_init(&sh.desc_full[i], 1);
-            mbar_init(&sh.desc_free[i], TILE_EPI_WARPS + 1 + TILE_QUERY_WARPS + (F::CONVERT ? TILE_CONV_WARPS : 0));
+            mbar_init(&sh.desc_free[i], F::EPI + 1 + TILE_QUERY_WARPS + (F::CONVERT ? TILE_CONV_WARPS : 0));
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sh.raw_free[i], TILE_CONV_WARPS);
             mbar_init(&sh.item_full[i], TILE_QUERY_WARPS);
-            mbar_init(&sh.item_free[i], TILE_EPI_WARPS);
+            mbar_init(&sh.item_free[i], F::EPI);
             mbar_init(&sh.b_free[i], 1);
             mbar_init(&sh.acc_full[i], 1);
-            mbar_init(&sh.acc_free[i], TILE_EPI_WARPS);
+            mbar_init(&sh.acc_free[i], F::EPI);
         }
         sh.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == TILE_EPI_WARPS) {
+    if (warp == F::EPI) {
         tmem_alloc(&sh.tmem_base, 2 * TILE_ACC_COLS);
     }
     tc_fence_before_sync();
@@ -353,7 +393,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
         return it.len != 0;
     };
 
-    if (warp == TILE_EPI_WARPS + 1) {
+    if (warp == F::EPI + 1) {
         // ---------------- the work queue and the copies of rows ----------------
         const uint32_t n_items = p.queue[0];
         uint32_t stage = 0, phase = 0, filled = 0, raw = 0;
@@ -430,9 +470,9 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                     } else if (lane == 0) {
                         uint64_t* bar = F::CONVERT ? &sh.raw_full[stage] : &sh.full[stage];
                         mbar_expect_tx(bar, STAGE);
-                        if (FMT == ROW_F32) {
+                        if (F::SPLIT) {
                             tma_load_2d(dst, &p.map, piece * 64, it.lbeg + r0, bar);
-                            tma_load_2d(dst + TILE_A_TERM, &p.map, piece * 64 + 32, it.lbeg + r0, bar);
+                            tma_load_2d(dst + TILE_A_TERM, &p.map, FMT == ROW_F32 ? piece * 64 + 32 : (pieces + piece) * 64, it.lbeg + r0, bar);
                         } else {
                             tma_load_2d(dst, &p.map, piece * 64, it.lbeg + r0, bar);
                         }
@@ -448,7 +488,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                 break;
             }
         }
-    } else if (warp == TILE_EPI_WARPS) {
+    } else if (warp == F::EPI) {
         // ---------------- MMA issue (one thread) ----------------
         if (elect_one()) {
             const uint64_t a0 = FMT == ROW_SQ8 ? umma_desc(smem_u32(smem), 128, 1024) : umma_desc_sw128(smem_u32(smem));
@@ -497,7 +537,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                             } else {
                                 umma_bf16(d_tmem, a + ks * A_STEP, b + ks * 2, idesc, accumulate);
                             }
-                            if (FMT == ROW_F32) {   // lo terms of the rows against hi terms of the queries
+                            if (F::SPLIT) {   // lo terms of the rows against hi terms of the queries
                                 umma_bf16(d_tmem, a + (TILE_A_TERM >> 4) + ks * A_STEP, b + ks * 2, idesc_lo, 1u);
                             }
                         }
@@ -522,10 +562,10 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
             }
         }
         __syncwarp();
-    } else if (warp > TILE_EPI_WARPS + 1 && warp < TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS) {
+    } else if (warp > F::EPI + 1 && warp < F::EPI + 2 + TILE_QUERY_WARPS) {
         // ---------------- an item ahead: the queries' terms (B) and constants ----------------
         // Query j belongs to warp j % 4 of the role, lane j / 4 of it: no warp waits for another.
-        const uint32_t qwarp = warp - (TILE_EPI_WARPS + 2);
+        const uint32_t qwarp = warp - (F::EPI + 2);
         const uint32_t j = lane * TILE_QUERY_WARPS + qwarp;
         TileItem it;
         for (uint32_t n = 0; next_item(n, it); ++n) {
@@ -580,9 +620,9 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
             asm volatile("cp.async.wait_all;" ::: "memory");
             tile_publish(&sh.item_full[slot], lane);
         }
-    } else if (F::CONVERT && warp >= TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS) {
+    } else if (F::CONVERT && warp >= F::EPI + 2 + TILE_QUERY_WARPS) {
         // ---------------- stored rows -> operands, in shared memory ----------------
-        const uint32_t cwarp = warp - (TILE_EPI_WARPS + 2 + TILE_QUERY_WARPS);
+        const uint32_t cwarp = warp - (F::EPI + 2 + TILE_QUERY_WARPS);
         constexpr uint32_t ROWS = 128 / TILE_CONV_WARPS;     // of every tile, for a warp
         const uint32_t kc = lane & 7u, rr = cwarp * ROWS + (lane >> 3);   // eight lanes per row, four rows at a time
         uint32_t stage = 0, phase = 0, filled = 0, raw = 0;
@@ -657,9 +697,9 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                 }
             }
         }
-    } else if (warp < TILE_EPI_WARPS) {
-        // ---------------- epilogue: one thread per row of the tile, two warps per 32 rows share the queries ----------------
-        const uint32_t quarter = warp & 3u, half = warp >> 2;
+    } else if (warp < F::EPI) {
+        // ---------------- epilogue: one thread per row of the tile, the warps of 32 rows share the queries ----------------
+        const uint32_t quarter = warp & 3u, share = warp >> 2;
         const uint32_t row = quarter * 32 + lane;
         uint32_t tile = 0;
         TileItem it;
@@ -705,7 +745,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                 const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * TILE_ACC_COLS;
                 if (r0 + quarter * 32 < it.len) {   // (the warp's rows are one group of 32 scores)
                     uint32_t* const scores = reinterpret_cast<uint32_t*>(p.t.scores) + r;
-                    for (uint32_t g = half * 8; g < it.nqt; g += 16) {
+                    for (uint32_t g = share * 8; g < it.nqt; g += COL_STEP) {
                         uint32_t v1[8], v2[8], v3[8];
                         tmem_load_8(taddr + g, v1);
                         if (F::B_TERMS >= 2) {
@@ -741,7 +781,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                                 v = fmaf(x1 * qn2, f * sh.c1[slot][j], fmaf(qn2, qn2, x0));
                             } else {
                                 float ip = __uint_as_float(v1[i]);
-                                if (FMT == ROW_F32) {
+                                if (F::SPLIT) {
                                     ip += __uint_as_float(v2[i]);
                                 }
                                 v = fmaf(p.l2 != 0 ? -2.0f : -1.0f, ip, x0);   // (a negated NaN would rank first)
@@ -780,7 +820,7 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
         tc_drain_pause();   // a wait gave up: let the copies and MMAs still in flight land before the CTA lets go
         __syncthreads();
     }
-    if (warp == TILE_EPI_WARPS) {
+    if (warp == F::EPI) {
         tmem_dealloc(tmem_base, 2 * TILE_ACC_COLS);
     }
 }
