@@ -125,6 +125,17 @@ def test_means_of_clusters_of_all_lengths(engine, oracle, dim):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("dim", [13, 61, 62, 64, 125, 126, 200])     # the three elements behind a row within, at and past a piece of 64
+@pytest.mark.parametrize("offset,spread", [(0.0, 0.2), (40.0, 0.05)])
+def test_training_with_the_bias_among_the_products(engine, oracle, dim, offset, spread):
+    n, k, iters = 1500, 70, 3
+    x = (offset + mixture(43, n, dim, 40, spread)).astype(np.float32)
+    x[5] *= np.float32(30)      # one element far larger than the rest: the others keep few bits
+    want_c, want_l, _, _ = oracle.kmeans_run(x, x[:k].copy(), iters)
+    got_c, got_l, _ = engine.kmeans_train(x, x[:k].copy(), iters)
+    assert np.array_equal(got_l, want_l) and np.array_equal(got_c, want_c)
+
+
 # ---- SQ8 batches that rule lists out -----------------------------------------------------------------------------
 @pytest.mark.parametrize("dim,k", [(16, 10), (96, 16), (96, 17), (112, 48), (128, 49), (130, 112), (130, 113), (256, 10), (300, 10)])
 @pytest.mark.parametrize("metric", [0, 1])

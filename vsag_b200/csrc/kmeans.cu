@@ -261,19 +261,21 @@ kmeans_norms_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, const
     }
 }
 
-// margin[i] = by_shifted * max|c - shift| * |x_i - shift| + by_plain * max|c| * |x_i|, and with `prev` bound[i] = the
-// row's score against its previous centroid, |c'|^2 - 2 <c', x'> over shifted vectors (+inf when it has none).  Eight
+// margin[i] = by_shifted * max|c - shift| * |x_i - shift| + by_plain * max|c| * |x_i| + by_square * max|c - shift|^2, and with `prev`
+// bound[i] = the row's score against its previous centroid, |c'|^2 - 2 <c', x'> over shifted vectors (+inf when it has none), both
+// in units of the products (times `unit`).  Eight
 // lanes per row.  Centroids that do not fit the fp16 scale (limit) leave no column out: the margin becomes infinite.
 __global__ void __launch_bounds__(256)
 kmeans_row_prep_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, const float* __restrict__ shift,
                        const float* __restrict__ c_shifted, const float* __restrict__ cs_sq, uint32_t k, const int32_t* __restrict__ prev,
                        const float* __restrict__ x_norm, const float* __restrict__ xs_norm, const float* __restrict__ extremes,
-                       float by_shifted, float by_plain, float limit, float* __restrict__ margin, float* __restrict__ bound) {
+                       float by_shifted, float by_plain, float by_square, float limit, float unit, float* __restrict__ margin,
+                       float* __restrict__ bound) {
     const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x) >> 3;
     const uint32_t sub = threadIdx.x & 7u;
     if (i < n && sub == 0) {
-        const float m = by_shifted * extremes[1] * xs_norm[i] + by_plain * extremes[2] * x_norm[i];
-        margin[i] = extremes[0] <= limit ? m : INFINITY;
+        const float m = by_shifted * extremes[1] * xs_norm[i] + by_plain * extremes[2] * x_norm[i] + by_square * extremes[1] * extremes[1];
+        margin[i] = extremes[0] <= limit ? m * unit : INFINITY;
     }
     if (prev == nullptr) {
         return;
@@ -308,7 +310,7 @@ kmeans_row_prep_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, co
         ip += __shfl_xor_sync(0xffffffffu, ip, off);
     }
     if (i < n && sub == 0) {
-        bound[i] = l >= 0 && static_cast<uint32_t>(l) < k ? fmaf(-2.0f, ip, __ldg(cs_sq + l)) : INFINITY;
+        bound[i] = l >= 0 && static_cast<uint32_t>(l) < k ? fmaf(-2.0f, ip, __ldg(cs_sq + l)) * unit : INFINITY;
     }
 }
 
@@ -395,7 +397,8 @@ constexpr uint32_t KMEANS_FEW_ROWS = 4096;               // undecided rows that 
 //
 // The scores are |c'|^2 - 2 <c', x'> over vectors minus a common shift (the centroids' mean: it changes no comparison
 // of a row and takes the data's offset out of the errors), with x' and c' rounded to one fp16 term each, scaled so that
-// the largest element is near 2^14: an error of at most 2 (2 * 2^-11 + 2^-22) |x'| |c'| per score.  A column further
+// the largest element is near 2^top: an error of at most 2 (2 * 2^-11 + 2^-22) |x'| |c'| per score, and of the sums, which hold |c'|^2
+// among their products, (dim + 16) 2^-23 |c'|^2 (elements below 2^-14 scaled, 2^-25 of the largest, round absolutely: far less).  A column further
 // than twice that (plus the rounding of the reference's own chain) behind a row's best is not its winner; the columns
 // within are scored exactly.  A third of the MMAs that split bf16 terms take; those (2^-16 of the plain norms) remain for data
 // whose shifted rows still crowd within the fp16 margin -- when more than a sixteenth of the rows came out undecided.
@@ -403,8 +406,12 @@ static int
 kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t dim,
                  const float* centroids_dev, uint32_t k, int32_t* labels_dev, float* best_dev,
                  const int32_t* prev_labels_dev) {
-    const uint32_t chunks = (dim + TC_KC - 1) / TC_KC;
-    const size_t c_elems = tc_tiled_elems(k, dim);
+    const size_t c_elems = tc_tiled_elems(k, dim + TC_BIAS_DIMS);
+    // Elements are scaled to below 2^top: the sum of their squares, whose half is a column's bias, stays below 2^30.
+    int top_exponent = 14;
+    while (top_exponent > 1 && std::ldexp(static_cast<double>(dim), 2 * top_exponent) > std::ldexp(1.0, 30)) {
+        --top_exponent;
+    }
     cudaStream_t st = current_stream();
     const uint32_t norm_blocks = 16u * static_cast<uint32_t>(sm_count());
     VB_TRY(ws.c_hi.reserve(c_elems));
@@ -418,7 +425,7 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
         const bool whole = rows == n;
         const bool cached = whole && ws.tiled_rows == x_dev && ws.tiled_n == n && ws.tiled_dim == dim;
         if (!cached) {
-            const size_t x_elems = tc_tiled_elems(rows, dim);
+            const size_t x_elems = tc_tiled_elems(rows, dim + TC_BIAS_DIMS);
             VB_TRY(ws.x_hi.reserve(x_elems));
             VB_TRY(ws.x_norm.reserve(rows));
             VB_TRY(ws.xs_norm.reserve(rows));
@@ -431,13 +438,13 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
             float top = 0.f;
             VB_CUDA(cudaMemcpyAsync(&top, ws.extremes.ptr, sizeof(float), cudaMemcpyDeviceToHost, st));
             VB_TRY(sync_stream());
-            // a power of two that puts the largest element into [2^13, 2^14); 0: the data do not fit (not finite, or all
-            // rows and centroids alike)
+            // a power of two that puts the largest element into [2^(top - 1), 2^top); 0: the data do not fit (not finite, or
+            // all rows and centroids alike)
             int exponent = 0;
             (void)std::frexp(top, &exponent);
-            ws.scale = top > 0.f && top < INFINITY && exponent > -100 && exponent < 100 ? std::ldexp(1.0f, 14 - exponent) : 0.f;
+            ws.scale = top > 0.f && top < INFINITY && exponent > -50 && exponent < 50 ? std::ldexp(1.0f, top_exponent - exponent) : 0.f;
             if (ws.scale != 0.f && !ws.half_off) {
-                VB_TRY(tc_pretile_f16(x_dev + r0 * dim, rows, dim, ws.shift.ptr, ws.scale, ws.x_hi.ptr));
+                VB_TRY(tc_pretile_f16(x_dev + r0 * dim, rows, dim, ws.shift.ptr, ws.scale, nullptr, ws.x_hi.ptr));
             } else {
                 VB_TRY(ws.x_lo.reserve(x_elems));
                 VB_TRY(tc_pretile_f32(x_dev + r0 * dim, rows, dim, ws.x_hi.ptr, ws.x_lo.ptr));
@@ -454,9 +461,10 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
         VB_LAUNCH(kmeans_norms_kernel, std::min(norm_blocks, (k + 7) / 8), 256, 0, centroids_dev, k, dim, ws.shift.ptr,
                   static_cast<float*>(nullptr), static_cast<float*>(nullptr), ws.c_shifted.ptr, ws.extremes.ptr, ws.extremes.ptr + 1);
         VB_TRY(row_sqnorm_f32(ws.c_shifted.ptr, k, dim, ws.cs_sq.ptr));
-        TcOperand a{ws.x_hi.ptr, half ? nullptr : ws.x_lo.ptr, rows, chunks}, b{ws.c_hi.ptr, nullptr, k, chunks};
+        const uint32_t depth = half ? dim + TC_BIAS_DIMS : dim, chunks = (depth + TC_KC - 1) / TC_KC;
+        TcOperand a{ws.x_hi.ptr, half ? nullptr : ws.x_lo.ptr, rows, chunks, depth}, b{ws.c_hi.ptr, nullptr, k, chunks, depth};
         if (half) {
-            VB_TRY(tc_pretile_f16(centroids_dev, k, dim, ws.shift.ptr, ws.scale, ws.c_hi.ptr));
+            VB_TRY(tc_pretile_f16(centroids_dev, k, dim, ws.shift.ptr, ws.scale, ws.cs_sq.ptr, ws.c_hi.ptr));
         } else {
             VB_TRY(ws.c_lo.reserve(c_elems));
             VB_TRY(tc_pretile_f32(centroids_dev, k, dim, ws.c_hi.ptr, ws.c_lo.ptr));
@@ -469,12 +477,13 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
         VB_LAUNCH(kmeans_row_prep_kernel, static_cast<uint32_t>((rows * 8 + 255) / 256), 256, 0, x_dev + r0 * dim, rows, dim, ws.shift.ptr,
                   ws.c_shifted.ptr, ws.cs_sq.ptr, k, prev_labels_dev != nullptr ? prev_labels_dev + r0 : nullptr, ws.x_norm.ptr,
                   half ? ws.xs_norm.ptr : ws.x_norm.ptr, ws.extremes.ptr, half ? 4.0e-3f : 1e-3f, chain,
-                  half ? 60000.0f / ws.scale : INFINITY, ws.row_margin.ptr, ws.row_bound.ptr);
+                  half ? static_cast<float>(dim + 16) * 2.4e-7f : 0.f, half ? std::ldexp(1.4f, top_exponent) / ws.scale : INFINITY,
+                  half ? 0.5f * ws.scale * ws.scale : 1.0f, ws.row_margin.ptr, ws.row_bound.ptr);
         const float* row_bound = prev_labels_dev != nullptr ? ws.row_bound.ptr : nullptr;
         uint32_t n_split = 1, n_flagged = 0;
         VB_TRY(ws.row_flags.reserve(rows));
         VB_CUDA(cudaMemsetAsync(ws.row_flags.ptr, 0, rows * sizeof(uint32_t), st));
-        VB_TRY(tc_candidates(ws.tc, a, b, half ? TC_HALF : 3, half ? -2.0f / (ws.scale * ws.scale) : -2.0f, ws.cs_sq.ptr, m, 0, ws.cand,
+        VB_TRY(tc_candidates(ws.tc, a, b, half ? TC_HALF : 3, half ? 1.0f : -2.0f, half ? static_cast<const float*>(nullptr) : ws.cs_sq.ptr, m, 0, ws.cand,
                              &n_split, ws.row_margin.ptr, row_bound, ws.row_flags.ptr, &n_flagged));
         const uint32_t per_row = n_split * m;
         float* best = best_dev != nullptr ? best_dev + r0 : nullptr;

@@ -38,11 +38,13 @@ widen_in(uint16_t v) {  // bf16 bit pattern
 // so a [128 x 64] chunk is 16 KiB contiguous: 8x8-element cores of 128 B, the 8 cores of an 8-row
 // group back to back (1 KiB per group).  Out-of-range rows / dimensions are zero.
 // ---------------------------------------------------------------------------------------------
+// HALF: (x - shift) * scale as fp16, and behind the last dimension three elements that add a column's bias to its products
+// (tc_pretile_f16): constants in the rows that sign is -1 for, else the bias as three fp16 terms.
 template <typename T, bool SPLIT, bool HALF = false>
 __global__ void
 tc_pretile_kernel(const T* __restrict__ src, uint64_t rows, uint32_t dim, uint32_t chunks,
                   uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, uint64_t total_units,
-                  const float* __restrict__ shift, float scale) {
+                  const float* __restrict__ shift, float scale, float sign, const float* __restrict__ bias) {
     uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // one 8-element core row
     if (u >= total_units) {
         return;
@@ -63,7 +65,23 @@ tc_pretile_kernel(const T* __restrict__ src, uint64_t rows, uint32_t dim, uint32
             x = widen_in(src[r * dim + e0 + i]);
         }
         if (HALF) {
-            h[i] = r < rows && e0 + i < dim ? __half_as_ushort(__float2half_rn(fminf(fmaxf((x - __ldg(shift + e0 + i)) * scale, -65504.0f), 65504.0f))) : uint16_t{0};
+            const uint32_t e = e0 + i;
+            float v = 0.f;
+            if (r < rows && e < dim) {
+                v = sign * (x - __ldg(shift + e)) * scale;
+            } else if (r < rows && e < dim + TC_BIAS_DIMS) {
+                const uint32_t term = e - dim;
+                if (bias == nullptr) {
+                    v = term == 0 ? 32768.0f : (term == 1 ? 16.0f : 0.0078125f);   // 2^15, 2^4, 2^-7
+                } else {
+                    // bias * scale^2 / 2 = 2^15 (t0 + 2^-11 t1 + 2^-22 t2)
+                    v = __ldg(bias + r) * (scale * 0.5f) * scale * (1.0f / 32768.0f);
+                    for (uint32_t j = 0; j < term; ++j) {
+                        v = (v - __half2float(__float2half_rn(v))) * 2048.0f;
+                    }
+                }
+            }
+            h[i] = __half_as_ushort(__float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f)));
             continue;
         }
         __nv_bfloat16 bh = __float2bfloat16_rn(x);
@@ -102,10 +120,12 @@ pretile_launch(const T* src, uint64_t rows, uint32_t dim, uint16_t* hi, uint16_t
     VB_CHECK_ARG(blocks <= 0x7fffffffu, "pretile: matrix too large");
     if (lo != nullptr) {
         auto kernel = tc_pretile_kernel<T, true>;
-        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units, static_cast<const float*>(nullptr), 1.0f);
+        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units, static_cast<const float*>(nullptr), 1.0f, 1.0f,
+                  static_cast<const float*>(nullptr));
     } else {
         auto kernel = tc_pretile_kernel<T, false>;
-        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units, static_cast<const float*>(nullptr), 1.0f);
+        VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src, rows, dim, chunks, hi, lo, units, static_cast<const float*>(nullptr), 1.0f, 1.0f,
+                  static_cast<const float*>(nullptr));
     }
     return 0;
 }
@@ -116,15 +136,16 @@ tc_pretile_f32(const float* src_dev, uint64_t rows, uint32_t dim, uint16_t* hi_d
 }
 
 int
-tc_pretile_f16(const float* src_dev, uint64_t rows, uint32_t dim, const float* shift_dev, float scale, uint16_t* dst_dev) {
+tc_pretile_f16(const float* src_dev, uint64_t rows, uint32_t dim, const float* shift_dev, float scale, const float* bias_dev,
+               uint16_t* dst_dev) {
     if (rows == 0) {
         return 0;
     }
-    const uint64_t units = tc_tiled_elems(rows, dim) / 8, blocks = (units + 255) / 256;
+    const uint64_t units = tc_tiled_elems(rows, dim + TC_BIAS_DIMS) / 8, blocks = (units + 255) / 256;
     VB_CHECK_ARG(blocks <= 0x7fffffffu, "pretile: matrix too large");
     auto kernel = tc_pretile_kernel<float, false, true>;
-    VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src_dev, rows, dim, (dim + TC_KC - 1) / TC_KC, dst_dev,
-              static_cast<uint16_t*>(nullptr), units, shift_dev, scale);
+    VB_LAUNCH(kernel, static_cast<uint32_t>(blocks), 256, 0, src_dev, rows, dim, (dim + TC_BIAS_DIMS + TC_KC - 1) / TC_KC, dst_dev,
+              static_cast<uint16_t*>(nullptr), units, shift_dev, scale, bias_dev != nullptr ? 1.0f : -1.0f, bias_dev);
     return 0;
 }
 
@@ -563,6 +584,12 @@ tc_candidates_kernel(const TcParams p) {
                                 const float4 b4 = *reinterpret_cast<const float4*>(&sh.bias[warp][i]);
                                 fma_pair(sc[i], sc[i + 1], __uint_as_float(r[i]), __uint_as_float(r[i + 1]), p.alpha, b4.x, b4.y);
                                 fma_pair(sc[i + 2], sc[i + 3], __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]), p.alpha, b4.z, b4.w);
+                            }
+                        } else if (SMALL_M && p.half != 0) {
+                            // (the products hold the bias and the sign already)
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                sc[i] = __uint_as_float(r[i]);
                             }
                         } else {
 #pragma unroll

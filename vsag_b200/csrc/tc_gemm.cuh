@@ -286,7 +286,7 @@ umma_idesc_f16(uint32_t m, uint32_t n) {
     return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
-constexpr uint32_t TC_HALF = 2;   // n_terms of tc_candidates for one scaled fp16 term per operand
+constexpr uint32_t TC_HALF = 2;   // n_terms of tc_candidates for one scaled fp16 term per operand (tc_pretile_f16; no alpha, no bias)
 
 // ---- host API (tc_gemm.cu) ------------------------------------------------------------------
 
@@ -302,8 +302,14 @@ int tc_pretile_f32(const float* src_dev, uint64_t rows, uint32_t dim, uint16_t* 
 // bf16 rows (bit patterns) -> tiled layout.
 int tc_pretile_bf16(const uint16_t* src_dev, uint64_t rows, uint32_t dim, uint16_t* hi_dev);
 
-// (fp32 rows - shift) * scale (a power of two) -> one fp16 term in the tiled layout; shift[dim] on the device.
-int tc_pretile_f16(const float* src_dev, uint64_t rows, uint32_t dim, const float* shift_dev, float scale, uint16_t* dst_dev);
+// Rows for scores that need no arithmetic after the products: columns are (c - shift) * scale as fp16 and three terms of
+// bias * scale^2 / 2 behind them, rows -(x - shift) * scale and three constants, so that a product is
+// (bias - 2 <c - shift, x - shift>) * scale^2 / 2.  (The epilogue's multiply-add per score and the columns' biases it reads were a quarter of
+// its instructions.)  scale: a power of two with sum of (c - shift)^2 scale^2 below 2^31; shift[dim] on the device; bias null: rows.
+// The operands have dim + TC_BIAS_DIMS elements a row.
+constexpr uint32_t TC_BIAS_DIMS = 3;
+int tc_pretile_f16(const float* src_dev, uint64_t rows, uint32_t dim, const float* shift_dev, float scale, const float* bias_dev,
+                   uint16_t* dst_dev);
 
 struct TcWorkspace {
     DevBuf<uint64_t> scratch;
@@ -313,7 +319,8 @@ struct TcWorkspace {
 // For every row of A the m best columns of B by alpha * <a, b> + bias, as keys in
 // out_dev[a_rows][lists][m]; the number of lists per row is
 // chosen here and returned in n_split_out.
-// n_terms: 1, 3, or TC_HALF for one scaled fp16 term per operand (alpha then undoes the scales).
+// n_terms: 1, 3, or TC_HALF for one scaled fp16 term per operand (m <= 4; scores, margins and bounds are then times scale^2 / 2, alpha 1 and
+// no bias).
 // row_margin_dev (optional, m <= 4 only): per row twice the largest error of a score; columns scoring worse than the
 // row's best by more than that are not nominated at all.  row_bound_dev (optional): with the margin (m <= 4), per
 // row the exact score of some column: nothing worse than it plus the margin is visited; with m > 4, per row a score
