@@ -18,7 +18,7 @@ constexpr uint32_t SELECT_GROUPS = 1024;          // group minima kept at most
 constexpr uint32_t SELECT_CAP = 2048;             // values collected at most
 constexpr uint32_t SELECT_RANKED = 256;           // keys sorted by counting, at most
 
-struct SelectScratch {
+struct alignas(16) SelectScratch {
     uint32_t hist[SELECT_BINS];
     uint32_t minima[SELECT_GROUPS];   // per group; the second pass reads them again
     uint32_t warp_part[32];

@@ -3087,7 +3087,8 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
         const uint8_t* drop = nullptr;
         if (pruning) {
             VB_TRY(ws.pair_drop.reserve(total));
-            VB_LAUNCH(pair_drop_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, probes_dev, total, nprobe,
+            // (two warps a CTA: how many pairs a warp has to test differs, and the CTA waits for all of them; 256 threads 153 us)
+            VB_LAUNCH(pair_drop_kernel, static_cast<uint32_t>((total + 63) / 64), 64, 0, probes_dev, total, nprobe,
                       ws.first_live.ptr, nlist, ix->shard_rank, ix->shard_world, ix->list_off.ptr, q_dev, ix->dim,
                       ix->ball_centre.ptr, ix->ball_radius.ptr, ix->ball_count.ptr, ws.thr.ptr, ix->metric,
                       ix->code_size, probe_dists_dev, ix->list_radius.ptr,

@@ -885,13 +885,15 @@ record_exact_distance(const uint8_t* rec, uint32_t dim, uint32_t row_bytes, cons
 // bounding the difference between score and exact distance, so when the kscan-th exact distance is below that the
 // result is the exact one.  Otherwise (scores crowded within the rounding of the arithmetic) every row of the query
 // is scored exactly here.
+// (seven CTAs an SM take 1000 queries together, 57 -> 41 us; the one-bit chain wants the registers, 244 -> 256)
 template <int FMT, bool L2, bool APPROX>
-__global__ void __launch_bounds__(PAIR_THREADS)
+__global__ void __launch_bounds__(PAIR_THREADS, FMT == ROW_RABITQ ? 5 : 7)
 scan_finalize_kernel(const ScanFinalize p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ SelectScratch sel;
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
-    __shared__ __align__(16) uint64_t best[1024];
+    // (sorted results take the place of the selection's histogram and minima, which are done with by then: seven CTAs an SM)
+    uint64_t* const best = reinterpret_cast<uint64_t*>(sel.hist);
     __shared__ uint32_t group_ids[APPROX ? FINAL_GROUPS : 1];
     __shared__ float part[PAIR_THREADS / 32];
     const PairScan& sc = p.scan;
