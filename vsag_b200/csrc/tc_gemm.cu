@@ -487,7 +487,7 @@ tc_candidates_kernel(const TcParams p) {
             uint32_t m_tile32, split32, tiles32;
             open_item(static_cast<uint32_t>(item), m_tile32, split32, tiles32);
             const uint64_t m_tile = m_tile32, split = split32;
-            const uint64_t t0 = 0, t1 = tiles32;   // the item's B tiles by their number within its share
+            const uint32_t t0 = 0, t1 = tiles32;   // the item's B tiles by their number within its share
             const uint64_t grow = m_tile * TC_BM + row;
             const bool valid_row = grow < p.a.rows;
             uint32_t cnt = 0;
@@ -503,16 +503,19 @@ tc_candidates_kernel(const TcParams p) {
             // bias of the warp's columns: fetched a whole step ahead into registers (lane = column of a block of 32), handed
             // to the other lanes through the warp's own shared-memory slot.  (A block ahead is less than L2 takes.)
             const bool has_bias = p.bias != nullptr;
-            // first global column of this warp's block `half` in the tile step that starts at B tile t
-            auto block_col = [&](uint64_t t, uint32_t half) -> uint64_t {
-                const uint32_t col = cgroup * warp_cols + half * 32;   // within the step's columns
-                return static_cast<uint64_t>(tile_at(split32, static_cast<uint32_t>(t) + col / TC_BN)) * TC_BN + col % TC_BN;
-            };
+            // This warp's columns of a step lie in one B tile, the step's first or second.  (32 bits and sums throughout: the block's
+            // address, worked out anew, was a tenth of the instructions.)
+            const uint32_t b_rows = static_cast<uint32_t>(p.b.rows);
+            const uint32_t in_step = cgroup * warp_cols / TC_BN, in_tile = cgroup * warp_cols % TC_BN;
+            const uint32_t tile0 = p.interleaved ? split32 : split32 * p.tiles_per_split, tile_inc = p.interleaved ? p.n_split : 1u;
+            // first global column of this warp in the tile step that starts at B tile t; its second block of 32 follows
+            auto first_col = [&](uint32_t t) -> uint32_t { return (tile0 + (t + in_step) * tile_inc) * p.tile_stride * TC_BN + in_tile; };
             float bias0 = 0.f, bias1 = 0.f, next0 = 0.f, next1 = 0.f;
-            auto bias_of = [&](uint64_t t, uint32_t half) -> float {
-                const uint64_t nn = t < t1 ? block_col(t, half) + lane : p.b.rows;
-                return nn < p.b.rows ? __ldg(p.bias + nn) : 0.f;
+            auto bias_of = [&](uint32_t t, uint32_t half) -> float {
+                const uint32_t nn = t < t1 ? first_col(t) + half * 32 + lane : b_rows;
+                return nn < b_rows ? __ldg(p.bias + nn) : 0.f;
             };
+            const bool rows_whole = __all_sync(0xffffffffu, valid_row);
             if (has_bias) {
                 next0 = bias_of(t0, 0);
                 next1 = step == 2 ? bias_of(t0, 1) : 0.f;
@@ -522,7 +525,7 @@ tc_candidates_kernel(const TcParams p) {
             const float margin = (SMALL_M && p.row_margin != nullptr && valid_row) ? __ldg(p.row_margin + grow) : -1.f;
             float bound = (margin >= 0.f && p.row_bound != nullptr) ? __ldg(p.row_bound + grow) + margin : INFINITY;
             uint32_t bc0 = 0xFFFFFFFFu, bc1 = 0xFFFFFFFFu, bc2 = 0xFFFFFFFFu, bc3 = 0xFFFFFFFFu;
-            for (uint64_t t = t0; t < t1 && ok; t += step, ++gtile) {
+            for (uint32_t t = t0; t < t1 && ok; t += step, ++gtile) {
                 const uint32_t acc = static_cast<uint32_t>(gtile & 1);
                 if (has_bias) {
                     bias0 = next0;
@@ -535,13 +538,12 @@ tc_candidates_kernel(const TcParams p) {
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t here = (t1 - t >= step) ? step : 1u;              // B tiles in this step
+                const bool tile_present = t + in_step < t1;                      // the warp's B tile exists
+                const uint32_t col0 = first_col(t);
                 for (uint32_t half = 0; half < step; ++half) {
-                const uint32_t step_col = cgroup * warp_cols + half * 32;
-                const bool tile_present = step_col / TC_BN < here;              // the block's B tile exists
-                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * acc_cols + step_col;
-                const uint64_t n0 = block_col(t, half);
-                const bool whole_tile = valid_row && tile_present && n0 + 32 <= p.b.rows;
+                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * acc_cols + cgroup * warp_cols + half * 32;
+                const uint32_t c0 = col0 + half * 32;
+                const bool cols_whole = tile_present && c0 + 32 <= b_rows, whole_tile = valid_row && cols_whole;
                 if (has_bias) {
                     __syncwarp();
                     sh.bias[warp][lane] = half == 0 ? bias0 : bias1;
@@ -572,11 +574,10 @@ tc_candidates_kernel(const TcParams p) {
                         continue;
                     }
 #endif
-                    const uint32_t c0 = static_cast<uint32_t>(n0);
                     // Scores of the block and their minimum first (two instructions per element);
                     // the selection code below runs only when the minimum beats the row's bound.
                     float sc[32];
-                    if (__all_sync(0xffffffffu, whole_tile)) {
+                    if (rows_whole && cols_whole) {
                         // the common case: every row and column of the block exists
                         if (has_bias) {
 #pragma unroll
@@ -599,7 +600,7 @@ tc_candidates_kernel(const TcParams p) {
                         }
                     } else {
                         const uint32_t cols_left = (tile_present && c0 < p.b.rows)
-                                                       ? static_cast<uint32_t>(min(static_cast<uint64_t>(32), p.b.rows - c0))
+                                                       ? min(32u, b_rows - c0)
                                                        : 0u;
 #pragma unroll
                         for (int i = 0; i < 32; i += 4) {
@@ -657,8 +658,7 @@ tc_candidates_kernel(const TcParams p) {
                     const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
                     if (MINIMA) {
                         if (valid_row && tile_present) {
-                            p.store[grow * p.store_ld + number_at(split32, static_cast<uint32_t>(t) + step_col / TC_BN) * (TC_BN / 32) +
-                                    step_col % TC_BN / 32] = mn;
+                            p.store[grow * p.store_ld + number_at(split32, t + in_step) * (TC_BN / 32) + in_tile / 32 + half] = mn;
                         }
                         continue;
                     }
