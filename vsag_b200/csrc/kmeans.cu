@@ -1085,17 +1085,17 @@ kpp_run_rounds(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, uint64_
     if (resident) {
         p.per = resident_per;
     } else {
-        const uint64_t most = std::min<uint64_t>(std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, 32 * kpp_run(false)), (n + RS_ROWS - 1) / RS_ROWS);
+        const uint64_t most = std::min<uint64_t>(std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, RS_ROWS * KPP_RUN), (n + RS_ROWS - 1) / RS_ROWS);
         p.per = (n + most - 1) / most;
     }
     const uint64_t grid = (n + p.per - 1) / p.per;
-    if (grid > 32 * kpp_run(resident)) {
+    if (grid > (resident ? 32 : RS_ROWS) * KPP_RUN || (!resident && n > 0xFFFFFFFFull)) {   // (a row's number is a word of 32 bits)
         return 0;
     }
     p.first = first;
     DevBuf<double> draws;
-    DevBuf<unsigned long long> words;   // the sums' two sets, the row's, and whether a wait gave up
-    const size_t n_words = 4 * grid + dim + 1;
+    DevBuf<unsigned long long> words;   // the sums' two sets, the row's, whether a wait gave up, and the sums' count
+    const size_t n_words = 4 * grid + dim + 2;
     VB_TRY(draws.reserve(k));
     VB_TRY(words.reserve(n_words));
     VB_CUDA(cudaMemsetAsync(words.ptr, 0, n_words * sizeof(unsigned long long), current_stream()));
@@ -1105,6 +1105,7 @@ kpp_run_rounds(const float* x_dev, uint64_t n, uint32_t dim, uint32_t k, uint64_
     p.part = words.ptr;
     p.row = words.ptr + 4 * grid;
     p.failed = reinterpret_cast<uint32_t*>(words.ptr + 4 * grid + dim);
+    p.count = words.ptr + 4 * grid + dim + 1;
     p.spin_limit = tc_spin_limit();
     p.centroids = centroids_dev;
     p.picked = picked_dev;

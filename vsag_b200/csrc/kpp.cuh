@@ -11,7 +11,10 @@
 // which the sums, the pick and then its row were read, 7.05 us a round of 64,000 x 96 rows; 5.5 this way.)  The words of two
 // rounds do not meet: a CTA writes its sum of round r + 2 when it has the row of round r + 1, to which every CTA's sum of that
 // round belongs, written after it had read all sums of round r; there are two sets of them.  One warp of a CTA reads the sums: with
-// a thread for each, 148 CTAs' polls of the same few lines held one another up.
+// a thread for each, 148 CTAs' polls of the same few lines held one another up.  So do the polls of four CTAs an SM, which the streamed form
+// has, while some still wait for rows: there the sums are counted in, and one thread of a CTA polls the count and then the
+// number of the row (a round of 285,015 x 145 rows: 48 us
+// with grid barriers, 74 with polled sums, 42.6 this way).
 #pragma once
 
 #include "block_select.cuh"
@@ -19,10 +22,28 @@
 
 namespace vb200 {
 
-// CTAs whose sums a lane of the first warp reads; so the launch has 32 times that many at most.
-constexpr uint32_t
-kpp_run(bool resident) {
-    return resident ? 5 : 20;
+// CTAs whose sums a lane of the first warp reads (streamed: a thread of the CTA); so the launch has 32 (RS_ROWS) times that many at most.
+constexpr uint32_t KPP_RUN = 5;
+
+// Counts this CTA's sum in and waits until all have been; false when they do not come.
+__device__ __forceinline__ bool
+kpp_count_in(unsigned long long* count, unsigned long long all, uint32_t limit) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
+    for (uint32_t spin = 0; spin < limit; ++spin) {
+        unsigned long long seen;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(count) : "memory");
+        if (seen >= all) {
+            return true;
+        }
+    }
+    return false;
+}
+
+__device__ __forceinline__ double
+kpp_sum_of(const unsigned long long* at) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(at) : "memory");
+    return v;
 }
 
 struct KppRounds {
@@ -33,8 +54,9 @@ struct KppRounds {
     uint64_t first;               // the row picked in round 0
     const double* u;              // [k] the rounds' uniform draws (entry 0 unused)
     float* min_d;                 // [n] squared distance to the nearest centre (streamed form)
-    unsigned long long* part;     // [2][grid][2] words of the partial sums; zero before the launch
-    unsigned long long* row;      // [dim] words of the picked row; zero before the launch
+    unsigned long long* part;     // [2][grid][2] words of the partial sums (streamed: the sums, in [0]); zero before the launch
+    unsigned long long* count;    // [1] sums counted in (streamed form); zero before the launch
+    unsigned long long* row;      // [dim] words of the picked row (streamed: [0] its number); zero before the launch
     float* centroids;             // [k x dim]
     int64_t* picked;              // [k] or null
     uint32_t* state;              // [0] first round that found no row apart from the centres (0xFFFFFFFF: none)
@@ -158,7 +180,7 @@ kpp_rounds_kernel(const KppRounds p) {
         }
     }
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr uint32_t RUN = kpp_run(RESIDENT);
+    constexpr uint32_t RUN = KPP_RUN;
     bool ok = true;
     for (uint32_t round = 1; round < p.k; ++round) {
         // distances: difference, then one FMA per dimension in ascending order
@@ -226,7 +248,58 @@ kpp_rounds_kernel(const KppRounds p) {
         }
         __syncthreads();
         unsigned long long* part = p.part + static_cast<size_t>(round & 1u) * grid * 2;
-        if (warp == 0) {
+        if (!RESIDENT) {
+            if (threadIdx.x == 0) {
+                double v = 0.0;
+                for (uint32_t w = 0; w < T / 32; ++w) {
+                    v += scan[w];
+                }
+                asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(part + blockIdx.x * 2), "d"(v) : "memory");
+                ok = kpp_count_in(p.count, static_cast<unsigned long long>(round) * grid, p.spin_limit);
+                s_owner = 0xFFFFFFFFu;
+                s_row = ~0ull;
+            }
+            if (__syncthreads_or(ok ? 0 : 1) != 0) {
+                break;
+            }
+            const uint32_t g0 = threadIdx.x * RUN;
+            double in[RUN], local = 0.0;
+#pragma unroll
+            for (uint32_t i = 0; i < RUN; ++i) {
+                in[i] = g0 + i < grid ? kpp_sum_of(part + (g0 + i) * 2) : 0.0;
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < RUN; ++i) {
+                local += in[i];
+            }
+            const double upto = block_inclusive_sum_f64<T>(local, scan);
+            if (threadIdx.x == T - 1) {
+                s_total = upto;
+                s_thr = upto * __ldg(p.u + round);
+            }
+            __syncthreads();
+            // (every thread whose run ends at or past the threshold names the first CTA of its run that does; the least counts)
+            uint32_t first = 0xFFFFFFFFu;
+            double base = upto - local;
+            if (upto >= s_thr && g0 < grid) {
+#pragma unroll
+                for (uint32_t i = 0; i < RUN; ++i) {
+                    if (first == 0xFFFFFFFFu && g0 + i < grid) {
+                        const double next = base + in[i];
+                        if (next >= s_thr || i + 1 == RUN || g0 + i + 1 == grid) {
+                            first = g0 + i;
+                        } else {
+                            base = next;
+                        }
+                    }
+                }
+                atomicMin(&s_owner, first);
+            }
+            __syncthreads();
+            if (first != 0xFFFFFFFFu && first == s_owner) {
+                s_base = base;
+            }
+        } else if (warp == 0) {
             double v = lane < T / 32 ? scan[lane] : 0.0;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -336,14 +409,29 @@ kpp_rounds_kernel(const KppRounds p) {
                 }
                 pick = s_row != ~0ull ? s_row : row0 + mine - 1;
             }
+            if (!RESIDENT && threadIdx.x == 0) {
+                kpp_put(p.row, static_cast<uint32_t>(pick), round);
+            }
             for (uint32_t d = threadIdx.x; d < dim; d += T) {
                 const float v = RESIDENT ? rows[(pick - row0) * stride + d] : __ldg(p.x + pick * dim + d);
-                kpp_put(p.row + d, __float_as_uint(v), round);
+                if (RESIDENT) {
+                    kpp_put(p.row + d, __float_as_uint(v), round);
+                }
                 c[d] = v;
                 p.centroids[static_cast<uint64_t>(round) * dim + d] = v;
             }
             if (threadIdx.x == 0 && p.picked != nullptr) {
                 p.picked[round] = static_cast<int64_t>(pick);
+            }
+        } else if (!RESIDENT) {
+            if (threadIdx.x == 0) {
+                s_row = kpp_get(p.row, round, p.spin_limit, &ok);
+            }
+            if (__syncthreads_or(ok ? 0 : 1) != 0) {
+                break;
+            }
+            for (uint32_t d = threadIdx.x; d < dim; d += T) {
+                c[d] = __ldg(p.x + s_row * dim + d);
             }
         } else {
             for (uint32_t d = threadIdx.x; d < dim; d += T) {
