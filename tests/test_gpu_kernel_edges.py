@@ -169,3 +169,25 @@ def test_tiles_equal_queries_one_by_one(engine, oracle, quant, dim, nq):
     got = ix.search_filtered(q, k, 3, bucket_ids=lists)
     one = [ix.search_filtered(q[i:i + 1].copy(), k, 3, bucket_ids=lists[:1]) for i in range(nq)]
     exactly(got, (np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])))
+
+
+# ---- SQ8 lists that two to four queries share ---------------------------------------------------------------------
+@pytest.mark.parametrize("metric", [0, 1])
+@pytest.mark.parametrize("dim,nq", [(16, 19), (100, 15), (130, 19), (528, 12), (2049, 10)])
+def test_rows_streamed_for_several_queries(engine, dim, nq, metric):
+    """Lists of one row, of 128, of an item (256 rows) and one more, of several items, with up to as many queries as come, and bytes
+    enough in all (1.5e8); with and without a filter the results are those of the queries one by one."""
+    sizes = [1, 5, 128, 129, 256, 257, 700] + [int(1.6e8 * 50 / (nq * 10 * dim)) // 43] * 43
+    labels = np.repeat(np.arange(50, dtype=np.int32), sizes)
+    n, k, nprobe = labels.size, 12, 10
+    x, q = mixture(71, n, dim, 9, 0.4), mixture(72, nq, dim, 9, 0.4)
+    ix = engine.IvfHandle(dim, metric, 50, engine.QUANT_SQ8)
+    ix.train(x, iters=1, init=np.ascontiguousarray(x[:50]))
+    ix.add(x, np.arange(n, dtype=np.int64), labels=labels)
+    rng = np.random.default_rng(dim)
+    lists = np.stack([rng.permutation(np.r_[np.arange(7), rng.choice(np.arange(7, 50), 3, replace=False)]) for _ in range(nq)]).astype(np.int32)
+    gone = np.full((n + 31) // 32, 0x11111111, np.uint32)
+    for bits in (None, gone):
+        got = ix.search_filtered(q, k, nprobe, bucket_ids=lists, deny_inner_bits=bits)
+        one = [ix.search_filtered(q[i:i + 1].copy(), k, nprobe, bucket_ids=lists[i:i + 1], deny_inner_bits=bits) for i in range(nq)]
+        exactly(got, (np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])))

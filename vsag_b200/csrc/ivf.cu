@@ -3240,6 +3240,9 @@ ivf_search_keys(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, ui
 // Bytes of host inputs and results that pass through pinned memory of the handle: below this the copies of
 // pageable memory cost more in driver time than the transfer itself.
 constexpr size_t PINNED_IO_BYTES = 256 * 1024;
+// From two queries per probed list on SQ8 rows are streamed for several of them, where the rows are bytes enough to pay for the grouping
+// (as pairs / shared, us: 384 MB of rows 252 / 218, 600 MB 267 / 245, 180 MB 447 / 354, 200 MB 254 / 250; 128 MB 202 / 201, 19 MB 89 / 95).
+constexpr double SHARED_MIN_QUERIES = 2.0, SHARED_MIN_BYTES = 1.5e8;
 constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which tiles pay (3.1: 141 us as pairs, 162 as tiles)
 
 // Shared memory of pair_scan_kernel and of scan_finalize_kernel; qstride: floats of a query as the codec's chain reads it (the
@@ -3374,25 +3377,25 @@ position_mask_kernel(const ScanParams p, uint64_t n, uint32_t* __restrict__ mask
     }
 }
 
-// Groups the pairs by list and scans the lists as tiles into the score buffer.
+// Groups the pairs by list: items of up to `segment` rows against up to qt queries each.
 static int
-launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& plan) {
+group_by_list(vb200_ivf* ix, const PairScan& sc, uint64_t nq, uint32_t qt, uint32_t segment, TileGroup* out, uint64_t* max_items) {
     SearchWorkspace& ws = ix->ws;
     const uint32_t nlist = ix->nlist, nprobe = sc.nprobe;
     const uint64_t pairs = nq * nprobe;
     // sum over lists of ceil(pairs / qt) * ceil(rows / segment), from above
-    const uint64_t max_items = nq * sc.t.stride / (static_cast<uint64_t>(plan.qt) * TILE_SEGMENT) + pairs / plan.qt +
-                               ix->n_stored / TILE_SEGMENT + std::min<uint64_t>(pairs, nlist) + 1;
+    *max_items = nq * sc.t.stride / (static_cast<uint64_t>(qt) * segment) + pairs / qt + ix->n_stored / segment + std::min<uint64_t>(pairs, nlist) + 1;
     VB_TRY(ws.tile_tables.reserve(3 * static_cast<size_t>(nlist) + 2));
     VB_TRY(ws.tile_pairs.reserve(pairs));
-    VB_TRY(ws.tile_items.reserve(max_items));
+    VB_TRY(ws.tile_items.reserve(*max_items));
     TileGroup g{};
     g.count = ws.tile_count.ptr;
     g.rank = ws.tile_rank.ptr;
     g.probes = sc.probes;
     g.pairs = static_cast<uint32_t>(pairs);
     g.nlist = nlist;
-    g.qt = plan.qt;
+    g.qt = qt;
+    g.segment = segment;
     g.order = ix->scan_order.ptr;
     g.list_off = ix->list_off.ptr;
     g.pair_off = ws.tile_tables.ptr;
@@ -3406,6 +3409,38 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     g.group_off = ix->quant == VB200_QUANT_SQ8 ? ix->group_off.ptr : nullptr;
     VB_LAUNCH(tile_places_kernel, 1, 1024, 0, g);
     VB_LAUNCH(tile_scatter_kernel, static_cast<uint32_t>((std::max<uint64_t>(pairs, nlist) + 255) / 256), 256, 0, g);
+    *out = g;
+    return 0;
+}
+
+static size_t
+shared_scan_smem(const vb200_ivf* ix) {
+    return RS_STAGES * RS_STAGE + SHARED_QUERIES * 3 * static_cast<size_t>(ix->dpad);
+}
+
+// The scan of SQ8 lists whose rows a few queries share, into the score buffer.
+static int
+launch_shared_scan(vb200_ivf* ix, const PairScan& sc, uint64_t nq) {
+    TileGroup g{};
+    uint64_t max_items = 0;
+    VB_TRY(group_by_list(ix, sc, nq, SHARED_QUERIES, SHARED_SEGMENT, &g, &max_items));
+    auto kernel = ix->metric == VB200_METRIC_L2 ? shared_scan_kernel<true> : shared_scan_kernel<false>;
+    const size_t smem = shared_scan_smem(ix);
+    VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
+    int per_sm = 0;
+    VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, RS_ROWS, smem));
+    const uint64_t grid = std::min<uint64_t>(max_items, static_cast<uint64_t>(sm_count()) * static_cast<uint32_t>(std::max(per_sm, 1)));
+    VB_LAUNCH(kernel, static_cast<uint32_t>(grid), RS_ROWS, smem, sc, g.items, g.queue, g.tile_pairs);
+    return 0;
+}
+
+// Scans the lists as tiles into the score buffer.
+static int
+launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& plan) {
+    SearchWorkspace& ws = ix->ws;
+    TileGroup g{};
+    uint64_t max_items = 0;
+    VB_TRY(group_by_list(ix, sc, nq, plan.qt, TILE_SEGMENT, &g, &max_items));
     TileScan t{};
     t.s = sc.s;
     t.t = sc.t;
@@ -3527,6 +3562,9 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     VB_TRY(ws.query_rows.reserve(nq));
     VB_TRY(ws.pair_scores.reserve(slice * stride));
     const uint32_t qstride8 = plan != nullptr ? plan->pieces * 128 : ix->dpad;   // bytes of an int8 term
+    const bool shared = plan == nullptr && sq8 && slice == nq && nq * nprobe >= SHARED_MIN_QUERIES * nlist &&
+                        static_cast<double>(nq) * nprobe * ix->n_stored / nlist * ix->code_size >= SHARED_MIN_BYTES &&
+                        nq * nprobe < (uint64_t{1} << 31) && shared_scan_smem(ix) <= 110 * 1024 && ix->dpad % 16 == 0;
     if (sq8) {
         VB_TRY(ws.qw8.reserve(nq * 3 * qstride8));
         VB_TRY(ws.qscale.reserve(nq));
@@ -3560,10 +3598,10 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         pp.qa = ws.qa.ptr;
     }
     // (reserved at their full size, so that what is cleared is what a later search may use)
-    if ((plan != nullptr && ws.tile_count.cap < nlist) || (rerank && ws.rerank_done.cap < nq)) {
+    if (((plan != nullptr || shared) && ws.tile_count.cap < nlist) || (rerank && ws.rerank_done.cap < nq)) {
         ws.counts_clear = false;
     }
-    VB_TRY(ws.tile_count.reserve(plan != nullptr ? nlist : 0));
+    VB_TRY(ws.tile_count.reserve(plan != nullptr || shared ? nlist : 0));
     VB_TRY(ws.rerank_done.reserve(rerank ? nq : 0));
     if (!ws.counts_clear) {
         if (ws.tile_count.cap > 0) {
@@ -3575,7 +3613,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         VB_CUDA(cudaMemsetAsync(ws.scalars.ptr + 4, 0, sizeof(uint64_t), st));   // (a scan that gave up left its flag)
     }
     ws.counts_clear = false;   // until this search has come to its end
-    if (plan != nullptr) {
+    if (plan != nullptr || shared) {
         VB_TRY(ws.tile_rank.reserve(nq * nprobe));
         pp.count = ws.tile_count.ptr;
         pp.rank = ws.tile_rank.ptr;
@@ -3717,6 +3755,8 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         }
         if (plan != nullptr) {
             VB_TRY(launch_tiles(ix, g.scan, nq, *plan));
+        } else if (shared) {
+            VB_TRY(launch_shared_scan(ix, g.scan, nq));
         } else {
             const uint64_t blocks = n * nprobe * g.scan.per_pair;
             VB_CHECK_ARG(blocks <= 0x7fffffffull, "query batch too large");

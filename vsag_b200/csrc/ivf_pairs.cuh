@@ -747,7 +747,7 @@ pair_scan_kernel(const PairScan p) {
                        const uint32_t pos = lbeg + static_cast<uint32_t>(row);
                        float v;
                        if constexpr (FMT == ROW_SQ8) {
-                           const float f = sq8_term_sum(acc.a1, acc.a2, acc.a3, p.s.dim <= SQ8_NARROW_DIMS);
+                           const float f = sq8_term_sum(acc.a1[0], acc.a2[0], acc.a3[0], p.s.dim <= SQ8_NARROW_DIMS);
                            v = fmaf(cq, f, p.s.coef_b * __ldg(p.s.code_norm + pos)) + qa;
                        } else if constexpr (FMT == ROW_RABITQ) {
                            const float* tail = reinterpret_cast<const float*>(rows + row * p.s.code_stride + p.row_bytes);

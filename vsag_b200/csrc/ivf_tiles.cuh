@@ -100,6 +100,7 @@ struct TileGroup {
     const uint32_t* rank;     // [pairs]
     const int32_t* probes;    // [pairs]
     uint32_t pairs, nlist, qt;
+    uint32_t segment;         // rows of an item at most (a multiple of 8)
     const uint32_t* order;    // [nlist] lists, longest first: items that finish last are short
     const uint32_t* list_off;
     uint32_t* pair_off;       // [nlist]
@@ -132,7 +133,7 @@ tile_places_kernel(const TileGroup g) {
         for (uint32_t j = 0; j < PER; ++j) {
             cnt[j] = list[j] != 0xFFFFFFFFu ? g.count[list[j]] : 0u;
             its[j] = cnt[j] > 0 ? (cnt[j] + g.qt - 1) / g.qt *
-                                      ((__ldg(g.list_off + list[j] + 1) - __ldg(g.list_off + list[j]) + TILE_SEGMENT - 1) / TILE_SEGMENT)
+                                      ((__ldg(g.list_off + list[j] + 1) - __ldg(g.list_off + list[j]) + g.segment - 1) / g.segment)
                                 : 0u;
             sum += cnt[j];
             tiles += its[j];
@@ -182,11 +183,75 @@ tile_scatter_kernel(const TileGroup g) {
         const uint32_t lbeg = __ldg(g.list_off + e);
         const uint32_t len = n > 0 ? __ldg(g.list_off + e + 1) - lbeg : 0u;
         const uint32_t goff = g.group_off != nullptr ? __ldg(g.group_off + e) : 0u;
-        for (uint32_t row0 = 0; row0 < len; row0 += TILE_SEGMENT) {
+        for (uint32_t row0 = 0; row0 < len; row0 += g.segment) {
             for (uint32_t i = 0; i * g.qt < n; ++i) {
-                *dst++ = TileItem{lbeg + row0, min(len - row0, TILE_SEGMENT), p0 + i * g.qt, min(g.qt, n - i * g.qt), row0, goff + row0 / 8, 0u, 0u};
+                *dst++ = TileItem{lbeg + row0, min(len - row0, g.segment), p0 + i * g.qt, min(g.qt, n - i * g.qt), row0, goff + row0 / 8, 0u, 0u};
             }
         }
+    }
+}
+
+// ---- SQ8 lists that a few queries probe ----------------------------------------------------
+// pair_scan_kernel reads a list's rows once for every query, and what bounds it is that traffic from L2 (100 queries of 640
+// dimensions, three per list: 1 GB, 144 us).  With two to four queries per list, too few for tensor-core tiles, the pairs are grouped by
+// list all the same and a CTA streams up to SHARED_SEGMENT rows of a list past up to SHARED_QUERIES of them: 99 us, 111 with the grouping.
+constexpr int SHARED_QUERIES = 4;
+constexpr uint32_t SHARED_SEGMENT = 256;
+
+template <bool L2>
+__global__ void __launch_bounds__(RS_ROWS)
+shared_scan_kernel(const PairScan p, const TileItem* __restrict__ items, uint32_t* __restrict__ queue, const TilePair* __restrict__ pairs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_item;
+    unsigned char* const terms = smem + RS_STAGES * RS_STAGE;
+    const uint32_t n_items = queue[0], per_query = 3 * p.qstride;
+    for (;;) {
+        __syncthreads();   // (the item before is done with the queries)
+        if (threadIdx.x == 0) {
+            s_item = atomicAdd(queue + 1, 1u);
+        }
+        __syncthreads();
+        if (s_item >= n_items) {
+            return;
+        }
+        const uint4 head = __ldg(reinterpret_cast<const uint4*>(items + s_item));
+        const uint32_t lbeg = head.x, len = head.y, pair0 = head.z, live = head.w, row0 = __ldg(&items[s_item].row0);
+        float qa[SHARED_QUERIES], cq[SHARED_QUERIES];
+        uint32_t* out[SHARED_QUERIES];
+#pragma unroll
+        for (int j = 0; j < SHARED_QUERIES; ++j) {
+            if (static_cast<uint32_t>(j) < live) {
+                const TilePair pair = pairs[pair0 + j];
+                qa[j] = __ldg(p.s.qa + pair.q);
+                cq[j] = p.s.coef_c * __ldg(p.qscale + pair.q);
+                out[j] = reinterpret_cast<uint32_t*>(p.t.scores) + pair.out + row0;
+                const uint4* src = reinterpret_cast<const uint4*>(p.qw8 + static_cast<uint64_t>(pair.q) * per_query);
+                for (uint32_t i = threadIdx.x; i < per_query / 16; i += RS_ROWS) {
+                    reinterpret_cast<uint4*>(terms + j * per_query)[i] = __ldg(src + i);
+                }
+            } else {
+                qa[j] = cq[j] = 0.f;
+                out[j] = nullptr;
+            }
+        }
+        RowAcc<ROW_SQ8, L2, SHARED_QUERIES> acc;
+        acc.live = live;
+        row_stream<16>(p.s.codes + static_cast<uint64_t>(lbeg) * p.s.code_stride, p.s.code_stride, p.row_bytes, p.s.dim, len, 0, 1, smem,
+                       reinterpret_cast<const float*>(terms), p.qstride, acc, [&](uint64_t row, bool valid) {
+                           if (!valid) {
+                               return;
+                           }
+                           const uint32_t pos = lbeg + static_cast<uint32_t>(row);
+                           const float norm = p.s.coef_b * __ldg(p.s.code_norm + pos);
+                           const bool filtered = p.s.filter_pos_inner != nullptr && scan_row_filtered(p.s, pos);
+#pragma unroll
+                           for (int j = 0; j < SHARED_QUERIES; ++j) {
+                               if (static_cast<uint32_t>(j) < live) {
+                                   const float f = sq8_term_sum(acc.a1[j], acc.a2[j], acc.a3[j], p.s.dim <= SQ8_NARROW_DIMS);
+                                   out[j][row] = filtered ? SCORE_FILTERED : __float_as_uint(fmaf(cq[j], f, norm) + qa[j]);
+                               }
+                           }
+                       });
     }
 }
 

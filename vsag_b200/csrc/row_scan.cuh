@@ -107,35 +107,45 @@ sq8_term_sum(int32_t a1, int32_t a2, int32_t a3, bool narrow) {
     return fmaf(low, 1.0f / 64516.0f, static_cast<float>(a1));
 }
 
-// Three integer sums over the int8 weight terms of one query, [3][qstride] bytes behind `q`; terms past the
-// last dimension are zero.
+// Three integer sums over the int8 weight terms of each of QN queries, [QN][3][qstride] bytes behind `q`; terms past the
+// last dimension are zero.  `live`: queries there are (the others cost a test).
 template <bool L2, int QN>
 struct RowAcc<ROW_SQ8, L2, QN> {
     static constexpr uint32_t UNIT_DIMS = 16;
-    int32_t a1, a2, a3;
+    int32_t a1[QN], a2[QN], a3[QN];
+    uint32_t live = QN;
     __device__ __forceinline__ void
     clear() {
-        a1 = a2 = a3 = 0;
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            a1[i] = a2[i] = a3[i] = 0;
+        }
     }
     __device__ __forceinline__ void
     unit(const uint4& w, const float* q, uint32_t qstride, uint32_t d0) {
-        const int8_t* t = reinterpret_cast<const int8_t*>(q) + d0;
-        const int4 t1 = *reinterpret_cast<const int4*>(t), t2 = *reinterpret_cast<const int4*>(t + qstride),
-                   t3 = *reinterpret_cast<const int4*>(t + 2 * qstride);
         const int c0 = static_cast<int>(w.x ^ 0x80808080u), c1 = static_cast<int>(w.y ^ 0x80808080u),
                   c2 = static_cast<int>(w.z ^ 0x80808080u), c3 = static_cast<int>(w.w ^ 0x80808080u);
-        a1 = __dp4a(c0, t1.x, a1);
-        a2 = __dp4a(c0, t2.x, a2);
-        a3 = __dp4a(c0, t3.x, a3);
-        a1 = __dp4a(c1, t1.y, a1);
-        a2 = __dp4a(c1, t2.y, a2);
-        a3 = __dp4a(c1, t3.y, a3);
-        a1 = __dp4a(c2, t1.z, a1);
-        a2 = __dp4a(c2, t2.z, a2);
-        a3 = __dp4a(c2, t3.z, a3);
-        a1 = __dp4a(c3, t1.w, a1);
-        a2 = __dp4a(c3, t2.w, a2);
-        a3 = __dp4a(c3, t3.w, a3);
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            if (QN > 1 && static_cast<uint32_t>(i) >= live) {
+                break;
+            }
+            const int8_t* t = reinterpret_cast<const int8_t*>(q) + i * 3 * qstride + d0;
+            const int4 t1 = *reinterpret_cast<const int4*>(t), t2 = *reinterpret_cast<const int4*>(t + qstride),
+                       t3 = *reinterpret_cast<const int4*>(t + 2 * qstride);
+            a1[i] = __dp4a(c0, t1.x, a1[i]);
+            a2[i] = __dp4a(c0, t2.x, a2[i]);
+            a3[i] = __dp4a(c0, t3.x, a3[i]);
+            a1[i] = __dp4a(c1, t1.y, a1[i]);
+            a2[i] = __dp4a(c1, t2.y, a2[i]);
+            a3[i] = __dp4a(c1, t3.y, a3[i]);
+            a1[i] = __dp4a(c2, t1.z, a1[i]);
+            a2[i] = __dp4a(c2, t2.z, a2[i]);
+            a3[i] = __dp4a(c2, t3.z, a3[i]);
+            a1[i] = __dp4a(c3, t1.w, a1[i]);
+            a2[i] = __dp4a(c3, t2.w, a2[i]);
+            a3[i] = __dp4a(c3, t3.w, a3[i]);
+        }
     }
     __device__ __forceinline__ void
     tail(const uint4& w, const float* q, uint32_t qstride, uint32_t d0, uint32_t) {
