@@ -3243,6 +3243,7 @@ constexpr size_t PINNED_IO_BYTES = 256 * 1024;
 // From two queries per probed list on SQ8 rows are streamed for several of them, where the rows are bytes enough to pay for the grouping
 // (as pairs / shared, us: 384 MB of rows 252 / 218, 600 MB 267 / 245, 180 MB 447 / 354, 200 MB 254 / 250; 128 MB 202 / 201, 19 MB 89 / 95).
 constexpr double SHARED_MIN_QUERIES = 2.0, SHARED_MIN_BYTES = 1.5e8;
+constexpr int FINAL_FEW = 4;               // queries an SM up to which the finalising kernel keeps its registers (see there)
 constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which tiles pay (3.1: 141 us as pairs, 162 as tiles)
 
 // Shared memory of pair_scan_kernel and of scan_finalize_kernel; qstride: floats of a query as the codec's chain reads it (the
@@ -3707,7 +3708,10 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     const size_t scan_smem = score_scan_smem(ix, f.scan.qstride), final_smem = score_final_smem(ix, nprobe, plan != nullptr ? f.scan.qstride : 0);
     void (*scan_kernel)(const PairScan) = nullptr;
     void (*final_kernel)(const ScanFinalize) = nullptr;
-#define VB_FINAL(FMT, APPROX) (l2 ? scan_finalize_kernel<FMT, true, APPROX> : scan_finalize_kernel<FMT, false, APPROX>)
+    const bool many = std::min(slice, nq) > FINAL_FEW * static_cast<uint64_t>(sm_count());
+#define VB_FINAL(FMT, APPROX)                                                                                            \
+    (l2 ? (many ? scan_finalize_kernel<FMT, true, APPROX, 7> : scan_finalize_kernel<FMT, true, APPROX, FINAL_FEW>)         \
+        : (many ? scan_finalize_kernel<FMT, false, APPROX, 7> : scan_finalize_kernel<FMT, false, APPROX, FINAL_FEW>))
 #define VB_PAIRS(FMT)                                                                       \
     {                                                                                       \
         scan_kernel = l2 ? pair_scan_kernel<FMT, true> : pair_scan_kernel<FMT, false>;      \
@@ -3723,7 +3727,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         case VB200_QUANT_FP16: VB_PAIRS(ROW_FP16) break;
         default:
             scan_kernel = pair_scan_kernel<ROW_RABITQ, true>;
-            final_kernel = plan != nullptr ? scan_finalize_kernel<ROW_RABITQ, true, true> : scan_finalize_kernel<ROW_RABITQ, true, false>;
+            final_kernel = plan != nullptr ? scan_finalize_kernel<ROW_RABITQ, true, true, 5> : scan_finalize_kernel<ROW_RABITQ, true, false, 5>;
             break;
     }
 #undef VB_PAIRS

@@ -885,9 +885,10 @@ record_exact_distance(const uint8_t* rec, uint32_t dim, uint32_t row_bytes, cons
 // bounding the difference between score and exact distance, so when the kscan-th exact distance is below that the
 // result is the exact one.  Otherwise (scores crowded within the rounding of the arithmetic) every row of the query
 // is scored exactly here.
-// (seven CTAs an SM take 1000 queries together, 57 -> 41 us; the one-bit chain wants the registers, 244 -> 256)
-template <int FMT, bool L2, bool APPROX>
-__global__ void __launch_bounds__(PAIR_THREADS, FMT == ROW_RABITQ ? 5 : 7)
+// CTAS: CTAs an SM that the registers leave room for.  (Seven take 1000 queries together, 57 -> 41 us; the one-bit chain wants the
+// registers, 244 -> 256, and so do few queries, for which nothing else hides the loads: 32 take 46 us, with seven 54.)
+template <int FMT, bool L2, bool APPROX, int CTAS>
+__global__ void __launch_bounds__(PAIR_THREADS, CTAS)
 scan_finalize_kernel(const ScanFinalize p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ SelectScratch sel;
