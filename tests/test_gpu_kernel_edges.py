@@ -86,7 +86,7 @@ def test_routing_by_chains(engine, oracle, metric, dim, nq, nlist):
     assert np.array_equal(np.asarray(got), np.asarray(want))
 
 
-@pytest.mark.parametrize("nq,nlist", [(20, 900), (300, 1500)])      # by distances, and by scores that are re-scored
+@pytest.mark.parametrize("nq,nlist", [(20, 900), (300, 1000), (300, 1500), (1300, 1500)])   # by distances, and by scores; a warp, a CTA a query
 @pytest.mark.parametrize("metric", [0, 1])
 @pytest.mark.parametrize("dim", [18, 32])                           # rows of 8- and of 16-byte alignment
 def test_routing_with_coinciding_centroids(engine, oracle, nq, nlist, metric, dim):

@@ -2447,7 +2447,14 @@ launch_prepare(const PairsPrepare& p, uint64_t nq) {
     const uint32_t wanted = p.scores != nullptr ? p.ncand : p.nprobe;
     const size_t query = p.scores != nullptr ? p.dim * sizeof(float) : 0;
     const size_t warp_smem = PREPARE_WARPS * prepare_warp_bytes(p.scores != nullptr, p.dim);
-    if (wanted <= WARP_SELECT_MAX && p.nprobe <= WARP_SELECT_MAX && p.repeats == nullptr && warp_smem <= 64 * 1024) {
+    // A warp takes longer over a query than a CTA, the more so the more lists and the more wanted of them, but there are many warps (a CTA
+    // each / a warp each, us a search: 1 query of 1024 lists, 127 wanted 62 / 70, 32 wanted 58 / 59, of 4000 lists 62 / 82; 1000
+    // queries of 1024 lists 198 / 191, of 4000 lists 199 / 205; 2500 of those 287 / 275).  Long rows to re-score move the line (1000
+    // queries of 4096 lists, 72 candidates of 960 dimensions: the kernel takes 122 / 97).
+    const bool selects = p.scores != nullptr || p.dist != nullptr;
+    const bool warps = !selects || (wanted <= 48 && p.nlist <= 1024) || nq * 1024 >= 3ull * sm_count() * (1024 + p.nlist) ||
+                       (p.scores != nullptr && p.dim >= 256 && nq >= 4ull * sm_count());
+    if (warps && wanted <= WARP_SELECT_MAX && p.nprobe <= WARP_SELECT_MAX && p.repeats == nullptr && warp_smem <= 64 * 1024) {
         VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_warps_kernel), warp_smem));
         VB_LAUNCH(pairs_prepare_warps_kernel, static_cast<uint32_t>((nq + PREPARE_WARPS - 1) / PREPARE_WARPS), PREPARE_WARPS * 32, warp_smem, p, nq);
         return 0;
