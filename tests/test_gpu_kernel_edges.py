@@ -138,17 +138,17 @@ def test_training_with_the_bias_among_the_products(engine, oracle, dim, offset, 
 
 # ---- SQ8 batches that rule lists out -----------------------------------------------------------------------------
 @pytest.mark.parametrize("dim,k", [(16, 10), (96, 16), (96, 17), (112, 48), (128, 49), (130, 112), (130, 113), (256, 10), (300, 10)])
-@pytest.mark.parametrize("metric", [0, 1])
-def test_pruned_batches_equal_unpruned_ones(engine, dim, k, metric):
-    n, nlist, nprobe, nq = 40_003, 20, 12, 200      # 2000 rows a list, 4.8e6 rows scanned
+@pytest.mark.parametrize("metric,nq", [(0, 200), (1, 200), (0, 3603), (1, 3603)])      # results by a CTA, and by a warp a query
+def test_pruned_batches_equal_unpruned_ones(engine, dim, k, metric, nq):
+    n, nlist, nprobe, step = 40_003, 20, 12, nq // 25      # 2000 rows a list, 4.8e6 rows scanned
     x, q = mixture(51, n, dim, 60, 0.3), mixture(52, nq, dim, 60, 0.3)
     ix = engine.IvfHandle(dim, metric, nlist, engine.QUANT_SQ8)
     ix.train(x[::8].copy(), iters=2)
     ix.add(x, np.arange(n, dtype=np.int64))
-    want = [ix.search(q[i:i + 1].copy(), k, nprobe) for i in range(0, nq, 8)]
+    want = [ix.search(q[i:i + 1].copy(), k, nprobe) for i in range(0, nq, step)]
     got = ix.search(q, k, nprobe)
-    assert np.array_equal(got[1][::8], np.concatenate([w[1] for w in want]))
-    assert np.array_equal(got[0][::8], np.concatenate([w[0] for w in want]))
+    assert np.array_equal(got[1][::step], np.concatenate([w[1] for w in want]))
+    assert np.array_equal(got[0][::step], np.concatenate([w[0] for w in want]))
 
 
 # ---- tiles ------------------------------------------------------------------------------------------------------

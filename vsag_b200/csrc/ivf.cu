@@ -2069,6 +2069,8 @@ route_pick_warp_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t 
 // Dynamic shared memory: [2][dim] lower and diff, per warp [FINISH_KEYS] keys and the query.
 constexpr uint32_t FINISH_KEYS = WARP_SELECT_CAP;
 constexpr uint32_t FINISH_MAX_SCAN = 128, FINISH_MAX_DIM = 4096;
+// Few queries are better off with a CTA each and three launches (642 queries 22 us / 40 here, 585 with 42 keys 38 / 73, 10,000 103 / 61).
+constexpr uint64_t FINISH_MIN_QUERIES = 3584;
 constexpr uint32_t FINISH_WARPS = 4;
 
 template <bool L2, int R>
@@ -3113,7 +3115,7 @@ ivf_scan_device(vb200_ivf* ix, const float* q_dev, uint64_t nq, uint32_t kfinal,
     VB_CUDA(cudaEventRecord(ix->ev_scan_end, st));
     ix->scan_timed = true;
     // (a warp sorts what few slots hold; unpruned a query's slots are all written, nprobe * kscan keys, and a CTA merges them)
-    if (sq8 && kscan <= FINISH_MAX_SCAN && ws.pruning && !ix->use_residual && ix->dim <= FINISH_MAX_DIM) {
+    if (sq8 && nq >= FINISH_MIN_QUERIES && kscan <= FINISH_MAX_SCAN && ws.pruning && !ix->use_residual && ix->dim <= FINISH_MAX_DIM) {
         VB_TRY(launch_sq8_finish(ix, q_dev, nq, nprobe, kscan, kfinal, ws.part.ptr, ws.slot_written.ptr, ws.keys.ptr));
         g_scan_profile.mark(st);   // merge
         return 0;
