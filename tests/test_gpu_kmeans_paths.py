@@ -31,3 +31,22 @@ def test_training_where_nominations_decide_nothing(engine, oracle, n):
     want_c, want_l, _, _ = oracle.kmeans_run(x, init, iters)
     got_c, got_l, _ = engine.kmeans_train(x, init, iters)
     assert np.array_equal(got_l, want_l) and np.array_equal(got_c, want_c)
+
+
+@pytest.mark.parametrize("dim", [5, 32, 200])
+@pytest.mark.parametrize("top", [1e6, 1e8, 1e9, 1e11])
+def test_rows_beside_one_that_is_far_larger(engine, oracle, dim, top):
+    """The scale of the fp16 operands follows the largest element: the others become subnormal, their squares vanish, and the
+    margin has to say so.  Labels are the oracle's, and with centroids as near to one another as the rows (not to the large
+    row) those of 64-bit distances too."""
+    n, k = 3000, 70
+    x = mixture(45, n, dim, 50, 0.2)
+    c = np.ascontiguousarray(x[100:100 + k])
+    x[5] = np.float32(top)
+    got = engine.kmeans_assign(x, c)
+    assert np.array_equal(got, oracle.kmeans_assign(x, c)[0])
+    rest = np.r_[0:5, 6:n]
+    d = ((x[rest, None, :].astype(np.float64) - c[None].astype(np.float64)) ** 2).sum(-1)
+    two = np.sort(d, 1)[:, :2]
+    clear = two[:, 1] - two[:, 0] > 1e-4 * (two[:, 0] + dim)      # (far above the rounding of a chain of fp32 products)
+    assert clear.mean() > 0.5 and np.array_equal(got[rest][clear], d.argmin(1)[clear])

@@ -263,19 +263,19 @@ kmeans_norms_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, const
 
 // margin[i] = by_shifted * max|c - shift| * |x_i - shift| + by_plain * max|c| * |x_i| + by_square * max|c - shift|^2, and with `prev`
 // bound[i] = the row's score against its previous centroid, |c'|^2 - 2 <c', x'> over shifted vectors (+inf when it has none), both
-// in units of the products (times `unit`).  Eight
+// in units of the products (times `unit`); to the margin, in those units, floor_each (max|c - shift| + |x_i - shift|) + floor.  Eight
 // lanes per row.  Centroids that do not fit the fp16 scale (limit) leave no column out: the margin becomes infinite.
 __global__ void __launch_bounds__(256)
 kmeans_row_prep_kernel(const float* __restrict__ x, uint64_t n, uint32_t dim, const float* __restrict__ shift,
                        const float* __restrict__ c_shifted, const float* __restrict__ cs_sq, uint32_t k, const int32_t* __restrict__ prev,
                        const float* __restrict__ x_norm, const float* __restrict__ xs_norm, const float* __restrict__ extremes,
-                       float by_shifted, float by_plain, float by_square, float limit, float unit, float* __restrict__ margin,
-                       float* __restrict__ bound) {
+                       float by_shifted, float by_plain, float by_square, float floor_each, float floor, float limit, float unit,
+                       float* __restrict__ margin, float* __restrict__ bound) {
     const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x) >> 3;
     const uint32_t sub = threadIdx.x & 7u;
     if (i < n && sub == 0) {
         const float m = by_shifted * extremes[1] * xs_norm[i] + by_plain * extremes[2] * x_norm[i] + by_square * extremes[1] * extremes[1];
-        margin[i] = extremes[0] <= limit ? m * unit : INFINITY;
+        margin[i] = extremes[0] <= limit ? m * unit + (floor_each * (extremes[1] + xs_norm[i]) + floor) : INFINITY;
     }
     if (prev == nullptr) {
         return;
@@ -398,7 +398,9 @@ constexpr uint32_t KMEANS_FEW_ROWS = 4096;               // undecided rows that 
 // The scores are |c'|^2 - 2 <c', x'> over vectors minus a common shift (the centroids' mean: it changes no comparison
 // of a row and takes the data's offset out of the errors), with x' and c' rounded to one fp16 term each, scaled so that
 // the largest element is near 2^top: an error of at most 2 (2 * 2^-11 + 2^-22) |x'| |c'| per score, and of the sums, which hold |c'|^2
-// among their products, (dim + 16) 2^-23 |c'|^2 (elements below 2^-14 scaled, 2^-25 of the largest, round absolutely: far less).  A column further
+// among their products, (dim + 16) 2^-23 |c'|^2.  Scaled elements below 2^-14 round absolutely, by 2^-25, which is 2^-25 sqrt(dim) (|x'| + |c'|) of a
+// scaled product, and the last of the bias's three terms by 2^-25 * 2^-7: next to nothing for rows of one size, and everything for the rows of
+// ordinary size beside one that is 1e8 times as large, whose scaled squares vanish.  A column further
 // than twice that (plus the rounding of the reference's own chain) behind a row's best is not its winner; the columns
 // within are scored exactly.  A third of the MMAs that split bf16 terms take; those (2^-16 of the plain norms) remain for data
 // whose shifted rows still crowd within the fp16 margin -- when more than a sixteenth of the rows came out undecided.
@@ -472,12 +474,14 @@ kmeans_assign_tc(KMeansWorkspace& ws, const float* x_dev, uint64_t n, uint32_t d
         }
         // margins: twice the error of a nominating score, and of the exact chains that decide (2 (dim + 2) 2^-24 each)
         const float chain = 4.0f * static_cast<float>(dim + 8) * 6.0e-8f;
+        const float floor_each = half ? std::ldexp(std::sqrt(static_cast<float>(dim)) * 1.001f, -24) * ws.scale : 0.f;
+        const float floor = half ? std::ldexp(1.0f, -31) + std::ldexp(static_cast<float>(dim), -49) : 0.f;
         VB_TRY(ws.row_margin.reserve(rows));
         VB_TRY(ws.row_bound.reserve(rows));
         VB_LAUNCH(kmeans_row_prep_kernel, static_cast<uint32_t>((rows * 8 + 255) / 256), 256, 0, x_dev + r0 * dim, rows, dim, ws.shift.ptr,
                   ws.c_shifted.ptr, ws.cs_sq.ptr, k, prev_labels_dev != nullptr ? prev_labels_dev + r0 : nullptr, ws.x_norm.ptr,
                   half ? ws.xs_norm.ptr : ws.x_norm.ptr, ws.extremes.ptr, half ? 4.0e-3f : 1e-3f, chain,
-                  half ? static_cast<float>(dim + 16) * 2.4e-7f : 0.f, half ? std::ldexp(1.4f, top_exponent) / ws.scale : INFINITY,
+                  half ? static_cast<float>(dim + 16) * 2.4e-7f : 0.f, floor_each, floor, half ? std::ldexp(1.4f, top_exponent) / ws.scale : INFINITY,
                   half ? 0.5f * ws.scale * ws.scale : 1.0f, ws.row_margin.ptr, ws.row_bound.ptr);
         const float* row_bound = prev_labels_dev != nullptr ? ws.row_bound.ptr : nullptr;
         uint32_t n_split = 1, n_flagged = 0;
