@@ -15,12 +15,17 @@ def exactly(got, want):
 
 
 # ---- exact batches that keep what passes a threshold from a sample of the rows --------------------------------
-# 4 (k + 16) minima of 32 rows in every eighth tile of 128: from 17,281 rows with k 1, 26,497 with k 10, 60,033 with k 42
+# 4 (k + 16) groups of 32 in an eighth of the rows: from 17,408 rows with k 1, 26,624 with k 10, 59,392 with k 42
 @pytest.mark.parametrize("quant,metric,n,dim,nq,k", [
-    ("fp32", 0, 17_280, 33, 9, 1),        # the most rows without a sample, rows of 4-byte alignment
-    ("fp32", 0, 17_281, 33, 9, 1),        # the fewest with one; the last tile of the rows holds one
+    ("fp32", 0, 17_280, 33, 9, 1),        # rows of 4-byte alignment
+    ("fp32", 0, 17_281, 33, 9, 1),        # the last tile of the rows holds one
+    ("fp32", 0, 17_407, 33, 9, 1),        # the most rows without a sample
+    ("fp32", 0, 17_408, 33, 9, 1),        # the fewest with one
+    ("fp32", 0, 18_433, 33, 9, 1),        # the last tile of the rows holds one
     ("fp32", 1, 26_497, 96, 129, 10),     # two row tiles of queries, six of eight k-steps
+    ("fp32", 1, 26_625, 96, 129, 10),
     ("bf16", 0, 26_600, 50, 128, 10),
+    ("bf16", 0, 26_700, 50, 128, 10),
     ("bf16", 1, 60_100, 200, 300, 42),
     ("fp32", 0, 70_000, 16, 1000, 10),    # a sixteenth of the rows as a sample
 ])
@@ -46,6 +51,33 @@ def test_exact_batches_by_threshold(engine, oracle, quant, metric, n, dim, nq, k
     else:
         want = oracle.bf_search_bf16(oracle.float_to_bf16(base[left]), q[some], k, metric=metric)
     exactly((few[0][some], few[1][some]), (np.where(want[0] >= 0, left[want[0]], -1), want[1]))
+
+
+# the fewest rows with an eighth, a sixteenth and a thirty-second as the sample: 4 (k + 16) groups of 32 in it
+@pytest.mark.parametrize("n,k", [(17_408, 1), (26_624, 10), (53_248, 10), (106_496, 10), (119_000, 42)])
+@pytest.mark.parametrize("quant", ["QUANT_FP32", "QUANT_BF16"])
+@pytest.mark.parametrize("metric", [0, 1])
+def test_exact_batches_do_not_depend_on_the_order_of_the_rows(engine, quant, metric, n, k):
+    """Rows of a cluster stored together, or clusters in turn: what the sample lets through fits as it does for mixed rows, so no
+    query is left to the exact pass, which would be two launches more."""
+    dim, nq, clusters = 20, 150, 96
+    rng = np.random.default_rng(n)
+    centres = rng.uniform(-1, 1, (clusters, dim))
+    member = rng.integers(0, clusters, n)
+    q = (centres[rng.integers(0, clusters, nq)] + 0.2 * rng.standard_normal((nq, dim))).astype(np.float32)
+    launches = []
+    for order in ("mixed", "together", "in turn"):
+        which = {"mixed": member, "together": np.sort(member), "in turn": np.arange(n) % clusters}[order]
+        base = (centres[which] + 0.2 * rng.standard_normal((n, dim))).astype(np.float32)
+        ix = engine.BfHandle(dim, metric, getattr(engine, quant))
+        ix.add(base, np.arange(n, dtype=np.int64))
+        ix.search(q, k)
+        before = engine.kernel_launches()
+        got = ix.search(q, k)
+        launches.append(engine.kernel_launches() - before)
+        one = [ix.search(q[i:i + 1].copy(), k) for i in range(0, nq, 10)]
+        assert np.array_equal(got[1][::10], np.concatenate([o[1] for o in one]))
+    assert launches == launches[:1] * 3
 
 
 @pytest.mark.parametrize("kind", ["equal", "far", "nan"])

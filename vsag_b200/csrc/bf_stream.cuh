@@ -210,11 +210,12 @@ bf_rows_kernel(const float* __restrict__ scores, uint64_t ld, uint32_t n, const 
     }
 }
 
-// thr[q] = the next float above the kcand-th smallest of the query's n minima (+inf with fewer numbers among them).  A CTA per query.
+// thr[q] = the next float above the kcand-th smallest of the query's n minima (+inf with fewer numbers among them), and
+// spilled[q] = 0.  A CTA per query.
 constexpr int BF_THRESHOLD_THREADS = 128;
 
 __global__ void __launch_bounds__(BF_THRESHOLD_THREADS)
-bf_threshold_kernel(const float* __restrict__ minima, uint32_t n, uint32_t kcand, float* __restrict__ thr) {
+bf_threshold_kernel(const float* __restrict__ minima, uint32_t n, uint32_t kcand, float* __restrict__ thr, uint32_t* __restrict__ spilled) {
     __shared__ SelectScratch sel;
     const float* mine = minima + static_cast<uint64_t>(blockIdx.x) * n;
     uint32_t upto;
@@ -222,13 +223,16 @@ bf_threshold_kernel(const float* __restrict__ minima, uint32_t n, uint32_t kcand
                                                              kcand + kcand / 8 + 8, sel, &upto);
     if (threadIdx.x == 0) {
         thr[blockIdx.x] = bound >= ORDERED_INF ? INFINITY : ordered_to_float(bound + 1);
+        spilled[blockIdx.x] = 0;
     }
 }
 
 // The rows that score below a query's threshold, as tc_collect left them, to the query's results.
 struct BfCollected {
     const uint64_t* keys;     // [queries][lists][cap] nominating score and row
-    const uint32_t* count;    // [queries][lists] entries offered
+    const uint32_t* count;    // [queries][lists] entries offered; those past `cap` are in the spill
+    const uint64_t* spill;    // [queries][room]
+    const uint32_t* spilled;  // [queries] entries offered to it
     const float* thr;         // [queries]
     uint32_t lists, cap;
     uint32_t room;            // entries of one query that shared memory holds
@@ -246,7 +250,7 @@ struct BfCollected {
 // keeps k.  A query is sure of its results when the k-th of them is nearer than the last nominated score -- or the threshold, if
 // no row below it was left out -- allows any other row to be.  When it is not, all collected rows are re-scored, after which
 // only those above the threshold are left out; what is not sure then, or did not fit, is listed for the exact pass.
-// Dynamic shared memory: [room] keys, [lists + 1] places, the query.
+// Dynamic shared memory: [room] keys, [lists + 2] places, the query.
 template <typename E, int T>
 __global__ void __launch_bounds__(T)
 bf_collected_kernel(const BfCollected p) {
@@ -255,10 +259,9 @@ bf_collected_kernel(const BfCollected p) {
     __shared__ __align__(16) uint64_t keys[SELECT_CAP];
     __shared__ __align__(16) uint64_t best[1024];
     __shared__ float s_qq, s_top;
-    __shared__ uint32_t s_over;
     uint64_t* all = reinterpret_cast<uint64_t*>(smem);
     uint32_t* place = reinterpret_cast<uint32_t*>(all + p.room);
-    float* qf = reinterpret_cast<float*>(place + p.lists + 1);
+    float* qf = reinterpret_cast<float*>(place + p.lists + 2);
     const uint64_t q = blockIdx.x;
     const uint32_t dim = p.dim;
     const bool l2 = p.metric == VB200_METRIC_L2;
@@ -266,22 +269,15 @@ bf_collected_kernel(const BfCollected p) {
     for (uint32_t d = threadIdx.x; d < dim; d += T) {
         qf[d] = widen(static_cast<const E*>(p.queries)[q * dim + d]);
     }
-    if (threadIdx.x == 0) {
-        s_over = 0;
-    }
     __syncthreads();
-    // where each list's entries begin
+    // where each list's entries begin, the spill's as the last of them
     const uint32_t* count = p.count + q * p.lists;
     uint32_t total = 0;
-    for (uint32_t l0 = 0; l0 < p.lists; l0 += T) {
+    for (uint32_t l0 = 0; l0 <= p.lists; l0 += T) {
         const uint32_t l = l0 + threadIdx.x;
-        uint32_t c = l < p.lists ? __ldg(count + l) : 0u;
-        if (c > p.cap) {
-            s_over = 1;
-            c = p.cap;
-        }
+        const uint32_t c = l < p.lists ? min(__ldg(count + l), p.cap) : (l == p.lists ? __ldg(p.spilled + q) : 0u);
         const uint32_t incl = block_inclusive_sum<T>(c, sel.warp_part);
-        if (l < p.lists) {
+        if (l <= p.lists) {
             place[l] = total + incl - c;
         }
         if (threadIdx.x == T - 1) {
@@ -291,10 +287,10 @@ bf_collected_kernel(const BfCollected p) {
         total = sel.total;
     }
     if (threadIdx.x == 0) {
-        place[p.lists] = total;
+        place[p.lists + 1] = total;
     }
     __syncthreads();
-    if (s_over != 0 || total > p.room) {
+    if (total > p.room) {   // (so a spill that is not whole is not read)
         if (threadIdx.x == 0) {
             p.m.unsure[1 + atomicAdd(p.m.unsure, 1u)] = p.m.q_base + static_cast<uint32_t>(q);
         }
@@ -302,7 +298,7 @@ bf_collected_kernel(const BfCollected p) {
     }
     const uint64_t* mine = p.keys + q * p.lists * p.cap;
     for (uint32_t i = threadIdx.x; i < total; i += T) {
-        uint32_t lo = 0, hi = p.lists;   // the list that holds entry i is the last one that begins at or before it
+        uint32_t lo = 0, hi = p.lists + 1;   // the list that holds entry i is the last one that begins at or before it
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
             if (place[mid] <= i) {
@@ -311,7 +307,7 @@ bf_collected_kernel(const BfCollected p) {
                 hi = mid;
             }
         }
-        all[i] = __ldg(mine + static_cast<uint64_t>(lo) * p.cap + (i - place[lo]));
+        all[i] = __ldg((lo < p.lists ? mine + static_cast<uint64_t>(lo) * p.cap : p.spill + q * p.room) + (i - place[lo]));
     }
     __syncthreads();
     // a few more than the `keep` smallest of `all`, unsorted, in keys; how many.  No other is below *left (ORDERED_INF: no other)

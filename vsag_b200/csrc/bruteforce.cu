@@ -254,8 +254,14 @@ struct vb200_bf {
     // tensor-core path: the base (and per search the queries) as tiled bf16 terms
     DevBuf<uint16_t> base_hi, base_lo, q_hi, q_lo;
     bool tiled_valid = false;
+    // of the tiled rows, one of every sample_stride (0: none taken yet) with its score bias, see bf_take_sample
+    DevBuf<uint16_t> sample_hi, sample_lo;
+    DevBuf<float> sample_bias;
+    uint32_t sample_stride = 0;
     DevBuf<uint64_t> tc_out;
     DevBuf<uint32_t> list_count;   // entries of every list of tc_out
+    DevBuf<uint64_t> spill;        // entries of a query that its lists have no room for, with their number
+    DevBuf<uint32_t> spilled;
     DevBuf<uint64_t> sh_local, sh_all;   // sharded search: this rank's packed [keys | labels] and the gathered ones
     DevBuf<float> row_bound;   // per query: the kcand-th candidate score after the column ranges searched so far
     TcWorkspace tc;
@@ -570,6 +576,7 @@ bf_tile_base(vb200_bf* ix) {
         VB_TRY(tc_pretile_f32(ix->base_f32.ptr, ix->n, ix->dim, ix->base_hi.ptr, ix->base_lo.ptr));
     }
     ix->tiled_valid = true;
+    ix->sample_stride = 0;
     return 0;
 }
 
@@ -807,14 +814,14 @@ bf_margin(const vb200_bf* ix) {
 }
 
 // Batches over many rows: no score is written that a threshold rules out.
-//   sample   the smallest score of every 32 rows in one tile of 128 in `stride`; of those minima the kcand-th smallest is a score
+//   sample   one row in `stride`, and of every 32 of those the smallest score; of these minima the kcand-th smallest is a score
 //            that kcand rows reach, so the rows with the kcand best scores are among those that do not pass it
 //   collect  one pass over all rows appends what does not pass the query's threshold to its lists, about kcand * stride entries
 //   rows     a CTA per query selects, re-scores and writes its results (bf_collected_kernel)
 // 1000 queries over 100k x 128 fp32 rows, k 10: 13, 5, 75 and 47 us, where 121 wrote the scores and 174 selected from them.
 struct BfSample {
     uint32_t stride = 0;       // 0: the rows are too few for a sample
-    uint64_t tiles = 0;        // in the sample
+    uint64_t groups = 0;       // of 32 rows in the sample
     double most = 0.0;         // rows that a query may collect
 };
 constexpr uint32_t BF_COLLECT_KEYS = 12288;          // of a query, at most (96 KiB of shared memory)
@@ -834,9 +841,8 @@ bf_sample(uint64_t n, uint32_t dim, uint32_t kcand) {
     if (dim > BF_COLLECT_DIMS) {
         return s;
     }
-    const uint64_t tiles = (n + TC_BN - 1) / TC_BN;
     for (uint32_t stride = 32; stride >= 8; stride /= 2) {
-        const uint64_t taken = (tiles + stride - 1) / stride, minima = taken * (TC_BN / 32);
+        const uint64_t minima = n / (32 * stride);
         // a row's chance to be below: of a minimum it is kcand / minima
         const double p = 1.0 - std::pow(1.0 - std::min(0.99, static_cast<double>(kcand) / static_cast<double>(minima)), 1.0 / 32.0);
         // what a query may collect: the threshold is the kcand-th of a sample, its rank in all rows known to 1 / sqrt(kcand);
@@ -844,12 +850,73 @@ bf_sample(uint64_t n, uint32_t dim, uint32_t kcand) {
         const double most = p * static_cast<double>(n) * (1.0 + 6.0 / std::sqrt(static_cast<double>(kcand))) + 256.0;
         if (minima >= 4ull * kcand && most <= BF_COLLECT_KEYS) {
             s.stride = stride;
-            s.tiles = taken;
+            s.groups = minima;
             s.most = most;
             return s;
         }
     }
     return s;
+}
+
+// Row number `column` of a sample of `groups` times 32 of n rows.  The rows fall into as many stretches as the sample has rows, one
+// is taken of each, somewhere in it, and neighbouring stretches go to different groups of 32: what the sample tells does not depend
+// on the order of the rows.  (Whole tiles of 128 neighbours as a sample, with rows of a cluster stored together: the kcand-th
+// minimum was that of a far cluster, every query collected more than it has room for, and the exact pass took the batch.)
+__device__ __forceinline__ uint64_t
+bf_sample_row(uint64_t column, uint64_t groups, uint64_t n) {
+    const uint64_t total = groups * 32, s = (column & 31u) * groups + (column >> 5);
+    const uint64_t first = s * n / total, width = (s + 1) * n / total - first;
+    uint32_t h = static_cast<uint32_t>(s) * 0x9E3779B1u;   // (any fixed mixing of the bits: orders with a period are not in step with it)
+    h = (h ^ (h >> 15)) * 0x85EBCA6Bu;
+    h ^= h >> 13;
+    return first + ((h * width) >> 32);
+}
+
+// The tiled terms and the score biases of the sample's rows, 16 bytes of a term per thread, rows before units.
+__global__ void __launch_bounds__(256)
+bf_sample_kernel(const uint4* __restrict__ hi, const uint4* __restrict__ lo, const float* __restrict__ bias, uint64_t n, uint64_t groups,
+                 uint32_t chunks, uint4* __restrict__ out_hi, uint4* __restrict__ out_lo, float* __restrict__ out_bias) {
+    const uint64_t e = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
+    const uint64_t padded = (groups * 32 + TC_BN - 1) / TC_BN * TC_BN, column = e % padded;
+    const uint32_t unit = static_cast<uint32_t>(e / padded);   // eight dimensions
+    if (unit >= chunks * (TC_KC / 8)) {
+        return;
+    }
+    const bool there = column < groups * 32;
+    const uint64_t row = there ? bf_sample_row(column, groups, n) : 0;
+    auto place = [&](uint64_t r) -> uint64_t {   // of the 16 bytes in the tiled layout (tc_pretile_kernel)
+        return ((r / TC_BN * chunks + unit / 8) * 16 + r % TC_BN / 8) * 64 + unit % 8 * 8 + r % 8;
+    };
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    out_hi[place(column)] = there ? __ldg(hi + place(row)) : none;
+    if (lo != nullptr) {
+        out_lo[place(column)] = there ? __ldg(lo + place(row)) : none;
+    }
+    if (unit == 0 && there && bias != nullptr) {
+        out_bias[column] = __ldg(bias + row);
+    }
+}
+
+// Leaves the sample beside the tiled rows, where it stays until they change or a search wants another share of them.
+static int
+bf_take_sample(vb200_bf* ix, const BfSample& sample, const float* bias) {
+    if (ix->sample_stride == sample.stride) {
+        return 0;
+    }
+    ix->sample_stride = 0;
+    const uint64_t rows = sample.groups * 32, elems = tc_tiled_elems(rows, ix->dim);
+    const bool bf16 = ix->quant == VB200_QUANT_BF16;
+    VB_TRY(ix->sample_hi.reserve(elems));
+    VB_TRY(ix->sample_lo.reserve(bf16 ? 0 : elems));
+    VB_TRY(ix->sample_bias.reserve(bias != nullptr ? rows : 0));
+    const uint64_t blocks = (elems / 8 + 255) / 256;
+    VB_CHECK_ARG(blocks <= 0x7fffffffu, "too many rows for a sample");
+    VB_LAUNCH(bf_sample_kernel, static_cast<uint32_t>(blocks), 256, 0, reinterpret_cast<const uint4*>(ix->base_hi.ptr),
+              bf16 ? static_cast<const uint4*>(nullptr) : reinterpret_cast<const uint4*>(ix->base_lo.ptr), bias, ix->n, sample.groups,
+              (ix->dim + TC_KC - 1) / TC_KC, reinterpret_cast<uint4*>(ix->sample_hi.ptr), reinterpret_cast<uint4*>(ix->sample_lo.ptr),
+              ix->sample_bias.ptr);
+    ix->sample_stride = sample.stride;
+    return 0;
 }
 
 static int
@@ -860,13 +927,15 @@ bf_search_collected(vb200_bf* ix, const BfStaged& staged, const BfSample& sample
     const float* q_dev = staged.queries;
     const float alpha = l2 ? -2.0f : -1.0f;
     VB_TRY(bf_tile_base(ix));
+    VB_TRY(bf_take_sample(ix, sample, staged.bias));
     VB_TRY(bf_tile_queries(ix, q_dev, nq));
     const uint32_t chunks = (dim + TC_KC - 1) / TC_KC, terms = bf16 ? 1 : 3;
     const uint32_t kcand = static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n));
-    const uint64_t ld = sample.tiles * (TC_BN / 32);
+    const uint64_t ld = (sample.groups + 3) / 4 * 4;   // (whole tiles; groups past the last are +inf)
+    const uint32_t room = std::max<uint32_t>(512, std::min<uint32_t>(BF_COLLECT_KEYS, static_cast<uint32_t>(1.25 * sample.most) + 256));
     // whole row tiles whose lists fit
     TcCollect plan = tc_collect_plan(nq, ix->n, sample.most);
-    uint64_t slice = BF_COLLECT_SLOTS / (static_cast<uint64_t>(plan.lists) * plan.cap) / TC_BM * TC_BM;
+    uint64_t slice = BF_COLLECT_SLOTS / (static_cast<uint64_t>(plan.lists) * plan.cap + room) / TC_BM * TC_BM;
     slice = slice < TC_BM ? TC_BM : (slice > nq ? nq : slice);
     if (slice < nq) {
         const uint64_t parts = (nq + slice - 1) / slice;
@@ -877,33 +946,40 @@ bf_search_collected(vb200_bf* ix, const BfStaged& staged, const BfSample& sample
     VB_TRY(ix->row_bound.reserve(slice));
     VB_TRY(ix->tc_out.reserve(slice * plan.lists * plan.cap));
     VB_TRY(ix->list_count.reserve(slice * plan.lists));
+    VB_TRY(ix->spill.reserve(slice * room));
+    VB_TRY(ix->spilled.reserve(slice));
     VB_TRY(ix->unsure.reserve(nq + 2));
     VB_CUDA(cudaMemsetAsync(ix->unsure.ptr, 0, 2 * sizeof(uint32_t), current_stream()));
     int* const error_flag = reinterpret_cast<int*>(ix->unsure.ptr);
     const TcOperand b{ix->base_hi.ptr, bf16 ? nullptr : ix->base_lo.ptr, ix->n, chunks, dim};
+    const TcOperand sampled{ix->sample_hi.ptr, bf16 ? nullptr : ix->sample_lo.ptr, sample.groups * 32, chunks, dim};
+    const float* sampled_bias = staged.bias != nullptr ? ix->sample_bias.ptr : nullptr;
     BfCollected c{};
     c.keys = ix->tc_out.ptr;
     c.count = ix->list_count.ptr;
     c.thr = ix->row_bound.ptr;
     c.lists = plan.lists;
     c.cap = plan.cap;
-    c.room = std::max<uint32_t>(512, std::min<uint32_t>(BF_COLLECT_KEYS, static_cast<uint32_t>(1.25 * sample.most) + 256));
+    c.room = room;
+    c.spill = ix->spill.ptr;
+    c.spilled = ix->spilled.ptr;
     c.dim = dim;
     c.kcand = kcand;
     c.k = k;
     c.metric = ix->metric;
     c.labels = ix->labels.ptr;
     c.m = bf_margin(ix);
-    const size_t smem = static_cast<size_t>(c.room) * sizeof(uint64_t) + (plan.lists + 1) * sizeof(uint32_t) + dim * sizeof(float);
+    const size_t smem = static_cast<size_t>(c.room) * sizeof(uint64_t) + (plan.lists + 2) * sizeof(uint32_t) + dim * sizeof(float);
     VB_CHECK_ARG(smem <= 180 * 1024, "dim = %u is too large for the exact re-scoring step", dim);
     for (uint64_t q0 = 0; q0 < nq; q0 += slice) {
         const uint64_t m = std::min(slice, nq - q0);
         const size_t off = static_cast<size_t>(q0 / TC_BM) * chunks * TC_CHUNK_ELEMS;
         const TcOperand a{ix->q_hi.ptr + off, bf16 ? nullptr : ix->q_lo.ptr + off, m, chunks, dim};
-        VB_TRY(tc_minima(a, b, terms, alpha, staged.bias, sample.stride, ix->scores.ptr, ld, error_flag));
+        VB_TRY(tc_minima(a, sampled, terms, alpha, sampled_bias, ix->scores.ptr, ld, error_flag));
         VB_LAUNCH(bf_threshold_kernel, static_cast<uint32_t>(m), BF_THRESHOLD_THREADS, 0, ix->scores.ptr, static_cast<uint32_t>(ld), kcand,
-                  ix->row_bound.ptr);
-        VB_TRY(tc_collect(plan, a, b, terms, alpha, staged.bias, ix->row_bound.ptr, ix->tc_out.ptr, ix->list_count.ptr, error_flag));
+                  ix->row_bound.ptr, ix->spilled.ptr);
+        VB_TRY(tc_collect(plan, a, b, terms, alpha, staged.bias, ix->row_bound.ptr, ix->tc_out.ptr, ix->list_count.ptr,
+                          TcSpill{ix->spill.ptr, ix->spilled.ptr, room}, error_flag));
         c.queries = bf16 ? static_cast<const void*>(ix->q_bf16.ptr + q0 * dim) : q_dev + q0 * dim;
         c.base = bf16 ? static_cast<const void*>(ix->base_bf16.ptr) : ix->base_f32.ptr;
         c.ids = ids_dev + q0 * k;

@@ -204,13 +204,14 @@ tc_compact_row(uint64_t* my_buf, uint32_t& my_cnt, float& my_thr, uint32_t owner
 // selection, the scores themselves are stored; MODE 3: every column scoring below the row's fixed
 // threshold (row_bound) is appended, unsorted, to the row's output list of `cap` entries -- no
 // sorting at all, the caller sizes the lists from the threshold's expected pass rate and an
-// overflowing list sets bit 1 of the error flag.  MODE 4: one minimum per row and 32 columns is stored.
+// overflowing list sets bit 1 of the error flag.  MODE 4: one minimum per row and 32 columns is stored.  MODE 5: as 3, but what a
+// list has no room for goes to the row's spill.
 template <int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_candidates_kernel(const TcParams p) {
     constexpr bool SMALL_M = MODE == 0;
     constexpr bool STORE = MODE == 2;
-    constexpr bool THRESH = MODE == 3;
+    constexpr bool SPILL = MODE == 5, THRESH = MODE == 3 || SPILL;
     constexpr bool MINIMA = MODE == 4;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ TcShared sh;
@@ -226,7 +227,7 @@ tc_candidates_kernel(const TcParams p) {
     const uint32_t stage_bytes = ((p.a_resident ? 0u : n_terms_op) + n_terms_op * step) * TC_CHUNK_BYTES;
     const uint32_t chunks = p.a.chunks;
     const uint64_t m_tiles = (p.a.rows + TC_BM - 1) / TC_BM;
-    const uint64_t n_tiles = ((p.b.rows + TC_BN - 1) / TC_BN + p.tile_stride - 1) / p.tile_stride;   // that take part
+    const uint64_t n_tiles = (p.b.rows + TC_BN - 1) / TC_BN;
     const uint64_t n_items = m_tiles * p.n_split;
 
     if (threadIdx.x == 0) {
@@ -278,10 +279,9 @@ tc_candidates_kernel(const TcParams p) {
     };
     // B tile number u of share `split`.  (Row tiles that start a share at different tiles, so as not to ask L2 for the
     // same lines together, were slower: 91 against 86 ms over 6M x 768 rows.)
-    auto number_at = [&](uint32_t split, uint32_t u) -> uint32_t {
+    auto tile_at = [&](uint32_t split, uint32_t u) -> uint32_t {
         return p.interleaved ? split + u * p.n_split : split * p.tiles_per_split + u;
     };
-    auto tile_at = [&](uint32_t split, uint32_t u) -> uint32_t { return number_at(split, u) * p.tile_stride; };
     if (warp == TC_EPI_WARPS) {
         // ---------------- MMA issue (one thread) ----------------
         // Written for latency: 32-bit counters that wrap by compare instead of divide, descriptors
@@ -509,7 +509,7 @@ tc_candidates_kernel(const TcParams p) {
             const uint32_t in_step = cgroup * warp_cols / TC_BN, in_tile = cgroup * warp_cols % TC_BN;
             const uint32_t tile0 = p.interleaved ? split32 : split32 * p.tiles_per_split, tile_inc = p.interleaved ? p.n_split : 1u;
             // first global column of this warp in the tile step that starts at B tile t; its second block of 32 follows
-            auto first_col = [&](uint32_t t) -> uint32_t { return (tile0 + (t + in_step) * tile_inc) * p.tile_stride * TC_BN + in_tile; };
+            auto first_col = [&](uint32_t t) -> uint32_t { return (tile0 + (t + in_step) * tile_inc) * TC_BN + in_tile; };
             float bias0 = 0.f, bias1 = 0.f, next0 = 0.f, next1 = 0.f;
             auto bias_of = [&](uint32_t t, uint32_t half) -> float {
                 const uint32_t nn = t < t1 ? first_col(t) + half * 32 + lane : b_rows;
@@ -658,7 +658,7 @@ tc_candidates_kernel(const TcParams p) {
                     const float mn = fminf(min3(m4[0], m4[1], m4[2]), m4[3]);
                     if (MINIMA) {
                         if (valid_row && tile_present) {
-                            p.store[grow * p.store_ld + number_at(split32, t + in_step) * (TC_BN / 32) + in_tile / 32 + half] = mn;
+                            p.store[grow * p.store_ld + tile_at(split32, t + in_step) * (TC_BN / 32) + in_tile / 32 + half] = mn;
                         }
                         continue;
                     }
@@ -718,6 +718,11 @@ tc_candidates_kernel(const TcParams p) {
                                                     buf[cnt] = key;
                                                 } else if (cnt < p.cap) {
                                                     list[cnt] = key;
+                                                } else if (SPILL) {
+                                                    const uint32_t at = atomicAdd(p.spill_count + grow, 1u);
+                                                    if (at < p.spill_cap) {
+                                                        p.spill[grow * p.spill_cap + at] = key;
+                                                    }
                                                 }
                                                 ++cnt;
                                             }
@@ -739,7 +744,7 @@ tc_candidates_kernel(const TcParams p) {
             if (THRESH) {
                 if (valid_row) {
                     p.out_count[(grow * p.n_split + split) * TC_COL_GROUPS + cgroup] = cnt;
-                    if (cnt > p.cap) {
+                    if (!SPILL && cnt > p.cap) {
                         atomicOr(p.error_flag, 2);
                     }
                 }
@@ -868,7 +873,6 @@ tc_plan(TcParams& p, size_t sort_bytes, size_t* smem_bytes) {
     p.a_resident = resident ? 1u : 0u;
     p.wide = wide ? 1u : 0u;
     p.last_steps = p.a.dim != 0 ? (p.a.dim - (p.a.chunks - 1) * TC_KC + 15) / 16 : TC_KC / 16;
-    p.tile_stride = 1;
     *smem_bytes = fixed + stages * stage_bytes(resident, wide);
 }
 
@@ -1089,9 +1093,9 @@ tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, uint
 }
 
 int
-tc_minima(const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev, uint32_t tile_stride,
-          float* minima_dev, uint64_t ld, int* deferred_flag_dev) {
-    VB_CHECK_ARG(a.rows > 0 && b.rows > 0 && tile_stride > 0, "tc_minima: empty operand");
+tc_minima(const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev, float* minima_dev, uint64_t ld,
+          int* deferred_flag_dev) {
+    VB_CHECK_ARG(a.rows > 0 && b.rows > 0, "tc_minima: empty operand");
     VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_minima: operand depths differ");
     VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_minima: 1 or 3 terms");
     TcParams p{};
@@ -1100,9 +1104,8 @@ tc_minima(const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha,
     p.n_terms = n_terms;
     size_t smem = 0;
     tc_plan(p, 0, &smem);
-    p.tile_stride = tile_stride;
     const uint64_t m_tiles = (a.rows + TC_BM - 1) / TC_BM;
-    const uint64_t n_tiles = ((b.rows + TC_BN - 1) / TC_BN + tile_stride - 1) / tile_stride;
+    const uint64_t n_tiles = (b.rows + TC_BN - 1) / TC_BN;
     VB_CHECK_ARG(ld >= n_tiles * (TC_BN / 32), "tc_minima: rows of minima too short");
     const uint32_t sms = static_cast<uint32_t>(sm_count());
     uint64_t n_split = (2ull * sms + m_tiles - 1) / m_tiles;
@@ -1154,7 +1157,7 @@ tc_collect_plan(uint64_t a_rows, uint64_t b_rows, double expected_per_row) {
 
 int
 tc_collect(const TcCollect& plan, const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev,
-           const float* row_thr_dev, uint64_t* out_dev, uint32_t* out_count_dev, int* deferred_flag_dev) {
+           const float* row_thr_dev, uint64_t* out_dev, uint32_t* out_count_dev, const TcSpill& spill, int* deferred_flag_dev) {
     VB_CHECK_ARG(a.rows > 0 && b.rows > 0, "tc_collect: empty operand");
     VB_CHECK_ARG(a.chunks == b.chunks && a.chunks > 0, "tc_collect: operand depths differ");
     VB_CHECK_ARG(n_terms == 1 || n_terms == 3, "tc_collect: 1 or 3 terms");
@@ -1177,7 +1180,10 @@ tc_collect(const TcCollect& plan, const TcOperand& a, const TcOperand& b, uint32
     p.out_count = out_count_dev;
     p.error_flag = deferred_flag_dev;
     p.spin_limit = tc_spin_limit();
-    auto kernel = tc_candidates_kernel<3>;
+    p.spill = spill.keys;
+    p.spill_count = spill.count;
+    p.spill_cap = spill.cap;
+    auto kernel = tc_candidates_kernel<5>;
     VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(kernel), smem));
     VB_LAUNCH(kernel, static_cast<uint32_t>(items < sms ? items : sms), TC_THREADS, smem, p);
     return 0;

@@ -61,15 +61,17 @@ struct TcParams {
     uint32_t diag;            // timing experiments only: bit 0 skips the selection, bit 1 the MMAs
 #endif
     uint32_t last_steps;      // k-steps of 16 of the last chunk that hold anything
-    uint32_t tile_stride;     // B tiles 0, tile_stride, 2 tile_stride, ... take part (a sample of the columns); 1: all
     uint32_t interleaved;     // 1: share s holds tiles s, s + n_split, ...; the queue walks row tiles within a share
     uint64_t* scratch;        // [grid][128][TC_COL_GROUPS][cap] candidate buffers
     uint64_t* out;            // [a.rows][n_split][TC_COL_GROUPS][m] keys (ordered score << 32 | column), KEY_INF padded
                               // (threshold mode: [a.rows][n_split][TC_COL_GROUPS][cap], unsorted, with out_count)
     uint32_t* out_count;      // threshold mode: [a.rows][n_split][TC_COL_GROUPS] entries offered to each list
+    uint64_t* spill;          // spill mode: [a.rows][spill_cap] entries that a list had no room for, with spill_count [a.rows]
+    uint32_t* spill_count;
+    uint32_t spill_cap;
     uint32_t col_base;        // added to column indices in the keys
     float* store;             // score-matrix mode: [a.rows][store_ld] fp32 scores instead of candidates
-                              // (minima mode: the smallest score of every 32 columns that take part)
+                              // (minima mode: the smallest score of every 32 columns)
     uint64_t store_ld;        // row stride of `store` in floats (multiple of 4, store 16-byte aligned)
     uint32_t store_wide;      // 1: rows of `store` start on 32-byte boundaries
     int* error_flag;          // [0] set non-zero if a bounded wait gave up; [1] counts the rows flagged below
@@ -347,11 +349,11 @@ int tc_below_threshold(TcWorkspace& ws, const TcOperand& a, const TcOperand& b, 
                        uint32_t max_per_row, DevBuf<uint64_t>& out, DevBuf<uint32_t>& out_count, uint32_t* lists_out,
                        uint32_t* cap_out, bool* overflow_out, int* deferred_flag_dev = nullptr);
 
-// The smallest score of every 32 columns of B's tiles 0, tile_stride, 2 tile_stride, ... (128 columns each) as
-// minima_dev[a.rows][ld], ld >= 4 ceil(tiles / tile_stride); columns past the last row of B count as +inf.
+// The smallest score of every 32 columns of B's tiles (128 columns each) as minima_dev[a.rows][ld], ld >= 4 tiles; columns past the
+// last row of B count as +inf.
 // deferred_flag_dev: as for tc_below_threshold.
-int tc_minima(const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev, uint32_t tile_stride,
-              float* minima_dev, uint64_t ld, int* deferred_flag_dev);
+int tc_minima(const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev, float* minima_dev,
+              uint64_t ld, int* deferred_flag_dev);
 
 // tc_below_threshold for exact search over many rows: lists per row as many as the shares need, and shares that take B's tiles in turn, so
 // that rows stored near one another are spread over a row's lists.  out_dev[a.rows][lists][cap], out_count_dev[a.rows][lists].
@@ -359,8 +361,14 @@ struct TcCollect {
     uint32_t n_split, tiles_per_split, lists, cap;
 };
 TcCollect tc_collect_plan(uint64_t a_rows, uint64_t b_rows, double expected_per_row);
+// What the lists of a row have no room for: rows stored near one another may all fall into a few lists.
+struct TcSpill {
+    uint64_t* keys;      // [a.rows][cap]
+    uint32_t* count;     // [a.rows] entries offered; zero before the launch
+    uint32_t cap;
+};
 int tc_collect(const TcCollect& plan, const TcOperand& a, const TcOperand& b, uint32_t n_terms, float alpha, const float* bias_dev,
-               const float* row_thr_dev, uint64_t* out_dev, uint32_t* out_count_dev, int* deferred_flag_dev);
+               const float* row_thr_dev, uint64_t* out_dev, uint32_t* out_count_dev, const TcSpill& spill, int* deferred_flag_dev);
 
 // The whole score matrix alpha * <a, b> + bias as fp32 in scores_dev[a.rows][ld] (ld >= b.rows, a
 // multiple of 4, scores_dev 16-byte aligned), from the same tensor-core pipeline.
