@@ -137,3 +137,25 @@ def test_exact_search_without_room_for_a_second_copy(engine):
         assert np.array_equal(got[1], np.concatenate([w[1] for w in want]))
         assert np.array_equal(got[0], np.concatenate([w[0] for w in want]))
         got = ix.search(q, k)
+
+
+def test_exact_batches_with_lists_for_a_few_queries_at_a_time(engine):
+    """3000 queries over 400,000 rows collect some 300 MB of candidates.  With less than that left they go in smaller parts; the
+    search of more rows at a time, which a batch without any such room is left to, does not look for neighbours that the scores
+    cannot tell apart, and these rows lie far from the origin."""
+    import torch
+
+    n, dim, nq, k = 400_000, 16, 3000, 100
+    g = torch.Generator(device="cuda").manual_seed(8)
+    base = 80 + 0.01 * torch.randn((n, dim), generator=g, device="cuda")
+    q = (80 + 0.01 * torch.randn((nq, dim), generator=g, device="cuda")).cpu().numpy()
+    ix = engine.BfHandle(dim, 0)
+    ix.add(base, torch.arange(n, dtype=torch.int64, device="cuda"))
+    del base
+    ix.search(q[:9].copy(), k)                     # (the tiled copy of the rows)
+    some = slice(0, nq, 100)
+    one = [ix.search(v[None].copy(), k) for v in q[some]]
+    with LittleMemory(160 << 20):
+        got = ix.search(q, k)
+    assert np.array_equal(got[1][some], np.concatenate([o[1] for o in one]))
+    assert np.array_equal(got[0][some], np.concatenate([o[0] for o in one]))

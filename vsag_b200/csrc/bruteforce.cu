@@ -829,7 +829,8 @@ constexpr uint32_t BF_COLLECT_KEYS = 12288;          // of a query, at most (96 
 // 6M x 768 bf16 rows under the power limit: 89.2 ms against 87.2).
 constexpr double BF_COLLECT_PRODUCTS = 1.6e12;
 constexpr uint32_t BF_COLLECT_DIMS = 16384;          // the query lies beside them
-constexpr uint64_t BF_COLLECT_SLOTS = uint64_t{256} << 20;   // list entries of the queries that go together, at most (2 GiB)
+// List entries of the queries that go together, at most (2 GiB); where that is not to be had an eighth, and an eighth of that.
+constexpr uint64_t BF_COLLECT_SLOTS = uint64_t{256} << 20, BF_COLLECT_LEAST = BF_COLLECT_SLOTS / 64;
 
 // The sample takes a thirty-second of the rows, or the smallest larger power of two's share whose minima are four times kcand, so
 // that the threshold is near the kcand-th best of the sample; at most an eighth, beyond which the scores are as well written.
@@ -920,7 +921,7 @@ bf_take_sample(vb200_bf* ix, const BfSample& sample, const float* bias) {
 }
 
 static int
-bf_search_collected(vb200_bf* ix, const BfStaged& staged, const BfSample& sample, uint64_t nq, uint32_t k, int64_t* ids_dev,
+bf_search_collected(vb200_bf* ix, const BfStaged& staged, const BfSample& sample, uint64_t slots, uint64_t nq, uint32_t k, int64_t* ids_dev,
                     float* dists_dev) {
     const uint32_t dim = ix->dim;
     const bool l2 = ix->metric == VB200_METRIC_L2, bf16 = ix->quant == VB200_QUANT_BF16;
@@ -935,7 +936,7 @@ bf_search_collected(vb200_bf* ix, const BfStaged& staged, const BfSample& sample
     const uint32_t room = std::max<uint32_t>(512, std::min<uint32_t>(BF_COLLECT_KEYS, static_cast<uint32_t>(1.25 * sample.most) + 256));
     // whole row tiles whose lists fit
     TcCollect plan = tc_collect_plan(nq, ix->n, sample.most);
-    uint64_t slice = BF_COLLECT_SLOTS / (static_cast<uint64_t>(plan.lists) * plan.cap + room) / TC_BM * TC_BM;
+    uint64_t slice = slots / (static_cast<uint64_t>(plan.lists) * plan.cap + room) / TC_BM * TC_BM;
     slice = slice < TC_BM ? TC_BM : (slice > nq ? nq : slice);
     if (slice < nq) {
         const uint64_t parts = (nq + slice - 1) / slice;
@@ -1102,22 +1103,33 @@ vb200_bf_search_filtered(vb200_bf_t ix, const float* queries, uint64_t nq, uint3
         const BfSample sample = staged.masked ? BfSample{} : bf_sample(ix->n, ix->dim, static_cast<uint32_t>(std::min<uint64_t>(k + BF_SLACK, ix->n)));
         const double products = static_cast<double>(nq) * ix->n * ix->dim * (ix->quant == VB200_QUANT_BF16 ? 1 : 3);
         collected = sample.stride != 0 && products <= BF_COLLECT_PRODUCTS;
-        if (collected) {
-            rc = bf_search_collected(ix, staged, sample, nq, k, ids_dev, dists_dev);
-        } else if (scores) {
-            rc = bf_search_scores(ix, staged, nq, k, ids_dev, dists_dev);
-        }
-        if (rc == VB200_NO_ENOUGH_MEMORY) {
-            // the tiled copy of the rows did not fit beside them: the slab of scores needs none
+        auto out_of_memory = [&]() -> bool {   // then what the attempt has taken is given back
+            if (rc != VB200_NO_ENOUGH_MEMORY) {
+                return false;
+            }
             (void)cudaStreamSynchronize(current_stream());
-            collected = scores = false;
             if (!ix->tiled_valid) {
                 ix->base_hi.release();
                 ix->base_lo.release();
             }
             ix->scores.release();
             ix->tc_out.release();
+            ix->spill.release();
             rc = 0;
+            return true;
+        };
+        for (uint64_t slots = BF_COLLECT_SLOTS; collected; slots /= 8) {
+            rc = bf_search_collected(ix, staged, sample, slots, nq, k, ids_dev, dists_dev);
+            if (!out_of_memory()) {
+                break;
+            }
+            // (the tiled copy of the rows may be what did not fit)
+            collected = ix->tiled_valid && slots > BF_COLLECT_LEAST;
+            scores = scores && ix->tiled_valid;
+        }
+        if (rc == 0 && scores && !collected) {
+            rc = bf_search_scores(ix, staged, nq, k, ids_dev, dists_dev);
+            scores = !out_of_memory();   // (the slab of scores needs no tiled copy)
         }
     }
     if (rc == 0 && !few && !scores && !collected) {
