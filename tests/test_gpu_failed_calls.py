@@ -159,3 +159,67 @@ def test_exact_batches_with_lists_for_a_few_queries_at_a_time(engine):
         got = ix.search(q, k)
     assert np.array_equal(got[1][some], np.concatenate([o[1] for o in one]))
     assert np.array_equal(got[0][some], np.concatenate([o[0] for o in one]))
+
+
+def fp32_index(engine, n, dim, seed):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.rand((n, dim), generator=g, device="cuda")
+    ix = engine.IvfHandle(dim, 0, 16, engine.QUANT_FP32)
+    ix.train(x[:4000].contiguous(), iters=2, init=x[:16].contiguous())
+    ix.add(x, torch.arange(n, dtype=torch.int64, device="cuda"))
+    return ix, x[:200].cpu().numpy(), x[-500:].cpu().numpy()
+
+
+@pytest.mark.parametrize("dim", [65, 128])
+def test_only_repeated_batches_keep_a_second_copy_of_fp32_rows(engine, dim):
+    """The copy is there from the second batch by tiles on, its rows no longer than the rows themselves, and goes when rows are
+    added; the batches before and after it was made agree with single queries."""
+    n = 50_000
+    ix, q, more = fp32_index(engine, n, dim, 9)
+    alone = ix.memory_usage()
+    one = [ix.search(q[i:i + 1].copy(), 5, 8) for i in range(20)]
+    assert ix.memory_usage() == alone
+    for batch in range(3):
+        got = ix.search(q, 5, 8)
+        for j in (0, 1):
+            assert np.array_equal(got[j][:20], np.concatenate([o[j] for o in one]))
+        assert ix.memory_usage() - alone == (0 if batch == 0 else n * 4 * ((dim + 7) // 8 * 8))
+    ix.add(more, np.arange(n, n + len(more), dtype=np.int64))
+    assert ix.memory_usage() < alone * 1.1
+    got, one = ix.search(q, 5, 8), [ix.search(q[i:i + 1].copy(), 5, 8) for i in range(20)]
+    for j in (0, 1):
+        assert np.array_equal(got[j][:20], np.concatenate([o[j] for o in one]))
+
+
+def test_adding_to_an_index_of_more_than_a_third_of_the_memory(engine):
+    """640 MB of rows, and a second copy for the tile scan as large: an add needs room for the rows beside themselves, and 400 MB
+    are left."""
+    n, dim = 400_000, 400
+    ix, q, more = fp32_index(engine, n, dim, 10)
+    want = ix.search(q, 5, 8)
+    ix.search(q, 5, 8)
+    with LittleMemory(400 << 20):
+        ix.add(more, np.arange(n, n + len(more), dtype=np.int64))
+        assert ix.num_elements() == n + len(more)
+    got = ix.search(more, 2, 16)
+    assert np.array_equal(np.sort(got[0], 1)[:, 1], np.arange(n, n + len(more))) and np.array_equal(got[1], np.zeros_like(got[1]))
+    again = ix.search(q, 5, 8)
+    assert np.all(again[1] <= want[1])
+
+
+def test_a_batch_that_lacks_memory_gives_up_the_second_copy(engine):
+    """A deeper batch whose scores do not fit while the copy is held."""
+    n, dim = 400_000, 400
+    ix, q, _ = fp32_index(engine, n, dim, 11)
+    for _ in range(2):
+        ix.search(q[:80].copy(), 5, 2)
+    q = np.tile(q, (3, 1))
+    held = ix.memory_usage()
+    with LittleMemory(200 << 20):
+        got = ix.search(q, 5, 16)                   # 400,000 scores a query
+    assert ix.memory_usage() <= held - n * dim * 4
+    one = [ix.search(q[i:i + 1].copy(), 5, 16) for i in range(20)]
+    for j in (0, 1):
+        assert np.array_equal(got[j][:20], np.concatenate([o[j] for o in one]))

@@ -203,6 +203,24 @@ def test_tiles_equal_queries_one_by_one(engine, oracle, quant, dim, nq):
     exactly(got, (np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])))
 
 
+@pytest.mark.parametrize("dim,nq", [(16, 12), (33, 31), (64, 33), (65, 64), (72, 40), (128, 65), (200, 130), (520, 9)])
+@pytest.mark.parametrize("metric", [0, 1])
+def test_repeated_fp32_batches_equal_the_first(engine, dim, nq, metric):
+    """From the second on rows are read as two bf16 terms, a piece of 64 dimensions at a time with zeros behind the last."""
+    sizes, k = [1, 129, 2200], 10
+    labels = np.repeat(np.arange(3, dtype=np.int32), sizes)
+    x, q = mixture(63, labels.size, dim, 3, 0.4), mixture(64, nq, dim, 3, 0.4)
+    ix = engine.IvfHandle(dim, metric, 3, engine.QUANT_FP32)
+    ix.train(x, iters=1, init=np.ascontiguousarray(x[:3]))
+    ix.add(x, np.arange(labels.size, dtype=np.int64), labels=labels)
+    lists = np.tile(np.arange(3, dtype=np.int32), (nq, 1))
+    first, second = (ix.search_filtered(q, k, 3, bucket_ids=lists) for _ in range(2))
+    one = [ix.search_filtered(q[i:i + 1].copy(), k, 3, bucket_ids=lists[:1]) for i in range(nq)]
+    want = np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])
+    exactly(first, want)
+    exactly(second, want)
+
+
 # ---- SQ8 lists that two to four queries share ---------------------------------------------------------------------
 @pytest.mark.parametrize("metric", [0, 1])
 @pytest.mark.parametrize("dim,nq", [(16, 19), (100, 15), (130, 19), (528, 12), (2049, 10)])

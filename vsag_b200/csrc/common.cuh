@@ -138,26 +138,36 @@ struct DevBuf {
     }
     // Grow-only reservation; contents are not preserved.
     int reserve(size_t n) {
-        if (n <= cap) {
-            return 0;
-        }
-        release();
-        if (n == 0) {
-            return 0;
-        }
-        void* p = nullptr;
-        cudaError_t e = pool_malloc(&p, n * sizeof(T));
+        const cudaError_t e = grow(n);
         if (e != cudaSuccess) {
-            cudaGetLastError();
             VB_FAIL(VB200_NO_ENOUGH_MEMORY, "allocation of %zu bytes of device memory failed: %s", n * sizeof(T),
                     cudaGetErrorString(e));
         }
-        ptr = static_cast<T*>(p);
-        cap = n;
         return 0;
+    }
+    // The same for memory that the caller can do without: no error is reported.
+    bool try_reserve(size_t n) {
+        return grow(n) == cudaSuccess;
     }
     size_t bytes() const {
         return cap * sizeof(T);
+    }
+
+private:
+    cudaError_t grow(size_t n) {
+        if (n <= cap) {
+            return cudaSuccess;
+        }
+        release();
+        void* p = nullptr;
+        const cudaError_t e = pool_malloc(&p, n * sizeof(T));
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return e;
+        }
+        ptr = static_cast<T*>(p);
+        cap = n;
+        return cudaSuccess;
     }
 };
 

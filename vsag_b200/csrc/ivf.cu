@@ -152,7 +152,10 @@ struct vb200_ivf {
     uint32_t max_list_len = 0;   // the longest list this index (shard) holds
     CUtensorMap row_map{};       // the stored rows for the tile scan's copies (fp32, bf16, fp16, RaBitQ)
     bool has_row_map = false;
-    DevBuf<uint16_t> split;      // fp32: the rows' two bf16 terms, which row_map then covers; empty where memory was short
+    DevBuf<uint16_t> split;      // fp32: the rows' two bf16 terms, or empty (ivf_split_rows)
+    CUtensorMap split_map{};
+    bool split_due = false;      // a batch has gone through the tiles since the rows changed
+    bool split_off = false;      // there was no room for the terms
     DevBuf<float> row_max;       // [0] largest norm of a stored row, [1] RaBitQ: largest norm / |error term|
     std::vector<uint64_t> longest_rows;   // [nlist + 1] rows of the i longest lists together
     bool balls_valid = false;    // the covering balls describe the lists as they are stored
@@ -3444,6 +3447,73 @@ launch_shared_scan(vb200_ivf* ix, const PairScan& sc, uint64_t nq) {
     return 0;
 }
 
+using TensorMapEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The driver's cuTensorMapEncodeTiled, or null.
+static TensorMapEncode
+tensor_map_encode() {
+    static const TensorMapEncode encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<TensorMapEncode>(fn);
+    }();
+    return encode;
+}
+
+static void
+ivf_drop_split(vb200_ivf* ix) {
+    ix->split.release();
+    ix->split_due = ix->split_off = false;
+}
+
+// For a search that lacks memory: whether there were terms to give back (they are not made again before the rows change).
+static bool
+ivf_give_up_split(vb200_ivf* ix) {
+    const bool had = ix->split.ptr != nullptr;
+    ix->split.release();
+    ix->split_off = true;
+    return had;
+}
+
+// The two bf16 terms of fp32 rows, which the tile scan then reads in place of the rows: made in the second batch that goes through
+// the tiles after the rows changed (the first may be the only one, and loses no more by converting than the copy costs; searches
+// that are not tiled never have one), while they take at most half of the memory that is free, and given back before rows are added
+// and when a search lacks memory.  In ix->split, empty when there are none.
+static int
+ivf_split_rows(vb200_ivf* ix) {
+    if (ix->quant != VB200_QUANT_FP32 || ix->split.ptr != nullptr || !ix->split_due || ix->split_off) {
+        return 0;
+    }
+    ix->split_off = true;   // until the rows change, if what follows finds no room or no map
+    const uint64_t pitch = (ix->dim + 7) / 8 * 8, elems = ix->n_stored * 2 * pitch, blocks = (elems / 16 + 255) / 256;
+    const TensorMapEncode encode = tensor_map_encode();
+    DevBuf<uint16_t> terms;
+    size_t left = 0, all = 0;
+    VB_CUDA(cudaMemGetInfo(&left, &all));
+    if (encode == nullptr || blocks > 0x7fffffffull || elems * sizeof(uint16_t) > left / 2 || !terms.try_reserve(elems)) {
+        return 0;
+    }
+    // (element, term, row): what lies past a row's last element comes as zeros
+    const cuuint64_t extents[3] = {pitch, 2, ix->n_stored}, strides[2] = {pitch * sizeof(uint16_t), 2 * pitch * sizeof(uint16_t)};
+    const cuuint32_t boxes[3] = {64, 1, 128}, steps[3] = {1, 1, 1};
+    if (encode(&ix->split_map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, terms.ptr, extents, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        return 0;
+    }
+    VB_LAUNCH(split_rows_kernel, static_cast<uint32_t>(blocks), 256, 0, ix->codes.ptr, ix->n_stored, ix->dim, ix->code_stride,
+              static_cast<uint32_t>(pitch), terms.ptr);
+    ix->split = std::move(terms);
+    ix->split_off = false;
+    return 0;
+}
+
 // Scans the lists as tiles into the score buffer.
 static int
 launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& plan) {
@@ -3454,7 +3524,7 @@ launch_tiles(vb200_ivf* ix, const PairScan& sc, uint64_t nq, const TilePlan& pla
     TileScan t{};
     t.s = sc.s;
     t.t = sc.t;
-    t.map = ix->row_map;
+    t.map = ix->split.ptr != nullptr ? ix->split_map : ix->row_map;
     t.items = g.items;
     t.queue = g.queue;
     t.pairs = g.tile_pairs;
@@ -3587,6 +3657,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
     pp.probes = ws.probes.ptr;
     if (plan != nullptr) {
         VB_TRY(ws.pair_minima.reserve(nq * stride / 32));
+        VB_TRY(ivf_split_rows(ix));
     }
     pp.t = PairTable{ws.pair_base.ptr, ws.query_rows.ptr, stride, ws.pair_scores.ptr, plan != nullptr ? ws.pair_minima.ptr : nullptr};
     pp.queries = q_dev;
@@ -3824,6 +3895,7 @@ ivf_search_scores(vb200_ivf* ix, const float* queries, uint64_t nq, uint32_t k, 
         }
     }
     ws.counts_clear = true;
+    ix->split_due = ix->split_due || plan != nullptr;
     if (*repeated != 0) {
         *repeats = true;
         return 0;
@@ -4259,47 +4331,22 @@ ivf_append_row_data(vb200_ivf* ix, const int64_t* ids, const float* rows_dev, ui
     return 0;
 }
 
-// Dimensions of a term of a row in the copy that split_rows_kernel makes.
-static uint64_t
-split_pitch(uint32_t dim) {
-    return (dim + 63) / 64 * 64;
-}
-
 // The tensor map through which the tile scan copies stored rows, 128 at a time; false where there is none (SQ8 has a
 // tiled copy instead).
 static bool
-make_row_map(const vb200_ivf* ix, const uint8_t* codes, const uint16_t* split, uint64_t n, CUtensorMap* map) {
-    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static const Encode encode = [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult found{};
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess ||
-            found != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            fn = nullptr;
-        }
-        return reinterpret_cast<Encode>(fn);
-    }();
+make_row_map(const vb200_ivf* ix, const uint8_t* codes, uint64_t n, CUtensorMap* map) {
+    const TensorMapEncode encode = tensor_map_encode();
     if (encode == nullptr || n == 0 || n >= 0x7FFFFF00ull) {
         return false;
     }
     CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_UINT16;
     CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B;
-    cuuint64_t extent = ix->dim, pitch = ix->code_stride;
+    cuuint64_t extent = ix->dim;
     cuuint32_t box = 64;
-    const void* rows = codes;
     switch (ix->quant) {
         case VB200_QUANT_BF16:
         case VB200_QUANT_FP16: break;
         case VB200_QUANT_FP32:
-            if (split != nullptr) {
-                extent = split_pitch(ix->dim) * 2;
-                pitch = extent * sizeof(uint16_t);
-                rows = split;
-                break;
-            }
             type = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
             swizzle = CU_TENSOR_MAP_SWIZZLE_NONE;
             box = 32;
@@ -4315,9 +4362,9 @@ make_row_map(const vb200_ivf* ix, const uint8_t* codes, const uint16_t* split, u
             break;
         default: return false;
     }
-    const cuuint64_t extents[2] = {extent, n}, strides[1] = {pitch};
+    const cuuint64_t extents[2] = {extent, n}, strides[1] = {ix->code_stride};
     const cuuint32_t boxes[2] = {box, 128}, steps[2] = {1, 1};
-    return encode(map, type, 2, const_cast<void*>(rows), extents, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+    return encode(map, type, 2, const_cast<uint8_t*>(codes), extents, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -4398,17 +4445,9 @@ ivf_commit_lists(vb200_ivf* ix, DevBuf<uint8_t>& new_codes, DevBuf<uint32_t>& ne
         VB_TRY(sync_stream());   // goff is a local
         ix->kchunks = kchunks;
     }
-    DevBuf<uint16_t> new_split;
-    if (ix->quant == VB200_QUANT_FP32 && n_new_stored > 0) {
-        const uint64_t pitch = split_pitch(dim), blocks = (n_new_stored * (pitch / 8) + 255) / 256;
-        if (blocks <= 0x7fffffffull && new_split.reserve(n_new_stored * 2 * pitch) == 0) {   // (not there: tiles convert the rows)
-            VB_LAUNCH(split_rows_kernel, static_cast<uint32_t>(blocks), 256, 0, new_codes.ptr, n_new_stored, dim, stride,
-                      static_cast<uint32_t>(pitch), new_split.ptr);
-        }
-    }
     VB_TRY(sync_stream());
-    ix->has_row_map = make_row_map(ix, new_codes.ptr, new_split.ptr, n_new_stored, &ix->row_map);
-    ix->split = std::move(new_split);
+    ix->has_row_map = make_row_map(ix, new_codes.ptr, n_new_stored, &ix->row_map);
+    ivf_drop_split(ix);
     ix->codes_t = std::move(new_tiled);
     ix->group_off = std::move(new_group_off);
     ix->code_norm = std::move(new_norm);
@@ -4530,7 +4569,8 @@ vb200_ivf_add(vb200_ivf_t ix, const float* data, uint64_t count, const int64_t* 
                             cudaMemcpyHostToDevice, st));
     VB_CUDA(cudaMemcpyAsync(new_off_dev.ptr, new_off.data(), (nlist + 1) * sizeof(uint32_t),
                             cudaMemcpyHostToDevice, st));
-    // 4. regrown arrays
+    // 4. regrown arrays (beside the old ones, so the rows' terms make way)
+    ivf_drop_split(ix);
     DevBuf<uint8_t> new_codes;
     DevBuf<uint32_t> new_inner, dst_of_row;
     const uint32_t stride = ix->code_stride;
@@ -4860,12 +4900,16 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
             if (how != SCAN_GROUPED) {
                 ws.filter = filter;
                 bool repeats = false;
-                const int rc = ivf_search_scores(ix, queries, nq, k, kscan, np, rerank, how == SCAN_TILES ? &plan : nullptr, bucket_ids, ids,
-                                                 dists, &repeats);
-                ws.filter = nullptr;
-                if (rc != 0) {
-                    (void)cudaStreamSynchronize(current_stream());   // what was launched may use the workspace
+                int rc = 0;
+                for (bool once_more = true; once_more;) {
+                    rc = ivf_search_scores(ix, queries, nq, k, kscan, np, rerank, how == SCAN_TILES ? &plan : nullptr, bucket_ids, ids,
+                                           dists, &repeats);
+                    if (rc != 0) {
+                        (void)cudaStreamSynchronize(current_stream());   // what was launched may use the workspace
+                    }
+                    once_more = rc == VB200_NO_ENOUGH_MEMORY && ivf_give_up_split(ix);
                 }
+                ws.filter = nullptr;
                 if (rc == VB200_NO_ENOUGH_MEMORY) {
                     // up to a gigabyte of scores did not fit: the grouped scan keeps the k best of each pair instead
                     ws.pair_scores.release();
@@ -4880,7 +4924,12 @@ vb200_ivf_search_ex(vb200_ivf_t ix, const float* queries, uint64_t nq, uint32_t 
     VB_TRY(ws.out_dists.reserve(total));
     const uint64_t* keys = nullptr;
     ws.filter = filter;
-    const int search_status = ivf_search_keys(ix, queries, nq, k, nprobe, factor, bucket_ids, &keys);
+    int search_status = ivf_search_keys(ix, queries, nq, k, nprobe, factor, bucket_ids, &keys);
+    if (search_status == VB200_NO_ENOUGH_MEMORY && ix->split.ptr != nullptr) {
+        (void)cudaStreamSynchronize(current_stream());
+        (void)ivf_give_up_split(ix);
+        search_status = ivf_search_keys(ix, queries, nq, k, nprobe, factor, bucket_ids, &keys);
+    }
     ws.filter = nullptr;
     VB_TRY(search_status);
     VB_LAUNCH(keys_to_results_kernel, static_cast<uint32_t>((total + 255) / 256), 256, 0, keys, total,

@@ -13,9 +13,9 @@
 // issues the MMAs, eight warps drain them.  (With the loads, the conversions and the gathering of an item on the same
 // warps, and the item's constants read by the epilogue, the kernel waited for one latency after another: 390 to
 // 560 us instead of 279 for 1000 queries against 32 lists each of 500k x 128 fp32.)  How rows become operands:
-//   fp32        two bf16 terms x = hi + lo, from a copy of the rows that holds them (made with the lists; where there is no
-//               memory for it, made in place in shared memory, which a tile waits for: 280 us of the case above, 173
-//               from the copy); hi*hi + lo*hi and hi*lo are accumulated (the dropped terms are below 2^-16 |x||q|)
+//   fp32        two bf16 terms x = hi + lo, made in place in shared memory, which a tile waits for, or from the second batch after
+//               the rows changed on read from a copy that holds them, where there is memory for one (280 us of the case
+//               above, 173 from the copy, which takes 100 to make and as much memory as the rows); hi*hi + lo*hi and hi*lo are accumulated (the dropped terms are below 2^-16 |x||q|)
 //   bf16, fp16  the codes as they are (TMA with the 128-byte swizzle); every product is exact in fp32
 //   sq8         the tiled copy of the codes as signed bytes code - 128, against three int8 terms of the query's
 //               weights: exact int32 sums
@@ -289,7 +289,7 @@ split_bf16x8(const float (&x)[8], uint4& hi, uint4& lo) {
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// fp32 rows (16-byte aligned) -> [rows][2][pitch] bf16 terms, zero past dim; pitch = dim rounded up to 64.  A thread per eight dimensions.
+// fp32 rows (16-byte aligned) -> [rows][2][pitch] bf16 terms, zero past dim; pitch = dim rounded up to 8.  A thread per eight dimensions.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const uint8_t* __restrict__ rows, uint64_t n, uint32_t dim, uint32_t stride, uint32_t pitch, uint16_t* __restrict__ out) {
     const uint64_t e = static_cast<uint64_t>(blockIdx.x) * 256 + threadIdx.x;
@@ -343,6 +343,14 @@ tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint64_t*
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
         "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void
+tma_load_3d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
 
@@ -535,9 +543,12 @@ tile_scan_kernel(const __grid_constant__ TileScan p) {
                     } else if (lane == 0) {
                         uint64_t* bar = F::CONVERT ? &sh.raw_full[stage] : &sh.full[stage];
                         mbar_expect_tx(bar, STAGE);
-                        if (F::SPLIT) {
+                        if (FMT == ROW_F32_SPLIT) {
+                            tma_load_3d(dst, &p.map, piece * 64, 0, it.lbeg + r0, bar);
+                            tma_load_3d(dst + TILE_A_TERM, &p.map, piece * 64, 1, it.lbeg + r0, bar);
+                        } else if (FMT == ROW_F32) {
                             tma_load_2d(dst, &p.map, piece * 64, it.lbeg + r0, bar);
-                            tma_load_2d(dst + TILE_A_TERM, &p.map, FMT == ROW_F32 ? piece * 64 + 32 : (pieces + piece) * 64, it.lbeg + r0, bar);
+                            tma_load_2d(dst + TILE_A_TERM, &p.map, piece * 64 + 32, it.lbeg + r0, bar);
                         } else {
                             tma_load_2d(dst, &p.map, piece * 64, it.lbeg + r0, bar);
                         }
