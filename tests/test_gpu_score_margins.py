@@ -152,3 +152,31 @@ def test_crowded_scores_of_every_codec(engine, oracle, quant, offset, dim, k):
         else:     # one query goes pair by pair, which is the codec's own arithmetic
             one = [ix.search(q[i:i + 1].copy(), k, nlist) for i in range(nq)]
             exactly(got, (np.concatenate([o[0] for o in one]), np.concatenate([o[1] for o in one])))
+
+
+@pytest.mark.parametrize("dim", [1024, 2048, 3000])
+@pytest.mark.parametrize("value", [1.1, 0.7001, -0.3])
+def test_sq8_rows_that_differ_by_less_than_the_constant_of_a_query_rounds(engine, oracle, dim, value):
+    """Queries of one value throughout, so that the additions behind their constant all round the same way, and rows that differ
+    from one another in two codes of opposite weight.  Each batch is routed by the engine: the constant is a warp's or a CTA's."""
+    n, nlist, k = 1200, 4, 10
+    rng = np.random.default_rng(dim)
+    codes = np.zeros((n, dim), np.float32)
+    for r, (a, b) in enumerate(rng.integers(0, dim, (n, 2))):
+        codes[r, a] = rng.integers(1, 4)
+        codes[r, b] = rng.integers(1, 4)
+    x = codes / np.float32(255)
+    lower, diff = np.zeros(dim, np.float32), np.ones(dim, np.float32)
+    q = np.full((40, dim), value, np.float32)
+    q[np.arange(40), np.arange(40)] += np.float32(1e-6) * np.arange(40, dtype=np.float32)
+    for metric in (0, 1):
+        ix = engine.IvfHandle(dim, metric, nlist, engine.QUANT_SQ8)
+        ix.set_centroids(x[:nlist])
+        ix.set_sq8_model(lower, diff)
+        ix.add(x, np.arange(n, dtype=np.int64))
+        sizes, stored, inner = ix.get_lists()
+        off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+        probes = np.tile(np.arange(nlist, dtype=np.int32), (len(q), 1))
+        want = oracle.ivf_sq8_search(stored, off, inner, lower, diff, q, probes, k, metric)
+        for nq in (1, 3, 40) if dim <= 2048 else (1, 3):      # (more of longer rows are grouped, which keeps k + 16 and checks nothing)
+            exactly(ix.search(q[:nq].copy(), k, nlist), (want[0][:nq], want[1][:nq]))

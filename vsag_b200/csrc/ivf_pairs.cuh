@@ -375,6 +375,7 @@ pairs_prepare_kernel(const PairsPrepare p) {
 // 72 candidates of 960 dimensions: 122, 97.
 // Dynamic shared memory per warp: [WARP_SELECT_CAP] keys, and the stages of warp_rows and the query where candidates are re-scored.
 constexpr int PREPARE_WARPS = 2;
+constexpr int PREPARE_SUMS = PAIR_THREADS / 32;   // partial sums of a lane: 256 of a query, as a CTA's threads have them (scan_finalize_kernel's margin)
 
 __host__ __device__ inline size_t
 prepare_warp_bytes(bool rescore, uint32_t dim) {
@@ -509,13 +510,28 @@ pairs_prepare_warps_kernel(const PairsPrepare p, uint64_t nq) {
     if (p.qw8 == nullptr) {
         return;
     }
-    float qq = 0.f, qm = 0.f, wmax = 0.f;
-    for (uint32_t d = lane; d < p.dim; d += 32) {
-        const float v = __ldg(query + d);
-        qq = fmaf(v, v, qq);
-        qm = fmaf(v, __ldg(p.mid + d), qm);
-        wmax = fmaxf(wmax, fabsf(v * __ldg(p.scale + d)));
+    float qq_part[PREPARE_SUMS] = {}, qm_part[PREPARE_SUMS] = {}, wmax = 0.f;
+    for (uint32_t d0 = lane; d0 < p.dim; d0 += 32 * PREPARE_SUMS) {
+#pragma unroll
+        for (int j = 0; j < PREPARE_SUMS; ++j) {
+            const uint32_t d = d0 + 32 * j;
+            if (d < p.dim) {
+                const float v = __ldg(query + d);
+                qq_part[j] = fmaf(v, v, qq_part[j]);
+                qm_part[j] = fmaf(v, __ldg(p.mid + d), qm_part[j]);
+                wmax = fmaxf(wmax, fabsf(v * __ldg(p.scale + d)));
+            }
+        }
     }
+#pragma unroll
+    for (int w = PREPARE_SUMS / 2; w > 0; w /= 2) {
+#pragma unroll
+        for (int j = 0; j < w; ++j) {
+            qq_part[j] += qq_part[j + w];
+            qm_part[j] += qm_part[j + w];
+        }
+    }
+    float qq = qq_part[0], qm = qm_part[0];
     for (int o = 16; o > 0; o >>= 1) {
         qq += __shfl_xor_sync(0xffffffffu, qq, o);
         qm += __shfl_xor_sync(0xffffffffu, qm, o);
@@ -1026,7 +1042,7 @@ scan_finalize_kernel(const ScanFinalize p) {
             const float chain = EPS * static_cast<float>(dim + 16);   // rounding of a chain of dim products
             if constexpr (FMT == ROW_SQ8) {
                 // The integer sums are exact, so what remains is what the terms leave out; the chains behind |x|^2 and the exact
-                // distance (X^2 and d, or X Q); the query's constant, summed by 256 threads; and the rounding of the dequantized
+                // distance (X^2 and d, or X Q); the query's constant, 256 partial sums; and the rounding of the dequantized
                 // values and of the last few operations.  (One (dim + 16) 2^-23 of (Q + X + S)^2 for all of them was five
                 // times as large: of 100 results among 390 rows a list, 960 dimensions, some queries of every batch were
                 // never sure and scored all their rows, 5.9 ms instead of 0.3.)
