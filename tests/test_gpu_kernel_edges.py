@@ -118,7 +118,8 @@ def test_routing_by_chains(engine, oracle, metric, dim, nq, nlist):
     assert np.array_equal(np.asarray(got), np.asarray(want))
 
 
-@pytest.mark.parametrize("nq,nlist", [(20, 900), (300, 1000), (300, 1500), (1300, 1500)])   # by distances, and by scores; a warp, a CTA a query
+# by distances and by scores, a warp a query (the first two, the last) and a CTA
+@pytest.mark.parametrize("nq,nlist", [(20, 900), (300, 1000), (300, 1500), (1300, 1500), (100, 1500), (1600, 1400)])
 @pytest.mark.parametrize("metric", [0, 1])
 @pytest.mark.parametrize("dim", [18, 32])                           # rows of 8- and of 16-byte alignment
 def test_routing_with_coinciding_centroids(engine, oracle, nq, nlist, metric, dim):

@@ -2452,13 +2452,20 @@ launch_prepare(const PairsPrepare& p, uint64_t nq) {
     const uint32_t wanted = p.scores != nullptr ? p.ncand : p.nprobe;
     const size_t query = p.scores != nullptr ? p.dim * sizeof(float) : 0;
     const size_t warp_smem = PREPARE_WARPS * prepare_warp_bytes(p.scores != nullptr, p.dim);
-    // A warp takes longer over a query than a CTA, the more so the more lists and the more wanted of them, but there are many warps (a CTA
-    // each / a warp each, us a search: 1 query of 1024 lists, 127 wanted 62 / 70, 32 wanted 58 / 59, of 4000 lists 62 / 82; 1000
-    // queries of 1024 lists 198 / 191, of 4000 lists 199 / 205; 2500 of those 287 / 275).  Long rows to re-score move the line (1000
-    // queries of 4096 lists, 72 candidates of 960 dimensions: the kernel takes 122 / 97).
+    // A warp takes longer over a query than a CTA, the more so the more lists and the more wanted of them, but there are many warps: from six
+    // queries an SM on they pay, where the lists are not too many for the bytes that are re-scored (a CTA's waits for those cost it more).
+    // A routing of n lists, 32 of them wanted, of so many dimensions: us with a CTA / a warp per query
+    //   1024 n  32 dims   700 84 / 84, 900 95 / 88                    2048 n  32 dims   1500 108 / 108, 2000 127 / 117
+    //   1024 n 640 dims   600 110 / 116, 900 132 / 119                2048 n 256 dims   700 92 / 105, 900 107 / 107, 1500 132 / 120
+    //   4096 n 128 dims   1500 130 / 131, 4000 226 / 223              4096 n 640 dims   900 144 / 143, 2000 214 / 190
+    //   4096 n 256 dims   900 109 / 120, 1500 143 / 143, 4000 258 / 243
+    //   8192 n 256 dims   1500 166 / 167, 3000 261 / 295              8192 n 640 dims   600 140 / 166, 1500 229 / 217
+    //   16384 n 256 dims  500 114 / 174, 1500 205 / 291               16384 n 640 dims  1500 295 / 354
+    // (8 and 100 wanted lie about the same line).  Few of few lists are as fast either way and faster with a warp where launches are all there
+    // is: whole searches, 8 of 256 lists, 1 query 61.0 / 59.4, 250 105 / 100; 32 of 1024 lists, 1 68.2 / 69.5, 100 149 / 149, 300 133 / 135.
     const bool selects = p.scores != nullptr || p.dist != nullptr;
-    const bool warps = !selects || (wanted <= 48 && p.nlist <= 1024) || nq * 1024 >= 3ull * sm_count() * (1024 + p.nlist) ||
-                       (p.scores != nullptr && p.dim >= 256 && nq >= 4ull * sm_count());
+    const bool warps = !selects || (wanted <= 48 && p.nlist <= 1024) ||
+                       (nq >= 6ull * sm_count() && nq * (p.dim + 100) >= 130ull * p.nlist);
     if (warps && wanted <= WARP_SELECT_MAX && p.nprobe <= WARP_SELECT_MAX && p.repeats == nullptr && warp_smem <= 64 * 1024) {
         VB_TRY(allow_dynamic_smem(reinterpret_cast<const void*>(pairs_prepare_warps_kernel), warp_smem));
         VB_LAUNCH(pairs_prepare_warps_kernel, static_cast<uint32_t>((nq + PREPARE_WARPS - 1) / PREPARE_WARPS), PREPARE_WARPS * 32, warp_smem, p, nq);
