@@ -825,9 +825,11 @@ struct BfSample {
     double most = 0.0;         // rows that a query may collect
 };
 constexpr uint32_t BF_COLLECT_KEYS = 12288;          // of a query, at most (96 KiB of shared memory)
-// Above this many products of one term the sample's share of them is more than the merges of bf_search_keys cost (10,000 queries, k 100,
-// 6M x 768 bf16 rows under the power limit: 89.2 ms against 87.2).
-constexpr double BF_COLLECT_PRODUCTS = 1.6e12;
+// Above this many products of one term the sample's share of them is more than the merges of bf_search_keys cost.  Calls of the two, ms:
+//   10,000 queries  1M x 128 fp32 (3.8e12) k 10 5.7 / 7.8, k 100 6.7 / 10.8     200k x 768 fp32 (4.6e12) 8.6 / 9.8, 10.9 / 12.9
+//                   6M x 256 bf16 (1.5e13) k 10 28.7 / 29.8, k 100 29.6 / 33.6  6M x 768 bf16 (4.8e13) k 100 89.2 / 87.2 (at the power limit)
+//   and below: 3000 queries of 6M x 256 bf16 (4.6e12) 8.0 / 9.9, 300 (4.6e11) 1.1 / 2.0, 30 of 1M x 128 bf16 (3.8e9) 0.14 / 0.39.
+constexpr double BF_COLLECT_PRODUCTS = 2e13;
 constexpr uint32_t BF_COLLECT_DIMS = 16384;          // the query lies beside them
 // List entries of the queries that go together, at most (2 GiB); where that is not to be had an eighth, and an eighth of that.
 constexpr uint64_t BF_COLLECT_SLOTS = uint64_t{256} << 20, BF_COLLECT_LEAST = BF_COLLECT_SLOTS / 64;

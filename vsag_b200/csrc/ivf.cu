@@ -1755,8 +1755,9 @@ route_find_bin(const uint32_t* hist, uint32_t rank, uint32_t* s_bin, uint32_t* s
     __syncthreads();
 }
 
-// thr[q] = a score that at least `rank` of query q's `sample` approximate scores (scores[q][0 .. sample)) do not exceed, and at
-// most a sixteenth more, plus a margin of 1e-3 |q| max|c| that covers the rounding of the tensor-core scores on both
+// thr[q] = a score that at least `rank` of query q's `sample` approximate scores (scores[q][0 .. sample)) do not exceed, and usually at
+// most a sixteenth more (ties at the rank, or a range that one score stretches past 2^24 times their distances, leave more: lists that
+// then overflow are route_pick_kernel's), plus a margin of 1e-3 |q| max|c| that covers the rounding of the tensor-core scores on both
 // sides: the centroids that score below it exactly score below it approximately.  A warp per query holds the scores in
 // registers and halves the range of scores in question until that few are left over, which takes about ten counts of one
 // instruction per score (as a CTA per query with two rounds of a histogram 46 us for 10,000 queries and 1024 scores each; 18).
@@ -2072,7 +2073,10 @@ route_pick_warp_kernel(const float* __restrict__ queries, uint64_t nq, uint32_t 
 // Dynamic shared memory: [2][dim] lower and diff, per warp [FINISH_KEYS] keys and the query.
 constexpr uint32_t FINISH_KEYS = WARP_SELECT_CAP;
 constexpr uint32_t FINISH_MAX_SCAN = 128, FINISH_MAX_DIM = 4096;
-// Few queries are better off with a CTA each and three launches (642 queries 22 us / 40 here, 585 with 42 keys 38 / 73, 10,000 103 / 61).
+// Few queries are better off with a CTA each and three launches, many deep ones here (4M rows of 96 dimensions in 2048 lists, 32 probed; a
+// call with three launches / with this one, us):
+//   k 10   1000 queries 539 / 526, 2500 577 / 557, 3500 596 / 574, 8000 794 / 742      k 16  1000 650 / 660, 3500 710 / 709, 8000 859 / 828
+//   k 48   1000 692 / 705, 2500 734 / 737, 3500 805 / 800, 5000 850 / 838              k 100 1000 736 / 761, 2500 810 / 807, 5000 992 / 979
 constexpr uint64_t FINISH_MIN_QUERIES = 3584;
 constexpr uint32_t FINISH_WARPS = 4;
 
@@ -3262,7 +3266,10 @@ constexpr size_t PINNED_IO_BYTES = 256 * 1024;
 // From two queries per probed list on SQ8 rows are streamed for several of them, where the rows are bytes enough to pay for the grouping
 // (as pairs / shared, us: 384 MB of rows 252 / 218, 600 MB 267 / 245, 180 MB 447 / 354, 200 MB 254 / 250; 128 MB 202 / 201, 19 MB 89 / 95).
 constexpr double SHARED_MIN_QUERIES = 2.0, SHARED_MIN_BYTES = 1.5e8;
-constexpr int FINAL_FEW = 4;               // queries an SM up to which the finalising kernel keeps its registers (see there)
+// Queries an SM up to which the finalising kernel keeps its registers (500k x 128 rows, 8 of 1024 lists; a call with them / with seven CTAs an
+// SM, us: fp32 500 queries 590 / 595, 600 185 / 172, 1500 239 / 230, 10,000 994 / 898; SQ8 256 209 / 206, 500 296 / 301, 600 178 / 172,
+// 5000 482 / 444).
+constexpr int FINAL_FEW = 4;
 constexpr double TILE_MIN_QUERIES = 4.0;   // queries per probed list from which tiles pay (3.1: 141 us as pairs, 162 as tiles)
 
 // Shared memory of pair_scan_kernel and of scan_finalize_kernel; qstride: floats of a query as the codec's chain reads it (the
