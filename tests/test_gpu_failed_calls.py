@@ -223,3 +223,26 @@ def test_a_batch_that_lacks_memory_gives_up_the_second_copy(engine):
     one = [ix.search(q[i:i + 1].copy(), 5, 16) for i in range(20)]
     for j in (0, 1):
         assert np.array_equal(got[j][:20], np.concatenate([o[j] for o in one]))
+
+
+def test_a_refused_launch_does_not_fail_the_next_call(engine):
+    """A batch that is grouped over SQ8 rows of 3100 dimensions asks for more shared memory than there is and ends with an error;
+    calls on other handles, and small ones on this, go on."""
+    from vsag_b200 import _capi
+
+    dim, n = 3100, 300
+    x = mixture(12, n, dim, 4, 0.2)
+    ix = engine.IvfHandle(dim, 0, 4, engine.QUANT_SQ8)
+    ix.set_centroids(x[:4].copy())
+    ix.set_sq8_model(x.min(0), x.max(0) - x.min(0))
+    ix.add(x, np.arange(n, dtype=np.int64))
+    want = ix.search(x[:1].copy(), 3, 4)
+    with pytest.raises(_capi.VsagB200Error):
+        ix.search(x[:40].copy(), 3, 4)
+    bf = engine.BfHandle(24, 0)
+    bf.add(x[:, :24].copy(), np.arange(n, dtype=np.int64))
+    assert np.array_equal(bf.search(x[:5, :24].copy(), 1)[0][:, 0], np.arange(5))
+    with pytest.raises(_capi.VsagB200Error):
+        ix.search(x[:40].copy(), 3, 4)
+    again = ix.search(x[:1].copy(), 3, 4)
+    assert np.array_equal(again[0], want[0]) and np.array_equal(again[1], want[1])

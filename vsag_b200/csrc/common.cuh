@@ -46,6 +46,7 @@ int last_error_code();
     do {                                                                                    \
         cudaError_t _e = (expr);                                                            \
         if (_e != cudaSuccess) {                                                            \
+            (void)cudaGetLastError(); /* reported here, so not by the next call's launches */ \
             int _c = (_e == cudaErrorMemoryAllocation) ? VB200_NO_ENOUGH_MEMORY             \
                                                        : VB200_INTERNAL_ERROR;              \
             VB_FAIL(_c, "%s failed at %s:%d: %s", #expr, __FILE__, __LINE__,                \
