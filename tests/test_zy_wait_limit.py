@@ -78,3 +78,22 @@ def test_a_grouped_scan_that_gave_up_does_not_fail_the_next_tiled_one(engine):
     for k, want in ((200, deep), (5, shallow)):
         again = ix.search(q, k, 8)
         assert np.array_equal(again[0], want[0]) and np.array_equal(again[1], want[1])
+
+
+@pytest.mark.parametrize("n,dim", [(5000, 40), (90_000, 128)])      # rows that stay on the chip, and rows that are streamed
+def test_seeding_wait_runs_out_then_recovers(engine, oracle, n, dim):
+    """The CTAs of the seeding kernel poll one another's words."""
+    from vsag_b200 import _capi
+
+    x = mixture(407, n, dim, 16, 0.2)
+    want = engine.kmeans_init(x, 12, 47)
+    lib = _capi.load()
+    assert lib.vb200_debug_set_wait_limit(0) == 0
+    try:
+        with pytest.raises(_capi.VsagB200Error) as err:
+            engine.kmeans_init(x, 12, 47)
+        assert err.value.code == -2 and "bounded wait" in str(err.value)
+    finally:
+        assert lib.vb200_debug_set_wait_limit(-1) == 0
+    assert np.array_equal(engine.kmeans_init(x, 12, 47), want)
+    assert np.array_equal(want, oracle.kmeans_pp_init(x, 12, 47)[0])
