@@ -66,9 +66,6 @@ struct TcParams {
     uint64_t* out;            // [a.rows][n_split][TC_COL_GROUPS][m] keys (ordered score << 32 | column), KEY_INF padded
                               // (threshold mode: [a.rows][n_split][TC_COL_GROUPS][cap], unsorted, with out_count)
     uint32_t* out_count;      // threshold mode: [a.rows][n_split][TC_COL_GROUPS] entries offered to each list
-    uint64_t* spill;          // spill mode: [a.rows][spill_cap] entries that a list had no room for, with spill_count [a.rows]
-    uint32_t* spill_count;
-    uint32_t spill_cap;
     uint32_t col_base;        // added to column indices in the keys
     float* store;             // score-matrix mode: [a.rows][store_ld] fp32 scores instead of candidates
                               // (minima mode: the smallest score of every 32 columns)
@@ -79,6 +76,9 @@ struct TcParams {
     uint32_t* row_flags;      // m <= 4 mode with a margin, optional: [a.rows], set to 1 for a row one of whose
                               // lists ended full of columns within the margin of its best -- a column the list
                               // had no room for might be the exact winner, so the caller decides such rows exactly
+    uint64_t* spill;          // spill mode: [a.rows][spill_cap] entries that a list had no room for, with spill_count [a.rows]
+    uint32_t* spill_count;
+    uint32_t spill_cap;
 };
 
 // A kernel whose wait ran out returns only after this pause, so that the copies and MMAs it still
@@ -361,7 +361,7 @@ struct TcCollect {
     uint32_t n_split, tiles_per_split, lists, cap;
 };
 TcCollect tc_collect_plan(uint64_t a_rows, uint64_t b_rows, double expected_per_row);
-// What the lists of a row have no room for: rows stored near one another may all fall into a few lists.
+// Where a list that may not hold another block of 32 columns goes: rows stored near one another may all fall into a few lists.
 struct TcSpill {
     uint64_t* keys;      // [a.rows][cap]
     uint32_t* count;     // [a.rows] entries offered; zero before the launch
