@@ -61,6 +61,7 @@ struct TcParams {
     uint32_t diag;            // timing experiments only: bit 0 skips the selection, bit 1 the MMAs
 #endif
     uint32_t last_steps;      // k-steps of 16 of the last chunk that hold anything
+    uint32_t tile_factor;     // 1 (see tc_candidates_kernel)
     uint32_t interleaved;     // 1: share s holds tiles s, s + n_split, ...; the queue walks row tiles within a share
     uint64_t* scratch;        // [grid][128][TC_COL_GROUPS][cap] candidate buffers
     uint64_t* out;            // [a.rows][n_split][TC_COL_GROUPS][m] keys (ordered score << 32 | column), KEY_INF padded
